@@ -41,6 +41,11 @@ class EpPeers(C.Structure):
     _fields_ = [("rank", C.c_int), ("world", C.c_int), ("base", C.c_void_p * 8)]
 
 
+class DecStepArgs(C.Structure):
+    _fields_ = [(n, C.c_int) for n in ("B", "Tm", "L", "D", "H", "KV", "F", "E", "K")] + \
+               [(n, C.c_void_p) for n in ("layers", "emb", "tok", "pos", "cosb", "sinb", "nf", "fn", "ws")]
+
+
 PROTOTYPES = {
     "qlmb_last_error": (C.c_char_p, []),
     "qlmb_version": (ci, []),
@@ -95,6 +100,8 @@ PROTOTYPES = {
     "qlmb_gemv_decode_norm_stack": (ci, [vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, vp]),
     "qlmb_dec_qkv": (ci, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, vp]),
     "qlmb_gemv_decode_res_norm": (ci, [vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, vp]),
+    "qlmb_dec_step_bytes": (sz, [ci] * 8),
+    "qlmb_dec_step": (ci, [C.POINTER(DecStepArgs), vp]),
     "qlmb_dec_rope": (ci, [vp, ci, vp, vp, vp, ci, ci, ci, ci, vp]),
     "qlmb_dec_kv": (ci, [vp, vp, vp, vp, vp, ci, ci, ci, vp]),
     "qlmb_dec_attn": (ci, [vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, ci, vp]),

@@ -27,6 +27,7 @@ UNITS = {
     "qlmb_gemm.cu": [],
     "qlmb_linear.cu": [],
     "qlmb_gemv.cu": [],
+    "qlmb_decstep.cu": ["--fmad=false"],
     "qlmb_moe.cu": [],
     "qlmb_statefile.cu": [],
     "qlmb_q4n.cu": ["--fmad=false"],

@@ -1,0 +1,806 @@
+// One decode step's layers in ONE persistent launch (dec_step, cudalm.cu:7168-7212), up to eight live slots: embedding, then
+// per layer the q, k, v projections with the norm in front, cached attention, output projection + residual + norm,
+// router, the routed experts and their combination, and the final norm.  With so few rows a layer is 5 MB of weights,
+// which the memory system delivers in under a microsecond; what a step costs is latency: the chain of launches that
+// this replaces spent 4-6 us in each of nine launches per layer.
+//
+// One CTA of 512 threads per SM (cooperative launch); the seven phases of a layer are separated by grid barriers of about
+// 1100 cycles.  Between two barriers the longest chain of dependent instructions sets the time (about five cycles
+// each), so every phase is written for a short one:
+//   - a weight phase is a set of tasks of 256 output columns x 128 contraction rows: a warp takes eight rows, a lane one
+//     code word (eight columns) of each, so a load instruction covers a whole 128-byte line, the sums of a column stay
+//     in one lane, and the 16 warps' sums meet once in shared memory;
+//   - codes and scales of a phase whose choice of weights is known are in registers before its barrier is waited for;
+//   - slice sums go to the consumer as they are and are added there (its loads are independent of one another), in a
+//     fixed order, so a step is reproducible bit for bit;
+//   - the cached keys and values of an attention phase and the router's matrix reach shared memory before their barrier.
+// Products are fp32: x * scale times the exact digit, as in the kernels of the separate entry points.
+// Measured (12 layers, D 768, 32 experts top-2 of d_ff 1536, 128-256 cached positions, whole step with the head, a CUDA
+// graph replay): one slot 615 -> 285 us, eight slots 801 -> 511 us.  Above eight slots the chain stays: there the
+// experts' weights are a stream and no longer a latency.
+//
+// Built with --fmad=false (router arithmetic); fused multiply-adds are written out.
+#include <cuda_bf16.h>
+#include <string.h>
+#include "qlmb_common.cuh"
+#include "qlmb_internal.h"
+#include "qlmb_topk.cuh"
+
+namespace qlmb {
+
+struct DsLayer {                                          // the device table's row: pointers only (qlmb_dec_step_args)
+    const uint8_t *c[7];                                  // codes of wq, wk, wv, wo, w1, w3, w2
+    const float *s[7];                                    // their group scales
+    const float *an1, *an2, *wr;
+    bf16 *Kc, *Vc;
+    float *rt, *rprobs;
+    int *assign;
+    float *gate;
+};
+constexpr int DS_LAYER_WORDS = sizeof(DsLayer) / 8;
+
+struct DsArgs {
+    const DsLayer *layers;
+    int L, B, D, KD, H, KV, F, E, K, Tm;
+    int tq, td, tf;                                       // column tiles of q|k|v, of D and of F
+    uint32_t mq, md, mf, mr, mfs;                         // ceil(2^32 / n) of those and of the row slices of D and F
+    const float *emb; const int *tok, *pos; const float *cosb, *sinb, *nf;
+    bf16 *fn;
+    // workspace
+    unsigned *bar;
+    bf16 *x, *xn, *att, *fi, *fnorm;
+    float *pq, *po, *pg, *pd;                             // slice sums: [D/128][B][NQ], [D/128][B][D], [D/128][2 R][F], [F/128][R][D]
+    int *errword;
+};
+
+constexpr int DS_THREADS = 512, DS_WARPS = 16;
+constexpr int DS_ROWS = 128;                              // contraction rows of a task: eight per warp
+constexpr int DS_COLS = 256;
+constexpr int DS_MAX_B = 8, DS_MAX_R = 32;
+constexpr int DS_MAX_SL = 8;                              // row slices of D (D <= 1024)
+constexpr int DS_RED = DS_WARPS * 4 * DS_COLS * 4;        // up to four rows' sums of the 16 warps
+constexpr int DS_WR = 1024 * 32 * 4;                      // the router's matrix, or keys and values of an attention phase
+constexpr int DS_XS = 2 * DS_ROWS * 4;
+constexpr int DS_SLOT = DS_ROWS * 136, DS_DEPTH = 7;      // a task's codes and scales; tasks on their way (in the place of DS_WR)
+static_assert(DS_DEPTH * DS_SLOT <= DS_WR, "ring");
+constexpr int DS_SMEM = DS_RED + DS_WR + DS_XS;
+
+__device__ __forceinline__ uint32_t ds_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ds_cp16(uint32_t dst, const void *src)
+{ asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void ds_cp4(uint32_t dst, const void *src)
+{ asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void ds_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void ds_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ float ds_bf(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+__device__ __forceinline__ float ds_lo(uint32_t x) { return __uint_as_float(x << 16); }
+__device__ __forceinline__ float ds_hi(uint32_t x) { return __uint_as_float(x & 0xffff0000u); }
+__device__ __forceinline__ uint32_t ds_pack(float a, float b)
+{
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+__device__ __forceinline__ float4 ds_ld4(const float *p) { return __ldcg(reinterpret_cast<const float4 *>(p)); }
+__device__ __forceinline__ float4 ds_ldrow(const bf16 *p)
+{
+    const uint2 u = __ldcg(reinterpret_cast<const uint2 *>(p));
+    return make_float4(ds_lo(u.x), ds_hi(u.x), ds_lo(u.y), ds_hi(u.y));
+}
+__device__ __forceinline__ void ds_strow(bf16 *p, float4 v) { *reinterpret_cast<uint2 *>(p) = make_uint2(ds_pack(v.x, v.y), ds_pack(v.z, v.w)); }
+__device__ __forceinline__ float4 ds_bf4(float4 v) { return make_float4(ds_bf(v.x), ds_bf(v.y), ds_bf(v.z), ds_bf(v.w)); }
+__device__ __forceinline__ void ds_add4(float4 &a, const float4 b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
+__device__ __forceinline__ void ds_fma4(float4 &a, float g, const float4 b)
+{ a.x = __fmaf_rn(g, b.x, a.x); a.y = __fmaf_rn(g, b.y, a.y); a.z = __fmaf_rn(g, b.z, a.z); a.w = __fmaf_rn(g, b.w, a.w); }
+
+struct Shared {
+    DsLayer layer[2];
+    unsigned target;                                      // grid barrier: arrivals that the next wait needs
+    int pos[DS_MAX_B];
+    int npair, pexp[DS_MAX_R];                            // distinct experts of the step and their slots
+    unsigned pmask[DS_MAX_R];
+    float red[DS_WARPS];
+    float am[DS_WARPS], al[DS_WARPS];                     // attention: the warps' maxima and sums
+    float q[64];
+    alignas(16) bf16 kv[128];
+    float part[DS_WARPS * 64];
+    float logit[DS_WARPS * 32];
+};
+
+// ---- grid barrier: one monotonic counter per launch, reset by the last CTA to leave the kernel.  The wait is bounded by
+// two seconds of %globaltimer; when it runs out the abort word makes every later wait return at once.
+__device__ __forceinline__ unsigned long long ds_now() { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
+__device__ __forceinline__ void gb_arrive(const DsArgs &a, Shared &sh)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        sh.target += gridDim.x;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+    }
+}
+__device__ __noinline__ void gb_slow(unsigned *bar, unsigned target, int *errword)
+{
+    unsigned long long t0 = 0;
+    for (unsigned i = 0;; i++) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+        if (v >= target) return;
+        if ((i & 1023u) == 1023u) {
+            if (*(volatile unsigned *)(bar + 2)) return;
+            const unsigned long long t = ds_now();
+            if (!t0) t0 = t;
+            else if (t - t0 > 2000000000ull) {
+                if (atomicExch(bar + 2, 1u) == 0u && errword && atomicCAS(errword, 0, 200) == 0) {
+                    errword[1] = 400; errword[2] = (int)blockIdx.x; errword[3] = (int)target;
+                }
+                return;
+            }
+        }
+    }
+}
+__device__ __forceinline__ void gb_wait(const DsArgs &a, Shared &sh)
+{
+    if (threadIdx.x == 0) gb_slow(a.bar, sh.target, a.errword);
+    __syncthreads();
+}
+
+// ---- weight phases
+__device__ __forceinline__ int ds_div(int x, int n, uint32_t m) { return n == 1 ? x : (int)__umulhi((uint32_t)x, m); }   // m = ceil(2^32 / n)
+struct Words { uint32_t w[8]; float s[8]; };              // eight rows of a lane's eight columns, and their group scales
+__device__ __forceinline__ void ds_words(Words &r, const uint8_t *codes, const float *scales, int N, int col, int k0)
+{
+    const uint8_t *cp = codes + (size_t)k0 * (N >> 1) + (col >> 1);
+    const float *sp = scales + (size_t)k0 * (N >> 7) + (col >> 7);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        r.w[i] = __ldcs(reinterpret_cast<const uint32_t *>(cp));
+        r.s[i] = __ldg(sp);
+        cp += N >> 1; sp += N >> 7;
+    }
+}
+// eight nibbles of a code word as exact floats (two's complement, element 0 in the low nibble): a byte in 0..15 under
+// the exponent of 2^23 is 8388608 + byte, and (nibble ^ 8) - 8 is the value
+template <int C>
+__device__ __forceinline__ void ds_mul(const Words &r, const float (&x)[C][8], float (&acc)[C][8])
+{
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t w = r.w[i] ^ 0x88888888u, ev = w & 0x0F0F0F0Fu, od = (w >> 4) & 0x0F0F0F0Fu;
+        float d[8];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            d[2 * j] = __uint_as_float(__byte_perm(ev, 0x4B000000u, 0x7440 + j)) - 8388616.0f;
+            d[2 * j + 1] = __uint_as_float(__byte_perm(od, 0x4B000000u, 0x7440 + j)) - 8388616.0f;
+        }
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            const float xv = x[c][i] * r.s[i];
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc[c][j] = i == 0 ? xv * d[j] : __fmaf_rn(xv, d[j], acc[c][j]);
+        }
+    }
+}
+__device__ __forceinline__ void ds_x8(float (&x)[8], uint4 u)
+{
+    x[0] = ds_lo(u.x); x[1] = ds_hi(u.x); x[2] = ds_lo(u.y); x[3] = ds_hi(u.y);
+    x[4] = ds_lo(u.z); x[5] = ds_hi(u.z); x[6] = ds_lo(u.w); x[7] = ds_hi(u.w);
+}
+// the 16 warps' sums of C rows -> out[row(c) * N + col0 + column], warp order.  The caller syncs before `red` is used again.
+template <int C, typename RowPtr>
+__device__ __forceinline__ void ds_reduce(float *red, const float (&acc)[C][8], int n, int col0, int N, RowPtr row)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+        float4 *p = reinterpret_cast<float4 *>(red + (warp * C + c) * DS_COLS + lane * 8);
+        p[0] = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+        p[1] = make_float4(acc[c][4], acc[c][5], acc[c][6], acc[c][7]);
+    }
+    __syncthreads();
+    const int col = threadIdx.x & 255;
+    if (col0 + col < N) {
+#pragma unroll 1
+        for (int c = threadIdx.x >> 8; c < n; c += 2) {
+            float v = 0.0f;
+#pragma unroll
+            for (int w = 0; w < DS_WARPS; w++) v += red[(w * C + c) * DS_COLS + col];
+            __stcg(row(c) + col0 + col, v);
+        }
+    }
+}
+
+// q, k, v projections (KIND 0) and output projection (KIND 1): a task takes C of the B rows
+template <int KIND, int C>
+__device__ __forceinline__ void ds_dense(const DsArgs &a, Shared &sh, const DsLayer &ly, float *red)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tiles = KIND == 0 ? a.tq : a.td, NT = KIND == 0 ? a.D + 2 * a.KD : a.D, sl = a.D / DS_ROWS, n = tiles * sl * ((a.B + C - 1) / C);
+    const bf16 *X = KIND == 0 ? a.xn : a.att;
+    float *out = KIND == 0 ? a.pq : a.po;
+    bool first = true;
+#pragma unroll 1
+    for (int task = blockIdx.x; task < n; task += gridDim.x) {
+        const int ts = ds_div(task, tiles, KIND == 0 ? a.mq : a.md), col0 = (task - ts * tiles) * DS_COLS, ch = ds_div(ts, sl, a.mr);
+        const int slice = ts - ch * sl, k0 = slice * DS_ROWS + warp * 8, b0 = ch * C;
+        int col = col0 + lane * 8;
+        if (col >= NT) col = NT - 8;                      // lanes past the last column repeat it and are not read
+        int m = 3, N = a.D;
+        if (KIND == 0) {
+            m = 0;
+            if (col >= a.D) { col -= a.D; m = 1; N = a.KD; if (col >= a.KD) { col -= a.KD; m = 2; } }
+        }
+        Words w;
+        ds_words(w, ly.c[m], ly.s[m], N, col, k0);
+        if (first) { gb_wait(a, sh); first = false; } else __syncthreads();
+        uint4 xr[C];
+#pragma unroll
+        for (int c = 0; c < C; c++) xr[c] = b0 + c < a.B ? __ldcg(reinterpret_cast<const uint4 *>(X + (size_t)(b0 + c) * a.D + k0)) : make_uint4(0u, 0u, 0u, 0u);
+        float x[C][8], acc[C][8];
+#pragma unroll
+        for (int c = 0; c < C; c++) ds_x8(x[c], xr[c]);
+        ds_mul<C>(w, x, acc);
+        ds_reduce<C>(red, acc, a.B - b0 < C ? a.B - b0 : C, col0, NT, [&](int c) { return out + ((size_t)slice * a.B + b0 + c) * NT; });
+    }
+    if (first) gb_wait(a, sh);
+}
+
+// The experts' tasks.  An expert has one or two slots as a rule: a pass multiplies up to two, and the weights, the first
+// pass's activations and, in the down projection, the gate and up sums they are made of are requested a task ahead.
+struct ExTask { int pair, mat, slice, tile, s0, s1, n; unsigned rest; };     // s0, s1: the pass's slots (n of them), rest: those that follow
+__device__ __forceinline__ void ds_pass(ExTask &t, unsigned mask)
+{
+    t.s0 = __ffs(mask) - 1;
+    mask &= mask - 1;
+    t.n = mask ? 2 : 1;
+    t.s1 = mask ? __ffs(mask) - 1 : t.s0;
+    t.rest = mask & (mask - 1);
+}
+template <bool DOWN>
+__device__ __forceinline__ ExTask ds_ex_task(const DsArgs &a, const Shared &sh, int item)
+{
+    ExTask t;
+    if (DOWN) {
+        const int fs = a.F / DS_ROWS, q = ds_div(item, a.td, a.md);
+        t.tile = item - q * a.td; t.mat = 0;
+        t.pair = ds_div(q, fs, a.mfs);
+        t.slice = q - t.pair * fs;
+    } else {
+        const int sl = a.D / DS_ROWS, q = ds_div(item, a.tf, a.mf), pm = ds_div(q, sl, a.mr);
+        t.tile = item - q * a.tf;
+        t.slice = q - pm * sl;
+        t.mat = pm & 1; t.pair = pm >> 1;
+    }
+    ds_pass(t, sh.pmask[t.pair]);
+    return t;
+}
+// The codes and scales of a task go through a ring in shared memory, DS_DEPTH tasks ahead: with one task (17 KB per SM)
+// ahead a round of tasks took a memory latency.  Every warp copies and reads its own eight rows only.
+template <bool DOWN>
+__device__ __forceinline__ void ds_ex_request(const DsArgs &a, const Shared &sh, const DsLayer &ly, uint8_t *ring, int slot, const ExTask &t)
+{
+    const int N = DOWN ? a.D : a.F, m = DOWN ? 6 : 4 + t.mat, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t mat = (size_t)sh.pexp[t.pair] * a.D * a.F;
+    const int k0 = t.slice * DS_ROWS + warp * 8, r = lane >> 3, c = lane & 7;
+    const uint32_t d = ds_smem(ring + slot * DS_SLOT);
+    const bool in = t.tile * DS_COLS + c * 32 < N;        // N is a multiple of 128: the last tile may be half as wide
+    const uint8_t *p = ly.c[m] + mat / 2 + (size_t)(k0 + r) * (N >> 1) + (in ? t.tile * 128 + c * 16 : 0);
+    if (in) {
+        ds_cp16(d + warp * 1024 + lane * 16, p);
+        ds_cp16(d + warp * 1024 + 512 + lane * 16, p + (size_t)4 * (N >> 1));
+    }
+    const int g = 2 * t.tile + (lane & 1);
+    if (lane < 16 && g < (N >> 7)) ds_cp4(d + 16384 + warp * 64 + lane * 4, ly.s[m] + mat / 128 + (size_t)(k0 + (lane >> 1)) * (N >> 7) + g);
+}
+__device__ __forceinline__ void ds_ring_words(Words &w, const uint8_t *ring, int slot)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint8_t *p = ring + slot * DS_SLOT + warp * 1024 + lane * 4, *q = ring + slot * DS_SLOT + 16384 + warp * 64 + (lane >> 4) * 4;
+#pragma unroll
+    for (int i = 0; i < 8; i++) { w.w[i] = *reinterpret_cast<const uint32_t *>(p + i * 128); w.s[i] = *reinterpret_cast<const float *>(q + i * 8); }
+}
+// gate/up: this warp's eight activations of the pass's two slots
+struct GuActs { uint4 x0, x1; };
+__device__ __forceinline__ void ds_gu_acts(const DsArgs &a, GuActs &x, const ExTask &t)
+{
+    const bf16 *p = a.fnorm + t.slice * DS_ROWS + (threadIdx.x >> 5) * 8;
+    x.x0 = __ldcg(reinterpret_cast<const uint4 *>(p + (size_t)(t.s0 % a.B) * a.D));
+    x.x1 = __ldcg(reinterpret_cast<const uint4 *>(p + (size_t)(t.s1 % a.B) * a.D));
+}
+// down: gate and up sums of one row of the slice (threads 0 .. 127: first slot, 128 .. 255: second)
+struct DnActs { float g[DS_MAX_SL], u[DS_MAX_SL]; };
+__device__ __forceinline__ void ds_dn_acts(const DsArgs &a, DnActs &x, const ExTask &t)
+{
+    const int R = a.K * a.B, ns = a.D / DS_ROWS;
+    if ((int)threadIdx.x >= t.n * DS_ROWS) return;
+    const float *p = a.pg + (size_t)((int)threadIdx.x < DS_ROWS ? t.s0 : t.s1) * a.F + t.slice * DS_ROWS + (threadIdx.x & (DS_ROWS - 1));
+#pragma unroll
+    for (int s = 0; s < DS_MAX_SL; s++) {
+        x.g[s] = s < ns ? __ldcg(p) : 0.0f;
+        x.u[s] = s < ns ? __ldcg(p + (size_t)R * a.F) : 0.0f;
+        p += (size_t)2 * R * a.F;
+    }
+}
+__device__ __forceinline__ float ds_swiglu(const DnActs &x)
+{
+    float g = 0.0f, u = 0.0f;
+#pragma unroll
+    for (int s = 0; s < DS_MAX_SL; s++) { g += x.g[s]; u += x.u[s]; }
+    g = ds_bf(g); u = ds_bf(u);
+    return ds_bf(g * __fdividef(1.0f, 1.0f + __expf(-g)) * u);
+}
+template <bool DOWN, int C>
+__device__ __forceinline__ void ds_ex_pass(const DsArgs &a, float *red, const float *xs, const Words &w, const ExTask &t, const GuActs &xa)
+{
+    const int warp = threadIdx.x >> 5, R = a.K * a.B, N = DOWN ? a.D : a.F;
+    float x[C][8], acc[C][8];
+    if (DOWN) {
+#pragma unroll
+        for (int c = 0; c < C; c++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float4 v = *reinterpret_cast<const float4 *>(xs + c * DS_ROWS + warp * 8 + 4 * h);
+                x[c][4 * h] = v.x; x[c][4 * h + 1] = v.y; x[c][4 * h + 2] = v.z; x[c][4 * h + 3] = v.w;
+            }
+    } else {
+        ds_x8(x[0], xa.x0);
+        if (C > 1) ds_x8(x[C - 1], xa.x1);
+    }
+    ds_mul<C>(w, x, acc);
+    float *out = DOWN ? a.pd + (size_t)t.slice * R * a.D : a.pg + (size_t)(t.slice * 2 + t.mat) * R * a.F;
+    ds_reduce<C>(red, acc, t.n, t.tile * DS_COLS, N, [&](int c) { return out + (size_t)(c == 0 ? t.s0 : t.s1) * N; });
+}
+// The down projection's choice of weights is known: its barrier is waited for with the first tasks' weights on their way.
+template <bool DOWN>
+__device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, const DsLayer &ly, float *red, float *xs, uint8_t *ring, bool multi)
+{
+    const int n = DOWN ? sh.npair * (a.F / DS_ROWS) * a.td : sh.npair * 2 * (a.D / DS_ROWS) * a.tf;
+    int ask = blockIdx.x, item = blockIdx.x, slot = 0;
+#pragma unroll 1
+    for (int k = 0; k < DS_DEPTH; k++) {
+        if (ask < n) ds_ex_request<DOWN>(a, sh, ly, ring, k, ds_ex_task<DOWN>(a, sh, ask));
+        ds_commit();
+        ask += gridDim.x;
+    }
+    if (DOWN) gb_wait(a, sh);
+    if (item >= n) return;
+    ExTask t = ds_ex_task<DOWN>(a, sh, item);
+    GuActs ga;
+    DnActs da;
+    if (DOWN) ds_dn_acts(a, da, t); else ds_gu_acts(a, ga, t);
+    Words w;
+    bool fresh = true;
+#pragma unroll 1
+    for (;;) {
+        if (DOWN) {                                       // the slice's activations of this pass
+            if ((int)threadIdx.x < t.n * DS_ROWS) xs[threadIdx.x] = ds_swiglu(da);
+            __syncthreads();
+        }
+        if (fresh) {
+            ds_wait<DS_DEPTH - 1>();
+            __syncwarp();
+            ds_ring_words(w, ring, slot);
+            __syncwarp();
+            if (ask < n) ds_ex_request<DOWN>(a, sh, ly, ring, slot, ds_ex_task<DOWN>(a, sh, ask));
+            ds_commit();
+            ask += gridDim.x;
+            if (++slot == DS_DEPTH) slot = 0;
+        }
+        const ExTask cur = t;
+        const GuActs xa = ga;
+        fresh = !(multi && t.rest);                       // else: more slots of the same expert, same weights
+        if (!fresh) ds_pass(t, t.rest);
+        else {
+            item += gridDim.x;
+            if (item < n) t = ds_ex_task<DOWN>(a, sh, item);
+        }
+        if (item < n) { if (DOWN) ds_dn_acts(a, da, t); else ds_gu_acts(a, ga, t); }
+        if (multi && cur.n == 2) ds_ex_pass<DOWN, 2>(a, red, xs, w, cur, xa);
+        else ds_ex_pass<DOWN, 1>(a, red, xs, w, cur, xa);
+        if (item >= n) break;
+        __syncthreads();
+    }
+    ds_wait<0>();
+}
+
+// ---- attention of one (slot, head) by a CTA: the head's q, k, v rows from the projection's slice sums, rotation, cache
+// append; then every warp takes 16 of each 256 keys on its own with a running maximum, and the warps' results are merged
+// at the end.  Keys and values reach shared memory by asynchronous copies, four whole 128-byte rows per instruction (a
+// lane per key, eight 16-byte loads in 32 different lines each, held the load path for 6.5 thousand cycles per 256 keys):
+// the first 256 at the layer's start, the next ones while these are multiplied.  Lane (r = lane / 8, c = lane % 8)
+// multiplies dimensions 8c .. 8c + 7 of the keys 4i + r.
+constexpr int DS_KV = 16 * 256;                           // bytes of a warp's keys and values of one pass
+__device__ __forceinline__ void ds_kv_request(const DsArgs &a, const Shared &sh, const DsLayer &ly, uint8_t *kvs, int item, int blk)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, b = item / a.H, h = item - b * a.H, kvh = h / (a.H / a.KV);
+    const int t = sh.pos[b], s0 = blk * 256 + warp * 16, left = t < 0 || t >= a.Tm ? 0 : t - s0, r = lane >> 3;
+    if (left > 0) {
+        const size_t base = ((size_t)b * a.Tm + s0) * a.KD + kvh * 64 + (lane & 7) * 8;
+        const uint32_t d = ds_smem(kvs + (blk & 1) * DS_WARPS * DS_KV + warp * DS_KV) + lane * 16;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {                     // rows past the end repeat the first one and get no weight
+            const int k = (4 * i + r < left ? 4 * i + r : 0) * a.KD;
+            ds_cp16(d + i * 512, ly.Kc + base + k);
+            ds_cp16(d + i * 512 + 2048, ly.Vc + base + k);
+        }
+    }
+    ds_commit();
+}
+__device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const DsLayer &ly, uint8_t *kvs)
+{
+    const int item = blockIdx.x;
+    if (item >= a.B * a.H) { gb_wait(a, sh); return; }
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, b = item / a.H, h = item - b * a.H, rep = a.H / a.KV, kvh = h / rep;
+    const int t = sh.pos[b], r = lane >> 3, c8 = (lane & 7) * 8, mm = tid >> 6, i64 = tid & 63;
+    float *sc = sh.logit + warp * 16;                     // this warp's scores
+    const bool bad = t < 0 || t >= a.Tm;                  // a slot past its cache: nothing of it is read or written
+    float cs = 0.0f, sn = 0.0f;
+    if (tid < 128 && !bad) { cs = __ldg(a.cosb + (size_t)t * 32 + (i64 & 31)); sn = __ldg(a.sinb + (size_t)t * 32 + (i64 & 31)); }
+    gb_wait(a, sh);
+    if (bad) {
+        ds_wait<0>();
+        if (tid == 0 && h == 0) report_bad_index(a.errword, 302, b, t);
+        if (tid < 64) a.att[(size_t)b * a.D + h * 64 + tid] = __float2bfloat16_rn(0.0f);
+        return;
+    }
+    float x = 0.0f;
+    if (tid < 192) {                                      // one of the 64 columns of q, k or v
+        const int NQ = a.D + 2 * a.KD, ns = a.D / DS_ROWS;
+        const float *pp = a.pq + (size_t)b * NQ + (mm == 0 ? h * 64 : a.D + (mm - 1) * a.KD + kvh * 64) + i64;
+        float pv[DS_MAX_SL];
+#pragma unroll
+        for (int k = 0; k < DS_MAX_SL; k++) { pv[k] = k < ns ? __ldcg(pp) : 0.0f; pp += a.B * NQ; }
+#pragma unroll
+        for (int k = 0; k < DS_MAX_SL; k++) x += pv[k];
+        x = ds_bf(x);
+        sh.part[tid] = x;
+    }
+    __syncthreads();
+    if (tid < 192) {
+        if (mm < 2) {                                     // pairs (i, i + 32) of q and k
+            const float y = sh.part[tid ^ 32];
+            x = i64 < 32 ? x * cs - y * sn : x * cs + y * sn;
+        }
+        const bf16 xb = __float2bfloat16_rn(x);
+        if (mm == 0) sh.q[i64] = __bfloat162float(xb);
+        else {
+            sh.kv[tid - 64] = xb;
+            if (h == kvh * rep) (mm == 1 ? ly.Kc : ly.Vc)[((size_t)b * a.Tm + t) * a.KD + kvh * 64 + i64] = xb;
+        }
+    }
+    __syncthreads();
+    float m = -1e30f, l = 0.0f, o[8], q[8];
+#pragma unroll
+    for (int d = 0; d < 8; d++) { o[d] = 0.0f; q[d] = sh.q[c8 + d]; }
+#pragma unroll 1
+    for (int blk = 0; blk * 256 <= t; blk++) {
+        const int left = t - blk * 256 - warp * 16;       // this warp's keys 0 .. left of the pass, the last one new
+        uint8_t *mine = kvs + (blk & 1) * DS_WARPS * DS_KV + warp * DS_KV;
+        if ((blk + 1) * 256 <= t) { ds_kv_request(a, sh, ly, kvs, item, blk + 1); ds_wait<1>(); }
+        else ds_wait<0>();
+        if (left < 0) continue;
+        if (left < 16 && r < 2)                           // the new key and value are not read back from the cache
+            *reinterpret_cast<uint4 *>(mine + r * 2048 + left * 128 + c8 * 2) = *reinterpret_cast<const uint4 *>(sh.kv + r * 64 + c8);
+        __syncwarp();
+        float d[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint4 k = *reinterpret_cast<const uint4 *>(mine + i * 512 + lane * 16);
+            float d0 = q[0] * ds_lo(k.x), d1 = q[1] * ds_hi(k.x);
+            d0 = __fmaf_rn(q[2], ds_lo(k.y), d0); d1 = __fmaf_rn(q[3], ds_hi(k.y), d1);
+            d0 = __fmaf_rn(q[4], ds_lo(k.z), d0); d1 = __fmaf_rn(q[5], ds_hi(k.z), d1);
+            d0 = __fmaf_rn(q[6], ds_lo(k.w), d0); d1 = __fmaf_rn(q[7], ds_hi(k.w), d1);
+            d[i] = d0 + d1;
+        }
+#pragma unroll
+        for (int y = 1; y < 8; y <<= 1)
+#pragma unroll
+            for (int i = 0; i < 4; i++) d[i] += __shfl_xor_sync(0xffffffffu, d[i], y);
+        float mx = -1e30f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) { d[i] = 4 * i + r <= left ? d[i] * 0.125f : -1e30f; mx = fmaxf(mx, d[i]); }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+        const float mn = fmaxf(m, mx), corr = __expf(m - mn);
+        m = mn;
+        l *= corr;
+#pragma unroll
+        for (int e = 0; e < 8; e++) o[e] *= corr;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (4 * i + r <= left) {                      // (rows that were never copied must not meet a zero weight)
+                const float w = __expf(d[i] - mn);
+                const uint4 v = *reinterpret_cast<const uint4 *>(mine + 2048 + i * 512 + lane * 16);
+                l += w;
+                o[0] = __fmaf_rn(w, ds_lo(v.x), o[0]); o[1] = __fmaf_rn(w, ds_hi(v.x), o[1]);
+                o[2] = __fmaf_rn(w, ds_lo(v.y), o[2]); o[3] = __fmaf_rn(w, ds_hi(v.y), o[3]);
+                o[4] = __fmaf_rn(w, ds_lo(v.z), o[4]); o[5] = __fmaf_rn(w, ds_hi(v.z), o[5]);
+                o[6] = __fmaf_rn(w, ds_lo(v.w), o[6]); o[7] = __fmaf_rn(w, ds_hi(v.w), o[7]);
+            }
+        }
+        __syncwarp();                                     // before the keys after the next overwrite these
+    }
+    // l and o hold the lane's keys only: add the four key rows of the warp, then merge the warps
+#pragma unroll
+    for (int y = 8; y < 32; y <<= 1) {
+        l += __shfl_xor_sync(0xffffffffu, l, y);
+#pragma unroll
+        for (int e = 0; e < 8; e++) o[e] += __shfl_xor_sync(0xffffffffu, o[e], y);
+    }
+    __syncthreads();                                      // part held the projections' sums
+    if (r == 0) {
+        *reinterpret_cast<float4 *>(sh.part + warp * 64 + c8) = make_float4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<float4 *>(sh.part + warp * 64 + c8 + 4) = make_float4(o[4], o[5], o[6], o[7]);
+    }
+    if (lane == 0) { sh.am[warp] = m; sh.al[warp] = l; }
+    __syncthreads();
+    if (tid < 64) {
+        float M = sh.am[0], y = 0.0f, sum = 0.0f;
+#pragma unroll
+        for (int w = 1; w < DS_WARPS; w++) M = fmaxf(M, sh.am[w]);
+#pragma unroll 8
+        for (int w = 0; w < DS_WARPS; w++) { const float f = __expf(sh.am[w] - M); sum += f * sh.al[w]; y += f * sh.part[w * 64 + tid]; }
+        a.att[(size_t)b * a.D + h * 64 + tid] = __float2bfloat16_rn(__fdividef(y, sum));
+    }
+}
+
+// ---- rows: thread q < D / 4 owns columns 4q .. 4q + 3.  bf16 values in fp32 -> the normed bf16 row (and, for the router,
+// the same values as fp32 in xrow).  Every thread of the CTA takes part.
+__device__ __forceinline__ void ds_norm_store(const DsArgs &a, Shared &sh, const float4 x, const float *gamma, bf16 *dst, float *xrow)
+{
+    const int n = 4 * threadIdx.x;
+    float4 gm = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (n < a.D) gm = __ldg(reinterpret_cast<const float4 *>(gamma + n));
+    float ss = n < a.D ? x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w : 0.0f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((threadIdx.x & 31) == 0) sh.red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float tot = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; w++) tot += sh.red[w];         // D / 4 <= 256 threads: the warps beyond add nothing
+    const float rinv = 1.0f / sqrtf(tot / (float)a.D + 1e-5f);
+    if (n < a.D) {
+        const float4 o = ds_bf4(make_float4(x.x * rinv * gm.x, x.y * rinv * gm.y, x.z * rinv * gm.z, x.w * rinv * gm.w));
+        ds_strow(dst + n, o);
+        if (xrow) *reinterpret_cast<float4 *>(xrow + n) = o;
+    }
+}
+
+// The rows' owners are the last CTAs, which have no attention item: what they need besides sums (the router's matrix)
+// waits in shared memory since the layer's start.
+__device__ __forceinline__ int ds_row(const DsArgs &a) { const int b = (int)gridDim.x - 1 - (int)blockIdx.x; return b < a.B ? b : -1; }
+__device__ __forceinline__ void ds_wr_request(const DsArgs &a, const DsLayer &ly, float *wr)
+{
+#pragma unroll 1
+    for (int i = threadIdx.x * 4; i < a.D * a.E; i += DS_THREADS * 4) ds_cp16(ds_smem(wr + i), ly.wr + i);
+    ds_commit();
+}
+// residual, norm, router of a row
+__device__ __forceinline__ void ds_router(const DsArgs &a, Shared &sh, const DsLayer &ly, float *wr, float *xrow)
+{
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, b = ds_row(a);
+    gb_wait(a, sh);
+    if (b < 0) return;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int n = 4 * tid, ns = a.D / DS_ROWS;
+    if (n < a.D) {
+        float4 p[DS_MAX_SL], y = x;
+        const float *pp = a.po + (size_t)b * a.D + n;
+        x = ds_ldrow(a.x + (size_t)b * a.D + n);
+#pragma unroll
+        for (int k = 0; k < DS_MAX_SL; k++) { p[k] = k < ns ? ds_ld4(pp) : make_float4(0.f, 0.f, 0.f, 0.f); pp += a.B * a.D; }
+#pragma unroll
+        for (int k = 0; k < DS_MAX_SL; k++) ds_add4(y, p[k]);
+        ds_add4(x, ds_bf4(y));
+        x = ds_bf4(x);
+        ds_strow(a.fi + (size_t)b * a.D + n, x);
+    }
+    ds_norm_store(a, sh, x, ly.an2, a.fnorm + (size_t)b * a.D, xrow);
+    ds_wait<0>();
+    __syncthreads();
+    const int per = a.D / DS_WARPS, j0 = warp * per;      // a multiple of eight
+    float acc = 0.0f;
+    if (lane < a.E) {
+        const float *wp = wr + j0 * a.E + lane;
+#pragma unroll 2
+        for (int j = j0; j < j0 + per; j += 8) {
+            const float4 x0 = *reinterpret_cast<const float4 *>(xrow + j), x1 = *reinterpret_cast<const float4 *>(xrow + j + 4);
+            float w[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) { w[u] = *wp; wp += a.E; }
+            acc = __fmaf_rn(x0.x, w[0], acc); acc = __fmaf_rn(x0.y, w[1], acc); acc = __fmaf_rn(x0.z, w[2], acc); acc = __fmaf_rn(x0.w, w[3], acc);
+            acc = __fmaf_rn(x1.x, w[4], acc); acc = __fmaf_rn(x1.y, w[5], acc); acc = __fmaf_rn(x1.z, w[6], acc); acc = __fmaf_rn(x1.w, w[7], acc);
+        }
+    }
+    sh.logit[warp * 32 + lane] = acc;
+    __syncthreads();
+    if (warp == 0) {
+        float lg = 0.0f;
+        if (lane < a.E) {
+#pragma unroll
+            for (int w = 0; w < DS_WARPS; w++) lg += sh.logit[w * 32 + lane];
+            ly.rt[(size_t)b * a.E + lane] = lg;
+        }
+        router_topk_row(lg, b, lane, ly.rprobs, ly.assign, ly.gate, a.B, a.E, a.K, nullptr, 0);
+    }
+}
+
+// the step's distinct experts and the slots k * B + b of each (in order of first use)
+__device__ __forceinline__ void ds_experts(const DsArgs &a, Shared &sh, const DsLayer &ly)
+{
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x, R = a.K * a.B;
+        int e = -1;
+        if (lane < R) { e = __ldcg(ly.assign + lane); if ((unsigned)e >= (unsigned)a.E) e = 0; }
+        const unsigned m = __match_any_sync(0xffffffffu, e), lt = (1u << lane) - 1u;
+        const unsigned lead = __ballot_sync(0xffffffffu, e >= 0 && (m & lt) == 0u);
+        if ((lead >> lane) & 1u) { const int i = __popc(lead & lt); sh.pexp[i] = e; sh.pmask[i] = m; }
+        if (lane == 0) sh.npair = __popc(lead);
+    }
+    __syncthreads();
+}
+
+// gate-weighted combination, residual, the next norm of a row
+__device__ __forceinline__ void ds_combine(const DsArgs &a, Shared &sh, const DsLayer &ly, float *ys, int l)
+{
+    const int b = ds_row(a);
+    if (b < 0) return;
+    const int c = 4 * threadIdx.x;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < a.D) x = ds_ldrow(a.fi + (size_t)b * a.D + c);
+    if ((int)threadIdx.x < a.K) sh.red[threadIdx.x] = __ldcg(ly.gate + (size_t)threadIdx.x * a.B + b);    // K <= 16
+    const int half = threadIdx.x >> 8, n = 4 * (threadIdx.x & 255), R = a.K * a.B, ns = a.F / DS_ROWS;
+    if (n < a.D) {
+#pragma unroll 1
+        for (int k = half; k < a.K; k += 2) {
+            const float *p = a.pd + (size_t)(k * a.B + b) * a.D + n;
+            float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+            for (int s0 = 0; s0 < ns; s0 += 12) {         // twelve slices in flight: d_ff 1536 in one go
+                float4 v[12];
+#pragma unroll
+                for (int s = 0; s < 12; s++) { v[s] = s0 + s < ns ? ds_ld4(p) : make_float4(0.f, 0.f, 0.f, 0.f); p += (size_t)R * a.D; }
+#pragma unroll
+                for (int s = 0; s < 12; s++) ds_add4(y, v[s]);
+            }
+            *reinterpret_cast<float4 *>(ys + k * a.D + n) = ds_bf4(y);
+        }
+    }
+    __syncthreads();
+    if (c < a.D) {
+#pragma unroll 1
+        for (int k = 0; k < a.K; k++) ds_fma4(x, sh.red[k], *reinterpret_cast<const float4 *>(ys + k * a.D + c));
+        x = ds_bf4(x);
+        ds_strow(a.x + (size_t)b * a.D + c, x);
+    }
+    __syncthreads();                                      // red held the gates
+    if (l + 1 < a.L) ds_norm_store(a, sh, x, sh.layer[(l + 1) & 1].an1, a.xn + (size_t)b * a.D, nullptr);
+    else ds_norm_store(a, sh, x, a.nf, a.fn + (size_t)b * a.D, nullptr);
+}
+
+// C rows per task of the dense phases; MULTI: an expert can have more than one slot
+template <int C, bool MULTI>
+__global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constant__ DsArgs a)
+{
+    extern __shared__ __align__(128) uint8_t dsm[];
+    __shared__ Shared sh;
+    float *red = reinterpret_cast<float *>(dsm), *wr = reinterpret_cast<float *>(dsm + DS_RED), *xs = reinterpret_cast<float *>(dsm + DS_RED + DS_WR);
+    auto load_layer = [&](int l) {
+        if (threadIdx.x < DS_LAYER_WORDS)
+            reinterpret_cast<unsigned long long *>(&sh.layer[l & 1])[threadIdx.x] = __ldg(reinterpret_cast<const unsigned long long *>(a.layers + l) + threadIdx.x);
+    };
+    load_layer(0);
+    if (threadIdx.x < DS_MAX_B) sh.pos[threadIdx.x] = (int)threadIdx.x < a.B ? __ldg(a.pos + threadIdx.x) : 0;
+    if (threadIdx.x == 0) sh.target = 0u;
+    __syncthreads();
+    if (ds_row(a) >= 0) {                                 // embedding row and the first norm
+        const int b = ds_row(a), n = 4 * threadIdx.x;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (n < a.D) {
+            x = ds_bf4(__ldg(reinterpret_cast<const float4 *>(a.emb + (size_t)__ldg(a.tok + b) * a.D + n)));
+            ds_strow(a.x + (size_t)b * a.D + n, x);
+        }
+        ds_norm_store(a, sh, x, sh.layer[0].an1, a.xn + (size_t)b * a.D, nullptr);
+    }
+#pragma unroll 1
+    for (int l = 0; l < a.L; l++) {
+        const DsLayer &ly = sh.layer[l & 1];
+        gb_arrive(a, sh);
+        if (l + 1 < a.L) load_layer(l + 1);               // every thread has passed the sync in gb_arrive: the other half is free
+        if ((int)blockIdx.x < a.B * a.H) ds_kv_request(a, sh, ly, dsm + DS_RED, blockIdx.x, 0);
+        else if (ds_row(a) >= 0) ds_wr_request(a, ly, wr);
+        ds_dense<0, C>(a, sh, ly, red);
+        gb_arrive(a, sh);
+        ds_attention(a, sh, ly, dsm + DS_RED);
+        gb_arrive(a, sh);
+        ds_dense<1, C>(a, sh, ly, red);
+        gb_arrive(a, sh);
+        ds_router(a, sh, ly, wr, red);
+        gb_arrive(a, sh);
+        gb_wait(a, sh);
+        ds_experts(a, sh, ly);
+        ds_experts_phase<false>(a, sh, ly, red, xs, dsm + DS_RED, MULTI);
+        gb_arrive(a, sh);
+        ds_experts_phase<true>(a, sh, ly, red, xs, dsm + DS_RED, MULTI);
+        gb_arrive(a, sh);
+        gb_wait(a, sh);
+        ds_combine(a, sh, ly, red, l);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(a.bar + 1, 1u) == gridDim.x - 1) { a.bar[0] = 0u; a.bar[1] = 0u; a.bar[2] = 0u; __threadfence(); }
+    }
+}
+
+struct DsLayout { size_t x, xn, att, fi, fnorm, pq, po, pg, pd, bytes; };
+static DsLayout ds_layout(int B, int D, int KD, int F, int K)
+{
+    DsLayout w;
+    size_t cur = 256;
+    auto take = [&](size_t n) { const size_t at = cur; cur += (n + 255) & ~(size_t)255; return at; };
+    const size_t b = B, d = D, r = (size_t)K * B, sd = D / DS_ROWS, sf = F / DS_ROWS;
+    w.x = take(b * d * 2); w.xn = take(b * d * 2); w.att = take(b * d * 2); w.fi = take(b * d * 2); w.fnorm = take(b * d * 2);
+    w.pq = take(sd * b * (d + 2 * (size_t)KD) * 4);
+    w.po = take(sd * b * d * 4);
+    w.pg = take(sd * 2 * r * F * 4);
+    w.pd = take(sf * r * d * 4);
+    w.bytes = cur;
+    return w;
+}
+static bool ds_fits(int B, int Tm, int D, int H, int KV, int F, int E, int K)
+{
+    return B >= 1 && B <= DS_MAX_B && Tm >= 1 && Tm <= 4096 && D == H * 64 && D % 128 == 0 && D <= 1024 && KV >= 1 && H % KV == 0 &&
+           (KV * 64) % 128 == 0 && F >= 128 && F % 128 == 0 && E >= 1 && E <= 32 && K >= 1 && K <= E && K * B <= DS_MAX_R && K <= DS_WARPS && K * D * 4 <= DS_RED &&
+           B * (H + 1) <= sm_count();                     // a CTA has an attention item or owns a row
+}
+
+}  // namespace qlmb
+
+using namespace qlmb;
+
+extern "C" size_t qlmb_dec_step_bytes(int B, int Tm, int D, int H, int KV, int F, int E, int K)
+{
+    return ds_fits(B, Tm, D, H, KV, F, E, K) ? ds_layout(B, D, KV * 64, F, K).bytes : 0;
+}
+
+extern "C" int qlmb_dec_step(const qlmb_dec_step_args *p, void *stream)
+{
+    QLMB_REQUIRE(p && p->layers && p->emb && p->tok && p->pos && p->cosb && p->sinb && p->nf && p->fn && p->ws, "qlmb_dec_step: NULL argument");
+    QLMB_REQUIRE(p->L > 0, "qlmb_dec_step: L=%d", p->L);
+    if (!ds_fits(p->B, p->Tm, p->D, p->H, p->KV, p->F, p->E, p->K)) {
+        set_error("qlmb_dec_step: shape B %d Tm %d D %d H %d KV %d F %d E %d K %d is not supported", p->B, p->Tm, p->D, p->H, p->KV, p->F, p->E, p->K);
+        return QLMB_E_UNSUPPORTED;
+    }
+    QLMB_REQUIRE(((uintptr_t)p->ws & 255) == 0, "qlmb_dec_step: the workspace must be 256-byte aligned");
+    const DsLayout w = ds_layout(p->B, p->D, p->KV * 64, p->F, p->K);
+    uint8_t *ws = (uint8_t *)p->ws;
+    DsArgs a = {};
+    a.layers = (const DsLayer *)p->layers;
+    a.L = p->L; a.B = p->B; a.D = p->D; a.KD = p->KV * 64; a.H = p->H; a.KV = p->KV; a.F = p->F; a.E = p->E; a.K = p->K; a.Tm = p->Tm;
+    auto recip = [](int n) { return (uint32_t)((0x100000000ull + n - 1) / n); };       // exact quotients for the task numbers that occur
+    a.tq = (a.D + 2 * a.KD + DS_COLS - 1) / DS_COLS; a.td = (a.D + DS_COLS - 1) / DS_COLS; a.tf = (a.F + DS_COLS - 1) / DS_COLS;
+    a.mq = recip(a.tq); a.md = recip(a.td); a.mf = recip(a.tf); a.mr = recip(a.D / DS_ROWS); a.mfs = recip(a.F / DS_ROWS);
+    a.emb = p->emb; a.tok = p->tok; a.pos = p->pos; a.cosb = p->cosb; a.sinb = p->sinb; a.nf = p->nf; a.fn = (bf16 *)p->fn;
+    a.bar = (unsigned *)ws;
+    a.x = (bf16 *)(ws + w.x); a.xn = (bf16 *)(ws + w.xn); a.att = (bf16 *)(ws + w.att); a.fi = (bf16 *)(ws + w.fi); a.fnorm = (bf16 *)(ws + w.fnorm);
+    a.pq = (float *)(ws + w.pq); a.po = (float *)(ws + w.po); a.pg = (float *)(ws + w.pg); a.pd = (float *)(ws + w.pd);
+    a.errword = device_error_word();
+    // rows per task of the dense phases: the fewest with which the q, k, v tasks are one round of the device
+    int c = 1;
+    while (c < 4 && a.tq * (a.D / DS_ROWS) * ((p->B + c - 1) / c) > sm_count()) c *= 2;
+    const int v = p->B == 1 ? 0 : c == 1 ? 1 : c == 2 ? 2 : 3;
+    const void *kern = v == 0 ? (const void *)k_dec_step<1, false> : v == 1 ? (const void *)k_dec_step<1, true>
+                     : v == 2 ? (const void *)k_dec_step<2, true> : (const void *)k_dec_step<4, true>;
+    int dev = 0;
+    QLMB_CUDA(cudaGetDevice(&dev));
+    QLMB_REQUIRE(dev >= 0 && dev < 64, "device index %d", dev);
+    static bool attr_done[64][4];
+    if (!attr_done[dev][v]) {
+        QLMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DS_SMEM));
+        attr_done[dev][v] = true;
+    }
+    void *args[] = {&a};
+    QLMB_CUDA(cudaLaunchCooperativeKernel(kern, dim3((unsigned)sm_count()), dim3(DS_THREADS), args, (size_t)DS_SMEM, as_stream(stream)));
+    QLMB_LAUNCH_CHECK("k_dec_step");
+    return QLMB_OK;
+}

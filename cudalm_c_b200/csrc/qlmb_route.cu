@@ -5,65 +5,10 @@
 // and expert choices match that build bit for bit on the same logits.
 #include "qlmb_common.cuh"
 #include "qlmb_internal.h"
+#include "qlmb_topk.cuh"
 
 namespace qlmb {
 
-// exp as the reference CPU build computes it (cpu_kern.h:28-34): clamp,
-// two-part ln2 reduction, degree-6 polynomial, exponent by bit shift.
-__device__ __forceinline__ float exp_poly(float x)
-{
-    x = x < -87.0f ? -87.0f : (x > 88.0f ? 88.0f : x);
-    float k = rintf(x * 1.44269504089f);
-    float r = x - k * 0.693145751953125f;
-    r -= k * 1.428606765330187e-06f;
-    float p = 1.0f / 720;
-    p = 1.0f / 120 + r * p;
-    p = 1.0f / 24 + r * p;
-    p = 1.0f / 6 + r * p;
-    p = 0.5f + r * p;
-    p = 1.0f + r * p;
-    p = 1.0f + r * p;
-    return p * __uint_as_float((uint32_t)((int)k + 127) << 23);
-}
-
-// Same arithmetic with one warp per token and lane = expert (E <= 32): the
-// maximum is order-free, the softmax sum is still taken in expert order (every
-// lane adds the 32 shuffled terms sequentially) and the K selection rounds are
-// warp arg-max reductions with the lowest index winning ties, so the outputs are
-// bit-identical to the thread-per-token form above.
-// the softmax and the K selection rounds of token n by one warp; lg = the logit of expert `lane` (0 beyond E)
-__device__ __forceinline__ void router_topk_row(float lg, int n, int lane, float *rprobs, int *assign, float *gate, int N,
-                                                int E, int K, const float *bias, int bs)
-{
-    const bool live = lane < E;
-    float top = (live && lg > -1e30f) ? lg : -1e30f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-    float p = live ? exp_poly(lg - top) : 0.0f;
-    float sum = 0.0f;
-    for (int e = 0; e < E; e++) sum += __shfl_sync(0xffffffffu, p, e);
-    float inv = 1.0f / sum;
-    float pr = p * inv;
-    if (live) rprobs[(size_t)n * E + lane] = pr;
-    bool taken = false;
-    for (int k = 0; k < K; k++) {
-        float sc = pr + (bias && live ? bias[k * bs + lane] : 0.0f);
-        bool ok = live && !taken && (sc > -1e30f);
-        int idx = lane;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            float osc = __shfl_xor_sync(0xffffffffu, sc, o);
-            int oidx = __shfl_xor_sync(0xffffffffu, idx, o);
-            bool ook = __shfl_xor_sync(0xffffffffu, (int)ok, o) != 0;
-            bool take = ook && (!ok || osc > sc || (osc == sc && oidx < idx));
-            if (take) { sc = osc; idx = oidx; ok = true; }
-        }
-        int pick = ok ? idx : k;                    // NaN scores: stay in range
-        float g = __shfl_sync(0xffffffffu, pr, pick);
-        if (lane == 0) { assign[(size_t)k * N + n] = pick; gate[(size_t)k * N + n] = g; }
-        taken = taken || (lane == pick);
-    }
-}
 // More than 32 experts (up to 256): still one warp per token, lane l holds experts l, l + 32, ... (EPT per lane).
 // The softmax sum runs over the experts in ascending order (the term of expert e is fetched from lane e % 32), as the
 // reference's CPU kernel adds them (cpu_kern.h:413-425); each selection round takes every lane's best unused expert

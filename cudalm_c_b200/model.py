@@ -380,6 +380,8 @@ class Decoder:
         self.moes = [self._moe(l, B) for l in range(c.L)]
         self.emb_bf, _ = block.cast_bf16(model.emb, plain=True, transposed=False)
         self.logits = None
+        self._plan = False
+        self._step_plan()                                # ahead of the first step: a step may be captured in a graph
 
     def _moe(self, l, N):
         c, m = self.m.c, self.m
@@ -439,11 +441,34 @@ class Decoder:
         if getattr(self, "sp", None) is not None:
             self.sp[t] = self.sp[s]
 
-    def step(self, advance=True):
-        """dec_step: the token in self.tok at position self.pos for every slot; logits -> self.logits, greedy pick ->
-        self.otok / self.olp; with advance the pick becomes the next step's token.  Positions live on the device
-        only: a slot that has reached the end of its cache (pos == Tm) is not written or read by the kernels, which
-        record error 201 in the device error word instead (qlmb_check_device); the caller bounds the step count."""
+    def _step_plan(self):
+        """Arguments of the one-launch form of a step's layers (qlmb_dec_step); None where the shape needs the chain of
+        separate operators.  Everything it points to lives as long as the decoder."""
+        if self._plan is not False:
+            return self._plan
+        from ._lib import DecStepArgs, lib, ptr
+        c, m = self.m.c, self.m
+        shape = (self.B, self.Tm, c.D, c.H, c.KV, c.F, c.E, c.K)
+        nbytes = lib().qlmb_dec_step_bytes(*shape) if c.hd == 64 else 0
+        if not nbytes:
+            self._plan = None
+            return None
+        rows = []
+        for l, ly in enumerate(m.layers):
+            w, f, mo = ly["w"], m.fl[l], self.moes[l]
+            member = lambda nm: lib().qlmb_moe_arena_member(mo.arena_ptr, mo.N, mo.D, mo.F, mo.E, mo.K, nm)
+            rows.append([ptr(w[nm][i]) for i in (0, 1) for nm in QUANT[:4] + ("w1", "w3", "w2")] +
+                        [ptr(f["an1"]), ptr(f["an2"]), ptr(f["wr"]), ptr(self.K[l]), ptr(self.V[l])] +
+                        [member(nm) for nm in (b"rt", b"rprobs", b"assign", b"gate")])
+        self._table = torch.tensor(rows, dtype=torch.int64).to(m.dev)
+        self._ws = torch.zeros(nbytes, dtype=torch.uint8, device=m.dev)
+        self.fn = torch.empty(self.B, c.D, dtype=torch.bfloat16, device=m.dev)
+        self._plan = DecStepArgs(self.B, self.Tm, c.L, *shape[2:], ptr(self._table), ptr(m.emb), ptr(self.tok), ptr(self.pos),
+                                 ptr(self.cosb), ptr(self.sinb), ptr(m.nf), ptr(self.fn), ptr(self._ws))
+        return self._plan
+
+    def _layers_chain(self):
+        """The layers of a step as separate operators: shapes the one-launch form does not take."""
         from ._lib import check, lib, ptr, stream_ptr
         c, m, B = self.m.c, self.m, self.B
         L_ = lib()
@@ -480,6 +505,20 @@ class Decoder:
                 f_norm, _ = block.rmsnorm_fwd(f_in, f["an2"])
             x = self.moes[l].decode(f_in, f_norm)
         fn, _ = block.rmsnorm_fwd(x, m.nf)
+        return fn
+
+    def step(self, advance=True):
+        """dec_step: the token in self.tok at position self.pos for every slot; logits -> self.logits, greedy pick ->
+        self.otok / self.olp; with advance the pick becomes the next step's token.  Positions live on the device
+        only: a slot that has reached the end of its cache (pos == Tm) is not written or read by the kernels, which
+        record error 201 in the device error word instead (qlmb_check_device); the caller bounds the step count."""
+        from ._lib import check, lib, stream_ptr
+        plan = self._step_plan()
+        if plan is not None:
+            check(lib().qlmb_dec_step(plan, stream_ptr()))
+            fn = self.fn
+        else:
+            fn = self._layers_chain()
         self.logits = block.gemm_nt(fn, self.emb_bf, torch.float32, out=self.logits)
         self._pick()
         if advance:

@@ -246,6 +246,28 @@ int qlmb_linear_wgrad(float *dW, const void *dY, const void *X, int layout, int 
 int qlmb_gemv_decode(void *Y, const void *X, const int8_t *codes, const float *scales, int layout,
                      int B, int K, int N, int dtype, void *stream);
 
+/* The layers of one decode step (dec_step, cudalm.cu:7168-7212) in one persistent cooperative launch: embedding of
+ * `tok`, per layer norm + q, k, v + rotation + cache append + attention over the cached keys + output projection +
+ * residual + norm + router + routed experts, and the final norm into fn [B][D] (bf16), the head's input.  `layers` is a
+ * DEVICE table of L rows of 23 pointers: codes of wq, wk, wv, wo, w1, w3, w2; their scales in the same order; an1, an2,
+ * wr; the K and V caches [B][Tm][KV*64] (bf16); and the members rt, rprobs, assign, gate of the layer's MoE arena,
+ * which are filled as qlmb_moe_decode fills them.  ws = qlmb_dec_step_bytes(...) bytes, 256-byte aligned, zeroed once
+ * before its first use, not shared by steps that may overlap; a size of 0 means that the shape is not supported
+ * (supported: head dimension 64, D <= 1024, at most 8 slots, 32 experts and 32 routed slots, a CTA per attention item
+ * and row on the device) and the separate entry points do the step.  A slot whose position is outside its cache is reported and neither read nor written. */
+typedef struct qlmb_dec_step_args {
+    int B, Tm, L, D, H, KV, F, E, K;
+    const void *layers;
+    const float *emb;            /* [V][D] fp32 */
+    const int *tok, *pos;        /* [B] */
+    const float *cosb, *sinb;    /* [>= Tm][32] */
+    const float *nf;             /* [D] */
+    void *fn;
+    void *ws;
+} qlmb_dec_step_args;
+size_t qlmb_dec_step_bytes(int B, int Tm, int D, int H, int KV, int F, int E, int K);
+int qlmb_dec_step(const qlmb_dec_step_args *p, void *stream);
+
 /* ------------------------------------------------------- router + permutation */
 
 /* g_ab(f_norm, Wr) + k_router_topk (cudalm.cu:4158, 2515-2534).  If rt_in is

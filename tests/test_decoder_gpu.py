@@ -143,3 +143,47 @@ def test_sampler_topk_topp_temperature(cuda):
                 ok |= lo - 1e-4 <= u01 <= cum[i] + 1e-4
         assert ok, (b, cases[b], int(out[b]))
     q.check(q.lib().qlmb_check_device(None))
+
+
+@pytest.mark.parametrize("B,D,KV,E,K,F,fill,Tm", [
+    (1, 256, 4, 8, 2, 256, 1, 64),          # one key before the new one
+    (1, 768, 12, 32, 2, 1536, 255, 640),    # the last key of a 256-key pass is the new one
+    (2, 640, 2, 8, 1, 384, 256, 640),       # grouped heads, a column tile that is half empty, a second pass
+    (3, 128, 2, 4, 4, 128, 40, 64),         # every expert, one row slice
+    (8, 1024, 16, 32, 3, 640, 20, 32),      # 24 routed slots, experts with several slots, the widest model
+])
+def test_one_launch_step_equals_the_chain(cuda, B, D, KV, E, K, F, fill, Tm):
+    """qlmb_dec_step (up to eight slots) against the chain of separate operators: the same experts and the same cache rows
+    up to a bf16 rounding, the final norm's output within the rounding noise of bf16 activations; bit-reproducible."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import model
+    from cudalm_c_b200._lib import stream_ptr
+    cfg = model.Config(L=2, D=D, H=D // 64, KV=KV, hd=64, E=E, K=K, F=F, V=512, T=max(fill, 64), B=1)
+    m = model.QlmModel(cfg, cuda, seed=3)
+    d = model.Decoder(m, B, Tm)
+    g = torch.Generator(device=cuda); g.manual_seed(B)
+    d.prefill(torch.randint(0, cfg.V, (B, fill), generator=g, dtype=torch.int32, device=cuda))
+    pos = torch.randint((fill + 1) // 2, fill + 1, (B,), generator=g, dtype=torch.int32, device=cuda)
+    pos[0] = fill
+    d.pos2.copy_(pos.repeat(2))
+    plan = d._step_plan()
+    assert plan is not None
+    before = [t.clone() for t in d.K + d.V]
+    want = d._layers_chain().float()
+    experts = [mo.member("assign", (K, B), torch.int32).clone() for mo in d.moes]
+    caches = [t.clone() for t in d.K + d.V]
+    for t, b in zip(d.K + d.V, before):
+        t.copy_(b)
+    outs = []
+    for _ in range(2):
+        q.check(q.lib().qlmb_dec_step(plan, stream_ptr()))
+        outs.append(d.fn.float().clone())
+    torch.cuda.synchronize()
+    q.check(q.lib().qlmb_check_device(None))
+    assert torch.equal(*outs)
+    # a near-tie of two router logits may fall the other way for a choice or two
+    assert sum(int((e != mo.member("assign", (K, B), torch.int32)).sum()) for e, mo in zip(experts, d.moes)) <= 2
+    assert float(((outs[0] - want).norm(dim=1) / want.norm(dim=1)).median()) < 1e-2
+    for t, c, b in zip(d.K + d.V, caches, before):
+        assert float((t.float() - c.float()).abs().max()) < 2e-2
+        assert ((t != b).flatten(2).any(-1).sum(1) <= 1).all()              # at most the slot's own row changed
