@@ -202,7 +202,34 @@ def ptr(t):
     return t.data_ptr()
 
 
+class _Calls:
+    """The hot entry points without their qlmb_ prefix as native calls (csrc/pycalls.c): tensors, addresses or None for
+    pointers, a QlmbError for a status other than 0."""
+
+    def __getattr__(self, name):
+        lib()                                            # a missing library is reported the same way everywhere
+        try:
+            from . import _pycalls
+        except ImportError as e:
+            raise QlmbError("_pycalls.so does not load (%s): build it with `python -m cudalm_c_b200.build`" % e)
+        _pycalls.set_error_class(QlmbError)
+        f = getattr(_pycalls, name)
+        setattr(self, name, f)                           # later uses find it in the instance
+        return f
+
+
+calls = _Calls()
+_raw_stream = _current_device = None
+
+
 def stream_ptr(stream=None):
-    import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    """cudaStream_t of `stream`, or of the current stream of the current device."""
+    global _raw_stream, _current_device
+    if stream is not None:
+        return stream.cuda_stream
+    if _raw_stream is None:
+        import torch
+        torch.cuda.init()
+        _current_device = torch._C._cuda_getDevice
+        _raw_stream = torch._C._cuda_getCurrentRawStream # torch.cuda.current_stream() makes a Stream object: 3.4 us a call
+    return _raw_stream(_current_device())

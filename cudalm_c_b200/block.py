@@ -2,7 +2,7 @@
 k_embed, k_embed_bwd, k_softmax_ce; cudalm.cu:3630-3645, 5740, 5838, 6000) over the C ABI."""
 import torch
 
-from ._lib import BF16, F32, check, lib, ptr, stream_ptr
+from ._lib import BF16, F32, calls, check, lib, ptr, stream_ptr
 
 
 def _dt(t):
@@ -16,7 +16,7 @@ def _dt(t):
 def embed(emb, tok, dtype=torch.float32):
     N, D = tok.numel(), emb.shape[1]
     X = torch.empty(N, D, dtype=dtype, device=emb.device)
-    check(lib().qlmb_embed(ptr(X), _dt(X), ptr(emb), ptr(tok), N, D, stream_ptr()))
+    calls.embed(X, _dt(X), emb, tok, N, D, stream_ptr())
     return X
 
 
@@ -29,7 +29,7 @@ def rmsnorm_fwd(X, gamma, out_dtype=None, out=None):
     N, D = X.shape
     O = out if out is not None else torch.empty(N, D, dtype=out_dtype or X.dtype, device=X.device)
     rinv = torch.empty(N, dtype=torch.float32, device=X.device)
-    check(lib().qlmb_rmsnorm_fwd(ptr(O), _dt(O), ptr(rinv), ptr(X), _dt(X), ptr(gamma), N, D, stream_ptr()))
+    calls.rmsnorm_fwd(O, _dt(O), rinv, X, _dt(X), gamma, N, D, stream_ptr())
     return O, rinv
 
 
@@ -37,8 +37,7 @@ def rmsnorm_bwd(dx, X, gamma, rinv, dy, dgamma=None, accumulate=True):
     """dx (+)= the input gradient; dgamma += the gain gradient (e_rmsb accumulates into both)."""
     N, D = X.shape
     part = torch.empty(128 * D, dtype=torch.float32, device=X.device) if dgamma is not None else None
-    check(lib().qlmb_rmsnorm_bwd(ptr(dx), _dt(dx), 1 if accumulate else 0, ptr(dgamma), ptr(part), ptr(X), _dt(X), ptr(gamma),
-                                 ptr(rinv), ptr(dy), _dt(dy), N, D, stream_ptr()))
+    calls.rmsnorm_bwd(dx, _dt(dx), 1 if accumulate else 0, dgamma, part, X, _dt(X), gamma, rinv, dy, _dt(dy), N, D, stream_ptr())
 
 
 def rope_tables(T, hd, base=10000.0, device="cpu"):
@@ -51,7 +50,7 @@ def rope_tables(T, hd, base=10000.0, device="cpu"):
 
 def rope(buf, cosb, sinb, nh, hd, T, back=False):
     """In place on buf[N, nh*hd]."""
-    check(lib().qlmb_rope(ptr(buf), _dt(buf), ptr(cosb), ptr(sinb), buf.shape[0], nh, hd, T, 1 if back else 0, stream_ptr()))
+    calls.rope(buf, _dt(buf), cosb, sinb, buf.shape[0], nh, hd, T, 1 if back else 0, stream_ptr())
 
 
 def softmax_ce(logits, tgt, n_all, dl_dtype=None):
@@ -67,7 +66,7 @@ def gemm_nt(A, B, out_dtype=torch.float32, out=None, beta=0.0):
     M, K = A.shape
     N = B.shape[0]
     C_ = out if out is not None else torch.empty(M, N, dtype=out_dtype, device=A.device)
-    check(lib().qlmb_gemm_nt(ptr(C_), _dt(C_), ptr(A), ptr(B), M, K, N, beta, stream_ptr()))
+    calls.gemm_nt(C_, _dt(C_), A, B, M, K, N, beta, stream_ptr())
     return C_
 
 

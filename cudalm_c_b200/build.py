@@ -7,16 +7,19 @@ Every translation unit is compiled with
 bit-exact integer-state and router arithmetic add `--fmad=false` (a fused
 multiply-add changes the rounding the reference's CPU build produces).  The CUDA
 runtime is linked statically and the driver API is reached through
-cudaGetDriverEntryPoint, so the library loads on a machine without a GPU.
+cudaGetDriverEntryPoint, so the library loads on a machine without a GPU.  A small
+extension module with the hot entry points as plain C calls is built beside it.
 """
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libqlm_b200.so")
 OBJ = os.path.join(HERE, "build")
+PYCALLS = os.path.join(HERE, "_pycalls.so")          # plain C calls of the hot entry points for Python (csrc/pycalls.c)
 
 # translation unit -> extra flags
 UNITS = {
@@ -72,6 +75,10 @@ def build(force=False, verbose=False):
     if force or procs or not os.path.exists(OUT):
         cmd = [nvcc, "-shared", "-cudart", "static", "-o", OUT] + objs + ["-Xlinker", "--no-undefined", "-lpthread", "-ldl", "-lrt"]
         subprocess.check_call(cmd)
+    src = os.path.join(CSRC, "pycalls.c")
+    if force or _newer(src, PYCALLS, headers):
+        subprocess.check_call([os.environ.get("CC", "gcc"), "-shared", "-fPIC", "-O2", "-Wall", "-I", sysconfig.get_paths()["include"], "-o", PYCALLS, src,
+                               "-L", HERE, "-l:libqlm_b200.so", "-Wl,-rpath,$ORIGIN"])
     return OUT
 
 

@@ -6,7 +6,7 @@ KN = codes of W[K,N] (the reference's own [in,out] storage, applied with g_ab),
 NK = codes of W[N,K] (applied with g_abt)."""
 import torch
 
-from ._lib import BF16, F32, KN, NK, check, lib, ptr, stream_ptr  # noqa: F401
+from ._lib import BF16, F32, KN, NK, calls, stream_ptr  # noqa: F401
 
 
 def _dt(t):
@@ -20,16 +20,16 @@ def _dt(t):
 def linear_fwd(X, codes, scales, layout, N, R=None, out=None):
     """Y[M,N] = X[M,K] @ deq(W) (+ R)   -- g_ab / g_abt / g_ab_res."""
     M, K = X.shape
-    Y = out if out is not None else torch.empty((M, N), dtype=X.dtype, device=X.device)
-    check(lib().qlmb_linear_fwd(ptr(Y), ptr(X), ptr(codes), ptr(scales), layout, M, K, N, ptr(R), _dt(X), stream_ptr()))
+    Y = out if out is not None else X.new_empty((M, N))
+    calls.linear_fwd(Y, X, codes, scales, layout, M, K, N, R, _dt(X), stream_ptr())
     return Y
 
 
 def linear_dgrad(dY, codes, scales, layout, K, beta=0.0, out=None):
     """dX[M,K] = beta*dX + dY[M,N] @ deq(W)^T   -- g_abt_b / g_ab."""
     M, N = dY.shape
-    dX = out if out is not None else torch.empty((M, K), dtype=dY.dtype, device=dY.device)
-    check(lib().qlmb_linear_dgrad(ptr(dX), ptr(dY), ptr(codes), ptr(scales), layout, M, K, N, beta, _dt(dY), stream_ptr()))
+    dX = out if out is not None else dY.new_empty((M, K))
+    calls.linear_dgrad(dX, dY, codes, scales, layout, M, K, N, beta, _dt(dY), stream_ptr())
     return dX
 
 
@@ -37,13 +37,13 @@ def linear_wgrad(dW, dY, X, layout, beta=1.0):
     """dW (fp32, shape of W) = beta*dW + X^T dY (KN) or dY^T X (NK)   -- g_atb."""
     M, K = X.shape
     N = dY.shape[1]
-    check(lib().qlmb_linear_wgrad(ptr(dW), ptr(dY), ptr(X), layout, M, K, N, beta, _dt(X), stream_ptr()))
+    calls.linear_wgrad(dW, dY, X, layout, M, K, N, beta, _dt(X), stream_ptr())
     return dW
 
 
 def gemv_decode(X, codes, scales, layout, N, out=None):
     """Y[B,N] = X[B,K] @ deq(W) for B <= 64 live decode slots."""
     B, K = X.shape
-    Y = out if out is not None else torch.empty((B, N), dtype=X.dtype, device=X.device)
-    check(lib().qlmb_gemv_decode(ptr(Y), ptr(X), ptr(codes), ptr(scales), layout, B, K, N, _dt(X), stream_ptr()))
+    Y = out if out is not None else X.new_empty((B, N))
+    calls.gemv_decode(Y, X, codes, scales, layout, B, K, N, _dt(X), stream_ptr())
     return Y

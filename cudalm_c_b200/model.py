@@ -423,13 +423,13 @@ class Decoder:
         self.pos2 += 1
 
     def _pick(self):
-        from ._lib import check, lib, ptr, stream_ptr
+        from ._lib import calls, check, lib, ptr, stream_ptr
         if getattr(self, "sp", None) is not None:
             check(lib().qlmb_dec_sample(ptr(self.otok), ptr(self.olp), ptr(self.logits), ptr(self.sp), self.B, self.m.c.V,
                                         stream_ptr()))
             self.sp_step += 1
         else:
-            check(lib().qlmb_dec_greedy(ptr(self.otok), ptr(self.olp), ptr(self.logits), self.B, self.m.c.V, stream_ptr()))
+            calls.dec_greedy(self.otok, self.olp, self.logits, self.B, self.m.c.V, stream_ptr())
 
     def move(self, s, t):
         """dec_move (cudalm.cu:7222-7231): slot s's state into slot t (continuous batching keeps live slots first)."""
@@ -446,6 +446,7 @@ class Decoder:
         separate operators.  Everything it points to lives as long as the decoder."""
         if self._plan is not False:
             return self._plan
+        import ctypes as C
         from ._lib import DecStepArgs, lib, ptr
         c, m = self.m.c, self.m
         shape = (self.B, self.Tm, c.D, c.H, c.KV, c.F, c.E, c.K)
@@ -465,6 +466,7 @@ class Decoder:
         self.fn = torch.empty(self.B, c.D, dtype=torch.bfloat16, device=m.dev)
         self._plan = DecStepArgs(self.B, self.Tm, c.L, *shape[2:], ptr(self._table), ptr(m.emb), ptr(self.tok), ptr(self.pos),
                                  ptr(self.cosb), ptr(self.sinb), ptr(m.nf), ptr(self.fn), ptr(self._ws))
+        self._plan_addr = C.addressof(self._plan)
         return self._plan
 
     def _layers_chain(self):
@@ -512,10 +514,10 @@ class Decoder:
         self.otok / self.olp; with advance the pick becomes the next step's token.  Positions live on the device
         only: a slot that has reached the end of its cache (pos == Tm) is not written or read by the kernels, which
         record error 201 in the device error word instead (qlmb_check_device); the caller bounds the step count."""
-        from ._lib import check, lib, stream_ptr
+        from ._lib import calls, stream_ptr
         plan = self._step_plan()
         if plan is not None:
-            check(lib().qlmb_dec_step(plan, stream_ptr()))
+            calls.dec_step(self._plan_addr, stream_ptr())
             fn = self.fn
         else:
             fn = self._layers_chain()

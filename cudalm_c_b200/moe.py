@@ -1,8 +1,10 @@
 """Host-side mirror of the reference's MoE operators (cudalm.cu:2515-2534,
 3537-3602, 4151-4393): router_topk, moe_perm_all, moe_forward, moe_backward."""
+import ctypes as C
+
 import torch
 
-from ._lib import BF16, F32, MoeLayer, check, lib, ptr, stream_ptr
+from ._lib import BF16, F32, MoeLayer, calls, check, lib, ptr, stream_ptr
 
 
 def _dt(t):
@@ -67,6 +69,7 @@ class MoeLayerState:
         self.c = MoeLayer(N, D, F, E, K, BF16 if dtype == torch.bfloat16 else F32,
                           ptr(q1[0]), ptr(q3[0]), ptr(q2[0]), ptr(q1[1]), ptr(q3[1]), ptr(q2[1]),
                           ptr(wr), ptr(bias), bias_stride, aux)
+        self.c_addr = C.addressof(self.c)
         self.rows_cap = (K * N + E * 127 + 127) // 128 * 128
 
     def member(self, name, shape, dtype):
@@ -95,17 +98,16 @@ class MoeLayerState:
         if rt is not None:
             check(lib().qlmb_moe_forward_routed(self.c, self.arena_ptr, ptr(out), ptr(f_in), ptr(f_norm), ptr(rt), stream_ptr()))
         else:
-            check(lib().qlmb_moe_forward(self.c, self.arena_ptr, ptr(out), ptr(f_in), ptr(f_norm), stream_ptr()))
+            calls.moe_forward(self.c_addr, self.arena_ptr, out, f_in, f_norm, stream_ptr())
         return out
 
     def decode(self, f_in, f_norm, out=None):
         """The forward of a decode step: no stash; routed GEMVs when K*N <= 128."""
         out = out if out is not None else torch.empty_like(f_in)
-        check(lib().qlmb_moe_decode(self.c, self.arena_ptr, ptr(out), ptr(f_in), ptr(f_norm), stream_ptr()))
+        calls.moe_decode(self.c_addr, self.arena_ptr, out, f_in, f_norm, stream_ptr())
         return out
 
     def backward(self, dout, f_norm, dW1, dW3, dW2, dWr, beta=1.0, dfnorm=None):
         dfnorm = dfnorm if dfnorm is not None else torch.empty_like(dout)
-        check(lib().qlmb_moe_backward(self.c, self.arena_ptr, ptr(dfnorm), ptr(dout), ptr(f_norm), ptr(dW1),
-                                      ptr(dW3), ptr(dW2), ptr(dWr), beta, stream_ptr()))
+        calls.moe_backward(self.c_addr, self.arena_ptr, dfnorm, dout, f_norm, dW1, dW3, dW2, dWr, beta, stream_ptr())
         return dfnorm

@@ -12,7 +12,7 @@ import math
 import numpy as np
 import torch
 
-from ._lib import SPAN_DTYPE, check, lib, ptr, stream_ptr
+from ._lib import SPAN_DTYPE, calls, check, lib, ptr, stream_ptr
 
 
 def qd_bytes(nq, packed):
@@ -38,9 +38,8 @@ def qlm_render(P, d, s, spans_dev, nspan, group=128, packed=1, gi_base=0, ng=Non
 def qlm_step_launch(P, G, d, r, s, m8, m8s, v8, v8s, spans_dev, nspan, group, dmax, lr, b1, b2, wd, gscale,
                     gsp, inv_bc1, inv_sqrt_bc2, lrmode, t, adam, stat, packed, gi_base, ng):
     """Argument for argument the reference's qlm_step_launch (qlm.cuh:377-383)."""
-    check(lib().qlmb_step(ptr(P), ptr(G), ptr(d), ptr(r), ptr(s), ptr(m8), ptr(m8s), ptr(v8), ptr(v8s),
-                          ptr(spans_dev), nspan, group, dmax, lr, b1, b2, wd, gscale, ptr(gsp), inv_bc1,
-                          inv_sqrt_bc2, lrmode, t, adam, ptr(stat), packed, gi_base, ng, stream_ptr()))
+    calls.step(P, G, d, r, s, m8, m8s, v8, v8s, spans_dev, nspan, group, dmax, lr, b1, b2, wd, gscale, gsp, inv_bc1,
+               inv_sqrt_bc2, lrmode, t, adam, stat, packed, gi_base, ng, stream_ptr())
 
 
 def qlm_servo(d, r, s, spans_dev, nspan, group, dmax, f_hi, f_lo, packed=1):
@@ -61,8 +60,7 @@ def gnorm(G, sides=(), clip_side=0, out=None):
 
 def adamw(P, G, M, V, lr, b1, b2, wd, bc1, bc2, gs=None):
     """k_adamw for float spans; M, V are bf16 bit patterns (int16/uint16 storage)."""
-    check(lib().qlmb_adamw(ptr(P), ptr(G), ptr(M), ptr(V), P.numel(), lr, b1, b2, wd, bc1, bc2, ptr(gs),
-                           stream_ptr()))
+    calls.adamw(P, G, M, V, P.numel(), lr, b1, b2, wd, bc1, bc2, gs, stream_ptr())
 
 
 def sqsum(G, part64):
