@@ -104,9 +104,10 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
 
     if (smem_u32(at_smem) & 1023u) {          // the swizzled tiles need a 1 KiB-aligned base
         if (threadIdx.x == 0 && p.errword && atomicCAS(p.errword, 0, 201) == 0) { p.errword[1] = 100; p.errword[2] = (int)blockIdx.x; }
+        pdl_wait();
         return;
     }
-    if (__syncthreads_or(threadIdx.x == 0 && at_error_seen(p.errword))) return;   // uniform over the CTA
+    if (__syncthreads_or(threadIdx.x == 0 && at_error_seen(p.errword))) { pdl_wait(); return; }   // uniform over the CTA
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(q_full), 1);
         for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&kv_full[i]), 1); mbar_init(smem_u32(&kv_empty[i]), 1); }
@@ -123,6 +124,8 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();                               // barriers and TMEM above are this kernel's own; its inputs come below
+    pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tS = tmem_base, tPV = tmem_base + 128;
 
@@ -381,6 +384,8 @@ struct AttnBwdParams {
 
 __global__ void __launch_bounds__(256) k_attn_drow(float *drow, const bf16 *dA, const bf16 *O, int B, int T, int H)
 {
+    pdl_wait();
+    pdl_trigger();
     const size_t g = (size_t)blockIdx.x * 256 + threadIdx.x;
     if (g >= (size_t)B * T * H) return;
     const int h = (int)(g % H);
@@ -458,7 +463,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dkv(const __grid
         if (threadIdx.x == 0 && p.errword && atomicCAS(p.errword, 0, 201) == 0) { p.errword[1] = 200; p.errword[2] = (int)blockIdx.x; }
         return;
     }
-    if (__syncthreads_or(threadIdx.x == 0 && at_error_seen(p.errword))) return;   // uniform over the CTA
+    if (__syncthreads_or(threadIdx.x == 0 && at_error_seen(p.errword))) { pdl_wait(); return; }   // uniform over the CTA
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(kv_full), 1);
         for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&qd_full[i]), 2); mbar_init(smem_u32(&qd_empty[i]), 1); }
@@ -473,6 +478,8 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dkv(const __grid
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();                               // barriers and TMEM above are this kernel's own; its inputs come below
+    pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tS = tmem_base, tP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 320;
 
@@ -658,7 +665,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dq(const __grid_
         if (threadIdx.x == 0 && p.errword && atomicCAS(p.errword, 0, 201) == 0) { p.errword[1] = 300; p.errword[2] = (int)blockIdx.x; }
         return;
     }
-    if (__syncthreads_or(threadIdx.x == 0 && at_error_seen(p.errword))) return;   // uniform over the CTA
+    if (__syncthreads_or(threadIdx.x == 0 && at_error_seen(p.errword))) { pdl_wait(); return; }   // uniform over the CTA
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(qa_full), 1);
         for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&kv_full[i]), 1); mbar_init(smem_u32(&kv_empty[i]), 1); }
@@ -673,6 +680,8 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dq(const __grid_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();                               // barriers and TMEM above are this kernel's own; its inputs come below
+    pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tS = tmem_base, tP = tmem_base + 128, tdQ = tmem_base + 256;
 
@@ -867,7 +876,7 @@ extern "C" int qlmb_attn_fwd(void *O, float *lse, const void *Q, const void *K, 
         QLMB_CUDA(cudaFuncSetAttribute(k_attn_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_FWD_SMEM));
         configured_dev[dev_] = true;
     }
-    k_attn_fwd<<<(unsigned)(p.nqt * B * H), 320, AT_FWD_SMEM, as_stream(stream)>>>(p);
+    QLMB_CUDA(pdl_launch_small(k_attn_fwd, dim3((unsigned)(p.nqt * B * H)), dim3(320), AT_FWD_SMEM, as_stream(stream), p));
     QLMB_LAUNCH_CHECK("k_attn_fwd");
     return QLMB_OK;
 }
@@ -909,9 +918,9 @@ extern "C" int qlmb_attn_bwd(void *dQ, void *dK, void *dV, float *drow, const vo
     }
     cudaStream_t st = as_stream(stream);
     const size_t nrow = (size_t)B * T * H;
-    k_attn_drow<<<(unsigned)((nrow + 255) / 256), 256, 0, st>>>(drow, (const bf16 *)dA, (const bf16 *)O, B, T, H);
-    k_attn_bwd_dkv<<<(unsigned)(p.nqt * B * KV), AT_BWD_THREADS, AT_DKV_SMEM, st>>>(p);
-    k_attn_bwd_dq<<<(unsigned)(p.nqt * B * H), AT_BWD_THREADS, AT_DQ_SMEM, st>>>(p);
+    QLMB_CUDA(pdl_launch_small(k_attn_drow, dim3((unsigned)((nrow + 255) / 256)), dim3(256), 0, st, drow, (const bf16 *)dA, (const bf16 *)O, B, T, H));
+    QLMB_CUDA(pdl_launch_small(k_attn_bwd_dkv, dim3((unsigned)(p.nqt * B * KV)), dim3(AT_BWD_THREADS), AT_DKV_SMEM, st, p));
+    QLMB_CUDA(pdl_launch_small(k_attn_bwd_dq, dim3((unsigned)(p.nqt * B * H)), dim3(AT_BWD_THREADS), AT_DQ_SMEM, st, p));
     QLMB_LAUNCH_CHECK("k_attn_bwd");
     return QLMB_OK;
 }

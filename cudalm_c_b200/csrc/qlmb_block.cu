@@ -58,6 +58,8 @@ __device__ __forceinline__ float warp_max(float v)
 // X[n,:] = emb[tok[n],:]  (k_embed, cpu_kern.h:87-90).  One warp per token row.
 __global__ void __launch_bounds__(256) k_embed(void *X, int x_dtype, const float *emb, const int *tok, int N, int D)
 {
+    pdl_wait();
+    pdl_trigger();
     const int n = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (n >= N) return;
     const float *src = emb + (size_t)tok[n] * D;
@@ -71,6 +73,8 @@ __global__ void __launch_bounds__(256) k_embed(void *X, int x_dtype, const float
 template <int NV>
 __global__ void __launch_bounds__(256) k_embed_bwd(float *G, const void *dout, int dtype, const int *tok, int N, int D, int V)
 {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int stok[2048];
     const int v = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     float4 acc[NV];
@@ -117,6 +121,8 @@ __global__ void __launch_bounds__(256) k_embed_bwd(float *G, const void *dout, i
 __global__ void __launch_bounds__(256) k_rmsnorm_fwd(void *O, int o_dtype, float *rinv, const void *X, int x_dtype,
                                                      const float *gamma, int N, int D)
 {
+    pdl_wait();
+    pdl_trigger();
     const int n = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (n >= N) return;
     float ss = 0.0f;
@@ -138,6 +144,8 @@ __global__ void __launch_bounds__(256) k_rmsnorm_bwd(void *dx, int dx_dtype, int
                                                      const float *gamma, const float *rinv, const void *dy, int dy_dtype,
                                                      int N, int D)
 {
+    pdl_wait();
+    pdl_trigger();
     const int n = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (n >= N) return;
     float c = 0.0f;
@@ -166,6 +174,8 @@ __global__ void __launch_bounds__(256) k_rmsnorm_bwd(void *dx, int dx_dtype, int
 __global__ void __launch_bounds__(128) k_gamma_part(float *part, const void *X, int x_dtype, const float *rinv, const void *dy,
                                                     int dy_dtype, int N, int D)
 {
+    pdl_wait();
+    pdl_trigger();
     const int c = blockIdx.y, j = blockIdx.x * 128 + threadIdx.x;
     if (j >= D) return;
     const int r0 = (int)((long long)N * c / GAMMA_CH), r1 = (int)((long long)N * (c + 1) / GAMMA_CH);
@@ -185,6 +195,8 @@ __global__ void __launch_bounds__(128) k_gamma_part(float *part, const void *X, 
 }
 __global__ void __launch_bounds__(128) k_gamma_sum(float *G, const float *part, int D)
 {
+    pdl_wait();
+    pdl_trigger();
     const int j = blockIdx.x * 128 + threadIdx.x;
     if (j >= D) return;
     float a = 0.0f;
@@ -216,6 +228,8 @@ __global__ void __launch_bounds__(256) k_rope(void *buf, int dtype, const float 
 __global__ void __launch_bounds__(256) k_rope8(void *buf, int dtype, const float *cosb, const float *sinb, size_t total, int nh,
                                                int hd, int T, int back)
 {
+    pdl_wait();
+    pdl_trigger();
     const size_t g = (size_t)blockIdx.x * 256 + threadIdx.x;
     if (g >= total) return;
     const int hf = hd / 2, per = hf / 8, i = (int)(g % per) * 8;
@@ -251,6 +265,8 @@ __global__ void __launch_bounds__(256) k_rope8(void *buf, int dtype, const float
 __global__ void __launch_bounds__(256) k_softmax_ce(const void *lg, int lg_dtype, const int *tgt, float *loss, void *dl,
                                                     int dl_dtype, int V, int n_all)
 {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float red[8];
     __shared__ float bc;
     const size_t row = blockIdx.x;
@@ -414,6 +430,8 @@ __global__ void __launch_bounds__(128) k_dec_attn(bf16_t *O, const bf16_t *Q, co
 // log-probability of the pick.  One block per slot.
 __global__ void __launch_bounds__(256) k_dec_greedy(int *out, float *lp, const float *logits, int V)
 {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float rv[8], rs[8];
     __shared__ int ri[8];
     const int s = blockIdx.x, tid = threadIdx.x, w = tid >> 5, ln = tid & 31;
@@ -650,7 +668,7 @@ extern "C" int qlmb_embed(void *X, int x_dtype, const float *emb, const int *tok
     QLMB_REQUIRE(X && emb && tok && dtype_ok(x_dtype), "qlmb_embed: bad argument");
     QLMB_REQUIRE(D > 0 && D % 4 == 0, "qlmb_embed: D %d must be a multiple of 4", D);
     if (N <= 0) return QLMB_OK;
-    k_embed<<<(N + 7) / 8, 256, 0, as_stream(stream)>>>(X, x_dtype, emb, tok, N, D);
+    QLMB_CUDA(pdl_launch(true, k_embed, dim3((N + 7) / 8), dim3(256), 0, as_stream(stream), X, x_dtype, emb, tok, N, D));
     QLMB_LAUNCH_CHECK("k_embed");
     return QLMB_OK;
 }
@@ -662,9 +680,9 @@ extern "C" int qlmb_embed_bwd(float *G, const void *dout, int dtype, const int *
     if (N <= 0 || V <= 0) return QLMB_OK;
     const unsigned grid = (unsigned)((V + 7) / 8);
     cudaStream_t st = as_stream(stream);
-    if (D <= 512) k_embed_bwd<4><<<grid, 256, 0, st>>>(G, dout, dtype, tok, N, D, V);
-    else if (D <= 1024) k_embed_bwd<8><<<grid, 256, 0, st>>>(G, dout, dtype, tok, N, D, V);
-    else k_embed_bwd<16><<<grid, 256, 0, st>>>(G, dout, dtype, tok, N, D, V);
+    if (D <= 512) QLMB_CUDA(pdl_launch(true, k_embed_bwd<4>, dim3(grid), dim3(256), 0, st, G, dout, dtype, tok, N, D, V));
+    else if (D <= 1024) QLMB_CUDA(pdl_launch(true, k_embed_bwd<8>, dim3(grid), dim3(256), 0, st, G, dout, dtype, tok, N, D, V));
+    else QLMB_CUDA(pdl_launch(true, k_embed_bwd<16>, dim3(grid), dim3(256), 0, st, G, dout, dtype, tok, N, D, V));
     QLMB_LAUNCH_CHECK("k_embed_bwd");
     return QLMB_OK;
 }
@@ -675,7 +693,7 @@ extern "C" int qlmb_rmsnorm_fwd(void *O, int o_dtype, float *rinv, const void *X
     QLMB_REQUIRE(O && rinv && X && gamma && dtype_ok(o_dtype) && dtype_ok(x_dtype), "qlmb_rmsnorm_fwd: bad argument");
     QLMB_REQUIRE(D > 0 && D % 4 == 0 && ((uintptr_t)gamma & 15) == 0, "qlmb_rmsnorm_fwd: D %d must be a multiple of 4, gamma 16-byte aligned", D);
     if (N <= 0) return QLMB_OK;
-    k_rmsnorm_fwd<<<(N + 7) / 8, 256, 0, as_stream(stream)>>>(O, o_dtype, rinv, X, x_dtype, gamma, N, D);
+    QLMB_CUDA(pdl_launch(true, k_rmsnorm_fwd, dim3((N + 7) / 8), dim3(256), 0, as_stream(stream), O, o_dtype, rinv, X, x_dtype, gamma, N, D));
     QLMB_LAUNCH_CHECK("k_rmsnorm_fwd");
     return QLMB_OK;
 }
@@ -689,10 +707,10 @@ extern "C" int qlmb_rmsnorm_bwd(void *dx, int dx_dtype, int accumulate, float *d
     QLMB_REQUIRE(!dgamma || part, "qlmb_rmsnorm_bwd: the gain gradient needs the 128 x D scratch");
     if (N <= 0) return QLMB_OK;
     cudaStream_t st = as_stream(stream);
-    k_rmsnorm_bwd<<<(N + 7) / 8, 256, 0, st>>>(dx, dx_dtype, accumulate, X, x_dtype, gamma, rinv, dy, dy_dtype, N, D);
+    QLMB_CUDA(pdl_launch(true, k_rmsnorm_bwd, dim3((N + 7) / 8), dim3(256), 0, st, dx, dx_dtype, accumulate, X, x_dtype, gamma, rinv, dy, dy_dtype, N, D));
     if (dgamma) {
-        k_gamma_part<<<dim3((D + 127) / 128, GAMMA_CH), 128, 0, st>>>(part, X, x_dtype, rinv, dy, dy_dtype, N, D);
-        k_gamma_sum<<<(D + 127) / 128, 128, 0, st>>>(dgamma, part, D);
+        QLMB_CUDA(pdl_launch(true, k_gamma_part, dim3((D + 127) / 128, GAMMA_CH), dim3(128), 0, st, part, X, x_dtype, rinv, dy, dy_dtype, N, D));
+        QLMB_CUDA(pdl_launch(true, k_gamma_sum, dim3((D + 127) / 128), dim3(128), 0, st, dgamma, part, D));
     }
     QLMB_LAUNCH_CHECK("k_rmsnorm_bwd");
     return QLMB_OK;
@@ -706,7 +724,7 @@ extern "C" int qlmb_rope(void *buf, int dtype, const float *cosb, const float *s
     if (N <= 0) return QLMB_OK;
     if ((hd / 2) % 8 == 0 && (((uintptr_t)buf | (uintptr_t)cosb | (uintptr_t)sinb) & 15) == 0) {
         const size_t total = (size_t)N * nh * (hd / 16);
-        k_rope8<<<(unsigned)((total + 255) / 256), 256, 0, as_stream(stream)>>>(buf, dtype, cosb, sinb, total, nh, hd, T, back);
+        QLMB_CUDA(pdl_launch(true, k_rope8, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, as_stream(stream), buf, dtype, cosb, sinb, total, nh, hd, T, back));
     } else {
         const size_t total = (size_t)N * nh * (hd / 2);
         k_rope<<<(unsigned)((total + 255) / 256), 256, 0, as_stream(stream)>>>(buf, dtype, cosb, sinb, total, nh, hd, T, back);
@@ -721,7 +739,7 @@ extern "C" int qlmb_softmax_ce(const void *logits, int lg_dtype, const int *tgt,
     QLMB_REQUIRE(logits && tgt && loss && dlogits && dtype_ok(lg_dtype) && dtype_ok(dl_dtype), "qlmb_softmax_ce: bad argument");
     QLMB_REQUIRE(V > 0 && n_all > 0, "qlmb_softmax_ce: bad shape V %d n_all %d", V, n_all);
     if (rows <= 0) return QLMB_OK;
-    k_softmax_ce<<<(unsigned)rows, 256, 0, as_stream(stream)>>>(logits, lg_dtype, tgt, loss, dlogits, dl_dtype, V, n_all);
+    QLMB_CUDA(pdl_launch(true, k_softmax_ce, dim3((unsigned)rows), dim3(256), 0, as_stream(stream), logits, lg_dtype, tgt, loss, dlogits, dl_dtype, V, n_all));
     QLMB_LAUNCH_CHECK("k_softmax_ce");
     return QLMB_OK;
 }
@@ -775,7 +793,7 @@ extern "C" int qlmb_dec_greedy(int *out, float *lp, const float *logits, int B, 
 {
     QLMB_REQUIRE(out && lp && logits && V > 0, "qlmb_dec_greedy: bad argument");
     if (B <= 0) return QLMB_OK;
-    k_dec_greedy<<<(unsigned)B, 256, 0, as_stream(stream)>>>(out, lp, logits, V);
+    QLMB_CUDA(pdl_launch(true, k_dec_greedy, dim3((unsigned)B), dim3(256), 0, as_stream(stream), out, lp, logits, V));
     QLMB_LAUNCH_CHECK("k_dec_greedy");
     return QLMB_OK;
 }

@@ -48,8 +48,12 @@ struct ProfScope {
 // pdl_wait(), which returns once that kernel has completed and its writes are visible.  Rules kept by every such kernel:
 // every block executes pdl_wait() exactly once, before its first read of anything a kernel of the stream wrote, before
 // its first write, and before any early return; only data that no kernel of the step writes (the weights) is touched
-// ahead of it.  The caller decides per launch (`early`): with one to four rows per step the early blocks cost the
+// ahead of it.  Weights may be: a kernel that writes codes or scales never triggers, so whatever follows it starts after
+// its end, and a kernel that triggers does so after its own wait wherever a reader of weights can follow directly.
+// The caller decides per launch (`early`): with one to four rows per step the early blocks of the decode chain cost the
 // running kernel more than they gain (decode step 0.53 -> 0.56 ms at one slot, 0.85 -> 0.81 ms at eight, CUDA events).
+// The tensor-core kernels set up their barriers and TMEM, the streaming GEMV requests its first weights, the row kernels
+// do nothing ahead of the wait: what they save is the gap between two launches of a stream.
 // QLMB_PDL=0 turns the attribute off everywhere (the instructions are then no-ops).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -64,6 +68,15 @@ static inline cudaError_t pdl_launch(bool early, void (*kern)(KArgs...), dim3 gr
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = (early && pdl_enabled()) ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+// Early blocks gain the gap between two launches (about 1.5 us) but hold their SM while they wait.  Where other streams
+// have work for that SM (an expert layer's backward: 678 -> 700 us with every launch early) or a kernel has several waves
+// of blocks beside a small successor (attention of 8 x 1024 x 12 heads 257 -> 267 us) they cost more than they gain: the
+// former launches are never early, the latter only with up to two blocks per SM.
+template <typename... KArgs, typename... Args>
+static inline cudaError_t pdl_launch_small(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
+{
+    return pdl_launch((size_t)grid.x * grid.y * grid.z <= (size_t)2 * sm_count(), kern, grid, block, smem, st, args...);
 }
 
 // ---- device helpers --------------------------------------------------------

@@ -68,6 +68,8 @@ template <int N_> __device__ __forceinline__ void cp_async_wait() { asm volatile
 template <int XBF16>
 __global__ void __launch_bounds__(256) k_router_logits_tile(float *rt, const void *X, const float *Wr, int N, int D, int E)
 {
+    pdl_wait();
+    pdl_trigger();
     constexpr int NST = XBF16 ? 4 : 3;                   // stages
     constexpr int XROW = XBF16 ? 80 : 144;               // bytes per token row of a stage (64 / 128 + pad)
     __shared__ __align__(16) uint8_t xs[NST][RLT_TOK * XROW];
@@ -227,8 +229,8 @@ int router_logits(float *rt, const void *X, int x_dtype, const float *Wr, int N,
 {
     if (E <= 32 && (D % 8) == 0 && (((uintptr_t)X | (uintptr_t)Wr) & 15) == 0) {
         int blocks = (N + RLT_TOK - 1) / RLT_TOK;
-        if (x_dtype == QLMB_BF16) k_router_logits_tile<1><<<blocks, 256, 0, st>>>(rt, X, Wr, N, D, E);
-        else k_router_logits_tile<0><<<blocks, 256, 0, st>>>(rt, X, Wr, N, D, E);
+        if (x_dtype == QLMB_BF16) QLMB_CUDA(pdl_launch_small(k_router_logits_tile<1>, dim3(blocks), dim3(256), 0, st, rt, X, Wr, N, D, E));
+        else QLMB_CUDA(pdl_launch_small(k_router_logits_tile<0>, dim3(blocks), dim3(256), 0, st, rt, X, Wr, N, D, E));
     } else {
         k_router_logits<<<(N + RL_TOK - 1) / RL_TOK, 256, 0, st>>>(rt, X, x_dtype, Wr, N, D, E);
     }
@@ -241,6 +243,8 @@ int router_logits(float *rt, const void *X, int x_dtype, const float *Wr, int N,
 __global__ void __launch_bounds__(256) k_gather_rows(bf16 *Xp, const void *src, int dtype,
                                                      const int *perm, const int *nrows_dev, int nrows_host, int N, int D)
 {
+    pdl_wait();
+    pdl_trigger();
     int rows = nrows_dev ? *nrows_dev : nrows_host;
     int lane = threadIdx.x & 31;
     for (int j = blockIdx.x * 8 + (threadIdx.x >> 5); j < rows; j += gridDim.x * 8) {
@@ -270,7 +274,7 @@ int gather_rows(bf16 *Xp, const void *src, int dtype, const int *perm, const int
     int blocks = (max_rows + 7) / 8;
     int cap = sm_count() * 8;
     if (blocks > cap) blocks = cap;
-    k_gather_rows<<<blocks, 256, 0, st>>>(Xp, src, dtype, perm, nrows_dev, max_rows, N, D);
+    QLMB_CUDA(pdl_launch_small(k_gather_rows, dim3(blocks), dim3(256), 0, st, Xp, src, dtype, perm, nrows_dev, max_rows, N, D));
     QLMB_LAUNCH_CHECK("k_gather_rows");
     return QLMB_OK;
 }
@@ -282,6 +286,8 @@ __global__ void __launch_bounds__(256) k_combine_rows(void *out, const void *f_i
                                                       const bf16 *yp, const int *inv, const float *gate,
                                                       int N, int D, int K)
 {
+    pdl_wait();
+    pdl_trigger();
     int n = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (n >= N) return;
     for (int c = lane; c < D / 8; c += 32) {
@@ -302,7 +308,7 @@ __global__ void __launch_bounds__(256) k_combine_rows(void *out, const void *f_i
 int combine_rows(void *out, const void *f_in, int dtype, const bf16 *yp, const int *inv, const float *gate,
                  int N, int D, int K, cudaStream_t st)
 {
-    k_combine_rows<<<(N + 7) / 8, 256, 0, st>>>(out, f_in, dtype, yp, inv, gate, N, D, K);
+    QLMB_CUDA(pdl_launch_small(k_combine_rows, dim3((N + 7) / 8), dim3(256), 0, st, out, f_in, dtype, yp, inv, gate, N, D, K));
     QLMB_LAUNCH_CHECK("k_combine_rows");
     return QLMB_OK;
 }
@@ -944,6 +950,8 @@ int count_assign(int *counts, const int *assign, int KN, int E, cudaStream_t st)
 // ----------------------------------------------------------- conversions
 __global__ void __launch_bounds__(256) k_f32_to_bf16(bf16 *dst, const float *src, size_t n8, size_t n)
 {
+    pdl_wait();
+    pdl_trigger();
     size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
     size_t stride = (size_t)gridDim.x * 256;
     for (size_t c = i; c < n8; c += stride) {
@@ -961,7 +969,7 @@ int convert_f32_to_bf16(bf16 *dst, const float *src, size_t n, cudaStream_t st)
     size_t cap = (size_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
     if (blocks == 0) blocks = 1;
-    k_f32_to_bf16<<<(unsigned)blocks, 256, 0, st>>>(dst, src, n8, n);
+    QLMB_CUDA(pdl_launch(true, k_f32_to_bf16, dim3((unsigned)blocks), dim3(256), 0, st, dst, src, n8, n));
     QLMB_LAUNCH_CHECK("k_f32_to_bf16");
     return QLMB_OK;
 }

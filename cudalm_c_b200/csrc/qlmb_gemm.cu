@@ -578,6 +578,8 @@ k_gemm(const __grid_constant__ GemmParams p)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();                                          // barriers and TMEM above are this kernel's own; its operands come below
+    pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
 
     const int ntr = (SCHED == SCHED_ROWS) ? *p.ntiles_dev : 0;
@@ -864,7 +866,7 @@ int make_map(CUtensorMap *m, const void *base, CUtensorMapDataType dt, int esize
 }
 
 template <int BMODE, int EPI, int SCHED>
-static int launch_inst(const GemmParams &p, int grid, cudaStream_t st)
+static int launch_inst(const GemmParams &p, int grid, cudaStream_t st, bool early)
 {
     constexpr bool DEQ = (BMODE == B_DEQ_MN || BMODE == B_DEQ_K);
     constexpr int NSA = DEQ ? 3 : 4, NSB = DEQ ? 3 : 4, NSC = 4;
@@ -875,13 +877,13 @@ static int launch_inst(const GemmParams &p, int grid, cudaStream_t st)
         QLMB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured = true;
     }
-    kfn<<<grid, DEQ ? 576 : 320, smem, st>>>(p);
+    QLMB_CUDA(pdl_launch(early, kfn, dim3(grid), dim3(DEQ ? 576 : 320), smem, st, p));
     QLMB_LAUNCH_CHECK("k_gemm");
     return QLMB_OK;
 }
 
 template <int BMODE, int EPI, int SCHED, int DQG>
-static int launch_pair_g(const GemmParams &p, long long total, cudaStream_t st)
+static int launch_pair_g(const GemmParams &p, long long total, cudaStream_t st, bool early)
 {
     constexpr bool DEQ = (BMODE == B_DEQ_MN || BMODE == B_DEQ_K);
     constexpr size_t smem = 1024 + (size_t)(DEQ ? (EPI == EPI_SWIGLU_BWD ? 4 : 5) : 6) * (P_A_STAGE + P_B_STAGE) + (DEQ ? P_NSC * P_C_STAGE + P_S_RING : 0) + EPI_WARPS * epi_stage_bytes(EPI) + 512;
@@ -903,15 +905,15 @@ static int launch_pair_g(const GemmParams &p, long long total, cudaStream_t st)
         max_clusters = n;
     }
     long long clusters = total < max_clusters ? total : max_clusters;
-    kfn<<<(unsigned)(2 * clusters), DEQ ? 576 : 320, smem, st>>>(p);
+    QLMB_CUDA(pdl_launch(early, kfn, dim3((unsigned)(2 * clusters)), dim3(DEQ ? 576 : 320), smem, st, p));
     QLMB_LAUNCH_CHECK("k_gemm_pair");
     return QLMB_OK;
 }
 
 template <int BMODE, int EPI, int SCHED>
-static int launch_pair(const GemmParams &p, long long total, cudaStream_t st)
+static int launch_pair(const GemmParams &p, long long total, cudaStream_t st, bool early)
 {
-    return launch_pair_g<BMODE, EPI, SCHED, 2>(p, total, st);     // two dequant stage groups
+    return launch_pair_g<BMODE, EPI, SCHED, 2>(p, total, st, early);     // two dequant stage groups
 }
 
 // The two-SM form needs whole 256-column tiles (128 activation columns with the SwiGLU
@@ -1013,7 +1015,7 @@ int gemm_launch(const GemmLaunch &g, cudaStream_t st)
     if (total < grid) grid = (int)total;
     ProfScope prof(g.name ? g.name : "gemm", st);
 
-#define PAIR(BM_, EP_, SC_) if (pair && g.bmode == BM_ && g.epi == EP_ && g.sched == SC_) return launch_pair<BM_, EP_, SC_>(p, total, st)
+#define PAIR(BM_, EP_, SC_) if (pair && g.bmode == BM_ && g.epi == EP_ && g.sched == SC_) return launch_pair<BM_, EP_, SC_>(p, total, st, !g.beside)
     PAIR(B_DEQ_MN, EPI_STORE, SCHED_DENSE);
     PAIR(B_DEQ_K, EPI_STORE, SCHED_DENSE);
     PAIR(AB_TMA_MN, EPI_ACCUM, SCHED_DENSE);
@@ -1025,7 +1027,7 @@ int gemm_launch(const GemmLaunch &g, cudaStream_t st)
     PAIR(AB_TMA_MN, EPI_ACCUM, SCHED_GROUPK);
 #undef PAIR
 
-#define INST(BM_, EP_, SC_) if (g.bmode == BM_ && g.epi == EP_ && g.sched == SC_) return launch_inst<BM_, EP_, SC_>(p, grid, st)
+#define INST(BM_, EP_, SC_) if (g.bmode == BM_ && g.epi == EP_ && g.sched == SC_) return launch_inst<BM_, EP_, SC_>(p, grid, st, !g.beside)
     // dense linears
     INST(B_DEQ_MN, EPI_STORE, SCHED_DENSE);
     INST(B_DEQ_K, EPI_STORE, SCHED_DENSE);

@@ -50,6 +50,7 @@ struct GemmLaunch {
     // rank, possibly peer-mapped); rows with scatter_perm[j] < 0 are not written
     const int *scatter_perm; int scatter_kn; const void *scatter_out[8];
     const char *name;              // label for the optional per-kernel timing
+    bool beside;                   // other streams run work beside this launch: it does not start early
 };
 
 int gemm_launch(const GemmLaunch &g, cudaStream_t st);

@@ -185,6 +185,8 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
     __syncthreads();
     cluster_sync();
     tc_fence_after();
+    pdl_wait();                                          // barriers and TMEM above are this kernel's own; its operands come below
+    pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
 
     const int npairs = gridDim.x >> 1, pair = blockIdx.x >> 1;

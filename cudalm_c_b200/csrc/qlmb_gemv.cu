@@ -238,6 +238,9 @@ __global__ void __launch_bounds__(256, BT <= 2 ? 3 : 2) k_gemv_stream(void *Y, i
         }
     };
     fetch(0);                                            // the weights do not depend on the activations: request them first
+    // a kernel that writes codes never lets the next one start early, so they are complete here; what follows waits
+    pdl_wait();
+    pdl_trigger();
     for (int i = threadIdx.x; i < BT * kslice; i += 256) {
         const int b = i / kslice, k = k0 + i % kslice;
         gsm[i] = b < B ? ld_x(X, dtype, (size_t)b * K + k) : 0.0f;
@@ -1151,7 +1154,7 @@ static int gemv_decode_impl(void *Y, const void *X, const int8_t *codes, const f
         do { \
             static bool attr_done[64]; int dv = 0; QLMB_CUDA(cudaGetDevice(&dv)); \
             if (dv >= 0 && dv < 64 && !attr_done[dv]) { QLMB_CUDA(cudaFuncSetAttribute(k_gemv_stream<BT_, CPL_>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024)); attr_done[dv] = true; } \
-            k_gemv_stream<BT_, CPL_><<<g, 256, sm_b, st>>>(Y, dtype, (float *)ws2, X, (const uint8_t *)codes, scales, B, K, N, ksl, 65536u); \
+            QLMB_CUDA(pdl_launch((int)(g.x * g.y) <= sm_count(), k_gemv_stream<BT_, CPL_>, g, dim3(256), sm_b, st, Y, dtype, (float *)ws2, X, (const uint8_t *)codes, scales, B, K, N, ksl, 65536u)); \
         } while (0)
         if (cpl == 16) { if (bt == 1) GS_LAUNCH(1, 16); else if (bt == 2) GS_LAUNCH(2, 16); else GS_LAUNCH(4, 16); }
         else { if (bt == 1) GS_LAUNCH(1, 8); else if (bt == 2) GS_LAUNCH(2, 8); else GS_LAUNCH(4, 8); }

@@ -48,11 +48,15 @@ static int check_linear(const char *who, int layout, int M, int K, int N, int dt
 // row offsets of S equal slices (the `off` table of the grouped weight-gradient schedule)
 __global__ void k_slice_offsets(int *off, int S, int rows)
 {
+    pdl_wait();
+    pdl_trigger();
     if ((int)threadIdx.x <= S) off[threadIdx.x] = (int)threadIdx.x * rows;
 }
 // dW = beta * dW + part[0] + part[1] + ... in ascending slice order; n is a multiple of 4
 __global__ void __launch_bounds__(256) k_sum_slices(float *dW, const float *part, int S, size_t n, float beta)
 {
+    pdl_wait();
+    pdl_trigger();
     const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;
     if (i >= n) return;
     float4 a = *reinterpret_cast<const float4 *>(part + i);
@@ -161,14 +165,14 @@ extern "C" int qlmb_linear_wgrad(float *dW, const void *dY, const void *X, int l
     if (S > 1) {
         float *part = (float *)((uint8_t *)ws + conv);
         int *off = (int *)((uint8_t *)part + (size_t)S * Md * Nd * sizeof(float));
-        k_slice_offsets<<<1, 32, 0, st>>>(off, S, M / S);
+        QLMB_CUDA(pdl_launch(true, k_slice_offsets, dim3(1), dim3(32), 0, st, off, S, M / S));
         g.sched = SCHED_GROUPK;
         g.nseg = 1; g.M = Md; g.N = Nd; g.E = S; g.off = off;
         g.out = part; g.out_dtype = QLMB_F32; g.ldo = Nd; g.beta = 0.0f; g.name = "gemm_wgrad_slices";
         rc = gemm_launch(g, st);
         if (rc) return rc;
         const size_t n = (size_t)Md * Nd;
-        k_sum_slices<<<(unsigned)((n / 4 + 255) / 256), 256, 0, st>>>(dW, part, S, n, beta);
+        QLMB_CUDA(pdl_launch(true, k_sum_slices, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, st, dW, part, S, n, beta));
         QLMB_LAUNCH_CHECK("k_sum_slices");
         return QLMB_OK;
     }
@@ -214,6 +218,8 @@ namespace qlmb {
 // dst[c][r] = bf16(src[r][c]) through a padded 32 x 32 shared-memory tile
 __global__ void __launch_bounds__(256) k_cast_transpose(bf16 *dst, const float *src, int R, int Cc)
 {
+    pdl_wait();
+    pdl_trigger();
     __shared__ float t[32][33];
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     for (int i = ty; i < 32; i += 8) t[i][tx] = (r0 + i < R && c0 + tx < Cc) ? src[(size_t)(r0 + i) * Cc + c0 + tx] : 0.0f;
@@ -232,7 +238,7 @@ extern "C" int qlmb_cast_bf16(void *dst, void *dst_t, const float *src, int R, i
     cudaStream_t st = as_stream(stream);
     if (dst) { int rc = convert_f32_to_bf16((bf16 *)dst, src, (size_t)R * Cc, st); if (rc) return rc; }
     if (dst_t) {
-        k_cast_transpose<<<dim3((Cc + 31) / 32, (R + 31) / 32), 256, 0, st>>>((bf16 *)dst_t, src, R, Cc);
+        QLMB_CUDA(pdl_launch(true, k_cast_transpose, dim3((Cc + 31) / 32, (R + 31) / 32), dim3(256), 0, st, (bf16 *)dst_t, src, R, Cc));
         QLMB_LAUNCH_CHECK("k_cast_transpose");
     }
     return QLMB_OK;

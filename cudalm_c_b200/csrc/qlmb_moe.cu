@@ -128,7 +128,7 @@ static int experts_backward_gemms(const qlmb_moe_layer *L, const Arena &a, float
         w.a[0] = wg[i].A; w.a_rows = R; w.a_cols = wg[i].Ma;
         w.w[0] = wg[i].B; w.w_cols = wg[i].Nb;
         w.nseg = 1; w.M = wg[i].Ma; w.N = wg[i].Nb; w.E = E; w.off = a.off;
-        w.out = wg[i].out; w.out_dtype = QLMB_F32; w.ldo = wg[i].Nb; w.beta = beta; w.name = wg[i].name;
+        w.out = wg[i].out; w.out_dtype = QLMB_F32; w.ldo = wg[i].Nb; w.beta = beta; w.name = wg[i].name; w.beside = true;
         return gemm_launch(w, s);
     };
     cudaStream_t side = side_fork(st);
@@ -139,7 +139,7 @@ static int experts_backward_gemms(const qlmb_moe_layer *L, const Arena &a, float
     g.w[0] = L->w2_codes; g.scales[0] = L->w2_scales;
     g.w_rows = F; g.w_cols = D; g.nseg = 1; g.ksteps = D / 64; g.M = R; g.N = F; g.E = E;
     g.tile_info = a.tile_info; g.ntiles_dev = a.ntiles; g.max_row_tiles = R / 256 + E / 2 + 1;
-    g.gp = a.gp; g.up = a.up; g.dgp = a.dgp; g.dup = a.dup; g.ldo = F; g.name = "gemm_dact_swiglu_bwd";
+    g.gp = a.gp; g.up = a.up; g.dgp = a.dgp; g.dup = a.dup; g.ldo = F; g.name = "gemm_dact_swiglu_bwd"; g.beside = true;
     if ((rc = gemm_launch(g, st))) { side_join(side, st); return rc; }
     side_wait_main(side, st);
     GemmLaunch h = {};
@@ -148,7 +148,7 @@ static int experts_backward_gemms(const qlmb_moe_layer *L, const Arena &a, float
     h.w[0] = L->w1_codes; h.w[1] = L->w3_codes; h.scales[0] = L->w1_scales; h.scales[1] = L->w3_scales;
     h.w_rows = D; h.w_cols = F; h.nseg = 2; h.ksteps = F / 64; h.M = R; h.N = D; h.E = E;
     h.tile_info = a.tile_info; h.ntiles_dev = a.ntiles; h.max_row_tiles = R / 256 + E / 2 + 1;
-    h.out = a.dXp; h.out_dtype = QLMB_BF16; h.ldo = D; h.name = "gemm_dx";
+    h.out = a.dXp; h.out_dtype = QLMB_BF16; h.ldo = D; h.name = "gemm_dx"; h.beside = true;
     if (sc && sc->perm) { h.scatter_perm = sc->perm; h.scatter_kn = sc->kn; for (int i = 0; i < 8; i++) h.scatter_out[i] = sc->out[i]; }
     rc = gemm_launch(h, st);
     if (!rc) rc = wgrad(1, side);

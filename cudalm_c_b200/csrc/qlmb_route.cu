@@ -75,6 +75,8 @@ __global__ void __launch_bounds__(256) k_router_topk_warp(const float *rt, float
                                                           float *gate, int N, int E, int K,
                                                           const float *bias, int bs)
 {
+    pdl_wait();
+    pdl_trigger();
     int n = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (n >= N) return;
     router_topk_row(lane < E ? rt[(size_t)n * E + lane] : 0.0f, n, lane, rprobs, assign, gate, N, E, K, bias, bs);
@@ -207,6 +209,8 @@ __device__ __forceinline__ void perm_st_remote(int *local, uint32_t rank, int v)
 template <int RPT>
 __global__ void __launch_bounds__(PERM_THREADS) k_perm_cluster(const PermArgs a0, int sorts_stride_asn)
 {
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ int psm[];
     PermArgs a = a0;
     const int E = a.E, sort = blockIdx.y;
@@ -375,10 +379,12 @@ int perm_build(const int *assign, int N, int E, int K, int merged, int pad, int 
     const size_t smem = ((size_t)32 * E + 12 * (size_t)E + 1 + 9) * sizeof(int);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(C, sorts, 1); cfg.blockDim = dim3(PERM_THREADS, 1, 1); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = pdl_enabled() && sorts == 1 ? 2 : 1;
     if (sorts > 1) QLMB_CUDA(cudaMemsetAsync(bad_flag, 0, sizeof(int), st));
     cudaError_t le;
     if (rpw <= 1) le = cudaLaunchKernelEx(&cfg, k_perm_cluster<1>, a, len);
@@ -401,7 +407,7 @@ size_t perm_scratch_ints(int N, int E, int K, int merged)
 int router_topk(const float *rt, float *rprobs, int *assign, float *gate, int N, int E, int K,
                 const float *bias, int bs, cudaStream_t st)
 {
-    if (E <= 32) k_router_topk_warp<<<(N + 7) / 8, 256, 0, st>>>(rt, rprobs, assign, gate, N, E, K, bias, bs);
+    if (E <= 32) QLMB_CUDA(pdl_launch_small(k_router_topk_warp, dim3((N + 7) / 8), dim3(256), 0, st, rt, rprobs, assign, gate, N, E, K, bias, bs));
     else if (E <= 64) k_router_topk_wide<2><<<(N + 7) / 8, 256, 0, st>>>(rt, rprobs, assign, gate, N, E, K, bias, bs);
     else if (E <= 128) k_router_topk_wide<4><<<(N + 7) / 8, 256, 0, st>>>(rt, rprobs, assign, gate, N, E, K, bias, bs);
     else k_router_topk_wide<8><<<(N + 7) / 8, 256, 0, st>>>(rt, rprobs, assign, gate, N, E, K, bias, bs);
