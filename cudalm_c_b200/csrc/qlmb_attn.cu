@@ -61,12 +61,14 @@ __device__ __forceinline__ uint32_t at_test(uint32_t bar, uint32_t parity)     /
 __device__ __forceinline__ bool at_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *errword, int site)
 {
     if (mbar_try(bar, parity)) return true;
-    const unsigned long long t0 = at_now();
+    unsigned long long t0 = 0;                 // read on the slow path only
     for (uint32_t i = 0;; i++) {
         if (at_test(bar, parity)) return true;
         if ((i & 1023u) == 1023u) {
             if (*abort_flag) return false;
-            if (at_now() - t0 > AT_WAIT_NS) break;
+            const unsigned long long now = at_now();
+            if (!t0) t0 = now;
+            else if (now - t0 > AT_WAIT_NS) break;
         }
     }
     if (!*abort_flag) {
@@ -84,10 +86,7 @@ __device__ __forceinline__ float ex2(float x)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ bool attn_valid(int key, int i, int T, int win)
-{
-    return key <= i && key < T && (win <= 0 || key > i - win);
-}
+template <int M> struct AtMode { static constexpr int value = M; };     // which masks a tile needs
 
 __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ AttnFwdParams p)
 {
@@ -182,7 +181,7 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
         if (ok) ok = at_wait(smem_u32(&kv_full[0]), 0, abort_flag, p.errword, 111);
         if (ok) {
             tc_fence_after();
-            if (lane == 0) issue_s(0);
+            if (elect_one()) issue_s(0);
             __syncwarp();
         }
         for (int t = 0; ok && t < nt; t++) {
@@ -196,10 +195,10 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
                 ok = at_wait(smem_u32(&kv_full[st ^ 1]), ((uint32_t)(t + 1) >> 1) & 1u, abort_flag, p.errword, 113);
                 if (!ok) break;
                 tc_fence_after();
-                if (lane == 0) issue_s(st ^ 1);
+                if (elect_one()) issue_s(st ^ 1);
                 __syncwarp();
             }
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t a0 = smem_u32(sP), b0 = smem_u32(sV + st * AT_TILE);
 #pragma unroll
                 for (int kk = 0; kk < AT_BN / 16; kk++)
@@ -211,7 +210,7 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
             __syncwarp();
         }
         if (*abort_flag) {                    // let issued MMAs retire (bounded) before TMEM is released
-            if (lane == 0) tc_commit(smem_u32(spare));
+            if (elect_one()) tc_commit(smem_u32(spare));
             __syncwarp();
             for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(spare), 0); i++) {}
         }
@@ -254,6 +253,7 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
             ok = at_wait(smem_u32(s_full), (uint32_t)t & 1u, abort_flag, p.errword, 120);
             if (!ok) break;
             tc_fence_after();
+            const int klo = i - p.win - k0, khi = (i < p.T ? i : p.T - 1) - k0;
             // pass 1: maximum of this half of the row
             float mx = -1e30f;
 #pragma unroll
@@ -261,10 +261,15 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
                 uint32_t v[32];
                 tmem_ld32(tS + lane_base + hf * 64 + c * 32, v);
                 tmem_ld_wait();
-                if (masked) {
+                if (masked) {                  // keys lo < j <= hi of the 32
+                    const int lo = klo - c * 32, hi = khi - c * 32;
+                    if (p.win > 0) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (attn_valid(k0 + c * 32 + j, i, p.T, p.win)) mx = fmaxf(mx, __uint_as_float(v[j]));
+                        for (int j = 0; j < 32; j++) mx = fmaxf(mx, j <= hi && j > lo ? __uint_as_float(v[j]) : -1e30f);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; j++) mx = fmaxf(mx, j <= hi ? __uint_as_float(v[j]) : -1e30f);
+                    }
                 } else {
 #pragma unroll
                     for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(v[j]));
@@ -297,8 +302,9 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
                     float p0 = ex2(__uint_as_float(v[j]) * p.scale_log2 - m_new);
                     float p1 = ex2(__uint_as_float(v[j + 1]) * p.scale_log2 - m_new);
                     if (masked) {
-                        if (!attn_valid(k0 + c * 32 + j, i, p.T, p.win)) p0 = 0.0f;
-                        if (!attn_valid(k0 + c * 32 + j + 1, i, p.T, p.win)) p1 = 0.0f;
+                        const int jj = c * 32 + j;
+                        if (jj > khi || (p.win > 0 && jj <= klo)) p0 = 0.0f;
+                        if (jj + 1 > khi || (p.win > 0 && jj + 1 <= klo)) p1 = 0.0f;
                     }
                     rs += p0 + p1;
                     __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
@@ -364,17 +370,28 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
 // Both recompute the scores from Q, K and the saved log-sum-exp:  P = exp(S/sqrt(hd) - lse),
 // dS = P * (dP - D) / sqrt(hd) with dP = dA V^T and D = rowsum(dA * O) (k_attn_drow).
 //
+// The walked tiles are 64 wide, so that two CTAs fit an SM (100 / 80 KB of shared memory, 256 TMEM columns each): the
+// element-wise phase of one runs beside the MMAs of the other.
+// What bounds them (clock trace of 8 x 1024 x 12 heads): a step of a CTA takes 3.3 thousand cycles, 1.3 of them
+// element-wise work (one exponential per element: the special-function unit delivers 16 a cycle), the rest the
+// hand-shakes around the MMAs, which the other CTA fills in part.  128-wide tiles with one CTA per SM took 98 + 83 us;
+// 64-wide tiles 85 + 67 us; with the MMAs issued behind elect.sync and masks only on the edge tiles 67 + 49 us.
+//
 //   warp 0      TMA producer   resident tiles once, the walked tiles through a two-stage ring
-//   warp 1      MMA issuer     scores and dP (two 128 x 128 x 64 MMAs into TMEM), then the two
+//   warp 1      MMA issuer     scores and dP (two 128 x 64 x 64 MMAs into TMEM), then the two
 //                              accumulating products from P / dS in shared memory
-//   warps 2-17  element-wise   thread = one TMEM lane (a key for dkv, a query for dq) x 32 of the
-//                              128 columns: P and dS as bf16 into swizzled K-major tiles
-constexpr int AT_BWD_THREADS = 576;             // TMA warp, MMA warp, 16 element-wise warps
-constexpr int AT_DKV_SMEM = 2 * AT_TILE + 4 * AT_TILE + 2 * AT_P_BYTES + 2 * 2 * 128 * 4 + 256;
-constexpr int AT_DQ_SMEM = 2 * AT_TILE + 4 * AT_TILE + AT_P_BYTES + 256;
+//   warps 2-9   element-wise   thread = one TMEM lane (a key for dkv, a query for dq) x 32 of the
+//                              64 columns: P and dS as bf16 into swizzled K-major tiles.  The factor
+//                              1/sqrt(hd) of dS (a power of two) is applied to the finished sums.
+constexpr int AT_BI = 64;                       // queries (dkv) or keys (dq) per step
+constexpr int AT_ITILE = AT_BI * AT_HD * 2;     // bytes of a walked tile
+constexpr int AT_BWD_THREADS = 320;             // TMA warp, MMA warp, 8 element-wise warps
+constexpr int AT_DKV_SMEM = 2 * AT_TILE + 4 * AT_ITILE + 2 * AT_BN * AT_BI * 2 + 2 * 2 * AT_BI * 4 + 256;
+constexpr int AT_DQ_SMEM = 2 * AT_TILE + 4 * AT_ITILE + AT_BM * AT_BI * 2 + 256;
 
 struct AttnBwdParams {
-    alignas(64) CUtensorMap q_map, k_map, v_map, da_map;
+    alignas(64) CUtensorMap q_map, k_map, v_map, da_map;      // boxes of 128 rows (resident tiles)
+    alignas(64) CUtensorMap q_imap, k_imap, v_imap, da_imap;  // boxes of 64 rows (walked tiles)
     const float *lse, *drow;
     bf16 *dQ, *dK, *dV;
     int B, T, H, KV, win, nqt;
@@ -382,20 +399,17 @@ struct AttnBwdParams {
     int *errword;
 };
 
+// eight lanes per (token, head): a load instruction of a warp covers four whole 128-byte rows
 __global__ void __launch_bounds__(256) k_attn_drow(float *drow, const bf16 *dA, const bf16 *O, int B, int T, int H)
 {
     pdl_wait();
     pdl_trigger();
-    const size_t g = (size_t)blockIdx.x * 256 + threadIdx.x;
-    if (g >= (size_t)B * T * H) return;
-    const int h = (int)(g % H);
-    const size_t bt = g / H;
-    const uint4 *a = reinterpret_cast<const uint4 *>(dA + bt * (size_t)H * AT_HD + (size_t)h * AT_HD);
-    const uint4 *o = reinterpret_cast<const uint4 *>(O + bt * (size_t)H * AT_HD + (size_t)h * AT_HD);
+    const size_t g = ((size_t)blockIdx.x * 256 + threadIdx.x) >> 3;
+    const int c = threadIdx.x & 7;
+    const bool live = g < (size_t)B * T * H;
     float acc = 0.0f;
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-        const uint4 x = __ldg(a + u), y = __ldg(o + u);
+    if (live) {
+        const uint4 x = __ldg(reinterpret_cast<const uint4 *>(dA + g * AT_HD) + c), y = __ldg(reinterpret_cast<const uint4 *>(O + g * AT_HD) + c);
         const __nv_bfloat162 *xh = reinterpret_cast<const __nv_bfloat162 *>(&x), *yh = reinterpret_cast<const __nv_bfloat162 *>(&y);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -403,12 +417,18 @@ __global__ void __launch_bounds__(256) k_attn_drow(float *drow, const bf16 *dA, 
             acc += xf.x * yf.x + xf.y * yf.y;
         }
     }
-    const int b = (int)(bt / T), t = (int)(bt % T);
-    drow[((size_t)b * H + h) * T + t] = acc;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (live && c == 0) {
+        const size_t bt = g / H;
+        const int h = (int)(g % H), b = (int)(bt / T), t = (int)(bt % T);
+        drow[((size_t)b * H + h) * T + t] = acc;
+    }
 }
 
-// 32 fp32 TMEM columns of this thread's lane -> 64 bytes of bf16 in global memory (the load runs in every lane)
-__device__ __forceinline__ void attn_store_row32(bf16 *dst, uint32_t taddr, bool live)
+// 32 fp32 TMEM columns of this thread's lane, times mul -> 64 bytes of bf16 in global memory
+// (tcgen05.ld is warp-collective: every lane runs it, only live lanes store)
+__device__ __forceinline__ void attn_store_row32(bf16 *dst, uint32_t taddr, bool live, float mul)
 {
     uint32_t v[32];
     tmem_ld32(taddr, v);
@@ -418,41 +438,25 @@ __device__ __forceinline__ void attn_store_row32(bf16 *dst, uint32_t taddr, bool
         uint32_t w[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(v[u * 8 + 2 * k]), __uint_as_float(v[u * 8 + 2 * k + 1]));
+            __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(v[u * 8 + 2 * k]) * mul, __uint_as_float(v[u * 8 + 2 * k + 1]) * mul);
             w[k] = *reinterpret_cast<uint32_t *>(&h2);
         }
         if (live) *reinterpret_cast<uint4 *>(dst + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
-// 64 fp32 TMEM columns of this thread's lane -> one 128-byte row of bf16 in global memory
-// (tcgen05.ld is warp-collective: every lane runs it, only live lanes store)
-__device__ __forceinline__ void attn_store_row64(bf16 *dst, uint32_t taddr, bool live)
+__device__ __forceinline__ void attn_store_row64(bf16 *dst, uint32_t taddr, bool live, float mul)
 {
-#pragma unroll
-    for (int c = 0; c < 2; c++) {
-        uint32_t v[32];
-        tmem_ld32(taddr + c * 32, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            uint32_t w[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(v[u * 8 + 2 * k]), __uint_as_float(v[u * 8 + 2 * k + 1]));
-                w[k] = *reinterpret_cast<uint32_t *>(&h2);
-            }
-            if (live) *reinterpret_cast<uint4 *>(dst + c * 32 + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-    }
+    attn_store_row32(dst, taddr, live, mul);
+    attn_store_row32(dst + 32, taddr + 32, live, mul);
 }
 
-__global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dkv(const __grid_constant__ AttnBwdParams p)
+__global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid_constant__ AttnBwdParams p)
 {
     extern __shared__ __align__(1024) uint8_t at_smem[];
-    uint8_t *sK = at_smem, *sV = sK + AT_TILE, *sQ = sV + AT_TILE, *sA = sQ + 2 * AT_TILE;
-    uint8_t *sPt = sA + 2 * AT_TILE, *sSt = sPt + AT_P_BYTES;
-    float *sL = reinterpret_cast<float *>(sSt + AT_P_BYTES), *sD = sL + 2 * 128;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sD + 2 * 128);
+    uint8_t *sK = at_smem, *sV = sK + AT_TILE, *sQ = sV + AT_TILE, *sA = sQ + 2 * AT_ITILE;
+    uint8_t *sPt = sA + 2 * AT_ITILE, *sSt = sPt + AT_BN * AT_BI * 2;
+    float *sL = reinterpret_cast<float *>(sSt + AT_BN * AT_BI * 2), *sD = sL + 2 * AT_BI;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sD + 2 * AT_BI);
     uint64_t *kv_full = bars, *qd_full = bars + 1, *qd_empty = bars + 3, *s_full = bars + 5, *pds_full = bars + 6,
              *acc_done = bars + 7, *spare = bars + 8;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 10);
@@ -468,29 +472,30 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dkv(const __grid
         mbar_init(smem_u32(kv_full), 1);
         for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&qd_full[i]), 2); mbar_init(smem_u32(&qd_empty[i]), 1); }
         mbar_init(smem_u32(s_full), 1);
-        mbar_init(smem_u32(pds_full), 16);
+        mbar_init(smem_u32(pds_full), 8);
         mbar_init(smem_u32(acc_done), 1);
         mbar_init(smem_u32(spare), 1);
         *abort_flag = 0;
         fence_barrier_init();
     }
-    if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), 512); tmem_relinquish(); }
+    if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), 256); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     pdl_wait();                               // barriers and TMEM above are this kernel's own; its inputs come below
     pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t tS = tmem_base, tP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 320;
+    const uint32_t tS = tmem_base, tP = tmem_base + 64, tdV = tmem_base + 128, tdK = tmem_base + 192;
 
     // key tiles that see the most queries first
     const int BK_ = p.B * p.KV, grp = p.H / p.KV;
     const int kt = (int)blockIdx.x / BK_, bk = (int)blockIdx.x % BK_;
     const int b = bk / p.KV, kvh = bk % p.KV;
     const int k0 = kt * AT_BN;
-    int qt_hi = p.nqt - 1;
-    if (p.win > 0) { int hi = (k0 + AT_BN - 1 + p.win - 1) / AT_BM; if (hi < qt_hi) qt_hi = hi; }
-    const int nq = qt_hi - kt + 1, nit = nq * grp;        // iteration it: head kvh*grp + it / nq, query tile kt + it % nq
+    const int qt_lo = k0 / AT_BI;
+    int qt_hi = (p.T - 1) / AT_BI;
+    if (p.win > 0) { int hi = (k0 + AT_BN - 1 + p.win - 1) / AT_BI; if (hi < qt_hi) qt_hi = hi; }
+    const int nq = qt_hi - qt_lo + 1, nit = nq * grp;     // iteration it: head kvh*grp + it / nq, query tile qt_lo + it % nq
 
     if (warp == 0) {
         // =============================== producer ===============================
@@ -502,22 +507,22 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dkv(const __grid
             tma_load_2d(smem_u32(sV), &p.v_map, smem_u32(kv_full), kvh * AT_HD, b * p.T + k0);
         }
         for (int it = 0; ok && it < nit; it++) {
-            const int st = it & 1, h = kvh * grp + it / nq, q0 = (kt + it % nq) * AT_BM;
+            const int st = it & 1, h = kvh * grp + it / nq, q0 = (qt_lo + it % nq) * AT_BI;
             ok = at_wait(smem_u32(&qd_empty[st]), (((uint32_t)it >> 1) & 1u) ^ 1u, abort_flag, p.errword, 201);
             if (!ok) break;
             const uint32_t bar = smem_u32(&qd_full[st]);
             if (lane == 0) {
-                mbar_expect_tx(bar, 2 * AT_TILE);
-                tma_load_2d(smem_u32(sQ + st * AT_TILE), &p.q_map, bar, h * AT_HD, b * p.T + q0);
-                tma_load_2d(smem_u32(sA + st * AT_TILE), &p.da_map, bar, h * AT_HD, b * p.T + q0);
+                mbar_expect_tx(bar, 2 * AT_ITILE);
+                tma_load_2d(smem_u32(sQ + st * AT_ITILE), &p.q_imap, bar, h * AT_HD, b * p.T + q0);
+                tma_load_2d(smem_u32(sA + st * AT_ITILE), &p.da_imap, bar, h * AT_HD, b * p.T + q0);
             }
-            // log-sum-exp (log2 domain) and D of the 128 queries; queries past the sequence get +huge, so P = 0
+            // log-sum-exp (log2 domain) and D of the 64 queries; queries past the sequence get +huge, so P = 0
             const size_t rowb = ((size_t)b * p.H + h) * p.T;
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
+            for (int k = 0; k < AT_BI / 32; k++) {
                 const int c = lane + 32 * k, qi = q0 + c;
-                sL[st * 128 + c] = qi < p.T ? p.lse[rowb + qi] * 1.4426950408889634f : 1e30f;
-                sD[st * 128 + c] = qi < p.T ? p.drow[rowb + qi] : 0.0f;
+                sL[st * AT_BI + c] = qi < p.T ? p.lse[rowb + qi] * 1.4426950408889634f : 1e30f;
+                sD[st * AT_BI + c] = qi < p.T ? p.drow[rowb + qi] : 0.0f;
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar);
@@ -530,10 +535,10 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dkv(const __grid
         }
     } else if (warp == 1) {
         // =============================== MMA issuer ===============================
-        constexpr uint32_t IDESC_S = make_idesc(AT_BN, AT_BM, 0, 0);
+        constexpr uint32_t IDESC_S = make_idesc(AT_BN, AT_BI, 0, 0);
         constexpr uint32_t IDESC_ACC = make_idesc(AT_BN, AT_HD, 0, 1);
         auto issue_scores = [&](int st) {      // S^T = K Q^T, dP^T = V dA^T
-            const uint32_t k_ = smem_u32(sK), v_ = smem_u32(sV), q_ = smem_u32(sQ + st * AT_TILE), a_ = smem_u32(sA + st * AT_TILE);
+            const uint32_t k_ = smem_u32(sK), v_ = smem_u32(sV), q_ = smem_u32(sQ + st * AT_ITILE), a_ = smem_u32(sA + st * AT_ITILE);
 #pragma unroll
             for (int k16 = 0; k16 < AT_HD / 16; k16++)
                 tc_mma_bf16(tS, make_desc(k_ + k16 * 32, 16, 1024), make_desc(q_ + k16 * 32, 16, 1024), IDESC_S, k16 > 0);
@@ -546,7 +551,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dkv(const __grid
         if (ok) ok = at_wait(smem_u32(&qd_full[0]), 0, abort_flag, p.errword, 211);
         if (ok) {
             tc_fence_after();
-            if (lane == 0) issue_scores(0);
+            if (elect_one()) issue_scores(0);
             __syncwarp();
         }
         for (int it = 0; ok && it < nit; it++) {
@@ -560,18 +565,18 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dkv(const __grid
                 ok = at_wait(smem_u32(&qd_full[st ^ 1]), ((uint32_t)(it + 1) >> 1) & 1u, abort_flag, p.errword, 213);
                 if (!ok) break;
                 tc_fence_after();
-                if (lane == 0) issue_scores(st ^ 1);
+                if (elect_one()) issue_scores(st ^ 1);
                 __syncwarp();
             }
-            if (lane == 0) {
-                const uint32_t pt = smem_u32(sPt), dst = smem_u32(sSt), q_ = smem_u32(sQ + st * AT_TILE), a_ = smem_u32(sA + st * AT_TILE);
+            if (elect_one()) {
+                const uint32_t pt = smem_u32(sPt), dst = smem_u32(sSt), q_ = smem_u32(sQ + st * AT_ITILE), a_ = smem_u32(sA + st * AT_ITILE);
 #pragma unroll
-                for (int kk = 0; kk < AT_BM / 16; kk++)       // dV += P^T dA
-                    tc_mma_bf16(tdV, make_desc(pt + (kk >> 2) * (AT_BN * 128) + (kk & 3) * 32, 16, 1024),
+                for (int kk = 0; kk < AT_BI / 16; kk++)       // dV += P^T dA
+                    tc_mma_bf16(tdV, make_desc(pt + kk * 32, 16, 1024),
                                 make_desc(a_ + kk * 2048, 8192, 1024), IDESC_ACC, (it > 0 || kk > 0) ? 1u : 0u);
 #pragma unroll
-                for (int kk = 0; kk < AT_BM / 16; kk++)       // dK += dS^T Q
-                    tc_mma_bf16(tdK, make_desc(dst + (kk >> 2) * (AT_BN * 128) + (kk & 3) * 32, 16, 1024),
+                for (int kk = 0; kk < AT_BI / 16; kk++)       // dK += dS^T Q
+                    tc_mma_bf16(tdK, make_desc(dst + kk * 32, 16, 1024),
                                 make_desc(q_ + kk * 2048, 8192, 1024), IDESC_ACC, (it > 0 || kk > 0) ? 1u : 0u);
                 tc_commit(smem_u32(acc_done));
                 tc_commit(smem_u32(&qd_empty[st]));
@@ -579,49 +584,62 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dkv(const __grid
             __syncwarp();
         }
         if (*abort_flag) {
-            if (lane == 0) tc_commit(smem_u32(spare));
+            if (elect_one()) tc_commit(smem_u32(spare));
             __syncwarp();
             for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(spare), 0); i++) {}
         }
     } else {
         // =============================== element-wise ===============================
-        // warp = (TMEM lane quarter qr, 32-column chunk cq of the 128): hf = which 64-column sub-tile, c = chunk in it
-        const int qr = warp & 3, cq = (warp - 2) >> 2, hf = cq >> 1, c = cq & 1, r = qr * 32 + lane, key = k0 + r;
+        // warp = (TMEM lane quarter qr, 32-column chunk c of the 64)
+        const int qr = warp & 3, c = (warp - 2) >> 2, r = qr * 32 + lane, key = k0 + r;
         const uint32_t lane_base = (uint32_t)(qr * 32) << 16;
         bool ok = true;
         for (int it = 0; ok && it < nit; it++) {
-            const int st = it & 1, q0 = (kt + it % nq) * AT_BM;
+            const int st = it & 1, q0 = (qt_lo + it % nq) * AT_BI;
             const bool masked = (q0 < k0 + AT_BN - 1) || p.win > 0;
             ok = at_wait(smem_u32(&qd_full[st]), ((uint32_t)it >> 1) & 1u, abort_flag, p.errword, 220);      // lse / D in shared memory
             if (ok) ok = at_wait(smem_u32(s_full), (uint32_t)it & 1u, abort_flag, p.errword, 221);
             if (!ok) break;
             tc_fence_after();
-            const float *L2 = sL + st * 128 + hf * 64, *Dq = sD + st * 128 + hf * 64;
+            const float *L2 = sL + st * AT_BI + c * 32, *Dq = sD + st * AT_BI + c * 32;
             uint32_t sv[32], dv[32];                 // both TMEM loads of the step in flight: one round trip
-            tmem_ld32(tS + lane_base + cq * 32, sv);
-            tmem_ld32(tP + lane_base + cq * 32, dv);
+            tmem_ld32(tS + lane_base + c * 32, sv);
+            tmem_ld32(tP + lane_base + c * 32, dv);
             tmem_ld_wait();
             {
                 uint32_t pp[16], ds[16];
+                // MODE 0: every query sees the key; 1: causal edge, queries from j = lo on; 2: window, j below hi as well
+                auto compute = [&](auto mode, int lo, int hi) {
+                    constexpr int MODE = decltype(mode)::value;
 #pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    float pv[2], dsv[2];
+                    for (int j = 0; j < 32; j += 4) {
+                        const float4 l4 = *reinterpret_cast<const float4 *>(L2 + j), d4 = *reinterpret_cast<const float4 *>(Dq + j);
+                        const float ll[4] = {l4.x, l4.y, l4.z, l4.w}, dd[4] = {d4.x, d4.y, d4.z, d4.w};
+                        float pv[4], dsv[4];
 #pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const int col = c * 32 + j + e, qi = q0 + hf * 64 + col;
-                        float pe = ex2(__uint_as_float(sv[j + e]) * p.scale_log2 - L2[col]);
-                        if (masked && !(key <= qi && (p.win <= 0 || key > qi - p.win))) pe = 0.0f;
-                        pv[e] = pe;
-                        dsv[e] = pe * (__uint_as_float(dv[j + e]) - Dq[col]) * p.scale;
+                        for (int e = 0; e < 4; e++) {
+                            float pe = ex2(__uint_as_float(sv[j + e]) * p.scale_log2 - ll[e]);
+                            if (MODE == 1) pe = j + e >= lo ? pe : 0.0f;
+                            if (MODE == 2) pe = j + e >= lo && j + e < hi ? pe : 0.0f;
+                            pv[e] = pe;
+                            dsv[e] = pe * (__uint_as_float(dv[j + e]) - dd[e]);
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; e += 2) {
+                            __nv_bfloat162 h2 = __floats2bfloat162_rn(pv[e], pv[e + 1]);
+                            pp[(j + e) >> 1] = *reinterpret_cast<uint32_t *>(&h2);
+                            h2 = __floats2bfloat162_rn(dsv[e], dsv[e + 1]);
+                            ds[(j + e) >> 1] = *reinterpret_cast<uint32_t *>(&h2);
+                        }
                     }
-                    __nv_bfloat162 h2 = __floats2bfloat162_rn(pv[0], pv[1]);
-                    pp[j >> 1] = *reinterpret_cast<uint32_t *>(&h2);
-                    h2 = __floats2bfloat162_rn(dsv[0], dsv[1]);
-                    ds[j >> 1] = *reinterpret_cast<uint32_t *>(&h2);
-                }
+                };
+                const int lo = key - q0 - c * 32;         // query q0 + 32 c + j sees the key from j = lo on
+                if (!masked) compute(AtMode<0>(), 0, 0);
+                else if (p.win <= 0) compute(AtMode<1>(), lo, 0);
+                else compute(AtMode<2>(), lo, lo + p.win);
                 // the previous step's products must have read the P / dS tiles before they are overwritten
                 if (it > 0) ok = at_wait(smem_u32(acc_done), (uint32_t)(it - 1) & 1u, abort_flag, p.errword, 222);
-                uint8_t *prow = sPt + hf * (AT_BN * 128) + r * 128, *srow = sSt + hf * (AT_BN * 128) + r * 128;
+                uint8_t *prow = sPt + r * 128, *srow = sSt + r * 128;
                 if (ok) {
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
@@ -640,21 +658,21 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dkv(const __grid
         if (ok) ok = at_wait(smem_u32(acc_done), (uint32_t)(nit - 1) & 1u, abort_flag, p.errword, 223);
         if (ok) {
             tc_fence_after();
-            // chunks 0, 1: the two halves of the dV row; chunks 2, 3: of the dK row
-            bf16 *dst = (hf ? p.dK : p.dV) + ((size_t)b * p.T + key) * ((size_t)p.KV * AT_HD) + (size_t)kvh * AT_HD + c * 32;
-            attn_store_row32(dst, (hf ? tdK : tdV) + lane_base + c * 32, key < p.T);
+            // chunk 0: the dV row; chunk 1: the dK row
+            bf16 *dst = (c ? p.dK : p.dV) + ((size_t)b * p.T + key) * ((size_t)p.KV * AT_HD) + (size_t)kvh * AT_HD;
+            attn_store_row64(dst, (c ? tdK : tdV) + lane_base, key < p.T, c ? p.scale : 1.0f);
         }
         tc_fence_before();
     }
     __syncthreads();
-    if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+    if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
 }
 
-__global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dq(const __grid_constant__ AttnBwdParams p)
+__global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_constant__ AttnBwdParams p)
 {
     extern __shared__ __align__(1024) uint8_t at_smem[];
-    uint8_t *sQ = at_smem, *sA = sQ + AT_TILE, *sK = sA + AT_TILE, *sV = sK + 2 * AT_TILE, *sS = sV + 2 * AT_TILE;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sS + AT_P_BYTES);
+    uint8_t *sQ = at_smem, *sA = sQ + AT_TILE, *sK = sA + AT_TILE, *sV = sK + 2 * AT_ITILE, *sS = sV + 2 * AT_ITILE;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sS + AT_BM * AT_BI * 2);
     uint64_t *qa_full = bars, *kv_full = bars + 1, *kv_empty = bars + 3, *s_full = bars + 5, *ds_full = bars + 6,
              *acc_done = bars + 7, *spare = bars + 8;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 10);
@@ -670,28 +688,28 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dq(const __grid_
         mbar_init(smem_u32(qa_full), 1);
         for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&kv_full[i]), 1); mbar_init(smem_u32(&kv_empty[i]), 1); }
         mbar_init(smem_u32(s_full), 1);
-        mbar_init(smem_u32(ds_full), 16);
+        mbar_init(smem_u32(ds_full), 8);
         mbar_init(smem_u32(acc_done), 1);
         mbar_init(smem_u32(spare), 1);
         *abort_flag = 0;
         fence_barrier_init();
     }
-    if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), 512); tmem_relinquish(); }
+    if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), 256); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     pdl_wait();                               // barriers and TMEM above are this kernel's own; its inputs come below
     pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t tS = tmem_base, tP = tmem_base + 128, tdQ = tmem_base + 256;
+    const uint32_t tS = tmem_base, tP = tmem_base + 64, tdQ = tmem_base + 128;
 
     const int BH = p.B * p.H;
     const int qt = p.nqt - 1 - (int)blockIdx.x / BH, bh = (int)blockIdx.x % BH;
     const int b = bh / p.H, h = bh % p.H, kvh = h / (p.H / p.KV);
     const int q0 = qt * AT_BM;
     int kt_lo = 0;
-    if (p.win > 0) { int lo = q0 - p.win + 1; kt_lo = lo > 0 ? lo / AT_BN : 0; }
-    const int kt_hi = (q0 + AT_BM - 1 < p.T ? q0 + AT_BM - 1 : p.T - 1) / AT_BN;
+    if (p.win > 0) { int lo = q0 - p.win + 1; kt_lo = lo > 0 ? lo / AT_BI : 0; }
+    const int kt_hi = (q0 + AT_BM - 1 < p.T ? q0 + AT_BM - 1 : p.T - 1) / AT_BI;
     const int nt = kt_hi - kt_lo + 1;
 
     if (warp == 0) {
@@ -708,10 +726,10 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dq(const __grid_
             if (!ok) break;
             if (lane == 0) {
                 const uint32_t bar = smem_u32(&kv_full[st]);
-                const int row = b * p.T + (kt_lo + t) * AT_BN;
-                mbar_expect_tx(bar, 2 * AT_TILE);
-                tma_load_2d(smem_u32(sK + st * AT_TILE), &p.k_map, bar, kvh * AT_HD, row);
-                tma_load_2d(smem_u32(sV + st * AT_TILE), &p.v_map, bar, kvh * AT_HD, row);
+                const int row = b * p.T + (kt_lo + t) * AT_BI;
+                mbar_expect_tx(bar, 2 * AT_ITILE);
+                tma_load_2d(smem_u32(sK + st * AT_ITILE), &p.k_imap, bar, kvh * AT_HD, row);
+                tma_load_2d(smem_u32(sV + st * AT_ITILE), &p.v_imap, bar, kvh * AT_HD, row);
             }
             __syncwarp();
             issued = t + 1;
@@ -722,10 +740,10 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dq(const __grid_
                 for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(&kv_full[t & 1]), ((uint32_t)t >> 1) & 1u); i++) {}
         }
     } else if (warp == 1) {
-        constexpr uint32_t IDESC_S = make_idesc(AT_BM, AT_BN, 0, 0);
+        constexpr uint32_t IDESC_S = make_idesc(AT_BM, AT_BI, 0, 0);
         constexpr uint32_t IDESC_ACC = make_idesc(AT_BM, AT_HD, 0, 1);
         auto issue_scores = [&](int st) {      // S = Q K^T, dP = dA V^T
-            const uint32_t q_ = smem_u32(sQ), a_ = smem_u32(sA), k_ = smem_u32(sK + st * AT_TILE), v_ = smem_u32(sV + st * AT_TILE);
+            const uint32_t q_ = smem_u32(sQ), a_ = smem_u32(sA), k_ = smem_u32(sK + st * AT_ITILE), v_ = smem_u32(sV + st * AT_ITILE);
 #pragma unroll
             for (int k16 = 0; k16 < AT_HD / 16; k16++)
                 tc_mma_bf16(tS, make_desc(q_ + k16 * 32, 16, 1024), make_desc(k_ + k16 * 32, 16, 1024), IDESC_S, k16 > 0);
@@ -738,7 +756,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dq(const __grid_
         if (ok) ok = at_wait(smem_u32(&kv_full[0]), 0, abort_flag, p.errword, 311);
         if (ok) {
             tc_fence_after();
-            if (lane == 0) issue_scores(0);
+            if (elect_one()) issue_scores(0);
             __syncwarp();
         }
         for (int t = 0; ok && t < nt; t++) {
@@ -750,14 +768,14 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dq(const __grid_
                 ok = at_wait(smem_u32(&kv_full[st ^ 1]), ((uint32_t)(t + 1) >> 1) & 1u, abort_flag, p.errword, 313);
                 if (!ok) break;
                 tc_fence_after();
-                if (lane == 0) issue_scores(st ^ 1);
+                if (elect_one()) issue_scores(st ^ 1);
                 __syncwarp();
             }
-            if (lane == 0) {
-                const uint32_t s_ = smem_u32(sS), k_ = smem_u32(sK + st * AT_TILE);
+            if (elect_one()) {
+                const uint32_t s_ = smem_u32(sS), k_ = smem_u32(sK + st * AT_ITILE);
 #pragma unroll
-                for (int kk = 0; kk < AT_BN / 16; kk++)       // dQ += dS K
-                    tc_mma_bf16(tdQ, make_desc(s_ + (kk >> 2) * (AT_BM * 128) + (kk & 3) * 32, 16, 1024),
+                for (int kk = 0; kk < AT_BI / 16; kk++)       // dQ += dS K
+                    tc_mma_bf16(tdQ, make_desc(s_ + kk * 32, 16, 1024),
                                 make_desc(k_ + kk * 2048, 8192, 1024), IDESC_ACC, (t > 0 || kk > 0) ? 1u : 0u);
                 tc_commit(smem_u32(acc_done));
                 tc_commit(smem_u32(&kv_empty[st]));
@@ -765,44 +783,51 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dq(const __grid_
             __syncwarp();
         }
         if (*abort_flag) {
-            if (lane == 0) tc_commit(smem_u32(spare));
+            if (elect_one()) tc_commit(smem_u32(spare));
             __syncwarp();
             for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(spare), 0); i++) {}
         }
     } else {
-        const int qr = warp & 3, cq = (warp - 2) >> 2, hf = cq >> 1, c = cq & 1, r = qr * 32 + lane, i = q0 + r;
+        const int qr = warp & 3, c = (warp - 2) >> 2, r = qr * 32 + lane, i = q0 + r;
         const uint32_t lane_base = (uint32_t)(qr * 32) << 16;
         const size_t rowb = ((size_t)b * p.H + h) * p.T;
         const float L2 = i < p.T ? p.lse[rowb + i] * 1.4426950408889634f : 1e30f;
         const float Dq = i < p.T ? p.drow[rowb + i] : 0.0f;
         bool ok = true;
         for (int t = 0; ok && t < nt; t++) {
-            const int k0 = (kt_lo + t) * AT_BN;
-            const bool masked = (k0 + AT_BN - 1 > q0) || p.win > 0 || (k0 + AT_BN > p.T);
+            const int k0 = (kt_lo + t) * AT_BI;
+            const bool masked = (k0 + AT_BI - 1 > q0) || p.win > 0 || (k0 + AT_BI > p.T);
             ok = at_wait(smem_u32(s_full), (uint32_t)t & 1u, abort_flag, p.errword, 321);
             if (!ok) break;
             tc_fence_after();
             uint32_t sv[32], dv[32];                 // both TMEM loads of the step in flight: one round trip
-            tmem_ld32(tS + lane_base + cq * 32, sv);
-            tmem_ld32(tP + lane_base + cq * 32, dv);
+            tmem_ld32(tS + lane_base + c * 32, sv);
+            tmem_ld32(tP + lane_base + c * 32, dv);
             tmem_ld_wait();
             {
                 uint32_t ds[16];
+                auto compute = [&](auto mode, int lo, int hi) {       // keys lo < j <= hi of the thread's 32 (see k_attn_bwd_dkv)
+                    constexpr int MODE = decltype(mode)::value;
 #pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    float dsv[2];
+                    for (int j = 0; j < 32; j += 2) {
+                        float dsv[2];
 #pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const int key = k0 + hf * 64 + c * 32 + j + e;
-                        float pe = ex2(__uint_as_float(sv[j + e]) * p.scale_log2 - L2);
-                        if (masked && !attn_valid(key, i, p.T, p.win)) pe = 0.0f;
-                        dsv[e] = pe * (__uint_as_float(dv[j + e]) - Dq) * p.scale;
+                        for (int e = 0; e < 2; e++) {
+                            float pe = ex2(__uint_as_float(sv[j + e]) * p.scale_log2 - L2);
+                            if (MODE == 1) pe = j + e <= hi ? pe : 0.0f;
+                            if (MODE == 2) pe = j + e <= hi && j + e > lo ? pe : 0.0f;
+                            dsv[e] = pe * (__uint_as_float(dv[j + e]) - Dq);
+                        }
+                        __nv_bfloat162 h2 = __floats2bfloat162_rn(dsv[0], dsv[1]);
+                        ds[j >> 1] = *reinterpret_cast<uint32_t *>(&h2);
                     }
-                    __nv_bfloat162 h2 = __floats2bfloat162_rn(dsv[0], dsv[1]);
-                    ds[j >> 1] = *reinterpret_cast<uint32_t *>(&h2);
-                }
+                };
+                const int base = k0 + c * 32, hi = (i < p.T ? i : p.T - 1) - base;
+                if (!masked) compute(AtMode<0>(), 0, 0);
+                else if (p.win <= 0) compute(AtMode<1>(), 0, hi);
+                else compute(AtMode<2>(), i - p.win - base, hi);
                 if (t > 0) ok = at_wait(smem_u32(acc_done), (uint32_t)(t - 1) & 1u, abort_flag, p.errword, 322);   // dS tile free again
-                uint8_t *srow = sS + hf * (AT_BM * 128) + r * 128;
+                uint8_t *srow = sS + r * 128;
                 if (ok) {
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
@@ -820,27 +845,13 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 1) k_attn_bwd_dq(const __grid_
         if (ok) ok = at_wait(smem_u32(acc_done), (uint32_t)(nt - 1) & 1u, abort_flag, p.errword, 323);
         if (ok) {
             tc_fence_after();
-            {                                  // each of the row's four threads stores 16 of its 64 columns
-                bf16 *dst = p.dQ + ((size_t)b * p.T + i) * ((size_t)p.H * AT_HD) + (size_t)h * AT_HD + cq * 16;
-                uint32_t v[16];
-                tmem_ld16(tdQ + lane_base + cq * 16, v);          // warp-collective: all lanes, also those past the sequence
-                tmem_ld_wait();
-#pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(v[u * 8 + 2 * k]), __uint_as_float(v[u * 8 + 2 * k + 1]));
-                        w[k] = *reinterpret_cast<uint32_t *>(&h2);
-                    }
-                    if (i < p.T) *reinterpret_cast<uint4 *>(dst + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-                }
-            }
+            // each of the row's two threads stores half of it
+            attn_store_row32(p.dQ + ((size_t)b * p.T + i) * ((size_t)p.H * AT_HD) + (size_t)h * AT_HD + c * 32, tdQ + lane_base + c * 32, i < p.T, p.scale);
         }
         tc_fence_before();
     }
     __syncthreads();
-    if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+    if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
 }
 
 }  // namespace qlmb
@@ -891,14 +902,13 @@ extern "C" int qlmb_attn_bwd(void *dQ, void *dK, void *dV, float *drow, const vo
     AttnBwdParams p;
     memset(&p, 0, sizeof p);
     const unsigned long long rows = (unsigned long long)B * T, qw = (unsigned long long)H * hd, kw = (unsigned long long)KV * hd;
-    int rc = make_map(&p.q_map, Q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, qw, rows, qw * 2, AT_HD, AT_BM, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) return rc;
-    rc = make_map(&p.da_map, dA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, qw, rows, qw * 2, AT_HD, AT_BM, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) return rc;
-    rc = make_map(&p.k_map, K, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, kw, rows, kw * 2, AT_HD, AT_BN, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) return rc;
-    rc = make_map(&p.v_map, V, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, kw, rows, kw * 2, AT_HD, AT_BN, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) return rc;
+    struct { CUtensorMap *m; const void *base; unsigned long long width; unsigned box; } maps[8] = {
+        {&p.q_map, Q, qw, AT_BM}, {&p.da_map, dA, qw, AT_BM}, {&p.k_map, K, kw, AT_BN}, {&p.v_map, V, kw, AT_BN},
+        {&p.q_imap, Q, qw, AT_BI}, {&p.da_imap, dA, qw, AT_BI}, {&p.k_imap, K, kw, AT_BI}, {&p.v_imap, V, kw, AT_BI}};
+    for (auto &m : maps) {
+        const int rc = make_map(m.m, m.base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, m.width, rows, m.width * 2, AT_HD, m.box, CU_TENSOR_MAP_SWIZZLE_128B);
+        if (rc) return rc;
+    }
     p.lse = lse; p.drow = drow;
     p.dQ = (bf16 *)dQ; p.dK = (bf16 *)dK; p.dV = (bf16 *)dV;
     p.B = B; p.T = T; p.H = H; p.KV = KV; p.win = win;
@@ -918,7 +928,7 @@ extern "C" int qlmb_attn_bwd(void *dQ, void *dK, void *dV, float *drow, const vo
     }
     cudaStream_t st = as_stream(stream);
     const size_t nrow = (size_t)B * T * H;
-    QLMB_CUDA(pdl_launch_small(k_attn_drow, dim3((unsigned)((nrow + 255) / 256)), dim3(256), 0, st, drow, (const bf16 *)dA, (const bf16 *)O, B, T, H));
+    QLMB_CUDA(pdl_launch_small(k_attn_drow, dim3((unsigned)((nrow + 31) / 32)), dim3(256), 0, st, drow, (const bf16 *)dA, (const bf16 *)O, B, T, H));
     QLMB_CUDA(pdl_launch_small(k_attn_bwd_dkv, dim3((unsigned)(p.nqt * B * KV)), dim3(AT_BWD_THREADS), AT_DKV_SMEM, st, p));
     QLMB_CUDA(pdl_launch_small(k_attn_bwd_dq, dim3((unsigned)(p.nqt * B * H)), dim3(AT_BWD_THREADS), AT_DQ_SMEM, st, p));
     QLMB_LAUNCH_CHECK("k_attn_bwd");

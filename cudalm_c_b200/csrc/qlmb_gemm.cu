@@ -666,7 +666,7 @@ k_gemm(const __grid_constant__ GemmParams p)
                         if (!ok) break;
                     }
                     tc_fence_after();
-                    if (lane == 0) {
+                    if (elect_one()) {
                         const uint32_t a0 = smem_u32(sA + ra.idx * A_STAGE_BYTES);
                         const uint32_t b0 = smem_u32(sB + sb * B_STAGE_BYTES);
 #pragma unroll
@@ -690,12 +690,12 @@ k_gemm(const __grid_constant__ GemmParams p)
                 }
             }
             if (ok) {
-                if (lane == 0) tc_commit(smem_u32(&tmem_full[acc]));
+                if (elect_one()) tc_commit(smem_u32(&tmem_full[acc]));
                 __syncwarp();
             }
         }
         if (*abort_flag) {   // aborting: let issued MMAs retire (bounded) before TMEM is released
-            if (lane == 0) tc_commit(smem_u32(spare));
+            if (elect_one()) tc_commit(smem_u32(spare));
             __syncwarp();
             for (uint32_t i = 0; i < WAIT_LIMIT && !mbar_try(smem_u32(spare), 0); i++) {}
         }

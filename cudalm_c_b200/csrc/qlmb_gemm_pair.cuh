@@ -276,7 +276,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                         ok = mbar_wait_cluster(smem_u32(&full[rs.idx]), rs.phase, abort_flag, p.errword, 14);
                         if (!ok) break;
                         tc_fence_after();
-                        if (lane == 0) {
+                        if (elect_one()) {
                             const uint32_t a0 = smem_u32(sA + rs.idx * P_A_STAGE);
                             const uint32_t b0 = smem_u32(sB + rs.idx * P_B_STAGE);
 #pragma unroll
@@ -295,12 +295,12 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                     }
                 }
                 if (ok) {
-                    if (lane == 0) tc_commit2_both(smem_u32(&tmem_full[acc]));
+                    if (elect_one()) tc_commit2_both(smem_u32(&tmem_full[acc]));
                     __syncwarp();
                 }
             }
             if (*abort_flag) {
-                if (lane == 0) tc_commit2(smem_u32(spare));
+                if (elect_one()) tc_commit2(smem_u32(spare));
                 __syncwarp();
                 for (uint32_t i = 0; i < WAIT_LIMIT && !mbar_try(smem_u32(spare), 0); i++) {}
             }

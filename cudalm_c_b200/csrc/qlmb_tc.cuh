@@ -114,6 +114,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t v[16])
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// One lane of a converged warp, as a predicate that the compiler knows to hold for a single thread: the operands of what it
+// guards stay in uniform registers (with `lane == 0` each tcgen05.mma took about 120 cycles to issue).  The same lane every time.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 // Shared-memory matrix descriptor, 128-byte swizzle (Blackwell descriptor version 1).
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes)
 {
