@@ -79,6 +79,7 @@ CALL(step, 29, ARG_P(0); ARG_P(1); ARG_P(2); ARG_P(3); ARG_P(4); ARG_P(5); ARG_P
      ARG_F(13); ARG_F(14); ARG_F(15); ARG_F(16); ARG_F(17); ARG_P(18); ARG_F(19); ARG_F(20); ARG_I(21); ARG_U(22);
      ARG_I(23); ARG_P(24); ARG_I(25); ARG_I(26); ARG_I(27); ARG_P(28),
      p0, p1, p2, p3, p4, p5, p6, p7, p8, p9, i10, i11, i12, f13, f14, f15, f16, f17, p18, f19, f20, i21, u22, i23, p24, i25, i26, i27, p28)
+CALL(gnorm, 8, ARG_P(0); ARG_U(1); ARG_P(2); ARG_P(3); ARG_I(4); ARG_I(5); ARG_P(6); ARG_P(7), p0, (size_t)u1, p2, p3, i4, i5, p6, p7)
 CALL(dec_step, 2, ARG_P(0); ARG_P(1), p0, p1)
 CALL(dec_greedy, 6, ARG_P(0); ARG_P(1); ARG_P(2); ARG_I(3); ARG_I(4); ARG_P(5), p0, p1, p2, i3, i4, p5)
 
@@ -94,7 +95,7 @@ static PyObject *set_error_class(PyObject *self, PyObject *cls)
 static PyMethodDef methods[] = {
     ENTRY(gemv_decode), ENTRY(linear_fwd), ENTRY(linear_dgrad), ENTRY(linear_wgrad), ENTRY(gemm_nt), ENTRY(embed), ENTRY(rmsnorm_fwd),
     ENTRY(rmsnorm_bwd), ENTRY(rope), ENTRY(attn_fwd), ENTRY(attn_bwd), ENTRY(moe_forward), ENTRY(moe_decode), ENTRY(moe_backward), ENTRY(adamw),
-    ENTRY(step), ENTRY(dec_step), ENTRY(dec_greedy),
+    ENTRY(step), ENTRY(gnorm), ENTRY(dec_step), ENTRY(dec_greedy),
     {"set_error_class", set_error_class, METH_O, NULL},
     {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_pycalls", NULL, -1, methods, NULL, NULL, NULL, NULL};

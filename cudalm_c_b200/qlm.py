@@ -50,11 +50,11 @@ def qlm_servo(d, r, s, spans_dev, nspan, group, dmax, f_hi, f_lo, packed=1):
 def gnorm(G, sides=(), clip_side=0, out=None):
     """gs[0] = clip multiplier, gs[1] = norm (k_sqsum + k_gnorm, cudalm.cu:6442-6444)."""
     gs = out if out is not None else torch.empty(2, dtype=torch.float32, device=G.device)
-    ns = len(sides)
-    ptrs = (C.c_void_p * max(ns, 1))(*[x.data_ptr() for x in sides])
-    lens = (C.c_size_t * max(ns, 1))(*[x.numel() for x in sides])
-    check(lib().qlmb_gnorm(ptr(G), G.numel(), C.cast(ptrs, C.c_void_p), C.cast(lens, C.c_void_p), ns, clip_side,
-                           ptr(gs), stream_ptr()))
+    ns, ptrs, lens = len(sides), None, None
+    if ns:
+        ptrs = (C.c_void_p * ns)(*[x.data_ptr() for x in sides])
+        lens = (C.c_size_t * ns)(*[x.numel() for x in sides])
+    calls.gnorm(G, G.numel(), ptrs and C.addressof(ptrs), lens and C.addressof(lens), ns, clip_side, gs, stream_ptr())
     return gs
 
 

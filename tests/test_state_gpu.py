@@ -118,6 +118,39 @@ def test_fast_step_matches_oracle(cuda, oracle, with_p, use_gsp):
             assert (P.cpu().numpy() == Ph).all()
 
 
+@pytest.mark.parametrize("sizes", [(128 * 40, 128 * 33), (128 * 40 + 2, 128 * 33 + 4, 128 * 21, 128 * 9 + 6, 128 * 5, 128 * 7 + 126, 128 * 6),
+                                   (130, 128, 126, 2, 256)])
+def test_step_of_spans_at_any_even_element_matches_oracle(cuda, oracle, sizes):
+    """Spans whose groups start at every even offset, gradients with zeros, values whose squares vanish and large ones."""
+    rng = np.random.default_rng(11)
+    st = DevState(cuda, list(sizes), 128, 7, 1)
+    P0 = (rng.standard_normal(st.nq) * 0.02).astype(f32)
+    st.encode(dev(P0, cuda))
+    h = st.host()
+    d, r, s = h["d"].copy(), h["r"].copy(), h["s"].copy()
+    for i in range(len(st.sp)):
+        g0 = int(st.sp[i]["gi0"]); st.sp[i]["sref"] = f32(s[g0:g0 + int(st.sp[i]["ngrp"])].astype(np.float64).mean())
+    st.push_spans()
+    m8 = np.zeros(st.nq, np.int8); v8 = np.zeros(st.nq, np.uint8)
+    m8s = np.zeros(st.ng, f32); v8s = np.zeros(st.ng, f32)
+    Ph = np.zeros(st.nq, f32)
+    P = torch.zeros(st.nq, device=cuda)
+    for t in range(1, 6):
+        G = (rng.standard_normal(st.nq) * 1e-3).astype(f32)
+        for v in (0.0, 1e-21, -1e-25, 30.0):
+            G[rng.integers(0, st.nq, st.nq // 40 + 1)] = v
+        if t == 3:
+            G[:128 * 2] = 0.0
+        st.step(P, dev(G, cuda), t)
+        bc1 = f32(1) - f32(np.power(f32(0.9), f32(t))); bc2 = f32(1) - f32(np.power(f32(0.95), f32(t)))
+        oracle.step(Ph, G, d, r, s, m8, m8s, v8, v8s, st.sp, lr=3e-4, b1=0.9, b2=0.95, wd=0.1, gscale=1.0,
+                    inv_bc1=float(f32(1) / bc1), inv_sqrt_bc2=float(f32(1) / np.sqrt(bc2)), t=t)
+        h = st.host()
+        for k, v in dict(d=d, r=r, m8=m8, v8=v8, m8s=m8s, v8s=v8s).items():
+            assert (h[k] == v).all(), (k, t, int((h[k] != v).sum()))
+        assert (P.cpu().numpy() == Ph).all()
+
+
 def test_step_sharded_equals_whole(cuda):
     """ZeRO-1 style split: stepping group ranges separately gives the same bytes."""
     rng = np.random.default_rng(6)
