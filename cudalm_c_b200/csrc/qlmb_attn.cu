@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
         // =============================== TMA producer ===============================
         bool ok = true;
         int issued = 0;
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_expect_tx(smem_u32(q_full), AT_TILE);
             tma_load_2d(smem_u32(sQ), &p.q_map, smem_u32(q_full), h * AT_HD, b * p.T + q0);
         }
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
             const int st = t & 1;
             ok = at_wait(smem_u32(&kv_empty[st]), (((uint32_t)t >> 1) & 1u) ^ 1u, abort_flag, p.errword, 101);
             if (!ok) break;
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t bar = smem_u32(&kv_full[st]);
                 const int row = b * p.T + (kt_lo + t) * AT_BN;
                 mbar_expect_tx(bar, 2 * AT_TILE);
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
         // =============================== producer ===============================
         bool ok = true;
         int issued = 0;
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_expect_tx(smem_u32(kv_full), 2 * AT_TILE);
             tma_load_2d(smem_u32(sK), &p.k_map, smem_u32(kv_full), kvh * AT_HD, b * p.T + k0);
             tma_load_2d(smem_u32(sV), &p.v_map, smem_u32(kv_full), kvh * AT_HD, b * p.T + k0);
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
             ok = at_wait(smem_u32(&qd_empty[st]), (((uint32_t)it >> 1) & 1u) ^ 1u, abort_flag, p.errword, 201);
             if (!ok) break;
             const uint32_t bar = smem_u32(&qd_full[st]);
-            if (lane == 0) {
+            if (elect_one()) {
                 mbar_expect_tx(bar, 2 * AT_ITILE);
                 tma_load_2d(smem_u32(sQ + st * AT_ITILE), &p.q_imap, bar, h * AT_HD, b * p.T + q0);
                 tma_load_2d(smem_u32(sA + st * AT_ITILE), &p.da_imap, bar, h * AT_HD, b * p.T + q0);
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
     if (warp == 0) {
         bool ok = true;
         int issued = 0;
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_expect_tx(smem_u32(qa_full), 2 * AT_TILE);
             tma_load_2d(smem_u32(sQ), &p.q_map, smem_u32(qa_full), h * AT_HD, b * p.T + q0);
             tma_load_2d(smem_u32(sA), &p.da_map, smem_u32(qa_full), h * AT_HD, b * p.T + q0);
@@ -724,7 +724,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
             const int st = t & 1;
             ok = at_wait(smem_u32(&kv_empty[st]), (((uint32_t)t >> 1) & 1u) ^ 1u, abort_flag, p.errword, 301);
             if (!ok) break;
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t bar = smem_u32(&kv_full[st]);
                 const int row = b * p.T + (kt_lo + t) * AT_BI;
                 mbar_expect_tx(bar, 2 * AT_ITILE);

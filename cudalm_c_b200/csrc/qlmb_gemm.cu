@@ -205,16 +205,16 @@ __device__ __forceinline__ void blk_store_scattered(uint8_t *blk, int lane, bf16
     __syncwarp();
 }
 // The block layout is the 128-byte swizzle of a bulk tensor copy, so a staged block can leave as
-// one asynchronous store issued by lane 0.  blk_reuse() must precede the next write to the block.
+// one asynchronous store issued by the elected lane.  blk_reuse() must precede the next write to the block.
 __device__ __forceinline__ void blk_store_bulk(uint8_t *blk, int lane, const CUtensorMap *map, int x, int y)
 {
     fence_proxy_async();
     __syncwarp();
-    if (lane == 0) { tma_store_2d(map, smem_u32(blk), x, y); bulk_commit(); }
+    if (elect_one()) { tma_store_2d(map, smem_u32(blk), x, y); bulk_commit(); }
 }
 __device__ __forceinline__ void blk_reuse(int lane)
 {
-    if (lane == 0) bulk_wait_read();
+    if (elect_one()) bulk_wait_read();
     __syncwarp();
 }
 // staging bytes per epilogue warp
@@ -313,7 +313,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams &p, uint8_t *stag
                 }
                 fence_proxy_async();
                 __syncwarp();
-                if (lane == 0) {
+                if (elect_one()) {
                     if (p.beta != 0.0f) tma_reduce_add_2d(&p.o_map[0], smem_u32(stage), (int)(col0 + c * 32), (int)rbase);
                     else tma_store_2d(&p.o_map[0], smem_u32(stage), (int)(col0 + c * 32), (int)rbase);
                     bulk_commit();
@@ -463,9 +463,9 @@ struct EpiCtx { uint64_t *bar; uint32_t ph; };
 // computed, the load of the next tile's group 0 before its accumulator is ready.
 __device__ __forceinline__ void swiglu_bwd_issue(const GemmParams &p, uint8_t *buf, uint64_t *bar, int lane, int x, int y)
 {
-    if (lane == 0) bulk_wait_read();                     // stores that still read this buffer
+    if (elect_one()) bulk_wait_read();                     // stores that still read this buffer
     __syncwarp();
-    if (lane == 0) {
+    if (elect_one()) {
         mbar_expect_tx(smem_u32(bar), 4096);
         tma_load_2d(smem_u32(buf), &p.i_map[0], smem_u32(bar), x, y);
         tma_load_2d(smem_u32(buf + 2048), &p.i_map[1], smem_u32(bar), x, y);
@@ -514,7 +514,7 @@ __device__ __forceinline__ bool swiglu_bwd_bulk(const GemmParams &p, uint8_t *st
         }
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0) {
+        if (elect_one()) {
             tma_store_2d(&p.o_map[0], smem_u32(bg), (int)(col0 + j * 32), (int)rbase);
             tma_store_2d(&p.o_map[1], smem_u32(bu), (int)(col0 + j * 32), (int)rbase);
             bulk_commit();
@@ -596,7 +596,7 @@ k_gemm(const __grid_constant__ GemmParams p)
                 for (int ks = 0; ks < t.ksteps; ks++) {
                     ok = mbar_wait(smem_u32(&empty_a[ra.idx]), ra.phase ^ 1u, abort_flag, p.errword, 1);
                     if (!ok) break;
-                    if (lane == 0) {
+                    if (elect_one()) {
                         uint32_t bar = smem_u32(&full_a[ra.idx]);
                         uint32_t dstA = smem_u32(sA + ra.idx * A_STAGE_BYTES);
                         if (BMODE == AB_TMA_MN) {
@@ -621,7 +621,7 @@ k_gemm(const __grid_constant__ GemmParams p)
                     if (DEQ) {
                         ok = mbar_wait(smem_u32(&empty_c[rc.idx]), rc.phase ^ 1u, abort_flag, p.errword, 2);
                         if (!ok) break;
-                        if (lane == 0) {
+                        if (elect_one()) {
                             uint32_t bar = smem_u32(&full_c[rc.idx]);
                             uint32_t dstC = smem_u32(sC + rc.idx * C_STAGE_BYTES);
                             mbar_expect_tx(bar, C_STAGE_BYTES);
@@ -731,7 +731,7 @@ k_gemm(const __grid_constant__ GemmParams p)
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&tmem_empty[acc]));
         }
-        if (lane == 0) bulk_wait_all();                  // outstanding bulk stores of this warp
+        if (elect_one()) bulk_wait_all();                  // outstanding bulk stores of this warp
     } else if (DEQ) {
         // =============================== dequant warps ===============================
         const int dw = warp - (2 + EPI_WARPS);

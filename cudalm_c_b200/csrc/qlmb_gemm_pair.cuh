@@ -210,7 +210,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                 for (int ks = 0; ks < t.ksteps; ks++) {
                     ok = mbar_wait_idle(smem_u32(&empty[rs.idx]), rs.phase ^ 1u, abort_flag, p.errword, 11);
                     if (!ok) break;
-                    if (lane == 0) {
+                    if (elect_one()) {
                         if (leader) mbar_expect_tx(smem_u32(&full[rs.idx]), TX_BYTES);
                         const uint32_t bar = map_to_cta(smem_u32(&full[rs.idx]), 0);
                         const uint32_t dstA = smem_u32(sA + rs.idx * P_A_STAGE);
@@ -231,7 +231,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                     if (DEQ) {
                         ok = mbar_wait_idle(smem_u32(&empty_c[rc.idx]), rc.phase ^ 1u, abort_flag, p.errword, 12);
                         if (!ok) break;
-                        if (lane == 0) {
+                        if (elect_one()) {
                             uint32_t bar = smem_u32(&full_c[rc.idx]);
                             uint32_t dstC = smem_u32(sC + rc.idx * P_C_STAGE);
                             mbar_expect_tx(bar, P_C_STAGE);
@@ -341,7 +341,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                 if (leader) mbar_arrive(te); else mbar_arrive_remote(map_to_cta(te, 0));
             }
         }
-        if (lane == 0) bulk_wait_all();                  // outstanding bulk stores of this warp
+        if (elect_one()) bulk_wait_all();                  // outstanding bulk stores of this warp
     } else if (DEQ) {
         // =============================== dequant warps (both CTAs) ===============================
         // The warps form DQG groups; group g expands the stages whose running index is g modulo
