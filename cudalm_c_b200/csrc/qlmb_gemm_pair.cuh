@@ -16,7 +16,9 @@
 //   empty[s]       both     released by one tcgen05.commit that arrives in both CTAs
 //   tmem_full[a]   both     committed the same way after a tile's last step
 //   tmem_empty[a]  leader   8 local + 8 remote epilogue warps
-//   full_c/empty_c local    ring of packed-code tiles between the loader and the dequant warps
+//   full_c[s]      local    byte count of the stage's packed codes.  They are requested once empty[s] has completed, so
+//                           a dequant warp that sees them knows that stage s of B is free too, and the multiplies that
+//                           complete empty[s] came after the codes of stage s had been read: no further hand-shake.
 // No bulk copy in this file has more than one destination CTA.
 #pragma once
 
@@ -26,9 +28,6 @@ constexpr int P_BN = 256;                 // accumulator columns of the pair til
 constexpr int P_A_STAGE = BM * BK * 2;    // per CTA: 128 rows
 constexpr int P_B_STAGE = 128 * BK * 2;   // per CTA: 128 columns of B
 constexpr int P_C_STAGE = 128 * BK / 2;   // per CTA: codes of those columns
-constexpr int P_S_STAGE = 128 * 4;        // per CTA: the stage's group scales (up to 128 floats)
-constexpr int P_S_RING = 4096;            // the scale slots together, padded so that what follows stays 1 KiB aligned
-constexpr int P_NSC = 7;                  // depth of the code / scale ring
 
 __device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ void cluster_sync()
@@ -72,17 +71,6 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
 {
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(dst), "l"(map), "r"(cluster_bar), "r"(x), "r"(y) : "memory");
-}
-// 4-byte asynchronous copy global -> shared, and an mbarrier arrival that fires when all
-// earlier asynchronous copies of the calling thread have landed (the barrier's expected count
-// must include one such arrival per calling thread)
-__device__ __forceinline__ void cp_async4(void *dst, const void *src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_arrive(uint32_t bar)
-{
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_alloc2(uint32_t smem_dst, uint32_t ncols)
 { asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory"); }
@@ -142,11 +130,8 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
 {
     constexpr bool DEQ = (BMODE == B_DEQ_MN || BMODE == B_DEQ_K);
     constexpr bool DUAL = (EPI == EPI_SWIGLU);           // CTA 0 expands W1 (gate), CTA 1 expands W3 (up)
-    constexpr int NS = DEQ ? (EPI == EPI_SWIGLU_BWD ? 4 : 5) : 6, NSC = P_NSC;
+    constexpr int NS = DEQ ? (EPI == EPI_SWIGLU_BWD ? 4 : 5) : 6;
     constexpr int GW = DQ_WARPS / DQG;                   // dequant warps per stage group
-    // group scales: codes [K][N] need 64 new scales per stage, fetched by the producer warp into the
-    // stage's slot; codes [N][K] reuse a row's scale for two stages, each lane keeps its own in registers
-    constexpr bool S_SMEM = (BMODE == B_DEQ_MN);
     constexpr uint32_t IDESC = make_idesc(256, P_BN, BMODE == AB_TMA_MN ? 1 : 0, (BMODE == B_DEQ_MN || BMODE == AB_TMA_MN) ? 1 : 0);
     constexpr uint32_t TMEM_COLS = 2 * P_BN;
     constexpr uint32_t TX_BYTES = 2u * (P_A_STAGE + (DEQ ? 0 : P_B_STAGE));   // both CTAs' loads of a stage
@@ -156,14 +141,12 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
     uint8_t *sA = smem;
     uint8_t *sB = sA + NS * P_A_STAGE;
     uint8_t *sC = sB + NS * P_B_STAGE;
-    float *sS = reinterpret_cast<float *>(sC + (DEQ ? NSC * P_C_STAGE : 0));      // [NSC][128] group scales
-    uint8_t *sE = sC + (DEQ ? NSC * P_C_STAGE + P_S_RING : 0);
-    static_assert((P_C_STAGE % 1024) == 0 && (P_S_RING % 1024) == 0 && P_NSC * P_S_STAGE <= P_S_RING,
-                  "the epilogue staging blocks are bulk-tensor boxes with a 128-byte swizzle: 1 KiB alignment");
+    uint8_t *sE = sC + (DEQ ? NS * P_C_STAGE : 0);
+    static_assert((P_C_STAGE % 1024) == 0, "the epilogue staging blocks are bulk-tensor boxes with a 128-byte swizzle: 1 KiB alignment");
     uint64_t *bars = reinterpret_cast<uint64_t *>(sE + EPI_WARPS * epi_stage_bytes(EPI));
     uint64_t *full = bars, *empty = full + NS;
-    uint64_t *full_c = empty + NS, *empty_c = full_c + NSC;
-    uint64_t *tmem_full = empty_c + NSC, *tmem_empty = tmem_full + 2, *spare = tmem_empty + 2;
+    uint64_t *full_c = empty + NS;
+    uint64_t *tmem_full = full_c + NS, *tmem_empty = tmem_full + 2, *spare = tmem_empty + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(spare + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
@@ -173,7 +156,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < NS; i++) { mbar_init(smem_u32(&full[i]), 1 + (DEQ ? 2 * GW : 0)); mbar_init(smem_u32(&empty[i]), 1); }
-        for (int i = 0; i < NSC; i++) { mbar_init(smem_u32(&full_c[i]), S_SMEM ? 33 : 1); mbar_init(smem_u32(&empty_c[i]), GW); }
+        for (int i = 0; i < NS; i++) mbar_init(smem_u32(&full_c[i]), 1);
         for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&tmem_full[i]), 1); mbar_init(smem_u32(&tmem_empty[i]), 2 * EPI_WARPS); }
         mbar_init(smem_u32(spare), 1);
         for (int i = 0; i < 2 * EPI_WARPS; i++) mbar_init(smem_u32(bars + 48 + i), 1);   // epilogue input rings
@@ -198,65 +181,46 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
 
     if (warp == 0) {
         // =============================== TMA producer (both CTAs) ===============================
-        Ring rs = {0, 0}, rc = {0, 0};
-        bool ok = true;
-        // group scales of a stage (codes [K][N]): every lane copies its rows' scales into the stage's slot with
-        // 4-byte asynchronous copies and lets full_c[s] count their completion, so full_c[s]
-        // completes when the code bytes (expect_tx arrival of lane 0) and all 32 lanes' scales landed
-        const int gpr = p.w_cols / 128;
-        for (int tile = pair; ok && tile < total; tile += npairs) {
-            TileInfo t = decode_pair_tile<SCHED>(p, tile, ntr);
-            for (int seg = 0; ok && seg < p.nseg; seg++) {
-                for (int ks = 0; ks < t.ksteps; ks++) {
-                    ok = mbar_wait_idle(smem_u32(&empty[rs.idx]), rs.phase ^ 1u, abort_flag, p.errword, 11);
-                    if (!ok) break;
-                    if (elect_one()) {
-                        if (leader) mbar_expect_tx(smem_u32(&full[rs.idx]), TX_BYTES);
-                        const uint32_t bar = map_to_cta(smem_u32(&full[rs.idx]), 0);
-                        const uint32_t dstA = smem_u32(sA + rs.idx * P_A_STAGE);
-                        const uint32_t dstB = smem_u32(sB + rs.idx * P_B_STAGE);
+        // One thread runs the whole loop.  A stage must be requested within its 512 cycles of multiplies; with the election,
+        // the warp's reconvergence and the group scales (4-byte copies by all lanes) inside the loop it took 870.
+        if (elect_one()) {
+            Ring rs = {0, 0};
+            bool ok = true;
+            const uint32_t full0 = map_to_cta(smem_u32(full), 0), my_full = smem_u32(full), empty0 = smem_u32(empty);
+            const uint32_t full_c0 = smem_u32(full_c), sA0 = smem_u32(sA), sB0 = smem_u32(sB), sC0 = smem_u32(sC);
+            for (int tile = pair; ok && tile < total; tile += npairs) {
+                const TileInfo t = decode_pair_tile<SCHED>(p, tile, ntr);
+                const int xa = t.m0 + my_m, xb = t.n_t * P_BN + my_n;
+                for (int seg = 0; ok && seg < p.nseg; seg++) {
+                    const CUtensorMap *am = &p.a_map[seg], *wm = &p.w_map[DUAL ? (int)rank : seg];
+                    const int wrow = t.e * p.w_rows + (BMODE == B_DEQ_MN ? 0 : xb), wcol = DUAL ? t.n_t * 64 : xb / 2;
+                    for (int ks = 0; ks < t.ksteps; ks++) {
+                        ok = mbar_wait_idle(empty0 + rs.idx * 8u, rs.phase ^ 1u, abort_flag, p.errword, 11);
+                        if (!ok) break;
+                        if (leader) mbar_expect_tx(my_full + rs.idx * 8u, TX_BYTES);
+                        const uint32_t bar = full0 + rs.idx * 8u, dstA = sA0 + rs.idx * P_A_STAGE, dstB = sB0 + rs.idx * P_B_STAGE;
                         if (BMODE == AB_TMA_MN) {
                             const int row = t.row0 + ks * BK;
-                            tma_load_2d_pair(dstA, &p.a_map[0], bar, t.m0 + my_m, row);
-                            tma_load_2d_pair(dstA + 8192, &p.a_map[0], bar, t.m0 + my_m + 64, row);
-                            tma_load_2d_pair(dstB, &p.w_map[0], bar, t.n_t * P_BN + my_n, row);
-                            tma_load_2d_pair(dstB + 8192, &p.w_map[0], bar, t.n_t * P_BN + my_n + 64, row);
+                            tma_load_2d_pair(dstA, am, bar, xa, row);
+                            tma_load_2d_pair(dstA + 8192, am, bar, xa + 64, row);
+                            tma_load_2d_pair(dstB, wm, bar, xb, row);
+                            tma_load_2d_pair(dstB + 8192, wm, bar, xb + 64, row);
                         } else {
-                            tma_load_2d_pair(dstA, &p.a_map[seg], bar, ks * BK, t.m0 + my_m);
-                            if (BMODE == B_TMA_K) tma_load_2d_pair(dstB, &p.w_map[seg], bar, ks * BK, t.n_t * P_BN + my_n);
+                            tma_load_2d_pair(dstA, am, bar, ks * BK, xa);
+                            if (BMODE == B_TMA_K) tma_load_2d_pair(dstB, wm, bar, ks * BK, xb);
                         }
-                    }
-                    __syncwarp();
-                    rs.next(NS);
-                    if (DEQ) {
-                        ok = mbar_wait_idle(smem_u32(&empty_c[rc.idx]), rc.phase ^ 1u, abort_flag, p.errword, 12);
-                        if (!ok) break;
-                        if (elect_one()) {
-                            uint32_t bar = smem_u32(&full_c[rc.idx]);
-                            uint32_t dstC = smem_u32(sC + rc.idx * P_C_STAGE);
-                            mbar_expect_tx(bar, P_C_STAGE);
-                            if (BMODE == B_DEQ_MN) {
-                                int row = t.e * p.w_rows + ks * BK;
-                                if (DUAL) tma_load_2d(dstC, &p.w_map[rank], bar, t.n_t * 64, row);
-                                else tma_load_2d(dstC, &p.w_map[seg], bar, (t.n_t * P_BN + my_n) / 2, row);
-                            } else {
-                                tma_load_2d(dstC, &p.w_map[seg], bar, ks * (BK / 2), t.e * p.w_rows + t.n_t * P_BN + my_n);
-                            }
+                        if (DEQ) {
+                            const uint32_t cbar = full_c0 + rs.idx * 8u, dstC = sC0 + rs.idx * P_C_STAGE;
+                            mbar_expect_tx(cbar, P_C_STAGE);
+                            if (BMODE == B_DEQ_MN) tma_load_2d(dstC, wm, cbar, wcol, wrow + ks * BK);
+                            else tma_load_2d(dstC, wm, cbar, ks * (BK / 2), wrow);
                         }
-                        if (S_SMEM) {
-                            const float *sp = DUAL ? p.scales[rank] : p.scales[seg];
-                            float *sdst = sS + rc.idx * 128;
-                            const size_t b0 = (size_t)(t.e * p.w_rows + ks * BK) * gpr + (DUAL ? t.n_t * 128 : t.n_t * P_BN + my_n) / 128;
-#pragma unroll
-                            for (int i = 0; i < 2; i++) cp_async4(sdst + lane + 32 * i, sp + b0 + (size_t)(lane + 32 * i) * gpr);
-                            cp_async_arrive(smem_u32(&full_c[rc.idx]));
-                        }
-                        __syncwarp();
-                        rc.next(NSC);
+                        rs.next(NS);
                     }
                 }
             }
         }
+        __syncwarp();
     } else if (warp == 1) {
         if (leader) {
             // =============================== MMA issuer (leader CTA) ===============================
@@ -363,55 +327,52 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
             else dst0[i] = (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((c0 ^ (r & 7)) << 4));
         }
         constexpr uint32_t DST_STEP = (uint32_t)(PER * ROWS_I / 8) * 1024u;      // bytes per PER words
-        Ring rc = {0, 0}, rb = {0, 0};
+        Ring rb = {0, 0};
         bool ok = true;
         const uint32_t full0 = map_to_cta(smem_u32(&full[0]), 0);    // the leader's stage barriers
+        const uint32_t full_c0 = smem_u32(full_c);
         const int gpr = p.w_cols / 128;
+        // A warp's words of a stage lie in 16 (codes [K][N]) or 32 (codes [N][K]) rows, each with one scale: lane m requests
+        // that of row `srow` one stage ahead, and word i takes it from lane i * SPL + sub (one load and one conversion per
+        // lane and stage; eight of each per lane took 500 cycles of the 1900 that a group spent on its stage).
+        constexpr int SPL = BMODE == B_DEQ_MN ? 2 : 4;
+        static_assert(ITERS * SPL <= 32, "one scale per lane");
+        const int sub = BMODE == B_DEQ_MN ? lane >> 4 : lane >> 3;
+        const int m = BMODE == B_DEQ_MN ? lane & 15 : lane, srow = gw * SPL + m % SPL + m / SPL * ROWS_I;
         int kc = 0;                                                  // running stage index of this CTA
         for (int tile = pair; ok && tile < total; tile += npairs) {
             TileInfo t = decode_pair_tile<SCHED>(p, tile, ntr);
             for (int seg = 0; ok && seg < p.nseg; seg++) {
                 int ks = (g - kc % DQG + DQG) % DQG;                 // first stage of this group in the tile
-                for (int i = 0; i < ks && i < t.ksteps; i++) { rc.next(NSC); rb.next(NS); }
-                // codes [N][K]: scale of word i at stage ks is sp[sb + i * rstep + ks * 64 / 128]
-                const float *sp = p.scales[seg];
-                const int sb = (t.e * p.w_rows + t.n_t * P_BN + my_n + r0) * gpr, rstep = ROWS_I * gpr;
-                float cur[ITERS], nxt[ITERS];
-                if (!S_SMEM && ks < t.ksteps) {
-#pragma unroll
-                    for (int i = 0; i < ITERS; i++) cur[i] = __ldg(sp + sb + i * rstep + (ks * BK) / 128);
-                }
+                for (int i = 0; i < ks && i < t.ksteps; i++) rb.next(NS);
+                // one stage on is BK rows (codes [K][N]) or half a group (codes [N][K]) on
+                const float *sp = p.scales[DUAL ? (int)rank : seg]
+                    + (BMODE == B_DEQ_MN ? (t.e * p.w_rows + srow) * gpr + (DUAL ? t.n_t : (t.n_t * P_BN + my_n) / 128)
+                                         : (t.e * p.w_rows + t.n_t * P_BN + my_n + srow) * gpr);
+                const int sstep = BMODE == B_DEQ_MN ? BK * gpr : 0;
+                auto scale_at = [&](int k) { return __ldg(sp + (BMODE == B_DEQ_MN ? k * sstep : (k * BK) / 128)); };
+                float cur = ks < t.ksteps ? scale_at(ks) : 0.0f;
                 for (; ks < t.ksteps; ks += DQG) {
-                    if (!S_SMEM && ks + DQG < t.ksteps) {
-#pragma unroll
-                        for (int i = 0; i < ITERS; i++) nxt[i] = __ldg(sp + sb + i * rstep + ((ks + DQG) * BK) / 128);
-                    }
-                    ok = mbar_wait_idle(smem_u32(&full_c[rc.idx]), rc.phase, abort_flag, p.errword, 20);
+                    const float nxt = ks + DQG < t.ksteps ? scale_at(ks + DQG) : 0.0f;
+                    const __nv_bfloat162 s2 = __float2bfloat162_rn(cur);
+                    ok = mbar_wait(full_c0 + rb.idx * 8u, rb.phase, abort_flag, p.errword, 20);
                     if (!ok) break;
-                    const uint32_t *cw = reinterpret_cast<const uint32_t *>(sC + rc.idx * P_C_STAGE);
+                    const uint32_t *cw = reinterpret_cast<const uint32_t *>(sC + rb.idx * P_C_STAGE) + gw * 32 + lane;
                     uint32_t w[ITERS];
 #pragma unroll
-                    for (int i = 0; i < ITERS; i++) w[i] = cw[(i * GW + gw) * 32 + lane];
-                    if (S_SMEM) {
-                        const float *sc = sS + rc.idx * 128 + r0;    // scale of word i: sc[i * ROWS_I]
-#pragma unroll
-                        for (int i = 0; i < ITERS; i++) cur[i] = sc[i * ROWS_I];
-                    }
-                    ok = mbar_wait_idle(smem_u32(&empty[rb.idx]), rb.phase ^ 1u, abort_flag, p.errword, 21);
-                    if (!ok) break;
+                    for (int i = 0; i < ITERS; i++) w[i] = cw[i * GW * 32];
                     uint8_t *bdst = sB + rb.idx * P_B_STAGE;
 #pragma unroll
-                    for (int i = 0; i < ITERS; i++)
-                        *reinterpret_cast<uint4 *>(bdst + dst0[i % PER] + (uint32_t)(i / PER) * DST_STEP) = (BMODE == B_DEQ_MN) ? dequant8_perm(w[i], __float2bfloat162_rn(cur[i])) : dequant8(w[i], __float2bfloat162_rn(cur[i]));
+                    for (int i = 0; i < ITERS; i++) {
+                        const __nv_bfloat162 sw = __shfl_sync(0xffffffffu, s2, i * SPL + sub);
+                        *reinterpret_cast<uint4 *>(bdst + dst0[i % PER] + (uint32_t)(i / PER) * DST_STEP) = (BMODE == B_DEQ_MN) ? dequant8_perm(w[i], sw) : dequant8(w[i], sw);
+                    }
                     fence_proxy_async();
                     __syncwarp();
-                    if (lane == 0) { mbar_arrive_remote(full0 + (uint32_t)rb.idx * 8u); mbar_arrive(smem_u32(&empty_c[rc.idx])); }
-                    const int adv = ks + DQG <= t.ksteps ? DQG : t.ksteps - ks;
-                    for (int i = 0; i < adv; i++) { rc.next(NSC); rb.next(NS); }
-                    if (!S_SMEM) {
-#pragma unroll
-                        for (int i = 0; i < ITERS; i++) cur[i] = nxt[i];
-                    }
+                    if (elect_one()) mbar_arrive_remote(full0 + (uint32_t)rb.idx * 8u);
+                    rb.idx += ks + DQG <= t.ksteps ? DQG : t.ksteps - ks;
+                    if (rb.idx >= NS) { rb.idx -= NS; rb.phase ^= 1u; }
+                    cur = nxt;
                 }
                 kc += t.ksteps;
             }
