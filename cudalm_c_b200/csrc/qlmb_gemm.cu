@@ -217,8 +217,8 @@ __device__ __forceinline__ void blk_reuse(int lane)
     if (elect_one()) bulk_wait_read();
     __syncwarp();
 }
-// staging bytes per epilogue warp
-__host__ __device__ constexpr int epi_stage_bytes(int epi) { return epi == EPI_SWIGLU_BWD ? 8192 : 4096; }
+// staging bytes per epilogue warp: two blocks for the SwiGLU backward and (`two`) where fp32 output alternates between them
+__host__ __device__ constexpr int epi_stage_bytes(int epi, bool two) { return epi == EPI_SWIGLU_BWD || two ? 8192 : 4096; }
 
 struct Ring {
     int idx; uint32_t phase;
@@ -263,7 +263,7 @@ __device__ __forceinline__ bool swiglu_bwd_bulk(const GemmParams &p, uint8_t *st
 // address tbase; rbase = index of the warp's first row in the output, col0 = first
 // output column.  EPI_SWIGLU reads 64 gate columns at tbase and 64 up columns at
 // tbase + u_off and writes 64 activation columns.
-template <int EPI, bool NPERM = false>
+template <int EPI, bool TWO, bool NPERM = false>
 __device__ __forceinline__ void epilogue_rows(const GemmParams &p, uint8_t *stage, EpiCtx &ec, int lane, uint32_t tbase,
                                               long long rbase, long long col0, int valid, bool have_acc, uint32_t u_off)
 {
@@ -278,20 +278,19 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams &p, uint8_t *stag
         }
 #pragma unroll 1
         for (int half = 0; half < 2; half++) {
+            // the accumulators are read and rounded while the block's previous store still reads the staging buffer
+            uint32_t v[64];
+            tmem_ld32(tbase + half * 64, v);
+            tmem_ld32(tbase + half * 64 + 32, v + 32);
+            tmem_ld_wait();
+            uint4 w[8];
+            __nv_bfloat162 *hw = reinterpret_cast<__nv_bfloat162 *>(w);
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+                hw[i] = have_acc ? __floats2bfloat162_rn(__uint_as_float(v[acc_col<NPERM>(2 * i)]), __uint_as_float(v[acc_col<NPERM>(2 * i + 1)])) : __floats2bfloat162_rn(0.0f, 0.0f);
             if (p.o_tma && !p.scatter_perm) blk_reuse(lane);
-#pragma unroll 1
-            for (int cc = 0; cc < 2; cc++) {
-                uint32_t v[32];
-                tmem_ld32(tbase + half * 64 + cc * 32, v);
-                tmem_ld_wait();
-                uint4 w[4];
-                __nv_bfloat162 *hw = reinterpret_cast<__nv_bfloat162 *>(w);
 #pragma unroll
-                for (int i = 0; i < 16; i++)
-                    hw[i] = have_acc ? __floats2bfloat162_rn(__uint_as_float(v[acc_col<NPERM>(2 * i)]), __uint_as_float(v[acc_col<NPERM>(2 * i + 1)])) : __floats2bfloat162_rn(0.0f, 0.0f);
-#pragma unroll
-                for (int k = 0; k < 4; k++) *blk_vec(stage, lane, cc * 4 + k) = w[k];
-            }
+            for (int k = 0; k < 8; k++) *blk_vec(stage, lane, k) = w[k];
             if (p.scatter_perm) blk_store_scattered(stage, lane, mine, (int)(col0 + half * 64));
             else if (p.o_tma) blk_store_bulk(stage, lane, &p.o_map[0], (int)(col0 + half * 64), (int)rbase);
             else blk_store(stage, lane, reinterpret_cast<uint8_t *>((bf16 *)p.out + rbase * p.ldo + col0 + half * 64), p.ldo * 2, valid);
@@ -300,12 +299,15 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams &p, uint8_t *stag
         // fp32 output through bulk tensor copies: 32 rows x 32 columns (128-byte rows) per block;
         // beta = 1 adds into the tensor with a bulk reduction, so the old values are never read here
         if (!(p.beta != 0.0f && !have_acc)) {
+            uint8_t *const stage0 = stage;
 #pragma unroll 1
             for (int c = 0; c < 4; c++) {
                 uint32_t v[32];
                 tmem_ld32(tbase + c * 32, v);
                 tmem_ld_wait();
-                blk_reuse(lane);
+                uint8_t *const stage = stage0 + (TWO ? (c & 1) * 4096 : 0);
+                if (elect_one()) { if (TWO) bulk_wait_read1(); else bulk_wait_read(); }
+                __syncwarp();
 #pragma unroll
                 for (int k = 0; k < 8; k++) {
                     uint4 q = have_acc ? make_uint4(v[acc_col<NPERM>(4 * k)], v[acc_col<NPERM>(4 * k + 1)], v[acc_col<NPERM>(4 * k + 2)], v[acc_col<NPERM>(4 * k + 3)]) : make_uint4(0, 0, 0, 0);
@@ -375,12 +377,11 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams &p, uint8_t *stag
         const long long o = rbase * p.ldo + col0;
 #pragma unroll 1
         for (int pass = 0; pass < 3; pass++) {
-            if (p.o_tma) blk_reuse(lane);
-#pragma unroll 1
+            uint4 wv[8];
+#pragma unroll
             for (int c = 0; c < 4; c++) {
                 uint32_t g[16], u[16];
-                uint4 w[2];
-                __nv_bfloat162 *hw = reinterpret_cast<__nv_bfloat162 *>(w);
+                __nv_bfloat162 *hw = reinterpret_cast<__nv_bfloat162 *>(wv + 2 * c);
                 if (pass == 0) {
                     tmem_ld16(tbase + c * 16, g);
                     tmem_ld16(tbase + u_off + c * 16, u);
@@ -397,9 +398,10 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams &p, uint8_t *stag
 #pragma unroll
                     for (int k = 0; k < 8; k++) hw[k] = __floats2bfloat162_rn(__uint_as_float(g[acc_col<NPERM>(2 * k)]), __uint_as_float(g[acc_col<NPERM>(2 * k + 1)]));
                 }
-                *blk_vec(stage, lane, 2 * c) = w[0];
-                *blk_vec(stage, lane, 2 * c + 1) = w[1];
             }
+            if (p.o_tma) blk_reuse(lane);                    // the previous pass's store reads the buffer until here
+#pragma unroll
+            for (int k = 0; k < 8; k++) *blk_vec(stage, lane, k) = wv[k];
             bf16 *dst = pass == 0 ? p.ap : pass == 1 ? p.gp : p.up;
             if (p.o_tma) blk_store_bulk(stage, lane, &p.o_map[pass], (int)col0, (int)rbase);
             else blk_store(stage, lane, reinterpret_cast<uint8_t *>(dst + o), p.ldo * 2, valid);
@@ -555,7 +557,7 @@ k_gemm(const __grid_constant__ GemmParams p)
     uint8_t *sB = sA + NSA * A_STAGE_BYTES;
     uint8_t *sC = sB + NSB * B_STAGE_BYTES;
     uint8_t *sE = sC + (DEQ ? NSC * C_STAGE_BYTES : 0);       // 8 epilogue warps x 4 KiB staging
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sE + EPI_WARPS * epi_stage_bytes(EPI));
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sE + EPI_WARPS * epi_stage_bytes(EPI, false));
     uint64_t *full_a = bars, *empty_a = full_a + NSA, *full_b = empty_a + NSA, *empty_b = full_b + NSB;
     uint64_t *full_c = empty_b + NSB, *empty_c = full_c + NSC, *tmem_full = empty_c + NSC, *tmem_empty = tmem_full + 2;
     uint64_t *spare = tmem_empty + 2;
@@ -706,7 +708,7 @@ k_gemm(const __grid_constant__ GemmParams p)
         // registers, then the row pieces go through a swizzled 4 KiB staging buffer so that
         // every global store instruction writes whole row pieces.
         const int q = warp & 3, h = (warp - 2) >> 2;
-        uint8_t *stage = sE + (warp - 2) * epi_stage_bytes(EPI);
+        uint8_t *stage = sE + (warp - 2) * epi_stage_bytes(EPI, false);
         EpiCtx ec = {bars + 48 + 2 * (warp - 2), 0u};
         bool ok = true;
         int it = 0;
@@ -725,7 +727,7 @@ k_gemm(const __grid_constant__ GemmParams p)
             if (h < t.halves) {
                 const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * ACC_COLS + (uint32_t)h * BN;
                 const bool have_acc = (SCHED != SCHED_GROUPK) || t.ksteps > 0;
-                epilogue_rows<EPI>(p, stage, ec, lane, tbase, rbase, col0, valid, have_acc, BN / 2);
+                epilogue_rows<EPI, false>(p, stage, ec, lane, tbase, rbase, col0, valid, have_acc, BN / 2);
             }
             tc_fence_before();
             __syncwarp();
@@ -870,7 +872,7 @@ static int launch_inst(const GemmParams &p, int grid, cudaStream_t st, bool earl
 {
     constexpr bool DEQ = (BMODE == B_DEQ_MN || BMODE == B_DEQ_K);
     constexpr int NSA = DEQ ? 3 : 4, NSB = DEQ ? 3 : 4, NSC = 4;
-    constexpr size_t smem = 1024 + NSA * A_STAGE_BYTES + NSB * B_STAGE_BYTES + (DEQ ? NSC * C_STAGE_BYTES : 0) + EPI_WARPS * epi_stage_bytes(EPI) + 512;
+    constexpr size_t smem = 1024 + NSA * A_STAGE_BYTES + NSB * B_STAGE_BYTES + (DEQ ? NSC * C_STAGE_BYTES : 0) + EPI_WARPS * epi_stage_bytes(EPI, false) + 512;
     static bool configured = false;
     auto kfn = k_gemm<BMODE, EPI, SCHED>;
     if (!configured) {
@@ -886,7 +888,7 @@ template <int BMODE, int EPI, int SCHED, int DQG>
 static int launch_pair_g(const GemmParams &p, long long total, cudaStream_t st, bool early)
 {
     constexpr bool DEQ = (BMODE == B_DEQ_MN || BMODE == B_DEQ_K);
-    constexpr size_t smem = 1024 + (size_t)(DEQ ? (EPI == EPI_SWIGLU_BWD ? 4 : 5) * (P_A_STAGE + P_B_STAGE + P_C_STAGE) : 6 * (P_A_STAGE + P_B_STAGE)) + EPI_WARPS * epi_stage_bytes(EPI) + 512;
+    constexpr size_t smem = 1024 + (size_t)(DEQ ? (EPI == EPI_SWIGLU_BWD ? 4 : 5) * (P_A_STAGE + P_B_STAGE + P_C_STAGE) : 5 * (P_A_STAGE + P_B_STAGE)) + EPI_WARPS * epi_stage_bytes(EPI, !DEQ) + 512;
     // persistent kernel: every cluster must be resident at once, so the grid is the number of
     // clusters the device can hold at the same time (asked once per kernel instance)
     static int max_clusters = 0;

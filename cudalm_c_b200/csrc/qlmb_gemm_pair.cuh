@@ -130,7 +130,10 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
 {
     constexpr bool DEQ = (BMODE == B_DEQ_MN || BMODE == B_DEQ_K);
     constexpr bool DUAL = (EPI == EPI_SWIGLU);           // CTA 0 expands W1 (gate), CTA 1 expands W3 (up)
-    constexpr int NS = DEQ ? (EPI == EPI_SWIGLU_BWD ? 4 : 5) : 6;
+    constexpr int NS = EPI == EPI_SWIGLU_BWD ? 4 : 5;
+    // Without weights to expand there is room for a second staging block per epilogue warp (a sixth operand stage brought
+    // nothing): 16 KiB of fp32 per warp and tile no longer wait block by block for the store before
+    constexpr bool TWO = !DEQ;
     constexpr int GW = DQ_WARPS / DQG;                   // dequant warps per stage group
     constexpr uint32_t IDESC = make_idesc(256, P_BN, BMODE == AB_TMA_MN ? 1 : 0, (BMODE == B_DEQ_MN || BMODE == AB_TMA_MN) ? 1 : 0);
     constexpr uint32_t TMEM_COLS = 2 * P_BN;
@@ -143,7 +146,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
     uint8_t *sC = sB + NS * P_B_STAGE;
     uint8_t *sE = sC + (DEQ ? NS * P_C_STAGE : 0);
     static_assert((P_C_STAGE % 1024) == 0, "the epilogue staging blocks are bulk-tensor boxes with a 128-byte swizzle: 1 KiB alignment");
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sE + EPI_WARPS * epi_stage_bytes(EPI));
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sE + EPI_WARPS * epi_stage_bytes(EPI, TWO));
     uint64_t *full = bars, *empty = full + NS;
     uint64_t *full_c = empty + NS;
     uint64_t *tmem_full = full_c + NS, *tmem_empty = tmem_full + 2, *spare = tmem_empty + 2;
@@ -154,6 +157,10 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
     const uint32_t rank = cluster_rank();
     const bool leader = rank == 0;
 
+    if (warp == 1 && elect_one()) {                       // the copies' descriptors, ahead of their first use
+        for (int i = 0; i < (DUAL ? 1 : p.nseg); i++) prefetch_map(&p.a_map[i]);
+        for (int i = 0; i < (DUAL ? 2 : p.nseg); i++) prefetch_map(&p.w_map[i]);
+    }
     if (threadIdx.x == 0) {
         for (int i = 0; i < NS; i++) { mbar_init(smem_u32(&full[i]), 1 + (DEQ ? 2 * GW : 0)); mbar_init(smem_u32(&empty[i]), 1); }
         for (int i = 0; i < NS; i++) mbar_init(smem_u32(&full_c[i]), 1);
@@ -273,7 +280,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
         // =============================== epilogue (both CTAs) ===============================
         // warp (q, h): q = TMEM lane quarter (= warp id mod 4), h = which 128 of the 256 columns
         const int q = warp & 3, h = (warp - 2) >> 2;
-        uint8_t *stage = sE + (warp - 2) * epi_stage_bytes(EPI);
+        uint8_t *stage = sE + (warp - 2) * epi_stage_bytes(EPI, TWO);
         EpiCtx ec = {bars + 48 + 2 * (warp - 2), 0u};
         bool ok = true;
         int it = 0;
@@ -294,9 +301,9 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                 const bool have_acc = (SCHED != SCHED_GROUPK) || t.ksteps > 0;
                 const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * P_BN;
                 if (EPI == EPI_SWIGLU)
-                    epilogue_rows<EPI, BMODE == B_DEQ_MN>(p, stage, ec, lane, tbase + (uint32_t)h * 64, rbase, col0, valid, have_acc, 128);
+                    epilogue_rows<EPI, TWO, BMODE == B_DEQ_MN>(p, stage, ec, lane, tbase + (uint32_t)h * 64, rbase, col0, valid, have_acc, 128);
                 else
-                    epilogue_rows<EPI, BMODE == B_DEQ_MN>(p, stage, ec, lane, tbase + (uint32_t)h * 128, rbase, col0, valid, have_acc, 0);
+                    epilogue_rows<EPI, TWO, BMODE == B_DEQ_MN>(p, stage, ec, lane, tbase + (uint32_t)h * 128, rbase, col0, valid, have_acc, 0);
             }
             tc_fence_before();
             __syncwarp();
