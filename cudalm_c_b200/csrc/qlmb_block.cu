@@ -332,18 +332,25 @@ __global__ void __launch_bounds__(256) k_dec_kv(bf16_t *Kc, bf16_t *Vc, const bf
     const size_t o = ((size_t)b * Tm + t) * KD + j;
     Kc[o] = k[i]; Vc[o] = v[i];
 }
-// k_dec_attn (cudalm.cu:7031-7047): one block of four warps per (slot, head) over the cached keys lo..pos[b].
-// Pass 1: a thread takes every 128th key and computes its whole 64-wide dot product (16-byte loads), scores
-// go to shared memory, block-wide max and sum.  Pass 2: a lane owns two of the 64 output dimensions, each warp
-// walks a quarter of the keys (four value rows in flight, each one coalesced 128-byte line), and the four
-// partial outputs are added in warp order.  Head dimension 64, bf16 cache.
+// k_dec_attn (cudalm.cu:7031-7047): one block of four warps per (slot, head) over the cached keys lo..pos[b].  It is bound
+// by the cache reads, 128 bytes of K and of V per key.  Eight lanes share a row (16 bytes, eight dimensions each), so that a
+// load instruction of a warp covers four whole rows, and four of them are in flight per lane.  (A thread per key, each
+// walking its own row, took 20.6 us for 64 slots x 12 heads at 256 to 512 keys; this form 11.4.)
+// Pass 1: scores to shared memory, block-wide max and sum.  Pass 2: every lane sums its eight dimensions over its rows; the
+// sixteen partial outputs (four rows a warp, four warps) are added in a fixed order.  Head dimension 64, bf16 cache.
 #define DEC_TM_MAX 4096
+__device__ __forceinline__ void bf8_to_f(const uint4 &x, float f[8])
+{
+    const uint32_t u[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) { f[2 * k] = __uint_as_float(u[k] << 16); f[2 * k + 1] = __uint_as_float(u[k] & 0xffff0000u); }
+}
 __global__ void __launch_bounds__(128) k_dec_attn(bf16_t *O, const bf16_t *Q, const bf16_t *Kc, const bf16_t *Vc, const int *pos,
                                                   int win, int B, int Tm, int H, int KV, float scale, int *errword)
 {
     extern __shared__ float dec_sc[];                    // Tm scores
     __shared__ float red[4], part[4][64];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x, row = lane >> 3, c8 = (lane & 7) * 8;
     const int g = blockIdx.x;
     pdl_trigger();
     pdl_wait();                                          // positions, query and cache rows are written by the kernels before
@@ -351,31 +358,30 @@ __global__ void __launch_bounds__(128) k_dec_attn(bf16_t *O, const bf16_t *Q, co
     if (t < 0 || t >= Tm) { if (tid == 0 && h == 0) report_bad_index(errword, 302, b, t); return; }   // whole block: no score past the cache
     float *sc = dec_sc;
     const int lo = (win > 0 && t >= win) ? t - win + 1 : 0;
-    float q[64];
-    {
-        const uint4 *qp = reinterpret_cast<const uint4 *>(Q + (size_t)b * D + h * 64);
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const uint4 x = __ldg(qp + u);
-            const __nv_bfloat162 *xh = reinterpret_cast<const __nv_bfloat162 *>(&x);
-#pragma unroll
-            for (int k = 0; k < 4; k++) { const float2 f = __bfloat1622float2(xh[k]); q[u * 8 + 2 * k] = f.x; q[u * 8 + 2 * k + 1] = f.y; }
-        }
-    }
+    float q[8];
+    bf8_to_f(__ldg(reinterpret_cast<const uint4 *>(Q + (size_t)b * D + h * 64 + c8)), q);
+    const size_t base = (size_t)b * Tm * KD + kvh * 64 + c8;
+    const bf16_t *kb = Kc + base, *vb = Vc + base;
     float mx = -1e30f;
-    for (int s = lo + tid; s <= t; s += 128) {
-        const uint4 *kp = reinterpret_cast<const uint4 *>(Kc + ((size_t)b * Tm + s) * KD + kvh * 64);
-        float dot = 0.0f;
+    for (int s0 = lo + 4 * warp; s0 <= t; s0 += 64) {    // rows s0 + row, and 16, 32, 48 further
+        uint4 x[4];
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const uint4 x = kp[u];
-            const __nv_bfloat162 *xh = reinterpret_cast<const __nv_bfloat162 *>(&x);
-#pragma unroll
-            for (int k = 0; k < 4; k++) { const float2 f = __bfloat1622float2(xh[k]); dot += q[u * 8 + 2 * k] * f.x + q[u * 8 + 2 * k + 1] * f.y; }
+        for (int u = 0; u < 4; u++) {
+            const int s = s0 + 16 * u + row;
+            x[u] = *reinterpret_cast<const uint4 *>(kb + (size_t)(s <= t ? s : t) * KD);
         }
-        dot *= scale;
-        sc[s] = dot;
-        mx = fmaxf(mx, dot);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int s = s0 + 16 * u + row;
+            float f[8], dot = 0.0f;
+            bf8_to_f(x[u], f);
+#pragma unroll
+            for (int k = 0; k < 8; k++) dot += q[k] * f[k];
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+            dot *= scale;
+            if (s <= t) { if ((lane & 7) == 0) sc[s] = dot; mx = fmaxf(mx, dot); }
+        }
     }
     mx = warp_max(mx);
     if (lane == 0) red[warp] = mx;
@@ -388,36 +394,32 @@ __global__ void __launch_bounds__(128) k_dec_attn(bf16_t *O, const bf16_t *Q, co
     if (lane == 0) red[warp] = l;
     __syncthreads();
     l = (red[0] + red[1]) + (red[2] + red[3]);
-    // pass 2: warp w takes keys lo + w, lo + w + 4, ...
-    float a0 = 0.0f, a1 = 0.0f;
-    const bf16_t *vb = Vc + (size_t)b * Tm * KD + kvh * 64 + 2 * lane;
-    int s = lo + warp;
-    for (; s + 60 <= t; s += 64) {                       // sixteen value rows in flight, added in the same ascending order
-        float2 f[16]; float p[16];
+    float a[8] = {};
+    for (int s0 = lo + 4 * warp; s0 <= t; s0 += 64) {
+        uint4 x[4]; float p[4];
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            f[k] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(vb + (size_t)(s + 4 * k) * KD));
-            p[k] = sc[s + 4 * k];
+        for (int u = 0; u < 4; u++) {
+            const int s = s0 + 16 * u + row;
+            x[u] = *reinterpret_cast<const uint4 *>(vb + (size_t)(s <= t ? s : t) * KD);
+            p[u] = s <= t ? sc[s] : 0.0f;
         }
 #pragma unroll
-        for (int k = 0; k < 16; k++) { a0 += p[k] * f[k].x; a1 += p[k] * f[k].y; }
-    }
-    for (; s + 12 <= t; s += 16) {
-        float2 f[4]; float p[4];
+        for (int u = 0; u < 4; u++) {
+            float f[8];
+            bf8_to_f(x[u], f);
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            f[k] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(vb + (size_t)(s + 4 * k) * KD));
-            p[k] = sc[s + 4 * k];
+            for (int k = 0; k < 8; k++) a[k] += p[u] * f[k];
         }
+    }
 #pragma unroll
-        for (int k = 0; k < 4; k++) { a0 += p[k] * f[k].x; a1 += p[k] * f[k].y; }
+    for (int k = 0; k < 8; k++) {
+        a[k] += __shfl_xor_sync(0xffffffffu, a[k], 8);
+        a[k] += __shfl_xor_sync(0xffffffffu, a[k], 16);
     }
-    for (; s <= t; s += 4) {
-        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(vb + (size_t)s * KD));
-        const float p = sc[s];
-        a0 += p * f.x; a1 += p * f.y;
+    if (row == 0) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) part[warp][c8 + k] = a[k];
     }
-    part[warp][2 * lane] = a0; part[warp][2 * lane + 1] = a1;
     __syncthreads();
     if (warp == 0) {
         const float inv = 1.0f / l;

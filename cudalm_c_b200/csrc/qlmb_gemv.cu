@@ -568,11 +568,16 @@ __device__ __forceinline__ void digits_bf16(uint32_t w, uint32_t q[4])
     }
 }
 
-template <int MT>
-__global__ void __launch_bounds__(256, MT == 1 ? 2 : 1) k_gemv_mma(const __grid_constant__ Rows8 a)
+template <int N_> struct VecOfF;
+template <> struct VecOfF<2> { typedef float2 T; };
+template <> struct VecOfF<4> { typedef float4 T; };
+// NW warps per block: eight (512 columns), or four (256) where the last block of eight would be at most half full (N = 768:
+// a quarter of the warps would repeat columns).
+template <int MT, int NW>
+__global__ void __launch_bounds__(32 * NW, MT == 1 ? 16 / NW : (NW == 8 ? 1 : 3)) k_gemv_mma(const __grid_constant__ Rows8 a)
 {
-    constexpr int GR = 16 * MT, CW = 512, PADK = 8;
-    extern __shared__ __align__(16) uint8_t msm[];       // activations bf16 [GR][kslice + PADK], then scales [kslice][4]
+    constexpr int GR = 16 * MT, CW = 64 * NW, PADK = 8, NT = 32 * NW, NG = NW / 2;
+    extern __shared__ __align__(16) uint8_t msm[];       // activations bf16 [GR][kslice + PADK], then scales [kslice][NG]
     __shared__ int s_n, s_mat, s_x[GR], s_o[GR];
     __shared__ float s_rinv[GR];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -605,24 +610,25 @@ __global__ void __launch_bounds__(256, MT == 1 ? 2 : 1) k_gemv_mma(const __grid_
     const int steps = kslice / 16;                       // a multiple of four: kslice is a multiple of 64
 #pragma unroll
     for (int u = 0; u < 4; u++) fetch(u);
-    // the slice's group scales for the block's four column groups: [kslice][4] floats behind the activations
+    // the slice's group scales for the block's NG column groups: [kslice][NG] floats behind the activations
     float *ssc = reinterpret_cast<float *>(msm + (size_t)GR * ldx * sizeof(bf16));
     {
         const int g0 = blockIdx.x * (CW / 128), gmax = N / 128 - 1;
-        if (g0 + 3 <= gmax && (srow & 3) == 0) {                  // four neighbouring scales of a row in one load
-            for (int i = threadIdx.x; i < kslice; i += 256)
-                reinterpret_cast<float4 *>(ssc)[i] = __ldg(reinterpret_cast<const float4 *>(scales + (size_t)(k0 + i) * srow + g0));
+        if (g0 + NG - 1 <= gmax && (srow & (NG - 1)) == 0) {      // NG neighbouring scales of a row in one load
+            typedef typename VecOfF<NG>::T V;
+            for (int i = threadIdx.x; i < kslice; i += NT)
+                reinterpret_cast<V *>(ssc)[i] = __ldg(reinterpret_cast<const V *>(scales + (size_t)(k0 + i) * srow + g0));
         } else {
-            for (int i = threadIdx.x; i < kslice * 4; i += 256) {
-                const int gq = g0 + (i & 3) < gmax ? g0 + (i & 3) : gmax;
-                ssc[i] = __ldg(scales + (size_t)(k0 + (i >> 2)) * srow + gq);
+            for (int i = threadIdx.x; i < kslice * NG; i += NT) {
+                const int gq = g0 + (i % NG) < gmax ? g0 + (i % NG) : gmax;
+                ssc[i] = __ldg(scales + (size_t)(k0 + i / NG) * srow + gq);
             }
         }
     }
     if (!a.perm) pdl_wait();                             // codes and scales above do not depend on the kernels before; the rows below do
     const bool vec = a.x_dtype == QLMB_BF16;                     // bf16 rows are staged in 16-byte pieces, four loads in flight
-    if (a.gamma) {                                       // 1 / rms of every row over the whole K: warp w takes rows w, w + 8, ...
-        for (int r = warp; r < nrow; r += 8) {
+    if (a.gamma) {                                       // 1 / rms of every row over the whole K: warp w takes rows w, w + NW, ...
+        for (int r = warp; r < nrow; r += NW) {
             float ss = 0.0f;
             if (vec) {
                 const uint4 *xr = reinterpret_cast<const uint4 *>(reinterpret_cast<const bf16 *>(a.X) + (size_t)s_x[r] * K);
@@ -643,18 +649,18 @@ __global__ void __launch_bounds__(256, MT == 1 ? 2 : 1) k_gemv_mma(const __grid_
     }
     if (vec) {
         const int cpr = kslice / 8, total = GR * cpr;
-        for (int i0 = threadIdx.x; i0 < total; i0 += 4 * 256) {
+        for (int i0 = threadIdx.x; i0 < total; i0 += 4 * NT) {
             uint4 v[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const int i = i0 + j * 256, b = i / cpr, kc = i - b * cpr;
+                const int i = i0 + j * NT, b = i / cpr, kc = i - b * cpr;
                 v[j] = make_uint4(0u, 0u, 0u, 0u);
                 if (i < total && b < nrow)
                     v[j] = __ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const bf16 *>(a.X) + (size_t)s_x[b] * K + k0 + kc * 8));
             }
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const int i = i0 + j * 256, b = i / cpr, kc = i - b * cpr;
+                const int i = i0 + j * NT, b = i / cpr, kc = i - b * cpr;
                 if (i >= total) continue;
                 if (a.gamma && b < nrow) {
                     __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&v[j]);
@@ -670,7 +676,7 @@ __global__ void __launch_bounds__(256, MT == 1 ? 2 : 1) k_gemv_mma(const __grid_
             }
         }
     } else {
-        for (int i = threadIdx.x; i < GR * kslice; i += 256) {
+        for (int i = threadIdx.x; i < GR * kslice; i += NT) {
             const int b = i / kslice, kk = i % kslice;
             float x = 0.0f;
             if (b < nrow) {
@@ -689,13 +695,13 @@ __global__ void __launch_bounds__(256, MT == 1 ? 2 : 1) k_gemv_mma(const __grid_
 #pragma unroll
             for (int i = 0; i < 4; i++) acc[m][c][i] = 0.0f;
     const bf16 *xa = xs + g * ldx + 2 * t;               // A fragment of step 0: rows g, g + 8 (per 16-row tile), columns 2t.., 2t + 8..
-    const float *sl = ssc + (2 * t) * 4 + (warp >> 1);   // scale of the lane's first row of step 0 for this warp's column group
+    const float *sl = ssc + (2 * t) * NG + (warp >> 1);   // scale of the lane's first row of step 0 for this warp's column group
     auto use = [&](int slot) {
         uint32_t q[4][4];
 #pragma unroll
         for (int r = 0; r < 4; r++) digits_bf16(w[slot][r], q[r]);
-        const __nv_bfloat162 s01 = __floats2bfloat162_rn(sl[0], sl[4]), s23 = __floats2bfloat162_rn(sl[32], sl[36]);
-        sl += 64;
+        const __nv_bfloat162 s01 = __floats2bfloat162_rn(sl[0], sl[NG]), s23 = __floats2bfloat162_rn(sl[8 * NG], sl[9 * NG]);
+        sl += 16 * NG;
         uint32_t af[MT][4];
 #pragma unroll
         for (int m = 0; m < MT; m++) {
@@ -775,36 +781,55 @@ static int rows8_launch(Rows8 a, int nz, int ns, cudaStream_t st)
     return QLMB_OK;
 }
 
-// K slices of a k_gemv_mma launch with nz groups of 16 * mt rows: a divisor of K / 64 such that the activation tile
-// fits 64 KiB of shared memory, about two blocks per SM in total
-static int mma_slices(int K, int N, int nz, int mt)
+// Shape of a k_gemv_mma launch over nz groups of 16 * mt rows: warps per block and K slices.  A slice is a whole number of
+// 64-row units and its activation tile fits 64 KiB.  The device takes `slots` blocks at a time, a block needs its steps of
+// sixteen rows and about ten steps' time to start and to stage its rows: the slice count with the least rounds * (steps + 10)
+// wins (gate and up of 64 slots and 32 experts, 768 x 1536: 3 slices instead of 2).
+struct MmaPlan { int nw, nb, ns; };
+static MmaPlan mma_plan(int K, int N, int nz, int mt)
 {
-    const int nb = (N + 511) / 512, units = K / 64, kmax = mt == 1 ? 1024 : 512;
-    int want = (2 * sm_count() + nb * nz / 2) / (nb * nz), best = 0, smallest = 0;
-    if (want < 1) want = 1;
+    MmaPlan p;
+    p.nw = (N % 512) && (N % 512) <= 256 ? 4 : 8;
+    p.nb = (N + 64 * p.nw - 1) / (64 * p.nw);
+    const int units = K / 64, kmax = mt == 1 ? 1024 : 512;
+    const int slots = sm_count() * (mt == 1 ? 16 / p.nw : (p.nw == 8 ? 1 : 3));
+    long long best = -1;
+    p.ns = units;
     for (int d = 1; d <= units; d++) {
         if (units % d || K / d > kmax) continue;
-        if (!smallest) smallest = d;
-        if (d <= want) best = d;
+        const long long rounds = ((long long)p.nb * nz * d + slots - 1) / slots, cost = rounds * (K / d / 16 + 10);
+        if (best < 0 || cost < best) { best = cost; p.ns = d; }
     }
-    return best ? best : smallest;
+    return p;
 }
-static int mma_launch(Rows8 a, int nz, int ns, int mt, cudaStream_t st)
+// Rows per group: 32 share one expansion of the weights, but a matrix too small to give every SM a block that way is bound by
+// a block's own serial work, which 16 rows halve (with four-warp blocks for the ragged widths: the four projections and the down product of a 768-wide
+// layer at 64 slots 42 -> 26 us)
+static int mma_mt(int B, int K, int N, int nmat)
 {
-    const int nb = (a.N + 511) / 512;
-    a.kslice = a.K / ns;
+    if (B <= 16) return 1;
+    return ((N + 511) / 512) * nmat * ((B + 31) / 32) * (K / 64) >= 2 * sm_count() ? 2 : 1;
+}
+static int mma_launch(Rows8 a, int nz, const MmaPlan &pl, int mt, cudaStream_t st)
+{
+    a.kslice = a.K / pl.ns;
     a.k65536 = 65536u;
-    const size_t sm_b = (size_t)16 * mt * (a.kslice + 8) * sizeof(bf16) + (size_t)a.kslice * 4 * sizeof(float);
+    const size_t sm_b = (size_t)16 * mt * (a.kslice + 8) * sizeof(bf16) + (size_t)a.kslice * (pl.nw / 2) * sizeof(float);
     static bool attr_done[64];
     int dv = 0;
     QLMB_CUDA(cudaGetDevice(&dv));
     if (dv >= 0 && dv < 64 && !attr_done[dv]) {
-        QLMB_CUDA(cudaFuncSetAttribute(k_gemv_mma<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-        QLMB_CUDA(cudaFuncSetAttribute(k_gemv_mma<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+        QLMB_CUDA(cudaFuncSetAttribute(k_gemv_mma<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+        QLMB_CUDA(cudaFuncSetAttribute(k_gemv_mma<1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+        QLMB_CUDA(cudaFuncSetAttribute(k_gemv_mma<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+        QLMB_CUDA(cudaFuncSetAttribute(k_gemv_mma<2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
         attr_done[dv] = true;
     }
-    if (mt == 1) QLMB_CUDA(pdl_launch(true, k_gemv_mma<1>, dim3(nb, ns, nz), dim3(256), sm_b, st, a));
-    else QLMB_CUDA(pdl_launch(true, k_gemv_mma<2>, dim3(nb, ns, nz), dim3(256), sm_b, st, a));
+    const dim3 grid(pl.nb, pl.ns, nz), block(32 * pl.nw);
+    if (mt == 1 && pl.nw == 8) QLMB_CUDA(pdl_launch(true, k_gemv_mma<1, 8>, grid, block, sm_b, st, a));
+    else if (mt == 1) QLMB_CUDA(pdl_launch(true, k_gemv_mma<1, 4>, grid, block, sm_b, st, a));
+    else if (pl.nw == 8) QLMB_CUDA(pdl_launch(true, k_gemv_mma<2, 8>, grid, block, sm_b, st, a));
+    else QLMB_CUDA(pdl_launch(true, k_gemv_mma<2, 4>, grid, block, sm_b, st, a));
     QLMB_LAUNCH_CHECK("k_gemv_mma");
     return QLMB_OK;
 }
@@ -1021,7 +1046,8 @@ int moe_decode_experts(const qlmb_moe_layer *L, void *out, const void *f_in, con
         int rc = perm_ready ? 0 : perm_build(assign, N, L->E, K, 1, 1, perm, nullptr, off, counts, bad, nullptr, nullptr, nullptr, st);
         if (rc) return rc;
         const int zmax = L->E + R / 16;                  // sum over the experts of ceil(count / 16) never exceeds this
-        const int ns1 = mma_slices(D, F, 2 * L->E, 1), ns2 = mma_slices(F, D, L->E, 1);
+        const MmaPlan pl1 = mma_plan(D, F, 2 * L->E, 1), pl2 = mma_plan(F, D, L->E, 1);
+        const int ns1 = pl1.ns, ns2 = pl2.ns;
         const size_t pg_n = (size_t)ns1 * 2 * R * F, pd_n = (size_t)ns2 * R * D;
         void *ws = nullptr;
         if ((rc = workspace((pg_n + pd_n) * sizeof(float) + (size_t)R * F * sizeof(bf16) + 256, &ws))) return rc;
@@ -1032,13 +1058,13 @@ int moe_decode_experts(const qlmb_moe_layer *L, void *out, const void *f_in, con
         a.codes = (const uint8_t *)L->w1_codes; a.scales = L->w1_scales; a.codes2 = (const uint8_t *)L->w3_codes; a.scales2 = L->w3_scales;
         a.e_codes = (size_t)D * F / 2; a.e_scales = (size_t)D * F / 128;
         a.rows_out = 2 * R; a.perm = perm; a.off = off; a.E = L->E; a.ntok = N; a.x_by_token = 1; a.zdual = zmax; a.R = R;
-        if ((rc = mma_launch(a, 2 * zmax, ns1, 1, st))) return rc;
+        if ((rc = mma_launch(a, 2 * zmax, pl1, 1, st))) return rc;
         pdl_launch(N > 4, k_gemv_finish_swiglu, dim3((unsigned)(((size_t)R * F + 255) / 256)), dim3(256), 0, st, act, pg, pg + (size_t)R * F, ns1, (size_t)R * F, (size_t)2 * R * F);
         Rows8 b = {};
         b.part = pd; b.X = act; b.x_dtype = QLMB_BF16; b.K = F; b.N = D;
         b.codes = (const uint8_t *)L->w2_codes; b.scales = L->w2_scales; b.e_codes = (size_t)D * F / 2; b.e_scales = (size_t)D * F / 128;
         b.rows_out = R; b.perm = perm; b.off = off; b.E = L->E; b.ntok = N; b.x_by_token = 0; b.zdual = 0; b.R = R;
-        if ((rc = mma_launch(b, zmax, ns2, 1, st))) return rc;
+        if ((rc = mma_launch(b, zmax, pl2, 1, st))) return rc;
         pdl_launch(N > 4, k_gemv_finish_combine, dim3((unsigned)(((size_t)N * D + 255) / 256)), dim3(256), 0, st, (bf16 *)out, (const bf16 *)f_in, pd, gate, ns2, N, K, D);
         QLMB_LAUNCH_CHECK("moe_decode_experts");
         return QLMB_OK;
@@ -1110,15 +1136,17 @@ static int gemv_decode_impl(void *Y, const void *X, const int8_t *codes, const f
         // groups of eight rows per pass over the weights (fp32 multiply-adds; the 256-row tensor-core tiles would be
         // seven eighths padding for a handful of rows)
         const bool tc = dtype == QLMB_BF16 && (N % 64) == 0;
-        const int mt = B > 16 ? 2 : 1;
-        const int nz = tc ? (B + 16 * mt - 1) / (16 * mt) : (B + 7) / 8, ns = tc ? mma_slices(K, N, nz, mt) : rows8_slices(K, N, nz);
+        const int mt = mma_mt(B, K, N, 1);
+        const int nz = tc ? (B + 16 * mt - 1) / (16 * mt) : (B + 7) / 8;
+        const MmaPlan pl = mma_plan(K, N, nz, mt);
+        const int ns = tc ? pl.ns : rows8_slices(K, N, nz);
         void *wsr = nullptr;
         int rcr = workspace((size_t)ns * B * N * sizeof(float), &wsr);
         if (rcr) return rcr;
         Rows8 a = {};
         a.part = (float *)wsr; a.X = X; a.x_dtype = dtype; a.K = K; a.N = N;
         a.codes = (const uint8_t *)codes; a.scales = scales; a.B = B; a.nmat = 1; a.rows_out = B;
-        if ((rcr = tc ? mma_launch(a, nz, ns, mt, st) : rows8_launch(a, nz, ns, st))) return rcr;
+        if ((rcr = tc ? mma_launch(a, nz, pl, mt, st) : rows8_launch(a, nz, ns, st))) return rcr;
         if (fr) pdl_launch(B > 4, k_gemv_finish_res_norm, dim3(B), dim3(256), 0, st, (bf16 *)Y, (bf16 *)fr->Fn, a.part, ns, B, N, (const bf16 *)fr->res, fr->gamma);
         else pdl_launch(B > 4, k_gemv_finish, dim3((unsigned)(((size_t)B * N + 255) / 256)), dim3(256), 0, st, Y, dtype, a.part, ns, (size_t)B * N);
         QLMB_LAUNCH_CHECK("qlmb_gemv_decode");
@@ -1228,9 +1256,10 @@ static int gemv_stack_impl(void *Y, const void *X, const int8_t *codes, const fl
     nslice = (K + kslice - 1) / kslice;
     const bool groups = B > 4;                           // more than four rows: groups share one pass over a matrix
     const bool tc = groups && dtype == QLMB_BF16 && (N % 64) == 0;   // bf16 rows: warp-level MMAs, 16 or 32 rows per group
-    const int mt = B > 16 ? 2 : 1;
+    const int mt = mma_mt(B, K, N, nmat);
     const int nz = tc ? nmat * ((B + 16 * mt - 1) / (16 * mt)) : nmat * ((B + 7) / 8);
-    if (groups) nslice = tc ? mma_slices(K, N, nz, mt) : rows8_slices(K, N, nz);
+    const MmaPlan pl = mma_plan(K, N, nz, mt);
+    if (groups) nslice = tc ? pl.ns : rows8_slices(K, N, nz);
     void *ws = nullptr;
     int rc = workspace((size_t)nslice * R * N * sizeof(float), &ws);
     if (rc) return rc;
@@ -1240,7 +1269,7 @@ static int gemv_stack_impl(void *Y, const void *X, const int8_t *codes, const fl
         a.part = part; a.X = X; a.x_dtype = dtype; a.K = K; a.N = N;
         a.codes = (const uint8_t *)codes; a.scales = scales; a.e_codes = (size_t)K * N / 2; a.e_scales = (size_t)K * N / 128;
         a.B = B; a.nmat = nmat; a.rows_out = R; a.gamma = gamma;
-        if ((rc = tc ? mma_launch(a, nz, nslice, mt, st) : rows8_launch(a, nz, nslice, st))) return rc;
+        if ((rc = tc ? mma_launch(a, nz, pl, mt, st) : rows8_launch(a, nz, nslice, st))) return rc;
     } else if ((size_t)nblk * nslice * R <= (size_t)2 * sm_count())
         launch_kn<1, 4>(B > 4, dim3(nblk, nslice, R), (size_t)kslice * sizeof(float), st, part, X, dtype, (const uint8_t *)codes, scales, 1, K, N, kslice, nullptr, (size_t)K * N / 2, (size_t)K * N / 128, B, gamma);
     else

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) k_router_small(float *rt, const void *X, 
         __threadfence();                                 // this token's choices are visible before its ticket is
     }
     if (!perm) return;
-    __shared__ int s_last, s_asn[256], s_off[33], s_bad;
+    __shared__ int s_last, s_cnt[8][32], s_off[33], s_bad;
     __syncthreads();
     if (threadIdx.x == 0) { s_last = atomicAdd(&g_router_ticket, 1u) == (unsigned)(N - 1); s_bad = 0; }
     __syncthreads();
@@ -147,12 +147,18 @@ __global__ void __launch_bounds__(256) k_router_small(float *rt, const void *X, 
     if (t < R) {
         my = __ldcg(assign + t);
         if (my < 0 || my >= E) { atomicMax(&s_bad, 1); my = -1; }
-        s_asn[t] = my;
     }
+    // stable rank of a slot among its expert's: lower lanes of its warp with the same choice, and the warps before
+    s_cnt[warp][e] = 0;
+    __syncwarp();
+    const unsigned same = __match_any_sync(0xffffffffu, my);
+    const int rank = __popc(same & ((1u << e) - 1u));
+    if (my >= 0 && rank == 0) s_cnt[warp][my] = __popc(same);
     __syncthreads();
-    if (warp == 0) {                                     // lane = expert: count, exclusive scan, offsets
+    if (warp == 0) {                                     // lane = expert: the warps' counts become their starts, exclusive scan
         int c = 0;
-        if (e < E) for (int i = 0; i < R; i++) c += s_asn[i] == e;
+#pragma unroll
+        for (int w = 0; w < 8; w++) { const int v = s_cnt[w][e]; s_cnt[w][e] = c; c += v; }
         int incl = c;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, d); if (e >= d) incl += v; }
@@ -160,11 +166,7 @@ __global__ void __launch_bounds__(256) k_router_small(float *rt, const void *X, 
         if (e == E - 1) { s_off[E] = incl; off[E] = incl; }
     }
     __syncthreads();
-    if (my >= 0) {
-        int rank = 0;
-        for (int i = 0; i < t; i++) rank += s_asn[i] == my;
-        perm[s_off[my] + rank] = t;
-    }
+    if (my >= 0) perm[s_off[my] + s_cnt[warp][my] + rank] = t;
     if (t == 0) { if (bad) *bad = s_bad; g_router_ticket = 0u; }
 }
 
