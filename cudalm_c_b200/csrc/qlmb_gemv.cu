@@ -547,8 +547,8 @@ __global__ void __launch_bounds__(256, 2) k_gemv_rows8(const __grid_constant__ R
 // of eight MMAs.  tcgen05.mma takes its operands from shared memory, which for a kernel that streams every weight
 // exactly once would add a store, a proxy fence and a barrier round trip per stage; the register form needs none.
 // Warp = 64 output columns x the K slice; lane (g = lane / 4, t = lane % 4) loads the code word of columns 8g .. 8g+7
-// for the rows 2t, 2t+1, 2t+8, 2t+9 of every 16-row step, expands it to exact bf16 digits (d = (136 + d) - 136),
-// and pairs the rows with byte permutes into the B fragments of eight MMAs: MMA c uses column 8q + c of the tile
+// for the rows 2t, 2t+1, 2t+8, 2t+9 of every 16-row step, pairs the rows and expands them to exact bf16 digits
+// (d = (136 + d) - 136), the B fragments of eight MMAs: MMA c uses column 8q + c of the tile
 // for q = 0..7.  The group scale of a row (one per row for the 64 columns, which lie in one group of 128) multiplies
 // the activations: A = bf16(x * bf16(s)), the rounding the GEMM engine applies to its rendered weights.
 __device__ __forceinline__ void mma_bf16_16816(float c[4], const uint32_t a[4], uint32_t b0, uint32_t b1)
@@ -556,15 +556,17 @@ __device__ __forceinline__ void mma_bf16_16816(float c[4], const uint32_t a[4], 
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// four registers of exact bf16 digit pairs (elements j and j + 4 of the word in register j)
-__device__ __forceinline__ void digits_bf16(uint32_t w, uint32_t q[4])
+// Column c of two rows' code words as one register of exact bf16 digits, the first row's low: the words' halves are
+// exchanged first, so that a nibble pair already is the B fragment (expanding the words one by one and pairing the rows
+// afterwards took 60 instructions for four words instead of 48).
+__device__ __forceinline__ void digits_pair_bf16(uint32_t w0, uint32_t w1, uint32_t q[8])
 {
-    const uint32_t k136 = 0x43084308u;
+    const uint32_t k136 = 0x43084308u, h[2] = {__byte_perm(w0, w1, 0x5410), __byte_perm(w0, w1, 0x7632)};
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        uint32_t x = nib_pair_f(w >> (4 * j));
+    for (int c = 0; c < 8; c++) {
+        uint32_t x = nib_pair_f(h[c >> 2] >> (4 * (c & 3)));
         __nv_bfloat162 v = __hsub2(*reinterpret_cast<__nv_bfloat162 *>(&x), *reinterpret_cast<const __nv_bfloat162 *>(&k136));
-        q[j] = *reinterpret_cast<uint32_t *>(&v);
+        q[c] = *reinterpret_cast<uint32_t *>(&v);
     }
 }
 
@@ -697,9 +699,9 @@ __global__ void __launch_bounds__(32 * NW, MT == 1 ? 16 / NW : (NW == 8 ? 1 : 3)
     const bf16 *xa = xs + g * ldx + 2 * t;               // A fragment of step 0: rows g, g + 8 (per 16-row tile), columns 2t.., 2t + 8..
     const float *sl = ssc + (2 * t) * NG + (warp >> 1);   // scale of the lane's first row of step 0 for this warp's column group
     auto use = [&](int slot) {
-        uint32_t q[4][4];
-#pragma unroll
-        for (int r = 0; r < 4; r++) digits_bf16(w[slot][r], q[r]);
+        uint32_t b0[8], b1[8];                           // rows (2t, 2t+1) and (2t+8, 2t+9) of the eight columns
+        digits_pair_bf16(w[slot][0], w[slot][1], b0);
+        digits_pair_bf16(w[slot][2], w[slot][3], b1);
         const __nv_bfloat162 s01 = __floats2bfloat162_rn(sl[0], sl[NG]), s23 = __floats2bfloat162_rn(sl[8 * NG], sl[9 * NG]);
         sl += 16 * NG;
         uint32_t af[MT][4];
@@ -713,16 +715,9 @@ __global__ void __launch_bounds__(32 * NW, MT == 1 ? 16 / NW : (NW == 8 ? 1 : 3)
             af[m][2] = *reinterpret_cast<uint32_t *>(&a2); af[m][3] = *reinterpret_cast<uint32_t *>(&a3);
         }
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            // column j: the low halves of rows (2t, 2t+1) and (2t+8, 2t+9); column j + 4: the high halves
-            const uint32_t b0l = __byte_perm(q[0][j], q[1][j], 0x5410), b1l = __byte_perm(q[2][j], q[3][j], 0x5410);
-            const uint32_t b0h = __byte_perm(q[0][j], q[1][j], 0x7632), b1h = __byte_perm(q[2][j], q[3][j], 0x7632);
+        for (int c = 0; c < 8; c++)
 #pragma unroll
-            for (int m = 0; m < MT; m++) {
-                mma_bf16_16816(acc[m][j], af[m], b0l, b1l);
-                mma_bf16_16816(acc[m][j + 4], af[m], b0h, b1h);
-            }
-        }
+            for (int m = 0; m < MT; m++) mma_bf16_16816(acc[m][c], af[m], b0[c], b1[c]);
         xa += 16;
     };
     for (int i = 0; i < steps; i += 4) {
@@ -906,6 +901,7 @@ __global__ void __launch_bounds__(256) k_gemv_finish(void *Y, int dtype, const f
     size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
     if (i >= BN_) return;
     float s = 0.0f;
+#pragma unroll 4
     for (int k = 0; k < nslice; k++) s += part[(size_t)k * BN_ + i];
     if (dtype == QLMB_BF16) ((bf16 *)Y)[i] = __float2bfloat16_rn(s);
     else ((float *)Y)[i] = s;
@@ -928,7 +924,8 @@ __global__ void __launch_bounds__(256) k_gemv_finish_res_norm(bf16 *F, bf16 *Fn,
         v[c] = 0.0f; rs[c] = 0.0f; gm[c] = 0.0f;
         if (n < N) { rs[c] = __bfloat162float(res[(size_t)b * N + n]); gm[c] = gamma[n]; }
     }
-    for (int k = 0; k < nslice; k++) {                   // slice order ascending per column, the columns' loads independent
+#pragma unroll 4
+    for (int k = 0; k < nslice; k++) {                   // slice order ascending per column, four slices' loads in flight
 #pragma unroll
         for (int c = 0; c < 8; c++) {
             const int n = threadIdx.x + 256 * c;
@@ -983,6 +980,7 @@ __global__ void __launch_bounds__(256) k_gemv_finish_qkv(bf16 *Y, bf16 *Kc, bf16
     if (t < 0 || t >= Tm) { if (i == 0 && h == 0 && m == 0) report_bad_index(errword, 303, b, t); return; }
     const size_t o = (size_t)row * N + (size_t)h * hd + i;
     float x = 0.0f, y = 0.0f;
+#pragma unroll 4
     for (int k = 0; k < nslice; k++) { x += part[(size_t)k * RN + o]; y += part[(size_t)k * RN + o + hf]; }
     x = __bfloat162float(__float2bfloat16_rn(x)); y = __bfloat162float(__float2bfloat16_rn(y));
     if (m < 2) {
@@ -1008,6 +1006,7 @@ __global__ void __launch_bounds__(256) k_gemv_finish_swiglu(bf16 *act, const flo
     const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
     if (i >= RN) return;
     float g = 0.0f, u = 0.0f;
+#pragma unroll 4
     for (int k = 0; k < nslice; k++) { g += pg[(size_t)k * slice_stride + i]; u += pu[(size_t)k * slice_stride + i]; }
     // the stash of the training path holds g and u as bf16; round the same way before the product
     g = __bfloat162float(__float2bfloat16_rn(g)); u = __bfloat162float(__float2bfloat16_rn(u));
@@ -1027,6 +1026,7 @@ __global__ void __launch_bounds__(256) k_gemv_finish_combine(bf16 *out, const bf
     for (int k = 0; k < Kk; k++) {
         const size_t o = ((size_t)k * ntok + n) * D + j;
         float y = 0.0f;
+#pragma unroll 4
         for (int s = 0; s < nslice; s++) y += part[(size_t)s * RN + o];
         y = __bfloat162float(__float2bfloat16_rn(y));
         acc += gate[(size_t)k * ntok + n] * y;

@@ -98,13 +98,15 @@ __global__ void __launch_bounds__(256) k_router_small(float *rt, const void *X, 
     __shared__ float part[8][32];
     const int n = blockIdx.x, warp = threadIdx.x >> 5, e = threadIdx.x & 31;
     const int per = (D + 7) / 8, j0 = warp * per, j1 = j0 + per < D ? j0 + per : D;
-    // 32 rows of Wr in flight per lane (the loads depend neither on the sum nor on the activations: the first batch is
-    // requested before the row is staged); the sum itself stays in ascending order
-    float w[32];
+    // 96 rows of Wr in flight per lane (the loads depend neither on the sum nor on the activations: the first batch, at
+    // D = 768 the whole share of a warp, is requested before the row is staged; in batches of 32 the block waited for three
+    // rounds to L2); the sum itself stays in ascending order
+    constexpr int UB = 96;
+    float w[UB];
     pdl_trigger();
     if (e < E) {
 #pragma unroll
-        for (int u = 0; u < 32; u++) w[u] = j0 + u < j1 ? __ldg(Wr + (size_t)(j0 + u) * E + e) : 0.0f;
+        for (int u = 0; u < UB; u++) w[u] = j0 + u < j1 ? __ldg(Wr + (size_t)(j0 + u) * E + e) : 0.0f;
     }
     pdl_wait();                                          // the router matrix above is no kernel's output; the row below is
     for (int j = threadIdx.x; j < D; j += 256)
@@ -112,13 +114,13 @@ __global__ void __launch_bounds__(256) k_router_small(float *rt, const void *X, 
     __syncthreads();
     float acc = 0.0f;
     if (e < E) {
-        for (int j = j0; j < j1; j += 32) {
+        for (int j = j0; j < j1; j += UB) {
             if (j > j0) {
 #pragma unroll
-                for (int u = 0; u < 32; u++) w[u] = j + u < j1 ? __ldg(Wr + (size_t)(j + u) * E + e) : 0.0f;
+                for (int u = 0; u < UB; u++) w[u] = j + u < j1 ? __ldg(Wr + (size_t)(j + u) * E + e) : 0.0f;
             }
 #pragma unroll
-            for (int u = 0; u < 32; u++)
+            for (int u = 0; u < UB; u++)
                 if (j + u < j1) acc = __fmaf_rn(rs_x[j + u], w[u], acc);
         }
     }
