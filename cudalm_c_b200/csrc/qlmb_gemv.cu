@@ -576,7 +576,7 @@ template <> struct VecOfF<4> { typedef float4 T; };
 // NW warps per block: eight (512 columns), or four (256) where the last block of eight would be at most half full (N = 768:
 // a quarter of the warps would repeat columns).
 template <int MT, int NW>
-__global__ void __launch_bounds__(32 * NW, MT == 1 ? 16 / NW : (NW == 8 ? 1 : 3)) k_gemv_mma(const __grid_constant__ Rows8 a)
+__global__ void __launch_bounds__(32 * NW, MT == 1 ? (NW == 8 ? 3 : 4) : (NW == 8 ? 1 : 3)) k_gemv_mma(const __grid_constant__ Rows8 a)
 {
     constexpr int GR = 16 * MT, CW = 64 * NW, PADK = 8, NT = 32 * NW, NG = NW / 2;
     extern __shared__ __align__(16) uint8_t msm[];       // activations bf16 [GR][kslice + PADK], then scales [kslice][NG]
@@ -787,7 +787,7 @@ static MmaPlan mma_plan(int K, int N, int nz, int mt)
     p.nw = (N % 512) && (N % 512) <= 256 ? 4 : 8;
     p.nb = (N + 64 * p.nw - 1) / (64 * p.nw);
     const int units = K / 64, kmax = mt == 1 ? 1024 : 512;
-    const int slots = sm_count() * (mt == 1 ? 16 / p.nw : (p.nw == 8 ? 1 : 3));
+    const int slots = sm_count() * (mt == 1 ? (p.nw == 8 ? 3 : 4) : (p.nw == 8 ? 1 : 3));
     long long best = -1;
     p.ns = units;
     for (int d = 1; d <= units; d++) {
@@ -1046,7 +1046,9 @@ int moe_decode_experts(const qlmb_moe_layer *L, void *out, const void *f_in, con
         int rc = perm_ready ? 0 : perm_build(assign, N, L->E, K, 1, 1, perm, nullptr, off, counts, bad, nullptr, nullptr, nullptr, st);
         if (rc) return rc;
         const int zmax = L->E + R / 16;                  // sum over the experts of ceil(count / 16) never exceeds this
-        const MmaPlan pl1 = mma_plan(D, F, 2 * L->E, 1), pl2 = mma_plan(F, D, L->E, 1);
+        // the groups that will hold rows, about: the experts that R random choices hit (the others' blocks return at once)
+        const int hit = (int)ceil(L->E * (1.0 - pow(1.0 - 1.0 / L->E, R)));
+        const MmaPlan pl1 = mma_plan(D, F, 2 * hit, 1), pl2 = mma_plan(F, D, hit, 1);
         const int ns1 = pl1.ns, ns2 = pl2.ns;
         const size_t pg_n = (size_t)ns1 * 2 * R * F, pd_n = (size_t)ns2 * R * D;
         void *ws = nullptr;
