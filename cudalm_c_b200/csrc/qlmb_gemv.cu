@@ -211,10 +211,13 @@ __device__ __forceinline__ uint32_t nib_pair_f(uint32_t w)
 }
 
 template <int BT, int CPL, int U = 4>
-__global__ void __launch_bounds__(256, BT <= 2 ? 3 : 2) k_gemv_stream(void *Y, int dtype, float *part, const void *X, const uint8_t *codes,
-                                                     const float *scales, int B, int K, int N, int kslice, uint32_t k65536)
+__global__ void __launch_bounds__(256, 2) k_gemv_stream(void *Y, int dtype, float *part, const void *X, const uint8_t *codes,
+                                                     const float *scales, int B, int K, int N, uint32_t k65536, int trigger_first)
 {
-    // kslice is a multiple of 64 that divides K: every warp owns kslice / 8 rows, a whole number of batches
+    // the K / 64 units of 64 rows are dealt to gridDim.y slices as evenly as they go: every warp owns kslice / 8 rows, a
+    // whole number of batches
+    const int units = K / 64, ubase = units / gridDim.y, urem = units % gridDim.y, y_ = blockIdx.y;
+    const int kslice = 64 * (ubase + (y_ < urem)), k0 = 64 * (y_ * ubase + (y_ < urem ? y_ : urem));
     constexpr int WPL = CPL / 8, CW = 32 * CPL;
     extern __shared__ float gsm[];                       // activations [BT][kslice]; later the reduction tree [4][BT][CW]
     __shared__ int s_last;
@@ -222,12 +225,14 @@ __global__ void __launch_bounds__(256, BT <= 2 ? 3 : 2) k_gemv_stream(void *Y, i
     int n0 = blockIdx.x * CW + lane * CPL;
     const bool live = n0 < N;
     if (!live) n0 = N - CPL;                             // lanes past the last column repeat valid loads and store nothing
-    const int k0 = blockIdx.y * kslice;
     const size_t cstep = (size_t)8 * (N / 2), sstep = (size_t)8 * (N / 128);
     const uint8_t *cp = codes + (size_t)(k0 + warp) * (N / 2) + n0 / 2;
     const float *sp = scales + (size_t)(k0 + warp) * (N / 128) + n0 / 128;
-    uint32_t w[2][U][WPL];
-    float sc[2][U];
+    // NB batches of U rows in flight per warp.  With two, every half round waited for the loads issued half a round before:
+    // 4096 x 16384, one row, 17.2 us against 13.2 (with the late trigger below).
+    constexpr int NB = BT <= 2 ? 4 : 3;
+    uint32_t w[NB][U][WPL];
+    float sc[NB][U];
     auto fetch = [&](int buf) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
@@ -237,10 +242,16 @@ __global__ void __launch_bounds__(256, BT <= 2 ? 3 : 2) k_gemv_stream(void *Y, i
             cp += cstep; sp += sstep;
         }
     };
-    fetch(0);                                            // the weights do not depend on the activations: request them first
+    const int nbatch = kslice / (8 * U);
+#pragma unroll
+    for (int i = 0; i < NB - 1; i++)                     // the weights do not depend on the activations: request them first
+        if (i < nbatch) fetch(i);
     // a kernel that writes codes never lets the next one start early, so they are complete here; what follows waits
     pdl_wait();
-    pdl_trigger();
+    // The next kernel may start at once where this one leaves SMs idle.  Otherwise its blocks would sit in slots that this
+    // one's loads need (65.5 -> 71.7 us for four 4096 x 16384): it may start once the weights have been read, and its launch
+    // and its first loads fall into this kernel's reduction.
+    if (trigger_first) pdl_trigger();
     for (int i = threadIdx.x; i < BT * kslice; i += 256) {
         const int b = i / kslice, k = k0 + i % kslice;
         gsm[i] = b < B ? ld_x(X, dtype, (size_t)b * K + k) : 0.0f;
@@ -277,12 +288,15 @@ __global__ void __launch_bounds__(256, BT <= 2 ? 3 : 2) k_gemv_stream(void *Y, i
         }
         xr += 8 * U;
     };
-    for (int r = 0; r < kslice / 8; r += 2 * U) {        // two batches per round: the buffer indices stay compile-time constants
-        fetch(1);
-        use(0);
-        if (r + 2 * U < kslice / 8) fetch(0);
-        use(1);
+    for (int r = 0; r < nbatch; r += NB) {               // NB batches per round: the buffer indices stay compile-time constants
+#pragma unroll
+        for (int i = 0; i < NB; i++) {
+            if (r + i >= nbatch) break;
+            if (r + i + NB - 1 < nbatch) fetch((i + NB - 1) % NB);
+            use(i);
+        }
     }
+    if (!trigger_first) pdl_trigger();
     float y[BT][CPL];
 #pragma unroll
     for (int b = 0; b < BT; b++)
@@ -342,8 +356,25 @@ __global__ void __launch_bounds__(256, BT <= 2 ? 3 : 2) k_gemv_stream(void *Y, i
     for (int i = threadIdx.x; i < BT * CW; i += 256) {
         const int b = i / CW, n = blockIdx.x * CW + i % CW;
         if (b < B && n < N) {
+            // slices ascending, eight loads in flight (one after the other they took most of the kernel's last 5 us)
+            const float *pp = part + (size_t)b * N + n;
+            const size_t ps = (size_t)B * N;
             float v = 0.0f;
-            for (int s = 0; s < nslice; s++) v += __ldcg(part + ((size_t)s * B + b) * N + n);
+            int s = 0;
+            for (; s + 8 <= nslice; s += 8) {
+                float x[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) x[k] = __ldcg(pp + (s + k) * ps);
+#pragma unroll
+                for (int k = 0; k < 8; k++) v += x[k];
+            }
+            if (s < nslice) {
+                float x[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) x[k] = s + k < nslice ? __ldcg(pp + (s + k) * ps) : 0.0f;
+#pragma unroll
+                for (int k = 0; k < 8; k++) v += x[k];
+            }
             if (dtype == QLMB_BF16) ((bf16 *)Y)[(size_t)b * N + n] = __float2bfloat16_rn(v);
             else ((float *)Y)[(size_t)b * N + n] = v;
         }
@@ -576,7 +607,7 @@ template <> struct VecOfF<4> { typedef float4 T; };
 // NW warps per block: eight (512 columns), or four (256) where the last block of eight would be at most half full (N = 768:
 // a quarter of the warps would repeat columns).
 template <int MT, int NW>
-__global__ void __launch_bounds__(32 * NW, MT == 1 ? (NW == 8 ? 3 : 4) : (NW == 8 ? 1 : 3)) k_gemv_mma(const __grid_constant__ Rows8 a)
+__global__ void __launch_bounds__(32 * NW, MT == 1 ? 16 / NW : (NW == 8 ? 1 : 3)) k_gemv_mma(const __grid_constant__ Rows8 a)
 {
     constexpr int GR = 16 * MT, CW = 64 * NW, PADK = 8, NT = 32 * NW, NG = NW / 2;
     extern __shared__ __align__(16) uint8_t msm[];       // activations bf16 [GR][kslice + PADK], then scales [kslice][NG]
@@ -787,7 +818,7 @@ static MmaPlan mma_plan(int K, int N, int nz, int mt)
     p.nw = (N % 512) && (N % 512) <= 256 ? 4 : 8;
     p.nb = (N + 64 * p.nw - 1) / (64 * p.nw);
     const int units = K / 64, kmax = mt == 1 ? 1024 : 512;
-    const int slots = sm_count() * (mt == 1 ? (p.nw == 8 ? 3 : 4) : (p.nw == 8 ? 1 : 3));
+    const int slots = sm_count() * (mt == 1 ? 16 / p.nw : (p.nw == 8 ? 1 : 3));
     long long best = -1;
     p.ns = units;
     for (int d = 1; d <= units; d++) {
@@ -1164,16 +1195,23 @@ static int gemv_decode_impl(void *Y, const void *X, const int8_t *codes, const f
         const int cpl = N >= 8192 ? 16 : 8, cw = 32 * cpl;
         const int nb = (N + cw - 1) / cw;
         QLMB_REQUIRE(nb <= 2048, "qlmb_gemv_decode: N=%d", N);
-        // K slices: a divisor of K / 64 (slices are whole multiples of 64 rows), about three blocks per SM in total
-        const int units = K / 64;
-        // (measured at 4096 x 16384, one row: 3 blocks per SM in total 14.3 us, 6: 16.4 us, 12: 18.6 us -- the staging,
-        // the warp tree and the ticket are a fixed cost per block; a ring of bulk copies per row into shared memory
-        // instead of register prefetch was slower, 29 us)
-        int want = (3 * sm_count() + nb / 2) / nb, ns = 1;
-        for (int d = 1; d <= units; d++)
-            if (units % d == 0 && d <= want && (size_t)bt * (K / d) * sizeof(float) <= 64 * 1024) ns = d;
-        while ((size_t)bt * (K / ns) * sizeof(float) > 64 * 1024 && ns < units) { ns++; while (units % ns) ns++; }
-        const int ksl = K / ns;
+        // K slices of whole 64-row units, as even as they go, in one round of up to three blocks per SM (two with four
+        // rows): of those the count for which an SM's share of units, with a third of a unit per block for staging and the
+        // reduction, is the smallest; one or two blocks alone do not cover the latency of their loads.  (4096 x 16384, one
+        // row, 32 column blocks: 8 equal slices, 256 blocks, took 16.4 us, now 13.2 with what follows.  A ring of
+        // bulk copies per row into shared memory instead of register prefetch was slower, 29 us.)
+        const int units = K / 64, most = 2;
+        int ns = 0;
+        float best = 0.0f;
+        for (int d = 1; d <= units; d++) {
+            const int per_sm = (nb * d + sm_count() - 1) / sm_count(), umax = (units + d - 1) / d;
+            if ((size_t)bt * umax * 64 * sizeof(float) > 64 * 1024) continue;
+            if (ns && per_sm > most) break;
+            const int rounds = (per_sm + most - 1) / most;
+            const float cost = per_sm * (umax + 0.33f) * (per_sm == 1 ? 1.2f : 1.0f) + (rounds - 1) * 2.0f;
+            if (!ns || cost < best) { best = cost; ns = d; }
+        }
+        const int ksl = (units + ns - 1) / ns * 64;
         void *ws2 = nullptr;
         int rc2 = workspace((size_t)ns * B * N * sizeof(float), &ws2);
         if (rc2) return rc2;
@@ -1184,7 +1222,7 @@ static int gemv_decode_impl(void *Y, const void *X, const int8_t *codes, const f
         do { \
             static bool attr_done[64]; int dv = 0; QLMB_CUDA(cudaGetDevice(&dv)); \
             if (dv >= 0 && dv < 64 && !attr_done[dv]) { QLMB_CUDA(cudaFuncSetAttribute(k_gemv_stream<BT_, CPL_>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024)); attr_done[dv] = true; } \
-            QLMB_CUDA(pdl_launch((int)(g.x * g.y) <= sm_count(), k_gemv_stream<BT_, CPL_>, g, dim3(256), sm_b, st, Y, dtype, (float *)ws2, X, (const uint8_t *)codes, scales, B, K, N, ksl, 65536u)); \
+            QLMB_CUDA(pdl_launch(true, k_gemv_stream<BT_, CPL_>, g, dim3(256), sm_b, st, Y, dtype, (float *)ws2, X, (const uint8_t *)codes, scales, B, K, N, 65536u, (int)((int)(g.x * g.y) <= sm_count()))); \
         } while (0)
         if (cpl == 16) { if (bt == 1) GS_LAUNCH(1, 16); else if (bt == 2) GS_LAUNCH(2, 16); else GS_LAUNCH(4, 16); }
         else { if (bt == 1) GS_LAUNCH(1, 8); else if (bt == 2) GS_LAUNCH(2, 8); else GS_LAUNCH(4, 8); }
