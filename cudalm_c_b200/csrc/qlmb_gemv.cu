@@ -862,12 +862,112 @@ static int mma_launch(Rows8 a, int nz, const MmaPlan &pl, int mt, cudaStream_t s
 
 // ---- codes W[N][K] (groups along K).  A warp owns 4 consecutive output columns (rows of W) and a
 // K slice; lanes stride over the code words of the slice, 4 words (one per column) per step share the
-// activation values; the scale multiplies the 8-element partial dot product of each word.
+// activation values; the scale multiplies the 8-element partial dot product of each word.  NB steps are in flight, the
+// first of them requested before the activations are staged (16 bytes at a time): with two, and one activation after the
+// other, 4096 x 16384 took 31 us for one row, now 21.7.  A single slice writes Y itself.
 template <int BT>
-__global__ void __launch_bounds__(256, BT <= 2 ? 4 : 2) k_gemv_nk(float *part, const void *X, int dtype, const uint8_t *codes,
+__global__ void __launch_bounds__(256, BT == 1 ? 4 : BT == 2 ? 3 : 2) k_gemv_nk(void *Y, float *part, const void *X, int dtype, const uint8_t *codes,
                                                  const float *scales, int B, int K, int N, int kslice)
 {
-    extern __shared__ float xs[];               // [BT][kslice]
+    extern __shared__ __align__(16) float xs[];  // [BT][kslice]
+    constexpr int NB = BT <= 2 ? 3 : 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = (blockIdx.x * 8 + warp) * 4;
+    const int k0 = blockIdx.y * kslice, k1 = k0 + kslice < K ? k0 + kslice : K;
+    const int gpr = K / 128, nw = (k1 - k0) / 8;             // code words of the slice
+    const bool live = n0 < N;                                // N is a multiple of 128: all four columns or none
+    const uint8_t *cp = codes + ((size_t)(live ? n0 : 0) * K + k0) / 2;
+    const float *sp = scales + (size_t)(live ? n0 : 0) * gpr + k0 / 128;
+    uint32_t w[NB][4];
+    float sc[NB][4];
+    auto fetch = [&](int buf, int kw) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            w[buf][c] = kw < nw ? __ldcs(reinterpret_cast<const uint32_t *>(cp + (size_t)c * (K / 2)) + kw) : 0u;
+            sc[buf][c] = kw < nw ? __ldg(sp + c * gpr + kw / 16) : 0.0f;
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < NB - 1; i++) fetch(i, lane + 32 * i);
+    pdl_wait();                                              // the codes are no running kernel's output, the rows are
+    // B <= BT
+    if (dtype == QLMB_BF16) {
+        for (int i = threadIdx.x; i < BT * (kslice / 8); i += 256) {
+            const int b = i / (kslice / 8), k = (i % (kslice / 8)) * 8;
+            float4 lo = make_float4(0, 0, 0, 0), hi = lo;
+            if (b < B && k0 + k < k1) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4 *>((const bf16 *)X + (size_t)b * K + k0 + k));
+                lo = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+                hi = make_float4(__uint_as_float(v.z << 16), __uint_as_float(v.z & 0xffff0000u), __uint_as_float(v.w << 16), __uint_as_float(v.w & 0xffff0000u));
+            }
+            float4 *d = reinterpret_cast<float4 *>(xs + b * kslice + k);
+            d[0] = lo; d[1] = hi;
+        }
+    } else {
+        for (int i = threadIdx.x; i < BT * (kslice / 4); i += 256) {
+            const int b = i / (kslice / 4), k = (i % (kslice / 4)) * 4;
+            float4 v = make_float4(0, 0, 0, 0);
+            if (b < B && k0 + k < k1) v = __ldg(reinterpret_cast<const float4 *>((const float *)X + (size_t)b * K + k0 + k));
+            *reinterpret_cast<float4 *>(xs + b * kslice + k) = v;
+        }
+    }
+    __syncthreads();
+    if (!live) return;
+    float acc[4][BT];
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+#pragma unroll
+        for (int b = 0; b < BT; b++) acc[c][b] = 0.0f;
+    for (int r = lane; r < nw; r += 32 * NB) {
+#pragma unroll
+        for (int i = 0; i < NB; i++) {
+            const int kw = r + 32 * i;
+            fetch((i + NB - 1) % NB, kw + 32 * (NB - 1));
+            if (kw >= nw) break;
+            float d[4][8];
+#pragma unroll
+            for (int c = 0; c < 4; c++) unpack8(w[i][c], d[c]);
+#pragma unroll
+            for (int b = 0; b < BT; b++) {
+                const float4 x0 = *reinterpret_cast<const float4 *>(&xs[b * kslice + kw * 8]);
+                const float4 x1 = *reinterpret_cast<const float4 *>(&xs[b * kslice + kw * 8 + 4]);
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const float t = x0.x * d[c][0] + x0.y * d[c][1] + x0.z * d[c][2] + x0.w * d[c][3] +
+                                    x1.x * d[c][4] + x1.y * d[c][5] + x1.z * d[c][6] + x1.w * d[c][7];
+                    acc[c][b] += sc[i][c] * t;
+                }
+            }
+        }
+    }
+    pdl_trigger();                                       // the weights have been read
+    const bool direct_bf = gridDim.y == 1 && dtype == QLMB_BF16;
+    float *const dst = gridDim.y > 1 ? part + (size_t)blockIdx.y * B * N : (float *)Y;
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+#pragma unroll
+        for (int b = 0; b < BT; b++) {
+            float v = acc[c][b];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0 && b < B) {
+                const size_t o = (size_t)b * N + n0 + c;
+                if (direct_bf) ((bf16 *)Y)[o] = __float2bfloat16_rn(v);
+                else dst[o] = v;
+            }
+        }
+}
+
+// The same for more than four rows, eight per pass over the slice: their accumulators leave no registers for a step ahead,
+// and with the wider staging above it was slower (30 fp32 rows against 2048 x 2048: 35 us, this form 31).
+__global__ void __launch_bounds__(256, 2) k_gemv_nk8(float *part, const void *X, int dtype, const uint8_t *codes,
+                                                 const float *scales, int B, int K, int N, int kslice)
+{
+    constexpr int BT = 8;
+    extern __shared__ float xs8[];              // [BT][kslice]
+    float *xs = xs8;
+    pdl_wait();
+    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = (blockIdx.x * 8 + warp) * 4;
     const int k0 = blockIdx.y * kslice, k1 = k0 + kslice < K ? k0 + kslice : K;
@@ -1187,7 +1287,8 @@ static int gemv_decode_impl(void *Y, const void *X, const int8_t *codes, const f
     }
     if (!fr && B > 4 && dtype == QLMB_BF16 && (K % 64) == 0)
         return qlmb_linear_fwd(Y, X, codes, scales, layout, B, K, N, nullptr, dtype, stream);
-    const int bt = B <= 1 ? 1 : B <= 2 ? 2 : B <= 4 ? 4 : 8;
+    // (rows at an odd address: the eight-row form of the [N][K] kernel reads them element by element)
+    const int bt = layout == QLMB_NK && ((uintptr_t)X & 15) ? 8 : B <= 1 ? 1 : B <= 2 ? 2 : B <= 4 ? 4 : 8;
     static int stream_on = -1;
     if (stream_on < 0) { const char *e = getenv("QLMB_GEMV_STREAM"); stream_on = (e && atoi(e) == 0) ? 0 : 1; }
     if (stream_on && !fr && layout == QLMB_KN && bt <= 4) {
@@ -1234,7 +1335,7 @@ static int gemv_decode_impl(void *Y, const void *X, const int8_t *codes, const f
     // a multiple of 8 rows, and small enough for the activation tile in shared memory
     const int nblk = layout == QLMB_KN ? (N + 255) / 256 : (N + 31) / 32;
     // K slices for 4 (bt <= 2) or 2 blocks per SM
-    int nslice = ((bt <= 2 ? 4 : 2) * sm_count()) / nblk;
+    int nslice = ((bt == 1 || (bt == 2 && layout == QLMB_KN) ? 4 : bt == 2 ? 3 : 2) * sm_count()) / nblk;
     if (nslice > K / 64) nslice = K / 64;
     if (nslice < 1) nslice = 1;
     int kslice = ((K + nslice - 1) / nslice + 127) / 128 * 128;
@@ -1246,13 +1347,8 @@ static int gemv_decode_impl(void *Y, const void *X, const int8_t *codes, const f
     float *part = (float *)ws;
     const size_t smem = (size_t)bt * kslice * sizeof(float);
     const dim3 grid(nblk, nslice);
-#define GV_LAUNCH(KERN) \
-    do { \
-        if (bt == 1) KERN<1><<<grid, 256, smem, st>>>(part, X, dtype, (const uint8_t *)codes, scales, B, K, N, kslice); \
-        else if (bt == 2) KERN<2><<<grid, 256, smem, st>>>(part, X, dtype, (const uint8_t *)codes, scales, B, K, N, kslice); \
-        else if (bt == 4) KERN<4><<<grid, 256, smem, st>>>(part, X, dtype, (const uint8_t *)codes, scales, B, K, N, kslice); \
-        else KERN<8><<<grid, 256, smem, st>>>(part, X, dtype, (const uint8_t *)codes, scales, B, K, N, kslice); \
-    } while (0)
+#define GV_LAUNCH(BT_) \
+    QLMB_CUDA(pdl_launch(true, k_gemv_nk<BT_>, grid, dim3(256), smem, st, Y, part, X, dtype, (const uint8_t *)codes, scales, B, K, N, kslice))
     if (layout == QLMB_KN && bt == 1 && (size_t)nblk * nslice <= (size_t)2 * sm_count())
         launch_kn<1, 4>(B > 4, grid, smem, st, part, X, dtype, (const uint8_t *)codes, scales, B, K, N, kslice);
     else if (layout == QLMB_KN) {
@@ -1261,7 +1357,11 @@ static int gemv_decode_impl(void *Y, const void *X, const int8_t *codes, const f
         else if (bt == 4) launch_kn<4, 2>(B > 4, grid, smem, st, part, X, dtype, (const uint8_t *)codes, scales, B, K, N, kslice);
         else launch_kn<8, 2>(B > 4, grid, smem, st, part, X, dtype, (const uint8_t *)codes, scales, B, K, N, kslice);
     }
-    else GV_LAUNCH(k_gemv_nk);
+    else {
+        if (bt == 1) GV_LAUNCH(1); else if (bt == 2) GV_LAUNCH(2); else if (bt == 4) GV_LAUNCH(4);
+        else QLMB_CUDA(pdl_launch(true, k_gemv_nk8, grid, dim3(256), smem, st, part, X, dtype, (const uint8_t *)codes, scales, B, K, N, kslice));
+        if (nslice == 1 && bt <= 4 && !fr) { QLMB_LAUNCH_CHECK("k_gemv_nk"); return QLMB_OK; }
+    }
 #undef GV_LAUNCH
     if (fr) pdl_launch(B > 4, k_gemv_finish_res_norm, dim3(B), dim3(256), 0, st, (bf16 *)Y, (bf16 *)fr->Fn, part, nslice, B, N, (const bf16 *)fr->res, fr->gamma);
     else pdl_launch(B > 4, k_gemv_finish, dim3((unsigned)(((size_t)B * N + 255) / 256)), dim3(256), 0, st, Y, dtype, part, nslice, (size_t)B * N);

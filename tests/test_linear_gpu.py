@@ -165,6 +165,26 @@ def test_gemv_decode(cuda, oracle, B):
     assert rel(linear.gemv_decode(X, Q.d, Q.s, KN, 384), dev(Yo, cuda)) < 1e-5
 
 
+@pytest.mark.parametrize("B", [1, 2, 3, 4, 5, 16, 17, 33])
+def test_gemv_decode_edges(cuda, B):
+    """K slices of unequal length, widths that end inside a column block, the smallest shape, and rows that start at an
+    address no vector load can take."""
+    from cudalm_c_b200 import linear
+    from cudalm_c_b200._lib import KN, NK
+    for K, N in ((128, 128), (1664, 8320), (896, 2432), (640, 768)):
+        for lay in (KN, NK):
+            Q, W = quantise(cuda, K, N, 21) if lay == KN else quantise(cuda, N, K, 21)
+            Wm = W if lay == KN else W.T
+            for dt in (torch.float32, torch.bfloat16):
+                X = torch.randn(B, K, device=cuda).to(dt)
+                ref = X.float() @ Wm
+                tol = 3e-5 if dt == torch.float32 else 8e-3
+                assert rel(linear.gemv_decode(X, Q.d, Q.s, lay, N), ref) < tol, (K, N, lay, dt)
+                if B <= 4:
+                    odd = torch.empty(B * K + 1, device=cuda, dtype=dt)[1:].view(B, K).copy_(X)
+                    assert rel(linear.gemv_decode(odd, Q.d, Q.s, lay, N), ref) < tol, (K, N, lay, dt)
+
+
 def test_gemv_rejects_more_than_64_slots(cuda):
     import cudalm_c_b200 as q
     from cudalm_c_b200 import linear

@@ -44,6 +44,18 @@ def test_router_logits_fused(cuda, oracle):
         assert (rp.cpu().numpy() == rp2).all() and (asg.cpu().numpy() == asg2).all() and (gt.cpu().numpy() == gt2).all()
 
 
+@pytest.mark.parametrize("N", [1, 7, 9, 333, 4737])
+def test_router_logits_of_few_tokens_equal_the_tiled_ones(cuda, N):
+    """The few-token kernel sums every logit in the tiled kernel's order: the rows of a short batch carry the bits they
+    have inside a long one."""
+    from cudalm_c_b200 import moe
+    for D, E in ((768, 32), (256, 8), (1024, 5)):
+        X = torch.randn(6000, D, device=cuda).bfloat16()
+        Wr = torch.randn(D, E, device=cuda) * 0.02
+        whole = moe.router_topk(X=X, Wr=Wr, K=1)[0]
+        assert torch.equal(moe.router_topk(X=X[:N], Wr=Wr, K=1)[0], whole[:N]), (D, E)
+
+
 @pytest.mark.parametrize("E,K", [(33, 2), (48, 3), (64, 8), (100, 2), (128, 1), (200, 4), (256, 8)])
 def test_router_topk_wide_matches_oracle(cuda, oracle, E, K):
     """More than 32 experts (one warp per token, several experts per lane): probabilities, choices and gates equal
