@@ -118,21 +118,46 @@ __global__ void __launch_bounds__(256) k_embed_bwd(float *G, const void *dout, i
 
 // ------------------------------------------------------------------ RMSNorm
 // O = X * rinv * gamma, rinv = 1/sqrt(mean(x^2) + 1e-5)  (k_rmsnorm, cpu_kern.h:103-109).  Warp per row.
-__global__ void __launch_bounds__(256) k_rmsnorm_fwd(void *O, int o_dtype, float *rinv, const void *X, int x_dtype,
-                                                     const float *gamma, int N, int D)
+template <int o_dtype, int x_dtype>
+__global__ void __launch_bounds__(256) k_rmsnorm_fwd(void *O, float *rinv, const void *X, const float *gamma, int N, int D)
 {
     pdl_wait();
     pdl_trigger();
     const int n = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (n >= N) return;
+    // rows of up to 1024 columns stay in registers; longer ones are read again for the second pass
+    constexpr int NV = 8;
+    float4 v[NV];
     float ss = 0.0f;
-    for (int j = lane * 4; j < D; j += 128) {
-        const float4 x = blk_ld4(X, x_dtype, (size_t)n * D + j);
-        ss += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+    if (D <= 128 * NV) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            const int j = lane * 4 + k * 128;
+            if (j < D) v[k] = blk_ld4(X, x_dtype, (size_t)n * D + j);
+        }
+#pragma unroll
+        for (int k = 0; k < NV; k++)
+            if (lane * 4 + k * 128 < D) ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+    } else {
+        for (int j = lane * 4; j < D; j += 128) {
+            const float4 x = blk_ld4(X, x_dtype, (size_t)n * D + j);
+            ss += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+        }
     }
     ss = warp_sum(ss);
     const float s = 1.0f / sqrtf(ss / (float)D + 1e-5f);
     if (lane == 0) rinv[n] = s;
+    if (D <= 128 * NV) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            const int j = lane * 4 + k * 128;
+            if (j < D) {
+                const float4 x = v[k], g = __ldg(reinterpret_cast<const float4 *>(gamma + j));
+                blk_st4(O, o_dtype, (size_t)n * D + j, make_float4(x.x * s * g.x, x.y * s * g.y, x.z * s * g.z, x.w * s * g.w));
+            }
+        }
+        return;
+    }
     for (int j = lane * 4; j < D; j += 128) {
         const float4 x = blk_ld4(X, x_dtype, (size_t)n * D + j);
         const float4 g = *reinterpret_cast<const float4 *>(gamma + j);
@@ -203,6 +228,84 @@ __global__ void __launch_bounds__(128) k_gamma_sum(float *G, const float *part, 
     for (int c = 0; c < GAMMA_CH; c++) a += part[(size_t)c * D + j];
     G[j] += a;
 }
+// Both at once for rows of up to 128 * NV columns: block c owns the rows of chunk c, warp w its rows r0 + w, r0 + w + 16,
+// ..., each read once, all of it in flight; a lane adds the gain terms of its columns over the warp's rows, the warps' sums
+// are added in order.  As two kernels 8192 x 768 bf16 took 18 + 11 us, the inputs read three times; together 14.7.
+// (The types are template arguments: with a run-time choice per load the loads no longer overlap, 37 us.)
+template <int NV, int DXT, int XT, int DYT>
+__global__ void __launch_bounds__(512) k_rmsnorm_bwd_gamma(void *dx, int accumulate, float *part, const void *X, const float *gamma,
+                                                           const float *rinv, const void *dy, int N, int D)
+{
+    extern __shared__ __align__(16) float gsum[];        // [16][D]
+    pdl_wait();
+    pdl_trigger();
+    const int c = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r0 = (int)((long long)N * c / GAMMA_CH), r1 = (int)((long long)N * (c + 1) / GAMMA_CH);
+    float4 acc[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) acc[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int n = r0 + warp; n < r1; n += 16) {
+        float4 x[NV], d[NV], q[NV];
+        const size_t o = (size_t)n * D;
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            const int j = lane * 4 + k * 128;
+            if (j < D) {
+                x[k] = blk_ld4(X, XT, o + j); d[k] = blk_ld4(dy, DYT, o + j);
+                if (accumulate) q[k] = blk_ld4(dx, DXT, o + j);
+            }
+        }
+        const float s = __ldg(rinv + n);
+        float t = 0.0f;
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            const int j = lane * 4 + k * 128;
+            if (j < D) {
+                const float4 g = __ldg(reinterpret_cast<const float4 *>(gamma + j));
+                t += x[k].x * g.x * d[k].x + x[k].y * g.y * d[k].y + x[k].z * g.z * d[k].z + x[k].w * g.w * d[k].w;
+                acc[k].x += x[k].x * s * d[k].x; acc[k].y += x[k].y * s * d[k].y; acc[k].z += x[k].z * s * d[k].z; acc[k].w += x[k].w * s * d[k].w;
+            }
+        }
+        t = warp_sum(t);
+        const float cf = s * s * s / (float)D * t;
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            const int j = lane * 4 + k * 128;
+            if (j < D) {
+                const float4 g = __ldg(reinterpret_cast<const float4 *>(gamma + j));
+                float4 r = make_float4(s * g.x * d[k].x - cf * x[k].x, s * g.y * d[k].y - cf * x[k].y, s * g.z * d[k].z - cf * x[k].z, s * g.w * d[k].w - cf * x[k].w);
+                if (accumulate) { r.x += q[k].x; r.y += q[k].y; r.z += q[k].z; r.w += q[k].w; }
+                blk_st4(dx, DXT, o + j, r);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        const int j = lane * 4 + k * 128;
+        if (j < D) *reinterpret_cast<float4 *>(gsum + warp * D + j) = acc[k];
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < D; j += 512) {
+        float a = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 16; w++) a += gsum[w * D + j];
+        part[(size_t)c * D + j] = a;
+    }
+}
+template <int NV, int DXT, int XT, int DYT>
+static int launch_bwd_gamma(void *dx, int accumulate, float *part, const void *X, const float *gamma, const float *rinv, const void *dy,
+                            int N, int D, cudaStream_t st)
+{
+    static bool done[64];
+    int dev = 0;
+    QLMB_CUDA(cudaGetDevice(&dev));
+    QLMB_REQUIRE(dev >= 0 && dev < 64, "device index %d", dev);
+    auto kern = k_rmsnorm_bwd_gamma<NV, DXT, XT, DYT>;
+    if (!done[dev]) { QLMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024)); done[dev] = true; }
+    QLMB_CUDA(pdl_launch(true, kern, dim3(GAMMA_CH), dim3(512), (size_t)16 * D * sizeof(float), st, dx, accumulate, part, X, gamma, rinv, dy, N, D));
+    return QLMB_OK;
+}
+
 // ------------------------------------------------------------------ rotary embedding
 // In place on buf[N, nh, hd]; position of row n is n % T; pairs (i, i + hd/2)  (k_rope, cpu_kern.h:139-152).
 __global__ void __launch_bounds__(256) k_rope(void *buf, int dtype, const float *cosb, const float *sinb, size_t total, int nh,
@@ -224,7 +327,8 @@ __global__ void __launch_bounds__(256) k_rope(void *buf, int dtype, const float 
 }
 
 // hd/2 a multiple of 8: a thread rotates 8 consecutive pairs with 16-byte accesses
-__global__ void __launch_bounds__(256) k_rope8(void *buf, int dtype, const float *cosb, const float *sinb, size_t total, int nh,
+template <int dtype>                                     // a run-time type per load keeps the loads from overlapping
+__global__ void __launch_bounds__(256) k_rope8(void *buf, const float *cosb, const float *sinb, size_t total, int nh,
                                                int hd, int T, int back)
 {
     pdl_wait();
@@ -753,7 +857,9 @@ extern "C" int qlmb_rmsnorm_fwd(void *O, int o_dtype, float *rinv, const void *X
     QLMB_REQUIRE(O && rinv && X && gamma && dtype_ok(o_dtype) && dtype_ok(x_dtype), "qlmb_rmsnorm_fwd: bad argument");
     QLMB_REQUIRE(D > 0 && D % 4 == 0 && ((uintptr_t)gamma & 15) == 0, "qlmb_rmsnorm_fwd: D %d must be a multiple of 4, gamma 16-byte aligned", D);
     if (N <= 0) return QLMB_OK;
-    QLMB_CUDA(pdl_launch(true, k_rmsnorm_fwd, dim3((N + 7) / 8), dim3(256), 0, as_stream(stream), O, o_dtype, rinv, X, x_dtype, gamma, N, D));
+    auto kern = o_dtype == QLMB_BF16 ? (x_dtype == QLMB_BF16 ? k_rmsnorm_fwd<QLMB_BF16, QLMB_BF16> : k_rmsnorm_fwd<QLMB_BF16, QLMB_F32>)
+                                     : (x_dtype == QLMB_BF16 ? k_rmsnorm_fwd<QLMB_F32, QLMB_BF16> : k_rmsnorm_fwd<QLMB_F32, QLMB_F32>);
+    QLMB_CUDA(pdl_launch(true, kern, dim3((N + 7) / 8), dim3(256), 0, as_stream(stream), O, rinv, X, gamma, N, D));
     QLMB_LAUNCH_CHECK("k_rmsnorm_fwd");
     return QLMB_OK;
 }
@@ -767,6 +873,16 @@ extern "C" int qlmb_rmsnorm_bwd(void *dx, int dx_dtype, int accumulate, float *d
     QLMB_REQUIRE(!dgamma || part, "qlmb_rmsnorm_bwd: the gain gradient needs the 128 x D scratch");
     if (N <= 0) return QLMB_OK;
     cudaStream_t st = as_stream(stream);
+    // one pass where the gain gradient is wanted, a bf16 row of up to 768 columns stays in a warp's registers and the 128
+    // chunks hold enough rows that their 16 warps are busy
+    if (dgamma && D <= 768 && N >= 16 * GAMMA_CH && dx_dtype == QLMB_BF16 && x_dtype == QLMB_BF16 && dy_dtype == QLMB_BF16) {
+        const int rc = D <= 512 ? launch_bwd_gamma<4, QLMB_BF16, QLMB_BF16, QLMB_BF16>(dx, accumulate, part, X, gamma, rinv, dy, N, D, st)
+                                : launch_bwd_gamma<6, QLMB_BF16, QLMB_BF16, QLMB_BF16>(dx, accumulate, part, X, gamma, rinv, dy, N, D, st);
+        if (rc) return rc;
+        QLMB_CUDA(pdl_launch(true, k_gamma_sum, dim3((D + 127) / 128), dim3(128), 0, st, dgamma, part, D));
+        QLMB_LAUNCH_CHECK("k_rmsnorm_bwd");
+        return QLMB_OK;
+    }
     QLMB_CUDA(pdl_launch(true, k_rmsnorm_bwd, dim3((N + 7) / 8), dim3(256), 0, st, dx, dx_dtype, accumulate, X, x_dtype, gamma, rinv, dy, dy_dtype, N, D));
     if (dgamma) {
         QLMB_CUDA(pdl_launch(true, k_gamma_part, dim3((D + 127) / 128, GAMMA_CH), dim3(128), 0, st, part, X, x_dtype, rinv, dy, dy_dtype, N, D));
@@ -784,7 +900,7 @@ extern "C" int qlmb_rope(void *buf, int dtype, const float *cosb, const float *s
     if (N <= 0) return QLMB_OK;
     if ((hd / 2) % 8 == 0 && (((uintptr_t)buf | (uintptr_t)cosb | (uintptr_t)sinb) & 15) == 0) {
         const size_t total = (size_t)N * nh * (hd / 16);
-        QLMB_CUDA(pdl_launch(true, k_rope8, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, as_stream(stream), buf, dtype, cosb, sinb, total, nh, hd, T, back));
+        QLMB_CUDA(pdl_launch(true, dtype == QLMB_BF16 ? k_rope8<QLMB_BF16> : k_rope8<QLMB_F32>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, as_stream(stream), buf, cosb, sinb, total, nh, hd, T, back));
     } else {
         const size_t total = (size_t)N * nh * (hd / 2);
         k_rope<<<(unsigned)((total + 255) / 256), 256, 0, as_stream(stream)>>>(buf, dtype, cosb, sinb, total, nh, hd, T, back);
