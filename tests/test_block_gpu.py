@@ -70,6 +70,42 @@ def test_rmsnorm(cuda, ref, dt):
     assert rel(dg.cpu().numpy(), dgr) < 1e-5
 
 
+@pytest.mark.parametrize("N,D", [(2047, 768), (2048, 768), (2051, 512), (4099, 640), (2048, 1024), (3000, 128)])
+def test_rmsnorm_backward_of_many_bf16_rows(cuda, N, D):
+    """Backward and gain gradient on both sides of the one-pass form's limits, against fp32 autograd."""
+    from cudalm_c_b200 import block
+    X = torch.randn(N, D, device=cuda).bfloat16(); dy = torch.randn(N, D, device=cuda).bfloat16()
+    gamma = 1.0 + 0.1 * torch.randn(D, device=cuda)
+    O, rinv = block.rmsnorm_fwd(X, gamma)
+    x, g = X.float().requires_grad_(), gamma.clone().requires_grad_()
+    y = x * torch.rsqrt((x * x).mean(1, keepdim=True) + 1e-5) * g
+    y.backward(dy.float())
+    assert rel(O.float().cpu().numpy(), y.detach().cpu().numpy()) < 1e-2
+    for acc in (False, True):
+        dx = torch.randn(N, D, device=cuda).bfloat16(); dg = torch.ones(D, device=cuda)
+        want = x.grad + (dx.float() if acc else 0.0)
+        block.rmsnorm_bwd(dx, X, gamma, rinv, dy, dgamma=dg, accumulate=acc)
+        assert rel(dx.float().cpu().numpy(), want.cpu().numpy()) < 1e-2
+        assert rel((dg - 1.0).cpu().numpy(), g.grad.cpu().numpy()) < 1e-4
+
+
+@pytest.mark.parametrize("V", [8, 1000, 2052, 16384, 16392])
+def test_softmax_ce_row_lengths(cuda, V):
+    """Both forms of the kernel: rows that fit the registers, rows that do not or start off a 16-byte boundary."""
+    from cudalm_c_b200 import block
+    lg = torch.randn(37, V, device=cuda) * 3.0
+    tgt = torch.randint(0, V, (37,), device=cuda, dtype=torch.int32); tgt[5] = -1; tgt[0] = V - 1; tgt[1] = 0
+    loss, dl = block.softmax_ce(lg, tgt, 36, dl_dtype=torch.float32)
+    keep = tgt >= 0
+    p = torch.softmax(lg, 1)
+    ref_loss = -torch.log(p[torch.arange(37, device=cuda)[keep], tgt[keep].long()] + 1e-12)
+    want = p.clone()
+    want[torch.arange(37, device=cuda)[keep], tgt[keep].long()] -= 1.0
+    want = want / 36.0 * keep[:, None]
+    assert rel(dl.cpu().numpy(), want.cpu().numpy()) < 1e-5
+    assert rel(loss[keep].cpu().numpy(), ref_loss.cpu().numpy()) < 1e-5 and float(loss[5]) == 0.0
+
+
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 def test_rope(cuda, ref, dt):
     from cudalm_c_b200 import block
