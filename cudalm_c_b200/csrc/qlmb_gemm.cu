@@ -245,8 +245,9 @@ __device__ __forceinline__ TileInfo decode_tile(const GemmParams &p, int tile, i
         t.e = tile / per;
         int r = tile % per;
         t.m0 = (r % p.tiles_m) * (MH * BM); t.n_t = r / p.tiles_m;
-        t.row0 = p.off[t.e];
-        t.ksteps = (p.off[t.e + 1] - p.off[t.e]) / BK;
+        // without a table: E equal slices of ksteps stages
+        t.row0 = p.off ? p.off[t.e] : t.e * p.ksteps * BK;
+        t.ksteps = p.off ? (p.off[t.e + 1] - p.off[t.e]) / BK : p.ksteps;
         t.halves = (t.m0 + BM < p.M) ? 2 : 1;
     }
     return t;

@@ -140,6 +140,21 @@ def test_empty_and_unsupported(cuda):
     q.check(q.lib().qlmb_check_device(None))
 
 
+@pytest.mark.parametrize("M", [1023, 1025, 2047, 4161, 8191])
+def test_linear_wgrad_of_ragged_row_slices(cuda, M):
+    """Rows that do not divide into the slices: the last slice ends early, or lies past the rows altogether."""
+    from cudalm_c_b200 import linear
+    from cudalm_c_b200._lib import KN, NK
+    for K, N in ((256, 256), (384, 640)):
+        X = torch.randn(M, K, device=cuda).bfloat16(); dY = torch.randn(M, N, device=cuda).bfloat16()
+        for lay in (KN, NK):
+            ref = X.float().T @ dY.float() if lay == KN else dY.float().T @ X.float()
+            dW = torch.zeros(K * N, device=cuda)
+            for beta in (0.0, 1.0):
+                linear.linear_wgrad(dW, dY, X, lay, beta=beta)
+                assert rel(dW.view(ref.shape), ref * (1.0 + beta)) < 1e-4, (K, N, lay, beta)
+
+
 @pytest.mark.parametrize("B", [1, 8, 64])
 def test_gemv_decode(cuda, oracle, B):
     """Decode path (M = live slots <= 64).  fp32 activations: fp32 accumulation of exact dequantised weights (the
