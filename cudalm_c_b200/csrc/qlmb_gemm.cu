@@ -919,14 +919,15 @@ static int launch_pair(const GemmParams &p, long long total, cudaStream_t st, bo
     return launch_pair_g<BMODE, EPI, SCHED, 2>(p, total, st, early);     // two dequant stage groups
 }
 
-// The two-SM form needs whole 256-column tiles (128 activation columns with the SwiGLU
-// epilogue); QLMB_GEMM_PAIR=0 forces the one-SM form.
+// The two-SM form takes 256-column tiles (128 activation columns with the SwiGLU epilogue); the last one may be half full.
+// It is the faster one even then, except for a single half tile: there the one-SM form's 128 columns are exact.
+// QLMB_GEMM_PAIR=0 forces the one-SM form.
 static bool use_pair(const GemmLaunch &g)
 {
     static int enabled = -1;
     if (enabled < 0) { const char *e = getenv("QLMB_GEMM_PAIR"); enabled = (e && atoi(e) == 0) ? 0 : 1; }
     if (!enabled) return false;
-    return g.epi == EPI_SWIGLU ? (g.N % 128 == 0) : (g.N % 256 == 0);
+    return g.N % 128 == 0 && (g.epi == EPI_SWIGLU || g.N >= 256);
 }
 
 int gemm_launch(const GemmLaunch &g, cudaStream_t st)
@@ -941,7 +942,7 @@ int gemm_launch(const GemmLaunch &g, cudaStream_t st)
     memset(&p, 0, sizeof p);
     p.nseg = g.nseg; p.ksteps = g.ksteps; p.M = g.M; p.N = g.N; p.E = g.E;
     p.tiles_m = (g.M + MH * BM - 1) / (MH * BM);
-    p.tiles_n = pair ? (dual ? g.N / 128 : g.N / 256) : (dual ? g.N / (BN / 2) : g.N / BN);
+    p.tiles_n = pair ? (dual ? g.N / 128 : (g.N + 255) / 256) : (dual ? g.N / (BN / 2) : g.N / BN);
     p.w_rows = g.w_rows; p.w_cols = g.w_cols;
     p.tile_info = g.tile_info; p.ntiles_dev = g.ntiles_dev; p.off = g.off;
     p.out = g.out; p.out_dtype = g.out_dtype; p.ldo = g.ldo; p.resid = g.resid; p.beta = g.beta;

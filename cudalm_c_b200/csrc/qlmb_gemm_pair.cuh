@@ -294,6 +294,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
             else { long long left = (long long)p.M - row0; valid = left < 0 ? 0 : (left < 32 ? (int)left : 32); }
             const long long rbase = (SCHED == SCHED_GROUPK) ? ((long long)t.e * p.M + row0) : row0;
             const long long col0 = (EPI == EPI_SWIGLU) ? (long long)t.n_t * 128 + h * 64 : (long long)t.n_t * P_BN + h * 128;
+            if (EPI != EPI_SWIGLU && col0 >= p.N) valid = 0;     // the half of a last tile that lies past the columns
             if (valid > 0) epilogue_prefetch<EPI>(p, stage, ec, lane, rbase, col0, valid);
             ok = mbar_wait_idle(smem_u32(&tmem_full[acc]), ((uint32_t)it >> 1) & 1u, abort_flag, p.errword, 19);
             if (!ok) break;
@@ -353,10 +354,12 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
             for (int seg = 0; ok && seg < p.nseg; seg++) {
                 int ks = (g - kc % DQG + DQG) % DQG;                 // first stage of this group in the tile
                 for (int i = 0; i < ks && i < t.ksteps; i++) rb.next(NS);
-                // one stage on is BK rows (codes [K][N]) or half a group (codes [N][K]) on
+                // one stage on is BK rows (codes [K][N]) or half a group (codes [N][K]) on; a half that lies past the
+                // columns expands zeros or the next matrix's codes with the scales of the half before it, for nobody
+                const int xs = t.n_t * P_BN + my_n < p.N ? t.n_t * P_BN + my_n : t.n_t * P_BN;
                 const float *sp = p.scales[DUAL ? (int)rank : seg]
-                    + (BMODE == B_DEQ_MN ? (t.e * p.w_rows + srow) * gpr + (DUAL ? t.n_t : (t.n_t * P_BN + my_n) / 128)
-                                         : (t.e * p.w_rows + t.n_t * P_BN + my_n + srow) * gpr);
+                    + (BMODE == B_DEQ_MN ? (t.e * p.w_rows + srow) * gpr + (DUAL ? t.n_t : xs / 128)
+                                         : (t.e * p.w_rows + xs + srow) * gpr);
                 const int sstep = BMODE == B_DEQ_MN ? BK * gpr : 0;
                 auto scale_at = [&](int k) { return __ldg(sp + (BMODE == B_DEQ_MN ? k * sstep : (k * BK) / 128)); };
                 float cur = ks < t.ksteps ? scale_at(ks) : 0.0f;

@@ -140,6 +140,21 @@ def test_empty_and_unsupported(cuda):
     q.check(q.lib().qlmb_check_device(None))
 
 
+@pytest.mark.parametrize("M,K,N", [(300, 384, 640), (129, 640, 1152), (1000, 1408, 896), (70, 128, 384)])
+def test_linear_widths_that_end_inside_a_column_tile(cuda, M, K, N):
+    """Odd multiples of 128 on the output side: the last 256-column tile is half full."""
+    from cudalm_c_b200 import linear
+    from cudalm_c_b200._lib import KN, NK
+    for lay in (KN, NK):
+        Q, W = quantise(cuda, K, N, 31) if lay == KN else quantise(cuda, N, K, 31)
+        Wm = W if lay == KN else W.T
+        for dt in (torch.float32, torch.bfloat16):
+            X, dY = torch.randn(M, K, device=cuda).to(dt), torch.randn(M, N, device=cuda).to(dt)
+            Y, dX = linear.linear_fwd(X, Q.d, Q.s, lay, N), linear.linear_dgrad(dY, Q.d, Q.s, lay, K)
+            assert Y.shape == (M, N) and rel(Y, X.float() @ Wm) < 8e-3, (lay, dt)
+            assert dX.shape == (M, K) and rel(dX, dY.float() @ Wm.T) < 8e-3, (lay, dt)
+
+
 @pytest.mark.parametrize("M", [1023, 1025, 2047, 4161, 8191])
 def test_linear_wgrad_of_ragged_row_slices(cuda, M):
     """Rows that do not divide into the slices: the last slice ends early, or lies past the rows altogether."""
