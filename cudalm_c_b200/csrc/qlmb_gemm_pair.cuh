@@ -203,7 +203,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                     const CUtensorMap *am = &p.a_map[seg], *wm = &p.w_map[DUAL ? (int)rank : seg];
                     const int wrow = t.e * p.w_rows + (BMODE == B_DEQ_MN ? 0 : xb), wcol = DUAL ? t.n_t * 64 : xb / 2;
                     for (int ks = 0; ks < t.ksteps; ks++) {
-                        ok = mbar_wait_idle(empty0 + rs.idx * 8u, rs.phase ^ 1u, abort_flag, p.errword, 11);
+                        ok = mbar_wait(empty0 + rs.idx * 8u, rs.phase ^ 1u, abort_flag, p.errword, 11);
                         if (!ok) break;
                         if (leader) mbar_expect_tx(my_full + rs.idx * 8u, TX_BYTES);
                         const uint32_t bar = full0 + rs.idx * 8u, dstA = sA0 + rs.idx * P_A_STAGE, dstB = sB0 + rs.idx * P_B_STAGE;
