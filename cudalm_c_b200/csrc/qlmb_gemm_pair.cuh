@@ -16,9 +16,15 @@
 //   empty[s]       both     released by one tcgen05.commit that arrives in both CTAs
 //   tmem_full[a]   both     committed the same way after a tile's last step
 //   tmem_empty[a]  leader   8 local + 8 remote epilogue warps
-//   full_c[s]      local    byte count of the stage's packed codes.  They are requested once empty[s] has completed, so
+//   full_c[j]      local    byte count of a stage's packed codes.  They are requested once empty[s] has completed, so
 //                           a dequant warp that sees them knows that stage s of B is free too, and the multiplies that
 //                           complete empty[s] came after the codes of stage s had been read: no further hand-shake.
+//                           The warps of one group take every second stage, so j counts stages modulo an even number: a
+//                           barrier then serves one group only, which waits for each of its phases.  (With one barrier
+//                           per stage of an odd ring a group met every second phase, and a parity cannot tell a phase
+//                           from the last but one: where the codes of the phase between were late, a warp expanded
+//                           what the stage held before.)  A group's next phase of barrier j cannot complete before the
+//                           group has seen this one: its copy waits for multiplies that need the group's stage.
 // No bulk copy in this file has more than one destination CTA.
 #pragma once
 
@@ -28,6 +34,8 @@ constexpr int P_BN = 256;                 // accumulator columns of the pair til
 constexpr int P_A_STAGE = BM * BK * 2;    // per CTA: 128 rows
 constexpr int P_B_STAGE = 128 * BK * 2;   // per CTA: 128 columns of B
 constexpr int P_C_STAGE = 128 * BK / 2;   // per CTA: codes of those columns
+// barriers for the codes of ns stages that dqg groups of warps take in turn: a multiple of both
+constexpr int pair_code_bars(int ns, int dqg) { return ns % dqg ? ns * dqg : ns; }
 
 __device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ void cluster_sync()
@@ -131,7 +139,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
 {
     constexpr bool DEQ = (BMODE == B_DEQ_MN || BMODE == B_DEQ_K);
     constexpr bool DUAL = (EPI == EPI_SWIGLU);           // CTA 0 expands W1 (gate), CTA 1 expands W3 (up)
-    constexpr int NS = EPI == EPI_SWIGLU_BWD ? 4 : 5;
+    constexpr int NS = EPI == EPI_SWIGLU_BWD ? 4 : 5, NCB = pair_code_bars(NS, DQG);
     // Without weights to expand there is room for a second staging block per epilogue warp (a sixth operand stage brought
     // nothing): 16 KiB of fp32 per warp and tile no longer wait block by block for the store before
     constexpr bool TWO = !DEQ;
@@ -150,7 +158,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
     uint64_t *bars = reinterpret_cast<uint64_t *>(sE + EPI_WARPS * epi_stage_bytes(EPI, TWO));
     uint64_t *full = bars, *empty = full + NS;
     uint64_t *full_c = empty + NS;
-    uint64_t *tmem_full = full_c + NS, *tmem_empty = tmem_full + 2, *spare = tmem_empty + 2;
+    uint64_t *tmem_full = full_c + NCB, *tmem_empty = tmem_full + 2, *spare = tmem_empty + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(spare + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
@@ -164,7 +172,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
     }
     if (threadIdx.x == 0) {
         for (int i = 0; i < NS; i++) { mbar_init(smem_u32(&full[i]), 1 + (DEQ ? 2 * GW : 0)); mbar_init(smem_u32(&empty[i]), 1); }
-        for (int i = 0; i < NS; i++) mbar_init(smem_u32(&full_c[i]), 1);
+        for (int i = 0; i < NCB; i++) mbar_init(smem_u32(&full_c[i]), 1);
         for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&tmem_full[i]), 1); mbar_init(smem_u32(&tmem_empty[i]), 2 * EPI_WARPS); }
         mbar_init(smem_u32(spare), 1);
         for (int i = 0; i < 2 * EPI_WARPS; i++) mbar_init(smem_u32(bars + 48 + i), 1);   // epilogue input rings
@@ -193,6 +201,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
         // the warp's reconvergence and the group scales (4-byte copies by all lanes) inside the loop it took 870.
         if (elect_one()) {
             Ring rs = {0, 0};
+            int cb = 0;                                  // barrier of the stage's codes
             bool ok = true;
             const uint32_t full0 = map_to_cta(smem_u32(full), 0), my_full = smem_u32(full), empty0 = smem_u32(empty);
             const uint32_t full_c0 = smem_u32(full_c), sA0 = smem_u32(sA), sB0 = smem_u32(sB), sC0 = smem_u32(sC);
@@ -218,10 +227,11 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                             if (BMODE == B_TMA_K) tma_load_2d_pair(dstB, wm, bar, ks * BK, xb);
                         }
                         if (DEQ) {
-                            const uint32_t cbar = full_c0 + rs.idx * 8u, dstC = sC0 + rs.idx * P_C_STAGE;
+                            const uint32_t cbar = full_c0 + cb * 8u, dstC = sC0 + rs.idx * P_C_STAGE;
                             mbar_expect_tx(cbar, P_C_STAGE);
                             if (BMODE == B_DEQ_MN) tma_load_2d(dstC, wm, cbar, wcol, wrow + ks * BK);
                             else tma_load_2d(dstC, wm, cbar, ks * (BK / 2), wrow);
+                            if (++cb == NCB) cb = 0;
                         }
                         rs.next(NS);
                     }
@@ -336,7 +346,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
             else dst0[i] = (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((c0 ^ (r & 7)) << 4));
         }
         constexpr uint32_t DST_STEP = (uint32_t)(PER * ROWS_I / 8) * 1024u;      // bytes per PER words
-        Ring rb = {0, 0};
+        Ring rb = {0, 0}, rc = {0, 0};                               // stage of B, barrier of its codes
         bool ok = true;
         const uint32_t full0 = map_to_cta(smem_u32(&full[0]), 0);    // the leader's stage barriers
         const uint32_t full_c0 = smem_u32(full_c);
@@ -353,7 +363,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
             TileInfo t = decode_pair_tile<SCHED>(p, tile, ntr);
             for (int seg = 0; ok && seg < p.nseg; seg++) {
                 int ks = (g - kc % DQG + DQG) % DQG;                 // first stage of this group in the tile
-                for (int i = 0; i < ks && i < t.ksteps; i++) rb.next(NS);
+                for (int i = 0; i < ks && i < t.ksteps; i++) { rb.next(NS); rc.next(NCB); }
                 // one stage on is BK rows (codes [K][N]) or half a group (codes [N][K]) on; a half that lies past the
                 // columns expands zeros or the next matrix's codes with the scales of the half before it, for nobody
                 const int xs = t.n_t * P_BN + my_n < p.N ? t.n_t * P_BN + my_n : t.n_t * P_BN;
@@ -366,7 +376,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                 for (; ks < t.ksteps; ks += DQG) {
                     const float nxt = ks + DQG < t.ksteps ? scale_at(ks + DQG) : 0.0f;
                     const __nv_bfloat162 s2 = __float2bfloat162_rn(cur);
-                    ok = mbar_wait(full_c0 + rb.idx * 8u, rb.phase, abort_flag, p.errword, 20);
+                    ok = mbar_wait(full_c0 + rc.idx * 8u, rc.phase, abort_flag, p.errword, 20);
                     if (!ok) break;
                     const uint32_t *cw = reinterpret_cast<const uint32_t *>(sC + rb.idx * P_C_STAGE) + gw * 32 + lane;
                     uint32_t w[ITERS];
@@ -381,8 +391,11 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                     fence_proxy_async();
                     __syncwarp();
                     if (elect_one()) mbar_arrive_remote(full0 + (uint32_t)rb.idx * 8u);
-                    rb.idx += ks + DQG <= t.ksteps ? DQG : t.ksteps - ks;
-                    if (rb.idx >= NS) { rb.idx -= NS; rb.phase ^= 1u; }
+                    const int adv = ks + DQG <= t.ksteps ? DQG : t.ksteps - ks;
+                    rb.idx += adv;
+                    if (rb.idx >= NS) rb.idx -= NS;
+                    rc.idx += adv;
+                    if (rc.idx >= NCB) { rc.idx -= NCB; rc.phase ^= 1u; }
                     cur = nxt;
                 }
                 kc += t.ksteps;

@@ -278,3 +278,31 @@ def test_unsupported_shapes_are_rejected(cuda):
         L, *_ = build_layer(cuda, 64, 128, 256, 4, 2, 1)
         L.c.D = 96
         L.forward(torch.zeros(64, 96, device=cuda), torch.zeros(64, 96, device=cuda))
+
+
+@pytest.mark.parametrize("N,D,F,E,K", [(16384, 768, 1536, 32, 2), (333, 768, 1536, 32, 2), (2000, 512, 1152, 8, 2)])
+def test_layer_repeats_itself_bit_for_bit(cuda, N, D, F, E, K):
+    """The same layer on the same inputs, weights from HBM every time: every output of forward and backward has one writer
+    and a fixed order, so a repeated call gives the same bits (a warp that expanded a late tile of codes would show)."""
+    from cudalm_c_b200 import moe, qlm
+    g = torch.Generator(device=cuda); g.manual_seed(N)
+    q = []
+    for _ in range(3):
+        Q = qlm.Qlm([(0, E * D * F)], E * D * F, cuda)
+        Q.init_from(torch.randn(E * D * F, device=cuda, generator=g) * 0.02, render=False)
+        q.append(Q)
+    L = moe.MoeLayerState(N, D, F, E, K, *((a.d, a.s) for a in q), torch.randn(D, E, device=cuda, generator=g) * 0.02, aux=0.03)
+    fi, fn, dout = (torch.randn(N, D, device=cuda, generator=g).bfloat16() for _ in range(3))
+    dW = [torch.zeros(E, D, F, device=cuda), torch.zeros(E, D, F, device=cuda), torch.zeros(E, F, D, device=cuda), torch.zeros(D, E, device=cuda)]
+    flush = torch.empty(1 << 28, dtype=torch.uint8, device=cuda)            # larger than L2
+    bad = torch.zeros(6, dtype=torch.int64, device=cuda)
+    first = None
+    for i in range(150):
+        flush.fill_(i & 255)
+        out = L.forward(fi, fn)
+        dfn = L.backward(dout, fn, *dW, beta=0.0)
+        now = [out, dfn] + dW
+        if first is None:
+            first = [t.clone() for t in now]
+        bad += torch.stack([(a != b).sum() for a, b in zip(first, now)])
+    assert bad.tolist() == [0] * 6
