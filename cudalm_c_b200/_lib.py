@@ -100,6 +100,8 @@ PROTOTYPES = {
     "qlmb_gemv_decode_norm_stack": (ci, [vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, vp]),
     "qlmb_dec_qkv": (ci, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, vp]),
     "qlmb_gemv_decode_res_norm": (ci, [vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, vp]),
+    "qlmb_quiet_begin": (ci, [vp]),
+    "qlmb_quiet_end": (ci, []),
     "qlmb_dec_step_bytes": (sz, [ci] * 8),
     "qlmb_dec_step": (ci, [C.POINTER(DecStepArgs), vp]),
     "qlmb_dec_rope": (ci, [vp, ci, vp, vp, vp, ci, ci, ci, ci, vp]),

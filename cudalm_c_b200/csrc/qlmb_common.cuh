@@ -50,6 +50,9 @@ struct ProfScope {
 // its first write, and before any early return; only data that no kernel of the step writes (the weights) is touched
 // ahead of it.  Weights may be: a kernel that writes codes or scales never triggers, so whatever follows it starts after
 // its end, and a kernel that triggers does so after its own wait wherever a reader of weights can follow directly.
+// Float parameters (the router matrix, gains, the embedding) are no weights in this sense: k_adamw_bf16 writes them and
+// triggers first.  They are brought into L2 ahead of the wait (prefetch_l2; the writer's stores arrive there too) and
+// loaded behind it, or ahead of it where `weights_quiet` tells that no writer can be running.
 // The caller decides per launch (`early`): with one to four rows per step the early blocks of the decode chain cost the
 // running kernel more than they gain (decode step 0.53 -> 0.56 ms at one slot, 0.85 -> 0.81 ms at eight, CUDA events).
 // The tensor-core kernels set up their barriers and TMEM, the streaming GEMV requests its first weights, the row kernels
@@ -57,6 +60,19 @@ struct ProfScope {
 // QLMB_PDL=0 turns the attribute off everywhere (the instructions are then no-ops).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(p))); }
+// A load that stays where it is written and passes by L1.  (__ldg promises that nothing writes the data while the kernel
+// runs, which does not hold for a kernel that starts before its predecessor's end.)
+__device__ __forceinline__ float ld_cg(const float *p)
+{
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)) : "memory");
+    return v;
+}
+// Between qlmb_quiet_begin(st) and qlmb_quiet_end() the calling thread launches nothing on `st` that writes weights or
+// float parameters.  The first launch that asks inside such a scope gets false and waits before it triggers, so every
+// writer queued before the scope has ended, and its stores are visible, before a later launch of the scope can start.
+bool weights_quiet(cudaStream_t st);
 bool pdl_enabled(void);                                  // qlmb_runtime.cu
 template <typename... KArgs, typename... Args>
 static inline cudaError_t pdl_launch(bool early, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)

@@ -59,6 +59,29 @@ int sm_count(void)
 }
 
 
+// ---- scopes in which nothing writes weights (pdl_launch) ----
+static thread_local struct { int depth; bool waited; cudaStream_t st; } t_quiet;
+bool weights_quiet(cudaStream_t st)
+{
+    if (t_quiet.depth == 0 || t_quiet.st != st) return false;
+    const bool known = t_quiet.waited;
+    t_quiet.waited = true;
+    return known;
+}
+}  // namespace qlmb
+extern "C" int qlmb_quiet_begin(void *stream)
+{
+    QLMB_REQUIRE(qlmb::t_quiet.depth == 0, "qlmb_quiet_begin: this thread is inside such a scope already");
+    qlmb::t_quiet.depth = 1; qlmb::t_quiet.waited = false; qlmb::t_quiet.st = qlmb::as_stream(stream);
+    return QLMB_OK;
+}
+extern "C" int qlmb_quiet_end(void)
+{
+    qlmb::t_quiet.depth = 0;
+    return QLMB_OK;
+}
+namespace qlmb {
+
 // ---- two library-owned streams per device for work that may overlap the caller's stream ----
 // side_fork() makes the side stream wait for everything queued on `st` so far, side_join()
 // makes `st` wait for everything queued on the side stream; side_wait_main() is a second

@@ -472,8 +472,15 @@ class Decoder:
     def _layers_chain(self):
         """The layers of a step as separate operators: shapes the one-launch form does not take."""
         from ._lib import check, lib, ptr, stream_ptr
-        c, m, B = self.m.c, self.m, self.B
         L_ = lib()
+        check(L_.qlmb_quiet_begin(stream_ptr()))          # a step writes no parameters: its kernels may read them early
+        try:
+            return self._chain(L_, check, ptr, stream_ptr)
+        finally:
+            L_.qlmb_quiet_end()
+
+    def _chain(self, L_, check, ptr, stream_ptr):
+        c, m, B = self.m.c, self.m, self.B
         x = block.embed(m.emb, self.tok, dtype=torch.bfloat16)
         for l, ly in enumerate(m.layers):
             w, f = ly["w"], m.fl[l]

@@ -83,6 +83,13 @@ int qlmb_selftest_stream_read(const void *W, unsigned long long row_bytes, int r
  * captured).  No reference counterpart (the reference uses the default stream only). */
 int qlmb_side_stream_enable(int on);
 
+/* Between the two calls the calling thread promises to queue nothing on `stream` that writes 4-bit codes, scales or float
+ * parameters (a copy or a kernel of its own included).  The decode entry points may then read these before the kernel in
+ * front of them has ended.  Scopes do not nest; a scope that is left open only withholds other streams' launches from it.
+ * Without a scope everything is read once the kernel in front has ended.  No reference counterpart. */
+int qlmb_quiet_begin(void *stream);
+int qlmb_quiet_end(void);
+
 /* Per-operator timing, the counterpart of the reference's CUDALM_PROF=3 event
  * timers (cudalm.cu:806-825): while enabled, every kernel launch of the MoE
  * and linear entry points is bracketed by CUDA events on its stream.

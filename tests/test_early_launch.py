@@ -1,0 +1,72 @@
+"""Kernels that start before the kernel in front of them has ended (programmatic dependent launches).
+
+What they read may be what that kernel writes: an optimizer step directly in front of a decode step writes the router
+matrix, the codes and the scales.  On the CPU the sources are held to the rule (nothing is loaded ahead of the wait); on
+the GPU results behind a writer equal those behind a synchronisation."""
+import os
+import re
+
+import pytest
+import torch
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "cudalm_c_b200", "csrc")
+# a global load: the intrinsics, the library's own load helpers, a load lambda of a kernel
+LOAD = re.compile(r"__ld\w+\s*\(|\bld_\w+\s*\(|\bfetch\s*\(")
+
+
+def kernels():
+    """(name, body without comments) of every __global__ function."""
+    out = []
+    for f in sorted(os.listdir(CSRC)):
+        if not f.endswith((".cu", ".cuh")):
+            continue
+        with open(os.path.join(CSRC, f)) as h:
+            src = re.sub(r"//[^\n]*", "", h.read())
+        for m in re.finditer(r"__global__\s+void\b", src):
+            i = src.index("{", m.end())
+            name = re.findall(r"(\bk_\w+)\s*\(", src[m.end():i])[0]
+            depth, j = 1, i + 1
+            while depth:
+                depth += {"{": 1, "}": -1}.get(src[j], 0)
+                j += 1
+            out.append((name, src[i:j]))
+    return out
+
+
+def test_router_matrix_is_read_behind_the_wait():
+    body = dict(kernels())["k_router_small"]
+    assert not LOAD.search(body[:body.index("pdl_wait()")])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", [5, 8, 64])
+def test_adamw_on_the_router_directly_before_a_decode_step(cuda, N):
+    """qlmb_adamw lets the next kernel start early and writes the router matrix that the next kernel multiplies with."""
+    from cudalm_c_b200 import moe, qlm
+    D, F, E, K = 1024, 128, 32, 2
+    g = torch.Generator(device=cuda); g.manual_seed(N)
+    q = []
+    for _ in range(3):
+        Q = qlm.Qlm([(0, E * D * F)], E * D * F, cuda)
+        Q.init_from(torch.randn(E * D * F, device=cuda, generator=g) * 0.02, render=False)
+        q.append(Q)
+    x, xn = (torch.randn(N, D, device=cuda, generator=g).bfloat16() for _ in range(2))
+    G = torch.randn(D * E, device=cuda, generator=g)
+    wr0 = torch.randn(D * E, device=cuda, generator=g) * 0.02
+
+    def steps(sync):
+        wr = wr0.clone()
+        M, V = (torch.zeros(D * E, dtype=torch.int16, device=cuda) for _ in range(2))
+        layer = moe.MoeLayerState(N, D, F, E, K, *((a.d, a.s) for a in q), wr.view(D, E), aux=0.0)
+        outs = []
+        for t in range(1, 9):
+            qlm.adamw(wr, G if t % 2 else -G, M, V, 0.05, 0.9, 0.95, 0.0, 1.0, 1.0)
+            if sync:
+                torch.cuda.synchronize()
+            layer.decode(x, xn)
+            outs.append(layer.member("rt", (N, E), torch.float32).clone())
+        return torch.stack(outs)
+    want = steps(True)
+    assert not torch.equal(want[0], want[1])
+    for _ in range(20):
+        assert torch.equal(steps(False), want)
