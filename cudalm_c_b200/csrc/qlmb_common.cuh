@@ -46,33 +46,30 @@ struct ProfScope {
 // A kernel launched with pdl_launch may start while the kernel before it in the stream is still running: its blocks
 // are scheduled as soon as every block of that kernel has called pdl_trigger() (or exited), and run up to their
 // pdl_wait(), which returns once that kernel has completed and its writes are visible.  Rules kept by every such kernel:
-// every block executes pdl_wait() exactly once, before its first read of anything a kernel of the stream wrote, before
-// its first write, and before any early return; only data that no kernel of the step writes (the weights) is touched
-// ahead of it.  Weights may be: a kernel that writes codes or scales never triggers, so whatever follows it starts after
-// its end, and a kernel that triggers does so after its own wait wherever a reader of weights can follow directly.
-// Float parameters (the router matrix, gains, the embedding) are no weights in this sense: k_adamw_bf16 writes them and
-// triggers first.  They are brought into L2 ahead of the wait (prefetch_l2; the writer's stores arrive there too) and
-// loaded behind it, or ahead of it where `weights_quiet` tells that no writer can be running.
+// every block executes pdl_wait() exactly once, before its first write, before any early return, and before it loads
+// anything that a kernel may write: activations, but the weights too (codes, scales, gains, the router matrix, the
+// embedding), for the kernel in front may be an optimizer's.  That a writer does not trigger is not enough: its successor
+// then starts when its blocks are done, but sees its stores only behind the wait.  Only where `weights_quiet` answers
+// QUIET, no writer of weights being able to run or to be unseen, are they loaded ahead of it.  (Prefetches into L2 ahead of
+// the wait, which would be allowed, cost more than they gain: a streaming GEMV of 4096 x 16384 14.3 -> 15 us.)
 // The caller decides per launch (`early`): with one to four rows per step the early blocks of the decode chain cost the
 // running kernel more than they gain (decode step 0.53 -> 0.56 ms at one slot, 0.85 -> 0.81 ms at eight, CUDA events).
-// The tensor-core kernels set up their barriers and TMEM, the streaming GEMV requests its first weights, the row kernels
-// do nothing ahead of the wait: what they save is the gap between two launches of a stream.
+// The tensor-core kernels set up their barriers and TMEM, the others do nothing ahead of the wait: what they save is the
+// gap between two launches of a stream.
 // QLMB_PDL=0 turns the attribute off everywhere (the instructions are then no-ops).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(p))); }
-// A load that stays where it is written and passes by L1.  (__ldg promises that nothing writes the data while the kernel
-// runs, which does not hold for a kernel that starts before its predecessor's end.)
-__device__ __forceinline__ float ld_cg(const float *p)
-{
-    float v;
-    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)) : "memory");
-    return v;
-}
+// What a kernel reads behind its wait it reads with ordinary loads: __ldg and the like promise that nothing writes the data
+// while the kernel runs, which does not hold for a kernel that starts before its predecessor's end, and the compiler may
+// move them over the wait.  What it reads ahead of the wait passes by L1, which nothing has emptied since the writer.
+__device__ __forceinline__ float ld_cg(const float *p)   // stays where it is written
+{ float v; asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)) : "memory"); return v; }
 // Between qlmb_quiet_begin(st) and qlmb_quiet_end() the calling thread launches nothing on `st` that writes weights or
-// float parameters.  The first launch that asks inside such a scope gets false and waits before it triggers, so every
-// writer queued before the scope has ended, and its stores are visible, before a later launch of the scope can start.
-bool weights_quiet(cudaStream_t st);
+// float parameters.  The first launch that asks inside such a scope gets QUIET_FIRST and waits before it triggers, so
+// every writer queued before the scope has ended, and its stores are visible, before a later launch of the scope, which
+// gets QUIET, can start.  Outside a scope the answer is 0.
+enum { QUIET_FIRST = 1, QUIET = 2 };
+int weights_quiet(cudaStream_t st);
 bool pdl_enabled(void);                                  // qlmb_runtime.cu
 template <typename... KArgs, typename... Args>
 static inline cudaError_t pdl_launch(bool early, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)

@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(256, NB == 4 ? 2 : (BT <= 2 ? 4 : 2)) k_gemv_k
                                                  const uint8_t *codes2 = nullptr, const float *scales2 = nullptr)
 {
     pdl_trigger();
-    if (row_expert) pdl_wait();                 // the expert choice is the work of a kernel before this one
+    pdl_wait();                                 // expert choice, rows and, where a writer of weights is in front, those too
     // routed form: blockIdx.z is an output row, it reads activation row z % ntok and one matrix of a stack; B must be 1 then
     size_t xrow = 0, prow = 0;
     int PB = B;
@@ -67,26 +67,22 @@ __global__ void __launch_bounds__(256, NB == 4 ? 2 : (BT <= 2 ? 4 : 2)) k_gemv_k
     const bool live = n0 < N;
     const uint8_t *cp = codes + (size_t)n0 / 2;
     const float *sp = scales + n0 / 128;
-    // four rows per batch (k, k+8, k+16, k+24), NB batches in flight; the first NB are requested before the
-    // activations are staged (the weights do not depend on them)
+    // four rows per batch (k, k+8, k+16, k+24), NB batches in flight, the first NB requested before the activations are
+    // staged; rows past the slice repeat its last one and are not used
     uint32_t w[NB][4];
     float sc[NB][4];
     auto fetch = [&](int buf, int k) {
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const int kk = k + 8 * u;
-            w[buf][u] = 0u; sc[buf][u] = 0.0f;
-            if (kk < k1) {
-                w[buf][u] = __ldcs(reinterpret_cast<const uint32_t *>(cp + (size_t)kk * N / 2));
-                sc[buf][u] = __ldg(sp + (size_t)kk * gpr);
-            }
+            const int kk = k + 8 * u < k1 ? k + 8 * u : k1 - 1;
+            w[buf][u] = *reinterpret_cast<const uint32_t *>(cp + (size_t)kk * N / 2);
+            sc[buf][u] = sp[(size_t)kk * gpr];
         }
     };
     if (live) {
 #pragma unroll
         for (int u = 0; u < NB; u++) fetch(u, k0 + warp + 32 * u);
     }
-    if (!row_expert) pdl_wait();                // the weights above do not depend on the kernels before; the rows below do
     // gamma (routed form, one activation row per block): the row is normalised on the way in, x * rinv * gamma rounded
     // to bf16 as the separate norm kernel stores it (e_rmsf in front of the q, k, v projections, cudalm.cu:7176)
     float rinv = 1.0f;
@@ -229,28 +225,28 @@ __global__ void __launch_bounds__(256, 2) k_gemv_stream(void *Y, int dtype, floa
     const uint8_t *cp = codes + (size_t)(k0 + warp) * (N / 2) + n0 / 2;
     const float *sp = scales + (size_t)(k0 + warp) * (N / 128) + n0 / 128;
     // NB batches of U rows in flight per warp.  With two, every half round waited for the loads issued half a round before:
-    // 4096 x 16384, one row, 17.2 us against 13.2 (with the late trigger below).
+    // 4096 x 16384, one row, 17.2 us against 13.2 (with the late trigger below).  (14.3 now that the first loads stand behind
+    // the wait for the kernel in front, which may have written the weights.)
     constexpr int NB = BT <= 2 ? 4 : 3;
     uint32_t w[NB][U][WPL];
     float sc[NB][U];
     auto fetch = [&](int buf) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            if (WPL == 2) { const uint2 t = __ldcs(reinterpret_cast<const uint2 *>(cp)); w[buf][u][0] = t.x; w[buf][u][WPL - 1] = t.y; }
-            else w[buf][u][0] = __ldcs(reinterpret_cast<const uint32_t *>(cp));
-            sc[buf][u] = __ldg(sp);
+            if (WPL == 2) { const uint2 t = *reinterpret_cast<const uint2 *>(cp); w[buf][u][0] = t.x; w[buf][u][WPL - 1] = t.y; }
+            else w[buf][u][0] = *reinterpret_cast<const uint32_t *>(cp);
+            sc[buf][u] = *sp;
             cp += cstep; sp += sstep;
         }
     };
     const int nbatch = kslice / (8 * U);
-#pragma unroll
-    for (int i = 0; i < NB - 1; i++)                     // the weights do not depend on the activations: request them first
-        if (i < nbatch) fetch(i);
-    // a kernel that writes codes never lets the next one start early, so they are complete here; what follows waits
     pdl_wait();
+#pragma unroll
+    for (int i = 0; i < NB - 1; i++)                     // requested before the activations are staged
+        if (i < nbatch) fetch(i);
     // The next kernel may start at once where this one leaves SMs idle.  Otherwise its blocks would sit in slots that this
     // one's loads need (65.5 -> 71.7 us for four 4096 x 16384): it may start once the weights have been read, and its launch
-    // and its first loads fall into this kernel's reduction.
+    // falls into this kernel's reduction.
     if (trigger_first) pdl_trigger();
     for (int i = threadIdx.x; i < BT * kslice; i += 256) {
         const int b = i / kslice, k = k0 + i % kslice;
@@ -451,11 +447,11 @@ __global__ void __launch_bounds__(256, 2) k_gemv_rows8(const __grid_constant__ R
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kslice = a.kslice, K = a.K, N = a.N;
     pdl_trigger();
-    if (a.perm) pdl_wait();                              // the slot order is the work of a kernel before this one
+    pdl_wait();
     if (warp == 0) group_lookup<BT>(a, lane, &s_n, &s_mat, s_x, s_o);
     __syncthreads();
     const int nrow = s_n;
-    if (nrow == 0) { if (!a.perm) pdl_wait(); return; }
+    if (nrow == 0) return;
     const int mat = s_mat & 0xffff, second = s_mat >> 16;
     const uint8_t *codes = (second ? a.codes2 : a.codes) + (size_t)mat * a.e_codes;
     const float *scales = (second ? a.scales2 : a.scales) + (size_t)mat * a.e_scales;
@@ -471,13 +467,12 @@ __global__ void __launch_bounds__(256, 2) k_gemv_rows8(const __grid_constant__ R
     auto fetch = [&](int buf) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            w[buf][u] = __ldg(reinterpret_cast<const uint32_t *>(cp));
-            sc[buf][u] = __ldg(sp);
+            w[buf][u] = *reinterpret_cast<const uint32_t *>(cp);
+            sc[buf][u] = *sp;
             cp += cstep; sp += sstep;
         }
     };
     fetch(0);
-    if (!a.perm) pdl_wait();                             // the weights above do not depend on the kernels before; the rows below do
     if (a.gamma) {                                       // warp w: 1 / rms of row w over the whole K
         if (warp < nrow) {
             float ss = 0.0f;
@@ -606,7 +601,10 @@ template <> struct VecOfF<2> { typedef float2 T; };
 template <> struct VecOfF<4> { typedef float4 T; };
 // NW warps per block: eight (512 columns), or four (256) where the last block of eight would be at most half full (N = 768:
 // a quarter of the warps would repeat columns).
-template <int MT, int NW>
+// AHEAD: nothing can be writing the weights (weights_quiet), which are loaded ahead of the wait.
+template <bool AHEAD, typename T>
+__device__ __forceinline__ T ld_w(const T *p) { return AHEAD ? __ldcg(p) : *p; }
+template <int MT, int NW, bool AHEAD>
 __global__ void __launch_bounds__(32 * NW, MT == 1 ? 16 / NW : (NW == 8 ? 1 : 3)) k_gemv_mma(const __grid_constant__ Rows8 a)
 {
     constexpr int GR = 16 * MT, CW = 64 * NW, PADK = 8, NT = 32 * NW, NG = NW / 2;
@@ -616,12 +614,13 @@ __global__ void __launch_bounds__(32 * NW, MT == 1 ? 16 / NW : (NW == 8 ? 1 : 3)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int kslice = a.kslice, K = a.K, N = a.N, ldx = kslice + PADK;
     bf16 *xs = reinterpret_cast<bf16 *>(msm);
-    pdl_trigger();
-    if (a.perm) pdl_wait();                              // the slot order is the work of a kernel before this one
+    if (AHEAD || !a.late) pdl_trigger();
+    if (!AHEAD) pdl_wait();
+    if (!AHEAD && a.late) pdl_trigger();
     if (warp == 0) group_lookup<GR>(a, lane, &s_n, &s_mat, s_x, s_o);
     __syncthreads();
     const int nrow = s_n;
-    if (nrow == 0) { if (!a.perm) pdl_wait(); return; }
+    if (nrow == 0) { if (AHEAD) pdl_wait(); return; }
     const int mat = s_mat & 0xffff, second = s_mat >> 16;
     const uint8_t *codes = (second ? a.codes2 : a.codes) + (size_t)mat * a.e_codes;
     const float *scales = (second ? a.scales2 : a.scales) + (size_t)mat * a.e_scales;
@@ -634,10 +633,10 @@ __global__ void __launch_bounds__(32 * NW, MT == 1 ? 16 / NW : (NW == 8 ? 1 : 3)
     const uint8_t *cp = codes + (size_t)(k0 + 2 * t) * crow + (cc + 8 * g) / 2;
     uint32_t w[4][4];
     auto fetch = [&](int slot) {
-        w[slot][0] = __ldg(reinterpret_cast<const uint32_t *>(cp));
-        w[slot][1] = __ldg(reinterpret_cast<const uint32_t *>(cp + crow));
-        w[slot][2] = __ldg(reinterpret_cast<const uint32_t *>(cp + 8 * crow));
-        w[slot][3] = __ldg(reinterpret_cast<const uint32_t *>(cp + 9 * crow));
+        w[slot][0] = ld_w<AHEAD>(reinterpret_cast<const uint32_t *>(cp));
+        w[slot][1] = ld_w<AHEAD>(reinterpret_cast<const uint32_t *>(cp + crow));
+        w[slot][2] = ld_w<AHEAD>(reinterpret_cast<const uint32_t *>(cp + 8 * crow));
+        w[slot][3] = ld_w<AHEAD>(reinterpret_cast<const uint32_t *>(cp + 9 * crow));
         cp += 16 * crow;
     };
     const int steps = kslice / 16;                       // a multiple of four: kslice is a multiple of 64
@@ -650,15 +649,15 @@ __global__ void __launch_bounds__(32 * NW, MT == 1 ? 16 / NW : (NW == 8 ? 1 : 3)
         if (g0 + NG - 1 <= gmax && (srow & (NG - 1)) == 0) {      // NG neighbouring scales of a row in one load
             typedef typename VecOfF<NG>::T V;
             for (int i = threadIdx.x; i < kslice; i += NT)
-                reinterpret_cast<V *>(ssc)[i] = __ldg(reinterpret_cast<const V *>(scales + (size_t)(k0 + i) * srow + g0));
+                reinterpret_cast<V *>(ssc)[i] = ld_w<AHEAD>(reinterpret_cast<const V *>(scales + (size_t)(k0 + i) * srow + g0));
         } else {
             for (int i = threadIdx.x; i < kslice * NG; i += NT) {
                 const int gq = g0 + (i % NG) < gmax ? g0 + (i % NG) : gmax;
-                ssc[i] = __ldg(scales + (size_t)(k0 + i / NG) * srow + gq);
+                ssc[i] = ld_w<AHEAD>(scales + (size_t)(k0 + i / NG) * srow + gq);
             }
         }
     }
-    if (!a.perm) pdl_wait();                             // codes and scales above do not depend on the kernels before; the rows below do
+    if (AHEAD) pdl_wait();                               // the rows below are the work of the kernels before
     const bool vec = a.x_dtype == QLMB_BF16;                     // bf16 rows are staged in 16-byte pieces, four loads in flight
     if (a.gamma) {                                       // 1 / rms of every row over the whole K: warp w takes rows w, w + NW, ...
         for (int r = warp; r < nrow; r += NW) {
@@ -841,21 +840,21 @@ static int mma_launch(Rows8 a, int nz, const MmaPlan &pl, int mt, cudaStream_t s
     a.kslice = a.K / pl.ns;
     a.k65536 = 65536u;
     const size_t sm_b = (size_t)16 * mt * (a.kslice + 8) * sizeof(bf16) + (size_t)a.kslice * (pl.nw / 2) * sizeof(float);
+    const int quiet = weights_quiet(st);
+    const bool ahead = quiet == QUIET && !a.perm;                // (the routed form's weights depend on the slot order)
+    a.late = quiet == QUIET_FIRST;
+    typedef void (*Kern)(const Rows8);
+    static const Kern kerns[2][2][2] = {{{k_gemv_mma<1, 8, false>, k_gemv_mma<1, 8, true>}, {k_gemv_mma<1, 4, false>, k_gemv_mma<1, 4, true>}},
+                                        {{k_gemv_mma<2, 8, false>, k_gemv_mma<2, 8, true>}, {k_gemv_mma<2, 4, false>, k_gemv_mma<2, 4, true>}}};
     static bool attr_done[64];
     int dv = 0;
     QLMB_CUDA(cudaGetDevice(&dv));
     if (dv >= 0 && dv < 64 && !attr_done[dv]) {
-        QLMB_CUDA(cudaFuncSetAttribute(k_gemv_mma<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-        QLMB_CUDA(cudaFuncSetAttribute(k_gemv_mma<1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-        QLMB_CUDA(cudaFuncSetAttribute(k_gemv_mma<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-        QLMB_CUDA(cudaFuncSetAttribute(k_gemv_mma<2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+        for (int i = 0; i < 8; i++)
+            QLMB_CUDA(cudaFuncSetAttribute(kerns[i >> 2][(i >> 1) & 1][i & 1], cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
         attr_done[dv] = true;
     }
-    const dim3 grid(pl.nb, pl.ns, nz), block(32 * pl.nw);
-    if (mt == 1 && pl.nw == 8) QLMB_CUDA(pdl_launch(true, k_gemv_mma<1, 8>, grid, block, sm_b, st, a));
-    else if (mt == 1) QLMB_CUDA(pdl_launch(true, k_gemv_mma<1, 4>, grid, block, sm_b, st, a));
-    else if (pl.nw == 8) QLMB_CUDA(pdl_launch(true, k_gemv_mma<2, 8>, grid, block, sm_b, st, a));
-    else QLMB_CUDA(pdl_launch(true, k_gemv_mma<2, 4>, grid, block, sm_b, st, a));
+    QLMB_CUDA(pdl_launch(true, kerns[mt - 1][pl.nw == 4][ahead], dim3(pl.nb, pl.ns, nz), dim3(32 * pl.nw), sm_b, st, a));
     QLMB_LAUNCH_CHECK("k_gemv_mma");
     return QLMB_OK;
 }
@@ -864,7 +863,7 @@ static int mma_launch(Rows8 a, int nz, const MmaPlan &pl, int mt, cudaStream_t s
 // K slice; lanes stride over the code words of the slice, 4 words (one per column) per step share the
 // activation values; the scale multiplies the 8-element partial dot product of each word.  NB steps are in flight, the
 // first of them requested before the activations are staged (16 bytes at a time): with two, and one activation after the
-// other, 4096 x 16384 took 31 us for one row, now 21.7.  A single slice writes Y itself.
+// other, 4096 x 16384 took 31 us for one row, now 19.1.  A single slice writes Y itself.
 template <int BT>
 __global__ void __launch_bounds__(256, BT == 1 ? 4 : BT == 2 ? 3 : 2) k_gemv_nk(void *Y, float *part, const void *X, int dtype, const uint8_t *codes,
                                                  const float *scales, int B, int K, int N, int kslice)
@@ -883,13 +882,14 @@ __global__ void __launch_bounds__(256, BT == 1 ? 4 : BT == 2 ? 3 : 2) k_gemv_nk(
     auto fetch = [&](int buf, int kw) {
 #pragma unroll
         for (int c = 0; c < 4; c++) {
-            w[buf][c] = kw < nw ? __ldcs(reinterpret_cast<const uint32_t *>(cp + (size_t)c * (K / 2)) + kw) : 0u;
-            sc[buf][c] = kw < nw ? __ldg(sp + c * gpr + kw / 16) : 0.0f;
+            const int q = kw < nw ? kw : nw - 1;             // words past the slice repeat its last one and are not used
+            w[buf][c] = reinterpret_cast<const uint32_t *>(cp + (size_t)c * (K / 2))[q];
+            sc[buf][c] = sp[c * gpr + q / 16];
         }
     };
+    pdl_wait();
 #pragma unroll
     for (int i = 0; i < NB - 1; i++) fetch(i, lane + 32 * i);
-    pdl_wait();                                              // the codes are no running kernel's output, the rows are
     // B <= BT
     if (dtype == QLMB_BF16) {
         for (int i = threadIdx.x; i < BT * (kslice / 8); i += 256) {
@@ -991,11 +991,8 @@ __global__ void __launch_bounds__(256, 2) k_gemv_nk8(float *part, const void *X,
             float sc[4];
 #pragma unroll
             for (int c = 0; c < 4; c++) {
-                w[c] = 0u; sc[c] = 0.0f;
-                if (n0 + c < N) {
-                    w[c] = __ldcs(reinterpret_cast<const uint32_t *>(codes + ((size_t)(n0 + c) * K + k0) / 2) + kw);
-                    sc[c] = __ldg(scales + (size_t)(n0 + c) * gpr + (k0 + kw * 8) / 128);
-                }
+                w[c] = reinterpret_cast<const uint32_t *>(codes + ((size_t)(n0 + c) * K + k0) / 2)[kw];
+                sc[c] = scales[(size_t)(n0 + c) * gpr + (k0 + kw * 8) / 128];
             }
             float d[4][8];
 #pragma unroll
@@ -1296,11 +1293,11 @@ static int gemv_decode_impl(void *Y, const void *X, const int8_t *codes, const f
         const int cpl = N >= 8192 ? 16 : 8, cw = 32 * cpl;
         const int nb = (N + cw - 1) / cw;
         QLMB_REQUIRE(nb <= 2048, "qlmb_gemv_decode: N=%d", N);
-        // K slices of whole 64-row units, as even as they go, in one round of up to three blocks per SM (two with four
-        // rows): of those the count for which an SM's share of units, with a third of a unit per block for staging and the
-        // reduction, is the smallest; one or two blocks alone do not cover the latency of their loads.  (4096 x 16384, one
-        // row, 32 column blocks: 8 equal slices, 256 blocks, took 16.4 us, now 13.2 with what follows.  A ring of
-        // bulk copies per row into shared memory instead of register prefetch was slower, 29 us.)
+        // K slices of whole 64-row units, as even as they go, in one round of up to two blocks per SM: of those the count for
+        // which an SM's share of units, with a third of a unit per block for staging and the reduction, is the smallest; one
+        // block alone does not cover the latency of its loads.  (4096 x 16384, one row, 32 column blocks: 8 equal slices,
+        // 256 blocks, took 16.4 us, these 13.2, and 14.3 with the first loads behind the wait for the kernel in front.  A
+        // ring of bulk copies per row into shared memory instead of register prefetch was slower, 29 us.)
         const int units = K / 64, most = 2;
         int ns = 0;
         float best = 0.0f;

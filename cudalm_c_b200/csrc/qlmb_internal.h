@@ -19,6 +19,7 @@ struct Rows8 {
     const int *perm, *off; int E, ntok, x_by_token, zdual, R;   // routed (perm != nullptr)
     const float *gamma;                                  // dense: rows are normalised on the way in (rinv * gamma, bf16)
     uint32_t k65536;
+    int late;                                            // trigger behind the wait (weights_quiet: QUIET_FIRST)
 };
 // ---- routing (qlmb_route.cu) ----
 int router_topk(const float *rt, float *rprobs, int *assign, float *gate, int N, int E, int K,

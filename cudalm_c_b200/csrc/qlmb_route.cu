@@ -99,20 +99,18 @@ __global__ void __launch_bounds__(256) k_router_small(float *rt, const void *X, 
     const int n = blockIdx.x, warp = threadIdx.x >> 5, e = threadIdx.x & 31;
     const int per = (D + 7) / 8, j0 = warp * per, j1 = j0 + per < D ? j0 + per : D;
     // 96 rows of Wr in flight per lane (at D = 768 the whole share of a warp; in batches of 32 the block waited for three
-    // rounds to L2); the sum itself stays in ascending order.  Wr may be what the kernel in front writes (qlmb_adamw): unless
-    // the launch is known to have no such writer, the blocks bring it into L2 ahead of the wait and load it behind.
+    // rounds to L2); the sum itself stays in ascending order.  Wr may be what the kernel in front writes (qlmb_adamw): it is
+    // loaded ahead of the wait only where the launch is known to have no such writer.
     // Every load is executed: rows past the share's end repeat its last one, lanes past the experts the last expert.
     constexpr int UB = 96;
     float w[UB];
     const int ec = e < E ? e : E - 1, jl = j1 > j0 ? j1 - 1 : 0;
-    if (!quiet) {
-        for (size_t o = ((size_t)n * 256 + threadIdx.x) * 32; o < (size_t)D * E; o += (size_t)N * 256 * 32) prefetch_l2(Wr + o);
-        pdl_wait();
-    }
-    pdl_trigger();
+    if (quiet != QUIET_FIRST) pdl_trigger();
+    if (quiet != QUIET) pdl_wait();
+    if (quiet == QUIET_FIRST) pdl_trigger();
 #pragma unroll
     for (int u = 0; u < UB; u++) w[u] = ld_cg(Wr + (size_t)(j0 + u < jl ? j0 + u : jl) * E + ec);
-    if (quiet) pdl_wait();                               // the row below is the work of the kernels before
+    if (quiet == QUIET) pdl_wait();                               // the row below is the work of the kernels before
     for (int j = threadIdx.x; j < D; j += 256)
         rs_x[j] = x_dtype == QLMB_BF16 ? __bfloat162float(((const bf16 *)X)[(size_t)n * D + j]) : ((const float *)X)[(size_t)n * D + j];
     __syncthreads();
@@ -432,7 +430,7 @@ int router_small(float *rt, const void *X, int x_dtype, const float *Wr, float *
     const bool fuse = perm && off && perm_done && K * N <= 256;      // the last block also groups the slots by expert
     if (fuse) *perm_done = 1;
     QLMB_CUDA(pdl_launch(N > 4, k_router_small, dim3(N), dim3(256), (size_t)D * sizeof(float), st, rt, X, x_dtype, Wr, rprobs, assign, gate, N, D, E, K, bias, bs,
-                         fuse ? perm : (int *)nullptr, off, counts, bad, (int)weights_quiet(st)));
+                         fuse ? perm : (int *)nullptr, off, counts, bad, weights_quiet(st)));
     QLMB_LAUNCH_CHECK("k_router_small");
     return QLMB_OK;
 }

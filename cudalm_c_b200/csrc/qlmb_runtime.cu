@@ -61,12 +61,12 @@ int sm_count(void)
 
 // ---- scopes in which nothing writes weights (pdl_launch) ----
 static thread_local struct { int depth; bool waited; cudaStream_t st; } t_quiet;
-bool weights_quiet(cudaStream_t st)
+int weights_quiet(cudaStream_t st)
 {
-    if (t_quiet.depth == 0 || t_quiet.st != st) return false;
+    if (t_quiet.depth == 0 || t_quiet.st != st) return 0;
     const bool known = t_quiet.waited;
     t_quiet.waited = true;
-    return known;
+    return known ? QUIET : QUIET_FIRST;
 }
 }  // namespace qlmb
 extern "C" int qlmb_quiet_begin(void *stream)

@@ -14,8 +14,17 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 LOAD = re.compile(r"__ld\w+\s*\(|\bld_\w+\s*\(|\bfetch\s*\(")
 
 
+def braces(src, i):
+    """The end of the block that opens at src[i]."""
+    depth, j = 1, i + 1
+    while depth:
+        depth += {"{": 1, "}": -1}.get(src[j], 0)
+        j += 1
+    return j
+
+
 def kernels():
-    """(name, body without comments) of every __global__ function."""
+    """(name, body without comments and without the bodies of its lambdas) of every __global__ function."""
     out = []
     for f in sorted(os.listdir(CSRC)):
         if not f.endswith((".cu", ".cuh")):
@@ -25,17 +34,29 @@ def kernels():
         for m in re.finditer(r"__global__\s+void\b", src):
             i = src.index("{", m.end())
             name = re.findall(r"(\bk_\w+)\s*\(", src[m.end():i])[0]
-            depth, j = 1, i + 1
-            while depth:
-                depth += {"{": 1, "}": -1}.get(src[j], 0)
-                j += 1
-            out.append((name, src[i:j]))
+            body = src[i:braces(src, i)]
+            while True:
+                lam = re.search(r"auto \w+ = \[[&=]?\]\s*\([^)]*\)\s*\{", body)
+                if not lam:
+                    break
+                body = body[:lam.start()] + body[braces(body, lam.end() - 1):]
+            out.append((name, body))
     return out
 
 
-def test_router_matrix_is_read_behind_the_wait():
-    body = dict(kernels())["k_router_small"]
-    assert not LOAD.search(body[:body.index("pdl_wait()")])
+def test_nothing_is_loaded_ahead_of_the_wait():
+    """In every kernel that can start early the first pdl_wait() stands in front of its first load, and only the name of a
+    launch without a writer of weights in front (QUIET, AHEAD) may make it conditional."""
+    seen = 0
+    for name, body in kernels():
+        if "pdl_wait()" not in body:
+            continue
+        seen += 1
+        head = body[:body.index("pdl_wait()")]
+        assert not LOAD.search(head), name
+        cond = re.findall(r"if \(([^;{}]*)\)\s*(?:\{[^{}]*)?$", head)
+        assert not cond or cond[0] in ("quiet != QUIET", "!AHEAD") or name.startswith("k_attn"), (name, cond)
+    assert seen > 30
 
 
 @pytest.mark.gpu
@@ -70,3 +91,32 @@ def test_adamw_on_the_router_directly_before_a_decode_step(cuda, N):
     assert not torch.equal(want[0], want[1])
     for _ in range(20):
         assert torch.equal(steps(False), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B", [1, 2, 4, 8, 33])
+@pytest.mark.parametrize("layout", ["KN", "NK"])
+def test_optimizer_step_directly_before_a_gemv(cuda, B, layout):
+    """The codes and scales that a GEMV multiplies with are those of the optimizer step in front of it."""
+    from cudalm_c_b200 import _lib, linear, qlm
+    K, N = 1024, 8192
+    g = torch.Generator(device=cuda); g.manual_seed(B)
+    w = torch.randn(K * N, device=cuda, generator=g) * 0.02
+    G = torch.randn(K * N, device=cuda, generator=g)
+    for dt in (torch.bfloat16, torch.float32):
+        x = torch.randn(B, K, device=cuda, generator=g).to(dt)
+
+        def steps(sync):
+            Q = qlm.Qlm([(0, K * N)], K * N, cuda)
+            Q.init_from(w, render=False)
+            outs = []
+            for t in range(1, 7):
+                Q.step(None, G if t % 2 else -G, 0.05, 0.9, 0.95, 0.1, t)
+                if sync:
+                    torch.cuda.synchronize()
+                outs.append(linear.gemv_decode(x, Q.d, Q.s, getattr(_lib, layout), N))
+            return torch.stack(outs)
+        want = steps(True)
+        assert not torch.equal(want[0], want[1])
+        for _ in range(4):
+            assert torch.equal(steps(False), want)
