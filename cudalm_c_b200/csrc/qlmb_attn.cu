@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(256) k_attn_drow(float *drow, const bf16 *dA, 
     const bool live = g < (size_t)B * T * H;
     float acc = 0.0f;
     if (live) {
-        const uint4 x = __ldg(reinterpret_cast<const uint4 *>(dA + g * AT_HD) + c), y = __ldg(reinterpret_cast<const uint4 *>(O + g * AT_HD) + c);
+        const uint4 x = *(reinterpret_cast<const uint4 *>(dA + g * AT_HD) + c), y = *(reinterpret_cast<const uint4 *>(O + g * AT_HD) + c);
         const __nv_bfloat162 *xh = reinterpret_cast<const __nv_bfloat162 *>(&x), *yh = reinterpret_cast<const __nv_bfloat162 *>(&y);
 #pragma unroll
         for (int k = 0; k < 4; k++) {

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm_fwd(void *O, float *rinv, const
         for (int k = 0; k < NV; k++) {
             const int j = lane * 4 + k * 128;
             if (j < D) {
-                const float4 x = v[k], g = __ldg(reinterpret_cast<const float4 *>(gamma + j));
+                const float4 x = v[k], g = *reinterpret_cast<const float4 *>(gamma + j);
                 blk_st4(O, o_dtype, (size_t)n * D + j, make_float4(x.x * s * g.x, x.y * s * g.y, x.z * s * g.z, x.w * s * g.w));
             }
         }
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(128) k_gamma_part(float *part, const void *X, 
         float x[8], d[8], r[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
-            x[k] = blk_ld(X, x_dtype, (size_t)(n + k) * D + j); d[k] = blk_ld(dy, dy_dtype, (size_t)(n + k) * D + j); r[k] = __ldg(rinv + n + k);
+            x[k] = blk_ld(X, x_dtype, (size_t)(n + k) * D + j); d[k] = blk_ld(dy, dy_dtype, (size_t)(n + k) * D + j); r[k] = rinv[n + k];
         }
 #pragma unroll
         for (int k = 0; k < 8; k++) acc += x[k] * r[k] * d[k];
@@ -255,13 +255,13 @@ __global__ void __launch_bounds__(512) k_rmsnorm_bwd_gamma(void *dx, int accumul
                 if (accumulate) q[k] = blk_ld4(dx, DXT, o + j);
             }
         }
-        const float s = __ldg(rinv + n);
+        const float s = rinv[n];
         float t = 0.0f;
 #pragma unroll
         for (int k = 0; k < NV; k++) {
             const int j = lane * 4 + k * 128;
             if (j < D) {
-                const float4 g = __ldg(reinterpret_cast<const float4 *>(gamma + j));
+                const float4 g = *reinterpret_cast<const float4 *>(gamma + j);
                 t += x[k].x * g.x * d[k].x + x[k].y * g.y * d[k].y + x[k].z * g.z * d[k].z + x[k].w * g.w * d[k].w;
                 acc[k].x += x[k].x * s * d[k].x; acc[k].y += x[k].y * s * d[k].y; acc[k].z += x[k].z * s * d[k].z; acc[k].w += x[k].w * s * d[k].w;
             }
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(512) k_rmsnorm_bwd_gamma(void *dx, int accumul
         for (int k = 0; k < NV; k++) {
             const int j = lane * 4 + k * 128;
             if (j < D) {
-                const float4 g = __ldg(reinterpret_cast<const float4 *>(gamma + j));
+                const float4 g = *reinterpret_cast<const float4 *>(gamma + j);
                 float4 r = make_float4(s * g.x * d[k].x - cf * x[k].x, s * g.y * d[k].y - cf * x[k].y, s * g.z * d[k].z - cf * x[k].z, s * g.w * d[k].w - cf * x[k].w);
                 if (accumulate) { r.x += q[k].x; r.y += q[k].y; r.z += q[k].z; r.w += q[k].w; }
                 blk_st4(dx, DXT, o + j, r);
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(128) k_dec_attn(bf16_t *O, const bf16_t *Q, co
     float *sc = dec_sc;
     const int lo = (win > 0 && t >= win) ? t - win + 1 : 0;
     float q[8];
-    bf8_to_f(__ldg(reinterpret_cast<const uint4 *>(Q + (size_t)b * D + h * 64 + c8)), q);
+    bf8_to_f(*reinterpret_cast<const uint4 *>(Q + (size_t)b * D + h * 64 + c8), q);
     const size_t base = (size_t)b * Tm * KD + kvh * 64 + c8;
     const bf16_t *kb = Kc + base, *vb = Vc + base;
     float mx = -1e30f;

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(256) k_router_logits_tile(float *rt, const voi
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     const int q = tid + i * 256, row = q >> 5, e = q & 31;
-                    ws[st][row][e] = (e < E && j0 + row < D) ? __ldg(Wr + (size_t)(j0 + row) * E + e) : 0.0f;
+                    ws[st][row][e] = (e < E && j0 + row < D) ? Wr[(size_t)(j0 + row) * E + e] : 0.0f;
                 }
             }
         }

@@ -187,7 +187,7 @@ __device__ __forceinline__ void blk_load(uint8_t *blk, int lane, const uint8_t *
     for (int j = 0; j < 8; j++) {
         const int r = j * 4 + (lane >> 3), c = lane & 7;
         uint4 x = make_uint4(0, 0, 0, 0);
-        if (r < valid_rows) x = __ldg(reinterpret_cast<const uint4 *>(g0 + (long long)r * pitch + c * 16));
+        if (r < valid_rows) x = *reinterpret_cast<const uint4 *>(g0 + (long long)r * pitch + c * 16);
         *blk_vec(blk, r, c) = x;
     }
 }
@@ -783,7 +783,7 @@ k_gemm(const __grid_constant__ GemmParams p)
 #pragma unroll
                 for (int i = 0; i < ITERS; i++) {
                     const float *sp = (DUAL && second[i]) ? sc1 : sseg;
-                    cur[i] = __ldg(sp + sbase[i]);
+                    cur[i] = sp[sbase[i]];
                 }
                 for (int ks = 0; ks < t.ksteps; ks++) {
                     // scales of the next step are requested before this step's tile is awaited
@@ -792,7 +792,7 @@ k_gemm(const __grid_constant__ GemmParams p)
                         for (int i = 0; i < ITERS; i++) {
                             const float *sp = (DUAL && second[i]) ? sc1 : sseg;
                             int idx = (BMODE == B_DEQ_MN) ? sbase[i] + (ks + 1) * sstep : sbase[i] + ((ks + 1) * BK) / 128;
-                            nxt[i] = __ldg(sp + idx);
+                            nxt[i] = sp[idx];
                         }
                     }
                     ok = mbar_wait(smem_u32(&full_c[rc.idx]), rc.phase, abort_flag, p.errword, 7);

@@ -371,7 +371,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                     + (BMODE == B_DEQ_MN ? (t.e * p.w_rows + srow) * gpr + (DUAL ? t.n_t : xs / 128)
                                          : (t.e * p.w_rows + xs + srow) * gpr);
                 const int sstep = BMODE == B_DEQ_MN ? BK * gpr : 0;
-                auto scale_at = [&](int k) { return __ldg(sp + (BMODE == B_DEQ_MN ? k * sstep : (k * BK) / 128)); };
+                auto scale_at = [&](int k) { return sp[(BMODE == B_DEQ_MN ? k * sstep : (k * BK) / 128)]; };
                 float cur = ks < t.ksteps ? scale_at(ks) : 0.0f;
                 for (; ks < t.ksteps; ks += DQG) {
                     const float nxt = ks + DQG < t.ksteps ? scale_at(ks + DQG) : 0.0f;

@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(32 * NW, MT == 1 ? 16 / NW : (NW == 8 ? 1 : 3)
             if (vec) {
                 const uint4 *xr = reinterpret_cast<const uint4 *>(reinterpret_cast<const bf16 *>(a.X) + (size_t)s_x[r] * K);
                 for (int kc = lane; kc < K / 8; kc += 32) {
-                    const uint4 v = __ldg(xr + kc);
+                    const uint4 v = xr[kc];
                     const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&v);
 #pragma unroll
                     for (int j = 0; j < 4; j++) { const float2 f = __bfloat1622float2(h[j]); ss += f.x * f.x; ss += f.y * f.y; }
@@ -688,7 +688,7 @@ __global__ void __launch_bounds__(32 * NW, MT == 1 ? 16 / NW : (NW == 8 ? 1 : 3)
                 const int i = i0 + j * NT, b = i / cpr, kc = i - b * cpr;
                 v[j] = make_uint4(0u, 0u, 0u, 0u);
                 if (i < total && b < nrow)
-                    v[j] = __ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const bf16 *>(a.X) + (size_t)s_x[b] * K + k0 + kc * 8));
+                    v[j] = *reinterpret_cast<const uint4 *>(reinterpret_cast<const bf16 *>(a.X) + (size_t)s_x[b] * K + k0 + kc * 8);
             }
 #pragma unroll
             for (int j = 0; j < 4; j++) {
@@ -896,7 +896,7 @@ __global__ void __launch_bounds__(256, BT == 1 ? 4 : BT == 2 ? 3 : 2) k_gemv_nk(
             const int b = i / (kslice / 8), k = (i % (kslice / 8)) * 8;
             float4 lo = make_float4(0, 0, 0, 0), hi = lo;
             if (b < B && k0 + k < k1) {
-                const uint4 v = __ldg(reinterpret_cast<const uint4 *>((const bf16 *)X + (size_t)b * K + k0 + k));
+                const uint4 v = *reinterpret_cast<const uint4 *>((const bf16 *)X + (size_t)b * K + k0 + k);
                 lo = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
                 hi = make_float4(__uint_as_float(v.z << 16), __uint_as_float(v.z & 0xffff0000u), __uint_as_float(v.w << 16), __uint_as_float(v.w & 0xffff0000u));
             }
@@ -907,7 +907,7 @@ __global__ void __launch_bounds__(256, BT == 1 ? 4 : BT == 2 ? 3 : 2) k_gemv_nk(
         for (int i = threadIdx.x; i < BT * (kslice / 4); i += 256) {
             const int b = i / (kslice / 4), k = (i % (kslice / 4)) * 4;
             float4 v = make_float4(0, 0, 0, 0);
-            if (b < B && k0 + k < k1) v = __ldg(reinterpret_cast<const float4 *>((const float *)X + (size_t)b * K + k0 + k));
+            if (b < B && k0 + k < k1) v = *reinterpret_cast<const float4 *>((const float *)X + (size_t)b * K + k0 + k);
             *reinterpret_cast<float4 *>(xs + b * kslice + k) = v;
         }
     }

@@ -884,7 +884,7 @@ __global__ void __launch_bounds__(256) k_sq_partial(const float *G, size_t n, do
     for (; i + 7 * 256 < hi; i += 8 * 256) {
         float v[8];
 #pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = __ldg(G + i + u * 256);
+        for (int u = 0; u < 8; u++) v[u] = G[i + u * 256];
 #pragma unroll
         for (int u = 0; u < 8; u++) { const double g = (double)v[u]; acc = __fma_rn(g, g, acc); }
     }

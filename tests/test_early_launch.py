@@ -23,8 +23,8 @@ def braces(src, i):
     return j
 
 
-def kernels():
-    """(name, body without comments and without the bodies of its lambdas) of every __global__ function."""
+def kernels(whole=False):
+    """(name, body without comments and, unless `whole`, without the bodies of its lambdas) of every __global__ function."""
     out = []
     for f in sorted(os.listdir(CSRC)):
         if not f.endswith((".cu", ".cuh")):
@@ -35,7 +35,7 @@ def kernels():
             i = src.index("{", m.end())
             name = re.findall(r"(\bk_\w+)\s*\(", src[m.end():i])[0]
             body = src[i:braces(src, i)]
-            while True:
+            while not whole:
                 lam = re.search(r"auto \w+ = \[[&=]?\]\s*\([^)]*\)\s*\{", body)
                 if not lam:
                     break
@@ -57,6 +57,12 @@ def test_nothing_is_loaded_ahead_of_the_wait():
         cond = re.findall(r"if \(([^;{}]*)\)\s*(?:\{[^{}]*)?$", head)
         assert not cond or cond[0] in ("quiet != QUIET", "!AHEAD") or name.startswith("k_attn"), (name, cond)
     assert seen > 30
+
+
+def test_no_early_kernel_promises_read_only_data():
+    """__ldg states that nothing writes the data while the kernel runs: not so beside a predecessor that still runs."""
+    for name, body in kernels(whole=True):
+        assert "pdl_wait()" not in body or "__ldg(" not in body, name
 
 
 @pytest.mark.gpu
