@@ -477,6 +477,7 @@ __device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const 
         if ((blk + 1) * 256 <= t) { ds_kv_request(a, sh, ly, kvs, item, blk + 1); ds_wait<1>(); }
         else ds_wait<0>();
         if (left < 0) continue;
+        __syncwarp();                                     // a lane has waited for its own copies only, and row `left` is one's target
         if (left < 16 && r < 2)                           // the new key and value are not read back from the cache
             *reinterpret_cast<uint4 *>(mine + r * 2048 + left * 128 + c8 * 2) = *reinterpret_cast<const uint4 *>(sh.kv + r * 64 + c8);
         __syncwarp();

@@ -151,6 +151,8 @@ def test_sampler_topk_topp_temperature(cuda):
     (2, 640, 2, 8, 1, 384, 256, 640),       # grouped heads, a column tile that is half empty, a second pass
     (3, 128, 2, 4, 4, 128, 40, 64),         # every expert, one row slice
     (8, 1024, 16, 32, 3, 640, 20, 32),      # 24 routed slots, experts with several slots, the widest model
+    (3, 768, 12, 32, 2, 1536, 640, 1024),   # two rows a task, the last of them alone; buffers of keys used a second time
+    (4, 768, 12, 32, 2, 512, 518, 1024),    # two rows a task; positions on both sides of 512
 ])
 def test_one_launch_step_equals_the_chain(cuda, B, D, KV, E, K, F, fill, Tm):
     """qlmb_dec_step (up to eight slots) against the chain of separate operators: the same experts and the same cache rows
@@ -181,9 +183,13 @@ def test_one_launch_step_equals_the_chain(cuda, B, D, KV, E, K, F, fill, Tm):
     torch.cuda.synchronize()
     q.check(q.lib().qlmb_check_device(None))
     assert torch.equal(*outs)
-    # a near-tie of two router logits may fall the other way for a choice or two
-    assert sum(int((e != mo.member("assign", (K, B), torch.int32)).sum()) for e, mo in zip(experts, d.moes)) <= 2
-    assert float(((outs[0] - want).norm(dim=1) / want.norm(dim=1)).median()) < 1e-2
+    # a near-tie of two router logits may fall the other way in one slot of a batch; every other slot is held to the bound:
+    # some twenty bf16 roundings in two layers, each of at most 2^-9 and together 2^-9 sqrt(20 / 3) = 5e-3 by their root mean
+    # square, times four for the largest of the slots
+    same = torch.stack([(e == mo.member("assign", (K, B), torch.int32)).all(0) for e, mo in zip(experts, d.moes)]).all(0)
+    assert int((~same).sum()) <= (B > 2)
+    err = (outs[0] - want).norm(dim=1) / want.norm(dim=1)
+    assert float(err[same].max()) < 2e-2, err.tolist()
     for t, c, b in zip(d.K + d.V, caches, before):
         assert float((t.float() - c.float()).abs().max()) < 2e-2
         assert ((t != b).flatten(2).any(-1).sum(1) <= 1).all()              # at most the slot's own row changed
