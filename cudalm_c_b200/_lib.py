@@ -100,6 +100,7 @@ PROTOTYPES = {
     "qlmb_gemv_decode_norm_stack": (ci, [vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, vp]),
     "qlmb_dec_qkv": (ci, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, vp]),
     "qlmb_gemv_decode_res_norm": (ci, [vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, vp]),
+    "qlmb_selftest_rounding": (ci, [ci, ci, ci, vp, vp]),
     "qlmb_quiet_begin": (ci, [vp]),
     "qlmb_quiet_end": (ci, []),
     "qlmb_dec_step_bytes": (sz, [ci] * 8),

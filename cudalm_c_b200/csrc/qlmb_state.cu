@@ -428,8 +428,8 @@ __global__ void __launch_bounds__(256) k_step_fast(StepArgs a)
 //    intermediate underflows: the path is taken only for y in [2^-40, 1]; below |x| = 2^-100 the quotient is so
 //    small that only its sign and whether it is zero reach the rounding, and both are preserved.  Any other
 //    group divides with the IEEE operator;
-//  * the root and the quotient of each element's update are taken the same way, two elements at a time, with a Newton
-//    step on the hardware's estimates (rcp_pair, sqrt_pair), wherever the lane's smallest and largest moments exclude
+//  * the root and the quotient of each element's update are taken the same way, two elements at a time (rcp_pair, sqrt_pair:
+//    Markstein's forms on the hardware's estimates), wherever the lane's smallest and largest moments exclude
 //    underflow, zero and NaN; other lanes use the IEEE operators;
 //  * the carry c with rr - 128c in [-64, 64] (rr = +-64 does not carry) is the integer nearest to rr / 128 * (1 - 2^-21):
 //    the factor takes every tie (odd multiples of 64) towards zero and moves nothing else across one, as |rr| < 2^20 + 256;
@@ -496,9 +496,12 @@ __device__ __forceinline__ float2 sround_magic(float2 v, uint32_t h0, uint32_t h
     asm("mul.rn.sat.f32 %0, %1, 0fFF000000;" : "=f"(p.y) : "f"(t.y));
     return pk_add(m, p);
 }
-// RN(1 / y) for a pair of normal numbers whose reciprocals are normal: the hardware's estimate and one Newton step,
-// equal to the IEEE reciprocal for every one of the 2^23 significands (counted on the device; the estimate depends on
-// the significand alone).
+// The next three are Markstein's forms for a machine with fused multiply-add (P. W. Markstein, Computation of elementary
+// functions on the IBM RISC System/6000 processor, IBM J. Res. Develop. 34, 1990), started from the hardware's estimates.
+// qlmb_selftest_rounding compares them with the IEEE operations over every number that k_step_pk hands them.
+//
+// RN(1 / y) for a pair: one Newton step with a fused residual from an estimate within one unit in the last place, which is
+// what PTX states for rcp.approx.ftz.  The theorem leaves out significands of ones only; the count covers them.
 __device__ __forceinline__ float2 rcp_pair(float2 y)
 {
     float2 r;
@@ -506,7 +509,8 @@ __device__ __forceinline__ float2 rcp_pair(float2 y)
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(y.y));
     return pk_fma(pk_fma(make_float2(-y.x, -y.y), r, bc2(1.0f)), r, r);
 }
-// RN(x / y) for a pair, r = RN(1 / y), nothing underflowing: see above k_step_pk
+// RN(x / y) for a pair, r = RN(1 / y), nothing underflowing (see above k_step_pk): q + (x - q y) r is the rounded quotient
+// for every q within one unit in the last place of it, which the first of the two steps makes x r
 __device__ __forceinline__ float2 div_pair(float2 x, float2 y, float2 r)
 {
     const float2 ny = make_float2(-y.x, -y.y);
@@ -520,9 +524,9 @@ __device__ __forceinline__ float2 div_pair(float2 x, float y, float r, float rl)
     const float2 q = pk_fma(x, bc2(r), pk_mul(x, bc2(rl)));
     return pk_fma(pk_fma(q, bc2(-y), x), bc2(r), q);
 }
-// RN(sqrt(x)) for a pair in [2^-80, 2^80]: g = x / sqrt(x) from the hardware's estimate and one correction
-// g + (x - g * g) / (2 sqrt(x)), equal to the IEEE square root for every significand and both parities of the exponent
-// (counted on the device)
+// RN(sqrt(x)) for a pair in [2^-80, 2^40]: g = x / sqrt(x) from the estimate and g + (x - g g) / (2 sqrt(x)) with the residual
+// fused.  The theorem wants g within one unit in the last place; the estimate's stated error (2^-22.9) does not promise
+// that for every x, the count does.
 __device__ __forceinline__ float2 sqrt_pair(float2 x)
 {
     float2 y;
@@ -651,7 +655,9 @@ __global__ void __launch_bounds__(256, 4) k_step_pk(const __grid_constant__ Step
         am = max3_nan(am, mn[p].x, mn[p].y); amn = min3_nan(amn, mn[p].x, mn[p].y);
         vm = max3_nan(vm, rv[p].x, rv[p].y); vmn = min3_nan(vmn, rv[p].x, rv[p].y);
     }
-    // the lane's numbers stay where no step of the root and the quotients below can underflow or overflow, and none is zero or NaN
+    // the lane's numbers stay where no step of the root and the quotients below can underflow or overflow, and none is zero
+    // or NaN: roots in [2^-40, 2^20], denominators in [1e-8, 2^41] (veps is in them), numerators in [2^-80, 2^80], quotients
+    // in [2^-121, 2^107]
     const bool ok = amn >= 8.6736174e-19f && am <= 1.1529215e18f && vmn >= 8.2718061e-25f && vm <= 1.0995116e12f && vs_old <= 1048576.0f && a.bc_ok;
     if (ok) {
         vm = sqrt_one(vm);                                            // the root is monotone
@@ -764,6 +770,39 @@ __global__ void __launch_bounds__(256, 4) k_step_pk(const __grid_constant__ Step
     } else {
         st8_even(a.m8 + qe, mo); st8_even(a.v8 + qe, vo);
     }
+}
+
+// ---- rcp_pair, sqrt_pair / sqrt_one and the two div_pair forms against the IEEE operations.  Forms 0 and 1: every
+// significand under every exponent of the range, two neighbours to a pair.  Forms 2 and 3: x / y for 2^23 drawn pairs per
+// exponent of y, x within 2^+-60 of it.
+__global__ void __launch_bounds__(256) k_selftest_rounding(int form, int exp_lo, unsigned long long *bad)
+{
+    const uint32_t m = (blockIdx.x * 256 + threadIdx.x) * 2, e = (uint32_t)(exp_lo + (int)blockIdx.y + 127) << 23;
+    const float2 y = make_float2(__uint_as_float(e | m), __uint_as_float(e | (m + 1)));
+    int n = 0;
+    if (form == 0) {
+        const float2 r = rcp_pair(y);
+        n = (r.x != __frcp_rn(y.x)) + (r.y != __frcp_rn(y.y));
+    } else if (form == 1) {
+        const float2 g = sqrt_pair(y);
+        n = (g.x != __fsqrt_rn(y.x)) + (g.y != __fsqrt_rn(y.y)) + (sqrt_one(y.x) != g.x) + (sqrt_one(y.y) != g.y);
+    } else {
+        const uint32_t h0 = mix32(((uint64_t)blockIdx.y << 32 | m) * QLMB_HASH_I), h1 = mix32(((uint64_t)blockIdx.y << 32 | (m + 1)) * QLMB_HASH_I);
+        auto draw = [&](uint32_t h) {
+            const int ex = exp_lo + (int)blockIdx.y + (int)(h >> 24) % 121 - 60;
+            return __uint_as_float((h << 31) | ((uint32_t)(ex + 127) << 23) | (h & 0x7fffffu));
+        };
+        const float2 x = make_float2(draw(h0), draw(h1));
+        float2 q;
+        if (form == 2) q = div_pair(x, y, rcp_pair(y));
+        else {                                               // many x over one y
+            const float2 d = make_float2(y.x, y.x), r = rcp_pair(d), rl = pk_mul(pk_fma(make_float2(-d.x, -d.y), r, bc2(1.0f)), r);
+            q = div_pair(x, d.x, r.x, rl.x);
+        }
+        n = (q.x != __fdiv_rn(x.x, y.x)) + (q.y != __fdiv_rn(x.y, form == 2 ? y.y : y.x));
+    }
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (n && (threadIdx.x & 31) == 0) atomicAdd(bad, (unsigned long long)n);
 }
 
 // ------------------------------------------------------------------ encode
@@ -1078,6 +1117,17 @@ extern "C" int qlmb_servo(int8_t *d, int8_t *r, float *s, const qlmb_span *sp, i
     if (ngrp <= 0) return QLMB_OK;
     k_servo<<<(ngrp + 7) / 8, 256, 0, as_stream(stream)>>>(d, r, s, sp, nspan, ngrp, group, dmax, f_hi, f_lo, packed);
     QLMB_LAUNCH_CHECK("k_servo");
+    return QLMB_OK;
+}
+
+extern "C" int qlmb_selftest_rounding(int form, int exp_lo, int exp_hi, unsigned long long *mismatches, void *stream)
+{
+    QLMB_REQUIRE(form >= 0 && form <= 3 && exp_lo >= -100 && exp_hi <= 100 && exp_lo <= exp_hi && (form < 2 || (exp_lo >= -40 && exp_hi <= 41)) && mismatches,
+                 "qlmb_selftest_rounding: form %d, exponents %d..%d", form, exp_lo, exp_hi);
+    cudaStream_t st = as_stream(stream);
+    QLMB_CUDA(cudaMemsetAsync(mismatches, 0, sizeof *mismatches, st));
+    k_selftest_rounding<<<dim3(1u << 14, (unsigned)(exp_hi - exp_lo + 1)), 256, 0, st>>>(form, exp_lo, mismatches);
+    QLMB_LAUNCH_CHECK("k_selftest_rounding");
     return QLMB_OK;
 }
 

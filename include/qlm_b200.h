@@ -75,6 +75,12 @@ int qlmb_selftest_wait_expires(int polls, void *stream);
  * first-load latency and the tail cost at that size; bench.py reports it beside the GEMV's. */
 int qlmb_selftest_stream_read(const void *W, unsigned long long row_bytes, int rows, int kslices, void *stream);
 
+/* No counterpart in the reference.  Counts where the integer AdamW's own reciprocal (form 0), square root (1) and quotients
+ * (2: per element, 3: many over one divisor) differ from the IEEE operations, for binary exponents exp_lo..exp_hi of the
+ * operand or divisor: every significand for forms 0 and 1, drawn dividends within 2^+-60 of the divisor for 2 and 3 (these
+ * within -40..41).  `mismatches` receives one number. */
+int qlmb_selftest_rounding(int form, int exp_lo, int exp_hi, unsigned long long *mismatches, void *stream);
+
 /* Work that does not depend on each other inside one call (the three expert weight-gradient GEMMs
  * of the MoE backward against d(act) and dX, the router's backward chain against all of them) runs on
  * library-owned side streams (two per device) and is joined back into the caller's stream before the

@@ -151,6 +151,46 @@ def test_step_of_spans_at_any_even_element_matches_oracle(cuda, oracle, sizes):
         assert (P.cpu().numpy() == Ph).all()
 
 
+@pytest.mark.parametrize("form,lo,hi", [(0, -40, 41), (1, -80, 40), (2, -27, 41), (3, -40, 0)])
+def test_roots_and_quotients_equal_the_ieee_operations(cuda, form, lo, hi):
+    """Every significand under every exponent that the packed step's guard admits (reciprocals and roots), 2^23 drawn
+    dividends for each exponent of the divisor (quotients): no result differs."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200._lib import ptr, stream_ptr
+    bad = torch.full((1,), -1, dtype=torch.int64, device=cuda)
+    q.check(q.lib().qlmb_selftest_rounding(form, lo, hi, ptr(bad), stream_ptr()))
+    assert int(bad) == 0
+
+
+@pytest.mark.parametrize("inv_bc1,inv_sqrt_bc2", [(2.0 ** 20, 2.0 ** -20), (2.0 ** -20, 2.0 ** 20), (1.0, 1.0), (2.0 ** 20, 1.0), (2.0 ** 21, 0.0)])
+def test_step_with_extreme_moments_and_corrections_matches_oracle(cuda, oracle, inv_bc1, inv_sqrt_bc2):
+    """First moments up to 2^59 over roots down to 2^-39, and the other way round, under every bias correction that the
+    entry point takes: quotients beyond the largest float keep their sign, small ones their rounding."""
+    rng = np.random.default_rng(13)
+    st = DevState(cuda, [128 * 64], 128, 7, 1)
+    P0 = (rng.standard_normal(st.nq) * 0.02).astype(f32)
+    st.encode(dev(P0, cuda))
+    h = st.host()
+    d, r, s = h["d"].copy(), h["r"].copy(), h["s"].copy()
+    st.sp["sref"] = f32(s.astype(np.float64).mean()); st.push_spans()
+    m8 = rng.integers(-127, 128, st.nq).astype(np.int8); v8 = rng.integers(0, 256, st.nq).astype(np.uint8)
+    m8[:128 * 32] |= 1; v8[:128 * 32] |= 1                                   # half of the groups without a zero moment
+    e = rng.integers(0, 4, st.ng)
+    m8s = np.ldexp(f32(1), np.array([53, -59, 0, -10])[e]).astype(f32)
+    v8s = np.ldexp(f32(1), np.array([-39, 11, -12, -39])[e]).astype(f32)
+    G = (rng.standard_normal(st.nq) * 1e-12).astype(f32)
+    for k, v in dict(m8=m8, v8=v8, m8s=m8s, v8s=v8s).items():
+        getattr(st, k).copy_(torch.from_numpy(v))
+    st.q.qlm_step_launch(None, dev(G, cuda), st.d, st.r, st.s, st.m8, st.m8s, st.v8, st.v8s, st.spd, len(st.sp), 128, 7, 3e-4, 0.9,
+                         0.95, 0.1, 1.0, None, inv_bc1, inv_sqrt_bc2, 0, 1, 1, None, 1, 0, st.ng)
+    Ph = np.zeros(st.nq, f32)
+    oracle.step(Ph, G, d, r, s, m8, m8s, v8, v8s, st.sp, lr=3e-4, b1=0.9, b2=0.95, wd=0.1, gscale=1.0, inv_bc1=inv_bc1,
+                inv_sqrt_bc2=inv_sqrt_bc2, t=1)
+    h = st.host()
+    for k, v in dict(d=d, r=r, m8=m8, v8=v8, m8s=m8s, v8s=v8s).items():
+        assert (h[k] == v).all(), (k, int((h[k] != v).sum()))
+
+
 def test_step_sharded_equals_whole(cuda):
     """ZeRO-1 style split: stepping group ranges separately gives the same bytes."""
     rng = np.random.default_rng(6)
