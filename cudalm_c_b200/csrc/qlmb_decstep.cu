@@ -38,6 +38,8 @@ struct DsLayer {                                          // the device table's 
     float *gate;
 };
 constexpr int DS_LAYER_WORDS = sizeof(DsLayer) / 8;
+// alignment of the row's w-th pointer: 16 bytes where it is read in 16-byte pieces (the experts' codes, gains, router, caches)
+__device__ __forceinline__ unsigned ds_align_mask(int w) { return (w >= 4 && w < 7) || (w >= 14 && w < 19) ? 15u : 3u; }
 
 struct DsArgs {
     const DsLayer *layers;
@@ -692,7 +694,15 @@ __global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constan
     load_layer(0);
     if (threadIdx.x < DS_MAX_B) sh.pos[threadIdx.x] = (int)threadIdx.x < a.B ? __ldg(a.pos + threadIdx.x) : 0;
     if (threadIdx.x == 0) sh.target = 0u;
-    __syncthreads();
+    // Every CTA looks the whole table over (2 KB from L2, beside the loads above): a pointer that is missing or not aligned
+    // for its loads is reported, and the whole grid leaves before its first barrier.
+    int bad = 0;
+    for (int i = threadIdx.x; i < a.L * DS_LAYER_WORDS; i += DS_THREADS) {
+        const unsigned long long p = __ldg(reinterpret_cast<const unsigned long long *>(a.layers) + i);
+        if (!p || (p & ds_align_mask(i % DS_LAYER_WORDS))) bad = 1 + i;
+    }
+    if (bad && blockIdx.x == 0) report_bad_index(a.errword, 304, (bad - 1) / DS_LAYER_WORDS, (bad - 1) % DS_LAYER_WORDS);
+    if (__syncthreads_or(bad)) return;
     if (ds_row(a) >= 0) {                                 // embedding row and the first norm
         const int b = ds_row(a), n = 4 * threadIdx.x;
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -768,11 +778,14 @@ extern "C" int qlmb_dec_step(const qlmb_dec_step_args *p, void *stream)
 {
     QLMB_REQUIRE(p && p->layers && p->emb && p->tok && p->pos && p->cosb && p->sinb && p->nf && p->fn && p->ws, "qlmb_dec_step: NULL argument");
     QLMB_REQUIRE(p->L > 0, "qlmb_dec_step: L=%d", p->L);
+    QLMB_REQUIRE((((uintptr_t)p->emb | (uintptr_t)p->nf | (uintptr_t)p->fn) & 15) == 0 && ((uintptr_t)p->layers & 7) == 0 &&
+                 (((uintptr_t)p->tok | (uintptr_t)p->pos | (uintptr_t)p->cosb | (uintptr_t)p->sinb) & 3) == 0,
+                 "qlmb_dec_step: emb, nf and fn must be 16-byte aligned, layers 8, tok, pos, cosb and sinb 4");
+    QLMB_REQUIRE(((uintptr_t)p->ws & 255) == 0, "qlmb_dec_step: the workspace must be 256-byte aligned");
     if (!ds_fits(p->B, p->Tm, p->D, p->H, p->KV, p->F, p->E, p->K)) {
         set_error("qlmb_dec_step: shape B %d Tm %d D %d H %d KV %d F %d E %d K %d is not supported", p->B, p->Tm, p->D, p->H, p->KV, p->F, p->E, p->K);
         return QLMB_E_UNSUPPORTED;
     }
-    QLMB_REQUIRE(((uintptr_t)p->ws & 255) == 0, "qlmb_dec_step: the workspace must be 256-byte aligned");
     const DsLayout w = ds_layout(p->B, p->D, p->KV * 64, p->F, p->K);
     uint8_t *ws = (uint8_t *)p->ws;
     DsArgs a = {};

@@ -264,10 +264,13 @@ int qlmb_gemv_decode(void *Y, const void *X, const int8_t *codes, const float *s
  * residual + norm + router + routed experts, and the final norm into fn [B][D] (bf16), the head's input.  `layers` is a
  * DEVICE table of L rows of 23 pointers: codes of wq, wk, wv, wo, w1, w3, w2; their scales in the same order; an1, an2,
  * wr; the K and V caches [B][Tm][KV*64] (bf16); and the members rt, rprobs, assign, gate of the layer's MoE arena,
- * which are filled as qlmb_moe_decode fills them.  ws = qlmb_dec_step_bytes(...) bytes, 256-byte aligned, zeroed once
- * before its first use, not shared by steps that may overlap; a size of 0 means that the shape is not supported
- * (supported: head dimension 64, D <= 1024, at most 8 slots, 32 experts and 32 routed slots, a CTA per attention item
- * and row on the device) and the separate entry points do the step.  A slot whose position is outside its cache is reported and neither read nor written. */
+ * which are filled as qlmb_moe_decode fills them.  Of the row's pointers the codes of w1, w3, w2, the gains, wr and the
+ * caches must be 16-byte aligned, the others 4; a row that breaks this is reported through the device error word (site
+ * 304) and the step does nothing.  emb, nf and fn must be 16-byte aligned, the table 8.  ws = qlmb_dec_step_bytes(...)
+ * bytes, 256-byte aligned, zeroed once before its first use, not shared by steps that may overlap; a size of 0 means that
+ * the shape is not supported (supported: head dimension 64, D <= 1024, at most 8 slots, 32 experts and 32 routed slots, a
+ * CTA per attention item and row on the device) and the separate entry points do the step.  A slot whose position is
+ * outside its cache is reported and neither read nor written. */
 typedef struct qlmb_dec_step_args {
     int B, Tm, L, D, H, KV, F, E, K;
     const void *layers;

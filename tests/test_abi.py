@@ -96,6 +96,19 @@ def test_new_entry_points_reject_bad_arguments_without_a_gpu():
     assert L.qlmb_selftest_stream_read(None, 256, 8, 1, None) == 1
 
 
+def test_dec_step_rejects_misaligned_arguments_without_a_gpu():
+    import cudalm_c_b200 as q
+    from cudalm_c_b200._lib import DecStepArgs
+    L = q.lib()
+    shape = (2, 64, 2, 256, 4, 4, 256, 8, 2)
+    good = [4096] * 9
+    for i, (off, needle) in enumerate([(4, b"aligned"), (8, b"aligned"), (2, b"aligned"), (1, b"aligned"), (2, b"aligned"), (2, b"aligned"),
+                                       (4, b"aligned"), (8, b"aligned"), (128, b"256-byte")]):
+        bad = list(good)
+        bad[i] += off
+        assert L.qlmb_dec_step(DecStepArgs(*shape, *bad), None) == 1 and needle in L.qlmb_last_error(), i
+
+
 def test_header_is_plain_c_and_links_from_c(tmp_path):
     """include/qlm_b200.h compiles as C99 with warnings as errors and a C program linked against the library runs the
     argument-error paths (status + message, no exit) on a machine without a GPU."""

@@ -145,6 +145,32 @@ def test_sampler_topk_topp_temperature(cuda):
     q.check(q.lib().qlmb_check_device(None))
 
 
+def test_one_launch_step_reports_a_misaligned_table(cuda):
+    """A pointer of the device table that its loads cannot take: reported, nothing read through it, nothing written; the
+    next step runs as usual."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import model
+    from cudalm_c_b200._lib import stream_ptr
+    cfg = model.Config(L=2, D=256, H=4, KV=4, hd=64, E=8, K=2, F=256, V=512, T=64, B=1)
+    m = model.QlmModel(cfg, cuda, seed=3)
+    d = model.Decoder(m, 2, 64)
+    d.prefill(torch.randint(0, cfg.V, (2, 5), dtype=torch.int32, device=cuda))
+    plan = d._step_plan()
+    q.check(q.lib().qlmb_dec_step(plan, stream_ptr()))
+    want = d.fn.clone()
+    for l, word, off in ((0, 14, 4), (1, 4, 8), (1, 17, 2), (1, 22, 1), (0, 9, None)):
+        keep = d._table[l, word].clone()
+        d._table[l, word] = 0 if off is None else keep + off
+        d.fn.fill_(7.0)
+        q.check(q.lib().qlmb_dec_step(plan, stream_ptr()))
+        assert q.lib().qlmb_check_device(None) != 0 and b"site 304, block %d, detail %d" % (l, word) in q.lib().qlmb_last_error()
+        assert bool((d.fn == 7.0).all())
+        d._table[l, word] = keep
+        q.check(q.lib().qlmb_dec_step(plan, stream_ptr()))
+        q.check(q.lib().qlmb_check_device(None))
+        assert torch.equal(d.fn, want)
+
+
 @pytest.mark.parametrize("B,D,KV,E,K,F,fill,Tm", [
     (1, 256, 4, 8, 2, 256, 1, 64),          # one key before the new one
     (1, 768, 12, 32, 2, 1536, 255, 640),    # the last key of a 256-key pass is the new one
