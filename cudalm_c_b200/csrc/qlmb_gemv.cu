@@ -646,7 +646,8 @@ __global__ void __launch_bounds__(32 * NW, MT == 1 ? 16 / NW : (NW == 8 ? 1 : 3)
     float *ssc = reinterpret_cast<float *>(msm + (size_t)GR * ldx * sizeof(bf16));
     {
         const int g0 = blockIdx.x * (CW / 128), gmax = N / 128 - 1;
-        if (g0 + NG - 1 <= gmax && (srow & (NG - 1)) == 0) {      // NG neighbouring scales of a row in one load
+        // NG neighbouring scales of a row in one load, where every row's and the matrix's own address allow it
+        if (g0 + NG - 1 <= gmax && (srow & (NG - 1)) == 0 && ((uintptr_t)scales & (4 * NG - 1)) == 0) {
             typedef typename VecOfF<NG>::T V;
             for (int i = threadIdx.x; i < kslice; i += NT)
                 reinterpret_cast<V *>(ssc)[i] = ld_w<AHEAD>(reinterpret_cast<const V *>(scales + (size_t)(k0 + i) * srow + g0));

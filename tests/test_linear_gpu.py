@@ -215,6 +215,20 @@ def test_gemv_decode_edges(cuda, B):
                     assert rel(linear.gemv_decode(odd, Q.d, Q.s, lay, N), ref) < tol, (K, N, lay, dt)
 
 
+@pytest.mark.parametrize("N", [768, 1024, 2304])
+def test_gemv_decode_scales_at_any_group(cuda, N):
+    """The scales of a matrix that follows another span may start at any float."""
+    from cudalm_c_b200 import linear
+    from cudalm_c_b200._lib import KN
+    K = 256
+    Q, W = quantise(cuda, K, N, 5)
+    for off in (1, 2, 3):
+        s = torch.empty(Q.s.numel() + off, device=cuda)[off:].copy_(Q.s)
+        for B in (5, 17, 40):
+            X = torch.randn(B, K, device=cuda).bfloat16()
+            assert torch.equal(linear.gemv_decode(X, Q.d, s, KN, N), linear.gemv_decode(X, Q.d, Q.s, KN, N)), (off, B)
+
+
 def test_gemv_rejects_more_than_64_slots(cuda):
     import cudalm_c_b200 as q
     from cudalm_c_b200 import linear
