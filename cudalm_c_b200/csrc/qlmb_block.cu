@@ -557,12 +557,18 @@ __global__ void __launch_bounds__(128) k_dec_attn(bf16_t *O, const bf16_t *Q, co
     __syncthreads();
     l = (red[0] + red[1]) + (red[2] + red[3]);
     float a[8] = {};
+    const bool v16 = ((uintptr_t)Vc & 15) == 0;          // (a value cache may start at any pair of elements)
     for (int s0 = lo + 4 * warp; s0 <= t; s0 += 64) {
         uint4 x[4]; float p[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const int s = s0 + 16 * u + row;
-            x[u] = *reinterpret_cast<const uint4 *>(vb + (size_t)(s <= t ? s : t) * KD);
+            const bf16_t *v = vb + (size_t)(s <= t ? s : t) * KD;
+            if (v16) x[u] = *reinterpret_cast<const uint4 *>(v);
+            else {
+                const uint32_t *w = reinterpret_cast<const uint32_t *>(v);
+                x[u] = make_uint4(w[0], w[1], w[2], w[3]);
+            }
             p[u] = s <= t ? sc[s] : 0.0f;
         }
 #pragma unroll

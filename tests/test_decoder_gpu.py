@@ -145,6 +145,30 @@ def test_sampler_topk_topp_temperature(cuda):
     q.check(q.lib().qlmb_check_device(None))
 
 
+@pytest.mark.parametrize("win", [0, 100])
+def test_decode_attention_with_values_at_any_pair(cuda, win):
+    """A value cache that starts at a 4-byte address: the same bits as one that starts at 16."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200._lib import ptr, stream_ptr
+    B, Tm, H, KV = 6, 300, 8, 4
+    Q = torch.randn(B, H * 64, device=cuda).bfloat16()
+    K, V = (torch.randn(B, Tm, KV * 64, device=cuda).bfloat16() for _ in range(2))
+    pos = torch.tensor([0, 1, 63, 64, 200, 299], dtype=torch.int32, device=cuda)
+    outs = []
+    for off in (0, 2, 4, 6):
+        v = torch.empty(V.numel() + off, dtype=V.dtype, device=cuda)[off:].view_as(V).copy_(V)
+        O = torch.empty_like(Q)
+        q.check(q.lib().qlmb_dec_attn(ptr(O), ptr(Q), ptr(K), ptr(v), ptr(pos), win, B, Tm, H, KV, 64, stream_ptr()))
+        outs.append(O)
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    for b in range(B):
+        t = int(pos[b]); lo = max(0, t - win + 1) if win else 0
+        k, v = (c[b, lo:t + 1].float().view(-1, KV, 64).repeat_interleave(H // KV, 1) for c in (K, V))
+        p = torch.softmax(torch.einsum("hd,shd->hs", Q[b].float().view(H, 64), k) / 8.0, 1)
+        ref = torch.einsum("hs,shd->hd", p, v).reshape(-1)
+        assert float((outs[0][b].float() - ref).norm() / ref.norm()) < 1e-2
+
+
 def test_one_launch_step_reports_a_misaligned_table(cuda):
     """A pointer of the device table that its loads cannot take: reported, nothing read through it, nothing written; the
     next step runs as usual."""
