@@ -442,32 +442,53 @@ class Decoder:
             self.sp[t] = self.sp[s]
 
     def _step_plan(self):
-        """Arguments of the one-launch form of a step's layers (qlmb_dec_step); None where the shape needs the chain of
-        separate operators.  Everything it points to lives as long as the decoder."""
-        if self._plan is not False:
-            return self._plan
+        """Arguments of the one-launch form of a step's layers (qlmb_dec_step); None where the chain of separate operators
+        has to do it: shapes and addresses that the form does not take, or layer tensors that were replaced since the last
+        step while a stream capture forbids uploading their addresses.  Every tensor is looked up at every step, as the
+        chain does."""
         import ctypes as C
         from ._lib import DecStepArgs, lib, ptr
         c, m = self.m.c, self.m
-        shape = (self.B, self.Tm, c.D, c.H, c.KV, c.F, c.E, c.K)
-        nbytes = lib().qlmb_dec_step_bytes(*shape) if c.hd == 64 else 0
-        if not nbytes:
-            self._plan = None
+        if self._plan is False:
+            shape = (self.B, self.Tm, c.D, c.H, c.KV, c.F, c.E, c.K)
+            nbytes = lib().qlmb_dec_step_bytes(*shape) if c.hd == 64 else 0
+            if not nbytes:
+                self._plan = None
+                return None
+            self._ws = torch.zeros(nbytes, dtype=torch.uint8, device=m.dev)
+            self.fn = torch.empty(self.B, c.D, dtype=torch.bfloat16, device=m.dev)
+            self._members = {}                           # arena -> addresses of its members
+            self._tables = {}                            # address lists -> device tables; a captured step keeps using its own
+            self._plan = DecStepArgs(self.B, self.Tm, c.L, *shape[2:])
+            self._plan.fn, self._plan.ws = ptr(self.fn), ptr(self._ws)
+            self._plan_addr = C.addressof(self._plan)
+        if self._plan is None:
             return None
         rows = []
-        for l, ly in enumerate(m.layers):
-            w, f, mo = ly["w"], m.fl[l], self.moes[l]
-            member = lambda nm: lib().qlmb_moe_arena_member(mo.arena_ptr, mo.N, mo.D, mo.F, mo.E, mo.K, nm)
-            rows.append([ptr(w[nm][i]) for i in (0, 1) for nm in QUANT[:4] + ("w1", "w3", "w2")] +
-                        [ptr(f["an1"]), ptr(f["an2"]), ptr(f["wr"]), ptr(self.K[l]), ptr(self.V[l])] +
-                        [member(nm) for nm in (b"rt", b"rprobs", b"assign", b"gate")])
-        self._table = torch.tensor(rows, dtype=torch.int64).to(m.dev)
-        self._ws = torch.zeros(nbytes, dtype=torch.uint8, device=m.dev)
-        self.fn = torch.empty(self.B, c.D, dtype=torch.bfloat16, device=m.dev)
-        self._plan = DecStepArgs(self.B, self.Tm, c.L, *shape[2:], ptr(self._table), ptr(m.emb), ptr(self.tok), ptr(self.pos),
-                                 ptr(self.cosb), ptr(self.sinb), ptr(m.nf), ptr(self.fn), ptr(self._ws))
-        self._plan_addr = C.addressof(self._plan)
-        return self._plan
+        for ly, f, mo, k, v in zip(m.layers, m.fl, self.moes, self.K, self.V):
+            w, e = [ly["w"][nm] for nm in QUANT[:4]], mo.c
+            if e.bias:
+                return None
+            arena = self._members.get(mo.arena_ptr)
+            if arena is None:
+                arena = self._members[mo.arena_ptr] = [lib().qlmb_moe_arena_member(mo.arena_ptr, mo.N, mo.D, mo.F, mo.E, mo.K, nm)
+                                                       for nm in (b"rt", b"rprobs", b"assign", b"gate")]
+            rows.append((*[ptr(t[0]) for t in w], e.w1_codes, e.w3_codes, e.w2_codes, *[ptr(t[1]) for t in w], e.w1_scales, e.w3_scales,
+                         e.w2_scales, ptr(f["an1"]), ptr(f["an2"]), e.wr, ptr(k), ptr(v), *arena))
+        rows = tuple(rows)
+        p = self._plan
+        p.emb, p.tok, p.pos, p.cosb, p.sinb, p.nf = ptr(m.emb), ptr(self.tok), ptr(self.pos), ptr(self.cosb), ptr(self.sinb), ptr(m.nf)
+        table = self._tables.get(rows)
+        if table is None:
+            if torch.cuda.is_current_stream_capturing():
+                return None
+            if any(q & 15 for r in rows for q in (*r[4:7], *r[14:19])) or any(q & 3 for r in rows for q in r):
+                return None
+            table = self._tables[rows] = torch.tensor(rows, dtype=torch.int64).to(m.dev)
+        if (p.emb | p.nf) & 15:
+            return None
+        p.layers = ptr(table)
+        return p
 
     def _layers_chain(self):
         """The layers of a step as separate operators: shapes the one-launch form does not take."""

@@ -169,6 +169,57 @@ def test_decode_attention_with_values_at_any_pair(cuda, win):
         assert float((outs[0][b].float() - ref).norm() / ref.norm()) < 1e-2
 
 
+def test_step_after_tensors_were_replaced(cuda):
+    """A caller's own token and position tensors, caches and gains in the place of the decoder's: the next step works on
+    them, also one at an address that only the chain takes; a step captured before keeps its own."""
+    from cudalm_c_b200 import model
+    cfg = model.Config(L=2, D=256, H=4, KV=4, hd=64, E=8, K=2, F=256, V=512, T=64, B=1)
+    m = model.QlmModel(cfg, cuda, seed=3)
+
+    def fresh():
+        d = model.Decoder(m, 2, 64)
+        g = torch.Generator(device=cuda); g.manual_seed(5)
+        d.prefill(torch.randint(0, cfg.V, (2, 5), dtype=torch.int32, device=cuda, generator=g))
+        return d
+    tok = torch.tensor([17, 401], dtype=torch.int32, device=cuda)
+    d = fresh()
+    d.tok.copy_(tok)
+    want = d.step(advance=False).clone()
+    d = fresh()
+    first = d.step(advance=False).clone()
+    assert not torch.equal(first, want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        d.step(advance=False)
+    captured = (d.tok, list(d.K), list(d.V))
+    d.tok = tok.clone()                                                      # by value in the launch
+    assert torch.equal(d.step(advance=False), want)
+    d.K = [t.clone() for t in d.K]                                           # in the table
+    for t in d.K:
+        t[:, :5].neg_()
+    other = d.step(advance=False).clone()
+    assert not torch.equal(other, want)
+    for t in d.K:
+        t[:, :5].neg_()
+
+    def values(off):
+        return [torch.empty(t.numel() + off, dtype=t.dtype, device=cuda)[off:].view_as(t).copy_(t) for t in captured[2]]
+    d.V = values(8)
+    assert torch.equal(d.step(advance=False), want)
+    d.V = values(2)                                                          # not on 16 bytes: the chain
+    assert d._step_plan() is None
+    got = d.step(advance=False)
+    assert float((got - want).norm() / want.norm()) < 2e-2
+    d.V = values(16)
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):                           # no address can be uploaded here: the chain
+        assert d._step_plan() is None
+        d.step(advance=False)
+    assert torch.equal(d.step(advance=False), want)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(d.logits, first)
+
+
 def test_one_launch_step_reports_a_misaligned_table(cuda):
     """A pointer of the device table that its loads cannot take: reported, nothing read through it, nothing written; the
     next step runs as usual."""
@@ -182,14 +233,15 @@ def test_one_launch_step_reports_a_misaligned_table(cuda):
     plan = d._step_plan()
     q.check(q.lib().qlmb_dec_step(plan, stream_ptr()))
     want = d.fn.clone()
+    table, = d._tables.values()
     for l, word, off in ((0, 14, 4), (1, 4, 8), (1, 17, 2), (1, 22, 1), (0, 9, None)):
-        keep = d._table[l, word].clone()
-        d._table[l, word] = 0 if off is None else keep + off
+        keep = table[l, word].clone()
+        table[l, word] = 0 if off is None else keep + off
         d.fn.fill_(7.0)
         q.check(q.lib().qlmb_dec_step(plan, stream_ptr()))
         assert q.lib().qlmb_check_device(None) != 0 and b"site 304, block %d, detail %d" % (l, word) in q.lib().qlmb_last_error()
         assert bool((d.fn == 7.0).all())
-        d._table[l, word] = keep
+        table[l, word] = keep
         q.check(q.lib().qlmb_dec_step(plan, stream_ptr()))
         q.check(q.lib().qlmb_check_device(None))
         assert torch.equal(d.fn, want)
