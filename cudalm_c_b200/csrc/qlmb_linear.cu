@@ -1,5 +1,6 @@
 // Quantised linear entry points (the reference's g_ab / g_abt / g_abt_b / g_atb
 // call sites, cudalm.cu:3133-3202) on top of the tcgen05 GEMM engine.
+#include <mutex>
 #include "qlmb_common.cuh"
 #include "qlmb_gemm.cuh"
 
@@ -23,6 +24,36 @@ int workspace(size_t bytes, void **out)
     *out = g_ws[dev];
     return QLMB_OK;
 }
+
+// Scratch of one call, in stream order: calls on several streams and threads get memory of their own, under capture it
+// belongs to the graph, and nothing that a captured call uses is ever replaced by a larger piece (the shared piece above
+// is).  A pool per device keeps up to 64 MB between calls (16 slices on 74 tiles take 20) and gives the rest back.
+struct StreamScratch {
+    void *p = nullptr;
+    cudaStream_t st;
+    explicit StreamScratch(cudaStream_t s) : st(s) {}
+    bool get(size_t bytes)
+    {
+        static std::mutex mu;
+        static cudaMemPool_t pools[64];
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (!pools[dev]) {
+                cudaMemPoolProps props = {};
+                props.allocType = cudaMemAllocationTypePinned;
+                props.location.type = cudaMemLocationTypeDevice; props.location.id = dev;
+                uint64_t keep = (uint64_t)64 << 20;
+                if (cudaMemPoolCreate(&pools[dev], &props) != cudaSuccess) { pools[dev] = nullptr; cudaGetLastError(); return false; }
+                cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+            }
+        }
+        if (cudaMallocFromPoolAsync(&p, bytes, pools[dev], st) != cudaSuccess) { p = nullptr; cudaGetLastError(); return false; }
+        return true;
+    }
+    ~StreamScratch() { if (p) cudaFreeAsync(p, st); }
+};
 
 // bf16 view of an activation matrix: the matrix itself, or a converted copy in `slot`
 static int as_bf16(const void *x, int dtype, size_t n, bf16 *slot, const bf16 **out, cudaStream_t st)
@@ -145,9 +176,16 @@ extern "C" int qlmb_linear_wgrad(float *dW, const void *dY, const void *X, int l
         while (S < 16 && tiles * S * 2 <= pairs && stages / (2 * S) >= 8) S *= 2;
     }
     const size_t conv = dtype == QLMB_F32 ? ((((size_t)M * K * 2 + 255) & ~(size_t)255) + (((size_t)M * N * 2 + 255) & ~(size_t)255)) : 0;
-    const size_t part_bytes = S > 1 ? (size_t)S * Md * Nd * sizeof(float) + 256 : 0;
+    // Rows that divide evenly keep their slices' partial sums in the shared piece, behind the converted operands: a step
+    // that is captured after a first eager one finds it large enough, and an allocation and a free node for each of its
+    // calls would cost 0.6 % of a training step.  Other row counts, which need no scratch uncut, take their own.
+    const size_t part_bytes = S > 1 ? (size_t)S * Md * Nd * sizeof(float) : 0;
+    const bool shared = S > 1 && M % (256 * S) == 0;
+    StreamScratch own(st);
+    if (S > 1 && !shared && !own.get(part_bytes)) S = 1;
     void *ws = nullptr;
-    if (conv + part_bytes) { rc = workspace(conv + part_bytes, &ws); if (rc) return rc; }
+    if (conv || shared) { rc = workspace(conv + (shared ? part_bytes : 0), &ws); if (rc) return rc; }
+    float *part = shared ? (float *)((uint8_t *)ws + conv) : (float *)own.p;
     const bf16 *xb, *gb;
     bf16 *slot2 = conv ? (bf16 *)((uint8_t *)ws + (((size_t)M * K * 2 + 255) & ~(size_t)255)) : nullptr;
     rc = as_bf16(X, dtype, (size_t)M * K, (bf16 *)ws, &xb, st);
@@ -159,14 +197,13 @@ extern "C" int qlmb_linear_wgrad(float *dW, const void *dY, const void *X, int l
     g.a[0] = layout == QLMB_KN ? xb : gb; g.a_rows = M; g.a_cols = Md;
     g.w[0] = layout == QLMB_KN ? gb : xb; g.w_cols = Nd; g.w_rows = 0;
     if (S > 1) {
-        float *part = (float *)((uint8_t *)ws + conv);
         g.sched = SCHED_GROUPK;
         g.nseg = 1; g.ksteps = (stages + S - 1) / S; g.M = Md; g.N = Nd; g.E = S;
         g.out = part; g.out_dtype = QLMB_F32; g.ldo = Nd; g.beta = 0.0f; g.name = "gemm_wgrad_slices";
         rc = gemm_launch(g, st);
         if (rc) return rc;
         const size_t n = (size_t)Md * Nd;
-        QLMB_CUDA(pdl_launch(true, k_sum_slices, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, st, dW, part, S, n, beta));
+        QLMB_CUDA(pdl_launch(true, k_sum_slices, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, st, dW, (const float *)part, S, n, beta));
         QLMB_LAUNCH_CHECK("k_sum_slices");
         return QLMB_OK;
     }

@@ -170,6 +170,47 @@ def test_linear_wgrad_of_ragged_row_slices(cuda, M):
                 assert rel(dW.view(ref.shape), ref * (1.0 + beta)) < 1e-4, (K, N, lay, beta)
 
 
+def test_linear_wgrad_of_slices_under_capture_and_on_two_streams(cuda):
+    """The slices' partial sums are each call's own: the first sliced call of its size may be a captured one, a replay
+    is not disturbed by larger calls since, and two streams may run such calls at once."""
+    from cudalm_c_b200 import linear
+    from cudalm_c_b200._lib import KN
+    K = N = 256
+
+    def operands(M, seed):
+        g = torch.Generator(device=cuda); g.manual_seed(seed)
+        return tuple(torch.randn(M, n, device=cuda, generator=g).bfloat16() for n in (N, K)) + (torch.zeros(K * N, device=cuda),)
+    linear.linear_wgrad(torch.zeros(K * N, device=cuda), *operands(100, 0)[:2], KN, beta=0.0)
+    dy, x, dw = operands(5003, 1)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        linear.linear_wgrad(dw, dy, x, KN, beta=0.0)
+    big = operands(40001, 2)
+    linear.linear_wgrad(big[2], big[0], big[1], KN, beta=0.0)
+    for _ in range(3):
+        dw.fill_(-1.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert rel(dw.view(K, N), x.float().T @ dy.float()) < 1e-4
+    eager = torch.empty_like(dw)
+    linear.linear_wgrad(eager, dy, x, KN, beta=0.0)
+    assert torch.equal(eager, dw)
+    streams, sets = [torch.cuda.Stream() for _ in range(2)], [operands(9001, 3), operands(9001, 4)]
+    want = []
+    for a in sets:
+        linear.linear_wgrad(a[2], a[0], a[1], KN, beta=0.0)
+        want.append(a[2].clone())
+    outs = [[torch.empty_like(dw) for _ in range(50)] for _ in range(2)]
+    torch.cuda.synchronize()
+    for i in range(50):
+        for s, a, o in zip(streams, sets, outs):
+            with torch.cuda.stream(s):
+                linear.linear_wgrad(o[i], a[0], a[1], KN, beta=0.0)
+    torch.cuda.synchronize()
+    assert all(torch.equal(t, w) for o, w in zip(outs, want) for t in o)
+
+
 @pytest.mark.parametrize("B", [1, 8, 64])
 def test_gemv_decode(cuda, oracle, B):
     """Decode path (M = live slots <= 64).  fp32 activations: fp32 accumulation of exact dequantised weights (the
