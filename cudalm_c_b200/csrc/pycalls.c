@@ -1,16 +1,18 @@
 /* The entry points that a training step or a decode step calls many times, as plain C calls for Python: a ctypes call
  * converts each argument through its argtypes (about 2 us for ten), this takes them as they come.  A pointer argument is a
  * tensor (anything with data_ptr()), an address or None; a status other than 0 raises the exception class that
- * set_error() was given, with qlmb_last_error()'s text.  The remaining entry points are reached through ctypes. */
+ * set_error_class() was given, with qlmb_last_error()'s text.  The remaining entry points are reached through ctypes. */
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include "../../include/qlm_b200.h"
 
 static PyObject *error_class, *name_data_ptr;
 
+/* The converters run in the order of the arguments.  After the first that failed the others do nothing: no Python code
+ * may run with an exception set, and the caller is to see that one. */
 static void *as_ptr(PyObject *o)
 {
-    if (o == Py_None) return NULL;
+    if (o == Py_None || PyErr_Occurred()) return NULL;
     if (PyLong_CheckExact(o)) return PyLong_AsVoidPtr(o);
     PyObject *r = PyObject_CallMethodNoArgs(o, name_data_ptr);
     if (!r) return NULL;
@@ -18,9 +20,16 @@ static void *as_ptr(PyObject *o)
     Py_DECREF(r);
     return p;
 }
-static int as_int(PyObject *o) { return (int)PyLong_AsLong(o); }
-static float as_float(PyObject *o) { return (float)PyFloat_AsDouble(o); }
-static unsigned long long as_u64(PyObject *o) { return PyLong_AsUnsignedLongLong(o); }
+static int as_int(PyObject *o)
+{
+    if (PyErr_Occurred()) return 0;
+    const long v = PyLong_AsLong(o);
+    if (v == (int)v) return (int)v;
+    PyErr_SetString(PyExc_OverflowError, "argument does not fit a C int");
+    return 0;
+}
+static float as_float(PyObject *o) { return PyErr_Occurred() ? 0.0f : (float)PyFloat_AsDouble(o); }
+static unsigned long long as_u64(PyObject *o) { return PyErr_Occurred() ? 0 : PyLong_AsUnsignedLongLong(o); }
 
 static PyObject *done(int rc)
 {

@@ -96,6 +96,34 @@ def test_new_entry_points_reject_bad_arguments_without_a_gpu():
     assert L.qlmb_selftest_stream_read(None, 256, 8, 1, None) == 1
 
 
+def test_native_calls_report_the_first_wrong_argument():
+    """A conversion that fails leaves its own exception: no later argument's data_ptr() runs, no number is cut to an int."""
+    from cudalm_c_b200._lib import QlmbError, calls
+
+    class Tensor:
+        asked = 0
+
+        def data_ptr(self):
+            Tensor.asked += 1
+            return 4096
+    t = Tensor()
+    with pytest.raises(TypeError):
+        calls.embed(t, "bf16", t, t, 8, 8, None)
+    assert Tensor.asked == 1
+    with pytest.raises(AttributeError):
+        calls.embed(object(), 1, t, t, 8, 8, None)
+    assert Tensor.asked == 1
+    for big in (2 ** 32 + 8, -2 ** 31 - 1, 2 ** 70):
+        with pytest.raises(OverflowError):
+            calls.embed(t, 1, t, t, big, 8, None)
+    with pytest.raises(TypeError):
+        calls.gnorm(t, 1.5, None, None, 0, 0, t, None)
+    with pytest.raises(TypeError):
+        calls.embed(t, 1, t)
+    with pytest.raises(QlmbError, match="qlmb_embed"):
+        calls.embed(None, 1, t, t, 8, 8, None)
+
+
 def test_dec_step_rejects_misaligned_arguments_without_a_gpu():
     import cudalm_c_b200 as q
     from cudalm_c_b200._lib import DecStepArgs
