@@ -214,7 +214,7 @@ class _Calls:
         try:
             from . import _pycalls
         except ImportError as e:
-            raise QlmbError("_pycalls.so does not load (%s): build it with `python -m cudalm_c_b200.build`" % e)
+            raise QlmbError("the _pycalls extension does not load (%s): build it with `python -m cudalm_c_b200.build`" % e)
         _pycalls.set_error_class(QlmbError)
         f = getattr(_pycalls, name)
         setattr(self, name, f)                           # later uses find it in the instance

@@ -19,7 +19,9 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libqlm_b200.so")
 OBJ = os.path.join(HERE, "build")
-PYCALLS = os.path.join(HERE, "_pycalls.so")          # plain C calls of the hot entry points for Python (csrc/pycalls.c)
+# plain C calls of the hot entry points for Python (csrc/pycalls.c), under the name that only the interpreter loads whose
+# headers it was built with
+PYCALLS = os.path.join(HERE, "_pycalls" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 # translation unit -> extra flags
 UNITS = {
@@ -75,6 +77,9 @@ def build(force=False, verbose=False):
     if force or procs or not os.path.exists(OUT):
         cmd = [nvcc, "-shared", "-cudart", "static", "-o", OUT] + objs + ["-Xlinker", "--no-undefined", "-lpthread", "-ldl", "-lrt"]
         subprocess.check_call(cmd)
+    untagged = os.path.join(HERE, "_pycalls.so")         # the name of earlier builds, which any Python 3 would load
+    if os.path.exists(untagged):
+        os.remove(untagged)
     src = os.path.join(CSRC, "pycalls.c")
     if force or _newer(src, PYCALLS, headers):
         subprocess.check_call([os.environ.get("CC", "gcc"), "-shared", "-fPIC", "-O2", "-Wall", "-I", sysconfig.get_paths()["include"], "-o", PYCALLS, src,

@@ -96,6 +96,16 @@ def test_new_entry_points_reject_bad_arguments_without_a_gpu():
     assert L.qlmb_selftest_stream_read(None, 256, 8, 1, None) == 1
 
 
+def test_native_calls_belong_to_this_interpreter():
+    """The extension carries the tag of the interpreter it was built for."""
+    import sysconfig
+    import cudalm_c_b200._lib as m
+    m.calls.embed
+    from cudalm_c_b200 import _pycalls
+    assert _pycalls.__file__.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
+    assert not os.path.exists(os.path.join(os.path.dirname(_pycalls.__file__), "_pycalls.so"))
+
+
 def test_native_calls_report_the_first_wrong_argument():
     """A conversion that fails leaves its own exception: no later argument's data_ptr() runs, no number is cut to an int."""
     from cudalm_c_b200._lib import QlmbError, calls
