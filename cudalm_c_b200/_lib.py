@@ -222,17 +222,25 @@ class _Calls:
 
 
 calls = _Calls()
-_raw_stream = _current_device = None
+_current_stream = None
+
+
+def _stream_getter():
+    """The current stream's handle.  torch.cuda.current_stream() makes a Stream object, 3.4 us a call; the two functions
+    behind it are private, so a torch without them takes the public way."""
+    import torch
+    torch.cuda.init()
+    device, raw = getattr(torch._C, "_cuda_getDevice", None), getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if device is None or raw is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: raw(device())
 
 
 def stream_ptr(stream=None):
     """cudaStream_t of `stream`, or of the current stream of the current device."""
-    global _raw_stream, _current_device
+    global _current_stream
     if stream is not None:
         return stream.cuda_stream
-    if _raw_stream is None:
-        import torch
-        torch.cuda.init()
-        _current_device = torch._C._cuda_getDevice
-        _raw_stream = torch._C._cuda_getCurrentRawStream # torch.cuda.current_stream() makes a Stream object: 3.4 us a call
-    return _raw_stream(_current_device())
+    if _current_stream is None:
+        _current_stream = _stream_getter()
+    return _current_stream()

@@ -106,6 +106,17 @@ def test_native_calls_belong_to_this_interpreter():
     assert not os.path.exists(os.path.join(os.path.dirname(_pycalls.__file__), "_pycalls.so"))
 
 
+@pytest.mark.parametrize("missing", ["_cuda_getDevice", "_cuda_getCurrentRawStream"])
+def test_stream_without_private_functions(monkeypatch, missing):
+    import torch
+    import cudalm_c_b200._lib as m
+    monkeypatch.setattr(m, "_current_stream", None)
+    monkeypatch.setattr(torch.cuda, "init", lambda: None)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: type("S", (), dict(cuda_stream=4711)))
+    monkeypatch.delattr(torch._C, missing, raising=False)
+    assert m.stream_ptr() == 4711
+
+
 def test_native_calls_report_the_first_wrong_argument():
     """A conversion that fails leaves its own exception: no later argument's data_ptr() runs, no number is cut to an int."""
     from cudalm_c_b200._lib import QlmbError, calls
