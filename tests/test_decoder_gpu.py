@@ -81,6 +81,67 @@ def test_slot_past_its_cache_is_reported_not_written(cuda):
     assert torch.equal(row[1], keep[1]) and not torch.equal(row[0], keep[0])
 
 
+CHAIN = [(9, 256, 4, 2, 128), (17, 256, 2, 2, 256), (64, 768, 12, 2, 256), (12, 1152, 18, 2, 128)]      # B, D, KV, experts = choices, F
+
+
+@pytest.mark.parametrize("B,D,KV,E,F", CHAIN)
+def test_chain_matches_full_forward(cuda, B, D, KV, E, F):
+    """Steps of more than eight slots (and of a width beyond the one-launch form) go through the chain of separate operators:
+    the check above for them, slots at different positions.  Every token takes every expert, so that no near-tie of two
+    router logits decides between experts."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import block, model
+    cfg = model.Config(L=2, D=D, H=D // 64, KV=KV, hd=64, E=E, K=E, F=F, V=512, T=64, B=1)
+    m = model.QlmModel(cfg, cuda, seed=5)
+    g = torch.Generator(device=cuda); g.manual_seed(B)
+    n, k = 21, 3
+    ids = torch.randint(0, cfg.V, (B, n + k), generator=g, dtype=torch.int32, device=cuda)
+    dec = model.Decoder(m, B, 48)
+    assert dec._step_plan() is None
+    fn = m.forward(ids.reshape(-1).contiguous(), B=B, T=n + k, moes=[dec._moe(l, B * (n + k)) for l in range(cfg.L)])
+    ref = block.gemm_nt(fn, block.cast_bf16(m.emb)[0], torch.float32).view(B, n + k, cfg.V)
+    back = torch.arange(B, device=cuda, dtype=torch.int32) % 5             # slot b has n - back[b] tokens cached
+    dec.prefill(ids[:, :n].contiguous())
+    dec.pos2.sub_(back.repeat(2))
+    rows = torch.arange(B, device=cuda)
+    for j in range(k):
+        at = (dec.pos + 0).long()
+        dec.tok.copy_(ids[rows, at])
+        lg = dec.step(advance=False)
+        dec.advance()
+        want = ref[rows, at]
+        assert float((lg - want).abs().max()) < 5e-2
+        assert float((lg.argmax(-1) == want.argmax(-1)).float().mean()) > 0.98
+    torch.cuda.synchronize()
+    q.check(q.lib().qlmb_check_device(None))
+
+
+@pytest.mark.parametrize("B,D,KV,E,F", CHAIN)
+def test_chain_skips_a_slot_past_its_cache(cuda, B, D, KV, E, F):
+    """One slot's position outside the cache: reported, its cache rows untouched, the other slots' logits the same bits."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import model
+    cfg = model.Config(L=2, D=D, H=D // 64, KV=KV, hd=64, E=E, K=E, F=F, V=512, T=64, B=1)
+    m = model.QlmModel(cfg, cuda, seed=6)
+    dec = model.Decoder(m, B, 32)
+    g = torch.Generator(device=cuda); g.manual_seed(B)
+    dec.prefill(torch.randint(0, cfg.V, (B, 11), generator=g, dtype=torch.int32, device=cuda))
+    good = dec.step(advance=False).clone()
+    q.check(q.lib().qlmb_check_device(None))
+    others = torch.arange(B, device=cuda) != 3
+    for bad in (32, -1, 2 ** 30):
+        dec.pos2[3] = bad; dec.pos2[B + 3] = bad
+        keep = [t[3].clone() for t in dec.K + dec.V]
+        got = dec.step(advance=False)
+        torch.cuda.synchronize()
+        assert q.lib().qlmb_check_device(None) == 4 and b"error code 201" in q.lib().qlmb_last_error()
+        assert all(torch.equal(t[3], u) for t, u in zip(dec.K + dec.V, keep))
+        assert torch.equal(got[others], good[others])
+    dec.pos2[3] = 11; dec.pos2[B + 3] = 11
+    assert torch.equal(dec.step(advance=False), good)
+    q.check(q.lib().qlmb_check_device(None))
+
+
 def test_sampler_topk_topp_temperature(cuda):
     """k_dec_sample (cudalm.cu:7048-7108) against a float64 restatement of its algorithm: arg-max and
     log-probability, the top-k / top-p cut, and the pick that the (seed, step) hash selects from the tempered
@@ -142,6 +203,28 @@ def test_sampler_topk_topp_temperature(cuda):
                 lo = cum[i - 1] if i else 0.0
                 ok |= lo - 1e-4 <= u01 <= cum[i] + 1e-4
         assert ok, (b, cases[b], int(out[b]))
+    q.check(q.lib().qlmb_check_device(None))
+
+
+def test_one_launch_step_skips_a_slot_past_its_cache(cuda):
+    """The same for up to eight slots, which take one launch."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import model
+    cfg = model.Config(L=2, D=256, H=4, KV=4, hd=64, E=8, K=2, F=256, V=512, T=64, B=1)
+    m = model.QlmModel(cfg, cuda, seed=6)
+    dec = model.Decoder(m, 5, 32)
+    g = torch.Generator(device=cuda); g.manual_seed(1)
+    dec.prefill(torch.randint(0, cfg.V, (5, 11), generator=g, dtype=torch.int32, device=cuda))
+    assert dec._step_plan() is not None
+    good = dec.step(advance=False).clone()
+    for bad in (32, -1, 2 ** 30):
+        dec.pos2[3] = bad; dec.pos2[8] = bad
+        keep = [t[3].clone() for t in dec.K + dec.V]
+        got = dec.step(advance=False)
+        torch.cuda.synchronize()
+        assert q.lib().qlmb_check_device(None) == 4 and b"error code 201" in q.lib().qlmb_last_error()
+        assert all(torch.equal(t[3], u) for t, u in zip(dec.K + dec.V, keep))
+        assert torch.equal(got[[0, 1, 2, 4]], good[[0, 1, 2, 4]])
     q.check(q.lib().qlmb_check_device(None))
 
 
