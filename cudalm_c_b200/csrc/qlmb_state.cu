@@ -940,7 +940,7 @@ __global__ void __launch_bounds__(256) k_sq_partial(const float *G, size_t n, do
 }
 // Stage 2 (reference cudalm.cu:2807-2812): part[64*(1+nside)] -> gs[0..1].
 // The partials in parallel, then one thread adds them in order (one thread for everything took 27 us, most of it the
-// latency of 1024 dependent loads; now 4).
+// latency of 1024 dependent loads; now 3).
 __global__ void __launch_bounds__(256) k_gnorm_final(const double *sub, int nside, int clip_side, float *gs)
 {
     __shared__ float part[64 * 63];                      // nside <= 62

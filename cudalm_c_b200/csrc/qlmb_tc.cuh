@@ -116,9 +116,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t v[16])
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// One lane of a converged warp, as a predicate that the compiler knows to hold for a single thread: the operands of what it
-// guards stay in uniform registers (with `lane == 0` each tcgen05.mma and each bulk tensor copy took 120 to 400 cycles to issue).
-// The same lane every time, as bulk groups are kept per thread.
+// One lane of a converged warp, as a predicate that the compiler knows to hold for a single thread (with `lane == 0` each
+// tcgen05.mma and each bulk tensor copy took 120 to 400 cycles to issue).  The same lane every time, as bulk groups are kept
+// per thread.
 __device__ __forceinline__ bool elect_one()
 {
     uint32_t p;

@@ -23,11 +23,10 @@ __device__ __forceinline__ float exp_poly(float x)
     return p * __uint_as_float((uint32_t)((int)k + 127) << 23);
 }
 
-// Same arithmetic with one warp per token and lane = expert (E <= 32): the
-// maximum is order-free, the softmax sum is still taken in expert order (every
-// lane adds the 32 shuffled terms sequentially) and the K selection rounds are
-// warp maxima of an order-preserving integer, with the lowest index winning ties, so the outputs are
-// bit-identical to the thread-per-token form above.
+// One warp per token, lane = expert (E <= 32), with the arithmetic of the reference's CPU kernel (cpu_kern.h:413-425): the
+// maximum is order-free, the softmax sum is taken in expert order (every lane adds the 32 shuffled terms one after the
+// other) and the K selection rounds are warp maxima of an order-preserving integer, with the lowest index winning ties.
+//
 // unsigned integers in the order of the floats (never 0 for a number above -1e30); -0 counts as +0
 __device__ __forceinline__ unsigned order_key(float f)
 {
