@@ -578,6 +578,7 @@ __device__ __forceinline__ void st4_any(void *p, uint32_t v)
     b[0] = (uint8_t)v; *(uint16_t *)(b + 1) = (uint16_t)(v >> 8); b[3] = (uint8_t)(v >> 24);
 }
 
+template <bool V> struct Flag { static constexpr bool value = V; };
 template <bool WRITE_P>
 __global__ void __launch_bounds__(256, 4) k_step_pk(const __grid_constant__ StepArgs a)
 {
@@ -655,18 +656,41 @@ __global__ void __launch_bounds__(256, 4) k_step_pk(const __grid_constant__ Step
         am = max3_nan(am, mn[p].x, mn[p].y); amn = min3_nan(amn, mn[p].x, mn[p].y);
         vm = max3_nan(vm, rv[p].x, rv[p].y); vmn = min3_nan(vmn, rv[p].x, rv[p].y);
     }
-    // the lane's numbers stay where no step of the root and the quotients below can underflow or overflow, and none is zero
-    // or NaN: roots in [2^-40, 2^20], denominators in [1e-8, 2^41] (veps is in them), numerators in [2^-80, 2^80], quotients
+    // the lane's numbers stay where no step of the root and the quotients below can underflow or overflow, and none is
+    // NaN: roots in [2^-40, 2^20], denominators in [1e-8, 2^41] (veps is in them), numerators in [2^-80, 2^80], quotients
     // in [2^-121, 2^107]
-    const bool ok = amn >= 8.6736174e-19f && am <= 1.1529215e18f && vmn >= 8.2718061e-25f && vm <= 1.0995116e12f && vs_old <= 1048576.0f && a.bc_ok;
-    if (ok) {
-        vm = sqrt_one(vm);                                            // the root is monotone
+    constexpr float M_LO = 8.6736174e-19f, V_LO = 8.2718061e-25f;
+    const bool high = am <= 1.1529215e18f && vm <= 1.0995116e12f && vs_old <= 1048576.0f && a.bc_ok;
+    bool ok = amn >= M_LO && vmn >= V_LO && high;
+    auto update = [&](int p) {
+        const float2 den = pk_fma(pk_mul(rv[p], bc2(a.inv_sqrt_bc2)), one2, bc2(veps));
+        u[p] = div_pair(pk_mul(mn[p], bc2(a.inv_bc1)), den, rcp_pair(den));
+        u[p] = make_float2(lim_abs(u[p].x, 8.0f), lim_abs(u[p].y, 8.0f));
+    };
+    // Zeros are ordinary (gradients of rows and experts that no token reached), so a warp that meets one takes a form with
+    // the root's operand kept off zero, all its lanes the same one; the quotients take a zero dividend as it is.  Left to the
+    // IEEE operators, one zero in a hundred doubled the kernel's time: 125.8 M elements 0.67 -> 1.52 ms.
+    const bool dense = !__any_sync(__activemask(), !ok);
+    if (!dense) {
+        float m1 = INFINITY, v1 = INFINITY;
 #pragma unroll
         for (int p = 0; p < NP; p++) {
-            rv[p] = sqrt_pair(rv[p]);
-            const float2 den = pk_fma(pk_mul(rv[p], bc2(a.inv_sqrt_bc2)), one2, bc2(veps));
-            u[p] = div_pair(pk_mul(mn[p], bc2(a.inv_bc1)), den, rcp_pair(den));
-            u[p] = make_float2(lim_abs(u[p].x, 8.0f), lim_abs(u[p].y, 8.0f));
+            m1 = min3_nan(m1, mn[p].x == 0.0f ? 1.0f : mn[p].x, mn[p].y == 0.0f ? 1.0f : mn[p].y);
+            v1 = min3_nan(v1, rv[p].x == 0.0f ? 1.0f : rv[p].x, rv[p].y == 0.0f ? 1.0f : rv[p].y);
+        }
+        ok = m1 >= M_LO && v1 >= V_LO && high;
+    }
+    if (dense) {
+        vm = sqrt_one(vm);                                            // the root is monotone
+#pragma unroll
+        for (int p = 0; p < NP; p++) { rv[p] = sqrt_pair(rv[p]); update(p); }
+    } else if (ok) {
+        vm = vm > 0.0f ? sqrt_one(vm) : 0.0f;
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+            const float2 s = sqrt_pair(make_float2(fmaxf(rv[p].x, V_LO), fmaxf(rv[p].y, V_LO)));
+            rv[p] = make_float2(rv[p].x > 0.0f ? s.x : 0.0f, rv[p].y > 0.0f ? s.y : 0.0f);
+            update(p);
         }
     } else {
         am = 0.0f; vm = 0.0f;
@@ -729,22 +753,28 @@ __global__ void __launch_bounds__(256, 4) k_step_pk(const __grid_constant__ Step
         vm = fmaxf(vm, __shfl_xor_sync(tmask, vm, o));
     }
     const float2 top = make_float2(127.0f, 255.0f);
-    const float2 sc = div_pair(make_float2(am, vm), top, make_float2(1.0f / 127.0f, 1.0f / 255.0f));
+    float2 sc = div_pair(make_float2(am, vm), top, make_float2(1.0f / 127.0f, 1.0f / 255.0f));
+    if (!dense) sc = make_float2(am == 0.0f ? 1e-12f : sc.x, vm == 0.0f ? 1e-12f : sc.y);
     float2 mq[NP], vq[NP];
-    // 2^-40 <= scale <= 1: the quotients by reciprocal are exact there (see above)
-    if (ok && fminf(sc.x, sc.y) >= 9.094947e-13f && fmaxf(sc.x, sc.y) <= 1.0f) {
+    auto quantise = [&](auto zeros) {
         if (tl == 0) { a.m8s[gi] = sc.x; a.v8s[gi] = sc.y; }
         const float2 rc = rcp_pair(sc), rl = pk_mul(pk_fma(make_float2(-sc.x, -sc.y), rc, bc2(1.0f)), rc);
 #pragma unroll
         for (int p = 0; p < NP; p++) {
             const uint64_t ei = (uint64_t)(2 * p) * QLMB_HASH_I, ej = (uint64_t)(2 * p + 1) * QLMB_HASH_I;
-            // limits before the rounding give what limits after it would: they are integers.  No second moment is zero
-            // here, so none of them may become 0 (qlm.cuh:275-277).
+            // limits before the rounding give what limits after it would: they are integers.  A second moment that is not
+            // zero may not become 0 (qlm.cuh:275-277).
+            const float2 vlo = decltype(zeros)::value ? make_float2(rv[p].x > 0.0f ? 1.0f : 0.0f, rv[p].y > 0.0f ? 1.0f : 0.0f) : bc2(1.0f);
             const float2 qm = div_pair(mn[p], sc.x, rc.x, rl.x), qv = div_pair(rv[p], sc.y, rc.y, rl.y);
             mq[p] = sround_magic(make_float2(lim_abs(qm.x, 127.0f), lim_abs(qm.y, 127.0f)), mix32(km + ei), mix32(km + ej));
-            vq[p] = sround_magic(make_float2(fminf(fmaxf(qv.x, 1.0f), 255.0f), fminf(fmaxf(qv.y, 1.0f), 255.0f)), mix32(kv + ei), mix32(kv + ej));
+            vq[p] = sround_magic(make_float2(fminf(fmaxf(qv.x, vlo.x), 255.0f), fminf(fmaxf(qv.y, vlo.y), 255.0f)), mix32(kv + ei), mix32(kv + ej));
         }
-    } else {
+    };
+    // 2^-40 <= scale <= 1: the quotients by reciprocal are exact there (see above)
+    const bool scaled = fminf(sc.x, sc.y) >= 9.094947e-13f && fmaxf(sc.x, sc.y) <= 1.0f;
+    if (dense && scaled) quantise(Flag<false>());
+    else if (ok && scaled) quantise(Flag<true>());
+    else {
         const float ms = am > 0.0f ? am / 127.0f : 1e-12f;
         const float vs = vm > 0.0f ? vm / 255.0f : 1e-12f;
         if (tl == 0) { a.m8s[gi] = ms; a.v8s[gi] = vs; }

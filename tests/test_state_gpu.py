@@ -151,6 +151,39 @@ def test_step_of_spans_at_any_even_element_matches_oracle(cuda, oracle, sizes):
         assert (P.cpu().numpy() == Ph).all()
 
 
+@pytest.mark.parametrize("zeros", [0.0, 0.002, 0.02, 0.5, 0.99, 1.0])
+def test_step_of_sparse_gradients_matches_oracle(cuda, oracle, zeros):
+    """Gradients with zeros from the first step on (rows and experts that no token reached): zero moments, whole groups of
+    them, and groups whose other moments are tiny or large, beside dense warps."""
+    rng = np.random.default_rng(17)
+    st = DevState(cuda, [128 * 96, 128 * 33 + 2, 128 * 40], 128, 7, 1)
+    P0 = (rng.standard_normal(st.nq) * 0.02).astype(f32)
+    st.encode(dev(P0, cuda))
+    h = st.host()
+    d, r, s = h["d"].copy(), h["r"].copy(), h["s"].copy()
+    for i in range(len(st.sp)):
+        g0 = int(st.sp[i]["gi0"]); st.sp[i]["sref"] = f32(s[g0:g0 + int(st.sp[i]["ngrp"])].astype(np.float64).mean())
+    st.push_spans()
+    m8 = np.zeros(st.nq, np.int8); v8 = np.zeros(st.nq, np.uint8)
+    m8s = np.zeros(st.ng, f32); v8s = np.zeros(st.ng, f32)
+    Ph = np.zeros(st.nq, f32)
+    P = torch.zeros(st.nq, device=cuda)
+    never = rng.random(st.nq) < zeros / 2                     # elements that never have a gradient, others miss it now and then
+    for t in range(1, 7):
+        G = (rng.standard_normal(st.nq) * 1e-3).astype(f32)
+        G[never | (rng.random(st.nq) < zeros)] = 0.0
+        G[128 * 10:128 * 14] = 0.0                            # whole groups, in the middle of dense ones
+        G[128 * 20:128 * 21] *= f32(1e-17); G[128 * 22:128 * 23] *= f32(1e-30); G[128 * 24 + 5] = f32(1e20)
+        st.step(P, dev(G, cuda), t)
+        bc1 = f32(1) - f32(np.power(f32(0.9), f32(t))); bc2 = f32(1) - f32(np.power(f32(0.95), f32(t)))
+        oracle.step(Ph, G, d, r, s, m8, m8s, v8, v8s, st.sp, lr=3e-4, b1=0.9, b2=0.95, wd=0.1, gscale=1.0,
+                    inv_bc1=float(f32(1) / bc1), inv_sqrt_bc2=float(f32(1) / np.sqrt(bc2)), t=t)
+        h = st.host()
+        for k, v in dict(d=d, r=r, m8=m8, v8=v8, m8s=m8s, v8s=v8s).items():
+            assert (h[k] == v).all(), (k, t, int((h[k] != v).sum()))
+        assert (P.cpu().numpy() == Ph).all()
+
+
 @pytest.mark.parametrize("form,lo,hi", [(0, -40, 41), (1, -80, 40), (2, -27, 41), (3, -40, 0)])
 def test_roots_and_quotients_equal_the_ieee_operations(cuda, form, lo, hi):
     """Every significand under every exponent that the packed step's guard admits (reciprocals and roots), 2^23 drawn
