@@ -808,7 +808,7 @@ def run_adamw(args):
                           vs_baseline=None, dtype="int8/f32", data="synthetic",
                           config=dict(workload="integer AdamW step, flat 4-bit span (BASELINE config 3)", params=n,
                                       bytes_per_param=bpp, l2="1.4 GB of state per step exceeds the 126 MB L2"),
-                          roofline=dict(bound="hbm", kernel="k_step_fast", achieved=round(gbs, 1), peak=pk["hbm"] * world, unit="GB/s",
+                          roofline=dict(bound="hbm", kernel="k_step_pk", achieved=round(gbs, 1), peak=pk["hbm"] * world, unit="GB/s",
                                         frac=round(gbs / (pk["hbm"] * world), 4), traffic=None,
                                         peak_kind="copy bandwidth x %d GPU(s), of %s" % (world, pk["src"])),
                           cpu_baseline=cpu, gparams_per_s=round(n / (ms * 1e-3) / 1e9, 2), gpu_launches=args.steps,
