@@ -865,7 +865,7 @@ extern "C" int qlmb_rmsnorm_fwd(void *O, int o_dtype, float *rinv, const void *X
     if (N <= 0) return QLMB_OK;
     auto kern = o_dtype == QLMB_BF16 ? (x_dtype == QLMB_BF16 ? k_rmsnorm_fwd<QLMB_BF16, QLMB_BF16> : k_rmsnorm_fwd<QLMB_BF16, QLMB_F32>)
                                      : (x_dtype == QLMB_BF16 ? k_rmsnorm_fwd<QLMB_F32, QLMB_BF16> : k_rmsnorm_fwd<QLMB_F32, QLMB_F32>);
-    QLMB_CUDA(pdl_launch(true, kern, dim3((N + 7) / 8), dim3(256), 0, as_stream(stream), O, rinv, X, gamma, N, D));
+    QLMB_CUDA(pdl_launch(D <= 1024, kern, dim3((N + 7) / 8), dim3(256), 0, as_stream(stream), O, rinv, X, gamma, N, D));    // longer rows: long blocks
     QLMB_LAUNCH_CHECK("k_rmsnorm_fwd");
     return QLMB_OK;
 }
@@ -889,7 +889,8 @@ extern "C" int qlmb_rmsnorm_bwd(void *dx, int dx_dtype, int accumulate, float *d
         QLMB_LAUNCH_CHECK("k_rmsnorm_bwd");
         return QLMB_OK;
     }
-    QLMB_CUDA(pdl_launch(true, k_rmsnorm_bwd, dim3((N + 7) / 8), dim3(256), 0, st, dx, dx_dtype, accumulate, X, x_dtype, gamma, rinv, dy, dy_dtype, N, D));
+    // (not early: a warp walks a whole row three times)
+    QLMB_CUDA(pdl_launch(false, k_rmsnorm_bwd, dim3((N + 7) / 8), dim3(256), 0, st, dx, dx_dtype, accumulate, X, x_dtype, gamma, rinv, dy, dy_dtype, N, D));
     if (dgamma) {
         QLMB_CUDA(pdl_launch(true, k_gamma_part, dim3((D + 127) / 128, GAMMA_CH), dim3(128), 0, st, part, X, x_dtype, rinv, dy, dy_dtype, N, D));
         QLMB_CUDA(pdl_launch(true, k_gamma_sum, dim3((D + 127) / 128), dim3(128), 0, st, dgamma, part, D));
@@ -921,8 +922,10 @@ extern "C" int qlmb_softmax_ce(const void *logits, int lg_dtype, const int *tgt,
     QLMB_REQUIRE(logits && tgt && loss && dlogits && dtype_ok(lg_dtype) && dtype_ok(dl_dtype), "qlmb_softmax_ce: bad argument");
     QLMB_REQUIRE(V > 0 && n_all > 0, "qlmb_softmax_ce: bad shape V %d n_all %d", V, n_all);
     if (rows <= 0) return QLMB_OK;
-    // the register form where its 32 logits a thread hold the row and every row starts on 16 bytes
-    if (V <= 16384 && V % 8 == 0 && (((uintptr_t)logits | (uintptr_t)dlogits) & 15) == 0)
+    // The register form where its 32 logits a thread hold the row and every row starts on 16 bytes, and where one pass pays:
+    // rows of more than 8 KB (1024 rows of 16384 fp32 63.5 -> 26.8 us, of 4096 bf16 10.9 -> 11.5) or a single round of its
+    // two blocks per SM (64 rows of 1000: 3.6 -> 2.5; 1024 of them 5.6 -> 9.1)
+    if (V <= 16384 && V % 8 == 0 && ((size_t)V * (lg_dtype == QLMB_BF16 ? 2 : 4) > 8192 || rows <= 2 * sm_count()) && (((uintptr_t)logits | (uintptr_t)dlogits) & 15) == 0)
         QLMB_CUDA(pdl_launch(true, k_softmax_ce_row, dim3((unsigned)rows), dim3(512), 0, as_stream(stream), logits, lg_dtype, tgt, loss, dlogits, dl_dtype, V, n_all));
     else QLMB_CUDA(pdl_launch(true, k_softmax_ce, dim3((unsigned)rows), dim3(256), 0, as_stream(stream), logits, lg_dtype, tgt, loss, dlogits, dl_dtype, V, n_all));
     QLMB_LAUNCH_CHECK("k_softmax_ce");

@@ -289,8 +289,8 @@ int router_logits(float *rt, const void *X, int x_dtype, const float *Wr, int N,
         else QLMB_CUDA(pdl_launch_small(k_router_logits_few<0>, grid, dim3(256), few_smem, st, rt, X, Wr, N, D, E));
     } else if (E <= 32 && (D % 8) == 0 && (((uintptr_t)X | (uintptr_t)Wr) & 15) == 0) {
         int blocks = (N + RLT_TOK - 1) / RLT_TOK;
-        if (x_dtype == QLMB_BF16) QLMB_CUDA(pdl_launch_small(k_router_logits_tile<1>, dim3(blocks), dim3(256), 0, st, rt, X, Wr, N, D, E));
-        else QLMB_CUDA(pdl_launch_small(k_router_logits_tile<0>, dim3(blocks), dim3(256), 0, st, rt, X, Wr, N, D, E));
+        if (x_dtype == QLMB_BF16) QLMB_CUDA(pdl_launch(false, k_router_logits_tile<1>, dim3(blocks), dim3(256), 0, st, rt, X, Wr, N, D, E));
+        else QLMB_CUDA(pdl_launch(false, k_router_logits_tile<0>, dim3(blocks), dim3(256), 0, st, rt, X, Wr, N, D, E));
     } else {
         k_router_logits<<<(N + RL_TOK - 1) / RL_TOK, 256, 0, st>>>(rt, X, x_dtype, Wr, N, D, E);
     }

@@ -106,6 +106,22 @@ def test_softmax_ce_row_lengths(cuda, V):
     assert rel(loss[keep].cpu().numpy(), ref_loss.cpu().numpy()) < 1e-5 and float(loss[5]) == 0.0
 
 
+@pytest.mark.parametrize("rows,V", [(296, 512), (297, 512), (1024, 2048), (1024, 2056), (600, 4096), (600, 4104)])
+def test_softmax_ce_of_many_rows(cuda, rows, V):
+    """On both sides of the rule that picks the one-pass form (one round of blocks, or rows of more than 8 KB)."""
+    from cudalm_c_b200 import block
+    for dt, tol in ((torch.float32, 1e-5), (torch.bfloat16, 1e-2)):
+        lg = (torch.randn(rows, V, device=cuda) * 3.0).to(dt)
+        tgt = torch.randint(0, V, (rows,), device=cuda, dtype=torch.int32)
+        loss, dl = block.softmax_ce(lg, tgt, rows, dl_dtype=dt)
+        p = torch.softmax(lg.double(), 1)
+        at = (torch.arange(rows, device=cuda), tgt.long())
+        want_loss = -torch.log(p[at] + 1e-12)
+        p[at] -= 1.0
+        assert float((dl.double() - p / rows).norm() / (p / rows).norm()) < tol
+        assert float((loss.double() - want_loss).norm() / want_loss.norm()) < 1e-5
+
+
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 def test_rope(cuda, ref, dt):
     from cudalm_c_b200 import block
