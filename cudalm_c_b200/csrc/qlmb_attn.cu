@@ -929,11 +929,8 @@ extern "C" int qlmb_attn_bwd(void *dQ, void *dK, void *dV, float *drow, const vo
     cudaStream_t st = as_stream(stream);
     const size_t nrow = (size_t)B * T * H;
     QLMB_CUDA(pdl_launch_small(k_attn_drow, dim3((unsigned)((nrow + 31) / 32)), dim3(256), 0, st, drow, (const bf16 *)dA, (const bf16 *)O, B, T, H));
-    // early up to 1024 positions only: longer walks lose more to an uneven placement (1 x 8192, 4 heads: 760 -> 808 us)
-    const size_t small = (size_t)2 * sm_count();
-    const unsigned gkv = (unsigned)(p.nqt * B * KV), gq = (unsigned)(p.nqt * B * H);
-    QLMB_CUDA(pdl_launch(T <= 1024 && gkv <= small, k_attn_bwd_dkv, dim3(gkv), dim3(AT_BWD_THREADS), AT_DKV_SMEM, st, p));
-    QLMB_CUDA(pdl_launch(T <= 1024 && gq <= small, k_attn_bwd_dq, dim3(gq), dim3(AT_BWD_THREADS), AT_DQ_SMEM, st, p));
+    QLMB_CUDA(pdl_launch_small(k_attn_bwd_dkv, dim3((unsigned)(p.nqt * B * KV)), dim3(AT_BWD_THREADS), AT_DKV_SMEM, st, p));
+    QLMB_CUDA(pdl_launch_small(k_attn_bwd_dq, dim3((unsigned)(p.nqt * B * H)), dim3(AT_BWD_THREADS), AT_DQ_SMEM, st, p));
     QLMB_LAUNCH_CHECK("k_attn_bwd");
     return QLMB_OK;
 }
