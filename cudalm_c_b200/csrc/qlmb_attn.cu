@@ -2,18 +2,21 @@
 //
 // Forward, one CTA per (sequence, head, tile of 128 queries), two CTAs per SM:
 //
-//   warp 0      TMA producer   Q tile once; K and V tiles of 128 keys through a two-stage ring
-//   warp 1      MMA issuer     S = Q K^T (128 x 128 x 64) and PV = P V (128 x 64 x 128) with
-//                              tcgen05.mma, fp32 results in TMEM (S: 128 columns, PV: 64 columns)
-//   warps 2-9   softmax        two threads per query row (64 keys and 32 output dimensions each):
-//                              tcgen05.ld of the S row, running max / sum in the exp2 domain, P as
-//                              bf16 into shared memory in the 128-byte-swizzled K-major layout the
-//                              PV MMA reads, and O = O * corr + PV in registers
+//   warp 0      TMA producer   Q tile once; K and V tiles of 128 keys through a three-stage ring
+//   warp 1      MMA issuer     S = Q K^T (128 x 128 x 64) and O += P V (128 x 64 x 128) with tcgen05.mma; P is an
+//                              operand in TMEM, O stays there (S: 128 columns, O: 64, P: 64)
+//   warps 2-5   softmax        a thread per query row: the S row into 128 registers, running max / sum in the exp2
+//                              domain, P as bf16 back into TMEM, O rescaled there when a row of the warp has a new maximum
 //
-// The MMA warp issues PV(t) and S(t+1) back to back as soon as P(t) is in shared memory, so the
-// tensor core works on the next scores while the softmax warps fold PV(t) into O; the second CTA
-// of the SM fills the rest.  Every mbarrier wait is bounded (qlmb_tc.cuh): a wait that runs out
-// raises the CTA's abort flag, records its site in the device error word and all roles leave.
+// The scores of the next step are issued as soon as the softmax warps hold this step's in registers, so they are there when
+// those come back for them, and PV runs beside the next step's maximum.
+// What bounds it (8 x 1024 x 12 heads, clock trace): a step of a CTA takes 3.5 thousand cycles, 600 for the maximum, 300 for
+// O, 1750 for the 128 exponentials of a thread with their conversions, the rest hand-shakes; special-function unit 33 % busy,
+// issue slots 28 %: two softmax warps per scheduler do not cover their own latencies.  41 us; with two threads per row (an
+// exchange of the row's maximum per step), P through shared memory and O folded in registers it took 54.  A quarter of the
+// exponentials as polynomials on the multiply-add pipe: 42.3 instead of 41.2.
+// Every mbarrier wait is bounded (qlmb_tc.cuh): a wait that runs out raises the CTA's abort flag, records its site in the
+// device error word and all roles leave.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math.h>
@@ -27,8 +30,9 @@ constexpr int AT_BM = 128;                    // queries per CTA
 constexpr int AT_BN = 128;                    // keys per step
 constexpr int AT_HD = 64;
 constexpr int AT_TILE = AT_BM * AT_HD * 2;    // bytes of a Q, K or V tile
-constexpr int AT_P_BYTES = AT_BM * AT_BN * 2;
-constexpr int AT_FWD_SMEM = AT_TILE + 4 * AT_TILE + AT_P_BYTES + 768;   // + barriers (256 B) + one exchange word per query row
+constexpr int AT_FWD_NS = 3;                  // stages of the K / V ring
+constexpr int AT_FWD_SMEM = AT_TILE + 2 * AT_FWD_NS * AT_TILE + 256;   // + barriers
+constexpr int AT_FWD_THREADS = 192;
 
 struct AttnFwdParams {
     alignas(64) CUtensorMap q_map, k_map, v_map;
@@ -88,17 +92,53 @@ __device__ __forceinline__ float ex2(float x)
 }
 template <int M> struct AtMode { static constexpr int value = M; };     // which masks a tile needs
 
-__global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ AttnFwdParams p)
+// two floats in one 64-bit register: sm_100's two-wide multiply-add and add
+__device__ __forceinline__ uint64_t f2_packu(uint32_t a, uint32_t b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b)); return r; }
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) { return f2_packu(__float_as_uint(a), __float_as_uint(b)); }
+__device__ __forceinline__ void f2_unpack(uint64_t v, float &a, float &b)
+{
+    uint32_t x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(x), "=r"(y) : "l"(v));
+    a = __uint_as_float(x); b = __uint_as_float(y);
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+
+// 32 fp32 TMEM columns of this thread's lane, times mul -> 64 bytes of bf16 in global memory
+// (tcgen05.ld is warp-collective: every lane runs it, only live lanes store)
+__device__ __forceinline__ void attn_store_row32(bf16 *dst, uint32_t taddr, bool live, float mul)
+{
+    uint32_t v[32];
+    tmem_ld32(taddr, v);
+    tmem_ld_wait();
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        uint32_t w[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(v[u * 8 + 2 * k]) * mul, __uint_as_float(v[u * 8 + 2 * k + 1]) * mul);
+            w[k] = *reinterpret_cast<uint32_t *>(&h2);
+        }
+        if (live) *reinterpret_cast<uint4 *>(dst + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+__device__ __forceinline__ void attn_store_row64(bf16 *dst, uint32_t taddr, bool live, float mul)
+{
+    attn_store_row32(dst, taddr, live, mul);
+    attn_store_row32(dst + 32, taddr + 32, live, mul);
+}
+
+__global__ void __launch_bounds__(AT_FWD_THREADS, 2) k_attn_fwd(const __grid_constant__ AttnFwdParams p)
 {
     extern __shared__ __align__(1024) uint8_t at_smem[];
-    uint8_t *sQ = at_smem, *sK = sQ + AT_TILE, *sV = sK + 2 * AT_TILE, *sP = sV + 2 * AT_TILE;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sP + AT_P_BYTES);
-    uint64_t *q_full = bars, *kv_full = bars + 1, *kv_empty = bars + 3, *s_full = bars + 5, *p_full = bars + 6,
-             *o_full = bars + 7, *spare = bars + 8;
-    uint64_t *pair_bar = bars + 10;           // one per TMEM lane quarter: the two warps that share a query row meet here
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 14);
+    constexpr int NS = AT_FWD_NS;
+    uint8_t *sQ = at_smem, *sK = sQ + AT_TILE, *sV = sK + NS * AT_TILE;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sV + NS * AT_TILE);
+    uint64_t *q_full = bars, *s_full = bars + 1, *p_full = bars + 2, *o_full = bars + 3, *spare = bars + 4, *s_free = bars + 5,
+             *kv_full = bars + 6, *kv_empty = kv_full + NS;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(kv_empty + NS);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    int *xrow = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(bars) + 256);   // 128 words: running row maximum, then row sum
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (smem_u32(at_smem) & 1023u) {          // the swizzled tiles need a 1 KiB-aligned base
@@ -109,16 +149,15 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
     if (__syncthreads_or(threadIdx.x == 0 && at_error_seen(p.errword))) { pdl_wait(); return; }   // uniform over the CTA
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(q_full), 1);
-        for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&kv_full[i]), 1); mbar_init(smem_u32(&kv_empty[i]), 1); }
+        for (int i = 0; i < NS; i++) { mbar_init(smem_u32(&kv_full[i]), 1); mbar_init(smem_u32(&kv_empty[i]), 1); }
         mbar_init(smem_u32(s_full), 1);
-        mbar_init(smem_u32(p_full), 8);
-        for (int i = 0; i < 4; i++) mbar_init(smem_u32(&pair_bar[i]), 2);
+        mbar_init(smem_u32(s_free), 4);
+        mbar_init(smem_u32(p_full), 4);
         mbar_init(smem_u32(o_full), 1);
         mbar_init(smem_u32(spare), 1);
         *abort_flag = 0;
         fence_barrier_init();
     }
-    if (threadIdx.x >= 64 && threadIdx.x < 192) xrow[threadIdx.x - 64] = (int)0x80000000;      // below every encoded maximum
     if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), 256); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
@@ -126,7 +165,7 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
     pdl_wait();                               // barriers and TMEM above are this kernel's own; its inputs come below
     pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t tS = tmem_base, tPV = tmem_base + 128;
+    const uint32_t tS = tmem_base, tO = tmem_base + 128, tP = tmem_base + 192;
 
     // heaviest query tiles first
     const int BH = p.B * p.H;
@@ -147,8 +186,8 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
             tma_load_2d(smem_u32(sQ), &p.q_map, smem_u32(q_full), h * AT_HD, b * p.T + q0);
         }
         for (int t = 0; ok && t < nt; t++) {
-            const int st = t & 1;
-            ok = at_wait(smem_u32(&kv_empty[st]), (((uint32_t)t >> 1) & 1u) ^ 1u, abort_flag, p.errword, 101);
+            const int st = t % NS;
+            ok = at_wait(smem_u32(&kv_empty[st]), ((uint32_t)(t / NS) & 1u) ^ 1u, abort_flag, p.errword, 101);
             if (!ok) break;
             if (elect_one()) {
                 const uint32_t bar = smem_u32(&kv_full[st]);
@@ -163,8 +202,8 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
         if (*abort_flag) {
             // aborting: the copies this warp started must land before the CTA gives its shared memory back
             for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(q_full), 0); i++) {}
-            for (int t = issued > 2 ? issued - 2 : 0; t < issued; t++)
-                for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(&kv_full[t & 1]), ((uint32_t)t >> 1) & 1u); i++) {}
+            for (int t = issued > NS ? issued - NS : 0; t < issued; t++)
+                for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(&kv_full[t % NS]), (uint32_t)(t / NS) & 1u); i++) {}
         }
     } else if (warp == 1) {
         // =============================== MMA issuer ===============================
@@ -185,25 +224,25 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
             __syncwarp();
         }
         for (int t = 0; ok && t < nt; t++) {
-            const int st = t & 1;
+            const int st = t % NS;
+            // the next scores as soon as the softmax warps hold this step's in registers
+            if (t + 1 < nt) {
+                const int sn = (t + 1) % NS;
+                ok = at_wait(smem_u32(&kv_full[sn]), (uint32_t)((t + 1) / NS) & 1u, abort_flag, p.errword, 113);
+                if (ok) ok = at_wait(smem_u32(s_free), (uint32_t)t & 1u, abort_flag, p.errword, 114);
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) issue_s(sn);
+                __syncwarp();
+            }
             ok = at_wait(smem_u32(p_full), (uint32_t)t & 1u, abort_flag, p.errword, 112);
             if (!ok) break;
             tc_fence_after();
-            // the next scores first (the S columns are free once P is written): the softmax warps start on them while
-            // this step's PV runs; they fold PV(t) after their first pass and only then overwrite P
-            if (t + 1 < nt) {
-                ok = at_wait(smem_u32(&kv_full[st ^ 1]), ((uint32_t)(t + 1) >> 1) & 1u, abort_flag, p.errword, 113);
-                if (!ok) break;
-                tc_fence_after();
-                if (elect_one()) issue_s(st ^ 1);
-                __syncwarp();
-            }
             if (elect_one()) {
-                const uint32_t a0 = smem_u32(sP), b0 = smem_u32(sV + st * AT_TILE);
+                const uint32_t b0 = smem_u32(sV + st * AT_TILE);
 #pragma unroll
                 for (int kk = 0; kk < AT_BN / 16; kk++)
-                    tc_mma_bf16(tPV, make_desc(a0 + (kk >> 2) * (AT_BM * 128) + (kk & 3) * 32, 16, 1024),
-                                make_desc(b0 + kk * 2048, 8192, 1024), IDESC_PV, kk > 0);
+                    tc_mma_bf16_ta(tO, tP + kk * 8, make_desc(b0 + kk * 2048, 8192, 1024), IDESC_PV, (t > 0 || kk > 0) ? 1u : 0u);
                 tc_commit(smem_u32(o_full));
                 tc_commit(smem_u32(&kv_empty[st]));
             }
@@ -216,109 +255,101 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
         }
     } else {
         // =============================== softmax + output ===============================
-        // Two threads per query row: warps w and w + 4 share a TMEM lane quarter; thread (r, hf) takes keys
-        // [64 hf, 64 hf + 64) of every step and output dimensions [32 hf, 32 hf + 32).  The row maximum is a running
-        // atomicMax on one shared word per row (order-preserving integer image of the float): both threads add their
-        // half's maximum, meet on the quarter's mbarrier and read the same value.  No reset is needed: the running
-        // maximum only grows, and the next step's atomicMax cannot come before the partner has read this step's value,
-        // because the next scores are only issued after both warps arrived on p_full.
-        const int q = warp & 3, hf = (warp - 2) >> 2, r = q * 32 + lane, i = q0 + r;
+        const int q = warp & 3, r = q * 32 + lane, i = q0 + r;
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
-        const uint32_t pb = smem_u32(&pair_bar[q]);
-        uint32_t pphase = 0;
-        float m = -1e30f, l = 0.0f, corr_pend = 1.0f;
-        float o[32];
-#pragma unroll
-        for (int d = 0; d < 32; d++) o[d] = 0.0f;
+        const int iw = q0 + q * 32;                                     // the warp's first query
+        const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2);
+        float m = -1e30f, l = 0.0f;
         bool ok = true;
-        auto pair_sync = [&]() -> bool {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(pb);
-            const bool got = at_wait(pb, pphase, abort_flag, p.errword, 123);
-            pphase ^= 1u;
-            return got;
-        };
-        auto enc = [](float f) { const int b = __float_as_int(f); return b >= 0 ? b : b ^ 0x7fffffff; };
-        auto dec = [](int b) { return __int_as_float(b >= 0 ? b : b ^ 0x7fffffff); };
-        auto fold_pv = [&]() {                 // O = O * corr + PV for this thread's 32 output dimensions
-            uint32_t v[32];
-            tmem_ld32(tPV + lane_base + hf * 32, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; j++) o[j] = o[j] * corr_pend + __uint_as_float(v[j]);
-        };
         for (int t = 0; ok && t < nt; t++) {
-            const int k0 = (kt_lo + t) * AT_BN + hf * 64;               // first key of this thread's half
-            const bool masked = (k0 + 63 > q0) || p.win > 0 || (k0 + 64 > p.T);
+            const int k0 = (kt_lo + t) * AT_BN;
             ok = at_wait(smem_u32(s_full), (uint32_t)t & 1u, abort_flag, p.errword, 120);
             if (!ok) break;
             tc_fence_after();
-            const int klo = i - p.win - k0, khi = (i < p.T ? i : p.T - 1) - k0;
-            // pass 1: maximum of this half of the row
+            uint32_t v[2][64];
+#pragma unroll
+            for (int c = 0; c < 4; c++) tmem_ld32(tS + lane_base + c * 32, &v[c >> 1][(c & 1) * 32]);
+            tmem_ld_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(s_free));
+            // Halves of 64 keys: all of them visible to the warp's 32 queries, some, or none.  A key that a query does not
+            // see becomes -inf and gets the weight 0.
+            auto none = [&](int c) { return k0 + c * 64 > iw + 31 || (p.win > 0 && k0 + c * 64 + 63 <= iw - p.win); };
             float mx = -1e30f;
 #pragma unroll
             for (int c = 0; c < 2; c++) {
-                uint32_t v[32];
-                tmem_ld32(tS + lane_base + hf * 64 + c * 32, v);
-                tmem_ld_wait();
-                if (masked) {                  // keys lo < j <= hi of the 32
-                    const int lo = klo - c * 32, hi = khi - c * 32;
-                    if (p.win > 0) {
+                const int kc = k0 + c * 64;
+                if (none(c)) continue;
+                if (kc + 63 > iw || (p.win > 0 && kc <= iw + 31 - p.win)) {
+                    const int hi = i - kc, lo = p.win > 0 ? hi - p.win : -1;
 #pragma unroll
-                        for (int j = 0; j < 32; j++) mx = fmaxf(mx, j <= hi && j > lo ? __uint_as_float(v[j]) : -1e30f);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; j++) mx = fmaxf(mx, j <= hi ? __uint_as_float(v[j]) : -1e30f);
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; j++) mx = fmaxf(mx, __uint_as_float(v[j]));
+                    for (int j = 0; j < 64; j++) v[c][j] = j <= hi && j > lo ? v[c][j] : 0xff800000u;
                 }
+                float mm[8];                            // eight chains: a step of one takes its instruction's latency
+#pragma unroll
+                for (int j = 0; j < 8; j++) mm[j] = __uint_as_float(v[c][j]);
+#pragma unroll
+                for (int j = 8; j < 56; j += 16)
+#pragma unroll
+                    for (int e = 0; e < 8; e++) mm[e] = fmaxf(fmaxf(mm[e], __uint_as_float(v[c][j + e])), __uint_as_float(v[c][j + 8 + e]));
+#pragma unroll
+                for (int e = 0; e < 8; e++) mm[e] = fmaxf(mm[e], __uint_as_float(v[c][56 + e]));
+                mm[0] = fmaxf(fmaxf(mm[0], mm[1]), mm[2]); mm[3] = fmaxf(fmaxf(mm[3], mm[4]), mm[5]);
+                mm[0] = fmaxf(fmaxf(mm[0], mm[3]), fmaxf(mm[6], mm[7]));
+                mx = fmaxf(mx, mm[0] * p.scale_log2);
             }
-            atomicMax(&xrow[r], enc(fmaxf(mx * p.scale_log2, -1e30f)));
-            ok = pair_sync();
-            if (!ok) break;
-            const float m_new = dec(*reinterpret_cast<volatile int *>(&xrow[r]));
-            const float corr = ex2(m - m_new);
-            // the previous step's PV: its MMA was issued before this step's S, so it has completed
+            // the previous step's PV has read P and written O
             if (t > 0) {
                 ok = at_wait(smem_u32(o_full), (uint32_t)(t - 1) & 1u, abort_flag, p.errword, 121);
                 if (!ok) break;
                 tc_fence_after();
-                fold_pv();
             }
-            corr_pend = corr;
-            // pass 2: P = exp2(s - m) as bf16 into this half's swizzled K-major sub-tile, partial row sum
-            float rs = 0.0f;
-            uint8_t *rowp = sP + hf * (AT_BM * 128) + r * 128;
+            // m is the running maximum.  Where no row of the warp has a new one O stays in TMEM as it is.  (Moving m only for
+            // a growth of 2^8 saved 1.6 us of 42 at 8 x 1024 x 12 heads, but the largest weight is then no longer exactly 1
+            // and the error against float64 grew from 2.03e-3 to 2.07e-3.)
+            if (__any_sync(0xffffffffu, mx > m)) {
+                const float mn = fmaxf(m, mx), corr = ex2(m - mn);
+                m = mn;
+                l *= corr;
+                if (t > 0) {
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        uint32_t o[16];
+                        tmem_ld16(tO + lane_base + c * 16, o);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; j++) o[j] = __float_as_uint(__uint_as_float(o[j]) * corr);
+                        tmem_st16(tO + lane_base + c * 16, o);
+                    }
+                }
+            }
+            // P = exp2(s - m) as bf16 into the TMEM columns that PV reads as its A operand, partial row sums
+            const uint64_t negm2 = f2_pack(-m, -m);
+            uint64_t rs[2] = {f2_pack(0.0f, 0.0f), f2_pack(0.0f, 0.0f)};
 #pragma unroll
             for (int c = 0; c < 2; c++) {
-                uint32_t v[32];
-                tmem_ld32(tS + lane_base + hf * 64 + c * 32, v);
-                tmem_ld_wait();
-                uint32_t pk[16];
+                uint32_t pk[32];
+                if (none(c)) {
 #pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    float p0 = ex2(__uint_as_float(v[j]) * p.scale_log2 - m_new);
-                    float p1 = ex2(__uint_as_float(v[j + 1]) * p.scale_log2 - m_new);
-                    if (masked) {
-                        const int jj = c * 32 + j;
-                        if (jj > khi || (p.win > 0 && jj <= klo)) p0 = 0.0f;
-                        if (jj + 1 > khi || (p.win > 0 && jj + 1 <= klo)) p1 = 0.0f;
+                    for (int j = 0; j < 32; j++) pk[j] = 0u;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) {
+                        float x0, x1;
+                        f2_unpack(f2_fma(f2_packu(v[c][2 * j], v[c][2 * j + 1]), scale2, negm2), x0, x1);
+                        const float p0 = ex2(x0), p1 = ex2(x1);
+                        rs[j & 1] = f2_add(rs[j & 1], f2_pack(p0, p1));
+                        const __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
+                        pk[j] = *reinterpret_cast<const uint32_t *>(&h2);
                     }
-                    rs += p0 + p1;
-                    __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
-                    pk[j >> 1] = *reinterpret_cast<uint32_t *>(&h2);
                 }
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int unit = (c * 4 + u) ^ (r & 7);
-                    *reinterpret_cast<uint4 *>(rowp + unit * 16) = make_uint4(pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
-                }
+                tmem_st32(tP + lane_base + c * 32, pk);
             }
-            l = l * corr + rs;
-            m = m_new;
-            fence_proxy_async();
+            float r0, r1;
+            f2_unpack(f2_add(rs[0], rs[1]), r0, r1);
+            l += r0 + r1;
+            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(p_full));
@@ -326,33 +357,9 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
         if (ok) ok = at_wait(smem_u32(o_full), (uint32_t)(nt - 1) & 1u, abort_flag, p.errword, 122);
         if (ok) {
             tc_fence_after();
-            fold_pv();
-            // the row sum: the upper half hands its partial sum over, the lower half returns the total
-            float *xl = reinterpret_cast<float *>(xrow);
-            if (hf == 1) xl[r] = l;
-            ok = pair_sync();
-            if (ok) {
-                if (hf == 0) { l += *reinterpret_cast<volatile float *>(&xl[r]); xl[r] = l; }
-                ok = pair_sync();
-            }
-            if (ok) {
-                if (hf == 1) l = *reinterpret_cast<volatile float *>(&xl[r]);
-                if (i < p.T) {
-                    const float inv = 1.0f / l;
-                    bf16 *orow = p.O + ((size_t)b * p.T + i) * ((size_t)p.H * AT_HD) + (size_t)h * AT_HD + hf * 32;
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            __nv_bfloat162 h2 = __floats2bfloat162_rn(o[u * 8 + 2 * k] * inv, o[u * 8 + 2 * k + 1] * inv);
-                            w[k] = *reinterpret_cast<uint32_t *>(&h2);
-                        }
-                        *reinterpret_cast<uint4 *>(orow + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
-                    if (hf == 0) p.lse[((size_t)b * p.H + h) * p.T + i] = (m + log2f(l)) * 0.6931471805599453f;
-                }
-            }
+            const float inv = 1.0f / l;
+            attn_store_row64(p.O + ((size_t)b * p.T + i) * ((size_t)p.H * AT_HD) + (size_t)h * AT_HD, tO + lane_base, i < p.T, inv);
+            if (i < p.T) p.lse[((size_t)b * p.H + h) * p.T + i] = (m + log2f(l)) * 0.6931471805599453f;
         }
         tc_fence_before();
     }
@@ -372,10 +379,14 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
 //
 // The walked tiles are 64 wide, so that two CTAs fit an SM (100 / 80 KB of shared memory, 256 TMEM columns each): the
 // element-wise phase of one runs beside the MMAs of the other.
-// What bounds them (clock trace of 8 x 1024 x 12 heads): a step of a CTA takes 3.3 thousand cycles, 1.3 of them
-// element-wise work (one exponential per element: the special-function unit delivers 16 a cycle), the rest the
-// hand-shakes around the MMAs, which the other CTA fills in part.  128-wide tiles with one CTA per SM took 98 + 83 us;
-// 64-wide tiles 85 + 67 us; with the MMAs issued behind elect.sync and masks only on the edge tiles 67 + 49 us.
+// dq: the scores of the next step are issued as soon as the element-wise warps hold this step's in registers, dS is an operand
+// in TMEM.  dkv: P^T and dS^T are operands in TMEM too; its 256 columns leave them no room of their own, so they overwrite the
+// scores they were made of, and the next scores follow the accumulating products.
+// What bounds them (clock trace of 8 x 1024 x 12 heads): a step of a CTA takes 3.1 (dkv) and 1.6 (dq) thousand cycles, 1.3 and
+// 0.9 of them element-wise work, in dkv 1.7 the products and their hand-shakes, which the other CTA fills in part.  128-wide
+// tiles with one CTA per SM took 98 + 83 us; 64-wide tiles 85 + 67 us; with the MMAs issued behind elect.sync and masks only
+// on the edge tiles 67 + 49; these 62 + 38.  (dkv with the scores ahead and P^T, dS^T through shared memory: 62 as well, its
+// shared memory then busy 84 % of the time.)
 //
 //   warp 0      TMA producer   resident tiles once, the walked tiles through a two-stage ring
 //   warp 1      MMA issuer     scores and dP (two 128 x 64 x 64 MMAs into TMEM), then the two
@@ -386,8 +397,10 @@ __global__ void __launch_bounds__(320, 2) k_attn_fwd(const __grid_constant__ Att
 constexpr int AT_BI = 64;                       // queries (dkv) or keys (dq) per step
 constexpr int AT_ITILE = AT_BI * AT_HD * 2;     // bytes of a walked tile
 constexpr int AT_BWD_THREADS = 320;             // TMA warp, MMA warp, 8 element-wise warps
-constexpr int AT_DKV_SMEM = 2 * AT_TILE + 4 * AT_ITILE + 2 * AT_BN * AT_BI * 2 + 2 * 2 * AT_BI * 4 + 256;
-constexpr int AT_DQ_SMEM = 2 * AT_TILE + 4 * AT_ITILE + AT_BM * AT_BI * 2 + 256;
+constexpr int AT_DKV_NS = 4;                    // stages of the walked tiles in dkv
+constexpr int AT_DKV_SMEM = 2 * AT_TILE + 2 * AT_DKV_NS * AT_ITILE + 2 * AT_DKV_NS * AT_BI * 4 + 256;
+constexpr int AT_DQ_NS = 4;                     // stages of the walked tiles in dq
+constexpr int AT_DQ_SMEM = 2 * AT_TILE + 2 * AT_DQ_NS * AT_ITILE + 256;
 
 struct AttnBwdParams {
     alignas(64) CUtensorMap q_map, k_map, v_map, da_map;      // boxes of 128 rows (resident tiles)
@@ -426,40 +439,16 @@ __global__ void __launch_bounds__(256) k_attn_drow(float *drow, const bf16 *dA, 
     }
 }
 
-// 32 fp32 TMEM columns of this thread's lane, times mul -> 64 bytes of bf16 in global memory
-// (tcgen05.ld is warp-collective: every lane runs it, only live lanes store)
-__device__ __forceinline__ void attn_store_row32(bf16 *dst, uint32_t taddr, bool live, float mul)
-{
-    uint32_t v[32];
-    tmem_ld32(taddr, v);
-    tmem_ld_wait();
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-        uint32_t w[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(v[u * 8 + 2 * k]) * mul, __uint_as_float(v[u * 8 + 2 * k + 1]) * mul);
-            w[k] = *reinterpret_cast<uint32_t *>(&h2);
-        }
-        if (live) *reinterpret_cast<uint4 *>(dst + u * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-}
-__device__ __forceinline__ void attn_store_row64(bf16 *dst, uint32_t taddr, bool live, float mul)
-{
-    attn_store_row32(dst, taddr, live, mul);
-    attn_store_row32(dst + 32, taddr + 32, live, mul);
-}
-
 __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid_constant__ AttnBwdParams p)
 {
     extern __shared__ __align__(1024) uint8_t at_smem[];
-    uint8_t *sK = at_smem, *sV = sK + AT_TILE, *sQ = sV + AT_TILE, *sA = sQ + 2 * AT_ITILE;
-    uint8_t *sPt = sA + 2 * AT_ITILE, *sSt = sPt + AT_BN * AT_BI * 2;
-    float *sL = reinterpret_cast<float *>(sSt + AT_BN * AT_BI * 2), *sD = sL + 2 * AT_BI;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sD + 2 * AT_BI);
-    uint64_t *kv_full = bars, *qd_full = bars + 1, *qd_empty = bars + 3, *s_full = bars + 5, *pds_full = bars + 6,
-             *acc_done = bars + 7, *spare = bars + 8;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 10);
+    constexpr int NS = AT_DKV_NS;
+    uint8_t *sK = at_smem, *sV = sK + AT_TILE, *sQ = sV + AT_TILE, *sA = sQ + NS * AT_ITILE;
+    float *sL = reinterpret_cast<float *>(sA + NS * AT_ITILE), *sD = sL + NS * AT_BI;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sD + NS * AT_BI);
+    uint64_t *kv_full = bars, *s_full = bars + 1, *pds_full = bars + 2, *acc_done = bars + 3, *spare = bars + 4,
+             *qd_full = bars + 5, *qd_empty = qd_full + NS;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(qd_empty + NS);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -470,7 +459,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
     if (__syncthreads_or(threadIdx.x == 0 && at_error_seen(p.errword))) { pdl_wait(); return; }   // uniform over the CTA
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(kv_full), 1);
-        for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&qd_full[i]), 2); mbar_init(smem_u32(&qd_empty[i]), 1); }
+        for (int i = 0; i < NS; i++) { mbar_init(smem_u32(&qd_full[i]), 2); mbar_init(smem_u32(&qd_empty[i]), 1); }
         mbar_init(smem_u32(s_full), 1);
         mbar_init(smem_u32(pds_full), 8);
         mbar_init(smem_u32(acc_done), 1);
@@ -507,8 +496,8 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
             tma_load_2d(smem_u32(sV), &p.v_map, smem_u32(kv_full), kvh * AT_HD, b * p.T + k0);
         }
         for (int it = 0; ok && it < nit; it++) {
-            const int st = it & 1, h = kvh * grp + it / nq, q0 = (qt_lo + it % nq) * AT_BI;
-            ok = at_wait(smem_u32(&qd_empty[st]), (((uint32_t)it >> 1) & 1u) ^ 1u, abort_flag, p.errword, 201);
+            const int st = it % NS, h = kvh * grp + it / nq, q0 = (qt_lo + it % nq) * AT_BI;
+            ok = at_wait(smem_u32(&qd_empty[st]), ((uint32_t)(it / NS) & 1u) ^ 1u, abort_flag, p.errword, 201);
             if (!ok) break;
             const uint32_t bar = smem_u32(&qd_full[st]);
             if (elect_one()) {
@@ -530,8 +519,8 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
         }
         if (*abort_flag) {
             for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(kv_full), 0); i++) {}
-            for (int it = issued > 2 ? issued - 2 : 0; it < issued; it++)
-                for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(&qd_full[it & 1]), ((uint32_t)it >> 1) & 1u); i++) {}
+            for (int it = issued > NS ? issued - NS : 0; it < issued; it++)
+                for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(&qd_full[it % NS]), (uint32_t)(it / NS) & 1u); i++) {}
         }
     } else if (warp == 1) {
         // =============================== MMA issuer ===============================
@@ -555,33 +544,33 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
             __syncwarp();
         }
         for (int it = 0; ok && it < nit; it++) {
-            const int st = it & 1;
+            const int st = it % NS;
             ok = at_wait(smem_u32(pds_full), (uint32_t)it & 1u, abort_flag, p.errword, 212);
             if (!ok) break;
             tc_fence_after();
-            // the next step's scores first (their TMEM columns are free once P / dS are written), so that the
-            // element-wise warps work on them while the two accumulating products of this step run
-            if (it + 1 < nit) {
-                ok = at_wait(smem_u32(&qd_full[st ^ 1]), ((uint32_t)(it + 1) >> 1) & 1u, abort_flag, p.errword, 213);
-                if (!ok) break;
-                tc_fence_after();
-                if (elect_one()) issue_scores(st ^ 1);
-                __syncwarp();
-            }
             if (elect_one()) {
-                const uint32_t pt = smem_u32(sPt), dst = smem_u32(sSt), q_ = smem_u32(sQ + st * AT_ITILE), a_ = smem_u32(sA + st * AT_ITILE);
+                const uint32_t q_ = smem_u32(sQ + st * AT_ITILE), a_ = smem_u32(sA + st * AT_ITILE);
 #pragma unroll
                 for (int kk = 0; kk < AT_BI / 16; kk++)       // dV += P^T dA
-                    tc_mma_bf16(tdV, make_desc(pt + kk * 32, 16, 1024),
-                                make_desc(a_ + kk * 2048, 8192, 1024), IDESC_ACC, (it > 0 || kk > 0) ? 1u : 0u);
+                    tc_mma_bf16_ta(tdV, tS + (kk >> 1) * 32 + (kk & 1) * 8, make_desc(a_ + kk * 2048, 8192, 1024), IDESC_ACC, (it > 0 || kk > 0) ? 1u : 0u);
 #pragma unroll
                 for (int kk = 0; kk < AT_BI / 16; kk++)       // dK += dS^T Q
-                    tc_mma_bf16(tdK, make_desc(dst + kk * 32, 16, 1024),
-                                make_desc(q_ + kk * 2048, 8192, 1024), IDESC_ACC, (it > 0 || kk > 0) ? 1u : 0u);
+                    tc_mma_bf16_ta(tdK, tP + (kk >> 1) * 32 + (kk & 1) * 8, make_desc(q_ + kk * 2048, 8192, 1024), IDESC_ACC, (it > 0 || kk > 0) ? 1u : 0u);
                 tc_commit(smem_u32(acc_done));
                 tc_commit(smem_u32(&qd_empty[st]));
             }
             __syncwarp();
+            // the next scores overwrite the columns that these products read: the multiplies of a CTA run in the order of
+            // their issue, and acc_done makes sure of it
+            if (it + 1 < nit) {
+                const int sn = (it + 1) % NS;
+                ok = at_wait(smem_u32(&qd_full[sn]), (uint32_t)((it + 1) / NS) & 1u, abort_flag, p.errword, 213);
+                if (ok) ok = at_wait(smem_u32(acc_done), (uint32_t)it & 1u, abort_flag, p.errword, 214);
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) issue_scores(sn);
+                __syncwarp();
+            }
         }
         if (*abort_flag) {
             if (elect_one()) tc_commit(smem_u32(spare));
@@ -595,9 +584,9 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
         const uint32_t lane_base = (uint32_t)(qr * 32) << 16;
         bool ok = true;
         for (int it = 0; ok && it < nit; it++) {
-            const int st = it & 1, q0 = (qt_lo + it % nq) * AT_BI;
+            const int st = it % NS, q0 = (qt_lo + it % nq) * AT_BI;
             const bool masked = (q0 < k0 + AT_BN - 1) || p.win > 0;
-            ok = at_wait(smem_u32(&qd_full[st]), ((uint32_t)it >> 1) & 1u, abort_flag, p.errword, 220);      // lse / D in shared memory
+            ok = at_wait(smem_u32(&qd_full[st]), (uint32_t)(it / NS) & 1u, abort_flag, p.errword, 220);      // lse / D in shared memory
             if (ok) ok = at_wait(smem_u32(s_full), (uint32_t)it & 1u, abort_flag, p.errword, 221);
             if (!ok) break;
             tc_fence_after();
@@ -637,20 +626,11 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
                 if (!masked) compute(AtMode<0>(), 0, 0);
                 else if (p.win <= 0) compute(AtMode<1>(), lo, 0);
                 else compute(AtMode<2>(), lo, lo + p.win);
-                // the previous step's products must have read the P / dS tiles before they are overwritten
-                if (it > 0) ok = at_wait(smem_u32(acc_done), (uint32_t)(it - 1) & 1u, abort_flag, p.errword, 222);
-                uint8_t *prow = sPt + r * 128, *srow = sSt + r * 128;
-                if (ok) {
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int unit = (c * 4 + u) ^ (r & 7);
-                        *reinterpret_cast<uint4 *>(prow + unit * 16) = make_uint4(pp[4 * u], pp[4 * u + 1], pp[4 * u + 2], pp[4 * u + 3]);
-                        *reinterpret_cast<uint4 *>(srow + unit * 16) = make_uint4(ds[4 * u], ds[4 * u + 1], ds[4 * u + 2], ds[4 * u + 3]);
-                    }
-                }
+                // P^T and dS^T over the thread's own score columns: 16 words of 64 columns' bf16 pairs each
+                tmem_st16(tS + lane_base + c * 32, pp);
+                tmem_st16(tP + lane_base + c * 32, ds);
+                tmem_st_wait();
             }
-            if (!ok) break;
-            fence_proxy_async();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(pds_full));
@@ -671,11 +651,12 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
 __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_constant__ AttnBwdParams p)
 {
     extern __shared__ __align__(1024) uint8_t at_smem[];
-    uint8_t *sQ = at_smem, *sA = sQ + AT_TILE, *sK = sA + AT_TILE, *sV = sK + 2 * AT_ITILE, *sS = sV + 2 * AT_ITILE;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sS + AT_BM * AT_BI * 2);
-    uint64_t *qa_full = bars, *kv_full = bars + 1, *kv_empty = bars + 3, *s_full = bars + 5, *ds_full = bars + 6,
-             *acc_done = bars + 7, *spare = bars + 8;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 10);
+    constexpr int NS = AT_DQ_NS;
+    uint8_t *sQ = at_smem, *sA = sQ + AT_TILE, *sK = sA + AT_TILE, *sV = sK + NS * AT_ITILE;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sV + NS * AT_ITILE);
+    uint64_t *qa_full = bars, *s_full = bars + 1, *ds_full = bars + 2, *acc_done = bars + 3, *spare = bars + 4, *s_free = bars + 5,
+             *kv_full = bars + 6, *kv_empty = kv_full + NS;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(kv_empty + NS);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -686,8 +667,9 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
     if (__syncthreads_or(threadIdx.x == 0 && at_error_seen(p.errword))) { pdl_wait(); return; }   // uniform over the CTA
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(qa_full), 1);
-        for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&kv_full[i]), 1); mbar_init(smem_u32(&kv_empty[i]), 1); }
+        for (int i = 0; i < NS; i++) { mbar_init(smem_u32(&kv_full[i]), 1); mbar_init(smem_u32(&kv_empty[i]), 1); }
         mbar_init(smem_u32(s_full), 1);
+        mbar_init(smem_u32(s_free), 8);
         mbar_init(smem_u32(ds_full), 8);
         mbar_init(smem_u32(acc_done), 1);
         mbar_init(smem_u32(spare), 1);
@@ -701,7 +683,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
     pdl_wait();                               // barriers and TMEM above are this kernel's own; its inputs come below
     pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t tS = tmem_base, tP = tmem_base + 64, tdQ = tmem_base + 128;
+    const uint32_t tS = tmem_base, tP = tmem_base + 64, tdQ = tmem_base + 128, tdS = tmem_base + 192;
 
     const int BH = p.B * p.H;
     const int qt = p.nqt - 1 - (int)blockIdx.x / BH, bh = (int)blockIdx.x % BH;
@@ -721,8 +703,8 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
             tma_load_2d(smem_u32(sA), &p.da_map, smem_u32(qa_full), h * AT_HD, b * p.T + q0);
         }
         for (int t = 0; ok && t < nt; t++) {
-            const int st = t & 1;
-            ok = at_wait(smem_u32(&kv_empty[st]), (((uint32_t)t >> 1) & 1u) ^ 1u, abort_flag, p.errword, 301);
+            const int st = t % NS;
+            ok = at_wait(smem_u32(&kv_empty[st]), ((uint32_t)(t / NS) & 1u) ^ 1u, abort_flag, p.errword, 301);
             if (!ok) break;
             if (elect_one()) {
                 const uint32_t bar = smem_u32(&kv_full[st]);
@@ -736,8 +718,8 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
         }
         if (*abort_flag) {
             for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(qa_full), 0); i++) {}
-            for (int t = issued > 2 ? issued - 2 : 0; t < issued; t++)
-                for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(&kv_full[t & 1]), ((uint32_t)t >> 1) & 1u); i++) {}
+            for (int t = issued > NS ? issued - NS : 0; t < issued; t++)
+                for (uint32_t i = 0; i < AT_WAIT_LIMIT && !mbar_try(smem_u32(&kv_full[t % NS]), (uint32_t)(t / NS) & 1u); i++) {}
         }
     } else if (warp == 1) {
         constexpr uint32_t IDESC_S = make_idesc(AT_BM, AT_BI, 0, 0);
@@ -760,23 +742,24 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
             __syncwarp();
         }
         for (int t = 0; ok && t < nt; t++) {
-            const int st = t & 1;
+            const int st = t % NS;
+            if (t + 1 < nt) {                                 // next scores first, see k_attn_bwd_dkv
+                const int sn = (t + 1) % NS;
+                ok = at_wait(smem_u32(&kv_full[sn]), (uint32_t)((t + 1) / NS) & 1u, abort_flag, p.errword, 313);
+                if (ok) ok = at_wait(smem_u32(s_free), (uint32_t)t & 1u, abort_flag, p.errword, 314);
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) issue_scores(sn);
+                __syncwarp();
+            }
             ok = at_wait(smem_u32(ds_full), (uint32_t)t & 1u, abort_flag, p.errword, 312);
             if (!ok) break;
             tc_fence_after();
-            if (t + 1 < nt) {                                 // next scores first, see k_attn_bwd_dkv
-                ok = at_wait(smem_u32(&kv_full[st ^ 1]), ((uint32_t)(t + 1) >> 1) & 1u, abort_flag, p.errword, 313);
-                if (!ok) break;
-                tc_fence_after();
-                if (elect_one()) issue_scores(st ^ 1);
-                __syncwarp();
-            }
             if (elect_one()) {
-                const uint32_t s_ = smem_u32(sS), k_ = smem_u32(sK + st * AT_ITILE);
+                const uint32_t k_ = smem_u32(sK + st * AT_ITILE);
 #pragma unroll
                 for (int kk = 0; kk < AT_BI / 16; kk++)       // dQ += dS K
-                    tc_mma_bf16(tdQ, make_desc(s_ + kk * 32, 16, 1024),
-                                make_desc(k_ + kk * 2048, 8192, 1024), IDESC_ACC, (t > 0 || kk > 0) ? 1u : 0u);
+                    tc_mma_bf16_ta(tdQ, tdS + kk * 8, make_desc(k_ + kk * 2048, 8192, 1024), IDESC_ACC, (t > 0 || kk > 0) ? 1u : 0u);
                 tc_commit(smem_u32(acc_done));
                 tc_commit(smem_u32(&kv_empty[st]));
             }
@@ -804,6 +787,9 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
             tmem_ld32(tS + lane_base + c * 32, sv);
             tmem_ld32(tP + lane_base + c * 32, dv);
             tmem_ld_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(s_free));       // the next scores may overwrite these
             {
                 uint32_t ds[16];
                 auto compute = [&](auto mode, int lo, int hi) {       // keys lo < j <= hi of the thread's 32 (see k_attn_bwd_dkv)
@@ -826,18 +812,10 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
                 if (!masked) compute(AtMode<0>(), 0, 0);
                 else if (p.win <= 0) compute(AtMode<1>(), 0, hi);
                 else compute(AtMode<2>(), i - p.win - base, hi);
-                if (t > 0) ok = at_wait(smem_u32(acc_done), (uint32_t)(t - 1) & 1u, abort_flag, p.errword, 322);   // dS tile free again
-                uint8_t *srow = sS + r * 128;
-                if (ok) {
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int unit = (c * 4 + u) ^ (r & 7);
-                        *reinterpret_cast<uint4 *>(srow + unit * 16) = make_uint4(ds[4 * u], ds[4 * u + 1], ds[4 * u + 2], ds[4 * u + 3]);
-                    }
-                }
+                if (t > 0) ok = at_wait(smem_u32(acc_done), (uint32_t)(t - 1) & 1u, abort_flag, p.errword, 322);   // dS columns free again
+                if (ok) { tc_fence_after(); tmem_st16(tdS + lane_base + c * 16, ds); tmem_st_wait(); }
             }
             if (!ok) break;
-            fence_proxy_async();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(ds_full));
@@ -887,7 +865,7 @@ extern "C" int qlmb_attn_fwd(void *O, float *lse, const void *Q, const void *K, 
         QLMB_CUDA(cudaFuncSetAttribute(k_attn_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_FWD_SMEM));
         configured_dev[dev_] = true;
     }
-    QLMB_CUDA(pdl_launch_small(k_attn_fwd, dim3((unsigned)(p.nqt * B * H)), dim3(320), AT_FWD_SMEM, as_stream(stream), p));
+    QLMB_CUDA(pdl_launch_small(k_attn_fwd, dim3((unsigned)(p.nqt * B * H)), dim3(AT_FWD_THREADS), AT_FWD_SMEM, as_stream(stream), p));
     QLMB_LAUNCH_CHECK("k_attn_fwd");
     return QLMB_OK;
 }

@@ -91,3 +91,31 @@ def test_attn_backward(cuda, B, T, H, KV, win):
     assert rel(dV.float().cpu().numpy(), dVr) < 1e-2
     assert rel(dK.float().cpu().numpy(), dKr) < 1e-2
     assert rel(dQ.float().cpu().numpy(), dQr) < 1e-2
+
+
+@pytest.mark.parametrize("T", [1, 31, 33, 64, 65, 127, 129, 257])
+@pytest.mark.parametrize("win", [0, 1, 64, 129])
+def test_attn_edges(cuda, T, win):
+    """Sequence lengths around the tiles of 32, 64 and 128 rows, windows that end inside them, and scores that grow along the
+    keys, so that most steps of a row bring a new maximum and O is rescaled.  The bar is that of the tests above: P and dS are
+    bf16 (2^-9 each), O and the gradients are rounded once more, D is made of the rounded O."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import attn
+    B, H, KV = 2, 2, 1
+    _, (Qh, Kh, Vh) = inputs(B, T, H, KV, 11, cuda)
+    Kh = Kh * np.tile(1.0 + 2.0 * np.arange(T) / T, B)[:, None].astype(np.float32)
+    Kh = torch.from_numpy(Kh).to(torch.bfloat16).float().numpy()
+    g = torch.Generator(device="cpu"); g.manual_seed(13)
+    dA = torch.randn(B * T, H * 64, generator=g).to(torch.bfloat16)
+    Or, lr, dQr, dKr, dVr = torch_attention(Qh, Kh, Vh, B, T, H, KV, win, dA.float().numpy())
+    Qd, Kd, Vd = [torch.from_numpy(x).to(torch.bfloat16).to(cuda) for x in (Qh, Kh, Vh)]
+    O, lse = attn.attn_fwd(Qd, Kd, Vd, B, T, H, KV, win)
+    dQ, dK, dV, _ = attn.attn_bwd(Qd, Kd, Vd, O, dA.to(cuda), lse, B, T, H, KV, win)
+    torch.cuda.synchronize()
+    q.check(q.lib().qlmb_check_device(None))
+    norm = lambda a, b: float(np.linalg.norm(a.float().cpu().numpy().astype(np.float64) - b) / max(np.linalg.norm(b), 1e-3))
+    assert norm(O, Or) < 1e-2 and np.abs(lse.cpu().numpy() - lr).max() < 1e-3
+    # one visible key: dS is exactly zero in exact arithmetic, what is left is the rounding of O inside D
+    assert norm(dV, dVr) < 1e-2
+    if T > 1 and win != 1:
+        assert norm(dQ, dQr) < 1e-2 and norm(dK, dKr) < 1e-2
