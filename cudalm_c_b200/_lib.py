@@ -46,6 +46,11 @@ class DecStepArgs(C.Structure):
                [(n, C.c_void_p) for n in ("layers", "emb", "tok", "pos", "cosb", "sinb", "nf", "fn", "ws")]
 
 
+class Qkv(C.Structure):
+    _fields_ = [(n, C.c_int) for n in ("M", "D", "KD", "T")] + \
+               [("codes", C.c_void_p * 3), ("scales", C.c_void_p * 3), ("cosb", C.c_void_p), ("sinb", C.c_void_p)]
+
+
 PROTOTYPES = {
     "qlmb_last_error": (C.c_char_p, []),
     "qlmb_version": (ci, []),
@@ -112,6 +117,9 @@ PROTOTYPES = {
     "qlmb_dec_sample": (ci, [vp, vp, vp, vp, ci, ci, vp]),
     "qlmb_attn_fwd": (ci, [vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, ci, vp]),
     "qlmb_attn_bwd": (ci, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, ci, vp]),
+    "qlmb_attn_bwd_rope": (ci, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, ci, vp]),
+    "qlmb_qkv_fwd": (ci, [C.POINTER(Qkv), vp, vp, vp, vp, vp]),
+    "qlmb_qkv_bwd": (ci, [C.POINTER(Qkv), vp, vp, vp, vp, vp, vp, vp, vp, cf, vp]),
     "qlmb_adamw": (ci, [vp, vp, vp, vp, sz, cf, cf, cf, cf, cf, cf, vp, vp]),
     "qlmb_linear_fwd": (ci, [vp, vp, vp, vp, ci, ci, ci, ci, vp, ci, vp]),
     "qlmb_linear_dgrad": (ci, [vp, vp, vp, vp, ci, ci, ci, ci, cf, ci, vp]),

@@ -92,6 +92,43 @@ __device__ __forceinline__ float ex2(float x)
 }
 template <int M> struct AtMode { static constexpr int value = M; };     // which masks a tile needs
 
+// The same with the rotation of pairs (j, j + 32) undone: cp, sp = the row's 32 cosines and sines.  part 0: columns 0 .. 31 of the
+// row, 1: columns 32 .. 63, 2: all of it.
+__device__ __forceinline__ void attn_store_rot(bf16 *dst, uint32_t taddr, bool live, float mul, const float *cp, const float *sp, int part)
+{
+#pragma unroll
+    for (int ch = 0; ch < 2; ch++) {
+        uint32_t a[16], b[16];
+        tmem_ld16(taddr + 16 * ch, a);
+        tmem_ld16(taddr + 32 + 16 * ch, b);
+        tmem_ld_wait();
+        if (!live) continue;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            uint32_t lo[4], hi[4];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int j = 8 * u + 4 * k;
+                const float4 c = *reinterpret_cast<const float4 *>(cp + 16 * ch + j), s = *reinterpret_cast<const float4 *>(sp + 16 * ch + j);
+                const float cc[4] = {c.x, c.y, c.z, c.w}, ss[4] = {s.x, s.y, s.z, s.w};
+                float l4[4], h4[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const float x = __uint_as_float(a[j + e]) * mul, y = __uint_as_float(b[j + e]) * mul;
+                    l4[e] = x * cc[e] + y * ss[e];
+                    h4[e] = y * cc[e] - x * ss[e];
+                }
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const __nv_bfloat162 l2 = __floats2bfloat162_rn(l4[2 * e], l4[2 * e + 1]), h2 = __floats2bfloat162_rn(h4[2 * e], h4[2 * e + 1]);
+                    lo[2 * k + e] = *reinterpret_cast<const uint32_t *>(&l2); hi[2 * k + e] = *reinterpret_cast<const uint32_t *>(&h2);
+                }
+            }
+            if (part != 1) *reinterpret_cast<uint4 *>(dst + 16 * ch + 8 * u) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            if (part != 0) *reinterpret_cast<uint4 *>(dst + 32 + 16 * ch + 8 * u) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        }
+    }
+}
 // two floats in one 64-bit register: sm_100's two-wide multiply-add and add
 __device__ __forceinline__ uint64_t f2_packu(uint32_t a, uint32_t b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b)); return r; }
 __device__ __forceinline__ uint64_t f2_pack(float a, float b) { return f2_packu(__float_as_uint(a), __float_as_uint(b)); }
@@ -407,6 +444,7 @@ struct AttnBwdParams {
     alignas(64) CUtensorMap q_imap, k_imap, v_imap, da_imap;  // boxes of 64 rows (walked tiles)
     const float *lse, *drow;
     bf16 *dQ, *dK, *dV;
+    const float *cosb, *sinb;                                 // not NULL: dQ and dK leave rotated back
     int B, T, H, KV, win, nqt;
     float scale, scale_log2;
     int *errword;
@@ -640,7 +678,12 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
             tc_fence_after();
             // chunk 0: the dV row; chunk 1: the dK row
             bf16 *dst = (c ? p.dK : p.dV) + ((size_t)b * p.T + key) * ((size_t)p.KV * AT_HD) + (size_t)kvh * AT_HD;
-            attn_store_row64(dst, (c ? tdK : tdV) + lane_base, key < p.T, c ? p.scale : 1.0f);
+            if (c && p.cosb) {
+                const size_t pos = (size_t)(key < p.T ? key : 0) * 32;
+                attn_store_rot(dst, tdK + lane_base, key < p.T, p.scale, p.cosb + pos, p.sinb + pos, 2);
+            } else {
+                attn_store_row64(dst, (c ? tdK : tdV) + lane_base, key < p.T, c ? p.scale : 1.0f);
+            }
         }
         tc_fence_before();
     }
@@ -824,7 +867,13 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
         if (ok) {
             tc_fence_after();
             // each of the row's two threads stores half of it
-            attn_store_row32(p.dQ + ((size_t)b * p.T + i) * ((size_t)p.H * AT_HD) + (size_t)h * AT_HD + c * 32, tdQ + lane_base + c * 32, i < p.T, p.scale);
+            bf16 *dst = p.dQ + ((size_t)b * p.T + i) * ((size_t)p.H * AT_HD) + (size_t)h * AT_HD;
+            if (p.cosb) {
+                const size_t pos = (size_t)(i < p.T ? i : 0) * 32;
+                attn_store_rot(dst, tdQ + lane_base, i < p.T, p.scale, p.cosb + pos, p.sinb + pos, c);
+            } else {
+                attn_store_row32(dst + c * 32, tdQ + lane_base + c * 32, i < p.T, p.scale);
+            }
         }
         tc_fence_before();
     }
@@ -870,9 +919,9 @@ extern "C" int qlmb_attn_fwd(void *O, float *lse, const void *Q, const void *K, 
     return QLMB_OK;
 }
 
-extern "C" int qlmb_attn_bwd(void *dQ, void *dK, void *dV, float *drow, const void *Q, const void *K, const void *V,
-                             const void *O, const void *dA, const float *lse, int B, int T, int H, int KV, int hd,
-                             int win, void *stream)
+static int attn_bwd_impl(void *dQ, void *dK, void *dV, float *drow, const void *Q, const void *K, const void *V,
+                         const void *O, const void *dA, const float *lse, const float *cosb, const float *sinb, int B, int T,
+                         int H, int KV, int hd, int win, void *stream)
 {
     QLMB_REQUIRE(dQ && dK && dV && drow && Q && K && V && O && dA && lse, "qlmb_attn_bwd: NULL argument");
     QLMB_REQUIRE(hd == AT_HD, "qlmb_attn_bwd: head dimension %d (only 64 is built)", hd);
@@ -889,6 +938,7 @@ extern "C" int qlmb_attn_bwd(void *dQ, void *dK, void *dV, float *drow, const vo
     }
     p.lse = lse; p.drow = drow;
     p.dQ = (bf16 *)dQ; p.dK = (bf16 *)dK; p.dV = (bf16 *)dV;
+    p.cosb = cosb; p.sinb = sinb;
     p.B = B; p.T = T; p.H = H; p.KV = KV; p.win = win;
     p.nqt = (T + AT_BM - 1) / AT_BM;
     p.scale = 1.0f / sqrtf((float)hd);
@@ -911,4 +961,18 @@ extern "C" int qlmb_attn_bwd(void *dQ, void *dK, void *dV, float *drow, const vo
     QLMB_CUDA(pdl_launch_small(k_attn_bwd_dq, dim3((unsigned)(p.nqt * B * H)), dim3(AT_BWD_THREADS), AT_DQ_SMEM, st, p));
     QLMB_LAUNCH_CHECK("k_attn_bwd");
     return QLMB_OK;
+}
+
+extern "C" int qlmb_attn_bwd(void *dQ, void *dK, void *dV, float *drow, const void *Q, const void *K, const void *V,
+                             const void *O, const void *dA, const float *lse, int B, int T, int H, int KV, int hd,
+                             int win, void *stream)
+{
+    return attn_bwd_impl(dQ, dK, dV, drow, Q, K, V, O, dA, lse, nullptr, nullptr, B, T, H, KV, hd, win, stream);
+}
+extern "C" int qlmb_attn_bwd_rope(void *dQ, void *dK, void *dV, float *drow, const void *Q, const void *K, const void *V,
+                                  const void *O, const void *dA, const float *lse, const float *cosb, const float *sinb,
+                                  int B, int T, int H, int KV, int hd, int win, void *stream)
+{
+    QLMB_REQUIRE(cosb && sinb && ((((uintptr_t)cosb | (uintptr_t)sinb) & 15) == 0), "qlmb_attn_bwd_rope: tables must be given and 16-byte aligned");
+    return attn_bwd_impl(dQ, dK, dV, drow, Q, K, V, O, dA, lse, cosb, sinb, B, T, H, KV, hd, win, stream);
 }

@@ -40,13 +40,17 @@ constexpr int B_STAGE_BYTES = BN * BK * 2;
 constexpr int C_STAGE_BYTES = BN * BK / 2;
 
 struct GemmParams {
-    alignas(64) CUtensorMap a_map[2];
-    alignas(64) CUtensorMap w_map[2];
+    alignas(64) CUtensorMap a_map[3];
+    alignas(64) CUtensorMap w_map[3];
     alignas(64) CUtensorMap o_map[3];      // bf16 outputs written by bulk tensor stores (boxes of 32 rows x 64 columns)
     alignas(64) CUtensorMap i_map[2];      // SwiGLU backward: stashed gate / up, boxes of 32 rows x 32 columns
     int o_tma;                             // 1: o_map (and i_map) valid
-    const float *scales[2];
+    const float *scales[3];
     int nseg, ksteps;
+    int seg_steps[3], seg_gpr[3];          // stages and scale groups per stored row, by segment or matrix
+    int slices;                            // SCHED_SLICES: row slices per matrix
+    int mat_tile[2], mat_N[3];             // EPI_MATS: first column tile of matrices 1 and 2, columns of each
+    const float *cosb, *sinb; int rope_T, rope_mats;
     int M, N, E;
     int tiles_m, tiles_n;
     int w_rows, w_cols;
@@ -226,7 +230,8 @@ struct Ring {
 };
 
 // m0: first row of the tile; halves: how many 128-row halves carry rows (1 or 2)
-struct TileInfo { int m0, n_t, e, ksteps, row0, halves; };
+// mat: matrix of a tile of several (EPI_MATS, SCHED_SLICES)
+struct TileInfo { int m0, n_t, e, ksteps, row0, halves, mat; };
 
 template <int SCHED>
 __device__ __forceinline__ TileInfo decode_tile(const GemmParams &p, int tile, int ntr)
@@ -255,7 +260,9 @@ __device__ __forceinline__ TileInfo decode_tile(const GemmParams &p, int tile, i
 
 __device__ __forceinline__ float sigmoid_f(float z) { return __fdividef(1.0f, 1.0f + __expf(-z)); }
 
-struct EpiCtx;
+// Per-warp state: the SwiGLU-backward epilogue's input ring (two mbarriers, one per 4 KiB buffer, and the parity to wait for
+// next on each); the tile's matrix.
+struct EpiCtx { uint64_t *bar; uint32_t ph; int mat; };
 __device__ __forceinline__ bool swiglu_bwd_bulk(const GemmParams &p, uint8_t *stage, EpiCtx &ec, int lane, uint32_t tbase,
                                                 long long rbase, long long col0);
 
@@ -295,6 +302,50 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams &p, uint8_t *stag
             if (p.scatter_perm) blk_store_scattered(stage, lane, mine, (int)(col0 + half * 64));
             else if (p.o_tma) blk_store_bulk(stage, lane, &p.o_map[0], (int)(col0 + half * 64), (int)rbase);
             else blk_store(stage, lane, reinterpret_cast<uint8_t *>((bf16 *)p.out + rbase * p.ldo + col0 + half * 64), p.ldo * 2, valid);
+        }
+    } else if (EPI == EPI_MATS) {
+        // 64 columns are one head.  A rotated matrix turns its pairs (i, i + 32) in the staged block, where eight lanes hold a row
+        // (with a lane per row every load of the tables touched 32 lines, on the port that the multiplies read through): lane
+        // c has columns 8c .. 8c + 7 and gets their partners from lane c ^ 4.  The values are rounded to bf16 before as after, as
+        // a separate rotation of the stored projection does.
+        const bool rot = ec.mat < p.rope_mats;
+        const int pos = rot ? (int)((rbase + lane) % p.rope_T) : 0, tc = (lane & 3) * 8;
+        const float sgn = (lane & 4) ? 1.0f : -1.0f;
+#pragma unroll 1
+        for (int half = 0; half < 2; half++) {
+            uint32_t v[64];
+            tmem_ld32(tbase + half * 64, v);
+            tmem_ld32(tbase + half * 64 + 32, v + 32);
+            tmem_ld_wait();
+            uint4 w[8];
+            __nv_bfloat162 *hw = reinterpret_cast<__nv_bfloat162 *>(w);
+#pragma unroll
+            for (int i = 0; i < 32; i++) hw[i] = __floats2bfloat162_rn(__uint_as_float(v[acc_col<NPERM>(2 * i)]), __uint_as_float(v[acc_col<NPERM>(2 * i + 1)]));
+            blk_reuse(lane);
+#pragma unroll
+            for (int k = 0; k < 8; k++) *blk_vec(stage, lane, k) = w[k];
+            if (rot) {
+                __syncwarp();
+#pragma unroll 2
+                for (int j = 0; j < 8; j++) {
+                    const int r = j * 4 + (lane >> 3), at = __shfl_sync(0xffffffffu, pos, r) * 32 + tc;
+                    const float4 c0 = *reinterpret_cast<const float4 *>(p.cosb + at), c1 = *reinterpret_cast<const float4 *>(p.cosb + at + 4);
+                    const float4 s0 = *reinterpret_cast<const float4 *>(p.sinb + at), s1 = *reinterpret_cast<const float4 *>(p.sinb + at + 4);
+                    const float cc[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, ss[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+                    uint4 x = *blk_vec(stage, r, lane & 7);
+                    uint32_t *xw = reinterpret_cast<uint32_t *>(&x);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const uint32_t y = __shfl_xor_sync(0xffffffffu, xw[k], 4);
+                        const float x0 = __uint_as_float(xw[k] << 16), x1 = __uint_as_float(xw[k] & 0xffff0000u);
+                        const float y0 = __uint_as_float(y << 16), y1 = __uint_as_float(y & 0xffff0000u);
+                        const __nv_bfloat162 o = __floats2bfloat162_rn(fmaf(sgn * y0, ss[2 * k], x0 * cc[2 * k]), fmaf(sgn * y1, ss[2 * k + 1], x1 * cc[2 * k + 1]));
+                        xw[k] = *reinterpret_cast<const uint32_t *>(&o);
+                    }
+                    *blk_vec(stage, r, lane & 7) = x;
+                }
+            }
+            blk_store_bulk(stage, lane, &p.o_map[ec.mat], (int)(col0 + half * 64), (int)rbase);
         }
     } else if ((EPI == EPI_STORE || EPI == EPI_ACCUM) && p.out_dtype == QLMB_F32 && p.o_tma) {
         // fp32 output through bulk tensor copies: 32 rows x 32 columns (128-byte rows) per block;
@@ -455,10 +506,6 @@ __device__ __forceinline__ void epilogue_rows(const GemmParams &p, uint8_t *stag
         }
     }
 }
-
-// Per-warp state of the SwiGLU-backward epilogue's input ring: two mbarriers (one per 4 KiB buffer)
-// and the parity to wait for next on each.
-struct EpiCtx { uint64_t *bar; uint32_t ph; };
 
 // SwiGLU backward over bulk tensor copies: the warp's 128 columns are four groups of 32; a group's
 // gate and up pieces (32 rows x 64 bytes each) arrive by TMA in one of two buffers, the results
@@ -710,7 +757,7 @@ k_gemm(const __grid_constant__ GemmParams p)
         // every global store instruction writes whole row pieces.
         const int q = warp & 3, h = (warp - 2) >> 2;
         uint8_t *stage = sE + (warp - 2) * epi_stage_bytes(EPI, false);
-        EpiCtx ec = {bars + 48 + 2 * (warp - 2), 0u};
+        EpiCtx ec = {bars + 48 + 2 * (warp - 2), 0u, 0};
         bool ok = true;
         int it = 0;
         for (int tile = blockIdx.x; ok && tile < total; tile += gridDim.x, it++) {
@@ -930,14 +977,25 @@ static bool use_pair(const GemmLaunch &g)
     return g.N % 128 == 0 && (g.epi == EPI_SWIGLU || g.N >= 256);
 }
 
+bool gemm_pair_takes(int N)
+{
+    GemmLaunch g = {};
+    g.N = N;
+    return use_pair(g);
+}
+
 int gemm_launch(const GemmLaunch &g, cudaStream_t st)
 {
     int rc = load_encode();
     if (rc) return rc;
-    const bool dual = g.epi == EPI_SWIGLU;
-    QLMB_REQUIRE(g.N % (dual ? BN / 2 : BN) == 0, "gemm: N=%d is not a multiple of the %d-column tile", g.N, dual ? BN / 2 : BN);
-    QLMB_REQUIRE(g.sched != SCHED_GROUPK || g.M % BM == 0, "gemm: grouped weight gradient needs M=%d to be a multiple of %d", g.M, BM);
-    const bool pair = use_pair(g);
+    const bool dual = g.epi == EPI_SWIGLU, mats = g.epi == EPI_MATS, segs = mats && g.nseg > 1;
+    QLMB_REQUIRE(!mats || (g.nmat >= 1 && g.nmat <= 3 && g.nseg >= 1 && g.nseg <= 3 && (g.nmat == 1 || g.nseg == 1) && (!g.rope_mats || (g.cosb && g.sinb && g.rope_T > 0))), "gemm: %d matrices", g.nmat);
+    for (int i = 0; mats && i < g.nmat; i++)
+        QLMB_REQUIRE(gemm_pair_takes(g.N_mat[i]), "gemm: several matrices or segments need the two-SM form");
+    QLMB_REQUIRE(mats || g.N % (dual ? BN / 2 : BN) == 0, "gemm: N=%d is not a multiple of the %d-column tile", g.N, dual ? BN / 2 : BN);
+    const bool grouped = g.sched == SCHED_GROUPK || g.sched == SCHED_SLICES;
+    QLMB_REQUIRE(!grouped || g.M % BM == 0, "gemm: grouped weight gradient needs M=%d to be a multiple of %d", g.M, BM);
+    const bool pair = mats || use_pair(g);
     GemmParams p;
     memset(&p, 0, sizeof p);
     p.nseg = g.nseg; p.ksteps = g.ksteps; p.M = g.M; p.N = g.N; p.E = g.E;
@@ -950,47 +1008,62 @@ int gemm_launch(const GemmLaunch &g, cudaStream_t st)
     p.errword = device_error_word();
     p.scatter_perm = g.scatter_perm; p.scatter_kn = g.scatter_kn;
     for (int i = 0; i < 8; i++) p.scatter_out[i] = (bf16 *)g.scatter_out[i];
-    p.scales[0] = g.scales[0]; p.scales[1] = g.scales[1];
+    for (int i = 0; i < 3; i++) {
+        p.seg_steps[i] = segs ? g.seg_cols[i] / BK : g.ksteps;
+        p.seg_gpr[i] = (segs ? g.seg_cols[i] : mats ? g.N_mat[i] : g.w_cols) / 128;
+        p.mat_N[i] = mats ? g.N_mat[i] : g.N;
+    }
+    p.slices = g.nmat > 1 ? g.E / g.nmat : g.E;
+    if (mats) {
+        int t = 0;
+        for (int i = 0; i < g.nmat; i++) { t += (g.N_mat[i] + 255) / 256; if (i < 2) p.mat_tile[i] = t; }
+        if (g.nmat < 2) p.mat_tile[0] = t;
+        if (g.nmat < 3) p.mat_tile[1] = t;
+        p.tiles_n = t;
+        p.cosb = g.cosb; p.sinb = g.sinb; p.rope_T = g.rope_T; p.rope_mats = g.rope_mats;
+    }
     const unsigned long long wrows_total = (unsigned long long)g.E * g.w_rows;
-    for (int s = 0; s < (dual ? 2 : g.nseg); s++) {
+    const int nw = dual ? 2 : (mats && !segs) || g.bmode == AB_TMA_MN ? (g.nmat > 1 ? g.nmat : 1) : g.nseg;
+    for (int i = 0; i < 3; i++) p.scales[i] = g.scales[i];
+    for (int s = 0; s < nw; s++) {
+        const int a_cols = segs ? g.seg_cols[s] : g.a_cols, w_cols = segs ? g.seg_cols[s] : mats ? g.N_mat[s] : g.w_cols;
         if (g.bmode == AB_TMA_MN) {
-            if (s > 0) break;
             // Asrc [a_rows][M-dim], Bsrc [a_rows][N]; boxes of 64 columns x 64 rows
-            rc = make_map(&p.a_map[0], g.a[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, g.a_cols, g.a_rows, (unsigned long long)g.a_cols * 2, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+            if (s == 0) rc = make_map(&p.a_map[0], g.a[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, g.a_cols, g.a_rows, (unsigned long long)g.a_cols * 2, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B);
             if (rc) return rc;
-            rc = make_map(&p.w_map[0], g.w[0], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, g.w_cols, g.a_rows, (unsigned long long)g.w_cols * 2, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+            rc = make_map(&p.w_map[s], g.w[s], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, g.w_cols, g.a_rows, (unsigned long long)g.w_cols * 2, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B);
             if (rc) return rc;
             continue;
         }
-        if (!dual || s == 0) {
-            const void *a = g.a[dual ? 0 : s];
-            rc = make_map(&p.a_map[s], a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, g.a_cols, g.a_rows, (unsigned long long)g.a_cols * 2, 64, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+        if (!(dual || mats) || segs || s == 0) {
+            rc = make_map(&p.a_map[s], g.a[s], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a_cols, g.a_rows, (unsigned long long)a_cols * 2, 64, 128, CU_TENSOR_MAP_SWIZZLE_128B);
             if (rc) return rc;
         }
         if (g.bmode == B_TMA_K) {
             rc = make_map(&p.w_map[s], g.w[s], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, g.w_cols, wrows_total, (unsigned long long)g.w_cols * 2, 64, BN, CU_TENSOR_MAP_SWIZZLE_128B);
         } else if (g.bmode == B_DEQ_MN) {
-            QLMB_REQUIRE(g.w_cols % 128 == 0, "gemm: code matrix width %d is not a multiple of the 128-element group", g.w_cols);
-            rc = make_map(&p.w_map[s], g.w[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g.w_cols / 2, wrows_total, g.w_cols / 2, (dual && !pair) ? BN / 4 : BN / 2, 64, CU_TENSOR_MAP_SWIZZLE_NONE);
+            QLMB_REQUIRE(w_cols % 128 == 0, "gemm: code matrix width %d is not a multiple of the 128-element group", w_cols);
+            rc = make_map(&p.w_map[s], g.w[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w_cols / 2, wrows_total, w_cols / 2, (dual && !pair) ? BN / 4 : BN / 2, 64, CU_TENSOR_MAP_SWIZZLE_NONE);
         } else {
-            QLMB_REQUIRE(g.w_cols % 128 == 0, "gemm: code matrix width %d is not a multiple of the 128-element group", g.w_cols);
-            rc = make_map(&p.w_map[s], g.w[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, g.w_cols / 2, wrows_total, g.w_cols / 2, 32, BN, CU_TENSOR_MAP_SWIZZLE_NONE);
+            QLMB_REQUIRE(w_cols % 128 == 0, "gemm: code matrix width %d is not a multiple of the 128-element group", w_cols);
+            rc = make_map(&p.w_map[s], g.w[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w_cols / 2, wrows_total, w_cols / 2, 32, BN, CU_TENSOR_MAP_SWIZZLE_NONE);
         }
         if (rc) return rc;
     }
     // bf16 outputs leave through bulk tensor stores when their layout allows a tensor map
     {
         const unsigned long long orows = (g.sched == SCHED_ROWS) ? (unsigned long long)g.a_rows
-                                       : (g.sched == SCHED_GROUPK) ? (unsigned long long)g.E * g.M : (unsigned long long)g.M;
+                                       : grouped ? (unsigned long long)g.E * g.M : (unsigned long long)g.M;
         const void *optr[3] = {nullptr, nullptr, nullptr};
         int no = 0;
         const bool f32out = (g.epi == EPI_STORE || g.epi == EPI_ACCUM) && g.out_dtype == QLMB_F32 && !g.resid &&
                             (g.beta == 0.0f || g.beta == 1.0f);
         if (f32out) { optr[0] = g.out; no = 1; }
         else if (g.epi == EPI_STORE && g.out_dtype == QLMB_BF16 && !g.resid && g.beta == 0.0f) { optr[0] = g.out; no = 1; }
+        else if (mats) { for (no = 0; no < g.nmat; no++) optr[no] = g.outs[no]; }
         else if (g.epi == EPI_SWIGLU) { optr[0] = g.ap; optr[1] = g.gp; optr[2] = g.up; no = 3; }
         else if (g.epi == EPI_SWIGLU_BWD) { optr[0] = g.dgp; optr[1] = g.dup; no = 2; }
-        bool can = no > 0 && (g.ldo % 8) == 0 && (g.sched != SCHED_GROUPK || f32out) && orows > 0;
+        bool can = no > 0 && (mats || (g.ldo % 8) == 0) && (!grouped || f32out) && orows > 0;
         for (int i = 0; i < no && can; i++) can = optr[i] && (((uintptr_t)optr[i]) & 15) == 0;
         const bool bwd = g.epi == EPI_SWIGLU_BWD;           // 32-column boxes, 64-byte swizzle
         if (bwd) can = can && g.gp && g.up && ((((uintptr_t)g.gp) | ((uintptr_t)g.up)) & 15) == 0;
@@ -999,8 +1072,8 @@ int gemm_launch(const GemmLaunch &g, cudaStream_t st)
                 rc = make_map(&p.o_map[i], optr[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (unsigned long long)g.ldo, orows,
                               (unsigned long long)g.ldo * 4, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B);
             else
-                rc = make_map(&p.o_map[i], optr[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (unsigned long long)g.ldo, orows,
-                              (unsigned long long)g.ldo * 2, bwd ? 32 : 64, 32, bwd ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
+                rc = make_map(&p.o_map[i], optr[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (unsigned long long)(mats ? g.N_mat[i] : g.ldo), orows,
+                              (unsigned long long)(mats ? g.N_mat[i] : g.ldo) * 2, bwd ? 32 : 64, 32, bwd ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
             if (rc) return rc;
         }
         for (int i = 0; i < 2 && can && bwd; i++) {
@@ -1008,6 +1081,7 @@ int gemm_launch(const GemmLaunch &g, cudaStream_t st)
                           (unsigned long long)g.ldo, orows, (unsigned long long)g.ldo * 2, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
             if (rc) return rc;
         }
+        QLMB_REQUIRE(!mats || can, "gemm: the outputs of several matrices must be 16-byte aligned");
         p.o_tma = can ? 1 : 0;
     }
     long long total;
@@ -1021,6 +1095,8 @@ int gemm_launch(const GemmLaunch &g, cudaStream_t st)
 
 #define PAIR(BM_, EP_, SC_) if (pair && g.bmode == BM_ && g.epi == EP_ && g.sched == SC_) return launch_pair<BM_, EP_, SC_>(p, total, st, !g.beside)
     PAIR(B_DEQ_MN, EPI_STORE, SCHED_DENSE);
+    PAIR(B_DEQ_MN, EPI_MATS, SCHED_DENSE);
+    PAIR(B_DEQ_K, EPI_MATS, SCHED_DENSE);
     PAIR(B_DEQ_K, EPI_STORE, SCHED_DENSE);
     PAIR(AB_TMA_MN, EPI_ACCUM, SCHED_DENSE);
     PAIR(B_TMA_K, EPI_STORE, SCHED_DENSE);
@@ -1029,6 +1105,7 @@ int gemm_launch(const GemmLaunch &g, cudaStream_t st)
     PAIR(B_DEQ_K, EPI_SWIGLU_BWD, SCHED_ROWS);
     PAIR(B_DEQ_K, EPI_STORE, SCHED_ROWS);
     PAIR(AB_TMA_MN, EPI_ACCUM, SCHED_GROUPK);
+    PAIR(AB_TMA_MN, EPI_ACCUM, SCHED_SLICES);
 #undef PAIR
 
 #define INST(BM_, EP_, SC_) if (g.bmode == BM_ && g.epi == EP_ && g.sched == SC_) return launch_inst<BM_, EP_, SC_>(p, grid, st, !g.beside)

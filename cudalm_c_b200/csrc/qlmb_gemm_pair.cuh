@@ -106,12 +106,17 @@ __device__ __forceinline__ void tc_mma2_bf16(uint32_t tmem_d, uint64_t adesc, ui
 // Pair tile: 256 rows starting at m0 (CTA r owns rows m0 + 128 r ...), 256 output columns
 // starting at n_t * 256 (CTA r expands columns + 128 r); with the SwiGLU epilogue the pair
 // tile is 128 gate + 128 up columns of the same 128 activation columns.
-template <int SCHED>
+template <int SCHED, bool MATS = false>
 __device__ __forceinline__ TileInfo decode_pair_tile(const GemmParams &p, int tile, int ntr)
 {
     TileInfo t;
+    t.mat = 0;
     if (SCHED == SCHED_DENSE) {
         t.m0 = (tile % p.tiles_m) * 256; t.n_t = tile / p.tiles_m; t.e = 0; t.ksteps = p.ksteps; t.row0 = 0;
+        if (MATS && t.n_t >= p.mat_tile[0]) {            // the matrices' column tiles follow one another
+            t.mat = t.n_t >= p.mat_tile[1] ? 2 : 1;
+            t.n_t -= p.mat_tile[t.mat - 1];
+        }
         t.halves = (t.m0 + BM < p.M) ? 2 : 1;
     } else if (SCHED == SCHED_ROWS) {
         // column tiles fastest: the pairs that run side by side share a row tile of A (which can be
@@ -125,9 +130,10 @@ __device__ __forceinline__ TileInfo decode_pair_tile(const GemmParams &p, int ti
         t.e = tile / per;
         int r = tile % per;
         t.m0 = (r % p.tiles_m) * 256; t.n_t = r / p.tiles_m;
-        // without a table: E equal slices of ksteps stages
-        t.row0 = p.off ? p.off[t.e] : t.e * p.ksteps * BK;
-        t.ksteps = p.off ? (p.off[t.e + 1] - p.off[t.e]) / BK : p.ksteps;
+        // without a table: equal slices of ksteps stages (SCHED_SLICES: the same ones for each B matrix)
+        if (SCHED == SCHED_SLICES) t.mat = t.e / p.slices;
+        t.row0 = SCHED == SCHED_SLICES ? (t.e - t.mat * p.slices) * p.ksteps * BK : p.off ? p.off[t.e] : t.e * p.ksteps * BK;
+        t.ksteps = SCHED != SCHED_SLICES && p.off ? (p.off[t.e + 1] - p.off[t.e]) / BK : p.ksteps;
         t.halves = (t.m0 + BM < p.M) ? 2 : 1;
     }
     return t;
@@ -139,6 +145,8 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
 {
     constexpr bool DEQ = (BMODE == B_DEQ_MN || BMODE == B_DEQ_K);
     constexpr bool DUAL = (EPI == EPI_SWIGLU);           // CTA 0 expands W1 (gate), CTA 1 expands W3 (up)
+    constexpr bool GROUPED = SCHED == SCHED_GROUPK || SCHED == SCHED_SLICES;
+    constexpr bool MATS = (EPI == EPI_MATS);             // several matrices side by side, or segments of different lengths
     constexpr int NS = EPI == EPI_SWIGLU_BWD ? 4 : 5, NCB = pair_code_bars(NS, DQG);
     // Without weights to expand there is room for a second staging block per epilogue warp (a sixth operand stage brought
     // nothing): 16 KiB of fp32 per warp and tile no longer wait block by block for the store before
@@ -168,7 +176,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
 
     if (warp == 1 && elect_one()) {                       // the copies' descriptors, ahead of their first use
         for (int i = 0; i < (DUAL ? 1 : p.nseg); i++) prefetch_map(&p.a_map[i]);
-        for (int i = 0; i < (DUAL ? 2 : p.nseg); i++) prefetch_map(&p.w_map[i]);
+        for (int i = 0; i < (DUAL ? 2 : MATS && p.nseg == 1 ? 1 : p.nseg); i++) prefetch_map(&p.w_map[i]);
     }
     if (threadIdx.x == 0) {
         for (int i = 0; i < NS; i++) { mbar_init(smem_u32(&full[i]), 1 + (DEQ ? 2 * GW : 0)); mbar_init(smem_u32(&empty[i]), 1); }
@@ -206,12 +214,13 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
             const uint32_t full0 = map_to_cta(smem_u32(full), 0), my_full = smem_u32(full), empty0 = smem_u32(empty);
             const uint32_t full_c0 = smem_u32(full_c), sA0 = smem_u32(sA), sB0 = smem_u32(sB), sC0 = smem_u32(sC);
             for (int tile = pair; ok && tile < total; tile += npairs) {
-                const TileInfo t = decode_pair_tile<SCHED>(p, tile, ntr);
+                const TileInfo t = decode_pair_tile<SCHED, MATS>(p, tile, ntr);
                 const int xa = t.m0 + my_m, xb = t.n_t * P_BN + my_n;
                 for (int seg = 0; ok && seg < p.nseg; seg++) {
-                    const CUtensorMap *am = &p.a_map[seg], *wm = &p.w_map[DUAL ? (int)rank : seg];
+                    const CUtensorMap *am = &p.a_map[seg], *wm = &p.w_map[DUAL ? (int)rank : MATS || SCHED == SCHED_SLICES ? seg + t.mat : seg];
+                    const int nks = MATS ? p.seg_steps[seg] : t.ksteps;
                     const int wrow = t.e * p.w_rows + (BMODE == B_DEQ_MN ? 0 : xb), wcol = DUAL ? t.n_t * 64 : xb / 2;
-                    for (int ks = 0; ks < t.ksteps; ks++) {
+                    for (int ks = 0; ks < nks; ks++) {
                         ok = mbar_wait(empty0 + rs.idx * 8u, rs.phase ^ 1u, abort_flag, p.errword, 11);
                         if (!ok) break;
                         if (leader) mbar_expect_tx(my_full + rs.idx * 8u, TX_BYTES);
@@ -246,7 +255,7 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
             bool ok = true;
             int it = 0;
             for (int tile = pair; ok && tile < total; tile += npairs, it++) {
-                TileInfo t = decode_pair_tile<SCHED>(p, tile, ntr);
+                TileInfo t = decode_pair_tile<SCHED, MATS>(p, tile, ntr);
                 const int acc = it & 1;
                 ok = mbar_wait_cluster(smem_u32(&tmem_empty[acc]), (((uint32_t)it >> 1) & 1u) ^ 1u, abort_flag, p.errword, 13);
                 if (!ok) break;
@@ -254,7 +263,8 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                 const uint32_t tmem_d = tmem_base + (uint32_t)acc * P_BN;
                 uint32_t accumulate = 0;
                 for (int seg = 0; ok && seg < p.nseg; seg++) {
-                    for (int ks = 0; ks < t.ksteps; ks++) {
+                    const int nks = MATS ? p.seg_steps[seg] : t.ksteps;
+                    for (int ks = 0; ks < nks; ks++) {
                         ok = mbar_wait_cluster(smem_u32(&full[rs.idx]), rs.phase, abort_flag, p.errword, 14);
                         if (!ok) break;
                         tc_fence_after();
@@ -296,21 +306,22 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
         bool ok = true;
         int it = 0;
         for (int tile = pair; ok && tile < total; tile += npairs, it++) {
-            TileInfo t = decode_pair_tile<SCHED>(p, tile, ntr);
+            TileInfo t = decode_pair_tile<SCHED, MATS>(p, tile, ntr);
             const int acc = it & 1;
             const long long row0 = (long long)t.m0 + my_m + q * 32;
             int valid = 32;
             if (SCHED == SCHED_ROWS) valid = ((int)rank < t.halves) ? 32 : 0;
             else { long long left = (long long)p.M - row0; valid = left < 0 ? 0 : (left < 32 ? (int)left : 32); }
-            const long long rbase = (SCHED == SCHED_GROUPK) ? ((long long)t.e * p.M + row0) : row0;
+            const long long rbase = GROUPED ? ((long long)t.e * p.M + row0) : row0;
             const long long col0 = (EPI == EPI_SWIGLU) ? (long long)t.n_t * 128 + h * 64 : (long long)t.n_t * P_BN + h * 128;
-            if (EPI != EPI_SWIGLU && col0 >= p.N) valid = 0;     // the half of a last tile that lies past the columns
+            ec.mat = t.mat;
+            if (EPI != EPI_SWIGLU && col0 >= (MATS ? p.mat_N[t.mat] : p.N)) valid = 0;     // the half of a last tile that lies past the columns
             if (valid > 0) epilogue_prefetch<EPI>(p, stage, ec, lane, rbase, col0, valid);
             ok = mbar_wait_idle(smem_u32(&tmem_full[acc]), ((uint32_t)it >> 1) & 1u, abort_flag, p.errword, 19);
             if (!ok) break;
             tc_fence_after();
             if (valid > 0) {
-                const bool have_acc = (SCHED != SCHED_GROUPK) || t.ksteps > 0;
+                const bool have_acc = !GROUPED || t.ksteps > 0;
                 const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)acc * P_BN;
                 if (EPI == EPI_SWIGLU)
                     epilogue_rows<EPI, TWO, BMODE == B_DEQ_MN>(p, stage, ec, lane, tbase + (uint32_t)h * 64, rbase, col0, valid, have_acc, 128);
@@ -350,7 +361,6 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
         bool ok = true;
         const uint32_t full0 = map_to_cta(smem_u32(&full[0]), 0);    // the leader's stage barriers
         const uint32_t full_c0 = smem_u32(full_c);
-        const int gpr = p.w_cols / 128;
         // A warp's words of a stage lie in 16 (codes [K][N]) or 32 (codes [N][K]) rows, each with one scale: lane m requests
         // that of row `srow` one stage ahead, and word i takes it from lane i * SPL + sub (one load and one conversion per
         // lane and stage; eight of each per lane took 500 cycles of the 1900 that a group spent on its stage).
@@ -360,21 +370,23 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
         const int m = BMODE == B_DEQ_MN ? lane & 15 : lane, srow = gw * SPL + m % SPL + m / SPL * ROWS_I;
         int kc = 0;                                                  // running stage index of this CTA
         for (int tile = pair; ok && tile < total; tile += npairs) {
-            TileInfo t = decode_pair_tile<SCHED>(p, tile, ntr);
+            TileInfo t = decode_pair_tile<SCHED, MATS>(p, tile, ntr);
             for (int seg = 0; ok && seg < p.nseg; seg++) {
-                int ks = (g - kc % DQG + DQG) % DQG;                 // first stage of this group in the tile
-                for (int i = 0; i < ks && i < t.ksteps; i++) { rb.next(NS); rc.next(NCB); }
+                const int nks = MATS ? p.seg_steps[seg] : t.ksteps;
+                const int gpr = MATS ? p.seg_gpr[seg + t.mat] : p.w_cols / 128, cols = MATS ? p.mat_N[t.mat] : p.N;
+                int ks = (g - kc % DQG + DQG) % DQG;                 // first stage of this group in the segment
+                for (int i = 0; i < ks && i < nks; i++) { rb.next(NS); rc.next(NCB); }
                 // one stage on is BK rows (codes [K][N]) or half a group (codes [N][K]) on; a half that lies past the
                 // columns expands zeros or the next matrix's codes with the scales of the half before it, for nobody
-                const int xs = t.n_t * P_BN + my_n < p.N ? t.n_t * P_BN + my_n : t.n_t * P_BN;
-                const float *sp = p.scales[DUAL ? (int)rank : seg]
+                const int xs = t.n_t * P_BN + my_n < cols ? t.n_t * P_BN + my_n : t.n_t * P_BN;
+                const float *sp = p.scales[DUAL ? (int)rank : MATS ? seg + t.mat : seg]
                     + (BMODE == B_DEQ_MN ? (t.e * p.w_rows + srow) * gpr + (DUAL ? t.n_t : xs / 128)
                                          : (t.e * p.w_rows + xs + srow) * gpr);
                 const int sstep = BMODE == B_DEQ_MN ? BK * gpr : 0;
                 auto scale_at = [&](int k) { return sp[(BMODE == B_DEQ_MN ? k * sstep : (k * BK) / 128)]; };
-                float cur = ks < t.ksteps ? scale_at(ks) : 0.0f;
-                for (; ks < t.ksteps; ks += DQG) {
-                    const float nxt = ks + DQG < t.ksteps ? scale_at(ks + DQG) : 0.0f;
+                float cur = ks < nks ? scale_at(ks) : 0.0f;
+                for (; ks < nks; ks += DQG) {
+                    const float nxt = ks + DQG < nks ? scale_at(ks + DQG) : 0.0f;
                     const __nv_bfloat162 s2 = __float2bfloat162_rn(cur);
                     ok = mbar_wait(full_c0 + rc.idx * 8u, rc.phase, abort_flag, p.errword, 20);
                     if (!ok) break;
@@ -391,14 +403,14 @@ k_gemm_pair(const __grid_constant__ GemmParams p)
                     fence_proxy_async();
                     __syncwarp();
                     if (elect_one()) mbar_arrive_remote(full0 + (uint32_t)rb.idx * 8u);
-                    const int adv = ks + DQG <= t.ksteps ? DQG : t.ksteps - ks;
+                    const int adv = ks + DQG <= nks ? DQG : nks - ks;
                     rb.idx += adv;
                     if (rb.idx >= NS) rb.idx -= NS;
                     rc.idx += adv;
                     if (rc.idx >= NCB) { rc.idx -= NCB; rc.phase ^= 1u; }
                     cur = nxt;
                 }
-                kc += t.ksteps;
+                kc += nks;
             }
         }
     }

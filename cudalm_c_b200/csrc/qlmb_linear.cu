@@ -76,13 +76,17 @@ static int check_linear(const char *who, int layout, int M, int K, int N, int dt
     return QLMB_OK;
 }
 
-// dW = beta * dW + part[0] + part[1] + ... in ascending slice order; n is a multiple of 4
-__global__ void __launch_bounds__(256) k_sum_slices(float *dW, const float *part, int S, size_t n, float beta)
+// dW = beta * dW + part[0] + part[1] + ... in ascending slice order; n is a multiple of 4; a row of the grid per matrix
+struct SumMats { float *dW[3]; };
+template <bool MATS>
+__global__ void __launch_bounds__(256) k_sum_slices(const SumMats m, const float *part, int S, size_t n, float beta)
 {
     pdl_wait();
     pdl_trigger();
     const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;
     if (i >= n) return;
+    float *dW = m.dW[MATS ? blockIdx.y : 0];
+    if (MATS) part += (size_t)blockIdx.y * S * n;
     float4 a = *reinterpret_cast<const float4 *>(part + i);
     for (int s = 1; s < S; s++) {
         const float4 b = *reinterpret_cast<const float4 *>(part + (size_t)s * n + i);
@@ -149,6 +153,59 @@ extern "C" int qlmb_linear_dgrad(void *dX, const void *dY, const int8_t *codes, 
     return gemm_launch(g, st);
 }
 
+// The weight gradients of nmat matrices of one size on the same X: dW[i][K,N] = X^T dY[i] (KN) or dW[i][N,K] = dY[i]^T X (NK).
+// A small weight matrix gives few output tiles (768 x 768: 9 tiles of 256 x 256 for 74 SM pairs) over a
+// long contraction (the M rows).  Then the rows are cut into S slices that run as the "experts" of the
+// grouped weight-gradient schedule, each into its own partial, and the partials are added in ascending
+// slice order: every element still has one writer and a fixed order.
+// A slice keeps at least eight stages of 64 rows; the rows past M that the last ones name are zeros to the copies.
+// (Only row counts that divided evenly were cut before: 8191 rows of 384 x 640, forward and both gradients, 119 -> 39 us.)
+static int wgrad_mats(float *const *dW, const void *const *dY, int nmat, int S, const void *X, int layout, int M, int K, int N,
+                      float beta, int dtype, cudaStream_t st)
+{
+    const int Md = layout == QLMB_KN ? K : N, Nd = layout == QLMB_KN ? N : K, stages = (M + 63) / 64;
+    const size_t conv = dtype == QLMB_F32 ? ((((size_t)M * K * 2 + 255) & ~(size_t)255) + (((size_t)M * N * 2 + 255) & ~(size_t)255)) : 0;
+    // Rows that divide evenly keep their slices' partial sums in the shared piece, behind the converted operands: a step
+    // that is captured after a first eager one finds it large enough, and an allocation and a free node for each of its
+    // calls would cost 0.6 % of a training step.  Other row counts, which need no scratch uncut, take their own.
+    const size_t part_bytes = S > 1 ? (size_t)nmat * S * Md * Nd * sizeof(float) : 0;
+    const bool shared = S > 1 && M % (256 * S) == 0;
+    StreamScratch own(st);
+    if (S > 1 && !shared && !own.get(part_bytes)) S = 1;
+    if (S == 1 && nmat > 1) return -1;                   // the caller takes the matrices one by one
+    int rc;
+    void *ws = nullptr;
+    if (conv || shared) { rc = workspace(conv + (shared ? part_bytes : 0), &ws); if (rc) return rc; }
+    float *part = shared ? (float *)((uint8_t *)ws + conv) : (float *)own.p;
+    const bf16 *xb, *gb;
+    bf16 *slot2 = conv ? (bf16 *)((uint8_t *)ws + (((size_t)M * K * 2 + 255) & ~(size_t)255)) : nullptr;
+    rc = as_bf16(X, dtype, (size_t)M * K, (bf16 *)ws, &xb, st);
+    if (rc) return rc;
+    rc = as_bf16(dY[0], dtype, (size_t)M * N, slot2, &gb, st);
+    if (rc) return rc;
+    GemmLaunch g = {};
+    g.bmode = AB_TMA_MN; g.epi = EPI_ACCUM; g.sched = SCHED_DENSE;
+    g.a[0] = layout == QLMB_KN ? xb : gb; g.a_rows = M; g.a_cols = Md;
+    g.w[0] = layout == QLMB_KN ? gb : xb; g.w_cols = Nd; g.w_rows = 0;
+    if (S > 1) {
+        for (int i = 1; i < nmat; i++) g.w[i] = dY[i];
+        g.sched = nmat > 1 ? SCHED_SLICES : SCHED_GROUPK; g.nmat = nmat;
+        g.nseg = 1; g.ksteps = (stages + S - 1) / S; g.M = Md; g.N = Nd; g.E = nmat * S;
+        g.out = part; g.out_dtype = QLMB_F32; g.ldo = Nd; g.beta = 0.0f; g.name = "gemm_wgrad_slices";
+        rc = gemm_launch(g, st);
+        if (rc) return rc;
+        const size_t n = (size_t)Md * Nd;
+        SumMats m = {};
+        for (int i = 0; i < nmat; i++) m.dW[i] = dW[i];
+        QLMB_CUDA(pdl_launch(true, nmat > 1 ? k_sum_slices<true> : k_sum_slices<false>, dim3((unsigned)((n / 4 + 255) / 256), (unsigned)nmat), dim3(256), 0, st, m, (const float *)part, S, n, beta));
+        QLMB_LAUNCH_CHECK("k_sum_slices");
+        return QLMB_OK;
+    }
+    g.nseg = 1; g.ksteps = (M + 63) / 64; g.M = Md; g.N = Nd; g.E = 1;
+    g.out = dW[0]; g.out_dtype = QLMB_F32; g.ldo = Nd; g.beta = beta;
+    return gemm_launch(g, st);
+}
+
 extern "C" int qlmb_linear_wgrad(float *dW, const void *dY, const void *X, int layout, int M, int K, int N,
                                  float beta, int dtype, void *stream)
 {
@@ -161,55 +218,93 @@ extern "C" int qlmb_linear_wgrad(float *dW, const void *dY, const void *X, int l
         if (beta == 0.0f) QLMB_CUDA(cudaMemsetAsync(dW, 0, (size_t)K * N * sizeof(float), st));
         return QLMB_OK;
     }
-    // dW[K,N] = X^T dY (KN)   or   dW[N,K] = dY^T X (NK)
     const int Md = layout == QLMB_KN ? K : N, Nd = layout == QLMB_KN ? N : K;
-    // A small weight matrix gives few output tiles (768 x 768: 9 tiles of 256 x 256 for 74 SM pairs) over a
-    // long contraction (the M rows).  Then the rows are cut into S slices that run as the "experts" of the
-    // grouped weight-gradient schedule, each into its own partial, and the partials are added in ascending
-    // slice order: every element still has one writer and a fixed order.
-    // A slice keeps at least eight stages of 64 rows; the rows past M that the last ones name are zeros to the copies.
-    // (Only row counts that divided evenly were cut before: 8191 rows of 384 x 640, forward and both gradients, 119 -> 39 us.)
     int S = 1;
-    const int stages = (M + 63) / 64;
-    {
-        const int tiles = ((Md + 255) / 256) * ((Nd + 255) / 256), pairs = sm_count() / 2;
-        while (S < 16 && tiles * S * 2 <= pairs && stages / (2 * S) >= 8) S *= 2;
+    const int stages = (M + 63) / 64, tiles = ((Md + 255) / 256) * ((Nd + 255) / 256), pairs = sm_count() / 2;
+    while (S < 16 && tiles * S * 2 <= pairs && stages / (2 * S) >= 8) S *= 2;
+    return wgrad_mats(&dW, &dY, 1, S, X, layout, M, K, N, beta, dtype, st);
+}
+
+// ---- the three input projections of an attention block (gpu_forward's wq, wk, wv with k_rope, cudalm.cu:5651-5660, and their part
+// of gpu_backward).  Each of the three alone is one and a third rounds of tiles for 74 SM pairs at 8192 x 768 x 768.
+static int check_qkv(const char *who, const qlmb_qkv *p)
+{
+    QLMB_REQUIRE(p && p->cosb && p->sinb && p->T > 0, "%s: NULL argument", who);
+    for (int i = 0; i < 3; i++) QLMB_REQUIRE(p->codes[i] && p->scales[i], "%s: NULL weights", who);
+    int rc = check_linear(who, QLMB_KN, p->M, p->D, p->D, QLMB_BF16);
+    return rc ? rc : check_linear(who, QLMB_KN, p->M, p->D, p->KD, QLMB_BF16);
+}
+
+extern "C" int qlmb_qkv_fwd(const qlmb_qkv *p, void *Yq, void *Yk, void *Yv, const void *X, void *stream)
+{
+    int rc = check_qkv("qlmb_qkv_fwd", p);
+    if (rc || p->M == 0) return rc;
+    QLMB_REQUIRE(Yq && Yk && Yv && X, "qlmb_qkv_fwd: NULL argument");
+    cudaStream_t st = as_stream(stream);
+    void *const Y[3] = {Yq, Yk, Yv};
+    const int N[3] = {p->D, p->KD, p->KD};
+    // one launch over the column tiles of all three, q and k rotated on the way out
+    if (gemm_pair_takes(p->D) && gemm_pair_takes(p->KD) && ((((uintptr_t)Yq | (uintptr_t)Yk | (uintptr_t)Yv) & 15) == 0) &&
+        ((((uintptr_t)p->cosb | (uintptr_t)p->sinb) & 15) == 0)) {
+        GemmLaunch g = {};
+        g.bmode = B_DEQ_MN; g.epi = EPI_MATS; g.sched = SCHED_DENSE;
+        g.a[0] = X; g.a_rows = p->M; g.a_cols = p->D;
+        for (int i = 0; i < 3; i++) { g.w[i] = p->codes[i]; g.scales[i] = p->scales[i]; g.N_mat[i] = N[i]; g.outs[i] = Y[i]; }
+        g.w_rows = p->D; g.w_cols = p->D; g.nmat = 3;
+        g.nseg = 1; g.ksteps = p->D / 64; g.M = p->M; g.N = p->D; g.E = 1;
+        g.out_dtype = QLMB_BF16; g.ldo = p->D;
+        g.cosb = p->cosb; g.sinb = p->sinb; g.rope_T = p->T; g.rope_mats = 2; g.name = "gemm_qkv";
+        return gemm_launch(g, st);
     }
-    const size_t conv = dtype == QLMB_F32 ? ((((size_t)M * K * 2 + 255) & ~(size_t)255) + (((size_t)M * N * 2 + 255) & ~(size_t)255)) : 0;
-    // Rows that divide evenly keep their slices' partial sums in the shared piece, behind the converted operands: a step
-    // that is captured after a first eager one finds it large enough, and an allocation and a free node for each of its
-    // calls would cost 0.6 % of a training step.  Other row counts, which need no scratch uncut, take their own.
-    const size_t part_bytes = S > 1 ? (size_t)S * Md * Nd * sizeof(float) : 0;
-    const bool shared = S > 1 && M % (256 * S) == 0;
-    StreamScratch own(st);
-    if (S > 1 && !shared && !own.get(part_bytes)) S = 1;
-    void *ws = nullptr;
-    if (conv || shared) { rc = workspace(conv + (shared ? part_bytes : 0), &ws); if (rc) return rc; }
-    float *part = shared ? (float *)((uint8_t *)ws + conv) : (float *)own.p;
-    const bf16 *xb, *gb;
-    bf16 *slot2 = conv ? (bf16 *)((uint8_t *)ws + (((size_t)M * K * 2 + 255) & ~(size_t)255)) : nullptr;
-    rc = as_bf16(X, dtype, (size_t)M * K, (bf16 *)ws, &xb, st);
-    if (rc) return rc;
-    rc = as_bf16(dY, dtype, (size_t)M * N, slot2, &gb, st);
-    if (rc) return rc;
-    GemmLaunch g = {};
-    g.bmode = AB_TMA_MN; g.epi = EPI_ACCUM; g.sched = SCHED_DENSE;
-    g.a[0] = layout == QLMB_KN ? xb : gb; g.a_rows = M; g.a_cols = Md;
-    g.w[0] = layout == QLMB_KN ? gb : xb; g.w_cols = Nd; g.w_rows = 0;
-    if (S > 1) {
-        g.sched = SCHED_GROUPK;
-        g.nseg = 1; g.ksteps = (stages + S - 1) / S; g.M = Md; g.N = Nd; g.E = S;
-        g.out = part; g.out_dtype = QLMB_F32; g.ldo = Nd; g.beta = 0.0f; g.name = "gemm_wgrad_slices";
-        rc = gemm_launch(g, st);
-        if (rc) return rc;
-        const size_t n = (size_t)Md * Nd;
-        QLMB_CUDA(pdl_launch(true, k_sum_slices, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, st, dW, (const float *)part, S, n, beta));
-        QLMB_LAUNCH_CHECK("k_sum_slices");
-        return QLMB_OK;
+    for (int i = 0; i < 3; i++) {
+        if ((rc = qlmb_linear_fwd(Y[i], X, p->codes[i], p->scales[i], QLMB_KN, p->M, p->D, N[i], nullptr, QLMB_BF16, stream))) return rc;
+        if (i < 2 && (rc = qlmb_rope(Y[i], QLMB_BF16, p->cosb, p->sinb, p->M, N[i] / 64, 64, p->T, 0, stream))) return rc;
     }
-    g.nseg = 1; g.ksteps = (M + 63) / 64; g.M = Md; g.N = Nd; g.E = 1;
-    g.out = dW; g.out_dtype = QLMB_F32; g.ldo = Nd; g.beta = beta;
-    return gemm_launch(g, st);
+    return QLMB_OK;
+}
+
+extern "C" int qlmb_qkv_bwd(const qlmb_qkv *p, void *dX, float *dWq, float *dWk, float *dWv, const void *dq, const void *dk,
+                            const void *dv, const void *X, float beta, void *stream)
+{
+    int rc = check_qkv("qlmb_qkv_bwd", p);
+    if (rc) return rc;
+    QLMB_REQUIRE(dWq && dWk && dWv && (p->M == 0 || (dX && dq && dk && dv && X)), "qlmb_qkv_bwd: NULL argument");
+    QLMB_REQUIRE(beta == 0.0f || beta == 1.0f, "qlmb_qkv_bwd: beta %g", beta);
+    cudaStream_t st = as_stream(stream);
+    const int M = p->M, D = p->D, N[3] = {D, p->KD, p->KD};
+    const void *const dY[3] = {dq, dk, dv};
+    float *const dW[3] = {dWq, dWk, dWv};
+    if (M > 0 && gemm_pair_takes(D) && ((uintptr_t)dX & 15) == 0) {      // one contraction over the columns of dq, dk and dv
+        GemmLaunch g = {};
+        g.bmode = B_DEQ_K; g.epi = EPI_MATS; g.sched = SCHED_DENSE;
+        g.a_rows = M; g.a_cols = D; g.w_rows = D; g.w_cols = D; g.nmat = 1; g.N_mat[0] = D; g.outs[0] = dX;
+        for (int i = 0; i < 3; i++) { g.a[i] = dY[i]; g.w[i] = p->codes[i]; g.scales[i] = p->scales[i]; g.seg_cols[i] = N[i]; }
+        g.nseg = 3; g.ksteps = D / 64; g.M = M; g.N = D; g.E = 1;
+        g.out = dX; g.out_dtype = QLMB_BF16; g.ldo = D; g.name = "gemm_qkv_dgrad";
+        if ((rc = gemm_launch(g, st))) return rc;
+    } else if (M > 0) {
+        for (int i = 0; i < 3; i++)
+            if ((rc = qlmb_linear_dgrad(dX, dY[i], p->codes[i], p->scales[i], QLMB_KN, M, D, N[i], i ? 1.0f : 0.0f, QLMB_BF16, stream))) return rc;
+    }
+    // The three weight gradients as one launch where they are of one size: of the slice counts the one with the fewest rounds of
+    // tiles times stages, six stages for a tile's start and end, and the slices' partial sums at a stage's time per 2 MB.
+    if (M > 0 && p->KD == D && gemm_pair_takes(D)) {
+        const int stages = (M + 63) / 64, t1 = (D + 255) / 256, tiles = 3 * t1 * t1, pairs = sm_count() / 2;
+        const double mb2 = 3.0 * D * D * 8.0 / 2e6;
+        int S = 0;
+        double best = 0.0;
+        for (int s = 2; s <= 8 && stages / s >= 8; s++) {
+            const double c = (double)((tiles * s + pairs - 1) / pairs) * ((stages + s - 1) / s + 6) + s * mb2;
+            if (!S || c < best) { S = s; best = c; }
+        }
+        if (S) {
+            rc = wgrad_mats(dW, dY, 3, S, X, QLMB_KN, M, D, D, beta, QLMB_BF16, st);
+            if (rc >= 0) return rc;
+        }
+    }
+    for (int i = 0; i < 3; i++)
+        if ((rc = qlmb_linear_wgrad(dW[i], dY[i], X, QLMB_KN, M, D, N[i], beta, QLMB_BF16, stream))) return rc;
+    return QLMB_OK;
 }
 
 // Engine check (not part of the reference's operator surface): C[M,N] (fp32) =

@@ -6,7 +6,7 @@ KN = codes of W[K,N] (the reference's own [in,out] storage, applied with g_ab),
 NK = codes of W[N,K] (applied with g_abt)."""
 import torch
 
-from ._lib import BF16, F32, KN, NK, calls, stream_ptr  # noqa: F401
+from ._lib import BF16, F32, KN, NK, Qkv, calls, check, lib, ptr, stream_ptr  # noqa: F401
 
 
 def _dt(t):
@@ -39,6 +39,31 @@ def linear_wgrad(dW, dY, X, layout, beta=1.0):
     N = dY.shape[1]
     calls.linear_wgrad(dW, dY, X, layout, M, K, N, beta, _dt(X), stream_ptr())
     return dW
+
+
+def _qkv(M, D, KD, ws, cosb, sinb, T):
+    a = Qkv(M, D, KD, T)
+    for i, (codes, scales) in enumerate(ws):
+        a.codes[i], a.scales[i] = ptr(codes), ptr(scales)
+    a.cosb, a.sinb = ptr(cosb), ptr(sinb)
+    return a
+
+
+def qkv_fwd(X, ws, KD, cosb, sinb, T):
+    """q, k, v = X @ deq(W) for ws = three (codes, scales) pairs [D, D], [D, KD], [D, KD] (layout KN, bf16), q and k rotated."""
+    M, D = X.shape
+    q, k, v = X.new_empty((M, D)), X.new_empty((M, KD)), X.new_empty((M, KD))
+    check(lib().qlmb_qkv_fwd(_qkv(M, D, KD, ws, cosb, sinb, T), ptr(q), ptr(k), ptr(v), ptr(X), stream_ptr()))
+    return q, k, v
+
+
+def qkv_bwd(dWs, dq, dk, dv, X, ws, cosb, sinb, T, beta=1.0):
+    """dX of qkv_fwd's projections (dq and dk rotated back already); dWs (fp32) = beta * dWs + X^T [dq | dk | dv]."""
+    M, D = X.shape
+    dX = torch.empty_like(X)
+    check(lib().qlmb_qkv_bwd(_qkv(M, D, dk.shape[1], ws, cosb, sinb, T), ptr(dX), ptr(dWs[0]), ptr(dWs[1]), ptr(dWs[2]), ptr(dq),
+                             ptr(dk), ptr(dv), ptr(X), beta, stream_ptr()))
+    return dX
 
 
 def gemv_decode(X, codes, scales, layout, N, out=None):

@@ -238,11 +238,7 @@ class QlmModel:
             w, f = ly["w"], self.fl[l]
             mo = moes[l] if moes is not None else ly["moe"]
             a_norm, r1 = block.rmsnorm_fwd(x, f["an1"])
-            qh = linear.linear_fwd(a_norm, *w["wq"], KN, c.D)
-            kh = linear.linear_fwd(a_norm, *w["wk"], KN, c.KD)
-            vh = linear.linear_fwd(a_norm, *w["wv"], KN, c.KD)
-            block.rope(qh, self.cosb, self.sinb, c.H, c.hd, T)
-            block.rope(kh, self.cosb, self.sinb, c.KV, c.hd, T)
+            qh, kh, vh = linear.qkv_fwd(a_norm, (w["wq"], w["wk"], w["wv"]), c.KD, self.cosb, self.sinb, T)
             att, lse = attn.attn_fwd(qh, kh, vh, B, T, c.H, c.KV)
             f_in = linear.linear_fwd(att, *w["wo"], KN, c.D, R=x)
             if self.world > 1 and moes is None:
@@ -281,15 +277,10 @@ class QlmModel:
             block.rmsnorm_bwd(dout, s["f_in"], f["an2"], s["r2"], dfnorm, dgamma=g)          # dout now = d f_in
             d_att = linear.linear_dgrad(dout, *w["wo"], KN, c.D)
             linear.linear_wgrad(gv("wo", (c.D, c.D)), dout, s["att"], KN, beta=0.0)
-            dq, dk, dv, _ = attn.attn_bwd(s["q"], s["k"], s["v"], s["att"], d_att, s["lse"], c.B, c.T, c.H, c.KV)
-            block.rope(dq, self.cosb, self.sinb, c.H, c.hd, c.T, back=True)
-            block.rope(dk, self.cosb, self.sinb, c.KV, c.hd, c.T, back=True)
-            d_an = linear.linear_dgrad(dq, *w["wq"], KN, c.D)
-            linear.linear_dgrad(dk, *w["wk"], KN, c.D, beta=1.0, out=d_an)
-            linear.linear_dgrad(dv, *w["wv"], KN, c.D, beta=1.0, out=d_an)
-            linear.linear_wgrad(gv("wq", (c.D, c.D)), dq, s["a_norm"], KN, beta=0.0)
-            linear.linear_wgrad(gv("wk", (c.D, c.KD)), dk, s["a_norm"], KN, beta=0.0)
-            linear.linear_wgrad(gv("wv", (c.D, c.KD)), dv, s["a_norm"], KN, beta=0.0)
+            rot = (self.cosb, self.sinb)
+            dq, dk, dv, _ = attn.attn_bwd(s["q"], s["k"], s["v"], s["att"], d_att, s["lse"], c.B, c.T, c.H, c.KV, rope=rot)
+            d_an = linear.qkv_bwd((self._g(l, "wq"), self._g(l, "wk"), self._g(l, "wv")), dq, dk, dv, s["a_norm"],
+                                  (w["wq"], w["wk"], w["wv"]), *rot, c.T, beta=0.0)
             g = self._g(l, "an1"); g.zero_()
             block.rmsnorm_bwd(dout, s["a_in"], f["an1"], s["r1"], d_an, dgamma=g)             # dout now = d a_in
             if self.fused:

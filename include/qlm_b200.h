@@ -254,6 +254,21 @@ int qlmb_linear_dgrad(void *dX, const void *dY, const int8_t *codes, const float
 int qlmb_linear_wgrad(float *dW, const void *dY, const void *X, int layout, int M, int K, int N,
                       float beta, int dtype, void *stream);
 
+/* The input projections of an attention block on bf16 rows X [M][D] (gpu_forward, cudalm.cu:5651-5660): Yq [M][D], Yk and
+ * Yv [M][KD] = X W, W = codes of [D][D], [D][KD], [D][KD] (layout KN), q and k rotated as qlmb_rope does it with heads of 64
+ * (row n has position n % T; tables [>= T][32]).  D and KD must be multiples of 128.
+ * qlmb_qkv_bwd: dX = dq Wq^T + dk Wk^T + dv Wv^T (bf16, overwritten) and dW = beta * dW + X^T dY for each (fp32, beta in
+ * {0,1}); dq and dk are gradients of the projections, i.e. rotated back (qlmb_attn_bwd_rope, or qlmb_rope with back). */
+typedef struct qlmb_qkv {
+    int M, D, KD, T;
+    const int8_t *codes[3];
+    const float *scales[3];
+    const float *cosb, *sinb;
+} qlmb_qkv;
+int qlmb_qkv_fwd(const qlmb_qkv *p, void *Yq, void *Yk, void *Yv, const void *X, void *stream);
+int qlmb_qkv_bwd(const qlmb_qkv *p, void *dX, float *dWq, float *dWk, float *dWv, const void *dq, const void *dk,
+                 const void *dv, const void *X, float beta, void *stream);
+
 /* Decode path (cudalm.cu:7178-7198, g_ab with M = live slots <= 64):
  * Y[B,N] = X[B,K] * deq(W), weight-streaming kernel. */
 int qlmb_gemv_decode(void *Y, const void *X, const int8_t *codes, const float *scales, int layout,
@@ -653,6 +668,12 @@ int qlmb_attn_fwd(void *O, float *lse, const void *Q, const void *K, const void 
 int qlmb_attn_bwd(void *dQ, void *dK, void *dV, float *drow, const void *Q, const void *K, const void *V,
                   const void *O, const void *dA, const float *lse, int B, int T, int H, int KV, int hd,
                   int win, void *stream);
+
+/* The same with dQ and dK rotated back on the way out (qlmb_rope with back, tables [>= T][32], 16-byte aligned): the gradients of
+ * the projections. */
+int qlmb_attn_bwd_rope(void *dQ, void *dK, void *dV, float *drow, const void *Q, const void *K, const void *V,
+                       const void *O, const void *dA, const float *lse, const float *cosb, const float *sinb, int B, int T,
+                       int H, int KV, int hd, int win, void *stream);
 
 #ifdef __cplusplus
 }

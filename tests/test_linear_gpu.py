@@ -352,3 +352,53 @@ def test_dec_qkv_equals_the_separate_kernels(cuda, B):
     assert torch.equal(Kc[torch.arange(B), pos.long()], Y[B:2 * B]) and torch.equal(Vc[torch.arange(B), pos.long()], Y[2 * B:])
     assert rel(Kc, Kc2) < 1e-3 and rel(Vc, Vc2) < 1e-3
     assert int((Kc != 7.0).sum()) <= B * D and int((Vc != 7.0).sum()) <= B * D
+
+
+@pytest.mark.parametrize("M,D,KD,T", [(1, 256, 256, 1), (255, 384, 128, 85), (257, 512, 256, 200), (2100, 768, 768, 700), (640, 640, 640, 64)])
+def test_qkv_projections_against_float64(cuda, M, D, KD, T):
+    """The three projections with their rotation and both gradients, on one and on several row tiles, with widths that end inside
+    a column tile and the fallback of a width of 128.  Bar: bf16 operands and results."""
+    from cudalm_c_b200 import block, linear
+    N = (D, KD, KD)
+    ws, deq = zip(*[(lambda q, w: (q, w))(*quantise(cuda, D, n, 40 + i)) for i, n in enumerate(N)])
+    ws = [(q.d, q.s) for q in ws]
+    g = torch.Generator(device=cuda); g.manual_seed(7)
+    rnd = lambda c: torch.randn(M, c, device=cuda, generator=g).to(torch.bfloat16)
+    X, dq, dk, dv = rnd(D), rnd(D), rnd(KD), rnd(KD)
+    cosb, sinb = block.rope_tables(T, 64, device=cuda)
+    Y = linear.qkv_fwd(X, ws, KD, cosb, sinb, T)
+    pos = torch.arange(M, device=cuda) % T
+    c, s = cosb.double()[pos][:, None], sinb.double()[pos][:, None]
+    for i in range(3):
+        ref = X.double() @ deq[i].double()
+        if i < 2:
+            h = ref.view(M, N[i] // 64, 64)
+            a, b = h[..., :32], h[..., 32:]
+            ref = torch.cat([a * c - b * s, b * c + a * s], -1).reshape(M, N[i])
+        assert float((Y[i].double() - ref).norm() / ref.norm()) < 1e-2
+    for beta in (0.0, 1.0):
+        dW = [torch.ones(D * n, device=cuda) for n in N]
+        dX = linear.qkv_bwd(dW, dq, dk, dv, X, ws, cosb, sinb, T, beta=beta)
+        ref = sum(d.double() @ w.double().T for d, w in zip((dq, dk, dv), deq))
+        assert float((dX.double() - ref).norm() / ref.norm()) < 1e-2
+        for w, d in zip(dW, (dq, dk, dv)):
+            ref = X.double().T @ d.double()
+            # bf16 products are exact in fp32: the sums' roundings alone
+            assert float((w.view(D, -1).double() - beta - ref).norm() / ref.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("B,T,H,KV,win", [(2, 130, 4, 2, 0), (1, 64, 2, 2, 30), (1, 1, 2, 2, 0)])
+def test_attention_gradients_rotated_back_on_the_way_out(cuda, B, T, H, KV, win):
+    """Against the separate rotation, which rounds to bf16 once more."""
+    from cudalm_c_b200 import attn, block
+    g = torch.Generator(device=cuda); g.manual_seed(8)
+    rnd = lambda c: torch.randn(B * T, c * 64, device=cuda, generator=g).to(torch.bfloat16)
+    Q, K, V, dA = rnd(H), rnd(KV), rnd(KV), rnd(H)
+    rot = block.rope_tables(T, 64, device=cuda)
+    O, lse = attn.attn_fwd(Q, K, V, B, T, H, KV, win)
+    dQ, dK, dV, _ = attn.attn_bwd(Q, K, V, O, dA, lse, B, T, H, KV, win)
+    rQ, rK, rV, _ = attn.attn_bwd(Q, K, V, O, dA, lse, B, T, H, KV, win, rope=rot)
+    assert torch.equal(dV, rV)
+    for d, r, n in ((dQ, rQ, H), (dK, rK, KV)):
+        block.rope(d, *rot, n, 64, T, back=True)
+        assert float((d.float() - r.float()).norm()) <= 2 ** -7 * float(d.float().norm()) + 1e-6
