@@ -105,6 +105,8 @@ PROTOTYPES = {
     "qlmb_gemv_decode_norm_stack": (ci, [vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, vp]),
     "qlmb_dec_qkv": (ci, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, vp]),
     "qlmb_gemv_decode_res_norm": (ci, [vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, vp]),
+    "qlmb_dec_qkv_attn": (ci, [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, vp]),
+    "qlmb_dec_wo_moe": (ci, [C.POINTER(MoeLayer), vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     "qlmb_selftest_rounding": (ci, [ci, ci, ci, vp, vp]),
     "qlmb_quiet_begin": (ci, [vp]),
     "qlmb_quiet_end": (ci, []),

@@ -5,6 +5,7 @@
 #include <cuda_bf16.h>
 #include <math.h>
 #include "qlmb_common.cuh"
+#include "qlmb_internal.h"
 
 namespace qlmb {
 
@@ -507,11 +508,17 @@ __device__ __forceinline__ void bf8_to_f(const uint4 &x, float f[8])
 #pragma unroll
     for (int k = 0; k < 4; k++) { f[2 * k] = __uint_as_float(u[k] << 16); f[2 * k + 1] = __uint_as_float(u[k] & 0xffff0000u); }
 }
-__global__ void __launch_bounds__(128) k_dec_attn(bf16_t *O, const bf16_t *Q, const bf16_t *Kc, const bf16_t *Vc, const int *pos,
-                                                  int win, int B, int Tm, int H, int KV, float scale, int *errword)
+// FIN: the head's q, k and v come as the K slices of the stacked projections' GEMV (rows [3][B][H * 64], KV = H): they are added,
+// rotated and appended to the cache here, where they are read next (k_gemv_finish_qkv as a launch of its own took 7 us of a
+// layer's 97 at 64 slots).
+struct AttnFinish { const float *sums; const float *cosb, *sinb; int nslice; };
+template <bool FIN>
+__global__ void __launch_bounds__(128) k_dec_attn(bf16_t *O, const bf16_t *Q, bf16_t *Kc, bf16_t *Vc, const int *pos,
+                                                  int win, int B, int Tm, int H, int KV, float scale, int *errword, const AttnFinish fin)
 {
     extern __shared__ float dec_sc[];                    // Tm scores
     __shared__ float red[4], part[4][64];
+    __shared__ __align__(16) bf16_t sq[64];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x, row = lane >> 3, c8 = (lane & 7) * 8;
     const int g = blockIdx.x;
     pdl_trigger();
@@ -521,7 +528,29 @@ __global__ void __launch_bounds__(128) k_dec_attn(bf16_t *O, const bf16_t *Q, co
     float *sc = dec_sc;
     const int lo = (win > 0 && t >= win) ? t - win + 1 : 0;
     float q[8];
-    bf8_to_f(*reinterpret_cast<const uint4 *>(Q + (size_t)b * D + h * 64 + c8), q);
+    if (FIN) {
+        if (tid < 96) {                                  // pairs (i, i + 32) of q (m = 0), k and v
+            const int m = tid >> 5, i = tid & 31;
+            const size_t RN = (size_t)3 * B * D;
+            const float *sp = fin.sums + ((size_t)m * B + b) * D + h * 64 + i;
+            float x = 0.0f, y = 0.0f, cs = 1.0f, sn = 0.0f;
+            if (m < 2) { cs = fin.cosb[(size_t)t * 32 + i]; sn = fin.sinb[(size_t)t * 32 + i]; }
+#pragma unroll 4
+            for (int k = 0; k < fin.nslice; k++) { x += sp[(size_t)k * RN]; y += sp[(size_t)k * RN + 32]; }
+            x = __bfloat162float(__float2bfloat16_rn(x)); y = __bfloat162float(__float2bfloat16_rn(y));
+            if (m < 2) { const float xr = x * cs - y * sn, yr = y * cs + x * sn; x = xr; y = yr; }
+            const bf16_t xo = __float2bfloat16_rn(x), yo = __float2bfloat16_rn(y);
+            if (m == 0) { sq[i] = xo; sq[i + 32] = yo; }
+            else {
+                bf16_t *c = (m == 1 ? Kc : Vc) + ((size_t)b * Tm + t) * KD + h * 64 + i;
+                c[0] = xo; c[32] = yo;
+            }
+        }
+        __syncthreads();                                 // the block reads its own key and value back below
+        bf8_to_f(*reinterpret_cast<const uint4 *>(sq + c8), q);
+    } else {
+        bf8_to_f(*reinterpret_cast<const uint4 *>(Q + (size_t)b * D + h * 64 + c8), q);
+    }
     const size_t base = (size_t)b * Tm * KD + kvh * 64 + c8;
     const bf16_t *kb = Kc + base, *vb = Vc + base;
     float mx = -1e30f;
@@ -955,26 +984,45 @@ extern "C" int qlmb_dec_kv(void *Kc, void *Vc, const void *k, const void *v, con
     return QLMB_OK;
 }
 
-extern "C" int qlmb_dec_attn(void *O, const void *Q, const void *Kc, const void *Vc, const int *pos, int win, int B, int Tm,
-                             int H, int KV, int hd, void *stream)
+static int dec_attn_launch(void *O, const void *Q, void *Kc, void *Vc, const int *pos, int win, int B, int Tm, int H, int KV,
+                           const AttnFinish *fin, cudaStream_t st)
 {
-    QLMB_REQUIRE(O && Q && Kc && Vc && pos, "qlmb_dec_attn: NULL argument");
-    QLMB_REQUIRE(hd == 64 && H > 0 && KV > 0 && H % KV == 0 && Tm > 0 && Tm <= DEC_TM_MAX, "qlmb_dec_attn: hd %d H %d KV %d Tm %d", hd, H, KV, Tm);
-    if (B <= 0) return QLMB_OK;
-    const size_t smem = (size_t)Tm * sizeof(float);
     // the attribute belongs to a device's copy of the kernel: set it once per device of this process
     static bool configured_dev[64];
     int dev_ = 0;
     QLMB_CUDA(cudaGetDevice(&dev_));
     QLMB_REQUIRE(dev_ >= 0 && dev_ < 64, "device index %d", dev_);
     if (!configured_dev[dev_]) {
-        QLMB_CUDA(cudaFuncSetAttribute(k_dec_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_TM_MAX * (int)sizeof(float)));
+        QLMB_CUDA(cudaFuncSetAttribute(k_dec_attn<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_TM_MAX * (int)sizeof(float)));
+        QLMB_CUDA(cudaFuncSetAttribute(k_dec_attn<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_TM_MAX * (int)sizeof(float)));
         configured_dev[dev_] = true;
     }
-    QLMB_CUDA(pdl_launch(B > 4, k_dec_attn, dim3((unsigned)(B * H)), dim3(128), smem, as_stream(stream), (bf16_t *)O, (const bf16_t *)Q,
-                         (const bf16_t *)Kc, (const bf16_t *)Vc, pos, win, B, Tm, H, KV, 1.0f / sqrtf((float)hd), device_error_word()));
+    const AttnFinish none = {};
+    QLMB_CUDA(pdl_launch(B > 4, fin ? k_dec_attn<true> : k_dec_attn<false>, dim3((unsigned)(B * H)), dim3(128), (size_t)Tm * sizeof(float), st, (bf16_t *)O,
+                         (const bf16_t *)Q, (bf16_t *)Kc, (bf16_t *)Vc, pos, win, B, Tm, H, KV, 0.125f, device_error_word(), fin ? *fin : none));
     QLMB_LAUNCH_CHECK("k_dec_attn");
     return QLMB_OK;
+}
+
+extern "C" int qlmb_dec_attn(void *O, const void *Q, const void *Kc, const void *Vc, const int *pos, int win, int B, int Tm,
+                             int H, int KV, int hd, void *stream)
+{
+    QLMB_REQUIRE(O && Q && Kc && Vc && pos, "qlmb_dec_attn: NULL argument");
+    QLMB_REQUIRE(hd == 64 && H > 0 && KV > 0 && H % KV == 0 && Tm > 0 && Tm <= DEC_TM_MAX, "qlmb_dec_attn: hd %d H %d KV %d Tm %d", hd, H, KV, Tm);
+    if (B <= 0) return QLMB_OK;
+    return dec_attn_launch(O, Q, const_cast<void *>(Kc), const_cast<void *>(Vc), pos, win, B, Tm, H, KV, nullptr, as_stream(stream));
+}
+
+extern "C" int qlmb_dec_qkv_attn(void *O, void *Kc, void *Vc, const void *X, const float *gamma, const int8_t *codes, const float *scales,
+                                 const float *cosb, const float *sinb, const int *pos, int B, int D, int Tm, void *stream)
+{
+    QLMB_REQUIRE(O && Kc && Vc && X && gamma && codes && scales && cosb && sinb && pos, "qlmb_dec_qkv_attn: NULL argument");
+    QLMB_REQUIRE(B > 4 && B <= 64 && D > 0 && D % 128 == 0 && Tm > 0 && Tm <= DEC_TM_MAX, "qlmb_dec_qkv_attn: B %d D %d Tm %d", B, D, Tm);
+    cudaStream_t st = as_stream(stream);
+    AttnFinish fin = {};
+    fin.cosb = cosb; fin.sinb = sinb;
+    const int rc = gemv_stack_slices(&fin.sums, &fin.nslice, X, gamma, codes, scales, 3, B, D, D, 0, st);
+    return rc ? rc : dec_attn_launch(O, nullptr, Kc, Vc, pos, 0, B, Tm, D / 64, D / 64, &fin, st);
 }
 
 extern "C" int qlmb_dec_greedy(int *out, float *lp, const float *logits, int B, int V, void *stream)

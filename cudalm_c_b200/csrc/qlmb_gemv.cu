@@ -1163,6 +1163,41 @@ __global__ void __launch_bounds__(256) k_gemv_finish_combine(bf16 *out, const bf
     out[i] = __float2bfloat16_rn(acc);
 }
 
+struct ExpertPlan { MmaPlan pl1, pl2; size_t pg_n, pd_n; };
+static ExpertPlan expert_plan(const qlmb_moe_layer *L)
+{
+    const int D = L->D, F = L->F, R = L->K * L->N;
+    // the groups that will hold rows, about: the experts that R random choices hit (the others' blocks return at once)
+    const int hit = (int)ceil(L->E * (1.0 - pow(1.0 - 1.0 / L->E, R)));
+    ExpertPlan p = {mma_plan(D, F, 2 * hit, 1), mma_plan(F, D, hit, 1), 0, 0};
+    p.pg_n = (size_t)p.pl1.ns * 2 * R * F; p.pd_n = (size_t)p.pl2.ns * R * D;
+    return p;
+}
+size_t moe_decode_workspace(const qlmb_moe_layer *L)
+{
+    const size_t R = (size_t)L->K * L->N, act = R * L->F * sizeof(bf16) + 256;
+    if (R > 16) { const ExpertPlan p = expert_plan(L); return (p.pg_n + p.pd_n) * sizeof(float) + act; }
+    // (the slices of sixteen rows or fewer: at most one per 128 contraction rows)
+    return ((size_t)2 * (L->D / 128) * R * L->F + (size_t)(L->F / 128) * R * L->D) * sizeof(float) + act;
+}
+
+int gemv_stack_slices(const float **part, int *nslice, const void *X, const float *gamma, const int8_t *codes, const float *scales,
+                      int nmat, int B, int K, int N, size_t min_bytes, cudaStream_t st)
+{
+    const int R = nmat * B, mt = mma_mt(B, K, N, nmat), nz = nmat * ((B + 16 * mt - 1) / (16 * mt));
+    const MmaPlan pl = mma_plan(K, N, nz, mt);
+    const size_t need = (size_t)pl.ns * R * N * sizeof(float);
+    void *ws = nullptr;
+    int rc = workspace(need > min_bytes ? need : min_bytes, &ws);
+    if (rc) return rc;
+    Rows8 a = {};
+    a.part = (float *)ws; a.X = X; a.x_dtype = QLMB_BF16; a.K = K; a.N = N;
+    a.codes = (const uint8_t *)codes; a.scales = scales; a.e_codes = (size_t)K * N / 2; a.e_scales = (size_t)K * N / 128;
+    a.B = B; a.nmat = nmat; a.rows_out = R; a.gamma = gamma;
+    *part = a.part; *nslice = pl.ns;
+    return mma_launch(a, nz, pl, mt, st);
+}
+
 // Experts of a decode step with at most 128 routed rows: three routed GEMVs that read only the chosen experts'
 // codes (W1, W3: [E][D][F]; W2: [E][F][D]), SwiGLU and the gate-weighted combination in the slice-sum kernels.
 int moe_decode_experts(const qlmb_moe_layer *L, void *out, const void *f_in, const void *f_norm, const int *assign,
@@ -1175,11 +1210,10 @@ int moe_decode_experts(const qlmb_moe_layer *L, void *out, const void *f_in, con
         int rc = perm_ready ? 0 : perm_build(assign, N, L->E, K, 1, 1, perm, nullptr, off, counts, bad, nullptr, nullptr, nullptr, st);
         if (rc) return rc;
         const int zmax = L->E + R / 16;                  // sum over the experts of ceil(count / 16) never exceeds this
-        // the groups that will hold rows, about: the experts that R random choices hit (the others' blocks return at once)
-        const int hit = (int)ceil(L->E * (1.0 - pow(1.0 - 1.0 / L->E, R)));
-        const MmaPlan pl1 = mma_plan(D, F, 2 * hit, 1), pl2 = mma_plan(F, D, hit, 1);
+        const ExpertPlan ep = expert_plan(L);
+        const MmaPlan &pl1 = ep.pl1, &pl2 = ep.pl2;
         const int ns1 = pl1.ns, ns2 = pl2.ns;
-        const size_t pg_n = (size_t)ns1 * 2 * R * F, pd_n = (size_t)ns2 * R * D;
+        const size_t pg_n = ep.pg_n, pd_n = ep.pd_n;
         void *ws = nullptr;
         if ((rc = workspace((pg_n + pd_n) * sizeof(float) + (size_t)R * F * sizeof(bf16) + 256, &ws))) return rc;
         float *pg = (float *)ws, *pd = pg + pg_n;

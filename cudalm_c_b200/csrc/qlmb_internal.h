@@ -74,13 +74,20 @@ int router_logits_small(float *rt, const void *X, int x_dtype, const float *Wr, 
 // the same logits and the selection in one launch (qlmb_route.cu); larger shapes fall back to the two kernels
 // perm / off / counts / bad (optional): with at most 256 routed slots the same launch groups the slots by expert;
 // *perm_done tells the caller whether it did
+// the output projection's slice sums [nslice][N][D], residual and norm that k_router_small can take on the way
+struct RouterFinish { const float *part; const bf16 *res; const float *gamma; bf16 *F, *Fn; int nslice; };
 int router_small(float *rt, const void *X, int x_dtype, const float *Wr, float *rprobs, int *assign, float *gate, int N, int D,
                  int E, int K, const float *bias, int bs, cudaStream_t st, int *perm = nullptr, int *off = nullptr,
-                 int *counts = nullptr, int *bad = nullptr, int *perm_done = nullptr);
+                 int *counts = nullptr, int *bad = nullptr, int *perm_done = nullptr,
+                 const RouterFinish *fin = nullptr);
 // experts of a decode step with at most 64 routed rows (qlmb_gemv.cu): routed GEMVs over the chosen experts' codes
 // perm / off / counts / bad: scratch of the permutation (K*N, E + 1, E and 1 ints) for steps with more than 16 routed rows
 int moe_decode_experts(const qlmb_moe_layer *L, void *out, const void *f_in, const void *f_norm, const int *assign,
                        const float *gate, cudaStream_t st, int *perm = nullptr, int *off = nullptr, int *counts = nullptr,
                        int *bad = nullptr, int perm_ready = 0);
+size_t moe_decode_workspace(const qlmb_moe_layer *L);    // bytes it asks the shared workspace for
+// the K-slice sums of nmat stacked matrices' GEMV (5 to 64 bf16 rows) in the shared workspace, at least `min_bytes` of it
+int gemv_stack_slices(const float **part, int *nslice, const void *X, const float *gamma, const int8_t *codes, const float *scales,
+                      int nmat, int B, int K, int N, size_t min_bytes, cudaStream_t st);
 
 }  // namespace qlmb

@@ -259,6 +259,34 @@ extern "C" int qlmb_moe_decode(const qlmb_moe_layer *L, void *arena, void *out, 
     return moe_decode_experts(L, out, f_in, f_norm, a.assign, a.gate, st, a.perm, a.off, a.counts, a.bad, grouped);
 }
 
+// The output projection, residual and norm in front of it as well (dec_step, cudalm.cu:7188-7199): f_in = att deq(Wo) + res,
+// f_norm = its norm, out = qlmb_moe_decode(f_in, f_norm).  Five to 64 slots whose routed rows the grouped GEMVs take have the
+// projection's slice sums added by the router's launch.
+extern "C" int qlmb_dec_wo_moe(const qlmb_moe_layer *L, void *arena, void *out, void *f_in, void *f_norm, const void *att,
+                               const int8_t *wo_codes, const float *wo_scales, const void *res, const float *gamma, void *stream)
+{
+    int rc = check_layer("qlmb_dec_wo_moe", L);
+    if (rc) return rc;
+    QLMB_REQUIRE(arena && out && f_in && f_norm && att && wo_codes && wo_scales && res && gamma, "qlmb_dec_wo_moe: NULL argument");
+    const int N = L->N, D = L->D, E = L->E, K = L->K;
+    if (N <= 4 || N > 64 || K * N > 128 || L->dtype != QLMB_BF16 || E > 32 || D > 2048) {
+        if ((rc = qlmb_gemv_decode_res_norm(f_in, f_norm, att, wo_codes, wo_scales, res, gamma, N, D, D, stream))) return rc;
+        return qlmb_moe_decode(L, arena, out, f_in, f_norm, stream);
+    }
+    QLMB_REQUIRE(((uintptr_t)arena & 255) == 0, "qlmb_dec_wo_moe: arena must be 256-byte aligned");
+    Arena a = carve(arena, N, D, L->F, E, K);
+    cudaStream_t st = as_stream(stream);
+    // the slice sums are read behind the experts' request for the same piece: it must not be replaced by a larger one between
+    RouterFinish fin = {};
+    if ((rc = gemv_stack_slices(&fin.part, &fin.nslice, att, nullptr, wo_codes, wo_scales, 1, N, D, D, moe_decode_workspace(L), st))) return rc;
+    fin.res = (const bf16 *)res; fin.gamma = gamma; fin.F = (bf16 *)f_in; fin.Fn = (bf16 *)f_norm;
+    int grouped = 0;
+    const bool want = K * N > 16;
+    if ((rc = router_small(a.rt, nullptr, L->dtype, L->wr, a.rprobs, a.assign, a.gate, N, D, E, K, L->bias, L->bias_stride, st,
+                           want ? a.perm : nullptr, a.off, a.counts, a.bad, want ? &grouped : nullptr, &fin))) return rc;
+    return moe_decode_experts(L, out, f_in, f_norm, a.assign, a.gate, st, a.perm, a.off, a.counts, a.bad, grouped);
+}
+
 extern "C" int qlmb_moe_backward(const qlmb_moe_layer *L, void *arena, void *dfnorm, const void *dout,
                                  const void *f_norm, float *dW1, float *dW3, float *dW2, float *dWr,
                                  float beta, void *stream)

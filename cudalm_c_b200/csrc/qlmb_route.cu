@@ -90,9 +90,14 @@ __global__ void __launch_bounds__(256) k_router_topk_warp(const float *rt, float
 // off[0..E], counts[0..E), *bad = an expert id out of range.  The blocks take tickets after a fence, so the last one sees
 // every block's choices; the result does not depend on which block that is.
 __device__ unsigned g_router_ticket;
+// FIN: the rows come as the K slices of the output projection's GEMV: F = bf16(their sum) + residual (rounded to bf16 as the
+// separate kernels do) and Fn = F * rinv * gamma are made and stored on the way (k_gemv_finish_res_norm as a launch of its own took
+// 7 us of a layer's 97 at 64 slots).
+template <bool FIN>
 __global__ void __launch_bounds__(256) k_router_small(float *rt, const void *X, int x_dtype, const float *Wr, float *rprobs,
                                                       int *assign, float *gate, int N, int D, int E, int K,
-                                                      const float *bias, int bs, int *perm, int *off, int *counts, int *bad, int quiet)
+                                                      const float *bias, int bs, int *perm, int *off, int *counts, int *bad, int quiet,
+                                                      const RouterFinish fin)
 {
     extern __shared__ float rs_x[];                      // D activations
     __shared__ float part[8][32];
@@ -111,8 +116,54 @@ __global__ void __launch_bounds__(256) k_router_small(float *rt, const void *X, 
 #pragma unroll
     for (int u = 0; u < UB; u++) w[u] = ld_cg(Wr + (size_t)(j0 + u < jl ? j0 + u : jl) * E + ec);
     if (quiet == QUIET) pdl_wait();                               // the row below is the work of the kernels before
-    for (int j = threadIdx.x; j < D; j += 256)
-        rs_x[j] = x_dtype == QLMB_BF16 ? __bfloat162float(((const bf16 *)X)[(size_t)n * D + j]) : ((const float *)X)[(size_t)n * D + j];
+    if (FIN) {
+        __shared__ float red[8];
+        float v[8], rsd[8], gm[8], ss = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 8; c++) {                    // residual and gain are requested together with the slices
+            const int j = threadIdx.x + 256 * c;
+            v[c] = 0.0f; rsd[c] = 0.0f; gm[c] = 0.0f;
+            if (j < D) { rsd[c] = __bfloat162float(fin.res[(size_t)n * D + j]); gm[c] = fin.gamma[j]; }
+        }
+#pragma unroll 4
+        for (int k = 0; k < fin.nslice; k++) {           // slice order ascending per column, four slices' loads in flight
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                const int j = threadIdx.x + 256 * c;
+                if (j < D) v[c] += fin.part[((size_t)k * N + n) * D + j];
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            const int j = threadIdx.x + 256 * c;
+            if (j < D) {
+                const bf16 f = __float2bfloat16_rn(__bfloat162float(__float2bfloat16_rn(v[c])) + rsd[c]);
+                fin.F[(size_t)n * D + j] = f;
+                v[c] = __bfloat162float(f);
+                ss = __fmaf_rn(v[c], v[c], ss);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (e == 0) red[warp] = ss;
+        __syncthreads();
+        float tot = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; w++) tot += red[w];
+        const float rinv = 1.0f / sqrtf(tot / (float)D + 1e-5f);
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            const int j = threadIdx.x + 256 * c;
+            if (j < D) {
+                const bf16 y = __float2bfloat16_rn(v[c] * rinv * gm[c]);
+                fin.Fn[(size_t)n * D + j] = y;
+                rs_x[j] = __bfloat162float(y);
+            }
+        }
+    } else {
+        for (int j = threadIdx.x; j < D; j += 256)
+            rs_x[j] = x_dtype == QLMB_BF16 ? __bfloat162float(((const bf16 *)X)[(size_t)n * D + j]) : ((const float *)X)[(size_t)n * D + j];
+    }
     __syncthreads();
     float acc = 0.0f;
     for (int j = j0; j < j1; j += UB) {
@@ -420,8 +471,10 @@ int router_topk(const float *rt, float *rprobs, int *assign, float *gate, int N,
 }
 
 int router_small(float *rt, const void *X, int x_dtype, const float *Wr, float *rprobs, int *assign, float *gate, int N, int D,
-                 int E, int K, const float *bias, int bs, cudaStream_t st, int *perm, int *off, int *counts, int *bad, int *perm_done)
+                 int E, int K, const float *bias, int bs, cudaStream_t st, int *perm, int *off, int *counts, int *bad, int *perm_done,
+                 const RouterFinish *fin)
 {
+    QLMB_REQUIRE(!fin || (N <= 64 && E <= 32 && D <= 2048), "router_small: N=%d E=%d D=%d with slice sums", N, E, D);
     if (perm_done) *perm_done = 0;
     if (N > 64 || E > 32 || D > 8192) {
         int rc = router_logits_small(rt, X, x_dtype, Wr, N, D, E, st);
@@ -429,8 +482,9 @@ int router_small(float *rt, const void *X, int x_dtype, const float *Wr, float *
     }
     const bool fuse = perm && off && perm_done && K * N <= 256;      // the last block also groups the slots by expert
     if (fuse) *perm_done = 1;
-    QLMB_CUDA(pdl_launch(N > 4, k_router_small, dim3(N), dim3(256), (size_t)D * sizeof(float), st, rt, X, x_dtype, Wr, rprobs, assign, gate, N, D, E, K, bias, bs,
-                         fuse ? perm : (int *)nullptr, off, counts, bad, weights_quiet(st)));
+    const RouterFinish none = {};
+    QLMB_CUDA(pdl_launch(N > 4, fin ? k_router_small<true> : k_router_small<false>, dim3(N), dim3(256), (size_t)D * sizeof(float), st, rt, X, x_dtype, Wr, rprobs, assign,
+                         gate, N, D, E, K, bias, bs, fuse ? perm : (int *)nullptr, off, counts, bad, weights_quiet(st), fin ? *fin : none));
     QLMB_LAUNCH_CHECK("k_router_small");
     return QLMB_OK;
 }

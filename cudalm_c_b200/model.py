@@ -496,7 +496,14 @@ class Decoder:
         x = block.embed(m.emb, self.tok, dtype=torch.bfloat16)
         for l, ly in enumerate(m.layers):
             w, f = ly["w"], m.fl[l]
-            if c.KD == c.D and 3 * B <= 256:
+            att = torch.empty(B, c.D, dtype=torch.bfloat16, device=m.dev)
+            if c.KD == c.D and 4 < B <= 64:
+                # wq, wk, wv are consecutive spans of one shape: one GEMV launch for the three with the norm in front of them
+                # applied while the row is staged; the attention adds its head's slice sums, rotates and appends them
+                check(L_.qlmb_dec_qkv_attn(ptr(att), ptr(self.K[l]), ptr(self.V[l]), ptr(x), ptr(f["an1"]), ptr(w["wq"][0]), ptr(w["wq"][1]),
+                                           ptr(self.cosb), ptr(self.sinb), ptr(self.pos), B, c.D, self.Tm, stream_ptr()))
+                qh = None
+            elif c.KD == c.D and 3 * B <= 256:
                 # wq, wk, wv are consecutive spans of one shape: one GEMV launch pair for the three; the norm in front of
                 # them is applied while the row is staged, the finish rotates q and k and appends k, v to the caches
                 qkv = torch.empty(3 * B, c.D, dtype=torch.bfloat16, device=m.dev)
@@ -511,9 +518,17 @@ class Decoder:
                 check(L_.qlmb_dec_rope(ptr(qh), 1, ptr(self.cosb), ptr(self.sinb), ptr(self.pos), B, c.H, c.hd, self.Tm, stream_ptr()))
                 check(L_.qlmb_dec_rope(ptr(kh), 1, ptr(self.cosb), ptr(self.sinb), ptr(self.pos), B, c.KV, c.hd, self.Tm, stream_ptr()))
                 check(L_.qlmb_dec_kv(ptr(self.K[l]), ptr(self.V[l]), ptr(kh), ptr(vh), ptr(self.pos), B, self.Tm, c.KD, stream_ptr()))
-            att = torch.empty(B, c.D, dtype=torch.bfloat16, device=m.dev)
-            check(L_.qlmb_dec_attn(ptr(att), ptr(qh), ptr(self.K[l]), ptr(self.V[l]), ptr(self.pos), 0, B, self.Tm, c.H, c.KV,
-                                   c.hd, stream_ptr()))
+            if qh is not None:
+                check(L_.qlmb_dec_attn(ptr(att), ptr(qh), ptr(self.K[l]), ptr(self.V[l]), ptr(self.pos), 0, B, self.Tm, c.H, c.KV,
+                                       c.hd, stream_ptr()))
+            if 4 < B <= 64 and c.D <= 2048:
+                # wo; its slice sums, the residual add and the FFN's input norm in the router's launch; the experts
+                f_in, f_norm, out = (torch.empty(B, c.D, dtype=torch.bfloat16, device=m.dev) for _ in range(3))
+                mo = self.moes[l]
+                check(L_.qlmb_dec_wo_moe(mo.c, mo.arena_ptr, ptr(out), ptr(f_in), ptr(f_norm), ptr(att), ptr(w["wo"][0]), ptr(w["wo"][1]),
+                                         ptr(x), ptr(f["an2"]), stream_ptr()))
+                x = out
+                continue
             if B <= 256 and c.D <= 2048:
                 # wo, the residual add and the FFN's input norm: one GEMV launch pair
                 f_in = torch.empty(B, c.D, dtype=torch.bfloat16, device=m.dev)

@@ -621,6 +621,15 @@ int qlmb_dec_qkv(void *Y, void *Kc, void *Vc, const void *X, const float *gamma,
 int qlmb_gemv_decode_res_norm(void *F, void *Fn, const void *X, const int8_t *codes, const float *scales, const void *res,
                               const float *gamma, int B, int K, int N, void *stream);
 
+/* qlmb_dec_qkv and qlmb_dec_attn (no window, heads of 64) of five to 64 slots in one launch pair: the attention's blocks add the
+ * projections' slice sums of their head, rotate and append them.  O [B][D]; the caches as in qlmb_dec_qkv. */
+int qlmb_dec_qkv_attn(void *O, void *Kc, void *Vc, const void *X, const float *gamma, const int8_t *codes, const float *scales,
+                      const float *cosb, const float *sinb, const int *pos, int B, int D, int Tm, void *stream);
+/* qlmb_gemv_decode_res_norm (K = N = D) and qlmb_moe_decode of L->N slots: f_in = att deq(Wo) + res, f_norm = its norm with
+ * gamma, out = the layer's output; all of them bf16 [N][D]. */
+int qlmb_dec_wo_moe(const qlmb_moe_layer *L, void *arena, void *out, void *f_in, void *f_norm, const void *att,
+                    const int8_t *wo_codes, const float *wo_scales, const void *res, const float *gamma, void *stream);
+
 /* ---- decoder: one new token per live slot (dec_step, cudalm.cu:7166-7212) ----
  * The K/V cache of a layer is bf16 [B, Tm, KV*hd]; pos[b] (device) is the position of slot b's new token.
  * k_dec_rope (cudalm.cu:7023-7027): rotate the single row of each slot by the angle of pos[b]; the tables have Tm rows,

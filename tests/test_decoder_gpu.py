@@ -378,3 +378,69 @@ def test_one_launch_step_equals_the_chain(cuda, B, D, KV, E, K, F, fill, Tm):
     for t, c, b in zip(d.K + d.V, caches, before):
         assert float((t.float() - c.float()).abs().max()) < 2e-2
         assert ((t != b).flatten(2).any(-1).sum(1) <= 1).all()              # at most the slot's own row changed
+
+
+@pytest.mark.parametrize("B,D,Tm", [(5, 128, 40), (16, 768, 300), (17, 256, 64), (33, 512, 100), (64, 768, 1024)])
+def test_decode_attention_on_the_projections_slice_sums(cuda, B, D, Tm):
+    """q, k, v, rotation, append and attention in two launches: the same bits, in output and caches, as the separate entries; a
+    slot past its cache is reported and left alone."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import block, qlm
+    from cudalm_c_b200._lib import ptr, stream_ptr
+    g = torch.Generator(device=cuda); g.manual_seed(B)
+    Q = qlm.Qlm([(0, 3 * D * D)], 3 * D * D, cuda)
+    Q.init_from(torch.randn(3 * D * D, device=cuda, generator=g) * 0.02, render=False)
+    x = torch.randn(B, D, device=cuda, generator=g).bfloat16()
+    gamma = torch.rand(D, device=cuda, generator=g) + 0.5
+    cosb, sinb = block.rope_tables(Tm, 64, device=cuda)
+    pos = torch.randint(0, Tm, (B,), device=cuda, generator=g, dtype=torch.int32)
+    pos[0], pos[1] = 0, Tm - 1
+    for past in (False, True):
+        if past:
+            pos[2] = Tm
+        c1 = [torch.randn(B, Tm, D, device=cuda, generator=g).bfloat16() for _ in range(2)]
+        c2 = [t.clone() for t in c1]
+        o1, o2 = (torch.full((B, D), 3.0, device=cuda).bfloat16() for _ in range(2))
+        y = torch.empty(3 * B, D, dtype=torch.bfloat16, device=cuda)
+        q.check(q.lib().qlmb_dec_qkv(ptr(y), ptr(c1[0]), ptr(c1[1]), ptr(x), ptr(gamma), ptr(Q.d), ptr(Q.s), ptr(cosb), ptr(sinb),
+                                     ptr(pos), B, D, 64, Tm, stream_ptr()))
+        q.check(q.lib().qlmb_dec_attn(ptr(o1), ptr(y), ptr(c1[0]), ptr(c1[1]), ptr(pos), 0, B, Tm, D // 64, D // 64, 64, stream_ptr()))
+        if past:
+            assert q.lib().qlmb_check_device(None) == 4
+        q.check(q.lib().qlmb_dec_qkv_attn(ptr(o2), ptr(c2[0]), ptr(c2[1]), ptr(x), ptr(gamma), ptr(Q.d), ptr(Q.s), ptr(cosb),
+                                          ptr(sinb), ptr(pos), B, D, Tm, stream_ptr()))
+        torch.cuda.synchronize()
+        if past:
+            assert q.lib().qlmb_check_device(None) == 4 and b"error code 201" in q.lib().qlmb_last_error()
+        assert torch.equal(o1, o2) and all(torch.equal(a, b) for a, b in zip(c1, c2))
+    q.check(q.lib().qlmb_check_device(None))
+
+
+@pytest.mark.parametrize("N,D,F,E,K", [(5, 256, 256, 8, 2), (9, 128, 384, 4, 1), (33, 768, 512, 32, 2), (64, 768, 1536, 32, 2),
+                                       (64, 256, 256, 16, 2), (64, 256, 256, 8, 4)])
+def test_output_projection_and_experts_in_one_call(cuda, N, D, F, E, K):
+    """wo, residual, norm and the expert layer: the same bits as the two entries, with the slice sums added in the router's launch
+    and (4 x 64 routed rows) without."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import moe, qlm
+    from cudalm_c_b200._lib import ptr, stream_ptr
+    g = torch.Generator(device=cuda); g.manual_seed(N + D)
+
+    def weights(n):
+        Q = qlm.Qlm([(0, n)], n, cuda)
+        Q.init_from(torch.randn(n, device=cuda, generator=g) * 0.02, render=False)
+        return Q.d, Q.s
+    wo, w1, w3, w2 = weights(D * D), weights(E * D * F), weights(E * D * F), weights(E * F * D)
+    wr = torch.randn(D, E, device=cuda, generator=g) * 0.1
+    layer = moe.MoeLayerState(N, D, F, E, K, w1, w3, w2, wr, aux=0.0)
+    att, res = (torch.randn(N, D, device=cuda, generator=g).bfloat16() for _ in range(2))
+    gamma = torch.rand(D, device=cuda, generator=g) + 0.5
+    a, b = ([torch.zeros(N, D, device=cuda).bfloat16() for _ in range(3)] for _ in range(2))
+    q.check(q.lib().qlmb_gemv_decode_res_norm(ptr(a[0]), ptr(a[1]), ptr(att), ptr(wo[0]), ptr(wo[1]), ptr(res), ptr(gamma), N, D, D,
+                                              stream_ptr()))
+    layer.decode(a[0], a[1], out=a[2])
+    q.check(q.lib().qlmb_dec_wo_moe(layer.c, layer.arena_ptr, ptr(b[2]), ptr(b[0]), ptr(b[1]), ptr(att), ptr(wo[0]), ptr(wo[1]),
+                                    ptr(res), ptr(gamma), stream_ptr()))
+    torch.cuda.synchronize()
+    assert float(a[2].float().norm()) > 0 and all(torch.equal(x, y) for x, y in zip(a, b))
+    q.check(q.lib().qlmb_check_device(None))
