@@ -20,6 +20,7 @@ struct Rows8 {
     const float *gamma;                                  // dense: rows are normalised on the way in (rinv * gamma, bf16)
     uint32_t k65536;
     int late;                                            // trigger behind the wait (weights_quiet: QUIET_FIRST)
+    int own;                                             // routed: blocks z < own hold expert z's first group
 };
 // ---- routing (qlmb_route.cu) ----
 int router_topk(const float *rt, float *rprobs, int *assign, float *gate, int N, int E, int K,

@@ -444,3 +444,50 @@ def test_output_projection_and_experts_in_one_call(cuda, N, D, F, E, K):
     torch.cuda.synchronize()
     assert float(a[2].float().norm()) > 0 and all(torch.equal(x, y) for x, y in zip(a, b))
     q.check(q.lib().qlmb_check_device(None))
+
+
+@pytest.mark.parametrize("counts", [[64] + [0] * 7, [16, 17, 0, 1, 15, 33, 46, 0], [8] * 16, [0] * 15 + [128]])
+def test_expert_rows_in_groups_of_sixteen(cuda, counts):
+    """Routings that fill an expert's first group of sixteen rows in part, fully, and several more, and leave experts without
+    rows: against float64 over the same choices."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import moe, qlm
+    E, K, D, F = len(counts), 2, 128, 256
+    N = sum(counts) // K
+    g = torch.Generator(device=cuda); g.manual_seed(E + counts[0])
+
+    def weights(n):
+        Q = qlm.Qlm([(0, n)], n, cuda)
+        P = torch.randn(n, device=cuda, generator=g) * 0.02
+        Q.init_from(P)
+        return (Q.d, Q.s), P.double()
+    (q1, p1), (q3, p3), (q2, p2) = weights(E * D * F), weights(E * D * F), weights(E * F * D)
+    # token n's choices: two different experts where the counts allow it, through router rows that carry them
+    slots = [e for e, c in enumerate(counts) for _ in range(c)]
+    pairs = [(slots[i], slots[i + N]) for i in range(N)]
+    x = torch.randn(N, D, device=cuda, generator=g) * 0.1
+    x[:, :2 * E] = 0.0
+    for n, (a, b) in enumerate(pairs):
+        x[n, a] += 4.0
+        x[n, E + b] += 3.0
+    x = x.bfloat16()
+    wr = torch.zeros(D, E, device=cuda)
+    wr[torch.arange(E), torch.arange(E)] = 4.0
+    wr[E + torch.arange(E), torch.arange(E)] = 4.0
+    layer = moe.MoeLayerState(N, D, F, E, K, q1, q3, q2, wr, aux=0.0)
+    res = torch.randn(N, D, device=cuda, generator=g).bfloat16()
+    out = layer.decode(res, x)
+    torch.cuda.synchronize()
+    q.check(q.lib().qlmb_check_device(None))
+    assign = layer.member("assign", (K, N), torch.int32).long()
+    gate = layer.member("gate", (K, N), torch.float32).double()
+    ref = res.double()
+    w1, w3, w2 = p1.view(E, D, F), p3.view(E, D, F), p2.view(E, F, D)
+    for k in range(K):
+        for n in range(N):
+            e = int(assign[k, n])
+            h = x[n].double()
+            gg = h @ w1[e]
+            ref[n] += gate[k, n] * ((gg * torch.sigmoid(gg) * (h @ w3[e])) @ w2[e])
+    # bf16 weights' scales, activations and results: 2^-9 each
+    assert float((out.double() - ref).norm() / (ref - res.double()).norm().clamp_min(1e-6)) < 2e-2 + 2 ** -8 * float(ref.norm() / (ref - res.double()).norm())
