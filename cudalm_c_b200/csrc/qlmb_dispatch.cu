@@ -512,89 +512,82 @@ int router_bwd(float *drt, const float *rprobs, const int *assign, const float *
 // --------------------------------------------------------------- unpermute
 // dfnorm[n,j] = sum_k dXp[inv[k,n], j] + sum_e drt[n,e] * Wr[j,e]
 // (reference k_scatter_add + g_abt_b(drt, Wr), cudalm.cu:4368-4390).
-// WrT is Wr transposed ([E][D], written by k_transpose_wr into scratch), so that a
-// feature slice of it is staged with 16-byte copies.
-__global__ void __launch_bounds__(256) k_transpose_wr(float *WrT, const float *Wr, int D, int E)
-{
-    int i = blockIdx.x * 256 + threadIdx.x;
-    if (i < D * E) { int j = i / E, e = i % E; WrT[(size_t)e * D + j] = Wr[i]; }
-}
-// Register-tiled: a block owns 256 features and walks over tiles of 32 tokens; warp = 4 tokens,
-// lane = features [4*lane, 4*lane+4) and [128+4*lane, ...) of the block's slice.  The slice of WrT
-// is staged in shared memory once per block, the tokens' drt rows and row indices per tile.
-// With PEER the permuted rows live in the arena of the rank that owns the slot's expert
-// (rows = that arena's row index per slot, read through the peer pointers).
-#define UPT_TOK 32
+// A block holds 256 features of Wr in shared memory, transposed as it is loaded; its warps then work on their own: four
+// tokens at a time, a lane eight features (4 * lane .. and 128 + 4 * lane ..).  The rows of a token's first two copies are
+// requested before the products and added behind them, the next tokens' row indices and gradients a round ahead, and nothing
+// is shared between warps.  (Whole blocks in step, the rows first, then the products, and a launch of its own for the
+// transposition: 31 + 2.5 us for 8192 tokens of 768, 32 experts; here 19.6, and 30.5 with three blocks per SM, whose 80 registers
+// spill.)
 #define UPT_F 256
-template <bool PEER>
-__global__ void __launch_bounds__(256, 3) k_unpermute_rows_tile(void *dfnorm, int dtype, const bf16 *dXp, PeerPtrs dXpP,
-                                                                const int *rows, const int *assign, int el, const float *drt,
-                                                                const float *WrT, int N, int D, int E, int K)
+__global__ void __launch_bounds__(256, 2) k_unpermute_rows_tile(void *dfnorm, int dtype, const bf16 *dXp, const int *rows,
+                                                                const float *drt, const float *Wr, int N, int D, int E, int K)
 {
     __shared__ __align__(16) float ws[32][UPT_F];
-    __shared__ __align__(16) float drs[UPT_TOK][32];
-    __shared__ int srow[UPT_TOK][8], sown[UPT_TOK][8];
+    __shared__ __align__(16) float drs[8][4][32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int j0 = blockIdx.y * UPT_F;
-    const int jA = j0 + lane * 4, jB = jA + 128;
-    for (int i = tid; i < 32 * (UPT_F / 4); i += 256) {
-        const int e = i / (UPT_F / 4), c = i % (UPT_F / 4), j = j0 + c * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (e < E && j < D) v = __ldg(reinterpret_cast<const float4 *>(WrT + (size_t)e * D + j));
-        *reinterpret_cast<float4 *>(&ws[e][c * 4]) = v;
-    }
-    const int ntiles = (N + UPT_TOK - 1) / UPT_TOK;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int n0 = tile * UPT_TOK;
-        __syncthreads();                                 // the previous tile's reads of drs / srow are done
-        for (int i = tid; i < UPT_TOK * K; i += 256) {
-            const int t = i / K, k = i % K, n = n0 + t;
-            int row = -1, own = 0;
-            if (n < N) {
-                const size_t slot = (size_t)k * N + n;
-                row = rows ? __ldg(rows + slot) : (int)slot;
-                if (PEER) own = __ldg(assign + slot) / el;
+    const int j0 = blockIdx.y * UPT_F, jA = j0 + lane * 4, jB = jA + 128;
+    const int groups = (N + 3) / 4, stride = gridDim.x * 8;
+    int g = blockIdx.x * 8 + warp;
+    // lane 8 t + k: row of token t's copy k (K <= 8); lane e: the four tokens' gradients of expert e's logit
+    auto index_of = [&](int grp) {
+        const int n = grp * 4 + (lane >> 3), k = lane & 7;
+        if (grp >= groups || n >= N || k >= K) return -1;
+        const size_t slot = (size_t)k * N + n;
+        return rows ? __ldg(rows + slot) : (int)slot;
+    };
+    auto grads_of = [&](int grp, float d[4]) {
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            const int n = grp * 4 + t;
+            d[t] = grp < groups && n < N && lane < E ? drt[(size_t)n * E + lane] : 0.0f;
+        }
+    };
+    int row = index_of(g);
+    float dn[4];
+    grads_of(g, dn);
+    {                                                    // thread = feature: its row of Wr
+        const int j = j0 + tid;
+        const float *w = Wr + (size_t)j * E;
+        if (j < D && (E & 3) == 0 && ((uintptr_t)Wr & 15) == 0) {
+            for (int e = 0; e < 32; e += 4) {
+                const float4 v = e < E ? __ldg(reinterpret_cast<const float4 *>(w + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                ws[e][tid] = v.x; ws[e + 1][tid] = v.y; ws[e + 2][tid] = v.z; ws[e + 3][tid] = v.w;
             }
-            srow[t][k] = row; sown[t][k] = own;
+        } else {
+            for (int e = 0; e < 32; e++) ws[e][tid] = j < D && e < E ? __ldg(w + e) : 0.0f;
         }
-        for (int i = tid; i < UPT_TOK * 32; i += 256) {
-            const int n = n0 + (i >> 5), e = i & 31;
-            drs[i >> 5][e] = (n < N && e < E) ? drt[(size_t)n * E + e] : 0.0f;
-        }
-        __syncthreads();
-        // the K permuted rows of the warp's 4 tokens: all loads of one k are in flight together
+    }
+    __syncthreads();
+    for (; g < groups; g += stride) {
+        uint2 qa[2][4], qb[2][4];
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const int rk = __shfl_sync(0xffffffffu, row, t * 8 + k);
+                qa[k][t] = qb[k][t] = make_uint2(0u, 0u);
+                if (rk >= 0) {
+                    const bf16 *src = dXp + (size_t)rk * D;
+                    if (jA < D) qa[k][t] = *reinterpret_cast<const uint2 *>(src + jA);
+                    if (jB < D) qb[k][t] = *reinterpret_cast<const uint2 *>(src + jB);
+                }
+            }
+        const int cur = row;
+        row = index_of(g + stride);
+#pragma unroll
+        for (int t = 0; t < 4; t++) drs[warp][t][lane] = dn[t];
+        __syncwarp();
+        grads_of(g + stride, dn);
         float acc[4][8];
 #pragma unroll
         for (int t = 0; t < 4; t++)
 #pragma unroll
             for (int i = 0; i < 8; i++) acc[t][i] = 0.0f;
-        for (int k = 0; k < K; k++) {
-            uint2 qa[4], qb[4];
-#pragma unroll
-            for (int t = 0; t < 4; t++) {
-                const int row = srow[warp * 4 + t][k];
-                qa[t] = qb[t] = make_uint2(0u, 0u);
-                if (row >= 0) {
-                    const bf16 *src = (PEER ? (const bf16 *)dXpP.p[sown[warp * 4 + t][k]] : dXp) + (size_t)row * D;
-                    if (jA < D) qa[t] = *reinterpret_cast<const uint2 *>(src + jA);
-                    if (jB < D) qb[t] = *reinterpret_cast<const uint2 *>(src + jB);
-                }
-            }
-#pragma unroll
-            for (int t = 0; t < 4; t++) {
-                float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&qa[t].x));
-                float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&qa[t].y));
-                acc[t][0] += a.x; acc[t][1] += a.y; acc[t][2] += b.x; acc[t][3] += b.y;
-                a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&qb[t].x));
-                b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&qb[t].y));
-                acc[t][4] += a.x; acc[t][5] += a.y; acc[t][6] += b.x; acc[t][7] += b.y;
-            }
-        }
 #pragma unroll 2
         for (int e4 = 0; e4 < 32; e4 += 4) {
             float4 dv[4];
 #pragma unroll
-            for (int t = 0; t < 4; t++) dv[t] = *reinterpret_cast<const float4 *>(&drs[warp * 4 + t][e4]);
+            for (int t = 0; t < 4; t++) dv[t] = *reinterpret_cast<const float4 *>(&drs[warp][t][e4]);
 #pragma unroll
             for (int k4 = 0; k4 < 4; k4++) {
                 const float4 wa = *reinterpret_cast<const float4 *>(&ws[e4 + k4][lane * 4]);
@@ -607,15 +600,38 @@ __global__ void __launch_bounds__(256, 3) k_unpermute_rows_tile(void *dfnorm, in
                 }
             }
         }
+        __syncwarp();                                    // before the next gradients are written
 #pragma unroll
         for (int t = 0; t < 4; t++) {
-            const int n = n0 + warp * 4 + t;
+            const int n = g * 4 + t;
+            float x[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) x[i] = 0.0f;
+            auto add = [&](const uint2 &u, const uint2 &v) {
+                const uint32_t w[4] = {u.x, u.y, v.x, v.y};
+#pragma unroll
+                for (int i = 0; i < 4; i++) { x[2 * i] += __uint_as_float(w[i] << 16); x[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u); }
+            };
+            add(qa[0][t], qb[0][t]);
+            if (K > 1) add(qa[1][t], qb[1][t]);
+            for (int k = 2; k < K; k++) {
+                const int rk = __shfl_sync(0xffffffffu, cur, t * 8 + k);
+                uint2 u = make_uint2(0u, 0u), v = u;
+                if (rk >= 0) {
+                    const bf16 *src = dXp + (size_t)rk * D;
+                    if (jA < D) u = *reinterpret_cast<const uint2 *>(src + jA);
+                    if (jB < D) v = *reinterpret_cast<const uint2 *>(src + jB);
+                }
+                add(u, v);
+            }
             if (n >= N) continue;
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int j = h ? jB : jA;
                 if (j >= D) continue;
-                const float *v = &acc[t][h * 4];
+                float v[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) v[i] = x[h * 4 + i] + acc[t][h * 4 + i];
                 if (dtype == QLMB_BF16) {
                     uint2 q;
                     *reinterpret_cast<__nv_bfloat162 *>(&q.x) = __floats2bfloat162_rn(v[0], v[1]);
@@ -630,12 +646,12 @@ __global__ void __launch_bounds__(256, 3) k_unpermute_rows_tile(void *dfnorm, in
 }
 static dim3 unpermute_grid(int N, int D)
 {
-    const int ny = (D + UPT_F - 1) / UPT_F, ntiles = (N + UPT_TOK - 1) / UPT_TOK;
-    int gx = 3 * sm_count() / ny;
+    const int ny = (D + UPT_F - 1) / UPT_F, groups = ((N + 3) / 4 + 7) / 8;
+    int gx = 2 * sm_count() / ny;
     if (gx < 1) gx = 1;
-    if (gx > ntiles) gx = ntiles;
-    const int per = (ntiles + gx - 1) / gx;              // whole tiles per block, evenly
-    gx = (ntiles + per - 1) / per;
+    if (gx > groups) gx = groups;
+    const int per = (groups + gx - 1) / gx;              // whole rounds per block, evenly
+    gx = (groups + per - 1) / per;
     return dim3(gx, ny);
 }
 
@@ -680,12 +696,10 @@ __global__ void __launch_bounds__(256) k_unpermute_rows(void *dfnorm, int dtype,
 }
 
 int unpermute_rows(void *dfnorm, int dtype, const bf16 *dXp, const int *inv, const float *drt, const float *Wr,
-                   float *wrt_scratch, int N, int D, int E, int K, cudaStream_t st)
+                   int N, int D, int E, int K, cudaStream_t st)
 {
-    if (E <= 32 && (D % 8) == 0 && wrt_scratch) {
-        k_transpose_wr<<<(D * E + 255) / 256, 256, 0, st>>>(wrt_scratch, Wr, D, E);
-        PeerPtrs none = {};
-        k_unpermute_rows_tile<false><<<unpermute_grid(N, D), 256, 0, st>>>(dfnorm, dtype, dXp, none, inv, nullptr, 1, drt, wrt_scratch, N, D, E, K);
+    if (E <= 32 && (D % 8) == 0 && K <= 8) {
+        k_unpermute_rows_tile<<<unpermute_grid(N, D), 256, 0, st>>>(dfnorm, dtype, dXp, inv, drt, Wr, N, D, E, K);
     } else {
         size_t smem = (size_t)UP_TOK * E * sizeof(float) + (size_t)UP_TOK * K * sizeof(int);
         k_unpermute_rows<<<(N + UP_TOK - 1) / UP_TOK, 256, smem, st>>>(dfnorm, dtype, dXp, inv, drt, Wr, N, D, E, K);

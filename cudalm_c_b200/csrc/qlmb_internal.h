@@ -50,7 +50,7 @@ int router_bwd(float *drt, const float *rprobs, const int *assign, const float *
                const int *counts, int N, int E, int K, float aux, cudaStream_t st);
 // dfnorm[n,:] = sum_k dXp[inv[k*N+n],:] + drt[n,:] * Wr^T
 int unpermute_rows(void *dfnorm, int dtype, const bf16 *dXp, const int *inv, const float *drt,
-                   const float *Wr, float *wrt_scratch /* D*E floats */, int N, int D, int E, int K,
+                   const float *Wr, int N, int D, int E, int K,
                    cudaStream_t st);
 // dWr[D,E] = beta*dWr + fnorm^T drt ; scratch holds 192*D*E floats
 int router_wgrad(float *dWr, const void *fnorm, int dtype, const float *drt, float *scratch, int N,

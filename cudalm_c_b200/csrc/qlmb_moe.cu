@@ -316,7 +316,7 @@ extern "C" int qlmb_moe_backward(const qlmb_moe_layer *L, void *arena, void *dfn
     if (rc) return rc;
 
     ProfScope ps("unpermute_rows", st);
-    return unpermute_rows(dfnorm, L->dtype, a.dXp, a.inv, a.drt, L->wr, a.wrt, N, D, E, K, st);
+    return unpermute_rows(dfnorm, L->dtype, a.dXp, a.inv, a.drt, L->wr, N, D, E, K, st);
 }
 
 // ===================================================================== expert parallelism
@@ -378,7 +378,7 @@ extern "C" int qlmb_moe_route_backward(const qlmb_moe_layer *L, void *arena, voi
     { ProfScope ps("router_bwd", st); if ((rc = router_bwd(a.drt, a.rprobs, a.assign, a.d_gate, a.counts, N, E, K, L->aux, st))) return rc; }
     cudaStream_t side = side_fork(st, 1);
     { ProfScope ps("router_wgrad", side); rc = router_wgrad(dWr, f_norm, L->dtype, a.drt, a.wr_scratch, N, D, E, beta, side); }
-    if (!rc) { ProfScope ps("unpermute_rows", st); rc = unpermute_rows(dfnorm, L->dtype, (const bf16 *)dXs, a.inv, a.drt, L->wr, a.wrt, N, D, E, K, st); }
+    if (!rc) { ProfScope ps("unpermute_rows", st); rc = unpermute_rows(dfnorm, L->dtype, (const bf16 *)dXs, a.inv, a.drt, L->wr, N, D, E, K, st); }
     side_join(side, st);
     return rc;
 }
@@ -567,7 +567,7 @@ extern "C" int qlmb_ep_route_backward(const qlmb_moe_layer *H, void *harena, con
     { ProfScope ps("router_wgrad", side); rc = router_wgrad(dWr, f_norm, H->dtype, h.drt, h.wr_scratch, N, D, E, beta, side); }
     // dXs is in slot order (k*N + n): no row index needed
     if (!rc) { ProfScope ps("unpermute_rows", st);
-               rc = unpermute_rows(dfnorm, H->dtype, (const bf16 *)dXs, nullptr, h.drt, H->wr, h.wrt, N, D, E, K, st); }
+               rc = unpermute_rows(dfnorm, H->dtype, (const bf16 *)dXs, nullptr, h.drt, H->wr, N, D, E, K, st); }
     side_join(side, st);
     return rc;
 }
