@@ -152,51 +152,6 @@ __global__ void __launch_bounds__(256) k_router_logits_tile(float *rt, const voi
     }
 }
 
-// Few tokens: eight per block, warp = token, lane = expert, the block's rows and the whole router matrix in shared memory
-// by one round of asynchronous copies.  The tiled kernel above walks the features in 24 chunks whose latency nothing
-// hides when its grid is a few blocks (333 tokens: 6 blocks, 19.6 us; here 42 blocks).  Every output is summed over the
-// features in ascending order with fused multiply-adds, as there: the same bits.
-#define RLF_TOK 8
-template <int XBF16>
-__global__ void __launch_bounds__(256) k_router_logits_few(float *rt, const void *X, const float *Wr, int N, int D, int E)
-{
-    extern __shared__ __align__(16) uint8_t rlf_sm[];
-    float *ws = reinterpret_cast<float *>(rlf_sm);       // [D][E]
-    uint8_t *xs = rlf_sm + (size_t)D * E * 4;            // [RLF_TOK][D]
-    pdl_wait();
-    pdl_trigger();
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n0 = blockIdx.x * RLF_TOK, n = n0 + warp;
-    const int xrow = D * (XBF16 ? 2 : 4);
-    const int tok = N - n0 < RLF_TOK ? N - n0 : RLF_TOK;
-    for (int i = tid * 16; i < tok * xrow; i += 256 * 16) cp_async16(xs + i, (const uint8_t *)X + (size_t)n0 * xrow + i, true);
-    for (int i = tid * 4; i < D * E; i += 256 * 4) cp_async16(ws + i, Wr + i, true);
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-    if (n >= N || lane >= E) return;
-    const uint8_t *row = xs + warp * xrow;
-    const float *w = ws + lane;
-    float acc = 0.0f;
-#pragma unroll 2
-    for (int j = 0; j < D; j += 8) {
-        float x[8], wv[8];
-        if (XBF16) {
-            const uint4 q = *reinterpret_cast<const uint4 *>(row + j * 2);
-            const uint32_t u[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-            for (int k = 0; k < 4; k++) { x[2 * k] = __uint_as_float(u[k] << 16); x[2 * k + 1] = __uint_as_float(u[k] & 0xffff0000u); }
-        } else {
-#pragma unroll
-            for (int k = 0; k < 8; k++) x[k] = reinterpret_cast<const float *>(row)[j + k];
-        }
-#pragma unroll
-        for (int k = 0; k < 8; k++) { wv[k] = *w; w += E; }
-#pragma unroll
-        for (int k = 0; k < 8; k++) acc = __fmaf_rn(x[k], wv[k], acc);
-    }
-    rt[(size_t)n * E + lane] = acc;
-}
-
 // General shape (E > 32 or Wr too large for shared memory): a block owns 32 tokens,
 // the token tile is staged 256 features at a time.
 #define RL_TOK 32
@@ -236,58 +191,9 @@ __global__ void __launch_bounds__(256) k_router_logits(float *rt, const void *X,
     }
 }
 
-// A handful of rows (a decode step): one block per token, lane = expert, eight warps each sum one eighth of the
-// features in ascending order (loads of Wr rows are independent of the running sums, so they pipeline), and the
-// eight partial sums are added in warp order.  Deterministic, but a different summation order than the tiled
-// kernel, hence only used where no backward pass reads the logits.
-__global__ void __launch_bounds__(256) k_router_logits_small(float *rt, const void *X, int x_dtype, const float *Wr, int D, int E)
-{
-    extern __shared__ float rl_x[];                      // D activations
-    __shared__ float part[8][32];
-    const int n = blockIdx.x, warp = threadIdx.x >> 5, e = threadIdx.x & 31;
-    for (int j = threadIdx.x; j < D; j += 256) rl_x[j] = ld_act(X, x_dtype, (size_t)n * D + j);
-    __syncthreads();
-    const int per = (D + 7) / 8, j0 = warp * per, j1 = j0 + per < D ? j0 + per : D;
-    float acc = 0.0f;
-    if (e < E) {
-#pragma unroll 8
-        for (int j = j0; j < j1; j++) acc += rl_x[j] * __ldg(Wr + (size_t)j * E + e);
-    }
-    part[warp][e] = acc;
-    __syncthreads();
-    if (warp == 0 && e < E) {
-        float s = part[0][e];
-#pragma unroll
-        for (int w = 1; w < 8; w++) s += part[w][e];
-        rt[(size_t)n * E + e] = s;
-    }
-}
-int router_logits_small(float *rt, const void *X, int x_dtype, const float *Wr, int N, int D, int E, cudaStream_t st)
-{
-    if (N > 64 || E > 32 || D > 8192) return router_logits(rt, X, x_dtype, Wr, N, D, E, st);
-    k_router_logits_small<<<N, 256, (size_t)D * sizeof(float), st>>>(rt, X, x_dtype, Wr, D, E);
-    QLMB_LAUNCH_CHECK("k_router_logits_small");
-    return QLMB_OK;
-}
-
 int router_logits(float *rt, const void *X, int x_dtype, const float *Wr, int N, int D, int E, cudaStream_t st)
 {
-    const size_t few_smem = (size_t)D * E * 4 + (size_t)RLF_TOK * D * (x_dtype == QLMB_BF16 ? 2 : 4);
-    if (E <= 32 && (D % 8) == 0 && (D * E) % 4 == 0 && (((uintptr_t)X | (uintptr_t)Wr) & 15) == 0 && few_smem <= 200 * 1024 && N <= (x_dtype == QLMB_BF16 ? 32 : 16) * sm_count()) {
-        // up to four rounds of blocks, two with fp32 rows (768 x 32: 2000 tokens 24.5 -> 19.1 us, 4736 25.3 -> 36.7): beyond that the tiled kernel's grid fills the device and it reads the matrix less often
-        static bool few_done[64];
-        int dev = 0;
-        QLMB_CUDA(cudaGetDevice(&dev));
-        QLMB_REQUIRE(dev >= 0 && dev < 64, "device index %d", dev);
-        if (!few_done[dev]) {
-            QLMB_CUDA(cudaFuncSetAttribute(k_router_logits_few<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            QLMB_CUDA(cudaFuncSetAttribute(k_router_logits_few<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            few_done[dev] = true;
-        }
-        const dim3 grid((N + RLF_TOK - 1) / RLF_TOK);
-        if (x_dtype == QLMB_BF16) QLMB_CUDA(pdl_launch_small(k_router_logits_few<1>, grid, dim3(256), few_smem, st, rt, X, Wr, N, D, E));
-        else QLMB_CUDA(pdl_launch_small(k_router_logits_few<0>, grid, dim3(256), few_smem, st, rt, X, Wr, N, D, E));
-    } else if (E <= 32 && (D % 8) == 0 && (((uintptr_t)X | (uintptr_t)Wr) & 15) == 0) {
+    if (E <= 32 && (D % 8) == 0 && (((uintptr_t)X | (uintptr_t)Wr) & 15) == 0) {
         int blocks = (N + RLT_TOK - 1) / RLT_TOK;
         if (x_dtype == QLMB_BF16) QLMB_CUDA(pdl_launch(false, k_router_logits_tile<1>, dim3(blocks), dim3(256), 0, st, rt, X, Wr, N, D, E));
         else QLMB_CUDA(pdl_launch(false, k_router_logits_tile<0>, dim3(blocks), dim3(256), 0, st, rt, X, Wr, N, D, E));
@@ -1120,9 +1026,7 @@ extern "C" int qlmb_router_topk(const float *rt_in, float *rt_out, const void *X
     if (!rt) {
         QLMB_REQUIRE(X && Wr && rt_out && D > 0, "qlmb_router_topk: logits need X, Wr and rt_out");
         QLMB_REQUIRE(x_dtype == QLMB_F32 || x_dtype == QLMB_BF16, "qlmb_router_topk: dtype %d", x_dtype);
-        int rc = router_logits(rt_out, X, x_dtype, Wr, N, D, E, as_stream(stream));
-        if (rc) return rc;
-        rt = rt_out;
+        return router_logits_topk(rt_out, X, x_dtype, Wr, rprobs, assign, gate, N, D, E, K, bias, bias_stride, as_stream(stream));
     }
     return router_topk(rt, rprobs, assign, gate, N, E, K, bias, bias_stride, as_stream(stream));
 }

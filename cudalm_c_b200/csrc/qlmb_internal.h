@@ -32,6 +32,9 @@ int perm_build(const int *assign, int N, int E, int K, int merged, int pad, int 
                int experts_per_rank = 0);
 
 // ---- row kernels (qlmb_dispatch.cu) ----
+// router_logits and router_topk; few tokens in one launch
+int router_logits_topk(float *rt, const void *X, int x_dtype, const float *Wr, float *rprobs, int *assign, float *gate, int N, int D,
+                       int E, int K, const float *bias, int bs, cudaStream_t st);
 int router_logits(float *rt, const void *X, int x_dtype, const float *Wr, int N, int D, int E,
                   cudaStream_t st);
 // Xp[j,:] = src[perm[j] % N,:] as bf16 (zero rows where perm[j] < 0); rows = *nrows_dev, or
@@ -71,7 +74,6 @@ int convert_f32_to_bf16(bf16 *dst, const float *src, size_t n, cudaStream_t st);
 struct GemmProblem;   // see qlmb_gemm.cuh
 
 // router logits of a few rows (decode): deterministic, not the tiled kernel's summation order
-int router_logits_small(float *rt, const void *X, int x_dtype, const float *Wr, int N, int D, int E, cudaStream_t st);
 // the same logits and the selection in one launch (qlmb_route.cu); larger shapes fall back to the two kernels
 // perm / off / counts / bad (optional): with at most 256 routed slots the same launch groups the slots by expert;
 // *perm_done tells the caller whether it did

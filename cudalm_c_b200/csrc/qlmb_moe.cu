@@ -195,7 +195,7 @@ extern "C" int qlmb_moe_forward_routed(const qlmb_moe_layer *L, void *arena, voi
     QLMB_REQUIRE(rt_in, "qlmb_moe_forward_routed: NULL logits");
     return moe_forward_impl(L, arena, out, f_in, f_norm, stream, false, rt_in);
 }
-// small_router: the logits of a decode step's few rows come from k_router_logits_small (another summation order
+// small_router: the logits of a decode step's few rows come from k_router_small (another summation order
 // than the tiled kernel; nothing reads them in a backward pass)
 static int moe_forward_impl(const qlmb_moe_layer *L, void *arena, void *out, const void *f_in, const void *f_norm,
                             void *stream, bool small_router, const float *rt_in)
@@ -217,10 +217,8 @@ static int moe_forward_impl(const qlmb_moe_layer *L, void *arena, void *out, con
     } else if (small_router) {
         if ((rc = router_small(a.rt, f_norm, L->dtype, L->wr, a.rprobs, a.assign, a.gate, N, D, E, K, L->bias, L->bias_stride, st))) return rc;
     } else {
-        { ProfScope ps("router_logits", st);
-        if ((rc = router_logits(a.rt, f_norm, L->dtype, L->wr, N, D, E, st))) return rc; }
-        { ProfScope ps("router_topk", st);
-        if ((rc = router_topk(a.rt, a.rprobs, a.assign, a.gate, N, E, K, L->bias, L->bias_stride, st))) return rc; }
+        ProfScope ps("router", st);
+        if ((rc = router_logits_topk(a.rt, f_norm, L->dtype, L->wr, a.rprobs, a.assign, a.gate, N, D, E, K, L->bias, L->bias_stride, st))) return rc;
     }
     // expert grouping, padded to 128-row tiles (cudalm.cu:4189)
     { ProfScope ps("perm_build", st);
@@ -334,8 +332,8 @@ extern "C" int qlmb_moe_route(const qlmb_moe_layer *L, void *arena, void *Xs, co
     const int N = L->N, D = L->D, F = L->F, E = L->E, K = L->K;
     Arena a = carve(arena, N, D, F, E, K);
     cudaStream_t st = as_stream(stream);
-    { ProfScope ps("router_logits", st); if ((rc = router_logits(a.rt, f_norm, L->dtype, L->wr, N, D, E, st))) return rc; }
-    { ProfScope ps("router_topk", st); if ((rc = router_topk(a.rt, a.rprobs, a.assign, a.gate, N, E, K, L->bias, L->bias_stride, st))) return rc; }
+    { ProfScope ps("router", st);
+      if ((rc = router_logits_topk(a.rt, f_norm, L->dtype, L->wr, a.rprobs, a.assign, a.gate, N, D, E, K, L->bias, L->bias_stride, st))) return rc; }
     { ProfScope ps("perm_build", st);
       if ((rc = perm_build(a.assign, N, E, K, 1, 1, a.perm, a.inv, a.off, a.counts, a.bad, nullptr, nullptr, a.chunk, st))) return rc; }
     ProfScope ps("gather_rows", st);
@@ -473,8 +471,8 @@ extern "C" int qlmb_ep_route(const qlmb_moe_layer *L, void *harena, const void *
     const int N = L->N, D = L->D, E = L->E, K = L->K;
     Arena a = carve(harena, N, D, L->F, E, K);
     cudaStream_t st = as_stream(stream);
-    { ProfScope ps("router_logits", st); if ((rc = router_logits(a.rt, f_norm, L->dtype, L->wr, N, D, E, st))) return rc; }
-    { ProfScope ps("router_topk", st); if ((rc = router_topk(a.rt, a.rprobs, a.assign, a.gate, N, E, K, L->bias, L->bias_stride, st))) return rc; }
+    { ProfScope ps("router", st);
+      if ((rc = router_logits_topk(a.rt, f_norm, L->dtype, L->wr, a.rprobs, a.assign, a.gate, N, D, E, K, L->bias, L->bias_stride, st))) return rc; }
     ProfScope ps("count_assign", st);
     return count_assign(a.counts, a.assign, K * N, E, st);
 }

@@ -82,9 +82,61 @@ __global__ void __launch_bounds__(256) k_router_topk_warp(const float *rt, float
     router_topk_row(lane < E ? rt[(size_t)n * E + lane] : 0.0f, n, lane, rprobs, assign, gate, N, E, K, bias, bs);
 }
 
-// A decode step's few rows: logits and selection in one launch, one block per token.  The logits are those of
-// k_router_logits_small (lane = expert, eight warps each sum one eighth of the features in ascending order with fused
-// multiply-adds, the eight partial sums added in warp order); warp 0 then runs the selection above on them.
+// Logits and selection of few tokens: eight tokens per block, warp = token, lane = expert, the block's rows and the whole router
+// matrix in shared memory by one round of asynchronous copies.  The tiled kernel walks the features in 24 chunks whose latency
+// nothing hides when its grid is a few blocks (333 tokens: 6 blocks, 19.6 us; here 42 blocks).  Every output is summed over the
+// features in ascending order with fused multiply-adds, as there: the same bits.
+#define RLF_TOK 8
+template <int XBF16>
+__global__ void __launch_bounds__(256) k_router_few(float *rt, const void *X, const float *Wr, float *rprobs, int *assign, float *gate,
+                                                    int N, int D, int E, int K, const float *bias, int bs)
+{
+    extern __shared__ __align__(16) uint8_t rlf_sm[];
+    float *ws = reinterpret_cast<float *>(rlf_sm);       // [D][E]
+    uint8_t *xs = rlf_sm + (size_t)D * E * 4;            // [RLF_TOK][D]
+    pdl_wait();
+    pdl_trigger();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n0 = blockIdx.x * RLF_TOK, n = n0 + warp;
+    const int xrow = D * (XBF16 ? 2 : 4);
+    const int tok = N - n0 < RLF_TOK ? N - n0 : RLF_TOK;
+    auto copy16 = [](void *dst, const void *src) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+    };
+    for (int i = tid * 16; i < tok * xrow; i += 256 * 16) copy16(xs + i, (const uint8_t *)X + (size_t)n0 * xrow + i);
+    for (int i = tid * 4; i < D * E; i += 256 * 4) copy16(ws + i, Wr + i);
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (n >= N) return;
+    float acc = 0.0f;
+    if (lane < E) {
+        const uint8_t *row = xs + warp * xrow;
+        const float *w = ws + lane;
+#pragma unroll 2
+        for (int j = 0; j < D; j += 8) {
+            float x[8], wv[8];
+            if (XBF16) {
+                const uint4 q = *reinterpret_cast<const uint4 *>(row + j * 2);
+                const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int k = 0; k < 4; k++) { x[2 * k] = __uint_as_float(u[k] << 16); x[2 * k + 1] = __uint_as_float(u[k] & 0xffff0000u); }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 8; k++) x[k] = reinterpret_cast<const float *>(row)[j + k];
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) { wv[k] = *w; w += E; }
+#pragma unroll
+            for (int k = 0; k < 8; k++) acc = __fmaf_rn(x[k], wv[k], acc);
+        }
+        rt[(size_t)n * E + lane] = acc;
+    }
+    __syncwarp();
+    router_topk_row(acc, n, lane, rprobs, assign, gate, N, E, K, bias, bs);
+}
+
+// A decode step's few rows: logits and selection in one launch, one block per token.  Lane = expert,
+// eight warps each sum one eighth of the features in ascending order with fused multiply-adds, the eight partial sums are added in
+// warp order (another order than the kernels above, hence only where no backward pass reads the logits); warp 0 then selects.
 // With perm != NULL (at most 256 routed slots) the block that finishes last also groups the K*N slots by expert in
 // stable order (what k_perm_cluster does in a launch of its own): perm[off[e] ..] = the slots of expert e ascending,
 // off[0..E], counts[0..E), *bad = an expert id out of range.  The blocks take tickets after a fence, so the last one sees
@@ -470,16 +522,37 @@ int router_topk(const float *rt, float *rprobs, int *assign, float *gate, int N,
     return QLMB_OK;
 }
 
+int router_logits_topk(float *rt, const void *X, int x_dtype, const float *Wr, float *rprobs, int *assign, float *gate, int N, int D,
+                       int E, int K, const float *bias, int bs, cudaStream_t st)
+{
+    const bool xb = x_dtype == QLMB_BF16;
+    const size_t smem = (size_t)D * E * 4 + (size_t)RLF_TOK * D * (xb ? 2 : 4);
+    if (E <= 32 && (D % 8) == 0 && (D * E) % 4 == 0 && (((uintptr_t)X | (uintptr_t)Wr) & 15) == 0 && smem <= 200 * 1024 && N <= (xb ? 32 : 16) * sm_count()) {
+        // up to four rounds of blocks, two with fp32 rows (768 x 32: 2000 tokens 24.5 -> 19.1 us, 4736 25.3 -> 36.7): beyond that the tiled kernel's grid fills the device and it reads the matrix less often
+        static bool few_done[64];
+        int dev = 0;
+        QLMB_CUDA(cudaGetDevice(&dev));
+        QLMB_REQUIRE(dev >= 0 && dev < 64, "device index %d", dev);
+        if (!few_done[dev]) {
+            QLMB_CUDA(cudaFuncSetAttribute(k_router_few<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+            QLMB_CUDA(cudaFuncSetAttribute(k_router_few<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+            few_done[dev] = true;
+        }
+        QLMB_CUDA(pdl_launch_small(xb ? k_router_few<1> : k_router_few<0>, dim3((N + RLF_TOK - 1) / RLF_TOK), dim3(256), smem, st, rt, X, Wr, rprobs, assign, gate, N, D, E, K, bias, bs));
+        QLMB_LAUNCH_CHECK("k_router_few");
+        return QLMB_OK;
+    }
+    const int rc = router_logits(rt, X, x_dtype, Wr, N, D, E, st);
+    return rc ? rc : router_topk(rt, rprobs, assign, gate, N, E, K, bias, bs, st);
+}
+
 int router_small(float *rt, const void *X, int x_dtype, const float *Wr, float *rprobs, int *assign, float *gate, int N, int D,
                  int E, int K, const float *bias, int bs, cudaStream_t st, int *perm, int *off, int *counts, int *bad, int *perm_done,
                  const RouterFinish *fin)
 {
     QLMB_REQUIRE(!fin || (N <= 64 && E <= 32 && D <= 2048), "router_small: N=%d E=%d D=%d with slice sums", N, E, D);
     if (perm_done) *perm_done = 0;
-    if (N > 64 || E > 32 || D > 8192) {
-        int rc = router_logits_small(rt, X, x_dtype, Wr, N, D, E, st);
-        return rc ? rc : router_topk(rt, rprobs, assign, gate, N, E, K, bias, bs, st);
-    }
+    if (N > 64 || E > 32 || D > 8192) return router_logits_topk(rt, X, x_dtype, Wr, rprobs, assign, gate, N, D, E, K, bias, bs, st);
     const bool fuse = perm && off && perm_done && K * N <= 256;      // the last block also groups the slots by expert
     if (fuse) *perm_done = 1;
     const RouterFinish none = {};
