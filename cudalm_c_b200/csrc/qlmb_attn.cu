@@ -412,7 +412,8 @@ __global__ void __launch_bounds__(AT_FWD_THREADS, 2) k_attn_fwd(const __grid_con
 //   k_attn_bwd_dq   one CTA per (sequence, head, tile of 128 queries), walks the key tiles;
 //                   dQ accumulates in TMEM.
 // Both recompute the scores from Q, K and the saved log-sum-exp:  P = exp(S/sqrt(hd) - lse),
-// dS = P * (dP - D) / sqrt(hd) with dP = dA V^T and D = rowsum(dA * O) (k_attn_drow).
+// dS = P * (dP - D) / sqrt(hd) with dP = dA V^T and D = rowsum(dA * O).  dq runs first: its threads make D of their own row, beside
+// the first tiles' copies, and leave it for dkv (a launch of its own for D read dA and O once more: 6.5 us at 8 x 1024 x 12).
 //
 // The walked tiles are 64 wide, so that two CTAs fit an SM (100 / 80 KB of shared memory, 256 TMEM columns each): the
 // element-wise phase of one runs beside the MMAs of the other.
@@ -437,45 +438,20 @@ constexpr int AT_BWD_THREADS = 320;             // TMA warp, MMA warp, 8 element
 constexpr int AT_DKV_NS = 4;                    // stages of the walked tiles in dkv
 constexpr int AT_DKV_SMEM = 2 * AT_TILE + 2 * AT_DKV_NS * AT_ITILE + 2 * AT_DKV_NS * AT_BI * 4 + 256;
 constexpr int AT_DQ_NS = 4;                     // stages of the walked tiles in dq
-constexpr int AT_DQ_SMEM = 2 * AT_TILE + 2 * AT_DQ_NS * AT_ITILE + 256;
+constexpr int AT_DQ_SMEM = 2 * AT_TILE + 2 * AT_DQ_NS * AT_ITILE + 2 * AT_BM * 4 + 256;    // + the halves of D, barriers
 
 struct AttnBwdParams {
     alignas(64) CUtensorMap q_map, k_map, v_map, da_map;      // boxes of 128 rows (resident tiles)
     alignas(64) CUtensorMap q_imap, k_imap, v_imap, da_imap;  // boxes of 64 rows (walked tiles)
-    const float *lse, *drow;
+    const float *lse;
+    float *drow;                                              // written by dq, read by dkv
+    const bf16 *O, *dA;
     bf16 *dQ, *dK, *dV;
     const float *cosb, *sinb;                                 // not NULL: dQ and dK leave rotated back
     int B, T, H, KV, win, nqt;
     float scale, scale_log2;
     int *errword;
 };
-
-// eight lanes per (token, head): a load instruction of a warp covers four whole 128-byte rows
-__global__ void __launch_bounds__(256) k_attn_drow(float *drow, const bf16 *dA, const bf16 *O, int B, int T, int H)
-{
-    pdl_wait();
-    pdl_trigger();
-    const size_t g = ((size_t)blockIdx.x * 256 + threadIdx.x) >> 3;
-    const int c = threadIdx.x & 7;
-    const bool live = g < (size_t)B * T * H;
-    float acc = 0.0f;
-    if (live) {
-        const uint4 x = *(reinterpret_cast<const uint4 *>(dA + g * AT_HD) + c), y = *(reinterpret_cast<const uint4 *>(O + g * AT_HD) + c);
-        const __nv_bfloat162 *xh = reinterpret_cast<const __nv_bfloat162 *>(&x), *yh = reinterpret_cast<const __nv_bfloat162 *>(&y);
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const float2 xf = __bfloat1622float2(xh[k]), yf = __bfloat1622float2(yh[k]);
-            acc += xf.x * yf.x + xf.y * yf.y;
-        }
-    }
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (live && c == 0) {
-        const size_t bt = g / H;
-        const int h = (int)(g % H), b = (int)(bt / T), t = (int)(bt % T);
-        drow[((size_t)b * H + h) * T + t] = acc;
-    }
-}
 
 __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid_constant__ AttnBwdParams p)
 {
@@ -696,7 +672,8 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
     extern __shared__ __align__(1024) uint8_t at_smem[];
     constexpr int NS = AT_DQ_NS;
     uint8_t *sQ = at_smem, *sA = sQ + AT_TILE, *sK = sA + AT_TILE, *sV = sK + NS * AT_ITILE;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sV + NS * AT_ITILE);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sV + NS * AT_ITILE + 2 * AT_BM * 4);
+    float *sD = reinterpret_cast<float *>(sV + NS * AT_ITILE);
     uint64_t *qa_full = bars, *s_full = bars + 1, *ds_full = bars + 2, *acc_done = bars + 3, *spare = bars + 4, *s_free = bars + 5,
              *kv_full = bars + 6, *kv_empty = kv_full + NS;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(kv_empty + NS);
@@ -818,7 +795,28 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
         const uint32_t lane_base = (uint32_t)(qr * 32) << 16;
         const size_t rowb = ((size_t)b * p.H + h) * p.T;
         const float L2 = i < p.T ? p.lse[rowb + i] * 1.4426950408889634f : 1e30f;
-        const float Dq = i < p.T ? p.drow[rowb + i] : 0.0f;
+        float Dq = 0.0f;
+        {                                            // this thread's half of D, then both halves in order
+            if (i < p.T) {
+                const size_t at = ((size_t)b * p.T + i) * ((size_t)p.H * AT_HD) + (size_t)h * AT_HD + c * 32;
+                uint4 x[4], y[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) { x[u] = reinterpret_cast<const uint4 *>(p.dA + at)[u]; y[u] = reinterpret_cast<const uint4 *>(p.O + at)[u]; }
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const uint32_t xw[4] = {x[u].x, x[u].y, x[u].z, x[u].w}, yw[4] = {y[u].x, y[u].y, y[u].z, y[u].w};
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        Dq += __uint_as_float(xw[k] << 16) * __uint_as_float(yw[k] << 16);
+                        Dq += __uint_as_float(xw[k] & 0xffff0000u) * __uint_as_float(yw[k] & 0xffff0000u);
+                    }
+                }
+            }
+            sD[c * AT_BM + r] = Dq;
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            Dq = sD[r] + sD[AT_BM + r];
+            if (c == 0 && i < p.T) p.drow[rowb + i] = Dq;
+        }
         bool ok = true;
         for (int t = 0; ok && t < nt; t++) {
             const int k0 = (kt_lo + t) * AT_BI;
@@ -936,7 +934,7 @@ static int attn_bwd_impl(void *dQ, void *dK, void *dV, float *drow, const void *
         const int rc = make_map(m.m, m.base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, m.width, rows, m.width * 2, AT_HD, m.box, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc) return rc;
     }
-    p.lse = lse; p.drow = drow;
+    p.lse = lse; p.drow = drow; p.O = (const bf16 *)O; p.dA = (const bf16 *)dA;
     p.dQ = (bf16 *)dQ; p.dK = (bf16 *)dK; p.dV = (bf16 *)dV;
     p.cosb = cosb; p.sinb = sinb;
     p.B = B; p.T = T; p.H = H; p.KV = KV; p.win = win;
@@ -955,10 +953,8 @@ static int attn_bwd_impl(void *dQ, void *dK, void *dV, float *drow, const void *
         configured_dev[dev_] = true;
     }
     cudaStream_t st = as_stream(stream);
-    const size_t nrow = (size_t)B * T * H;
-    QLMB_CUDA(pdl_launch_small(k_attn_drow, dim3((unsigned)((nrow + 31) / 32)), dim3(256), 0, st, drow, (const bf16 *)dA, (const bf16 *)O, B, T, H));
-    QLMB_CUDA(pdl_launch_small(k_attn_bwd_dkv, dim3((unsigned)(p.nqt * B * KV)), dim3(AT_BWD_THREADS), AT_DKV_SMEM, st, p));
     QLMB_CUDA(pdl_launch_small(k_attn_bwd_dq, dim3((unsigned)(p.nqt * B * H)), dim3(AT_BWD_THREADS), AT_DQ_SMEM, st, p));
+    QLMB_CUDA(pdl_launch_small(k_attn_bwd_dkv, dim3((unsigned)(p.nqt * B * KV)), dim3(AT_BWD_THREADS), AT_DKV_SMEM, st, p));
     QLMB_LAUNCH_CHECK("k_attn_bwd");
     return QLMB_OK;
 }
