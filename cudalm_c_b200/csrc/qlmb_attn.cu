@@ -453,6 +453,32 @@ struct AttnBwdParams {
     int *errword;
 };
 
+// What a cluster of CTAs needs to add its members' sums
+__device__ __forceinline__ void at_cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t at_map(uint32_t local, uint32_t rank)
+{
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float4 at_ld4(uint32_t a)
+{
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void at_st4(bf16 *dst, const float4 v)
+{
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2 *>(dst) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+}
+
+// SPLIT: the query heads of a key/value head on a cluster of CTAs, one each, which add their sums at the end
+template <bool SPLIT>
 __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid_constant__ AttnBwdParams p)
 {
     extern __shared__ __align__(1024) uint8_t at_smem[];
@@ -470,7 +496,8 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
         if (threadIdx.x == 0 && p.errword && atomicCAS(p.errword, 0, 201) == 0) { p.errword[1] = 200; p.errword[2] = (int)blockIdx.x; }
         return;
     }
-    if (__syncthreads_or(threadIdx.x == 0 && at_error_seen(p.errword))) { pdl_wait(); return; }   // uniform over the CTA
+    // SPLIT: the CTAs of a cluster read one another's shared memory at the end, so none leaves early
+    if (!SPLIT && __syncthreads_or(threadIdx.x == 0 && at_error_seen(p.errword))) { pdl_wait(); return; }   // uniform over the CTA
     if (threadIdx.x == 0) {
         mbar_init(smem_u32(kv_full), 1);
         for (int i = 0; i < NS; i++) { mbar_init(smem_u32(&qd_full[i]), 2); mbar_init(smem_u32(&qd_empty[i]), 1); }
@@ -492,13 +519,14 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
 
     // key tiles that see the most queries first
     const int BK_ = p.B * p.KV, grp = p.H / p.KV;
-    const int kt = (int)blockIdx.x / BK_, bk = (int)blockIdx.x % BK_;
+    const int rank = SPLIT ? (int)blockIdx.x % grp : 0, unit = SPLIT ? (int)blockIdx.x / grp : (int)blockIdx.x;
+    const int kt = unit / BK_, bk = unit % BK_;
     const int b = bk / p.KV, kvh = bk % p.KV;
     const int k0 = kt * AT_BN;
     const int qt_lo = k0 / AT_BI;
     int qt_hi = (p.T - 1) / AT_BI;
     if (p.win > 0) { int hi = (k0 + AT_BN - 1 + p.win - 1) / AT_BI; if (hi < qt_hi) qt_hi = hi; }
-    const int nq = qt_hi - qt_lo + 1, nit = nq * grp;     // iteration it: head kvh*grp + it / nq, query tile qt_lo + it % nq
+    const int nq = qt_hi - qt_lo + 1, nit = SPLIT ? nq : nq * grp;     // iteration it: head kvh*grp + it / nq (SPLIT: + rank), query tile qt_lo + it % nq
 
     if (warp == 0) {
         // =============================== producer ===============================
@@ -510,7 +538,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
             tma_load_2d(smem_u32(sV), &p.v_map, smem_u32(kv_full), kvh * AT_HD, b * p.T + k0);
         }
         for (int it = 0; ok && it < nit; it++) {
-            const int st = it % NS, h = kvh * grp + it / nq, q0 = (qt_lo + it % nq) * AT_BI;
+            const int st = it % NS, h = kvh * grp + (SPLIT ? rank : it / nq), q0 = (qt_lo + it % nq) * AT_BI;
             ok = at_wait(smem_u32(&qd_empty[st]), ((uint32_t)(it / NS) & 1u) ^ 1u, abort_flag, p.errword, 201);
             if (!ok) break;
             const uint32_t bar = smem_u32(&qd_full[st]);
@@ -652,19 +680,67 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dkv(const __grid
         if (ok) ok = at_wait(smem_u32(acc_done), (uint32_t)(nit - 1) & 1u, abort_flag, p.errword, 223);
         if (ok) {
             tc_fence_after();
-            // chunk 0: the dV row; chunk 1: the dK row
-            bf16 *dst = (c ? p.dK : p.dV) + ((size_t)b * p.T + key) * ((size_t)p.KV * AT_HD) + (size_t)kvh * AT_HD;
-            if (c && p.cosb) {
-                const size_t pos = (size_t)(key < p.T ? key : 0) * 32;
-                attn_store_rot(dst, tdK + lane_base, key < p.T, p.scale, p.cosb + pos, p.sinb + pos, 2);
+            if (SPLIT) {                             // this head's sums as fp32 over the tiles, dV | dK, row r: unit u at u ^ (r & 7)
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    uint32_t v[32];
+                    tmem_ld32((c ? tdK : tdV) + lane_base + k * 32, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int u = 0; u < 8; u++)
+                        *reinterpret_cast<uint4 *>(at_smem + r * 512 + (((c * 16 + k * 8 + u) ^ (r & 7)) << 4)) = make_uint4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+                }
             } else {
-                attn_store_row64(dst, (c ? tdK : tdV) + lane_base, key < p.T, c ? p.scale : 1.0f);
+                // chunk 0: the dV row; chunk 1: the dK row
+                bf16 *dst = (c ? p.dK : p.dV) + ((size_t)b * p.T + key) * ((size_t)p.KV * AT_HD) + (size_t)kvh * AT_HD;
+                if (c && p.cosb) {
+                    const size_t pos = (size_t)(key < p.T ? key : 0) * 32;
+                    attn_store_rot(dst, tdK + lane_base, key < p.T, p.scale, p.cosb + pos, p.sinb + pos, 2);
+                } else {
+                    attn_store_row64(dst, (c ? tdK : tdV) + lane_base, key < p.T, c ? p.scale : 1.0f);
+                }
             }
         }
         tc_fence_before();
     }
     __syncthreads();
     if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
+    if (SPLIT) {
+        // every CTA adds 128 / grp of the rows over the group's heads, in the heads' order.  A row is 24 items: four columns of dV,
+        // or four of dK with the four that the rotation pairs them with.
+        at_cluster_sync();
+        const int rows = AT_BN / grp;
+        const uint32_t base = smem_u32(at_smem);
+        for (int x = threadIdx.x; x < rows * 24; x += AT_BWD_THREADS) {
+            const int r = rank * rows + x / 24, u = x % 24, key = k0 + r;
+            const bool isk = u >= 16;
+            float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
+            for (int g = 0; g < grp; g++) {
+                const uint32_t peer = at_map(base, (uint32_t)g) + r * 512;
+                const float4 v = at_ld4(peer + ((u ^ (r & 7)) << 4));
+                s0.x += v.x; s0.y += v.y; s0.z += v.z; s0.w += v.w;
+                if (isk) {
+                    const float4 w = at_ld4(peer + (((u + 8) ^ (r & 7)) << 4));
+                    s1.x += w.x; s1.y += w.y; s1.z += w.z; s1.w += w.w;
+                }
+            }
+            if (key >= p.T) continue;
+            const size_t at = ((size_t)b * p.T + key) * ((size_t)p.KV * AT_HD) + (size_t)kvh * AT_HD;
+            if (!isk) { at_st4(p.dV + at + 4 * u, s0); continue; }
+            const int j = 4 * (u - 16);
+            s0.x *= p.scale; s0.y *= p.scale; s0.z *= p.scale; s0.w *= p.scale;
+            s1.x *= p.scale; s1.y *= p.scale; s1.z *= p.scale; s1.w *= p.scale;
+            if (p.cosb) {
+                const float4 cs = *reinterpret_cast<const float4 *>(p.cosb + (size_t)key * 32 + j), sn = *reinterpret_cast<const float4 *>(p.sinb + (size_t)key * 32 + j);
+                const float4 lo = make_float4(s0.x * cs.x + s1.x * sn.x, s0.y * cs.y + s1.y * sn.y, s0.z * cs.z + s1.z * sn.z, s0.w * cs.w + s1.w * sn.w);
+                s1 = make_float4(s1.x * cs.x - s0.x * sn.x, s1.y * cs.y - s0.y * sn.y, s1.z * cs.z - s0.z * sn.z, s1.w * cs.w - s0.w * sn.w);
+                s0 = lo;
+            }
+            at_st4(p.dK + at + j, s0);
+            at_st4(p.dK + at + 32 + j, s1);
+        }
+        at_cluster_sync();                                    // the others' shared memory stays until everyone has read it
+    }
 }
 
 __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_constant__ AttnBwdParams p)
@@ -948,13 +1024,27 @@ static int attn_bwd_impl(void *dQ, void *dK, void *dV, float *drow, const void *
     QLMB_CUDA(cudaGetDevice(&dev_));
     QLMB_REQUIRE(dev_ >= 0 && dev_ < 64, "device index %d", dev_);
     if (!configured_dev[dev_]) {
-        QLMB_CUDA(cudaFuncSetAttribute(k_attn_bwd_dkv, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_DKV_SMEM));
+        QLMB_CUDA(cudaFuncSetAttribute(k_attn_bwd_dkv<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_DKV_SMEM));
+        QLMB_CUDA(cudaFuncSetAttribute(k_attn_bwd_dkv<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_DKV_SMEM));
         QLMB_CUDA(cudaFuncSetAttribute(k_attn_bwd_dq, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_DQ_SMEM));
         configured_dev[dev_] = true;
     }
     cudaStream_t st = as_stream(stream);
     QLMB_CUDA(pdl_launch_small(k_attn_bwd_dq, dim3((unsigned)(p.nqt * B * H)), dim3(AT_BWD_THREADS), AT_DQ_SMEM, st, p));
-    QLMB_CUDA(pdl_launch_small(k_attn_bwd_dkv, dim3((unsigned)(p.nqt * B * KV)), dim3(AT_BWD_THREADS), AT_DKV_SMEM, st, p));
+    const int grp = H / KV, units = p.nqt * B * KV;
+    if ((grp == 2 || grp == 4 || grp == 8) && units <= 2 * sm_count()) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(units * grp)); cfg.blockDim = dim3(AT_BWD_THREADS); cfg.dynamicSmemBytes = AT_DKV_SMEM; cfg.stream = st;
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)grp; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at; cfg.numAttrs = units * grp <= 2 * sm_count() && pdl_enabled() ? 2 : 1;
+        QLMB_CUDA(cudaLaunchKernelEx(&cfg, k_attn_bwd_dkv<true>, p));
+    } else {
+        QLMB_CUDA(pdl_launch_small(k_attn_bwd_dkv<false>, dim3((unsigned)units), dim3(AT_BWD_THREADS), AT_DKV_SMEM, st, p));
+    }
     QLMB_LAUNCH_CHECK("k_attn_bwd");
     return QLMB_OK;
 }

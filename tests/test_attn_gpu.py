@@ -119,3 +119,29 @@ def test_attn_edges(cuda, T, win):
     assert norm(dV, dVr) < 1e-2
     if T > 1 and win != 1:
         assert norm(dQ, dQr) < 1e-2 and norm(dK, dKr) < 1e-2
+
+
+@pytest.mark.parametrize("B,T,H,KV,win", [(1, 300, 4, 1, 0), (2, 129, 8, 1, 50), (1, 64, 8, 2, 0), (75, 100, 8, 4, 0), (1, 200, 6, 2, 0)])
+def test_attn_gradients_of_grouped_heads(cuda, B, T, H, KV, win):
+    """Two, four and eight query heads on a key/value head, whose gradients a cluster adds, three heads and a grid that fills the
+    device, which one CTA walks; with and without the rotation undone.  Bars as above."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import attn, block
+    (Qd, Kd, Vd), (Qh, Kh, Vh) = inputs(B, T, H, KV, 21, cuda)
+    g = torch.Generator(device="cpu"); g.manual_seed(23)
+    dA = torch.randn(B * T, H * 64, generator=g).to(torch.bfloat16)
+    Or, lr, dQr, dKr, dVr = torch_attention(Qh, Kh, Vh, B, T, H, KV, win, dA.float().numpy())
+    O, lse = attn.attn_fwd(Qd, Kd, Vd, B, T, H, KV, win)
+    dQ, dK, dV, drow = attn.attn_bwd(Qd, Kd, Vd, O, dA.to(cuda), lse, B, T, H, KV, win)
+    again = attn.attn_bwd(Qd, Kd, Vd, O, dA.to(cuda), lse, B, T, H, KV, win)
+    rot = block.rope_tables(T, 64, device=cuda)
+    rQ, rK, rV, _ = attn.attn_bwd(Qd, Kd, Vd, O, dA.to(cuda), lse, B, T, H, KV, win, rope=rot)
+    torch.cuda.synchronize()
+    q.check(q.lib().qlmb_check_device(None))
+    assert all(torch.equal(a, b) for a, b in zip((dQ, dK, dV, drow), again)) and torch.equal(rV, dV)
+    norm = lambda a, b: float(np.linalg.norm(a.float().cpu().numpy().astype(np.float64) - b) / np.linalg.norm(b))
+    assert norm(O, Or) < 1e-2 and norm(dQ, dQr) < 1e-2 and norm(dK, dKr) < 1e-2 and norm(dV, dVr) < 1e-2
+    ref = (torch.from_numpy(Or).view(B, T, H, 64) * dA.double().view(B, T, H, 64)).sum(-1).permute(0, 2, 1).numpy()
+    assert np.abs(drow.cpu().numpy() - ref).max() < 2 ** -7 * np.abs(ref).max()
+    block.rope(dK, *rot, KV, 64, T, back=True)
+    assert float((dK.float() - rK.float()).norm()) <= 2 ** -7 * float(rK.float().norm())
