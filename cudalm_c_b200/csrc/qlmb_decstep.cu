@@ -16,7 +16,7 @@
 //   - the cached keys and values of an attention phase and the router's matrix reach shared memory before their barrier.
 // Products are fp32: x * scale times the exact digit, as in the kernels of the separate entry points.
 // Measured (12 layers, D 768, 32 experts top-2 of d_ff 1536, 128-256 cached positions, whole step with the head, a CUDA
-// graph replay): one slot 615 -> 285 us, eight slots 801 -> 511 us.  Above eight slots the chain stays: there the
+// graph replay): one slot 615 -> 278 us, eight slots 801 -> 476 us.  Above eight slots the chain stays: there the
 // experts' weights are a stream and no longer a latency.
 //
 // Built with --fmad=false (router arithmetic); fused multiply-adds are written out.
@@ -160,24 +160,32 @@ __device__ __forceinline__ void ds_words(Words &r, const uint8_t *codes, const f
     }
 }
 // eight nibbles of a code word as exact floats (two's complement, element 0 in the low nibble): a byte in 0..15 under
-// the exponent of 2^23 is 8388608 + byte, and (nibble ^ 8) - 8 is the value
+// the exponent of 2^23 is 8388608 + byte, and (nibble ^ 8) - 8 is the value.  Digits are made and multiplied two at a time:
+// with many experts chosen the tasks are bound by the instructions they issue (eight slots, with one barrier a pass instead
+// of two: 504 -> 476 us a step).
+struct Sums { uint64_t v[4]; };                           // a lane's eight columns of a row: pairs of neighbouring columns
+__device__ __forceinline__ uint64_t ds_two(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ uint64_t ds_two(uint32_t lo, uint32_t hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi)); return r; }
+__device__ __forceinline__ float2 ds_apart(uint64_t v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ uint64_t ds_fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ uint64_t ds_mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t ds_add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 template <int C>
-__device__ __forceinline__ void ds_mul(const Words &r, const float (&x)[C][8], float (&acc)[C][8])
+__device__ __forceinline__ void ds_mul(const Words &r, const float (&x)[C][8], Sums (&acc)[C])
 {
+    const uint64_t off = ds_two(-8388616.0f, -8388616.0f);
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const uint32_t w = r.w[i] ^ 0x88888888u, ev = w & 0x0F0F0F0Fu, od = (w >> 4) & 0x0F0F0F0Fu;
-        float d[8];
+        uint64_t d[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            d[2 * j] = __uint_as_float(__byte_perm(ev, 0x4B000000u, 0x7440 + j)) - 8388616.0f;
-            d[2 * j + 1] = __uint_as_float(__byte_perm(od, 0x4B000000u, 0x7440 + j)) - 8388616.0f;
-        }
+        for (int j = 0; j < 4; j++) d[j] = ds_add2(ds_two(__byte_perm(ev, 0x4B000000u, 0x7440 + j), __byte_perm(od, 0x4B000000u, 0x7440 + j)), off);
 #pragma unroll
         for (int c = 0; c < C; c++) {
-            const float xv = x[c][i] * r.s[i];
+            const float xs = x[c][i] * r.s[i];
+            const uint64_t xv = ds_two(xs, xs);
 #pragma unroll
-            for (int j = 0; j < 8; j++) acc[c][j] = i == 0 ? xv * d[j] : __fmaf_rn(xv, d[j], acc[c][j]);
+            for (int j = 0; j < 4; j++) acc[c].v[j] = i == 0 ? ds_mul2(xv, d[j]) : ds_fma2(xv, d[j], acc[c].v[j]);
         }
     }
 }
@@ -188,14 +196,17 @@ __device__ __forceinline__ void ds_x8(float (&x)[8], uint4 u)
 }
 // the 16 warps' sums of C rows -> out[row(c) * N + col0 + column], warp order.  The caller syncs before `red` is used again.
 template <int C, typename RowPtr>
-__device__ __forceinline__ void ds_reduce(float *red, const float (&acc)[C][8], int n, int col0, int N, RowPtr row)
+__device__ __forceinline__ void ds_reduce(float *red, const Sums (&acc)[C], int n, int col0, int N, RowPtr row)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
     for (int c = 0; c < C; c++) {
         float4 *p = reinterpret_cast<float4 *>(red + (warp * C + c) * DS_COLS + lane * 8);
-        p[0] = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
-        p[1] = make_float4(acc[c][4], acc[c][5], acc[c][6], acc[c][7]);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const float2 u = ds_apart(acc[c].v[2 * h]), v = ds_apart(acc[c].v[2 * h + 1]);
+            p[h] = make_float4(u.x, u.y, v.x, v.y);
+        }
     }
     __syncthreads();
     const int col = threadIdx.x & 255;
@@ -236,7 +247,8 @@ __device__ __forceinline__ void ds_dense(const DsArgs &a, Shared &sh, const DsLa
         uint4 xr[C];
 #pragma unroll
         for (int c = 0; c < C; c++) xr[c] = b0 + c < a.B ? __ldcg(reinterpret_cast<const uint4 *>(X + (size_t)(b0 + c) * a.D + k0)) : make_uint4(0u, 0u, 0u, 0u);
-        float x[C][8], acc[C][8];
+        float x[C][8];
+        Sums acc[C];
 #pragma unroll
         for (int c = 0; c < C; c++) ds_x8(x[c], xr[c]);
         ds_mul<C>(w, x, acc);
@@ -333,7 +345,8 @@ template <bool DOWN, int C>
 __device__ __forceinline__ void ds_ex_pass(const DsArgs &a, float *red, const float *xs, const Words &w, const ExTask &t, const GuActs &xa)
 {
     const int warp = threadIdx.x >> 5, R = a.K * a.B, N = DOWN ? a.D : a.F;
-    float x[C][8], acc[C][8];
+    float x[C][8];
+    Sums acc[C];
     if (DOWN) {
 #pragma unroll
         for (int c = 0; c < C; c++)
@@ -370,6 +383,10 @@ __device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, co
     if (DOWN) ds_dn_acts(a, da, t); else ds_gu_acts(a, ga, t);
     Words w;
     bool fresh = true;
+    // two places for the warps' sums in turn: a warp is past the barrier inside a pass only when every warp has added up
+    // the pass before, so one barrier a pass (two in the down projection, for xs) keeps both and xs safe
+    constexpr int HALF = DS_RED / 8;
+    int place = 0;
 #pragma unroll 1
     for (;;) {
         if (DOWN) {                                       // the slice's activations of this pass
@@ -395,10 +412,10 @@ __device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, co
             if (item < n) t = ds_ex_task<DOWN>(a, sh, item);
         }
         if (item < n) { if (DOWN) ds_dn_acts(a, da, t); else ds_gu_acts(a, ga, t); }
-        if (multi && cur.n == 2) ds_ex_pass<DOWN, 2>(a, red, xs, w, cur, xa);
-        else ds_ex_pass<DOWN, 1>(a, red, xs, w, cur, xa);
+        if (multi && cur.n == 2) ds_ex_pass<DOWN, 2>(a, red + place, xs, w, cur, xa);
+        else ds_ex_pass<DOWN, 1>(a, red + place, xs, w, cur, xa);
         if (item >= n) break;
-        __syncthreads();
+        place ^= HALF;
     }
     ds_wait<0>();
 }
