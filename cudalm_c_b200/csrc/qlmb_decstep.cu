@@ -4,20 +4,21 @@
 // which the memory system delivers in under a microsecond; what a step costs is latency: the chain of launches that
 // this replaces spent 4-6 us in each of nine launches per layer.
 //
-// One CTA of 512 threads per SM (cooperative launch); the seven phases of a layer are separated by grid barriers of about
-// 1100 cycles.  Between two barriers the longest chain of dependent instructions sets the time (about five cycles
-// each), so every phase is written for a short one:
+// One CTA of 512 threads per SM (cooperative launch); what the seven phases of a layer hand to one another is waited for
+// word by word (see DS_NONE below), a hop of 0.8 us, where a grid barrier between two phases and the loads behind it took
+// 1.3.  Between two hops the longest chain of dependent instructions sets the time (about five cycles each), so every
+// phase is written for a short one:
 //   - a weight phase is a set of tasks of 256 output columns x 128 contraction rows: a warp takes eight rows, a lane one
 //     code word (eight columns) of each, so a load instruction covers a whole 128-byte line, the sums of a column stay
 //     in one lane, and the 16 warps' sums meet once in shared memory;
-//   - codes and scales of a phase whose choice of weights is known are in registers before its barrier is waited for;
+//   - codes and scales of a phase whose choice of weights is known are in registers before its input is waited for;
 //   - slice sums go to the consumer as they are and are added there (its loads are independent of one another), in a
 //     fixed order, so a step is reproducible bit for bit;
-//   - the cached keys and values of an attention phase and the router's matrix reach shared memory before their barrier.
+//   - the cached keys and values of an attention phase and the router's matrix reach shared memory before their phase.
 // Products are fp32: x * scale times the exact digit, as in the kernels of the separate entry points.
 // Measured (12 layers, D 768, 32 experts top-2 of d_ff 1536, 128-256 cached positions, whole step with the head, a CUDA
-// graph replay): one slot 615 -> 278 us, eight slots 801 -> 476 us.  Above eight slots the chain stays: there the
-// experts' weights are a stream and no longer a latency.
+// graph replay): one slot 276 us with grid barriers, 201 now, eight slots 477 and 433 (the chain of launches: 615 and
+// 801).  Above eight slots the chain stays: there the experts' weights are a stream and no longer a latency.
 //
 // Built with --fmad=false (router arithmetic); fused multiply-adds are written out.
 #include <cuda_bf16.h>
@@ -48,10 +49,10 @@ struct DsArgs {
     uint32_t mq, md, mf, mr, mfs;                         // ceil(2^32 / n) of those and of the row slices of D and F
     const float *emb; const int *tok, *pos; const float *cosb, *sinb, *nf;
     bf16 *fn;
-    // workspace
+    // workspace: the header and three exchange slots
     unsigned *bar;
-    bf16 *x, *xn, *att, *fi, *fnorm;
-    float *pq, *po, *pg, *pd;                             // slice sums: [D/128][B][NQ], [D/128][B][D], [D/128][2 R][F], [F/128][R][D]
+    uint8_t *slots;
+    size_t slot_bytes, att, fnorm, asg, pq, po, pg, pd;   // offsets of a slot's parts; xn is at 0
     int *errword;
 };
 
@@ -63,9 +64,10 @@ constexpr int DS_MAX_SL = 8;                              // row slices of D (D 
 constexpr int DS_RED = DS_WARPS * 4 * DS_COLS * 4;        // up to four rows' sums of the 16 warps
 constexpr int DS_WR = 1024 * 32 * 4;                      // the router's matrix, or keys and values of an attention phase
 constexpr int DS_XS = 2 * DS_ROWS * 4;
+constexpr int DS_FN = DS_MAX_B * 1024 * 2;                // the rows that the experts take
 constexpr int DS_SLOT = DS_ROWS * 136, DS_DEPTH = 7;      // a task's codes and scales; tasks on their way (in the place of DS_WR)
 static_assert(DS_DEPTH * DS_SLOT <= DS_WR, "ring");
-constexpr int DS_SMEM = DS_RED + DS_WR + DS_XS;
+constexpr int DS_SMEM = DS_RED + DS_WR + DS_XS + DS_FN;
 
 __device__ __forceinline__ uint32_t ds_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ds_cp16(uint32_t dst, const void *src)
@@ -82,13 +84,6 @@ __device__ __forceinline__ uint32_t ds_pack(float a, float b)
     const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t *>(&v);
 }
-__device__ __forceinline__ float4 ds_ld4(const float *p) { return __ldcg(reinterpret_cast<const float4 *>(p)); }
-__device__ __forceinline__ float4 ds_ldrow(const bf16 *p)
-{
-    const uint2 u = __ldcg(reinterpret_cast<const uint2 *>(p));
-    return make_float4(ds_lo(u.x), ds_hi(u.x), ds_lo(u.y), ds_hi(u.y));
-}
-__device__ __forceinline__ void ds_strow(bf16 *p, float4 v) { *reinterpret_cast<uint2 *>(p) = make_uint2(ds_pack(v.x, v.y), ds_pack(v.z, v.w)); }
 __device__ __forceinline__ float4 ds_bf4(float4 v) { return make_float4(ds_bf(v.x), ds_bf(v.y), ds_bf(v.z), ds_bf(v.w)); }
 __device__ __forceinline__ void ds_add4(float4 &a, const float4 b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
 __device__ __forceinline__ void ds_fma4(float4 &a, float g, const float4 b)
@@ -96,53 +91,74 @@ __device__ __forceinline__ void ds_fma4(float4 &a, float g, const float4 b)
 
 struct Shared {
     DsLayer layer[2];
-    unsigned target;                                      // grid barrier: arrivals that the next wait needs
     int pos[DS_MAX_B];
     int npair, pexp[DS_MAX_R];                            // distinct experts of the step and their slots
     unsigned pmask[DS_MAX_R];
+    int srow[DS_MAX_R];                                   // the row of a slot
     float red[DS_WARPS];
     float am[DS_WARPS], al[DS_WARPS];                     // attention: the warps' maxima and sums
     float q[64];
     alignas(16) bf16 kv[128];
     float part[DS_WARPS * 64];
     float logit[DS_WARPS * 32];
+    float x[1024];                                        // a row owner's residual stream (bf16 values), thread q columns 4q .. 4q + 3
 };
 
-// ---- grid barrier: one monotonic counter per launch, reset by the last CTA to leave the kernel.  The wait is bounded by
-// two seconds of %globaltimer; when it runs out the abort word makes every later wait return at once.
-__device__ __forceinline__ unsigned long long ds_now() { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
-__device__ __forceinline__ void gb_arrive(const DsArgs &a, Shared &sh)
+// ---- exchange between the CTAs.  What a phase hands to the next one goes through 32-bit words that hold DS_NONE until
+// they are written: a reader loads the words it needs, all in flight at once, and loads them again while one of them is
+// DS_NONE.  A hop is a store and a load; with a grid barrier between the phases it was a store, a fence, an arrival, a
+// poll and a load.  DS_NONE is a NaN that no arithmetic makes (results are the canonical NaN), and ds_word keeps it out.
+// Layer l writes slot l of three, and its start clears the slot of layer l + 1, which layer l - 2 used (and the q, k, v
+// projections of layer l - 1, for xn).  A grid barrier per layer, arrived at behind the output projection and waited for
+// at the next layer's start, tells that the slot of two layers ago is read and the next one clear, long before the wait.
+// The launch leaves the slots as a further layer would find them; the header keeps which is next, and the shape that they
+// are laid out for: another one (or the zeros of a new workspace) clears all three first.
+constexpr uint32_t DS_NONE = 0xffffffffu;
+__device__ __forceinline__ uint32_t ds_word(uint32_t v) { return v == DS_NONE ? 0x7fff7fffu : v; }
+__device__ __forceinline__ void ds_put(void *p, uint32_t v) { asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
+__device__ __forceinline__ void ds_put(float *p, float v) { ds_put((void *)p, ds_word(__float_as_uint(v))); }
+__device__ __forceinline__ void ds_putrow(bf16 *p, float4 v)
 {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        sh.target += gridDim.x;
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
-    }
+    asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(ds_word(ds_pack(v.x, v.y))), "r"(ds_word(ds_pack(v.z, v.w))) : "memory");
 }
-__device__ __noinline__ void gb_slow(unsigned *bar, unsigned target, int *errword)
+__device__ __forceinline__ uint32_t ds_get(const void *p) { uint32_t v; asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory"); return v; }
+__device__ __forceinline__ uint4 ds_get4(const void *p)
 {
-    unsigned long long t0 = 0;
-    for (unsigned i = 0;; i++) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t ds_max4(uint4 v) { return max(max(v.x, v.y), max(v.z, v.w)); }
+__device__ __forceinline__ float4 ds_float4(uint4 v) { return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)); }
+// Waits are bounded by some seconds of polls (an L2 latency each); when one runs out, the abort word ends every other.
+__device__ __noinline__ bool ds_give_up(unsigned *bar, int *errword, unsigned polls)
+{
+    if (*(volatile unsigned *)(bar + 2)) return true;
+    if (polls < (1u << 23)) return false;
+    if (atomicExch(bar + 2, 1u) == 0u && errword && atomicCAS(errword, 0, 200) == 0) { errword[1] = 400; errword[2] = (int)blockIdx.x; errword[3] = (int)threadIdx.x; }
+    return true;
+}
+// load() = the largest of the words asked for
+template <typename Load> __device__ __forceinline__ void ds_poll(const DsArgs &a, Load load)
+{
+    unsigned i = 0;
+    while (load() == DS_NONE)
+        if ((++i & 1023u) == 0u && ds_give_up(a.bar, a.errword, i)) return;
+}
+// the grid barrier: one counter per launch, reset by the last CTA to leave the kernel
+__device__ __forceinline__ void gb_arrive(const DsArgs &a) { asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory"); }
+__device__ __forceinline__ void gb_wait(const DsArgs &a, unsigned target)
+{
+    for (unsigned i = 1;; i++) {
         unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-        if (v >= target) return;
-        if ((i & 1023u) == 1023u) {
-            if (*(volatile unsigned *)(bar + 2)) return;
-            const unsigned long long t = ds_now();
-            if (!t0) t0 = t;
-            else if (t - t0 > 2000000000ull) {
-                if (atomicExch(bar + 2, 1u) == 0u && errword && atomicCAS(errword, 0, 200) == 0) {
-                    errword[1] = 400; errword[2] = (int)blockIdx.x; errword[3] = (int)target;
-                }
-                return;
-            }
-        }
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+        if (v >= target || ((i & 1023u) == 0u && ds_give_up(a.bar, a.errword, i))) return;
     }
 }
-__device__ __forceinline__ void gb_wait(const DsArgs &a, Shared &sh)
+__device__ __forceinline__ void ds_clear(uint8_t *at, size_t bytes)
 {
-    if (threadIdx.x == 0) gb_slow(a.bar, sh.target, a.errword);
-    __syncthreads();
+    for (size_t i = (blockIdx.x * DS_THREADS + threadIdx.x) * 16; i < bytes; i += gridDim.x * DS_THREADS * 16)
+        *reinterpret_cast<uint4 *>(at + i) = make_uint4(DS_NONE, DS_NONE, DS_NONE, DS_NONE);
 }
 
 // ---- weight phases
@@ -216,19 +232,19 @@ __device__ __forceinline__ void ds_reduce(float *red, const Sums (&acc)[C], int 
             float v = 0.0f;
 #pragma unroll
             for (int w = 0; w < DS_WARPS; w++) v += red[(w * C + c) * DS_COLS + col];
-            __stcg(row(c) + col0 + col, v);
+            ds_put(row(c) + col0 + col, v);
         }
     }
 }
 
 // q, k, v projections (KIND 0) and output projection (KIND 1): a task takes C of the B rows
 template <int KIND, int C>
-__device__ __forceinline__ void ds_dense(const DsArgs &a, Shared &sh, const DsLayer &ly, float *red)
+__device__ __forceinline__ void ds_dense(const DsArgs &a, const DsLayer &ly, float *red, const uint8_t *in, uint8_t *slot)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles = KIND == 0 ? a.tq : a.td, NT = KIND == 0 ? a.D + 2 * a.KD : a.D, sl = a.D / DS_ROWS, n = tiles * sl * ((a.B + C - 1) / C);
-    const bf16 *X = KIND == 0 ? a.xn : a.att;
-    float *out = KIND == 0 ? a.pq : a.po;
+    const bf16 *X = reinterpret_cast<const bf16 *>(in);
+    float *out = reinterpret_cast<float *>(slot + (KIND == 0 ? a.pq : a.po));
     bool first = true;
 #pragma unroll 1
     for (int task = blockIdx.x; task < n; task += gridDim.x) {
@@ -243,10 +259,16 @@ __device__ __forceinline__ void ds_dense(const DsArgs &a, Shared &sh, const DsLa
         }
         Words w;
         ds_words(w, ly.c[m], ly.s[m], N, col, k0);
-        if (first) { gb_wait(a, sh); first = false; } else __syncthreads();
+        if (first) first = false; else __syncthreads();
         uint4 xr[C];
+        ds_poll(a, [&] {
+            uint32_t m = 0;
 #pragma unroll
-        for (int c = 0; c < C; c++) xr[c] = b0 + c < a.B ? __ldcg(reinterpret_cast<const uint4 *>(X + (size_t)(b0 + c) * a.D + k0)) : make_uint4(0u, 0u, 0u, 0u);
+            for (int c = 0; c < C; c++) xr[c] = b0 + c < a.B ? ds_get4(X + (size_t)(b0 + c) * a.D + k0) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int c = 0; c < C; c++) m = max(m, ds_max4(xr[c]));
+            return m;
+        });
         float x[C][8];
         Sums acc[C];
 #pragma unroll
@@ -254,7 +276,6 @@ __device__ __forceinline__ void ds_dense(const DsArgs &a, Shared &sh, const DsLa
         ds_mul<C>(w, x, acc);
         ds_reduce<C>(red, acc, a.B - b0 < C ? a.B - b0 : C, col0, NT, [&](int c) { return out + ((size_t)slice * a.B + b0 + c) * NT; });
     }
-    if (first) gb_wait(a, sh);
 }
 
 // The experts' tasks.  An expert has one or two slots as a rule: a pass multiplies up to two, and the weights, the first
@@ -311,25 +332,17 @@ __device__ __forceinline__ void ds_ring_words(Words &w, const uint8_t *ring, int
 #pragma unroll
     for (int i = 0; i < 8; i++) { w.w[i] = *reinterpret_cast<const uint32_t *>(p + i * 128); w.s[i] = *reinterpret_cast<const float *>(q + i * 8); }
 }
-// gate/up: this warp's eight activations of the pass's two slots
-struct GuActs { uint4 x0, x1; };
-__device__ __forceinline__ void ds_gu_acts(const DsArgs &a, GuActs &x, const ExTask &t)
-{
-    const bf16 *p = a.fnorm + t.slice * DS_ROWS + (threadIdx.x >> 5) * 8;
-    x.x0 = __ldcg(reinterpret_cast<const uint4 *>(p + (size_t)(t.s0 % a.B) * a.D));
-    x.x1 = __ldcg(reinterpret_cast<const uint4 *>(p + (size_t)(t.s1 % a.B) * a.D));
-}
 // down: gate and up sums of one row of the slice (threads 0 .. 127: first slot, 128 .. 255: second)
-struct DnActs { float g[DS_MAX_SL], u[DS_MAX_SL]; };
-__device__ __forceinline__ void ds_dn_acts(const DsArgs &a, DnActs &x, const ExTask &t)
+struct DnActs { uint32_t g[DS_MAX_SL], u[DS_MAX_SL]; };
+__device__ __forceinline__ void ds_dn_acts(const DsArgs &a, DnActs &x, const ExTask &t, const uint8_t *slot)
 {
     const int R = a.K * a.B, ns = a.D / DS_ROWS;
     if ((int)threadIdx.x >= t.n * DS_ROWS) return;
-    const float *p = a.pg + (size_t)((int)threadIdx.x < DS_ROWS ? t.s0 : t.s1) * a.F + t.slice * DS_ROWS + (threadIdx.x & (DS_ROWS - 1));
+    const float *p = reinterpret_cast<const float *>(slot + a.pg) + (size_t)((int)threadIdx.x < DS_ROWS ? t.s0 : t.s1) * a.F + t.slice * DS_ROWS + (threadIdx.x & (DS_ROWS - 1));
 #pragma unroll
     for (int s = 0; s < DS_MAX_SL; s++) {
-        x.g[s] = s < ns ? __ldcg(p) : 0.0f;
-        x.u[s] = s < ns ? __ldcg(p + (size_t)R * a.F) : 0.0f;
+        x.g[s] = s < ns ? ds_get(p) : 0u;
+        x.u[s] = s < ns ? ds_get(p + (size_t)R * a.F) : 0u;
         p += (size_t)2 * R * a.F;
     }
 }
@@ -337,12 +350,12 @@ __device__ __forceinline__ float ds_swiglu(const DnActs &x)
 {
     float g = 0.0f, u = 0.0f;
 #pragma unroll
-    for (int s = 0; s < DS_MAX_SL; s++) { g += x.g[s]; u += x.u[s]; }
+    for (int s = 0; s < DS_MAX_SL; s++) { g += __uint_as_float(x.g[s]); u += __uint_as_float(x.u[s]); }
     g = ds_bf(g); u = ds_bf(u);
     return ds_bf(g * __fdividef(1.0f, 1.0f + __expf(-g)) * u);
 }
 template <bool DOWN, int C>
-__device__ __forceinline__ void ds_ex_pass(const DsArgs &a, float *red, const float *xs, const Words &w, const ExTask &t, const GuActs &xa)
+__device__ __forceinline__ void ds_ex_pass(const DsArgs &a, const Shared &sh, float *red, const float *xs, const bf16 *fn, const Words &w, const ExTask &t, uint8_t *slot)
 {
     const int warp = threadIdx.x >> 5, R = a.K * a.B, N = DOWN ? a.D : a.F;
     float x[C][8];
@@ -356,16 +369,17 @@ __device__ __forceinline__ void ds_ex_pass(const DsArgs &a, float *red, const fl
                 x[c][4 * h] = v.x; x[c][4 * h + 1] = v.y; x[c][4 * h + 2] = v.z; x[c][4 * h + 3] = v.w;
             }
     } else {
-        ds_x8(x[0], xa.x0);
-        if (C > 1) ds_x8(x[C - 1], xa.x1);
+        const bf16 *p = fn + t.slice * DS_ROWS + warp * 8;
+        ds_x8(x[0], *reinterpret_cast<const uint4 *>(p + sh.srow[t.s0] * a.D));
+        if (C > 1) ds_x8(x[C - 1], *reinterpret_cast<const uint4 *>(p + sh.srow[t.s1] * a.D));
     }
     ds_mul<C>(w, x, acc);
-    float *out = DOWN ? a.pd + (size_t)t.slice * R * a.D : a.pg + (size_t)(t.slice * 2 + t.mat) * R * a.F;
+    float *out = reinterpret_cast<float *>(slot + (DOWN ? a.pd : a.pg)) + (DOWN ? (size_t)t.slice * R * a.D : (size_t)(t.slice * 2 + t.mat) * R * a.F);
     ds_reduce<C>(red, acc, t.n, t.tile * DS_COLS, N, [&](int c) { return out + (size_t)(c == 0 ? t.s0 : t.s1) * N; });
 }
-// The down projection's choice of weights is known: its barrier is waited for with the first tasks' weights on their way.
+// The down projection's choice of weights is known: its sums are waited for with the first tasks' weights on their way.
 template <bool DOWN>
-__device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, const DsLayer &ly, float *red, float *xs, uint8_t *ring, bool multi)
+__device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, const DsLayer &ly, float *red, float *xs, const bf16 *fn, uint8_t *ring, bool multi, uint8_t *slot8)
 {
     const int n = DOWN ? sh.npair * (a.F / DS_ROWS) * a.td : sh.npair * 2 * (a.D / DS_ROWS) * a.tf;
     int ask = blockIdx.x, item = blockIdx.x, slot = 0;
@@ -375,12 +389,10 @@ __device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, co
         ds_commit();
         ask += gridDim.x;
     }
-    if (DOWN) gb_wait(a, sh);
     if (item >= n) return;
     ExTask t = ds_ex_task<DOWN>(a, sh, item);
-    GuActs ga;
     DnActs da;
-    if (DOWN) ds_dn_acts(a, da, t); else ds_gu_acts(a, ga, t);
+    if (DOWN) ds_dn_acts(a, da, t, slot8);
     Words w;
     bool fresh = true;
     // two places for the warps' sums in turn: a warp is past the barrier inside a pass only when every warp has added up
@@ -390,7 +402,17 @@ __device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, co
 #pragma unroll 1
     for (;;) {
         if (DOWN) {                                       // the slice's activations of this pass
-            if ((int)threadIdx.x < t.n * DS_ROWS) xs[threadIdx.x] = ds_swiglu(da);
+            if ((int)threadIdx.x < t.n * DS_ROWS) {
+                unsigned i = 0;
+                for (;;) {
+                    uint32_t m = 0;
+#pragma unroll
+                    for (int s = 0; s < DS_MAX_SL; s++) m = max(m, max(da.g[s], da.u[s]));
+                    if (m != DS_NONE || ((++i & 1023u) == 0u && ds_give_up(a.bar, a.errword, i))) break;
+                    ds_dn_acts(a, da, t, slot8);
+                }
+                xs[threadIdx.x] = ds_swiglu(da);
+            }
             __syncthreads();
         }
         if (fresh) {
@@ -404,16 +426,15 @@ __device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, co
             if (++slot == DS_DEPTH) slot = 0;
         }
         const ExTask cur = t;
-        const GuActs xa = ga;
         fresh = !(multi && t.rest);                       // else: more slots of the same expert, same weights
         if (!fresh) ds_pass(t, t.rest);
         else {
             item += gridDim.x;
             if (item < n) t = ds_ex_task<DOWN>(a, sh, item);
         }
-        if (item < n) { if (DOWN) ds_dn_acts(a, da, t); else ds_gu_acts(a, ga, t); }
-        if (multi && cur.n == 2) ds_ex_pass<DOWN, 2>(a, red + place, xs, w, cur, xa);
-        else ds_ex_pass<DOWN, 1>(a, red + place, xs, w, cur, xa);
+        if (DOWN && item < n) ds_dn_acts(a, da, t, slot8);
+        if (multi && cur.n == 2) ds_ex_pass<DOWN, 2>(a, sh, red + place, xs, fn, w, cur, slot8);
+        else ds_ex_pass<DOWN, 1>(a, sh, red + place, xs, fn, w, cur, slot8);
         if (item >= n) break;
         place ^= HALF;
     }
@@ -443,32 +464,37 @@ __device__ __forceinline__ void ds_kv_request(const DsArgs &a, const Shared &sh,
     }
     ds_commit();
 }
-__device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const DsLayer &ly, uint8_t *kvs)
+__device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const DsLayer &ly, uint8_t *kvs, uint8_t *slot)
 {
     const int item = blockIdx.x;
-    if (item >= a.B * a.H) { gb_wait(a, sh); return; }
+    if (item >= a.B * a.H) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, b = item / a.H, h = item - b * a.H, rep = a.H / a.KV, kvh = h / rep;
     const int t = sh.pos[b], r = lane >> 3, c8 = (lane & 7) * 8, mm = tid >> 6, i64 = tid & 63;
-    float *sc = sh.logit + warp * 16;                     // this warp's scores
     const bool bad = t < 0 || t >= a.Tm;                  // a slot past its cache: nothing of it is read or written
     float cs = 0.0f, sn = 0.0f;
     if (tid < 128 && !bad) { cs = __ldg(a.cosb + (size_t)t * 32 + (i64 & 31)); sn = __ldg(a.sinb + (size_t)t * 32 + (i64 & 31)); }
-    gb_wait(a, sh);
+    bf16 *out = reinterpret_cast<bf16 *>(slot + a.att) + (size_t)b * a.D + h * 64 + tid;
     if (bad) {
         ds_wait<0>();
         if (tid == 0 && h == 0) report_bad_index(a.errword, 302, b, t);
-        if (tid < 64) a.att[(size_t)b * a.D + h * 64 + tid] = __float2bfloat16_rn(0.0f);
+        if (tid < 64 && !(tid & 1)) ds_put((void *)out, 0u);
         return;
     }
     float x = 0.0f;
     if (tid < 192) {                                      // one of the 64 columns of q, k or v
         const int NQ = a.D + 2 * a.KD, ns = a.D / DS_ROWS;
-        const float *pp = a.pq + (size_t)b * NQ + (mm == 0 ? h * 64 : a.D + (mm - 1) * a.KD + kvh * 64) + i64;
-        float pv[DS_MAX_SL];
+        const float *pp = reinterpret_cast<const float *>(slot + a.pq) + (size_t)b * NQ + (mm == 0 ? h * 64 : a.D + (mm - 1) * a.KD + kvh * 64) + i64;
+        uint32_t pv[DS_MAX_SL];
+        ds_poll(a, [&] {
+            uint32_t m = 0;
 #pragma unroll
-        for (int k = 0; k < DS_MAX_SL; k++) { pv[k] = k < ns ? __ldcg(pp) : 0.0f; pp += a.B * NQ; }
+            for (int k = 0; k < DS_MAX_SL; k++) pv[k] = k < ns ? ds_get(pp + (size_t)k * a.B * NQ) : 0u;
 #pragma unroll
-        for (int k = 0; k < DS_MAX_SL; k++) x += pv[k];
+            for (int k = 0; k < DS_MAX_SL; k++) m = max(m, pv[k]);
+            return m;
+        });
+#pragma unroll
+        for (int k = 0; k < DS_MAX_SL; k++) x += __uint_as_float(pv[k]);
         x = ds_bf(x);
         sh.part[tid] = x;
     }
@@ -558,7 +584,9 @@ __device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const 
         for (int w = 1; w < DS_WARPS; w++) M = fmaxf(M, sh.am[w]);
 #pragma unroll 8
         for (int w = 0; w < DS_WARPS; w++) { const float f = __expf(sh.am[w] - M); sum += f * sh.al[w]; y += f * sh.part[w * 64 + tid]; }
-        a.att[(size_t)b * a.D + h * 64 + tid] = __float2bfloat16_rn(__fdividef(y, sum));
+        y = __fdividef(y, sum);
+        const float z = __shfl_down_sync(0xffffffffu, y, 1);
+        if (!(tid & 1)) ds_put((void *)out, ds_word(ds_pack(y, z)));
     }
 }
 
@@ -580,7 +608,7 @@ __device__ __forceinline__ void ds_norm_store(const DsArgs &a, Shared &sh, const
     const float rinv = 1.0f / sqrtf(tot / (float)a.D + 1e-5f);
     if (n < a.D) {
         const float4 o = ds_bf4(make_float4(x.x * rinv * gm.x, x.y * rinv * gm.y, x.z * rinv * gm.z, x.w * rinv * gm.w));
-        ds_strow(dst + n, o);
+        ds_putrow(dst + n, o);
         if (xrow) *reinterpret_cast<float4 *>(xrow + n) = o;
     }
 }
@@ -595,26 +623,32 @@ __device__ __forceinline__ void ds_wr_request(const DsArgs &a, const DsLayer &ly
     ds_commit();
 }
 // residual, norm, router of a row
-__device__ __forceinline__ void ds_router(const DsArgs &a, Shared &sh, const DsLayer &ly, float *wr, float *xrow)
+__device__ __forceinline__ void ds_router(const DsArgs &a, Shared &sh, const DsLayer &ly, float *wr, float *xrow, uint8_t *slot)
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, b = ds_row(a);
-    gb_wait(a, sh);
     if (b < 0) return;
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
     const int n = 4 * tid, ns = a.D / DS_ROWS;
     if (n < a.D) {
-        float4 p[DS_MAX_SL], y = x;
-        const float *pp = a.po + (size_t)b * a.D + n;
-        x = ds_ldrow(a.x + (size_t)b * a.D + n);
+        uint4 p[DS_MAX_SL];
+        float4 y = x;
+        const float *pp = reinterpret_cast<const float *>(slot + a.po) + (size_t)b * a.D + n;
+        ds_poll(a, [&] {
+            uint32_t m = 0;
 #pragma unroll
-        for (int k = 0; k < DS_MAX_SL; k++) { p[k] = k < ns ? ds_ld4(pp) : make_float4(0.f, 0.f, 0.f, 0.f); pp += a.B * a.D; }
+            for (int k = 0; k < DS_MAX_SL; k++) p[k] = k < ns ? ds_get4(pp + (size_t)k * a.B * a.D) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-        for (int k = 0; k < DS_MAX_SL; k++) ds_add4(y, p[k]);
+            for (int k = 0; k < DS_MAX_SL; k++) m = max(m, ds_max4(p[k]));
+            return m;
+        });
+#pragma unroll
+        for (int k = 0; k < DS_MAX_SL; k++) ds_add4(y, ds_float4(p[k]));
+        x = *reinterpret_cast<const float4 *>(sh.x + n);
         ds_add4(x, ds_bf4(y));
         x = ds_bf4(x);
-        ds_strow(a.fi + (size_t)b * a.D + n, x);
+        *reinterpret_cast<float4 *>(sh.x + n) = x;
     }
-    ds_norm_store(a, sh, x, ly.an2, a.fnorm + (size_t)b * a.D, xrow);
+    ds_norm_store(a, sh, x, ly.an2, reinterpret_cast<bf16 *>(slot + a.fnorm) + (size_t)b * a.D, xrow);
     ds_wait<0>();
     __syncthreads();
     const int per = a.D / DS_WARPS, j0 = warp * per;      // a multiple of eight
@@ -640,47 +674,65 @@ __device__ __forceinline__ void ds_router(const DsArgs &a, Shared &sh, const DsL
             for (int w = 0; w < DS_WARPS; w++) lg += sh.logit[w * 32 + lane];
             ly.rt[(size_t)b * a.E + lane] = lg;
         }
-        router_topk_row(lg, b, lane, ly.rprobs, ly.assign, ly.gate, a.B, a.E, a.K, nullptr, 0);
+        int *asg = reinterpret_cast<int *>(slot + a.asg);
+        router_topk_row(lg, b, lane, ly.rprobs, ly.assign, ly.gate, a.B, a.E, a.K, nullptr, 0, [&](int at, int pick) { ds_put((void *)(asg + at), (uint32_t)pick); });
     }
 }
 
-// the step's distinct experts and the slots k * B + b of each (in order of first use)
-__device__ __forceinline__ void ds_experts(const DsArgs &a, Shared &sh, const DsLayer &ly)
+// the step's distinct experts and the slots k * B + b of each (in order of first use), and the rows that they take
+__device__ __forceinline__ void ds_experts(const DsArgs &a, Shared &sh, bf16 *fn, const uint8_t *slot)
 {
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x, R = a.K * a.B;
         int e = -1;
-        if (lane < R) { e = __ldcg(ly.assign + lane); if ((unsigned)e >= (unsigned)a.E) e = 0; }
+        if (lane < R) {
+            const int *p = reinterpret_cast<const int *>(slot + a.asg) + lane;
+            ds_poll(a, [&] { e = (int)ds_get(p); return (uint32_t)e; });
+            if ((unsigned)e >= (unsigned)a.E) e = 0;
+            sh.srow[lane] = lane % a.B;
+        }
+        __syncwarp();
         const unsigned m = __match_any_sync(0xffffffffu, e), lt = (1u << lane) - 1u;
         const unsigned lead = __ballot_sync(0xffffffffu, e >= 0 && (m & lt) == 0u);
         if ((lead >> lane) & 1u) { const int i = __popc(lead & lt); sh.pexp[i] = e; sh.pmask[i] = m; }
         if (lane == 0) sh.npair = __popc(lead);
     }
+    for (int i = DS_THREADS - 1 - (int)threadIdx.x; i < a.B * a.D / 8; i += DS_THREADS) {          // (warp 0, which is late, last)
+        uint4 v;
+        ds_poll(a, [&] { v = ds_get4(slot + a.fnorm + (size_t)i * 16); return ds_max4(v); });
+        *reinterpret_cast<uint4 *>(fn + (size_t)i * 8) = v;
+    }
     __syncthreads();
 }
 
 // gate-weighted combination, residual, the next norm of a row
-__device__ __forceinline__ void ds_combine(const DsArgs &a, Shared &sh, const DsLayer &ly, float *ys, int l)
+__device__ __forceinline__ void ds_combine(const DsArgs &a, Shared &sh, const DsLayer &ly, float *ys, int l, uint8_t *slot)
 {
     const int b = ds_row(a);
     if (b < 0) return;
     const int c = 4 * threadIdx.x;
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (c < a.D) x = ds_ldrow(a.fi + (size_t)b * a.D + c);
+    if (c < a.D) x = *reinterpret_cast<const float4 *>(sh.x + c);
     if ((int)threadIdx.x < a.K) sh.red[threadIdx.x] = __ldcg(ly.gate + (size_t)threadIdx.x * a.B + b);    // K <= 16
     const int half = threadIdx.x >> 8, n = 4 * (threadIdx.x & 255), R = a.K * a.B, ns = a.F / DS_ROWS;
     if (n < a.D) {
 #pragma unroll 1
         for (int k = half; k < a.K; k += 2) {
-            const float *p = a.pd + (size_t)(k * a.B + b) * a.D + n;
+            const float *p = reinterpret_cast<const float *>(slot + a.pd) + (size_t)(k * a.B + b) * a.D + n;
             float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
             for (int s0 = 0; s0 < ns; s0 += 12) {         // twelve slices in flight: d_ff 1536 in one go
-                float4 v[12];
+                uint4 v[12];
+                ds_poll(a, [&] {
+                    uint32_t m = 0;
 #pragma unroll
-                for (int s = 0; s < 12; s++) { v[s] = s0 + s < ns ? ds_ld4(p) : make_float4(0.f, 0.f, 0.f, 0.f); p += (size_t)R * a.D; }
+                    for (int s = 0; s < 12; s++) v[s] = s0 + s < ns ? ds_get4(p + (size_t)(s0 + s) * R * a.D) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-                for (int s = 0; s < 12; s++) ds_add4(y, v[s]);
+                    for (int s = 0; s < 12; s++) m = max(m, ds_max4(v[s]));
+                    return m;
+                });
+#pragma unroll
+                for (int s = 0; s < 12; s++) ds_add4(y, ds_float4(v[s]));
             }
             *reinterpret_cast<float4 *>(ys + k * a.D + n) = ds_bf4(y);
         }
@@ -690,10 +742,10 @@ __device__ __forceinline__ void ds_combine(const DsArgs &a, Shared &sh, const Ds
 #pragma unroll 1
         for (int k = 0; k < a.K; k++) ds_fma4(x, sh.red[k], *reinterpret_cast<const float4 *>(ys + k * a.D + c));
         x = ds_bf4(x);
-        ds_strow(a.x + (size_t)b * a.D + c, x);
+        *reinterpret_cast<float4 *>(sh.x + c) = x;
     }
     __syncthreads();                                      // red held the gates
-    if (l + 1 < a.L) ds_norm_store(a, sh, x, sh.layer[(l + 1) & 1].an1, a.xn + (size_t)b * a.D, nullptr);
+    if (l + 1 < a.L) ds_norm_store(a, sh, x, sh.layer[(l + 1) & 1].an1, reinterpret_cast<bf16 *>(slot) + (size_t)b * a.D, nullptr);
     else ds_norm_store(a, sh, x, a.nf, a.fn + (size_t)b * a.D, nullptr);
 }
 
@@ -704,13 +756,13 @@ __global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constan
     extern __shared__ __align__(128) uint8_t dsm[];
     __shared__ Shared sh;
     float *red = reinterpret_cast<float *>(dsm), *wr = reinterpret_cast<float *>(dsm + DS_RED), *xs = reinterpret_cast<float *>(dsm + DS_RED + DS_WR);
+    bf16 *fn = reinterpret_cast<bf16 *>(dsm + DS_RED + DS_WR + DS_XS);
     auto load_layer = [&](int l) {
         if (threadIdx.x < DS_LAYER_WORDS)
             reinterpret_cast<unsigned long long *>(&sh.layer[l & 1])[threadIdx.x] = __ldg(reinterpret_cast<const unsigned long long *>(a.layers + l) + threadIdx.x);
     };
     load_layer(0);
     if (threadIdx.x < DS_MAX_B) sh.pos[threadIdx.x] = (int)threadIdx.x < a.B ? __ldg(a.pos + threadIdx.x) : 0;
-    if (threadIdx.x == 0) sh.target = 0u;
     // Every CTA looks the whole table over (2 KB from L2, beside the loads above): a pointer that is missing or not aligned
     // for its loads is reported, and the whole grid leaves before its first barrier.
     int bad = 0;
@@ -720,59 +772,85 @@ __global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constan
     }
     if (bad && blockIdx.x == 0) report_bad_index(a.errword, 304, (bad - 1) / DS_LAYER_WORDS, (bad - 1) % DS_LAYER_WORDS);
     if (__syncthreads_or(bad)) return;
+    const unsigned shape0 = 1u + (unsigned)(a.B | a.D << 4 | a.KD << 15 | a.K << 26), shape1 = (unsigned)a.F;   // never 0; the last CTA writes them
+    const unsigned next = __ldcg(a.bar + 3);
+    unsigned gate = 0;                                    // arrivals that the next wait for the grid needs
+    if (__ldcg(a.bar + 4) != shape0 || __ldcg(a.bar + 5) != shape1) {
+        ds_clear(a.slots, 3 * a.slot_bytes);
+        gate += gridDim.x;
+        __syncthreads();
+        if (threadIdx.x == 0) { gb_arrive(a); gb_wait(a, gate); }
+        __syncthreads();
+    }
+    // slots of the layer before, this one and the one after
+    uint8_t *prev = a.slots + (next == 0 ? 2u : next - 1u) * a.slot_bytes, *cur = a.slots + next * a.slot_bytes, *after = a.slots + (next == 2 ? 0u : next + 1u) * a.slot_bytes;
     if (ds_row(a) >= 0) {                                 // embedding row and the first norm
         const int b = ds_row(a), n = 4 * threadIdx.x;
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
         if (n < a.D) {
             x = ds_bf4(__ldg(reinterpret_cast<const float4 *>(a.emb + (size_t)__ldg(a.tok + b) * a.D + n)));
-            ds_strow(a.x + (size_t)b * a.D + n, x);
+            *reinterpret_cast<float4 *>(sh.x + n) = x;
         }
-        ds_norm_store(a, sh, x, sh.layer[0].an1, a.xn + (size_t)b * a.D, nullptr);
+        ds_norm_store(a, sh, x, sh.layer[0].an1, reinterpret_cast<bf16 *>(prev) + (size_t)b * a.D, nullptr);
     }
 #pragma unroll 1
     for (int l = 0; l < a.L; l++) {
         const DsLayer &ly = sh.layer[l & 1];
-        gb_arrive(a, sh);
-        if (l + 1 < a.L) load_layer(l + 1);               // every thread has passed the sync in gb_arrive: the other half is free
+        __syncthreads();
+        if (l + 1 < a.L) load_layer(l + 1);               // every thread is past the layer before: the other half is free
         if ((int)blockIdx.x < a.B * a.H) ds_kv_request(a, sh, ly, dsm + DS_RED, blockIdx.x, 0);
         else if (ds_row(a) >= 0) ds_wr_request(a, ly, wr);
-        ds_dense<0, C>(a, sh, ly, red);
-        gb_arrive(a, sh);
-        ds_attention(a, sh, ly, dsm + DS_RED);
-        gb_arrive(a, sh);
-        ds_dense<1, C>(a, sh, ly, red);
-        gb_arrive(a, sh);
-        ds_router(a, sh, ly, wr, red);
-        gb_arrive(a, sh);
-        gb_wait(a, sh);
-        ds_experts(a, sh, ly);
-        ds_experts_phase<false>(a, sh, ly, red, xs, dsm + DS_RED, MULTI);
-        gb_arrive(a, sh);
-        ds_experts_phase<true>(a, sh, ly, red, xs, dsm + DS_RED, MULTI);
-        gb_arrive(a, sh);
-        gb_wait(a, sh);
-        ds_combine(a, sh, ly, red, l);
+        if (l > 0) {                                      // (every path to a store or a poll of this layer's slot has a barrier of the CTA on it)
+            gate += gridDim.x;
+            if (threadIdx.x == DS_THREADS - 1) gb_wait(a, gate);
+        }
+        ds_dense<0, C>(a, ly, red, prev, cur);
+        __syncthreads();
+        ds_clear(after, a.slot_bytes);
+        ds_attention(a, sh, ly, dsm + DS_RED, cur);
+        __syncthreads();
+        ds_dense<1, C>(a, ly, red, cur + a.att, cur);
+        __syncthreads();
+        if (l + 1 < a.L && threadIdx.x == DS_THREADS - 1) gb_arrive(a);
+        ds_router(a, sh, ly, wr, red, cur);
+        __syncthreads();
+        ds_experts(a, sh, fn, cur);
+        ds_experts_phase<false>(a, sh, ly, red, xs, fn, dsm + DS_RED, MULTI, cur);
+        __syncthreads();
+        ds_experts_phase<true>(a, sh, ly, red, xs, fn, dsm + DS_RED, MULTI, cur);
+        __syncthreads();
+        ds_combine(a, sh, ly, red, l, cur);
+        uint8_t *p = prev;
+        prev = cur; cur = after; after = p;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        if (atomicAdd(a.bar + 1, 1u) == gridDim.x - 1) { a.bar[0] = 0u; a.bar[1] = 0u; a.bar[2] = 0u; __threadfence(); }
+        if (atomicAdd(a.bar + 1, 1u) == gridDim.x - 1) {
+            a.bar[3] = (next + (unsigned)a.L) % 3u;
+            a.bar[4] = *(volatile unsigned *)(a.bar + 2) ? 0u : shape0;      // after an abort the slots hold anything
+            a.bar[5] = shape1;
+            a.bar[0] = 0u; a.bar[1] = 0u; a.bar[2] = 0u;
+            __threadfence();
+        }
     }
 }
 
-struct DsLayout { size_t x, xn, att, fi, fnorm, pq, po, pg, pd, bytes; };
+struct DsLayout { size_t att, fnorm, asg, pq, po, pg, pd, slot, bytes; };
 static DsLayout ds_layout(int B, int D, int KD, int F, int K)
 {
     DsLayout w;
-    size_t cur = 256;
+    size_t cur = 0;
     auto take = [&](size_t n) { const size_t at = cur; cur += (n + 255) & ~(size_t)255; return at; };
     const size_t b = B, d = D, r = (size_t)K * B, sd = D / DS_ROWS, sf = F / DS_ROWS;
-    w.x = take(b * d * 2); w.xn = take(b * d * 2); w.att = take(b * d * 2); w.fi = take(b * d * 2); w.fnorm = take(b * d * 2);
-    w.pq = take(sd * b * (d + 2 * (size_t)KD) * 4);
+    take(b * d * 2);                                      // xn
+    w.att = take(b * d * 2); w.fnorm = take(b * d * 2); w.asg = take(r * 4);
+    w.pq = take(sd * b * (d + 2 * (size_t)KD) * 4);       // slice sums: [D/128][B][NQ], [D/128][B][D], [D/128][2 R][F], [F/128][R][D]
     w.po = take(sd * b * d * 4);
     w.pg = take(sd * 2 * r * F * 4);
     w.pd = take(sf * r * d * 4);
-    w.bytes = cur;
+    w.slot = cur;
+    w.bytes = 256 + 3 * cur;
     return w;
 }
 static bool ds_fits(int B, int Tm, int D, int H, int KV, int F, int E, int K)
@@ -813,8 +891,8 @@ extern "C" int qlmb_dec_step(const qlmb_dec_step_args *p, void *stream)
     a.mq = recip(a.tq); a.md = recip(a.td); a.mf = recip(a.tf); a.mr = recip(a.D / DS_ROWS); a.mfs = recip(a.F / DS_ROWS);
     a.emb = p->emb; a.tok = p->tok; a.pos = p->pos; a.cosb = p->cosb; a.sinb = p->sinb; a.nf = p->nf; a.fn = (bf16 *)p->fn;
     a.bar = (unsigned *)ws;
-    a.x = (bf16 *)(ws + w.x); a.xn = (bf16 *)(ws + w.xn); a.att = (bf16 *)(ws + w.att); a.fi = (bf16 *)(ws + w.fi); a.fnorm = (bf16 *)(ws + w.fnorm);
-    a.pq = (float *)(ws + w.pq); a.po = (float *)(ws + w.po); a.pg = (float *)(ws + w.pg); a.pd = (float *)(ws + w.pd);
+    a.slots = ws + 256; a.slot_bytes = w.slot;
+    a.att = w.att; a.fnorm = w.fnorm; a.asg = w.asg; a.pq = w.pq; a.po = w.po; a.pg = w.pg; a.pd = w.pd;
     a.errword = device_error_word();
     // rows per task of the dense phases: the fewest with which the q, k, v tasks are one round of the device
     int c = 1;

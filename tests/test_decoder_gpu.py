@@ -380,6 +380,34 @@ def test_one_launch_step_equals_the_chain(cuda, B, D, KV, E, K, F, fill, Tm):
         assert ((t != b).flatten(2).any(-1).sum(1) <= 1).all()              # at most the slot's own row changed
 
 
+@pytest.mark.parametrize("L", [1, 2, 3, 4])
+def test_one_launch_steps_in_a_row_and_a_workspace_of_several_shapes(cuda, L):
+    """What the CTAs hand to one another lies in three slots used in turn across layers and launches, whatever the number of
+    layers leaves them at, and a workspace may go to another shape and come back: the same bits at every launch."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import model
+    from cudalm_c_b200._lib import ptr, stream_ptr
+    cfg = model.Config(L=L, D=256, H=4, KV=2, hd=64, E=8, K=2, F=384, V=512, T=64, B=1)
+    m = model.QlmModel(cfg, cuda, seed=3)
+    g = torch.Generator(device=cuda); g.manual_seed(L)
+    decs, want = [], []
+    for B in (1, 3, 8):
+        d = model.Decoder(m, B, 64)
+        d.prefill(torch.randint(0, cfg.V, (B, 20), generator=g, dtype=torch.int32, device=cuda))
+        q.check(q.lib().qlmb_dec_step(d._step_plan(), stream_ptr()))
+        decs.append(d)
+        want.append(d.fn.clone())
+    ws = torch.zeros(max(d._ws.numel() for d in decs), dtype=torch.uint8, device=cuda)
+    for i in (0, 0, 0, 0, 1, 1, 0, 2, 2, 2, 1, 0):
+        d = decs[i]
+        d._step_plan()
+        d._plan.ws = ptr(ws)
+        d.fn.fill_(7.0)
+        q.check(q.lib().qlmb_dec_step(d._plan, stream_ptr()))
+        assert torch.equal(d.fn, want[i]), i
+    q.check(q.lib().qlmb_check_device(None))
+
+
 @pytest.mark.parametrize("B,D,Tm", [(5, 128, 40), (16, 768, 300), (17, 256, 64), (33, 512, 100), (64, 768, 1024)])
 def test_decode_attention_on_the_projections_slice_sums(cuda, B, D, Tm):
     """q, k, v, rotation, append and attention in two launches: the same bits, in output and caches, as the separate entries; a
