@@ -17,7 +17,7 @@
 //   - the cached keys and values of an attention phase and the router's matrix reach shared memory before their phase.
 // Products are fp32: x * scale times the exact digit, as in the kernels of the separate entry points.
 // Measured (12 layers, D 768, 32 experts top-2 of d_ff 1536, 128-256 cached positions, whole step with the head, a CUDA
-// graph replay): one slot 276 us with grid barriers, 201 now, eight slots 477 and 433 (the chain of launches: 615 and
+// graph replay): one slot 276 us with grid barriers, 199 now, eight slots 477 and 415 (the chain of launches: 615 and
 // 801).  Above eight slots the chain stays: there the experts' weights are a stream and no longer a latency.
 //
 // Built with --fmad=false (router arithmetic); fused multiply-adds are written out.
@@ -95,13 +95,15 @@ struct Shared {
     int npair, pexp[DS_MAX_R];                            // distinct experts of the step and their slots
     unsigned pmask[DS_MAX_R];
     int srow[DS_MAX_R];                                   // the row of a slot
+    int ab, ah, akv, afirst;                                      // the CTA's attention item: slot, head, key/value head
     float red[DS_WARPS];
-    float am[DS_WARPS], al[DS_WARPS];                     // attention: the warps' maxima and sums
+    alignas(16) float am[DS_WARPS], al[DS_WARPS];                     // attention: the warps' maxima and sums
     float q[64];
     alignas(16) bf16 kv[128];
-    float part[DS_WARPS * 64];
+    alignas(16) float part[DS_WARPS * 64];
     float logit[DS_WARPS * 32];
-    float x[1024];                                        // a row owner's residual stream (bf16 values), thread q columns 4q .. 4q + 3
+    float gate[DS_WARPS];                                 // a row owner's gates
+    alignas(16) float x[1024];                                        // a row owner's residual stream (bf16 values), thread q columns 4q .. 4q + 3
 };
 
 // ---- exchange between the CTAs.  What a phase hands to the next one goes through 32-bit words that hold DS_NONE until
@@ -180,6 +182,7 @@ __device__ __forceinline__ void ds_words(Words &r, const uint8_t *codes, const f
 // with many experts chosen the tasks are bound by the instructions they issue (eight slots, with one barrier a pass instead
 // of two: 504 -> 476 us a step).
 struct Sums { uint64_t v[4]; };                           // a lane's eight columns of a row: pairs of neighbouring columns
+__device__ __forceinline__ uint64_t ds_pair(uint32_t x) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(x << 16), "r"(x & 0xffff0000u)); return r; }
 __device__ __forceinline__ uint64_t ds_two(float lo, float hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
 __device__ __forceinline__ uint64_t ds_two(uint32_t lo, uint32_t hi) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi)); return r; }
 __device__ __forceinline__ float2 ds_apart(uint64_t v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
@@ -238,23 +241,22 @@ __device__ __forceinline__ void ds_reduce(float *red, const Sums (&acc)[C], int 
 }
 
 // q, k, v projections (KIND 0) and output projection (KIND 1): a task takes C of the B rows
-template <int KIND, int C>
-__device__ __forceinline__ void ds_dense(const DsArgs &a, const DsLayer &ly, float *red, const uint8_t *in, uint8_t *slot)
+template <int C>
+__device__ __forceinline__ void ds_dense(const DsArgs &a, const DsLayer &ly, float *red, bool wo, const uint8_t *in, uint8_t *slot)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles = KIND == 0 ? a.tq : a.td, NT = KIND == 0 ? a.D + 2 * a.KD : a.D, sl = a.D / DS_ROWS, n = tiles * sl * ((a.B + C - 1) / C);
+    const int tiles = !wo ? a.tq : a.td, NT = !wo ? a.D + 2 * a.KD : a.D, sl = a.D / DS_ROWS, n = tiles * sl * ((a.B + C - 1) / C);
     const bf16 *X = reinterpret_cast<const bf16 *>(in);
-    float *out = reinterpret_cast<float *>(slot + (KIND == 0 ? a.pq : a.po));
+    float *out = reinterpret_cast<float *>(slot + (!wo ? a.pq : a.po));
     bool first = true;
 #pragma unroll 1
     for (int task = blockIdx.x; task < n; task += gridDim.x) {
-        const int ts = ds_div(task, tiles, KIND == 0 ? a.mq : a.md), col0 = (task - ts * tiles) * DS_COLS, ch = ds_div(ts, sl, a.mr);
+        const int ts = ds_div(task, tiles, !wo ? a.mq : a.md), col0 = (task - ts * tiles) * DS_COLS, ch = ds_div(ts, sl, a.mr);
         const int slice = ts - ch * sl, k0 = slice * DS_ROWS + warp * 8, b0 = ch * C;
         int col = col0 + lane * 8;
         if (col >= NT) col = NT - 8;                      // lanes past the last column repeat it and are not read
-        int m = 3, N = a.D;
-        if (KIND == 0) {
-            m = 0;
+        int m = wo ? 3 : 0, N = a.D;
+        if (!wo) {
             if (col >= a.D) { col -= a.D; m = 1; N = a.KD; if (col >= a.KD) { col -= a.KD; m = 2; } }
         }
         Words w;
@@ -289,11 +291,10 @@ __device__ __forceinline__ void ds_pass(ExTask &t, unsigned mask)
     t.s1 = mask ? __ffs(mask) - 1 : t.s0;
     t.rest = mask & (mask - 1);
 }
-template <bool DOWN>
-__device__ __forceinline__ ExTask ds_ex_task(const DsArgs &a, const Shared &sh, int item)
+__device__ __forceinline__ ExTask ds_ex_task(const DsArgs &a, const Shared &sh, bool down, int item)
 {
     ExTask t;
-    if (DOWN) {
+    if (down) {
         const int fs = a.F / DS_ROWS, q = ds_div(item, a.td, a.md);
         t.tile = item - q * a.td; t.mat = 0;
         t.pair = ds_div(q, fs, a.mfs);
@@ -309,10 +310,9 @@ __device__ __forceinline__ ExTask ds_ex_task(const DsArgs &a, const Shared &sh, 
 }
 // The codes and scales of a task go through a ring in shared memory, DS_DEPTH tasks ahead: with one task (17 KB per SM)
 // ahead a round of tasks took a memory latency.  Every warp copies and reads its own eight rows only.
-template <bool DOWN>
-__device__ __forceinline__ void ds_ex_request(const DsArgs &a, const Shared &sh, const DsLayer &ly, uint8_t *ring, int slot, const ExTask &t)
+__device__ __forceinline__ void ds_ex_request(const DsArgs &a, const Shared &sh, bool down, const DsLayer &ly, uint8_t *ring, int slot, const ExTask &t)
 {
-    const int N = DOWN ? a.D : a.F, m = DOWN ? 6 : 4 + t.mat, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int N = down ? a.D : a.F, m = down ? 6 : 4 + t.mat, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t mat = (size_t)sh.pexp[t.pair] * a.D * a.F;
     const int k0 = t.slice * DS_ROWS + warp * 8, r = lane >> 3, c = lane & 7;
     const uint32_t d = ds_smem(ring + slot * DS_SLOT);
@@ -354,13 +354,13 @@ __device__ __forceinline__ float ds_swiglu(const DnActs &x)
     g = ds_bf(g); u = ds_bf(u);
     return ds_bf(g * __fdividef(1.0f, 1.0f + __expf(-g)) * u);
 }
-template <bool DOWN, int C>
-__device__ __forceinline__ void ds_ex_pass(const DsArgs &a, const Shared &sh, float *red, const float *xs, const bf16 *fn, const Words &w, const ExTask &t, uint8_t *slot)
+template <int C>
+__device__ __forceinline__ void ds_ex_pass(const DsArgs &a, const Shared &sh, bool down, float *red, const float *xs, const bf16 *fn, const Words &w, const ExTask &t, uint8_t *slot)
 {
-    const int warp = threadIdx.x >> 5, R = a.K * a.B, N = DOWN ? a.D : a.F;
+    const int warp = threadIdx.x >> 5, R = a.K * a.B, N = down ? a.D : a.F;
     float x[C][8];
     Sums acc[C];
-    if (DOWN) {
+    if (down) {
 #pragma unroll
         for (int c = 0; c < C; c++)
 #pragma unroll
@@ -374,25 +374,24 @@ __device__ __forceinline__ void ds_ex_pass(const DsArgs &a, const Shared &sh, fl
         if (C > 1) ds_x8(x[C - 1], *reinterpret_cast<const uint4 *>(p + sh.srow[t.s1] * a.D));
     }
     ds_mul<C>(w, x, acc);
-    float *out = reinterpret_cast<float *>(slot + (DOWN ? a.pd : a.pg)) + (DOWN ? (size_t)t.slice * R * a.D : (size_t)(t.slice * 2 + t.mat) * R * a.F);
+    float *out = reinterpret_cast<float *>(slot + (down ? a.pd : a.pg)) + (down ? (size_t)t.slice * R * a.D : (size_t)(t.slice * 2 + t.mat) * R * a.F);
     ds_reduce<C>(red, acc, t.n, t.tile * DS_COLS, N, [&](int c) { return out + (size_t)(c == 0 ? t.s0 : t.s1) * N; });
 }
 // The down projection's choice of weights is known: its sums are waited for with the first tasks' weights on their way.
-template <bool DOWN>
-__device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, const DsLayer &ly, float *red, float *xs, const bf16 *fn, uint8_t *ring, bool multi, uint8_t *slot8)
+__device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, bool down, const DsLayer &ly, float *red, float *xs, const bf16 *fn, uint8_t *ring, bool multi, uint8_t *slot8)
 {
-    const int n = DOWN ? sh.npair * (a.F / DS_ROWS) * a.td : sh.npair * 2 * (a.D / DS_ROWS) * a.tf;
+    const int n = down ? sh.npair * (a.F / DS_ROWS) * a.td : sh.npair * 2 * (a.D / DS_ROWS) * a.tf;
     int ask = blockIdx.x, item = blockIdx.x, slot = 0;
 #pragma unroll 1
     for (int k = 0; k < DS_DEPTH; k++) {
-        if (ask < n) ds_ex_request<DOWN>(a, sh, ly, ring, k, ds_ex_task<DOWN>(a, sh, ask));
+        if (ask < n) ds_ex_request(a, sh, down, ly, ring, k, ds_ex_task(a, sh, down, ask));
         ds_commit();
         ask += gridDim.x;
     }
     if (item >= n) return;
-    ExTask t = ds_ex_task<DOWN>(a, sh, item);
+    ExTask t = ds_ex_task(a, sh, down, item);
     DnActs da;
-    if (DOWN) ds_dn_acts(a, da, t, slot8);
+    if (down) ds_dn_acts(a, da, t, slot8);
     Words w;
     bool fresh = true;
     // two places for the warps' sums in turn: a warp is past the barrier inside a pass only when every warp has added up
@@ -401,7 +400,7 @@ __device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, co
     int place = 0;
 #pragma unroll 1
     for (;;) {
-        if (DOWN) {                                       // the slice's activations of this pass
+        if (down) {                                       // the slice's activations of this pass
             if ((int)threadIdx.x < t.n * DS_ROWS) {
                 unsigned i = 0;
                 for (;;) {
@@ -420,7 +419,7 @@ __device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, co
             __syncwarp();
             ds_ring_words(w, ring, slot);
             __syncwarp();
-            if (ask < n) ds_ex_request<DOWN>(a, sh, ly, ring, slot, ds_ex_task<DOWN>(a, sh, ask));
+            if (ask < n) ds_ex_request(a, sh, down, ly, ring, slot, ds_ex_task(a, sh, down, ask));
             ds_commit();
             ask += gridDim.x;
             if (++slot == DS_DEPTH) slot = 0;
@@ -430,11 +429,11 @@ __device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, co
         if (!fresh) ds_pass(t, t.rest);
         else {
             item += gridDim.x;
-            if (item < n) t = ds_ex_task<DOWN>(a, sh, item);
+            if (item < n) t = ds_ex_task(a, sh, down, item);
         }
-        if (DOWN && item < n) ds_dn_acts(a, da, t, slot8);
-        if (multi && cur.n == 2) ds_ex_pass<DOWN, 2>(a, sh, red + place, xs, fn, w, cur, slot8);
-        else ds_ex_pass<DOWN, 1>(a, sh, red + place, xs, fn, w, cur, slot8);
+        if (down && item < n) ds_dn_acts(a, da, t, slot8);
+        if (multi && cur.n == 2) ds_ex_pass<2>(a, sh, down, red + place, xs, fn, w, cur, slot8);
+        else ds_ex_pass<1>(a, sh, down, red + place, xs, fn, w, cur, slot8);
         if (item >= n) break;
         place ^= HALF;
     }
@@ -448,9 +447,9 @@ __device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, co
 // the first 256 at the layer's start, the next ones while these are multiplied.  Lane (r = lane / 8, c = lane % 8)
 // multiplies dimensions 8c .. 8c + 7 of the keys 4i + r.
 constexpr int DS_KV = 16 * 256;                           // bytes of a warp's keys and values of one pass
-__device__ __forceinline__ void ds_kv_request(const DsArgs &a, const Shared &sh, const DsLayer &ly, uint8_t *kvs, int item, int blk)
+__device__ __forceinline__ void ds_kv_request(const DsArgs &a, const Shared &sh, const DsLayer &ly, uint8_t *kvs, int blk)
 {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, b = item / a.H, h = item - b * a.H, kvh = h / (a.H / a.KV);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, b = sh.ab, kvh = sh.akv;
     const int t = sh.pos[b], s0 = blk * 256 + warp * 16, left = t < 0 || t >= a.Tm ? 0 : t - s0, r = lane >> 3;
     if (left > 0) {
         const size_t base = ((size_t)b * a.Tm + s0) * a.KD + kvh * 64 + (lane & 7) * 8;
@@ -466,9 +465,8 @@ __device__ __forceinline__ void ds_kv_request(const DsArgs &a, const Shared &sh,
 }
 __device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const DsLayer &ly, uint8_t *kvs, uint8_t *slot)
 {
-    const int item = blockIdx.x;
-    if (item >= a.B * a.H) return;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, b = item / a.H, h = item - b * a.H, rep = a.H / a.KV, kvh = h / rep;
+    if ((int)blockIdx.x >= a.B * a.H) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, b = sh.ab, h = sh.ah, kvh = sh.akv;
     const int t = sh.pos[b], r = lane >> 3, c8 = (lane & 7) * 8, mm = tid >> 6, i64 = tid & 63;
     const bool bad = t < 0 || t >= a.Tm;                  // a slot past its cache: nothing of it is read or written
     float cs = 0.0f, sn = 0.0f;
@@ -508,18 +506,19 @@ __device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const 
         if (mm == 0) sh.q[i64] = __bfloat162float(xb);
         else {
             sh.kv[tid - 64] = xb;
-            if (h == kvh * rep) (mm == 1 ? ly.Kc : ly.Vc)[((size_t)b * a.Tm + t) * a.KD + kvh * 64 + i64] = xb;
+            if (sh.afirst) (mm == 1 ? ly.Kc : ly.Vc)[((size_t)b * a.Tm + t) * a.KD + kvh * 64 + i64] = xb;
         }
     }
     __syncthreads();
-    float m = -1e30f, l = 0.0f, o[8], q[8];
+    float m = -1e30f, l = 0.0f;
+    uint64_t o[4], q[4];                                  // pairs of neighbouring dimensions
 #pragma unroll
-    for (int d = 0; d < 8; d++) { o[d] = 0.0f; q[d] = sh.q[c8 + d]; }
+    for (int d = 0; d < 4; d++) { o[d] = 0ull; q[d] = ds_two(sh.q[c8 + 2 * d], sh.q[c8 + 2 * d + 1]); }
 #pragma unroll 1
     for (int blk = 0; blk * 256 <= t; blk++) {
         const int left = t - blk * 256 - warp * 16;       // this warp's keys 0 .. left of the pass, the last one new
         uint8_t *mine = kvs + (blk & 1) * DS_WARPS * DS_KV + warp * DS_KV;
-        if ((blk + 1) * 256 <= t) { ds_kv_request(a, sh, ly, kvs, item, blk + 1); ds_wait<1>(); }
+        if ((blk + 1) * 256 <= t) { ds_kv_request(a, sh, ly, kvs, blk + 1); ds_wait<1>(); }
         else ds_wait<0>();
         if (left < 0) continue;
         __syncwarp();                                     // a lane has waited for its own copies only, and row `left` is one's target
@@ -530,11 +529,8 @@ __device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const 
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const uint4 k = *reinterpret_cast<const uint4 *>(mine + i * 512 + lane * 16);
-            float d0 = q[0] * ds_lo(k.x), d1 = q[1] * ds_hi(k.x);
-            d0 = __fmaf_rn(q[2], ds_lo(k.y), d0); d1 = __fmaf_rn(q[3], ds_hi(k.y), d1);
-            d0 = __fmaf_rn(q[4], ds_lo(k.z), d0); d1 = __fmaf_rn(q[5], ds_hi(k.z), d1);
-            d0 = __fmaf_rn(q[6], ds_lo(k.w), d0); d1 = __fmaf_rn(q[7], ds_hi(k.w), d1);
-            d[i] = d0 + d1;
+            const float2 s = ds_apart(ds_fma2(q[3], ds_pair(k.w), ds_fma2(q[2], ds_pair(k.z), ds_fma2(q[1], ds_pair(k.y), ds_mul2(q[0], ds_pair(k.x))))));
+            d[i] = s.x + s.y;
         }
 #pragma unroll
         for (int y = 1; y < 8; y <<= 1)
@@ -549,17 +545,16 @@ __device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const 
         m = mn;
         l *= corr;
 #pragma unroll
-        for (int e = 0; e < 8; e++) o[e] *= corr;
+        for (int e = 0; e < 4; e++) o[e] = ds_mul2(o[e], ds_two(corr, corr));
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             if (4 * i + r <= left) {                      // (rows that were never copied must not meet a zero weight)
                 const float w = __expf(d[i] - mn);
                 const uint4 v = *reinterpret_cast<const uint4 *>(mine + 2048 + i * 512 + lane * 16);
+                const uint64_t ww = ds_two(w, w);
                 l += w;
-                o[0] = __fmaf_rn(w, ds_lo(v.x), o[0]); o[1] = __fmaf_rn(w, ds_hi(v.x), o[1]);
-                o[2] = __fmaf_rn(w, ds_lo(v.y), o[2]); o[3] = __fmaf_rn(w, ds_hi(v.y), o[3]);
-                o[4] = __fmaf_rn(w, ds_lo(v.z), o[4]); o[5] = __fmaf_rn(w, ds_hi(v.z), o[5]);
-                o[6] = __fmaf_rn(w, ds_lo(v.w), o[6]); o[7] = __fmaf_rn(w, ds_hi(v.w), o[7]);
+                o[0] = ds_fma2(ww, ds_pair(v.x), o[0]); o[1] = ds_fma2(ww, ds_pair(v.y), o[1]);
+                o[2] = ds_fma2(ww, ds_pair(v.z), o[2]); o[3] = ds_fma2(ww, ds_pair(v.w), o[3]);
             }
         }
         __syncwarp();                                     // before the keys after the next overwrite these
@@ -569,12 +564,15 @@ __device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const 
     for (int y = 8; y < 32; y <<= 1) {
         l += __shfl_xor_sync(0xffffffffu, l, y);
 #pragma unroll
-        for (int e = 0; e < 8; e++) o[e] += __shfl_xor_sync(0xffffffffu, o[e], y);
+        for (int e = 0; e < 4; e++) {
+            const float2 u = ds_apart(o[e]);
+            o[e] = ds_add2(o[e], ds_two(__shfl_xor_sync(0xffffffffu, u.x, y), __shfl_xor_sync(0xffffffffu, u.y, y)));
+        }
     }
     __syncthreads();                                      // part held the projections' sums
     if (r == 0) {
-        *reinterpret_cast<float4 *>(sh.part + warp * 64 + c8) = make_float4(o[0], o[1], o[2], o[3]);
-        *reinterpret_cast<float4 *>(sh.part + warp * 64 + c8 + 4) = make_float4(o[4], o[5], o[6], o[7]);
+        *reinterpret_cast<ulonglong2 *>(sh.part + warp * 64 + c8) = make_ulonglong2(o[0], o[1]);
+        *reinterpret_cast<ulonglong2 *>(sh.part + warp * 64 + c8 + 4) = make_ulonglong2(o[2], o[3]);
     }
     if (lane == 0) { sh.am[warp] = m; sh.al[warp] = l; }
     __syncthreads();
@@ -590,13 +588,19 @@ __device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const 
     }
 }
 
-// ---- rows: thread q < D / 4 owns columns 4q .. 4q + 3.  bf16 values in fp32 -> the normed bf16 row (and, for the router,
-// the same values as fp32 in xrow).  Every thread of the CTA takes part.
-__device__ __forceinline__ void ds_norm_store(const DsArgs &a, Shared &sh, const float4 x, const float *gamma, bf16 *dst, float *xrow)
+// ---- rows: thread q < D / 4 owns columns 4q .. 4q + 3
+//
+// this thread's columns of a gain, asked for before what the norm waits for
+__device__ __forceinline__ float4 ds_gain(const DsArgs &a, const float *gamma)
 {
     const int n = 4 * threadIdx.x;
-    float4 gm = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (n < a.D) gm = __ldg(reinterpret_cast<const float4 *>(gamma + n));
+    return n < a.D ? __ldg(reinterpret_cast<const float4 *>(gamma + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+// bf16 values in fp32 -> the normed bf16 row (and, for the router, the same values as fp32 in xrow).  Every thread of the
+// CTA takes part.
+__device__ __forceinline__ void ds_norm_store(const DsArgs &a, Shared &sh, const float4 x, const float4 gm, bf16 *dst, float *xrow)
+{
+    const int n = 4 * threadIdx.x;
     float ss = n < a.D ? x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w : 0.0f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -627,6 +631,7 @@ __device__ __forceinline__ void ds_router(const DsArgs &a, Shared &sh, const DsL
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, b = ds_row(a);
     if (b < 0) return;
+    const float4 gm = ds_gain(a, ly.an2);
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
     const int n = 4 * tid, ns = a.D / DS_ROWS;
     if (n < a.D) {
@@ -648,7 +653,7 @@ __device__ __forceinline__ void ds_router(const DsArgs &a, Shared &sh, const DsL
         x = ds_bf4(x);
         *reinterpret_cast<float4 *>(sh.x + n) = x;
     }
-    ds_norm_store(a, sh, x, ly.an2, reinterpret_cast<bf16 *>(slot + a.fnorm) + (size_t)b * a.D, xrow);
+    ds_norm_store(a, sh, x, gm, reinterpret_cast<bf16 *>(slot + a.fnorm) + (size_t)b * a.D, xrow);
     ds_wait<0>();
     __syncthreads();
     const int per = a.D / DS_WARPS, j0 = warp * per;      // a multiple of eight
@@ -675,7 +680,8 @@ __device__ __forceinline__ void ds_router(const DsArgs &a, Shared &sh, const DsL
             ly.rt[(size_t)b * a.E + lane] = lg;
         }
         int *asg = reinterpret_cast<int *>(slot + a.asg);
-        router_topk_row(lg, b, lane, ly.rprobs, ly.assign, ly.gate, a.B, a.E, a.K, nullptr, 0, [&](int at, int pick) { ds_put((void *)(asg + at), (uint32_t)pick); });
+        router_topk_row(lg, b, lane, ly.rprobs, ly.assign, ly.gate, a.B, a.E, a.K, nullptr, 0, 
+                        [&](int k, int pick, float g) { ds_put((void *)(asg + k * a.B + b), (uint32_t)pick); sh.gate[k] = g; });
     }
 }
 
@@ -689,7 +695,6 @@ __device__ __forceinline__ void ds_experts(const DsArgs &a, Shared &sh, bf16 *fn
             const int *p = reinterpret_cast<const int *>(slot + a.asg) + lane;
             ds_poll(a, [&] { e = (int)ds_get(p); return (uint32_t)e; });
             if ((unsigned)e >= (unsigned)a.E) e = 0;
-            sh.srow[lane] = lane % a.B;
         }
         __syncwarp();
         const unsigned m = __match_any_sync(0xffffffffu, e), lt = (1u << lane) - 1u;
@@ -706,14 +711,14 @@ __device__ __forceinline__ void ds_experts(const DsArgs &a, Shared &sh, bf16 *fn
 }
 
 // gate-weighted combination, residual, the next norm of a row
-__device__ __forceinline__ void ds_combine(const DsArgs &a, Shared &sh, const DsLayer &ly, float *ys, int l, uint8_t *slot)
+__device__ __forceinline__ void ds_combine(const DsArgs &a, Shared &sh, float *ys, int l, uint8_t *slot)
 {
     const int b = ds_row(a);
     if (b < 0) return;
     const int c = 4 * threadIdx.x;
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c < a.D) x = *reinterpret_cast<const float4 *>(sh.x + c);
-    if ((int)threadIdx.x < a.K) sh.red[threadIdx.x] = __ldcg(ly.gate + (size_t)threadIdx.x * a.B + b);    // K <= 16
+    const float4 gm = ds_gain(a, l + 1 < a.L ? sh.layer[(l + 1) & 1].an1 : a.nf);
     const int half = threadIdx.x >> 8, n = 4 * (threadIdx.x & 255), R = a.K * a.B, ns = a.F / DS_ROWS;
     if (n < a.D) {
 #pragma unroll 1
@@ -740,13 +745,11 @@ __device__ __forceinline__ void ds_combine(const DsArgs &a, Shared &sh, const Ds
     __syncthreads();
     if (c < a.D) {
 #pragma unroll 1
-        for (int k = 0; k < a.K; k++) ds_fma4(x, sh.red[k], *reinterpret_cast<const float4 *>(ys + k * a.D + c));
+        for (int k = 0; k < a.K; k++) ds_fma4(x, sh.gate[k], *reinterpret_cast<const float4 *>(ys + k * a.D + c));
         x = ds_bf4(x);
         *reinterpret_cast<float4 *>(sh.x + c) = x;
     }
-    __syncthreads();                                      // red held the gates
-    if (l + 1 < a.L) ds_norm_store(a, sh, x, sh.layer[(l + 1) & 1].an1, reinterpret_cast<bf16 *>(slot) + (size_t)b * a.D, nullptr);
-    else ds_norm_store(a, sh, x, a.nf, a.fn + (size_t)b * a.D, nullptr);
+    ds_norm_store(a, sh, x, gm, (l + 1 < a.L ? reinterpret_cast<bf16 *>(slot) : a.fn) + (size_t)b * a.D, nullptr);
 }
 
 // C rows per task of the dense phases; MULTI: an expert can have more than one slot
@@ -762,6 +765,11 @@ __global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constan
             reinterpret_cast<unsigned long long *>(&sh.layer[l & 1])[threadIdx.x] = __ldg(reinterpret_cast<const unsigned long long *>(a.layers + l) + threadIdx.x);
     };
     load_layer(0);
+    if (threadIdx.x == 0) {
+        const int rep = a.H / a.KV, b = (int)blockIdx.x / a.H, h = (int)blockIdx.x - b * a.H;
+        sh.ab = b; sh.ah = h; sh.akv = h / rep; sh.afirst = h % rep == 0;
+    }
+    if (threadIdx.x < DS_MAX_R) sh.srow[threadIdx.x] = (int)threadIdx.x % a.B;
     if (threadIdx.x < DS_MAX_B) sh.pos[threadIdx.x] = (int)threadIdx.x < a.B ? __ldg(a.pos + threadIdx.x) : 0;
     // Every CTA looks the whole table over (2 KB from L2, beside the loads above): a pointer that is missing or not aligned
     // for its loads is reported, and the whole grid leaves before its first barrier.
@@ -791,35 +799,42 @@ __global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constan
             x = ds_bf4(__ldg(reinterpret_cast<const float4 *>(a.emb + (size_t)__ldg(a.tok + b) * a.D + n)));
             *reinterpret_cast<float4 *>(sh.x + n) = x;
         }
-        ds_norm_store(a, sh, x, sh.layer[0].an1, reinterpret_cast<bf16 *>(prev) + (size_t)b * a.D, nullptr);
+        ds_norm_store(a, sh, x, ds_gain(a, sh.layer[0].an1), reinterpret_cast<bf16 *>(prev) + (size_t)b * a.D, nullptr);
     }
 #pragma unroll 1
     for (int l = 0; l < a.L; l++) {
         const DsLayer &ly = sh.layer[l & 1];
         __syncthreads();
         if (l + 1 < a.L) load_layer(l + 1);               // every thread is past the layer before: the other half is free
-        if ((int)blockIdx.x < a.B * a.H) ds_kv_request(a, sh, ly, dsm + DS_RED, blockIdx.x, 0);
+        if ((int)blockIdx.x < a.B * a.H) ds_kv_request(a, sh, ly, dsm + DS_RED, 0);
         else if (ds_row(a) >= 0) ds_wr_request(a, ly, wr);
         if (l > 0) {                                      // (every path to a store or a poll of this layer's slot has a barrier of the CTA on it)
             gate += gridDim.x;
             if (threadIdx.x == DS_THREADS - 1) gb_wait(a, gate);
         }
-        ds_dense<0, C>(a, ly, red, prev, cur);
-        __syncthreads();
-        ds_clear(after, a.slot_bytes);
-        ds_attention(a, sh, ly, dsm + DS_RED, cur);
-        __syncthreads();
-        ds_dense<1, C>(a, ly, red, cur + a.att, cur);
-        __syncthreads();
+        // The two dense phases and the two of the experts are one body of code each with several slots: with a body of
+        // their own, 122 KB of instructions went through the instruction cache every layer (eight slots 433 us, 418 so).
+        // With one slot, where less code is run, the body of their own is the faster one (204 and 199 us).
+        constexpr int TWICE = MULTI ? 1 : 2;
+#pragma unroll TWICE
+        for (int wo = 0; wo < 2; wo++) {
+            ds_dense<C>(a, ly, red, wo, wo ? cur + a.att : prev, cur);
+            __syncthreads();
+            if (wo) break;
+            ds_clear(after, a.slot_bytes);
+            ds_attention(a, sh, ly, dsm + DS_RED, cur);
+            __syncthreads();
+        }
         if (l + 1 < a.L && threadIdx.x == DS_THREADS - 1) gb_arrive(a);
         ds_router(a, sh, ly, wr, red, cur);
         __syncthreads();
         ds_experts(a, sh, fn, cur);
-        ds_experts_phase<false>(a, sh, ly, red, xs, fn, dsm + DS_RED, MULTI, cur);
-        __syncthreads();
-        ds_experts_phase<true>(a, sh, ly, red, xs, fn, dsm + DS_RED, MULTI, cur);
-        __syncthreads();
-        ds_combine(a, sh, ly, red, l, cur);
+#pragma unroll TWICE
+        for (int down = 0; down < 2; down++) {
+            ds_experts_phase(a, sh, down, ly, red, xs, fn, dsm + DS_RED, MULTI, cur);
+            __syncthreads();
+        }
+        ds_combine(a, sh, red, l, cur);
         uint8_t *p = prev;
         prev = cur; cur = after; after = p;
     }

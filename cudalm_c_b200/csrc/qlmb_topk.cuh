@@ -34,8 +34,8 @@ __device__ __forceinline__ unsigned order_key(float f)
     return (u & 0x80000000u) ? ~u : u | 0x80000000u;
 }
 // the softmax and the K selection rounds of token n by one warp; lg = the logit of expert `lane` (0 beyond E).  Lane 0
-// hands every choice, with its place in the assign table, to tell() besides.
-struct TellNobody { __device__ void operator()(int, int) const {} };
+// hands every round's choice and its gate to tell() besides.
+struct TellNobody { __device__ void operator()(int, int, float) const {} };
 template <typename Tell = TellNobody>
 __device__ __forceinline__ void router_topk_row(float lg, int n, int lane, float *rprobs, int *assign, float *gate, int N,
                                                 int E, int K, const float *bias, int bs, Tell tell = Tell())
@@ -59,7 +59,7 @@ __device__ __forceinline__ void router_topk_row(float lg, int n, int lane, float
         const unsigned best = __reduce_max_sync(0xffffffffu, key);
         const int pick = best ? __ffs(__ballot_sync(0xffffffffu, key == best)) - 1 : k;    // lowest index on ties; NaN scores: stay in range
         float g = __shfl_sync(0xffffffffu, pr, pick);
-        if (lane == 0) { assign[(size_t)k * N + n] = pick; gate[(size_t)k * N + n] = g; tell(k * N + n, pick); }
+        if (lane == 0) { assign[(size_t)k * N + n] = pick; gate[(size_t)k * N + n] = g; tell(k, pick, g); }
         taken = taken || (lane == pick);
     }
 }
