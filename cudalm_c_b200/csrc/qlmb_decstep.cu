@@ -1,4 +1,4 @@
-// One decode step's layers in ONE persistent launch (dec_step, cudalm.cu:7168-7212), up to eight live slots: embedding, then
+// One decode step's layers in ONE persistent launch (dec_step, cudalm.cu:7168-7212), up to 32 routed slots: embedding, then
 // per layer the q, k, v projections with the norm in front, cached attention, output projection + residual + norm,
 // router, the routed experts and their combination, and the final norm.  With so few rows a layer is 5 MB of weights,
 // which the memory system delivers in under a microsecond; what a step costs is latency: the chain of launches that
@@ -18,7 +18,7 @@
 // Products are fp32: x * scale times the exact digit, as in the kernels of the separate entry points.
 // Measured (12 layers, D 768, 32 experts top-2 of d_ff 1536, 128-256 cached positions, whole step with the head, a CUDA
 // graph replay): one slot 276 us with grid barriers, 199 now, eight slots 477 and 415 (the chain of launches: 615 and
-// 801).  Above eight slots the chain stays: there the experts' weights are a stream and no longer a latency.
+// 801).  Where the form ends stands at ds_fits: with many slots the experts' weights are a stream and no longer a latency.
 //
 // Built with --fmad=false (router arithmetic); fused multiply-adds are written out.
 #include <cuda_bf16.h>
@@ -59,14 +59,15 @@ struct DsArgs {
 constexpr int DS_THREADS = 512, DS_WARPS = 16;
 constexpr int DS_ROWS = 128;                              // contraction rows of a task: eight per warp
 constexpr int DS_COLS = 256;
-constexpr int DS_MAX_B = 8, DS_MAX_R = 32;
+constexpr int DS_MAX_B = 32, DS_MAX_R = 32;
 constexpr int DS_MAX_SL = 8;                              // row slices of D (D <= 1024)
 constexpr int DS_RED = DS_WARPS * 4 * DS_COLS * 4;        // up to four rows' sums of the 16 warps
 constexpr int DS_WR = 1024 * 32 * 4;                      // the router's matrix, or keys and values of an attention phase
 constexpr int DS_XS = 2 * DS_ROWS * 4;
-constexpr int DS_FN = DS_MAX_B * 1024 * 2;                // the rows that the experts take
+constexpr int DS_FN = 16384;                              // the rows that the experts take: this and what the ring leaves of DS_WR
 constexpr int DS_SLOT = DS_ROWS * 136, DS_DEPTH = 7;      // a task's codes and scales; tasks on their way (in the place of DS_WR)
-static_assert(DS_DEPTH * DS_SLOT <= DS_WR, "ring");
+static_assert(DS_DEPTH * DS_SLOT <= DS_WR && DS_DEPTH * DS_SLOT % 16 == 0, "ring");
+constexpr int DS_FN_ELEMS = (DS_WR - DS_DEPTH * DS_SLOT + DS_FN) / 2;
 constexpr int DS_SMEM = DS_RED + DS_WR + DS_XS + DS_FN;
 
 __device__ __forceinline__ uint32_t ds_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -463,9 +464,13 @@ __device__ __forceinline__ void ds_kv_request(const DsArgs &a, const Shared &sh,
     }
     ds_commit();
 }
-__device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const DsLayer &ly, uint8_t *kvs, uint8_t *slot)
+__device__ __forceinline__ void ds_item(const DsArgs &a, Shared &sh, int item)      // by one thread
 {
-    if ((int)blockIdx.x >= a.B * a.H) return;
+    const int rep = a.H / a.KV, b = item / a.H, h = item - b * a.H;
+    sh.ab = b; sh.ah = h; sh.akv = h / rep; sh.afirst = h % rep == 0;
+}
+__device__ __forceinline__ void ds_attention_item(const DsArgs &a, Shared &sh, const DsLayer &ly, uint8_t *kvs, uint8_t *slot)
+{
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, b = sh.ab, h = sh.ah, kvh = sh.akv;
     const int t = sh.pos[b], r = lane >> 3, c8 = (lane & 7) * 8, mm = tid >> 6, i64 = tid & 63;
     const bool bad = t < 0 || t >= a.Tm;                  // a slot past its cache: nothing of it is read or written
@@ -617,8 +622,28 @@ __device__ __forceinline__ void ds_norm_store(const DsArgs &a, Shared &sh, const
     }
 }
 
-// The rows' owners are the last CTAs, which have no attention item: what they need besides sums (the router's matrix)
-// waits in shared memory since the layer's start.
+// the CTA's items: one as a rule, whose first keys and values were asked for at the layer's start
+__device__ __forceinline__ void ds_attention(const DsArgs &a, Shared &sh, const DsLayer &ly, uint8_t *kvs, uint8_t *slot)
+{
+    const int n = a.B * a.H;
+#pragma unroll 1
+    for (int item = blockIdx.x; item < n; item += gridDim.x) {
+        if (item != (int)blockIdx.x) {
+            __syncthreads();
+            if (threadIdx.x == 0) ds_item(a, sh, item);
+            __syncthreads();
+            ds_kv_request(a, sh, ly, kvs, 0);
+        }
+        ds_attention_item(a, sh, ly, kvs, slot);
+    }
+    if ((int)(blockIdx.x + gridDim.x) < n) {              // back to the first one, for the next layer
+        __syncthreads();
+        if (threadIdx.x == 0) ds_item(a, sh, blockIdx.x);
+    }
+}
+
+// The rows' owners are the last CTAs, which have no attention item with few slots: what they need besides sums (the
+// router's matrix) waits in shared memory since the layer's start then, since the attention's end else.
 __device__ __forceinline__ int ds_row(const DsArgs &a) { const int b = (int)gridDim.x - 1 - (int)blockIdx.x; return b < a.B ? b : -1; }
 __device__ __forceinline__ void ds_wr_request(const DsArgs &a, const DsLayer &ly, float *wr)
 {
@@ -752,23 +777,22 @@ __device__ __forceinline__ void ds_combine(const DsArgs &a, Shared &sh, float *y
     ds_norm_store(a, sh, x, gm, (l + 1 < a.L ? reinterpret_cast<bf16 *>(slot) : a.fn) + (size_t)b * a.D, nullptr);
 }
 
-// C rows per task of the dense phases; MULTI: an expert can have more than one slot
-template <int C, bool MULTI>
+// C rows per task of the dense phases; MULTI: an expert can have more than one slot; MANY: a CTA more than one attention
+// item, or an item and a row (its loop around the attention costs the others 1 %)
+template <int C, bool MULTI, bool MANY>
 __global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constant__ DsArgs a)
 {
     extern __shared__ __align__(128) uint8_t dsm[];
     __shared__ Shared sh;
-    float *red = reinterpret_cast<float *>(dsm), *wr = reinterpret_cast<float *>(dsm + DS_RED), *xs = reinterpret_cast<float *>(dsm + DS_RED + DS_WR);
-    bf16 *fn = reinterpret_cast<bf16 *>(dsm + DS_RED + DS_WR + DS_XS);
+    float *red = reinterpret_cast<float *>(dsm), *wr = reinterpret_cast<float *>(dsm + DS_RED), *xs = reinterpret_cast<float *>(dsm + DS_RED + DS_WR + DS_FN);
+    bf16 *fn = reinterpret_cast<bf16 *>(dsm + DS_RED + DS_DEPTH * DS_SLOT);
+    const bool attends = (int)blockIdx.x < a.B * a.H, owns = ds_row(a) >= 0;
     auto load_layer = [&](int l) {
         if (threadIdx.x < DS_LAYER_WORDS)
             reinterpret_cast<unsigned long long *>(&sh.layer[l & 1])[threadIdx.x] = __ldg(reinterpret_cast<const unsigned long long *>(a.layers + l) + threadIdx.x);
     };
     load_layer(0);
-    if (threadIdx.x == 0) {
-        const int rep = a.H / a.KV, b = (int)blockIdx.x / a.H, h = (int)blockIdx.x - b * a.H;
-        sh.ab = b; sh.ah = h; sh.akv = h / rep; sh.afirst = h % rep == 0;
-    }
+    if (threadIdx.x == 0) ds_item(a, sh, blockIdx.x);
     if (threadIdx.x < DS_MAX_R) sh.srow[threadIdx.x] = (int)threadIdx.x % a.B;
     if (threadIdx.x < DS_MAX_B) sh.pos[threadIdx.x] = (int)threadIdx.x < a.B ? __ldg(a.pos + threadIdx.x) : 0;
     // Every CTA looks the whole table over (2 KB from L2, beside the loads above): a pointer that is missing or not aligned
@@ -780,7 +804,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constan
     }
     if (bad && blockIdx.x == 0) report_bad_index(a.errword, 304, (bad - 1) / DS_LAYER_WORDS, (bad - 1) % DS_LAYER_WORDS);
     if (__syncthreads_or(bad)) return;
-    const unsigned shape0 = 1u + (unsigned)(a.B | a.D << 4 | a.KD << 15 | a.K << 26), shape1 = (unsigned)a.F;   // never 0; the last CTA writes them
+    const unsigned shape0 = 1u + (unsigned)(a.B | a.D / 128 << 6 | a.KD / 64 << 10 | a.K << 15), shape1 = (unsigned)a.F;   // never 0; the last CTA writes them
     const unsigned next = __ldcg(a.bar + 3);
     unsigned gate = 0;                                    // arrivals that the next wait for the grid needs
     if (__ldcg(a.bar + 4) != shape0 || __ldcg(a.bar + 5) != shape1) {
@@ -792,7 +816,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constan
     }
     // slots of the layer before, this one and the one after
     uint8_t *prev = a.slots + (next == 0 ? 2u : next - 1u) * a.slot_bytes, *cur = a.slots + next * a.slot_bytes, *after = a.slots + (next == 2 ? 0u : next + 1u) * a.slot_bytes;
-    if (ds_row(a) >= 0) {                                 // embedding row and the first norm
+    if (owns) {                                           // embedding row and the first norm
         const int b = ds_row(a), n = 4 * threadIdx.x;
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
         if (n < a.D) {
@@ -806,8 +830,8 @@ __global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constan
         const DsLayer &ly = sh.layer[l & 1];
         __syncthreads();
         if (l + 1 < a.L) load_layer(l + 1);               // every thread is past the layer before: the other half is free
-        if ((int)blockIdx.x < a.B * a.H) ds_kv_request(a, sh, ly, dsm + DS_RED, 0);
-        else if (ds_row(a) >= 0) ds_wr_request(a, ly, wr);
+        if (attends) ds_kv_request(a, sh, ly, dsm + DS_RED, 0);
+        else if (owns) ds_wr_request(a, ly, wr);
         if (l > 0) {                                      // (every path to a store or a poll of this layer's slot has a barrier of the CTA on it)
             gate += gridDim.x;
             if (threadIdx.x == DS_THREADS - 1) gb_wait(a, gate);
@@ -822,8 +846,10 @@ __global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constan
             __syncthreads();
             if (wo) break;
             ds_clear(after, a.slot_bytes);
-            ds_attention(a, sh, ly, dsm + DS_RED, cur);
+            if (MANY) ds_attention(a, sh, ly, dsm + DS_RED, cur);
+            else if (attends) ds_attention_item(a, sh, ly, dsm + DS_RED, cur);
             __syncthreads();
+            if (MANY && attends && owns) ds_wr_request(a, ly, wr);
         }
         if (l + 1 < a.L && threadIdx.x == DS_THREADS - 1) gb_arrive(a);
         ds_router(a, sh, ly, wr, red, cur);
@@ -868,11 +894,17 @@ static DsLayout ds_layout(int B, int D, int KD, int F, int K)
     w.bytes = 256 + 3 * cur;
     return w;
 }
+// Above eight slots (six layers, us a step, this form and the chain): nine slots of D 768, 32 experts of 1536, two choices
+// 243 and 361, sixteen 336 and 394 (379 and 485 with 900 cached positions); sixteen of D 256, eight experts of 512 140 and
+// 238; 32 slots of D 256 with one choice of 32 or eight experts 180 and 293, 178 and 286.  With experts of many slots the
+// chain takes sixteen of an expert's rows to the tensor cores at a time, a pass here two: up to four slots per expert, and
+// up to 50 M products a matrix of all slots (four layers, twelve slots of D 1024, eight experts top-2: d_ff 2048, 50 M, 253
+// and 278; d_ff 4096, 100 M, 367 and 301).
 static bool ds_fits(int B, int Tm, int D, int H, int KV, int F, int E, int K)
 {
     return B >= 1 && B <= DS_MAX_B && Tm >= 1 && Tm <= 4096 && D == H * 64 && D % 128 == 0 && D <= 1024 && KV >= 1 && H % KV == 0 &&
            (KV * 64) % 128 == 0 && F >= 128 && F % 128 == 0 && E >= 1 && E <= 32 && K >= 1 && K <= E && K * B <= DS_MAX_R && K <= DS_WARPS && K * D * 4 <= DS_RED &&
-           B * (H + 1) <= sm_count();                     // a CTA has an attention item or owns a row
+           B * D <= DS_FN_ELEMS && (B <= 8 ? B * (H + 1) <= sm_count() : B <= sm_count() && K * B <= 4 * E && (size_t)K * B * D * F <= (size_t)48 << 20);
 }
 
 }  // namespace qlmb
@@ -912,13 +944,15 @@ extern "C" int qlmb_dec_step(const qlmb_dec_step_args *p, void *stream)
     // rows per task of the dense phases: the fewest with which the q, k, v tasks are one round of the device
     int c = 1;
     while (c < 4 && a.tq * (a.D / DS_ROWS) * ((p->B + c - 1) / c) > sm_count()) c *= 2;
-    const int v = p->B == 1 ? 0 : c == 1 ? 1 : c == 2 ? 2 : 3;
-    const void *kern = v == 0 ? (const void *)k_dec_step<1, false> : v == 1 ? (const void *)k_dec_step<1, true>
-                     : v == 2 ? (const void *)k_dec_step<2, true> : (const void *)k_dec_step<4, true>;
+    const void *kerns[7] = {(const void *)k_dec_step<1, false, false>, (const void *)k_dec_step<1, true, false>, (const void *)k_dec_step<2, true, false>,
+                            (const void *)k_dec_step<4, true, false>, (const void *)k_dec_step<1, true, true>, (const void *)k_dec_step<2, true, true>,
+                            (const void *)k_dec_step<4, true, true>};
+    const int v = p->B == 1 ? 0 : (c == 1 ? 1 : c == 2 ? 2 : 3) + (p->B > 8 ? 3 : 0);
+    const void *kern = kerns[v];
     int dev = 0;
     QLMB_CUDA(cudaGetDevice(&dev));
     QLMB_REQUIRE(dev >= 0 && dev < 64, "device index %d", dev);
-    static bool attr_done[64][4];
+    static bool attr_done[64][7];
     if (!attr_done[dev][v]) {
         QLMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DS_SMEM));
         attr_done[dev][v] = true;

@@ -283,9 +283,10 @@ int qlmb_gemv_decode(void *Y, const void *X, const int8_t *codes, const float *s
  * caches must be 16-byte aligned, the others 4; a row that breaks this is reported through the device error word (site
  * 304) and the step does nothing.  emb, nf and fn must be 16-byte aligned, the table 8.  ws = qlmb_dec_step_bytes(...)
  * bytes, 256-byte aligned, zeroed once before its first use, not shared by steps that may overlap; a size of 0 means that
- * the shape is not supported (supported: head dimension 64, D <= 1024, at most 8 slots, 32 experts and 32 routed slots, a
- * CTA per attention item and row on the device) and the separate entry points do the step.  A slot whose position is
- * outside its cache is reported and neither read nor written. */
+ * the shape is not supported and the separate entry points do the step.  Supported: head dimension 64, D <= 1024, at most
+ * 32 experts and 32 routed slots (K*B); up to 8 slots with a CTA per attention item and row on the device; above 8 slots
+ * with B*D <= 12800, K*B <= 4*E and K*B*D*F <= 48 * 2^20.  A slot whose position is outside its cache is reported and neither
+ * read nor written. */
 typedef struct qlmb_dec_step_args {
     int B, Tm, L, D, H, KV, F, E, K;
     const void *layers;

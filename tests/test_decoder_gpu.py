@@ -380,6 +380,68 @@ def test_one_launch_step_equals_the_chain(cuda, B, D, KV, E, K, F, fill, Tm):
         assert ((t != b).flatten(2).any(-1).sum(1) <= 1).all()              # at most the slot's own row changed
 
 
+@pytest.mark.parametrize("B,D,KV,E,K,F,fill,Tm", [
+    (9, 768, 12, 32, 2, 1536, 255, 640),    # the smallest; an attention item per CTA
+    (12, 1024, 16, 32, 2, 640, 20, 64),     # two items of a CTA, rows' owners among them; nearly all of the rows' room
+    (16, 640, 10, 8, 2, 384, 600, 640),     # 32 routed slots, four of each expert, several passes of keys
+    (32, 256, 2, 8, 1, 128, 40, 64),        # one choice a slot; grouped heads
+])
+def test_one_launch_step_of_more_slots_equals_the_chain(cuda, B, D, KV, E, K, F, fill, Tm):
+    """The same above eight slots, where the attention's items outnumber the CTAs or share them with the rows' owners."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import model
+    from cudalm_c_b200._lib import stream_ptr
+    cfg = model.Config(L=2, D=D, H=D // 64, KV=KV, hd=64, E=E, K=K, F=F, V=512, T=max(fill, 64), B=1)
+    m = model.QlmModel(cfg, cuda, seed=3)
+    d = model.Decoder(m, B, Tm)
+    g = torch.Generator(device=cuda); g.manual_seed(B)
+    d.prefill(torch.randint(0, cfg.V, (B, fill), generator=g, dtype=torch.int32, device=cuda))
+    pos = torch.randint((fill + 1) // 2, fill + 1, (B,), generator=g, dtype=torch.int32, device=cuda)
+    pos[0] = fill
+    d.pos2.copy_(pos.repeat(2))
+    plan = d._step_plan()
+    assert plan is not None
+    before = [t.clone() for t in d.K + d.V]
+    want = d._layers_chain().float()
+    chain = [(mo.member("assign", (K, B), torch.int32).clone(), mo.member("rt", (B, E), torch.float32).clone()) for mo in d.moes]
+    caches = [t.clone() for t in d.K + d.V]
+    for t, b in zip(d.K + d.V, before):
+        t.copy_(b)
+    outs = []
+    for _ in range(3):
+        q.check(q.lib().qlmb_dec_step(plan, stream_ptr()))
+        outs.append(d.fn.float().clone())
+    torch.cuda.synchronize()
+    q.check(q.lib().qlmb_check_device(None))
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    # the bound of the test above, 2e-2 of the norm, for the slots with the same experts.  A slot may differ from the first
+    # layer on where two of its logits are nearer than their noise: 5e-3 of a logit's root mean square each (the same
+    # roundings), sqrt(2) for a difference, times four
+    same = torch.ones(B, dtype=torch.bool, device=cuda)
+    for (e, rt), mo in zip(chain, d.moes):
+        now = (e == mo.member("assign", (K, B), torch.int32)).all(0)
+        top = rt.sort(dim=1, descending=True).values[:, :K + 1]
+        gap = (top[:, :-1] - top[:, 1:]).min(1).values / rt.pow(2).mean(1).sqrt()
+        assert bool((now | ~same | (gap < 4 * 2 ** 0.5 * 5e-3)).all()), gap[~now].tolist()
+        same &= now
+    assert int(same.sum()) >= B // 2
+    err = (outs[0] - want).norm(dim=1) / want.norm(dim=1)
+    assert float(err[same].max()) < 2e-2, err.tolist()
+    for i, (t, c, b) in enumerate(zip(d.K + d.V, caches, before)):
+        keep = same if i % cfg.L else torch.ones_like(same)                     # the first layer's rows come before any router
+        assert float((t.float() - c.float())[keep].abs().max()) < 2e-2
+        assert ((t != b).flatten(2).any(-1).sum(1) <= 1).all()              # at most the slot's own row changed
+
+
+def test_shapes_of_the_one_launch_step(cuda):
+    """Above eight slots the form is left to shapes with few slots per expert, moderate experts and rows that shared memory holds."""
+    import cudalm_c_b200 as q
+    takes = [bool(q.lib().qlmb_dec_step_bytes(B, 64, D, D // 64, D // 64, F, E, K))
+             for B, D, F, E, K in ((8, 1024, 8192, 8, 4), (9, 1024, 256, 8, 2), (12, 1024, 2048, 8, 2), (12, 1024, 2176, 8, 2), (13, 1024, 256, 32, 2),
+                                   (16, 768, 256, 8, 2), (16, 768, 256, 7, 2), (17, 512, 256, 32, 2), (32, 256, 256, 8, 1), (33, 256, 256, 32, 1))]
+    assert takes == [True, True, True, False, False, True, False, False, True, False]
+
+
 @pytest.mark.parametrize("L", [1, 2, 3, 4])
 def test_one_launch_steps_in_a_row_and_a_workspace_of_several_shapes(cuda, L):
     """What the CTAs hand to one another lies in three slots used in turn across layers and launches, whatever the number of
