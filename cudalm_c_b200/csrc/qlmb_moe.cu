@@ -16,7 +16,7 @@ namespace qlmb {
 
 struct Arena {
     size_t rows_cap;     // padded row capacity
-    float *rt, *rprobs, *gate, *d_gate, *drt, *wr_scratch, *wrt;
+    float *rt, *rprobs, *gate, *d_gate, *drt, *wr_scratch;
     int *assign, *perm, *inv, *off, *counts, *tile_info, *ntiles, *bad, *chunk;
     bf16 *Xp, *gp, *up, *ap, *yp, *dyp, *dgp, *dup, *dXp;
     size_t bytes;
@@ -45,7 +45,6 @@ static Arena carve(void *base, int N, int D, int F, int E, int K)
     MEMBER(d_gate, float, KN);
     MEMBER(drt, float, (size_t)N * E);
     MEMBER(wr_scratch, float, (size_t)192 * D * E);
-    MEMBER(wrt, float, (size_t)D * E);
     MEMBER(assign, int, KN);
     MEMBER(perm, int, R);
     MEMBER(inv, int, KN);
