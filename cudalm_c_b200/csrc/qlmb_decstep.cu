@@ -1,4 +1,4 @@
-// One decode step's layers in ONE persistent launch (dec_step, cudalm.cu:7168-7212), up to 32 routed slots: embedding, then
+// One decode step's layers in ONE persistent launch (dec_step, cudalm.cu:7168-7212), up to 64 routed slots: embedding, then
 // per layer the q, k, v projections with the norm in front, cached attention, output projection + residual + norm,
 // router, the routed experts and their combination, and the final norm.  With so few rows a layer is 5 MB of weights,
 // which the memory system delivers in under a microsecond; what a step costs is latency: the chain of launches that
@@ -59,7 +59,7 @@ struct DsArgs {
 constexpr int DS_THREADS = 512, DS_WARPS = 16;
 constexpr int DS_ROWS = 128;                              // contraction rows of a task: eight per warp
 constexpr int DS_COLS = 256;
-constexpr int DS_MAX_B = 32, DS_MAX_R = 32;
+constexpr int DS_MAX_B = 32, DS_MAX_R = 64;
 constexpr int DS_MAX_SL = 8;                              // row slices of D (D <= 1024)
 constexpr int DS_RED = DS_WARPS * 4 * DS_COLS * 4;        // up to four rows' sums of the 16 warps
 constexpr int DS_WR = 1024 * 32 * 4;                      // the router's matrix, or keys and values of an attention phase
@@ -93,8 +93,8 @@ __device__ __forceinline__ void ds_fma4(float4 &a, float g, const float4 b)
 struct Shared {
     DsLayer layer[2];
     int pos[DS_MAX_B];
-    int npair, pexp[DS_MAX_R];                            // distinct experts of the step and their slots
-    unsigned pmask[DS_MAX_R];
+    int npair, pexp[DS_MAX_R];                            // distinct experts of slots 0 .. 31 and of 32 .. 63 (expert | half << 8),
+    unsigned pmask[DS_MAX_R];                             // and their slots
     int srow[DS_MAX_R];                                   // the row of a slot
     int ab, ah, akv, afirst;                                      // the CTA's attention item: slot, head, key/value head
     float red[DS_WARPS];
@@ -283,16 +283,16 @@ __device__ __forceinline__ void ds_dense(const DsArgs &a, const DsLayer &ly, flo
 
 // The experts' tasks.  An expert has one or two slots as a rule: a pass multiplies up to two, and the weights, the first
 // pass's activations and, in the down projection, the gate and up sums they are made of are requested a task ahead.
-struct ExTask { int pair, mat, slice, tile, s0, s1, n; unsigned rest; };     // s0, s1: the pass's slots (n of them), rest: those that follow
+struct ExTask { int pair, mat, slice, tile, base, s0, s1, n; unsigned rest; };     // s0, s1: the pass's slots (n of them), rest: those that follow, of base on
 __device__ __forceinline__ void ds_pass(ExTask &t, unsigned mask)
 {
-    t.s0 = __ffs(mask) - 1;
+    t.s0 = t.base + __ffs(mask) - 1;
     mask &= mask - 1;
     t.n = mask ? 2 : 1;
-    t.s1 = mask ? __ffs(mask) - 1 : t.s0;
+    t.s1 = mask ? t.base + __ffs(mask) - 1 : t.s0;
     t.rest = mask & (mask - 1);
 }
-__device__ __forceinline__ ExTask ds_ex_task(const DsArgs &a, const Shared &sh, bool down, int item)
+__device__ __forceinline__ ExTask ds_ex_task(const DsArgs &a, const Shared &sh, bool down, bool many, int item)
 {
     ExTask t;
     if (down) {
@@ -306,6 +306,7 @@ __device__ __forceinline__ ExTask ds_ex_task(const DsArgs &a, const Shared &sh, 
         t.slice = q - pm * sl;
         t.mat = pm & 1; t.pair = pm >> 1;
     }
+    t.base = many ? sh.pexp[t.pair] >> 8 << 5 : 0;
     ds_pass(t, sh.pmask[t.pair]);
     return t;
 }
@@ -314,7 +315,7 @@ __device__ __forceinline__ ExTask ds_ex_task(const DsArgs &a, const Shared &sh, 
 __device__ __forceinline__ void ds_ex_request(const DsArgs &a, const Shared &sh, bool down, const DsLayer &ly, uint8_t *ring, int slot, const ExTask &t)
 {
     const int N = down ? a.D : a.F, m = down ? 6 : 4 + t.mat, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t mat = (size_t)sh.pexp[t.pair] * a.D * a.F;
+    const size_t mat = (size_t)(sh.pexp[t.pair] & 255) * a.D * a.F;
     const int k0 = t.slice * DS_ROWS + warp * 8, r = lane >> 3, c = lane & 7;
     const uint32_t d = ds_smem(ring + slot * DS_SLOT);
     const bool in = t.tile * DS_COLS + c * 32 < N;        // N is a multiple of 128: the last tile may be half as wide
@@ -379,18 +380,18 @@ __device__ __forceinline__ void ds_ex_pass(const DsArgs &a, const Shared &sh, bo
     ds_reduce<C>(red, acc, t.n, t.tile * DS_COLS, N, [&](int c) { return out + (size_t)(c == 0 ? t.s0 : t.s1) * N; });
 }
 // The down projection's choice of weights is known: its sums are waited for with the first tasks' weights on their way.
-__device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, bool down, const DsLayer &ly, float *red, float *xs, const bf16 *fn, uint8_t *ring, bool multi, uint8_t *slot8)
+__device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, bool down, const DsLayer &ly, float *red, float *xs, const bf16 *fn, uint8_t *ring, bool multi, bool many, uint8_t *slot8)
 {
     const int n = down ? sh.npair * (a.F / DS_ROWS) * a.td : sh.npair * 2 * (a.D / DS_ROWS) * a.tf;
     int ask = blockIdx.x, item = blockIdx.x, slot = 0;
 #pragma unroll 1
     for (int k = 0; k < DS_DEPTH; k++) {
-        if (ask < n) ds_ex_request(a, sh, down, ly, ring, k, ds_ex_task(a, sh, down, ask));
+        if (ask < n) ds_ex_request(a, sh, down, ly, ring, k, ds_ex_task(a, sh, down, many, ask));
         ds_commit();
         ask += gridDim.x;
     }
     if (item >= n) return;
-    ExTask t = ds_ex_task(a, sh, down, item);
+    ExTask t = ds_ex_task(a, sh, down, many, item);
     DnActs da;
     if (down) ds_dn_acts(a, da, t, slot8);
     Words w;
@@ -420,7 +421,7 @@ __device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, bo
             __syncwarp();
             ds_ring_words(w, ring, slot);
             __syncwarp();
-            if (ask < n) ds_ex_request(a, sh, down, ly, ring, slot, ds_ex_task(a, sh, down, ask));
+            if (ask < n) ds_ex_request(a, sh, down, ly, ring, slot, ds_ex_task(a, sh, down, many, ask));
             ds_commit();
             ask += gridDim.x;
             if (++slot == DS_DEPTH) slot = 0;
@@ -430,7 +431,7 @@ __device__ __forceinline__ void ds_experts_phase(const DsArgs &a, Shared &sh, bo
         if (!fresh) ds_pass(t, t.rest);
         else {
             item += gridDim.x;
-            if (item < n) t = ds_ex_task(a, sh, down, item);
+            if (item < n) t = ds_ex_task(a, sh, down, many, item);
         }
         if (down && item < n) ds_dn_acts(a, da, t, slot8);
         if (multi && cur.n == 2) ds_ex_pass<2>(a, sh, down, red + place, xs, fn, w, cur, slot8);
@@ -710,22 +711,28 @@ __device__ __forceinline__ void ds_router(const DsArgs &a, Shared &sh, const DsL
     }
 }
 
-// the step's distinct experts and the slots k * B + b of each (in order of first use), and the rows that they take
-__device__ __forceinline__ void ds_experts(const DsArgs &a, Shared &sh, bf16 *fn, const uint8_t *slot)
+// the step's distinct experts and the slots k * B + b of each (in order of first use, 32 slots at a time), and the rows that
+// they take
+__device__ __forceinline__ void ds_experts(const DsArgs &a, Shared &sh, bf16 *fn, const uint8_t *slot, bool many)
 {
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x, R = a.K * a.B;
-        int e = -1;
-        if (lane < R) {
-            const int *p = reinterpret_cast<const int *>(slot + a.asg) + lane;
-            ds_poll(a, [&] { e = (int)ds_get(p); return (uint32_t)e; });
-            if ((unsigned)e >= (unsigned)a.E) e = 0;
+        int first = 0;
+#pragma unroll 1
+        for (int h = 0; h < (many && R > 32 ? 2 : 1); h++) {
+            int e = -1;
+            if (h * 32 + lane < R) {
+                const int *p = reinterpret_cast<const int *>(slot + a.asg) + h * 32 + lane;
+                ds_poll(a, [&] { e = (int)ds_get(p); return (uint32_t)e; });
+                if ((unsigned)e >= (unsigned)a.E) e = 0;
+            }
+            __syncwarp();
+            const unsigned m = __match_any_sync(0xffffffffu, e), lt = (1u << lane) - 1u;
+            const unsigned lead = __ballot_sync(0xffffffffu, e >= 0 && (m & lt) == 0u);
+            if ((lead >> lane) & 1u) { const int i = first + __popc(lead & lt); sh.pexp[i] = e | h << 8; sh.pmask[i] = m; }
+            first += __popc(lead);
         }
-        __syncwarp();
-        const unsigned m = __match_any_sync(0xffffffffu, e), lt = (1u << lane) - 1u;
-        const unsigned lead = __ballot_sync(0xffffffffu, e >= 0 && (m & lt) == 0u);
-        if ((lead >> lane) & 1u) { const int i = __popc(lead & lt); sh.pexp[i] = e; sh.pmask[i] = m; }
-        if (lane == 0) sh.npair = __popc(lead);
+        if (lane == 0) sh.npair = first;
     }
     for (int i = DS_THREADS - 1 - (int)threadIdx.x; i < a.B * a.D / 8; i += DS_THREADS) {          // (warp 0, which is late, last)
         uint4 v;
@@ -778,7 +785,7 @@ __device__ __forceinline__ void ds_combine(const DsArgs &a, Shared &sh, float *y
 }
 
 // C rows per task of the dense phases; MULTI: an expert can have more than one slot; MANY: a CTA more than one attention
-// item, or an item and a row (its loop around the attention costs the others 1 %)
+// item, or an item and a row, and more than 32 routed slots (its loops cost the others 1 %)
 template <int C, bool MULTI, bool MANY>
 __global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constant__ DsArgs a)
 {
@@ -854,10 +861,10 @@ __global__ void __launch_bounds__(DS_THREADS, 1) k_dec_step(const __grid_constan
         if (l + 1 < a.L && threadIdx.x == DS_THREADS - 1) gb_arrive(a);
         ds_router(a, sh, ly, wr, red, cur);
         __syncthreads();
-        ds_experts(a, sh, fn, cur);
+        ds_experts(a, sh, fn, cur, MANY);
 #pragma unroll TWICE
         for (int down = 0; down < 2; down++) {
-            ds_experts_phase(a, sh, down, ly, red, xs, fn, dsm + DS_RED, MULTI, cur);
+            ds_experts_phase(a, sh, down, ly, red, xs, fn, dsm + DS_RED, MULTI, MANY, cur);
             __syncthreads();
         }
         ds_combine(a, sh, red, l, cur);
@@ -895,16 +902,17 @@ static DsLayout ds_layout(int B, int D, int KD, int F, int K)
     return w;
 }
 // Above eight slots (six layers, us a step, this form and the chain): nine slots of D 768, 32 experts of 1536, two choices
-// 243 and 361, sixteen 336 and 394 (379 and 485 with 900 cached positions); sixteen of D 256, eight experts of 512 140 and
+// 243 and 361, sixteen 340 and 394 (380 and 485 with 900 cached positions); sixteen of D 256, eight experts of 512 140 and
 // 238; 32 slots of D 256 with one choice of 32 or eight experts 180 and 293, 178 and 286.  With experts of many slots the
 // chain takes sixteen of an expert's rows to the tensor cores at a time, a pass here two: up to four slots per expert, and
 // up to 50 M products a matrix of all slots (four layers, twelve slots of D 1024, eight experts top-2: d_ff 2048, 50 M, 253
-// and 278; d_ff 4096, 100 M, 367 and 301).
+// and 278; d_ff 4096, 100 M, 367 and 301).  Above 32 routed slots up to 38 M: 24 slots of D 512, 16 experts top-2 of 1536
+// (38 M) 325 and 333, 32 of D 256, 16 experts of 512 165 and 289; 20 of D 640, 32 experts of 1536 (39 M) 394 and 384.
 static bool ds_fits(int B, int Tm, int D, int H, int KV, int F, int E, int K)
 {
     return B >= 1 && B <= DS_MAX_B && Tm >= 1 && Tm <= 4096 && D == H * 64 && D % 128 == 0 && D <= 1024 && KV >= 1 && H % KV == 0 &&
-           (KV * 64) % 128 == 0 && F >= 128 && F % 128 == 0 && E >= 1 && E <= 32 && K >= 1 && K <= E && K * B <= DS_MAX_R && K <= DS_WARPS && K * D * 4 <= DS_RED &&
-           B * D <= DS_FN_ELEMS && (B <= 8 ? B * (H + 1) <= sm_count() : B <= sm_count() && K * B <= 4 * E && (size_t)K * B * D * F <= (size_t)48 << 20);
+           (KV * 64) % 128 == 0 && F >= 128 && F % 128 == 0 && E >= 1 && E <= 32 && K >= 1 && K <= E && K * B <= (B <= 8 ? 32 : DS_MAX_R) && K <= DS_WARPS && K * D * 4 <= DS_RED &&
+           B * D <= DS_FN_ELEMS && (B <= 8 ? B * (H + 1) <= sm_count() : B <= sm_count() && K * B <= 4 * E && (size_t)K * B * D * F <= (size_t)(K * B <= 32 ? 48 : 36) << 20);
 }
 
 }  // namespace qlmb

@@ -284,9 +284,9 @@ int qlmb_gemv_decode(void *Y, const void *X, const int8_t *codes, const float *s
  * 304) and the step does nothing.  emb, nf and fn must be 16-byte aligned, the table 8.  ws = qlmb_dec_step_bytes(...)
  * bytes, 256-byte aligned, zeroed once before its first use, not shared by steps that may overlap; a size of 0 means that
  * the shape is not supported and the separate entry points do the step.  Supported: head dimension 64, D <= 1024, at most
- * 32 experts and 32 routed slots (K*B); up to 8 slots with a CTA per attention item and row on the device; above 8 slots
- * with B*D <= 12800, K*B <= 4*E and K*B*D*F <= 48 * 2^20.  A slot whose position is outside its cache is reported and neither
- * read nor written. */
+ * 32 experts; up to 8 slots with K*B <= 32 and a CTA per attention item and row on the device; above 8 and up to 32 slots
+ * with K*B <= 64, B*D <= 12800, K*B <= 4*E and K*B*D*F <= 48 * 2^20 (36 * 2^20 where K*B > 32).  A slot whose position is
+ * outside its cache is reported and neither read nor written. */
 typedef struct qlmb_dec_step_args {
     int B, Tm, L, D, H, KV, F, E, K;
     const void *layers;

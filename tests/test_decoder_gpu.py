@@ -385,6 +385,9 @@ def test_one_launch_step_equals_the_chain(cuda, B, D, KV, E, K, F, fill, Tm):
     (12, 1024, 16, 32, 2, 640, 20, 64),     # two items of a CTA, rows' owners among them; nearly all of the rows' room
     (16, 640, 10, 8, 2, 384, 600, 640),     # 32 routed slots, four of each expert, several passes of keys
     (32, 256, 2, 8, 1, 128, 40, 64),        # one choice a slot; grouped heads
+    (17, 512, 8, 32, 2, 384, 90, 128),      # 34 routed slots: two of them in the second half of the list
+    (32, 384, 6, 16, 2, 256, 30, 64),       # 64, most experts in both halves
+    (21, 128, 2, 16, 3, 128, 300, 640),     # 63 of three choices, one row slice
 ])
 def test_one_launch_step_of_more_slots_equals_the_chain(cuda, B, D, KV, E, K, F, fill, Tm):
     """The same above eight slots, where the attention's items outnumber the CTAs or share them with the rows' owners."""
@@ -438,8 +441,9 @@ def test_shapes_of_the_one_launch_step(cuda):
     import cudalm_c_b200 as q
     takes = [bool(q.lib().qlmb_dec_step_bytes(B, 64, D, D // 64, D // 64, F, E, K))
              for B, D, F, E, K in ((8, 1024, 8192, 8, 4), (9, 1024, 256, 8, 2), (12, 1024, 2048, 8, 2), (12, 1024, 2176, 8, 2), (13, 1024, 256, 32, 2),
-                                   (16, 768, 256, 8, 2), (16, 768, 256, 7, 2), (17, 512, 256, 32, 2), (32, 256, 256, 8, 1), (33, 256, 256, 32, 1))]
-    assert takes == [True, True, True, False, False, True, False, False, True, False]
+                                   (16, 768, 256, 8, 2), (16, 768, 256, 7, 2), (25, 512, 256, 32, 2), (26, 512, 256, 32, 2), (32, 256, 256, 16, 2), (32, 256, 256, 15, 2),
+                                   (22, 256, 256, 32, 3), (32, 256, 256, 8, 1), (33, 256, 256, 32, 1), (8, 256, 256, 8, 5))]
+    assert takes == [True, True, True, False, False, True, False, True, False, True, False, False, True, False, False]
 
 
 @pytest.mark.parametrize("L", [1, 2, 3, 4])
