@@ -56,7 +56,7 @@ def all_to_all_rows(out, inp, out_splits, in_splits, group=None):
 class ExpertParallelLayer:
     """One MoE layer with E/W local experts per rank (weak scaling: N tokens per rank)."""
 
-    launches_per_step = 27          # library kernels per forward+backward on a rank
+    launches_per_step = 26          # library kernels per forward+backward on a rank
 
     def __init__(self, cfg, dev, rank, world, seed=1234, aux=0.03, group=None, weights=None, row_capacity=None):
         from . import qlm
@@ -164,7 +164,7 @@ class PeerExpertParallelLayer:
     exchange only the routing table (one fixed-size all-gather) and two one-element all-reduces
     that act as stream-ordered barriers; nothing waits on the host."""
 
-    launches_per_step = 22          # library kernels per forward+backward on a rank
+    launches_per_step = 21          # library kernels per forward+backward on a rank
 
     def __init__(self, cfg, dev, rank, world, seed=1234, aux=0.03, group=None, weights=None, ext=None):
         """ext (a model's own storage instead of the synthetic weights and inputs of the bench):
