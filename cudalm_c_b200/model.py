@@ -497,7 +497,7 @@ class Decoder:
         for l, ly in enumerate(m.layers):
             w, f = ly["w"], m.fl[l]
             att = torch.empty(B, c.D, dtype=torch.bfloat16, device=m.dev)
-            if c.KD == c.D and 4 < B <= 64:
+            if c.KD == c.D and c.hd == 64 and 4 < B <= 64:
                 # wq, wk, wv are consecutive spans of one shape: one GEMV launch for the three with the norm in front of them
                 # applied while the row is staged; the attention adds its head's slice sums, rotates and appends them
                 check(L_.qlmb_dec_qkv_attn(ptr(att), ptr(self.K[l]), ptr(self.V[l]), ptr(x), ptr(f["an1"]), ptr(w["wq"][0]), ptr(w["wq"][1]),
