@@ -218,6 +218,7 @@ extern "C" int qlmb_linear_wgrad(float *dW, const void *dY, const void *X, int l
         if (beta == 0.0f) QLMB_CUDA(cudaMemsetAsync(dW, 0, (size_t)K * N * sizeof(float), st));
         return QLMB_OK;
     }
+    QLMB_REQUIRE(((uintptr_t)dW & 15) == 0, "qlmb_linear_wgrad: dW must be 16-byte aligned");
     const int Md = layout == QLMB_KN ? K : N, Nd = layout == QLMB_KN ? N : K;
     int S = 1;
     const int stages = (M + 63) / 64, tiles = ((Md + 255) / 256) * ((Nd + 255) / 256), pairs = sm_count() / 2;
@@ -240,12 +241,12 @@ extern "C" int qlmb_qkv_fwd(const qlmb_qkv *p, void *Yq, void *Yk, void *Yv, con
     int rc = check_qkv("qlmb_qkv_fwd", p);
     if (rc || p->M == 0) return rc;
     QLMB_REQUIRE(Yq && Yk && Yv && X, "qlmb_qkv_fwd: NULL argument");
+    QLMB_REQUIRE((((uintptr_t)Yq | (uintptr_t)Yk | (uintptr_t)Yv) & 15) == 0, "qlmb_qkv_fwd: the outputs must be 16-byte aligned");
     cudaStream_t st = as_stream(stream);
     void *const Y[3] = {Yq, Yk, Yv};
     const int N[3] = {p->D, p->KD, p->KD};
     // one launch over the column tiles of all three, q and k rotated on the way out
-    if (gemm_pair_takes(p->D) && gemm_pair_takes(p->KD) && ((((uintptr_t)Yq | (uintptr_t)Yk | (uintptr_t)Yv) & 15) == 0) &&
-        ((((uintptr_t)p->cosb | (uintptr_t)p->sinb) & 15) == 0)) {
+    if (gemm_pair_takes(p->D) && gemm_pair_takes(p->KD) && (((uintptr_t)p->cosb | (uintptr_t)p->sinb) & 15) == 0) {
         GemmLaunch g = {};
         g.bmode = B_DEQ_MN; g.epi = EPI_MATS; g.sched = SCHED_DENSE;
         g.a[0] = X; g.a_rows = p->M; g.a_cols = p->D;
@@ -270,11 +271,12 @@ extern "C" int qlmb_qkv_bwd(const qlmb_qkv *p, void *dX, float *dWq, float *dWk,
     if (rc) return rc;
     QLMB_REQUIRE(dWq && dWk && dWv && (p->M == 0 || (dX && dq && dk && dv && X)), "qlmb_qkv_bwd: NULL argument");
     QLMB_REQUIRE(beta == 0.0f || beta == 1.0f, "qlmb_qkv_bwd: beta %g", beta);
+    QLMB_REQUIRE(p->M == 0 || (((uintptr_t)dX | (uintptr_t)dWq | (uintptr_t)dWk | (uintptr_t)dWv) & 15) == 0, "qlmb_qkv_bwd: the outputs must be 16-byte aligned");
     cudaStream_t st = as_stream(stream);
     const int M = p->M, D = p->D, N[3] = {D, p->KD, p->KD};
     const void *const dY[3] = {dq, dk, dv};
     float *const dW[3] = {dWq, dWk, dWv};
-    if (M > 0 && gemm_pair_takes(D) && ((uintptr_t)dX & 15) == 0) {      // one contraction over the columns of dq, dk and dv
+    if (M > 0 && gemm_pair_takes(D)) {      // one contraction over the columns of dq, dk and dv
         GemmLaunch g = {};
         g.bmode = B_DEQ_K; g.epi = EPI_MATS; g.sched = SCHED_DENSE;
         g.a_rows = M; g.a_cols = D; g.w_rows = D; g.w_cols = D; g.nmat = 1; g.N_mat[0] = D; g.outs[0] = dX;

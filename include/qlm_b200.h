@@ -249,7 +249,7 @@ int qlmb_linear_fwd(void *Y, const void *X, const int8_t *codes, const float *sc
 int qlmb_linear_dgrad(void *dX, const void *dY, const int8_t *codes, const float *scales,
                       int layout, int M, int K, int N, float beta, int dtype, void *stream);
 
-/* g_atb (cudalm.cu:3190-3202): dW (fp32, the shape of W for `layout`)
+/* g_atb (cudalm.cu:3190-3202): dW (fp32, 16-byte aligned, the shape of W for `layout`)
  * = beta*dW + X^T dY resp. dY^T X; beta in {0,1} (the reference is always 1). */
 int qlmb_linear_wgrad(float *dW, const void *dY, const void *X, int layout, int M, int K, int N,
                       float beta, int dtype, void *stream);
@@ -258,7 +258,8 @@ int qlmb_linear_wgrad(float *dW, const void *dY, const void *X, int layout, int 
  * Yv [M][KD] = X W, W = codes of [D][D], [D][KD], [D][KD] (layout KN), q and k rotated as qlmb_rope does it with heads of 64
  * (row n has position n % T; tables [>= T][32]).  D and KD must be multiples of 128.
  * qlmb_qkv_bwd: dX = dq Wq^T + dk Wk^T + dv Wv^T (bf16, overwritten) and dW = beta * dW + X^T dY for each (fp32, beta in
- * {0,1}); dq and dk are gradients of the projections, i.e. rotated back (qlmb_attn_bwd_rope, or qlmb_rope with back). */
+ * {0,1}); dq and dk are gradients of the projections, i.e. rotated back (qlmb_attn_bwd_rope, or qlmb_rope with back).
+ * All outputs of both must be 16-byte aligned. */
 typedef struct qlmb_qkv {
     int M, D, KD, T;
     const int8_t *codes[3];

@@ -158,6 +158,31 @@ def test_dec_step_rejects_misaligned_arguments_without_a_gpu():
         assert L.qlmb_dec_step(DecStepArgs(*shape, *bad), None) == 1 and needle in L.qlmb_last_error(), i
 
 
+def test_misaligned_gradients_of_linears_are_refused_without_a_gpu():
+    """The weight gradients leave, and are added up, in 16-byte pieces: a pointer that is not aligned for them is an error of the
+    call, whichever form would take the shape (2048: sliced only when the three are made together)."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200._lib import Qkv
+    L = q.lib()
+    for D in (768, 2048):
+        p = Qkv(8192, D, D, 1024)
+        for i in range(3):
+            p.codes[i], p.scales[i] = 4096, 4096
+        p.cosb, p.sinb = 4096, 4096
+        for i in range(3):
+            outs = [4096] * 3
+            outs[i] += 4
+            assert L.qlmb_qkv_fwd(p, *outs, 4096, None) == 1 and b"qlmb_qkv_fwd: the outputs must be 16-byte aligned" in L.qlmb_last_error()
+        for i in range(4):
+            outs = [4096] * 4
+            outs[i] += 4
+            assert L.qlmb_qkv_bwd(p, *outs, 4096, 4096, 4096, 4096, 0.0, None) == 1
+            assert b"qlmb_qkv_bwd: the outputs must be 16-byte aligned" in L.qlmb_last_error()
+        for layout in (0, 1):
+            assert L.qlmb_linear_wgrad(4100, 4096, 4096, layout, 8192, D, D, 0.0, 1, None) == 1
+            assert b"qlmb_linear_wgrad: dW must be 16-byte aligned" in L.qlmb_last_error()
+
+
 def test_header_is_plain_c_and_links_from_c(tmp_path):
     """include/qlm_b200.h compiles as C99 with warnings as errors and a C program linked against the library runs the
     argument-error paths (status + message, no exit) on a machine without a GPU."""
