@@ -153,6 +153,15 @@ extern "C" int qlmb_linear_dgrad(void *dX, const void *dY, const int8_t *codes, 
     return gemm_launch(g, st);
 }
 
+// Row slices of one matrix's weight gradient [Md][Nd] over M rows
+static int wgrad_slices(int Md, int Nd, int M)
+{
+    const int stages = (M + 63) / 64, tiles = ((Md + 255) / 256) * ((Nd + 255) / 256), pairs = sm_count() / 2;
+    int S = 1;
+    while (S < 16 && tiles * S * 2 <= pairs && stages / (2 * S) >= 8) S *= 2;
+    return S;
+}
+
 // The weight gradients of nmat matrices of one size on the same X: dW[i][K,N] = X^T dY[i] (KN) or dW[i][N,K] = dY[i]^T X (NK).
 // A small weight matrix gives few output tiles (768 x 768: 9 tiles of 256 x 256 for 74 SM pairs) over a
 // long contraction (the M rows).  Then the rows are cut into S slices that run as the "experts" of the
@@ -168,8 +177,12 @@ static int wgrad_mats(float *const *dW, const void *const *dY, int nmat, int S, 
     // Rows that divide evenly keep their slices' partial sums in the shared piece, behind the converted operands: a step
     // that is captured after a first eager one finds it large enough, and an allocation and a free node for each of its
     // calls would cost 0.6 % of a training step.  Other row counts, which need no scratch uncut, take their own.
+    // Evenly: into the slices of one matrix alone, also where several are made together in another number of slices.  Calls
+    // whose single gradients have scratch of their own, or need none, may run on several streams at once and be replayed
+    // from a graph after larger ones.
     const size_t part_bytes = S > 1 ? (size_t)nmat * S * Md * Nd * sizeof(float) : 0;
-    const bool shared = S > 1 && M % (256 * S) == 0;
+    const int one = wgrad_slices(Md, Nd, M);
+    const bool shared = S > 1 && one > 1 && M % (256 * one) == 0;
     StreamScratch own(st);
     if (S > 1 && !shared && !own.get(part_bytes)) S = 1;
     if (S == 1 && nmat > 1) return -1;                   // the caller takes the matrices one by one
@@ -219,11 +232,7 @@ extern "C" int qlmb_linear_wgrad(float *dW, const void *dY, const void *X, int l
         return QLMB_OK;
     }
     QLMB_REQUIRE(((uintptr_t)dW & 15) == 0, "qlmb_linear_wgrad: dW must be 16-byte aligned");
-    const int Md = layout == QLMB_KN ? K : N, Nd = layout == QLMB_KN ? N : K;
-    int S = 1;
-    const int stages = (M + 63) / 64, tiles = ((Md + 255) / 256) * ((Nd + 255) / 256), pairs = sm_count() / 2;
-    while (S < 16 && tiles * S * 2 <= pairs && stages / (2 * S) >= 8) S *= 2;
-    return wgrad_mats(&dW, &dY, 1, S, X, layout, M, K, N, beta, dtype, st);
+    return wgrad_mats(&dW, &dY, 1, layout == QLMB_KN ? wgrad_slices(K, N, M) : wgrad_slices(N, K, M), X, layout, M, K, N, beta, dtype, st);
 }
 
 // ---- the three input projections of an attention block (gpu_forward's wq, wk, wv with k_rope, cudalm.cu:5651-5660, and their part

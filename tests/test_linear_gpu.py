@@ -402,3 +402,43 @@ def test_attention_gradients_rotated_back_on_the_way_out(cuda, B, T, H, KV, win)
     for d, r, n in ((dQ, rQ, H), (dK, rK, KV)):
         block.rope(d, *rot, n, 64, T, back=True)
         assert float((d.float() - r.float()).norm()) <= 2 ** -7 * float(d.float().norm()) + 1e-6
+
+
+@pytest.mark.parametrize("M,D", [(4608, 768), (1024, 1792)])
+def test_joint_weight_gradients_under_capture_and_on_two_streams(cuda, M, D):
+    """q, k and v's gradients in slices, where one matrix alone has scratch of its own (4608 rows: four slices that do not divide
+    them) or none (1792 columns: no slices): replays are not disturbed by larger calls since, two streams may run such calls at
+    once."""
+    from cudalm_c_b200 import block, linear
+    cosb, sinb = block.rope_tables(64, 64, device=cuda)
+    ws = [(lambda q: (q.d, q.s))(quantise(cuda, D, D, 60 + i)[0]) for i in range(3)]
+
+    def call(m, seed):
+        g = torch.Generator(device=cuda); g.manual_seed(seed)
+        x, dq, dk, dv = (torch.randn(m, D, device=cuda, generator=g).bfloat16() for _ in range(4))
+        return lambda dw: linear.qkv_bwd(dw, dq, dk, dv, x, ws, cosb, sinb, 64, beta=0.0)
+    new = lambda: [torch.full((D * D,), -1.0, device=cuda) for _ in range(3)]
+    one, two, dw = call(M, 1), call(M, 2), new()
+    want = []
+    for f in (one, two):
+        want.append(new())
+        f(want[-1])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        one(dw)
+    call(8 * 2048, 3)(new())                              # (rows that divide evenly: the largest shared piece of the shape)
+    for _ in range(3):
+        for t in dw:
+            t.fill_(-1.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(dw, want[0]))
+    streams, outs = [torch.cuda.Stream() for _ in range(2)], [[new() for _ in range(20)] for _ in range(2)]
+    torch.cuda.synchronize()
+    for i in range(20):
+        for s, f, o in zip(streams, (one, two), outs):
+            with torch.cuda.stream(s):
+                f(o[i])
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for o, w in zip(outs, want) for t in o for a, b in zip(t, w))
