@@ -446,7 +446,7 @@ struct AttnBwdParams {
     const float *lse;
     float *drow;                                              // written by dq, read by dkv
     const bf16 *O, *dA;
-    bf16 *dQ, *dK, *dV;
+    bf16 *dQ, *dK, *dV;                                       // dQ NULL: dq makes drow only
     const float *cosb, *sinb;                                 // not NULL: dQ and dK leave rotated back
     int B, T, H, KV, win, nqt;
     float scale, scale_log2;
@@ -938,7 +938,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
             if (lane == 0) mbar_arrive(smem_u32(ds_full));
         }
         if (ok) ok = at_wait(smem_u32(acc_done), (uint32_t)(nt - 1) & 1u, abort_flag, p.errword, 323);
-        if (ok) {
+        if (ok && p.dQ) {
             tc_fence_after();
             // each of the row's two threads stores half of it
             bf16 *dst = p.dQ + ((size_t)b * p.T + i) * ((size_t)p.H * AT_HD) + (size_t)h * AT_HD;
@@ -1030,7 +1030,13 @@ static int attn_bwd_impl(void *dQ, void *dK, void *dV, float *drow, const void *
         configured_dev[dev_] = true;
     }
     cudaStream_t st = as_stream(stream);
-    QLMB_CUDA(pdl_launch_small(k_attn_bwd_dq, dim3((unsigned)(p.nqt * B * H)), dim3(AT_BWD_THREADS), AT_DQ_SMEM, st, p));
+    // dQ in the place of Q or dA, which dkv reads as well: only drow comes first then, dQ behind dkv
+    const bool in_place = dQ == Q || dQ == dA;
+    auto launch_dq = [&](void *dst) {
+        p.dQ = (bf16 *)dst;
+        return pdl_launch_small(k_attn_bwd_dq, dim3((unsigned)(p.nqt * B * H)), dim3(AT_BWD_THREADS), AT_DQ_SMEM, st, p);
+    };
+    QLMB_CUDA(launch_dq(in_place ? nullptr : dQ));
     const int grp = H / KV, units = p.nqt * B * KV;
     if ((grp == 2 || grp == 4 || grp == 8) && units <= 2 * sm_count()) {
         cudaLaunchConfig_t cfg = {};
@@ -1045,6 +1051,7 @@ static int attn_bwd_impl(void *dQ, void *dK, void *dV, float *drow, const void *
     } else {
         QLMB_CUDA(pdl_launch_small(k_attn_bwd_dkv<false>, dim3((unsigned)units), dim3(AT_BWD_THREADS), AT_DKV_SMEM, st, p));
     }
+    if (in_place) QLMB_CUDA(launch_dq(dQ));
     QLMB_LAUNCH_CHECK("k_attn_bwd");
     return QLMB_OK;
 }

@@ -671,11 +671,12 @@ int qlmb_attn_fwd(void *O, float *lse, const void *Q, const void *K, const void 
                   int KV, int hd, int win, void *stream);
 
 /* Attention backward (gpu_backward, cudalm.cu:5918-5960: k_attn_drow, then dQ / dK / dV; CPU twins
- * cpu_kern.h:255-322).  drow[b,h,t] = sum_d dA * O is written first (B*H*T floats, also an output);
+ * cpu_kern.h:255-322).  drow[b,h,t] = sum_d dA * O (B*H*T floats) is an output as well;
  * dQ [B*T, H*hd], dK and dV [B*T, KV*hd] are bf16 and are overwritten (the reference zeroes its
- * buffers and accumulates once).  Every element has one writer and a fixed summation order:
- * dK/dV come from one CTA per (sequence, K/V head, key tile) that walks the heads of the group and the
- * query tiles, dQ from one CTA per (sequence, head, query tile). */
+ * buffers and accumulates once).  dQ may be in the place of Q, dA or O, at the cost of a second pass over
+ * the scores for the first two.  Every element has one writer and a fixed summation order:
+ * dQ comes from one CTA per (sequence, head, query tile), dK/dV from one CTA per (sequence, K/V head, key
+ * tile) that walks the heads of the group and the query tiles, or from a cluster of CTAs, one per head. */
 int qlmb_attn_bwd(void *dQ, void *dK, void *dV, float *drow, const void *Q, const void *K, const void *V,
                   const void *O, const void *dA, const float *lse, int B, int T, int H, int KV, int hd,
                   int win, void *stream);

@@ -150,3 +150,27 @@ def test_attn_gradients_of_grouped_heads(cuda, B, T, H, KV, win):
     assert np.abs(drow.cpu().numpy() - ref).max() < 2 ** -7 * np.abs(ref).max()
     block.rope(dK, *rot, KV, 64, T, back=True)
     assert float((dK.float() - rK.float()).norm()) <= 2 ** -7 * float(rK.float().norm())
+
+
+@pytest.mark.parametrize("B,T,H,KV,win,rope", [(2, 200, 4, 4, 0, False), (1, 130, 8, 2, 40, True), (3, 64, 2, 1, 0, True)])
+@pytest.mark.parametrize("place", ["Q", "dA", "O"])
+def test_dq_in_the_place_of_an_input(cuda, B, T, H, KV, win, rope, place):
+    """dQ over Q, dA or O: the bits of separate buffers, with one CTA and with a cluster for dK and dV."""
+    import cudalm_c_b200 as q
+    from cudalm_c_b200 import attn, block
+    from cudalm_c_b200._lib import ptr, stream_ptr
+    g = torch.Generator(device=cuda); g.manual_seed(31)
+    rnd = lambda c: torch.randn(B * T, c * 64, device=cuda, generator=g).to(torch.bfloat16)
+    t = dict(Q=rnd(H), K=rnd(KV), V=rnd(KV), dA=rnd(H))
+    t["O"], lse = attn.attn_fwd(t["Q"], t["K"], t["V"], B, T, H, KV, win)
+    rot = block.rope_tables(T, 64, device=cuda) if rope else None
+    want = attn.attn_bwd(t["Q"], t["K"], t["V"], t["O"], t["dA"], lse, B, T, H, KV, win, rope=rot)
+    dK, dV, drow = torch.empty_like(t["K"]), torch.empty_like(t["V"]), torch.empty_like(want[3])
+    args = [ptr(x) for x in (t[place], dK, dV, drow, t["Q"], t["K"], t["V"], t["O"], t["dA"], lse)]
+    if rope:
+        q.check(q.lib().qlmb_attn_bwd_rope(*args, ptr(rot[0]), ptr(rot[1]), B, T, H, KV, 64, win, stream_ptr()))
+    else:
+        q.check(q.lib().qlmb_attn_bwd(*args, B, T, H, KV, 64, win, stream_ptr()))
+    torch.cuda.synchronize()
+    q.check(q.lib().qlmb_check_device(None))
+    assert all(torch.equal(a, b) for a, b in zip((t[place], dK, dV, drow), want))
