@@ -63,9 +63,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
                  ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
 }
 
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, int y)     // one box into L2
-{ asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory"); }
-
 // shared -> global bulk tensor store of one box; rows or columns outside the tensor are not written
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t src, int x, int y)
 {
