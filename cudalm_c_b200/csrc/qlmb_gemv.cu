@@ -1447,31 +1447,37 @@ static int gemv_stack_impl(void *Y, const void *X, const int8_t *codes, const fl
                  "qlmb_gemv_decode_stack: nmat=%d B=%d K=%d N=%d", nmat, B, K, N);
     cudaStream_t st = as_stream(stream);
     const int R = nmat * B, nblk = (N + 255) / 256;
-    int nslice = (4 * sm_count()) / (nblk * R);
-    if (nslice > K / 64) nslice = K / 64;
-    if (nslice < 1) nslice = 1;
-    int kslice = ((K + nslice - 1) / nslice + 127) / 128 * 128;
-    nslice = (K + kslice - 1) / kslice;
-    const bool groups = B > 4;                           // more than four rows: groups share one pass over a matrix
-    const bool tc = groups && dtype == QLMB_BF16 && (N % 64) == 0;   // bf16 rows: warp-level MMAs, 16 or 32 rows per group
-    const int mt = mma_mt(B, K, N, nmat);
-    const int nz = tc ? nmat * ((B + 16 * mt - 1) / (16 * mt)) : nmat * ((B + 7) / 8);
-    const MmaPlan pl = mma_plan(K, N, nz, mt);
-    if (groups) nslice = tc ? pl.ns : rows8_slices(K, N, nz);
-    void *ws = nullptr;
-    int rc = workspace((size_t)nslice * R * N * sizeof(float), &ws);
-    if (rc) return rc;
-    float *part = (float *)ws;
-    if (groups) {
+    const float *part = nullptr;
+    int nslice = 0, rc;
+    if (B > 4 && dtype == QLMB_BF16) {                   // bf16 rows: warp-level MMAs, groups of 16 or 32 rows share one pass over a matrix
+        if ((rc = gemv_stack_slices(&part, &nslice, X, gamma, codes, scales, nmat, B, K, N, 0, st))) return rc;
+    } else if (B > 4) {                                  // fp32 rows: groups of eight
+        const int nz = nmat * ((B + 7) / 8);
+        nslice = rows8_slices(K, N, nz);
+        void *ws = nullptr;
+        if ((rc = workspace((size_t)nslice * R * N * sizeof(float), &ws))) return rc;
         Rows8 a = {};
-        a.part = part; a.X = X; a.x_dtype = dtype; a.K = K; a.N = N;
+        a.part = (float *)ws; a.X = X; a.x_dtype = dtype; a.K = K; a.N = N;
         a.codes = (const uint8_t *)codes; a.scales = scales; a.e_codes = (size_t)K * N / 2; a.e_scales = (size_t)K * N / 128;
         a.B = B; a.nmat = nmat; a.rows_out = R; a.gamma = gamma;
-        if ((rc = tc ? mma_launch(a, nz, pl, mt, st) : rows8_launch(a, nz, nslice, st))) return rc;
-    } else if ((size_t)nblk * nslice * R <= (size_t)2 * sm_count())
-        launch_kn<1, 4>(B > 4, dim3(nblk, nslice, R), (size_t)kslice * sizeof(float), st, part, X, dtype, (const uint8_t *)codes, scales, 1, K, N, kslice, nullptr, (size_t)K * N / 2, (size_t)K * N / 128, B, gamma);
-    else
-        launch_kn<1, 2>(B > 4, dim3(nblk, nslice, R), (size_t)kslice * sizeof(float), st, part, X, dtype, (const uint8_t *)codes, scales, 1, K, N, kslice, nullptr, (size_t)K * N / 2, (size_t)K * N / 128, B, gamma);
+        part = a.part;
+        if ((rc = rows8_launch(a, nz, nslice, st))) return rc;
+    } else {
+        nslice = (4 * sm_count()) / (nblk * R);
+        if (nslice > K / 64) nslice = K / 64;
+        if (nslice < 1) nslice = 1;
+        const int kslice = ((K + nslice - 1) / nslice + 127) / 128 * 128;
+        nslice = (K + kslice - 1) / kslice;
+        void *ws = nullptr;
+        if ((rc = workspace((size_t)nslice * R * N * sizeof(float), &ws))) return rc;
+        part = (float *)ws;
+        const dim3 grid(nblk, nslice, R);
+        const size_t ec = (size_t)K * N / 2, es = (size_t)K * N / 128;
+        if ((size_t)nblk * nslice * R <= (size_t)2 * sm_count())
+            launch_kn<1, 4>(false, grid, (size_t)kslice * sizeof(float), st, (float *)ws, X, dtype, (const uint8_t *)codes, scales, 1, K, N, kslice, nullptr, ec, es, B, gamma);
+        else
+            launch_kn<1, 2>(false, grid, (size_t)kslice * sizeof(float), st, (float *)ws, X, dtype, (const uint8_t *)codes, scales, 1, K, N, kslice, nullptr, ec, es, B, gamma);
+    }
     if (fr) pdl_launch(B > 4, k_gemv_finish_res_norm, dim3(R), dim3(256), 0, st, (bf16 *)Y, (bf16 *)fr->Fn, part, nslice, R, N, (const bf16 *)fr->res, fr->gamma);
     else if (fq) pdl_launch(B > 4, k_gemv_finish_qkv, dim3((unsigned)(((size_t)R * N / 2 + 255) / 256)), dim3(256), 0, st, (bf16 *)Y, (bf16 *)fq->Kc, (bf16 *)fq->Vc, part, nslice, B, N, fq->hd, fq->cosb, fq->sinb, fq->pos, fq->Tm, device_error_word());
     else pdl_launch(B > 4, k_gemv_finish, dim3((unsigned)(((size_t)R * N + 255) / 256)), dim3(256), 0, st, Y, dtype, part, nslice, (size_t)R * N);

@@ -89,7 +89,7 @@ int moe_decode_experts(const qlmb_moe_layer *L, void *out, const void *f_in, con
                        const float *gate, cudaStream_t st, int *perm = nullptr, int *off = nullptr, int *counts = nullptr,
                        int *bad = nullptr, int perm_ready = 0);
 size_t moe_decode_workspace(const qlmb_moe_layer *L);    // bytes it asks the shared workspace for
-// the K-slice sums of nmat stacked matrices' GEMV (5 to 64 bf16 rows) in the shared workspace, at least `min_bytes` of it
+// the K-slice sums of nmat stacked matrices' GEMV (more than four bf16 rows) in the shared workspace, at least `min_bytes` of it
 int gemv_stack_slices(const float **part, int *nslice, const void *X, const float *gamma, const int8_t *codes, const float *scales,
                       int nmat, int B, int K, int N, size_t min_bytes, cudaStream_t st);
 
