@@ -185,8 +185,11 @@ static int wgrad_mats(float *const *dW, const void *const *dY, int nmat, int S, 
     const bool shared = S > 1 && one > 1 && M % (256 * one) == 0;
     StreamScratch own(st);
     if (S > 1 && !shared && !own.get(part_bytes)) S = 1;
-    if (S == 1 && nmat > 1) return -1;                   // the caller takes the matrices one by one
-    int rc;
+    int rc = QLMB_OK;
+    if (S == 1 && nmat > 1) {                            // no scratch: one by one
+        for (int i = 0; i < nmat && !rc; i++) rc = wgrad_mats(dW + i, dY + i, 1, 1, X, layout, M, K, N, beta, dtype, st);
+        return rc;
+    }
     void *ws = nullptr;
     if (conv || shared) { rc = workspace(conv + (shared ? part_bytes : 0), &ws); if (rc) return rc; }
     float *part = shared ? (float *)((uint8_t *)ws + conv) : (float *)own.p;
@@ -308,10 +311,7 @@ extern "C" int qlmb_qkv_bwd(const qlmb_qkv *p, void *dX, float *dWq, float *dWk,
             const double c = (double)((tiles * s + pairs - 1) / pairs) * ((stages + s - 1) / s + 6) + s * mb2;
             if (!S || c < best) { S = s; best = c; }
         }
-        if (S) {
-            rc = wgrad_mats(dW, dY, 3, S, X, QLMB_KN, M, D, D, beta, QLMB_BF16, st);
-            if (rc >= 0) return rc;
-        }
+        if (S) return wgrad_mats(dW, dY, 3, S, X, QLMB_KN, M, D, D, beta, QLMB_BF16, st);
     }
     for (int i = 0; i < 3; i++)
         if ((rc = qlmb_linear_wgrad(dW[i], dY[i], X, QLMB_KN, M, D, N[i], beta, QLMB_BF16, stream))) return rc;
