@@ -92,8 +92,8 @@ __device__ __forceinline__ float ex2(float x)
 }
 template <int M> struct AtMode { static constexpr int value = M; };     // which masks a tile needs
 
-// The same with the rotation of pairs (j, j + 32) undone: cp, sp = the row's 32 cosines and sines.  part 0: columns 0 .. 31 of the
-// row, 1: columns 32 .. 63, 2: all of it.
+// 64 fp32 TMEM columns of this thread's lane, times mul, the rotation of pairs (j, j + 32) undone (cp, sp = the row's 32 cosines
+// and sines) -> bf16 in global memory.  part 0: columns 0 .. 31 of the row, 1: columns 32 .. 63, 2: all of it.
 __device__ __forceinline__ void attn_store_rot(bf16 *dst, uint32_t taddr, bool live, float mul, const float *cp, const float *sp, int part)
 {
 #pragma unroll
@@ -407,14 +407,15 @@ __global__ void __launch_bounds__(AT_FWD_THREADS, 2) k_attn_fwd(const __grid_con
 // ------------------------------------------------------------------ backward
 // Two kernels, so that every output element has one writer and a fixed summation order:
 //   k_attn_bwd_dkv  one CTA per (sequence, K/V head, tile of 128 keys), walks the heads of the
-//                   group and the query tiles that see these keys; dK and dV accumulate in TMEM.
+//                   group and the query tiles that see these keys; dK and dV accumulate in TMEM
+//                   (few such CTAs: a cluster of them, one per head).
 //   k_attn_bwd_dq   one CTA per (sequence, head, tile of 128 queries), walks the key tiles;
 //                   dQ accumulates in TMEM.
 // Both recompute the scores from Q, K and the saved log-sum-exp:  P = exp(S/sqrt(hd) - lse),
 // dS = P * (dP - D) / sqrt(hd) with dP = dA V^T and D = rowsum(dA * O).  dq runs first: its threads make D of their own row, beside
 // the first tiles' copies, and leave it for dkv (a launch of its own for D read dA and O once more: 6.5 us at 8 x 1024 x 12).
 //
-// The walked tiles are 64 wide, so that two CTAs fit an SM (100 / 80 KB of shared memory, 256 TMEM columns each): the
+// The walked tiles are 64 wide, so that two CTAs fit an SM (98 and 97 KiB of shared memory, 256 TMEM columns each): the
 // element-wise phase of one runs beside the MMAs of the other.
 // dq: the scores of the next step are issued as soon as the element-wise warps hold this step's in registers, dS is an operand
 // in TMEM.  dkv: P^T and dS^T are operands in TMEM too; its 256 columns leave them no room of their own, so they overwrite the
@@ -425,11 +426,12 @@ __global__ void __launch_bounds__(AT_FWD_THREADS, 2) k_attn_fwd(const __grid_con
 // on the edge tiles 67 + 49; these 62 + 38.  (dkv with the scores ahead and P^T, dS^T through shared memory: 62 as well, its
 // shared memory then busy 84 % of the time.)
 //
-//   warp 0      TMA producer   resident tiles once, the walked tiles through a two-stage ring
-//   warp 1      MMA issuer     scores and dP (two 128 x 64 x 64 MMAs into TMEM), then the two
-//                              accumulating products from P / dS in shared memory
+//   warp 0      TMA producer   resident tiles once, the walked tiles through a four-stage ring (dkv:
+//                              log-sum-exp and D of a tile's queries beside them)
+//   warp 1      MMA issuer     scores and dP (two 128 x 64 x 64 MMAs into TMEM), then the accumulating
+//                              products (dkv: two, dq: one) with P / dS in TMEM as the A operand
 //   warps 2-9   element-wise   thread = one TMEM lane (a key for dkv, a query for dq) x 32 of the
-//                              64 columns: P and dS as bf16 into swizzled K-major tiles.  The factor
+//                              64 columns: P and dS as pairs of bf16 back into TMEM.  The factor
 //                              1/sqrt(hd) of dS (a power of two) is applied to the finished sums.
 constexpr int AT_BI = 64;                       // queries (dkv) or keys (dq) per step
 constexpr int AT_ITILE = AT_BI * AT_HD * 2;     // bytes of a walked tile
@@ -838,7 +840,7 @@ __global__ void __launch_bounds__(AT_BWD_THREADS, 2) k_attn_bwd_dq(const __grid_
         }
         for (int t = 0; ok && t < nt; t++) {
             const int st = t % NS;
-            if (t + 1 < nt) {                                 // next scores first, see k_attn_bwd_dkv
+            if (t + 1 < nt) {                                 // the next scores as soon as the element-wise warps hold this step's
                 const int sn = (t + 1) % NS;
                 ok = at_wait(smem_u32(&kv_full[sn]), (uint32_t)((t + 1) / NS) & 1u, abort_flag, p.errword, 313);
                 if (ok) ok = at_wait(smem_u32(s_free), (uint32_t)t & 1u, abort_flag, p.errword, 314);
