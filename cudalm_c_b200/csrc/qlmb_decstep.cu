@@ -908,6 +908,11 @@ static DsLayout ds_layout(int B, int D, int KD, int F, int K)
 // up to 50 M products a matrix of all slots (four layers, twelve slots of D 1024, eight experts top-2: d_ff 2048, 50 M, 253
 // and 278; d_ff 4096, 100 M, 367 and 301).  Above 32 routed slots up to 38 M: 24 slots of D 512, 16 experts top-2 of 1536
 // (38 M) 325 and 333, 32 of D 256, 16 experts of 512 165 and 289; 20 of D 640, 32 experts of 1536 (39 M) 394 and 384.
+// Up to eight slots there is no such limit; one would lie at about 80 M products with more than sixteen routed slots, which the
+// chain takes in groups, and none below (three layers, eight slots of D 1024, eight experts, this form and the chain: two choices,
+// d_ff 4096 234 and 363, 8192 361 and 497; four choices, 2048 218 and 240, 3072 277 and 248, 4096 326 and 259, 8192 551 and 315).
+// Long caches speak for this form at any number of slots, although a CTA walks one slot and head on its own: 4000 positions, three
+// layers, nine slots of D 768 210 and 516, sixteen 326 and 576, 32 of D 384 259 and 519.
 static bool ds_fits(int B, int Tm, int D, int H, int KV, int F, int E, int K)
 {
     return B >= 1 && B <= DS_MAX_B && Tm >= 1 && Tm <= 4096 && D == H * 64 && D % 128 == 0 && D <= 1024 && KV >= 1 && H % KV == 0 &&

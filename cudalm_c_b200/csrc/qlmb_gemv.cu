@@ -1189,6 +1189,8 @@ __global__ void __launch_bounds__(256) k_gemv_finish_combine(bf16 *out, const bf
 // own: every expert's first group has blocks of its own, whose weights can be requested before the slots are known to be grouped.
 // Where a quarter of the experts or more would stay without rows that reads more for nothing than it saves (12 slots of 32
 // experts, 16.6 of them hit: 368 -> 373 us a step; 64 slots, 31.5 hit: 936 -> 928; 20 slots of 16 experts, 14.8 hit: 418 -> 378).
+// The rule counts on choices that spread.  With slots that are all alike it costs (three layers: 64 with the same two of 32 experts
+// 247 -> 251, 40 with the same one of 16 210 -> 220).
 struct ExpertPlan { MmaPlan pl1, pl2; size_t pg_n, pd_n; int own; };
 static ExpertPlan expert_plan(const qlmb_moe_layer *L)
 {
