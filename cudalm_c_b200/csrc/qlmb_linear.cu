@@ -27,7 +27,8 @@ int workspace(size_t bytes, void **out)
 
 // Scratch of one call, in stream order: calls on several streams and threads get memory of their own, under capture it
 // belongs to the graph, and nothing that a captured call uses is ever replaced by a larger piece (the shared piece above
-// is).  A pool per device keeps up to 64 MB between calls (16 slices on 74 tiles take 20) and gives the rest back.
+// is).  A pool per device keeps up to SCRATCH_KEPT between calls and gives the rest back at the next synchronisation.
+constexpr size_t SCRATCH_KEPT = (size_t)128 << 20;
 struct StreamScratch {
     void *p = nullptr;
     cudaStream_t st;
@@ -44,7 +45,7 @@ struct StreamScratch {
                 cudaMemPoolProps props = {};
                 props.allocType = cudaMemAllocationTypePinned;
                 props.location.type = cudaMemLocationTypeDevice; props.location.id = dev;
-                uint64_t keep = (uint64_t)64 << 20;
+                uint64_t keep = SCRATCH_KEPT;
                 if (cudaMemPoolCreate(&pools[dev], &props) != cudaSuccess) { pools[dev] = nullptr; cudaGetLastError(); return false; }
                 cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
             }
@@ -161,6 +162,11 @@ static int wgrad_slices(int Md, int Nd, int M)
     while (S < 16 && tiles * S * 2 <= pairs && stages / (2 * S) >= 8) S *= 2;
     return S;
 }
+static bool wgrad_even(int Md, int Nd, int M)             // ... cut into slices that are all as long
+{
+    const int S = wgrad_slices(Md, Nd, M);
+    return S > 1 && M % (256 * S) == 0;
+}
 
 // The weight gradients of nmat matrices of one size on the same X: dW[i][K,N] = X^T dY[i] (KN) or dW[i][N,K] = dY[i]^T X (NK).
 // A small weight matrix gives few output tiles (768 x 768: 9 tiles of 256 x 256 for 74 SM pairs) over a
@@ -181,8 +187,7 @@ static int wgrad_mats(float *const *dW, const void *const *dY, int nmat, int S, 
     // whose single gradients have scratch of their own, or need none, may run on several streams at once and be replayed
     // from a graph after larger ones.
     const size_t part_bytes = S > 1 ? (size_t)nmat * S * Md * Nd * sizeof(float) : 0;
-    const int one = wgrad_slices(Md, Nd, M);
-    const bool shared = S > 1 && one > 1 && M % (256 * one) == 0;
+    const bool shared = S > 1 && wgrad_even(Md, Nd, M);
     StreamScratch own(st);
     if (S > 1 && !shared && !own.get(part_bytes)) S = 1;
     int rc = QLMB_OK;
@@ -301,13 +306,16 @@ extern "C" int qlmb_qkv_bwd(const qlmb_qkv *p, void *dX, float *dWq, float *dWk,
             if ((rc = qlmb_linear_dgrad(dX, dY[i], p->codes[i], p->scales[i], QLMB_KN, M, D, N[i], i ? 1.0f : 0.0f, QLMB_BF16, stream))) return rc;
     }
     // The three weight gradients as one launch where they are of one size: of the slice counts the one with the fewest rounds of
-    // tiles times stages, six stages for a tile's start and end, and the slices' partial sums at a stage's time per 2 MB.
+    // tiles times stages, six stages for a tile's start and end, and the slices' partial sums at a stage's time per 2 MB.  Scratch
+    // of the call's own only as large as its pool keeps it: beyond, every step maps and unmaps it (dX and dW of 8192 x 4096 with a
+    // synchronisation every fourth call: 2118 us, three gradients one by one 1447).
     if (M > 0 && p->KD == D && gemm_pair_takes(D)) {
         const int stages = (M + 63) / 64, t1 = (D + 255) / 256, tiles = 3 * t1 * t1, pairs = sm_count() / 2;
         const double mb2 = 3.0 * D * D * 8.0 / 2e6;
+        const bool shared = wgrad_even(D, D, M);
         int S = 0;
         double best = 0.0;
-        for (int s = 2; s <= 8 && stages / s >= 8; s++) {
+        for (int s = 2; s <= 8 && stages / s >= 8 && (shared || (size_t)3 * s * D * D * sizeof(float) <= SCRATCH_KEPT); s++) {
             const double c = (double)((tiles * s + pairs - 1) / pairs) * ((stages + s - 1) / s + 6) + s * mb2;
             if (!S || c < best) { S = s; best = c; }
         }

@@ -404,11 +404,11 @@ def test_attention_gradients_rotated_back_on_the_way_out(cuda, B, T, H, KV, win)
         assert float((d.float() - r.float()).norm()) <= 2 ** -7 * float(d.float().norm()) + 1e-6
 
 
-@pytest.mark.parametrize("M,D", [(4608, 768), (1024, 1792)])
+@pytest.mark.parametrize("M,D", [(4608, 768), (1024, 1792), (1024, 2432)])
 def test_joint_weight_gradients_under_capture_and_on_two_streams(cuda, M, D):
     """q, k and v's gradients in slices, where one matrix alone has scratch of its own (4608 rows: four slices that do not divide
-    them) or none (1792 columns: no slices): replays are not disturbed by larger calls since, two streams may run such calls at
-    once."""
+    them) or none (1792 columns: no slices; 2432: one by one, two slices of the three are more than the scratch pool keeps): replays
+    are not disturbed by larger calls since, two streams may run such calls at once."""
     from cudalm_c_b200 import block, linear
     cosb, sinb = block.rope_tables(64, 64, device=cuda)
     ws = [(lambda q: (q.d, q.s))(quantise(cuda, D, D, 60 + i)[0]) for i in range(3)]
